@@ -45,10 +45,20 @@ int nsa_compress_fwd(const void* x, const void* w, const void* bias, void* y, co
                      const int32_t* cu_out, int nseq, int H, int D, int block, int stride, int max_out,
                      void* stream);
 /* The same forward for B equal-length sequences (x [B*T,H,D], T a multiple of stride): one tcgen05 GEMM per
- * (batch, head, 128 output rows) whose A tiles are TMA boxes over the overlapping windows; y [B,Tc,H,D] with
+ * 128 (position, head) rows whose A tiles are TMA boxes over the overlapping windows; y [B,Tc,H,D] with
  * Tc = (T-block)/stride + 1 (the Conv1d rule of nsa/compression_kv.py:298-307). */
 int nsa_compress_fwd_uniform(const void* x, const void* w, const void* bias, void* y, int B, int T, int H, int D,
                              int block, int stride, void* stream);
+/* The forward of both tensors in one launch of the tcgen05 GEMM.  Ragged sequences: cu_in / cu_out device int32 [nseq+1],
+ * total_in / total_out their last entries.  Equal lengths: cu_in = cu_out = NULL, nseq sequences of T tokens and Tc
+ * positions each.  Any length and start; w_k, w_v in the [block*D, D] layout.  split != 0: small problems may split the
+ * contraction (faster; the last bits then depend on how many positions there are). */
+int nsa_compress_fwd_kv(const void* k, const void* v, const void* w_k, const void* w_v, const void* bias_k,
+                        const void* bias_v, void* ck, void* cv, const int32_t* cu_in, const int32_t* cu_out, int nseq, int T,
+                        int Tc, long long total_in, long long total_out, int H, int D, int block, int stride, int split,
+                        void* stream);
+/* Conv1d weights [D,D,block] (out channel, in channel, offset) -> the [block*D, D] layout above; w_v / out_v may be NULL. */
+int nsa_conv_weight_layout(const void* w_k, const void* w_v, void* out_k, void* out_v, int D, int block, void* stream);
 /* Replaces _compress_kv.backward (nsa/compression_kv.py:219-266, kernels :62-171) and the Conv1d backward.
  * dy [out_tok,H,D] -> dx [tok,H,D] bf16 (NULL to skip), dw [block*D, D] fp32 (NULL to skip),
  * dbias [D] fp32 (NULL to skip).  ws: nsa_compress_bwd_workspace_bytes() bytes, needed when dw != NULL. */
@@ -56,6 +66,16 @@ int nsa_compress_bwd(const void* x, const void* w, const void* dy, void* dx, flo
                      size_t ws_bytes, const int32_t* cu_in, const int32_t* cu_out, int nseq, int H, int D,
                      int block, int stride, int max_in, int total_out, void* stream);
 size_t nsa_compress_bwd_workspace_bytes(int nseq, int H, int D, int block);
+/* The backward of both tensors as tcgen05 GEMMs, for block = stride or 2 * stride.  dk, dv: NULL to skip, accumulate != 0
+ * adds to them.  dw_mode: 0 = dw fp32 in the [block*D, D] layout (dbias fp32), 1 = the same in bf16 (dbias bf16), 2 = dw in
+ * the Conv1d layout [D,D,block] in bf16 (dbias bf16); each of dw_*, dbias_* may be NULL.  Sequences as in
+ * nsa_compress_fwd_kv.  ws: nsa_compress_bwd_kv_workspace_bytes() (0 = this geometry is not covered). */
+size_t nsa_compress_bwd_kv_workspace_bytes(int nseq, int Tc, long long total_out, int ragged, int H, int D, int block,
+                                           int stride);
+int nsa_compress_bwd_kv(const void* k, const void* v, const void* w_k, const void* w_v, const void* dck, const void* dcv,
+                        void* dk, void* dv, int accumulate, void* dw_k, void* dw_v, void* dbias_k, void* dbias_v, int dw_mode,
+                        void* ws, size_t ws_bytes, const int32_t* cu_in, const int32_t* cu_out, int nseq, int T, int Tc,
+                        long long total_in, long long total_out, int H, int D, int block, int stride, void* stream);
 /* No counterpart in the reference.  The same backward as nsa_compress_bwd for callers that must not allocate
  * device memory when they need it (a runtime that has already handed out all of its HBM, a plugin host that owns
  * the allocator): the fp32 partials of the dW reduction go to a 16 MiB device array built into the library, so
@@ -196,6 +216,23 @@ int nsa_cmp_attn_bwd_fused(const void* q, const void* ck, const void* cv, const 
                            float* delta, const void* gate, void* dgate, void* dq, int accumulate_dq, void* dck, void* dcv,
                            void* ws, size_t ws_bytes, int B, int T, int Tc, int Hq, int Hk, int D, int block, int stride,
                            int causal, float scale, int Tq, int q0, void* stream);
+
+/* ---- compressed cache of a generation loop ------------------------------------------------------------------
+ * No counterpart in the reference.  nsa_cache_plan is host arithmetic only (HOST int32 tables [nseq+1] of cumulative
+ * lengths; cu_old = cuc_old = NULL: everything is new) and fills
+ *   table [6*nseq+4] = new token offsets (nseq+1), new compressed offsets (nseq+1), old compressed offsets (nseq+1),
+ *                      offsets of the positions to compute (nseq+1), first of them per sequence (nseq), the sequences
+ *                      longest first (nseq);
+ *   info [3]         = compressed rows in all, longest compressed sequence, positions to compute.
+ * -17 if a sequence became shorter.  nsa_cache_build copies the table to table_dev, moves the rows of ck_old, cv_old
+ * (NULL if there are none) to their new offsets in ck, cv [info[0],H,D] and computes the remaining positions from
+ * k, v [total_in,H,D] with the Conv1d weights conv_k, conv_v [D,D,block].  w_ws: 2*block*D*D bf16 of scratch. */
+int nsa_cache_plan(const int32_t* cu_new, const int32_t* cu_old, const int32_t* cuc_old, int nseq, int block, int stride,
+                   int32_t* table, int32_t* info);
+int nsa_cache_build(const void* k, const void* v, const void* conv_k, const void* conv_v, const void* bias_k,
+                    const void* bias_v, void* w_ws, const void* ck_old, const void* cv_old, void* ck, void* cv,
+                    const int32_t* table, int32_t* table_dev, int nseq, long long total_in, int H, int D, int block, int stride,
+                    void* stream);
 
 /* ---- decode ---------------------------------------------------------------------------------------------
  * No entry point of the reference does this (its module assumes len(q) == len(k), nsa/nsa.py:97); it is the

@@ -22,6 +22,12 @@ SIGNATURES = {
     "nsa_kernel_launch_count": (L, []),
     "nsa_compress_fwd": (I, [P, P, P, P, P, P, I, I, I, I, I, I, P]),
     "nsa_compress_fwd_uniform": (I, [P, P, P, P, I, I, I, I, I, I, P]),
+    "nsa_compress_fwd_kv": (I, [P] * 10 + [I, I, I, L, L, I, I, I, I, I, P]),
+    "nsa_conv_weight_layout": (I, [P, P, P, P, I, I, P]),
+    "nsa_cache_plan": (I, [P, P, P, I, I, I, P, P]),
+    "nsa_cache_build": (I, [P] * 13 + [I, L, I, I, I, I, P]),
+    "nsa_compress_bwd_kv": (I, [P] * 8 + [I, P, P, P, P, I, P, Z, P, P, I, I, I, L, L, I, I, I, I, P]),
+    "nsa_compress_bwd_kv_workspace_bytes": (Z, [I, I, L, I, I, I, I, I]),
     "nsa_compress_bwd": (I, [P, P, P, P, P, P, P, Z, P, P, I, I, I, I, I, I, I, P]),
     "nsa_compress_bwd_workspace_bytes": (Z, [I, I, I, I]),
     "nsa_compress_bwd_noalloc": (I, [P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P]),
@@ -109,11 +115,12 @@ def sel_swa_fwd_workspace_bytes(B, T, Tq, Hq, Hkv, D, S, BS):
 
 
 def ptr(t):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current stream's handle (the raw getter: a torch.cuda.Stream object costs more than a kernel launch)."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def require(t, name, dtype=torch.bfloat16):

@@ -32,59 +32,66 @@ def _cu_tensor(values, device):
     return t
 
 
-class _CompressOne(torch.autograd.Function):
-    """y = compress(x; w, bias) for one tensor.  x [tok,H,D]; w [l*D, D]; bias [D] or None."""
+class _CompressPair(torch.autograd.Function):
+    """(ck, cv) = compress(k; w_k, b_k), compress(v; w_v, b_v).  k, v [tok,H,D]; weights [l*D, D]; biases [D] or None.
+    ``split``: see nsa_compress_fwd_kv; False where a block selection follows."""
 
     @staticmethod
-    def forward(ctx, x, w, bias, cu_in, cu_out, block, stride):
-        x = _lib.require(x, "x")
-        w = _lib.require(w, "w")
-        bias = _lib.require(bias, "bias")
-        tok, H, D = x.shape
-        if w.shape != (block * D, D):
-            raise ValueError("weight must have shape [block*D, D] = %s, got %s" % ((block * D, D), tuple(w.shape)))
-        nseq = len(cu_in) - 1
-        total_out = cu_out[-1]
-        max_out = max([cu_out[i + 1] - cu_out[i] for i in range(nseq)] + [0])
-        max_in = max([cu_in[i + 1] - cu_in[i] for i in range(nseq)] + [0])
-        y = torch.empty(total_out, H, D, dtype=torch.bfloat16, device=x.device)
-        cin, cout = _cu_tensor(cu_in, x.device), _cu_tensor(cu_out, x.device)
-        lens = [cu_in[i + 1] - cu_in[i] for i in range(nseq)]
-        uniform = (nseq > 0 and len(set(lens)) == 1 and lens[0] >= block and lens[0] % stride == 0
-                   and cu_out[1] - cu_out[0] == (lens[0] - block) // stride + 1)
-        if total_out > 0 and uniform:
-            _lib.check(_lib.lib().nsa_compress_fwd_uniform(_lib.ptr(x), _lib.ptr(w), _lib.ptr(bias), _lib.ptr(y), nseq,
-                                                           lens[0], H, D, block, stride, _lib.stream()),
-                       "nsa_compress_fwd_uniform")
-        elif total_out > 0:
-            _lib.check(_lib.lib().nsa_compress_fwd(_lib.ptr(x), _lib.ptr(w), _lib.ptr(bias), _lib.ptr(y), _lib.ptr(cin),
-                                                   _lib.ptr(cout), nseq, H, D, block, stride, max_out, _lib.stream()),
-                       "nsa_compress_fwd")
-        ctx.save_for_backward(x, w, cin, cout)
-        ctx.meta = (nseq, H, D, block, stride, max_in, total_out, bias is not None)
-        return y
-
-    @staticmethod
-    def backward(ctx, dy):
-        x, w, cin, cout = ctx.saved_tensors
-        nseq, H, D, block, stride, max_in, total_out, has_bias = ctx.meta
-        dy = _lib.require(dy, "dy")
-        need_x, need_w, need_b = ctx.needs_input_grad[0], ctx.needs_input_grad[1], has_bias and ctx.needs_input_grad[2]
-        dx = torch.empty_like(x) if need_x else None
-        dw = torch.empty(block * D, D, dtype=torch.float32, device=x.device) if need_w else None
-        db = torch.empty(D, dtype=torch.float32, device=x.device) if need_b else None
-        L = _lib.lib()
-        ws_bytes = L.nsa_compress_bwd_workspace_bytes(nseq, H, D, block) if need_w else 0
-        ws = torch.empty(ws_bytes, dtype=torch.uint8, device=x.device) if ws_bytes else None
+    def forward(ctx, k, v, w_k, w_v, b_k, b_v, cu_in, cu_out, block, stride, split):
+        k, v, w_k, w_v = (_lib.require(t, n) for t, n in ((k, "k"), (v, "v"), (w_k, "w_k"), (w_v, "w_v")))
+        b_k, b_v = _lib.require(b_k, "bias"), _lib.require(b_v, "bias")
+        tok, H, D = k.shape
+        for w in (w_k, w_v):
+            if w.shape != (block * D, D):
+                raise ValueError("weight must have shape [block*D, D] = %s, got %s" % ((block * D, D), tuple(w.shape)))
+        nseq, total_out = len(cu_in) - 1, cu_out[-1]
+        ck = torch.empty(total_out, H, D, dtype=torch.bfloat16, device=k.device)
+        cv = torch.empty(total_out, H, D, dtype=torch.bfloat16, device=k.device)
+        cin, cout = _cu_tensor(cu_in, k.device), _cu_tensor(cu_out, k.device)
+        P = _lib.ptr
         if total_out > 0:
-            _lib.check(L.nsa_compress_bwd(_lib.ptr(x), _lib.ptr(w), _lib.ptr(dy), _lib.ptr(dx), _lib.ptr(dw), _lib.ptr(db),
-                                          _lib.ptr(ws), ws_bytes, _lib.ptr(cin), _lib.ptr(cout), nseq, H, D, block, stride,
-                                          max_in, total_out, _lib.stream()), "nsa_compress_bwd")
-        else:
-            for t in (dx, dw, db):
-                if t is not None:
-                    t.zero_()
-        return dx, dw, db, None, None, None, None
+            _lib.check(_lib.lib().nsa_compress_fwd_kv(P(k), P(v), P(w_k), P(w_v), P(b_k), P(b_v), P(ck), P(cv), P(cin), P(cout),
+                                                      nseq, 0, 0, tok, total_out, H, D, block, stride, split,
+                                                      _lib.stream()),
+                       "nsa_compress_fwd_kv")
+        ctx.save_for_backward(k, v, w_k, w_v, cin, cout)
+        ctx.meta = (nseq, H, D, block, stride, max([b - a for a, b in zip(cu_in[:-1], cu_in[1:])] + [0]), total_out)
+        return ck, cv
+
+    @staticmethod
+    def backward(ctx, dck, dcv):
+        k, v, w_k, w_v, cin, cout = ctx.saved_tensors
+        nseq, H, D, block, stride, max_in, total_out = ctx.meta
+        L, P, need = _lib.lib(), _lib.ptr, ctx.needs_input_grad
+        ws_bytes = L.nsa_compress_bwd_kv_workspace_bytes(nseq, 0, total_out, 1, H, D, block, stride)
+        if ws_bytes and total_out > 0:   # both tensors on the tensor cores (block = stride or 2 * stride)
+            dck, dcv = _lib.require(dck, "dck"), _lib.require(dcv, "dcv")
+            dk, dv = (torch.empty_like(x) if n else None for x, n in ((k, need[0]), (v, need[1])))
+            dwk, dwv = (torch.empty_like(w) if n else None for w, n in ((w_k, need[2]), (w_v, need[3])))
+            dbk, dbv = (torch.empty(D, dtype=torch.bfloat16, device=k.device) if n else None for n in need[4:6])
+            ws = torch.empty(ws_bytes, dtype=torch.uint8, device=k.device) if any(need[2:6]) else None
+            _lib.check(L.nsa_compress_bwd_kv(P(k), P(v), P(w_k), P(w_v), P(dck), P(dcv), P(dk), P(dv), 0, P(dwk), P(dwv), P(dbk),
+                                             P(dbv), 1, P(ws), ws_bytes, P(cin), P(cout), nseq, 0, 0, k.shape[0], total_out, H, D,
+                                             block, stride, _lib.stream()), "nsa_compress_bwd_kv")
+            return dk, dv, dwk, dwv, dbk, dbv, None, None, None, None, None
+        ws_bytes = L.nsa_compress_bwd_workspace_bytes(nseq, H, D, block) if need[2] or need[3] else 0
+        ws = torch.empty(ws_bytes, dtype=torch.uint8, device=k.device) if ws_bytes else None
+        grads = []
+        for i, (x, w, dy) in enumerate(((k, w_k, dck), (v, w_v, dcv))):
+            dy = _lib.require(dy, "dy")
+            dx = torch.empty_like(x) if need[i] else None
+            dw = torch.empty(block * D, D, dtype=torch.float32, device=x.device) if need[2 + i] else None
+            db = torch.empty(D, dtype=torch.float32, device=x.device) if need[4 + i] else None
+            if total_out > 0:
+                _lib.check(L.nsa_compress_bwd(P(x), P(w), P(dy), P(dx), P(dw), P(db), P(ws), ws_bytes, P(cin), P(cout), nseq, H,
+                                              D, block, stride, max_in, total_out, _lib.stream()), "nsa_compress_bwd")
+            else:
+                for t in (dx, dw, db):
+                    if t is not None:
+                        t.zero_()
+            grads.append((dx, dw, db))
+        (dk, dwk, dbk), (dv, dwv, dbv) = grads
+        return dk, dv, dwk, dwv, dbk, dbv, None, None, None, None, None
 
 
 def _host_cu(cu_seq_len):
@@ -99,22 +106,40 @@ def compress_kv(k, v, w_k, w_v, cu_seq_len, block_stride, block_size):
     cu_out = [0]
     for i in range(len(cu_in) - 1):
         cu_out.append(cu_out[-1] + max(calc_compressed_len(cu_in[i + 1] - cu_in[i], block_stride, block_size), 0))
-    ck = _CompressOne.apply(k, w_k, None, cu_in, cu_out, block_size, block_stride)
-    cv = _CompressOne.apply(v, w_v, None, cu_in, cu_out, block_size, block_stride)
+    ck, cv = _CompressPair.apply(k, v, w_k, w_v, None, None, cu_in, cu_out, block_size, block_stride, True)
     return ck, cv, _cu_tensor(cu_out, k.device)
 
 
-def compress_conv(x, weight, bias, block, stride, B):
-    """Module-path compression of x [B*T,H,D] with an nn.Conv1d weight [D,D,block] and bias [D]:
-    the contraction of nsa/compression_kv.py:301-307, output [B,Tc,H,D] with Tc = (T-block)//stride + 1."""
-    tok, H, D = x.shape
-    T = tok // B
+class _ConvLayout(torch.autograd.Function):
+    """The two Conv1d weights [D,D,block] in the kernels' [block*D, D] layout (rows j*D+c, columns o), one launch."""
+
+    @staticmethod
+    def forward(ctx, w_k, w_v):
+        w_k, w_v = _lib.require(w_k, "compressor_k.weight"), _lib.require(w_v, "compressor_v.weight")
+        D, _, block = w_k.shape
+        ctx.dims = (D, block)
+        out_k, out_v = (torch.empty(block * D, D, dtype=torch.bfloat16, device=w_k.device) for _ in range(2))
+        P = _lib.ptr
+        _lib.check(_lib.lib().nsa_conv_weight_layout(P(w_k), P(w_v), P(out_k), P(out_v), D, block, _lib.stream()),
+                   "nsa_conv_weight_layout")
+        return out_k, out_v
+
+    @staticmethod
+    def backward(ctx, *grads):
+        D, block = ctx.dims
+        return tuple(g.view(block, D, D).permute(2, 1, 0) for g in grads)
+
+
+def compress_conv(k, v, compressor, B):
+    """Module-path compression of k, v [B*T,H,D] with the Conv1d parameters of a KVCompressor: the contraction of
+    nsa/compression_kv.py:301-307, outputs [B,Tc,H,D] with Tc = (T-block)//stride + 1."""
+    tok, H, D = k.shape
+    T, block, stride = tok // B, compressor.block_size, compressor.block_stride
     Tc = (T - block) // stride + 1 if T >= block else 0
-    cu_in = [T * i for i in range(B + 1)]
-    cu_out = [Tc * i for i in range(B + 1)]
-    wm = weight.permute(2, 1, 0).reshape(block * D, D)   # rows j*D+c, columns o (autograd permutes back)
-    y = _CompressOne.apply(x, wm, bias, cu_in, cu_out, block, stride)
-    return y.view(B, Tc, H, D)
+    w_k, w_v = _ConvLayout.apply(compressor.compressor_k.weight, compressor.compressor_v.weight)
+    ck, cv = _CompressPair.apply(k, v, w_k, w_v, compressor.compressor_k.bias, compressor.compressor_v.bias,
+                                 range(0, T * B + 1, T), [Tc * i for i in range(B + 1)], block, stride, False)
+    return ck.view(B, Tc, H, D), cv.view(B, Tc, H, D)
 
 
 class KVCompressorVarlen(nn.Module):
@@ -154,8 +179,7 @@ class KVCompressor(nn.Module):
         ``group`` repeats every KV head ``group`` times as the reference does; pass None to keep the
         compact [B,Tc,H,D] form, which the compressed-attention kernel reads directly."""
         B = cu_seq_len.shape[0] - 1
-        ck = compress_conv(k, self.compressor_k.weight, self.compressor_k.bias, self.block_size, self.block_stride, B)
-        cv = compress_conv(v, self.compressor_v.weight, self.compressor_v.bias, self.block_size, self.block_stride, B)
+        ck, cv = compress_conv(k, v, self, B)
         if group is not None:
             ck = ck.repeat_interleave(group, dim=2)
             cv = cv.repeat_interleave(group, dim=2)

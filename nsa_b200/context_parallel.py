@@ -141,9 +141,7 @@ def context_parallel_forward(module, q, k, v, group=None, zigzag=True, causal=Tr
         t0, t1 = lo * stride, (hi - 1) * stride + block
         ks = k_full[:, t0:t1].reshape(B * (t1 - t0), Hkv, D)
         vs = v_full[:, t0:t1].reshape(B * (t1 - t0), Hkv, D)
-        ck_part = compress_conv(ks, comp.compressor_k.weight, comp.compressor_k.bias, block, stride, B)
-        cv_part = compress_conv(vs, comp.compressor_v.weight, comp.compressor_v.bias, block, stride, B)
-        ckv_part = torch.cat([ck_part, cv_part], 2)
+        ckv_part = torch.cat(compress_conv(ks, vs, comp, B), 2)
     else:
         ckv_part = k_full.new_zeros(B, 0, 2 * Hkv, D) + 0 * (comp.compressor_k.weight.sum() + comp.compressor_v.weight.sum())
     ckv = _GatherRows.apply(ckv_part, [h_ - l_ for l_, h_ in ranges], group)

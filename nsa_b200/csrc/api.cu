@@ -64,7 +64,7 @@ int nsa_device_status(void) {
   cudaError_t e = cudaDeviceSynchronize();
   if (e != cudaSuccess) return fail(1000 + (int)e, "cudaDeviceSynchronize: %s", cudaGetErrorString(e));
   int worst = 0, v = 0;
-  int (*fns[])(int*) = {sel_status, sel_block_status, dense_status, kv_status, compress_status, misc_status, compress_tc_status, kv_tc_status, dense_dq_tc_status, gather_probe_status, dense_tc2_status, decode_status, sel_fwd_kv_status};
+  int (*fns[])(int*) = {sel_status, sel_block_status, dense_status, kv_status, compress_status, misc_status, compress_tc_status, compress_bwd_tc_status, kv_tc_status, dense_dq_tc_status, gather_probe_status, dense_tc2_status, decode_status, sel_fwd_kv_status};
   for (auto f : fns) {
     v = 0;
     const int rc = f(&v);
@@ -103,9 +103,83 @@ int nsa_compress_fwd_uniform(const void* x, const void* w, const void* bias, voi
   if (B <= 0 || H <= 0) return fail(-1, "nsa_compress_fwd_uniform: empty shape");
   if (stride <= 0 || block <= 0 || block % stride) return fail(-4, "nsa_compress_fwd_uniform: block must be a multiple of stride");
   if (T < block || T % stride) return fail(-10, "nsa_compress_fwd_uniform: T must be a multiple of stride and at least block");
-  if (stride > 256) return fail(-10, "nsa_compress_fwd_uniform: stride too large for a TMA box");
-  return launch_compress_fwd_uniform((const bf16*)x, (const bf16*)w, (const bf16*)bias, (bf16*)y, B, T, H, D, block, stride,
-                                     (cudaStream_t)stream);
+  if (!aligned16(x) || !aligned16(w) || !aligned16(y)) return fail(-5, "nsa_compress_fwd_uniform: pointers must be 16-byte aligned");
+  CompressFwdArgs a = {};
+  a.x[0] = (const bf16*)x; a.w[0] = (const bf16*)w; a.bias[0] = (const bf16*)bias; a.y[0] = (bf16*)y; a.ntensor = 1;
+  a.nseq = B; a.T = T; a.Tc = (T - block) / stride + 1; a.total_in = (long long)B * T;
+  a.H = H; a.D = D; a.l = block; a.d = stride;
+  return launch_compress_fwd_tc(a, (cudaStream_t)stream);
+}
+
+int nsa_compress_fwd_kv(const void* k, const void* v, const void* w_k, const void* w_v, const void* bias_k,
+                        const void* bias_v, void* ck, void* cv, const int32_t* cu_in, const int32_t* cu_out, int nseq, int T,
+                        int Tc, long long total_in, long long total_out, int H, int D, int block, int stride, int split,
+                        void* stream) {
+  if (!k || !v || !w_k || !w_v || !ck || !cv) return fail(-1, "nsa_compress_fwd_kv: null pointer");
+  if (nseq <= 0 || H <= 0 || total_in < 0) return fail(-1, "nsa_compress_fwd_kv: empty shape");
+  if (stride <= 0 || block <= 0 || block % stride) return fail(-4, "nsa_compress_fwd_kv: block must be a multiple of stride");
+  if (!aligned16(k) || !aligned16(v) || !aligned16(w_k) || !aligned16(w_v) || !aligned16(ck) || !aligned16(cv))
+    return fail(-5, "nsa_compress_fwd_kv: pointers must be 16-byte aligned");
+  if (!cu_in != !cu_out) return fail(-1, "nsa_compress_fwd_kv: cu_in and cu_out must be given together");
+  if (!cu_in && (total_in != (long long)nseq * T || (Tc > 0 && T < block + (Tc - 1) * stride)))
+    return fail(-10, "nsa_compress_fwd_kv: %d sequences of %d tokens do not hold %d positions each", nseq, T, Tc);
+  if (cu_in && total_out > 0 && total_in < block) return fail(-10, "nsa_compress_fwd_kv: fewer tokens than one block");
+  CompressFwdArgs a = {};
+  a.x[0] = (const bf16*)k; a.w[0] = (const bf16*)w_k; a.bias[0] = (const bf16*)bias_k; a.y[0] = (bf16*)ck;
+  a.x[1] = (const bf16*)v; a.w[1] = (const bf16*)w_v; a.bias[1] = (const bf16*)bias_v; a.y[1] = (bf16*)cv;
+  a.ntensor = 2; a.cu_in = cu_in; a.cu_out = cu_out; a.cu_row = cu_out; a.rows = total_out; a.split = split;
+  a.nseq = nseq; a.T = T; a.Tc = Tc; a.total_in = total_in; a.H = H; a.D = D; a.l = block; a.d = stride;
+  return launch_compress_fwd_tc(a, (cudaStream_t)stream);
+}
+
+int nsa_conv_weight_layout(const void* w_k, const void* w_v, void* out_k, void* out_v, int D, int block, void* stream) {
+  if (!w_k || !out_k || (!w_v != !out_v)) return fail(-1, "nsa_conv_weight_layout: null pointer");
+  if (D != 64 && D != 128) return fail(-2, "nsa_conv_weight_layout: head_dim %d not supported (64 or 128)", D);
+  if (block <= 0) return fail(-1, "nsa_conv_weight_layout: empty shape");
+  return launch_conv_weight((const bf16*)w_k, (const bf16*)w_v, (bf16*)out_k, (bf16*)out_v, D, block, (cudaStream_t)stream);
+}
+
+int nsa_cache_plan(const int32_t* cu_new, const int32_t* cu_old, const int32_t* cuc_old, int nseq, int block, int stride,
+                   int32_t* table, int32_t* info) {
+  if (!cu_new || !table || !info || (!cu_old != !cuc_old)) return fail(-1, "nsa_cache_plan: null pointer");
+  if (nseq < 0 || block <= 0 || stride <= 0) return fail(-1, "nsa_cache_plan: empty or negative shape");
+  const int rc = cache_plan(cu_new, cu_old, cuc_old, nseq, block, stride, table, info);
+  return rc ? fail(-17, "sequence %d became shorter", rc - 1) : 0;
+}
+
+int nsa_cache_build(const void* k, const void* v, const void* conv_k, const void* conv_v, const void* bias_k,
+                    const void* bias_v, void* w_ws, const void* ck_old, const void* cv_old, void* ck, void* cv,
+                    const int32_t* table, int32_t* table_dev, int nseq, long long total_in, int H, int D, int block, int stride,
+                    void* stream) {
+  if (!k || !v || !conv_k || !conv_v || !w_ws || !ck || !cv || !table || !table_dev) return fail(-1, "nsa_cache_build: null pointer");
+  if (nseq <= 0 || H <= 0) return fail(-1, "nsa_cache_build: empty shape");
+  if (D != 64 && D != 128) return fail(-2, "nsa_cache_build: head_dim %d not supported (64 or 128)", D);
+  if (block % stride) return fail(-4, "nsa_cache_build: block must be a multiple of stride");
+  if (!aligned16(k) || !aligned16(v) || !aligned16(w_ws) || !aligned16(ck) || !aligned16(cv) || !aligned16(ck_old) || !aligned16(cv_old))
+    return fail(-5, "nsa_cache_build: pointers must be 16-byte aligned");
+  cudaStream_t s = (cudaStream_t)stream;
+  const int n = nseq;
+  const int32_t* cu = table_dev;
+  const int32_t* cc = cu + n + 1;
+  const int32_t* old = cc + n + 1;
+  const int32_t* row = old + n + 1;
+  const int32_t* first = row + n + 1;
+  const long long nold = table[2 * (n + 1) + n], nnew = table[3 * (n + 1) + n];
+  if (table[n] > total_in) return fail(-10, "nsa_cache_build: the sequences end at token %d of %lld", table[n], total_in);
+  if (nold > 0 && (!ck_old || !cv_old)) return fail(-1, "nsa_cache_build: null pointer");
+  int rc = launch_upload_table(table, 6 * n + 4, table_dev, s);
+  if (!rc) rc = launch_move_rows((const bf16*)ck_old, (const bf16*)cv_old, (bf16*)ck, (bf16*)cv, old, cc, n, nold, H * D, s);
+  if (rc || nnew <= 0) return rc;
+  bf16* wk = (bf16*)w_ws;
+  bf16* wv = wk + (size_t)block * D * D;
+  rc = launch_conv_weight((const bf16*)conv_k, (const bf16*)conv_v, wk, wv, D, block, s);
+  if (rc) return rc;
+  CompressFwdArgs a = {};
+  a.x[0] = (const bf16*)k; a.w[0] = wk; a.bias[0] = (const bf16*)bias_k; a.y[0] = (bf16*)ck;
+  a.x[1] = (const bf16*)v; a.w[1] = wv; a.bias[1] = (const bf16*)bias_v; a.y[1] = (bf16*)cv;
+  a.ntensor = 2; a.cu_in = cu; a.cu_out = cc; a.cu_row = row; a.first = first; a.rows = nnew; a.split = 1;
+  a.nseq = n; a.total_in = total_in; a.H = H; a.D = D; a.l = block; a.d = stride;
+  return launch_compress_fwd_tc(a, s);
 }
 
 size_t nsa_compress_bwd_workspace_bytes(int nseq, int H, int D, int block) {
@@ -128,6 +202,36 @@ int nsa_compress_bwd(const void* x, const void* w, const void* dy, void* dx, flo
   a.ws = (float*)ws; a.cu_in = cu_in; a.cu_out = cu_out; a.nseq = nseq; a.H = H; a.D = D; a.l = block; a.d = stride;
   a.max_in = max_in; a.total_out = total_out;
   return launch_compress_bwd(a, (cudaStream_t)stream);
+}
+
+size_t nsa_compress_bwd_kv_workspace_bytes(int nseq, int Tc, long long total_out, int ragged, int H, int D, int block,
+                                           int stride) {
+  if (block <= 0 || stride <= 0 || H <= 0 || !compress_bwd_tc_supported(D, block, stride)) return 0;
+  return compress_bwd_tc_workspace_bytes(nseq, Tc, total_out, ragged != 0, H, D, block);
+}
+
+int nsa_compress_bwd_kv(const void* k, const void* v, const void* w_k, const void* w_v, const void* dck, const void* dcv,
+                        void* dk, void* dv, int accumulate, void* dw_k, void* dw_v, void* dbias_k, void* dbias_v, int dw_mode,
+                        void* ws, size_t ws_bytes, const int32_t* cu_in, const int32_t* cu_out, int nseq, int T, int Tc,
+                        long long total_in, long long total_out, int H, int D, int block, int stride, void* stream) {
+  if (!k || !v || !w_k || !w_v || !dck || !dcv) return fail(-1, "nsa_compress_bwd_kv: null pointer");
+  if (nseq <= 0 || H <= 0 || total_in <= 0 || total_out <= 0) return fail(-1, "nsa_compress_bwd_kv: empty shape");
+  if (D != 64 && D != 128) return fail(-2, "nsa_compress_bwd_kv: head_dim %d not supported (64 or 128)", D);
+  if (stride <= 0 || block <= 0 || !compress_bwd_tc_supported(D, block, stride))
+    return fail(-4, "nsa_compress_bwd_kv: block must be stride or 2 * stride (got %d, %d); use nsa_compress_bwd", block, stride);
+  if (dw_mode < 0 || dw_mode > 2) return fail(-16, "nsa_compress_bwd_kv: dw_mode must be 0, 1 or 2");
+  if (!cu_in != !cu_out) return fail(-1, "nsa_compress_bwd_kv: cu_in and cu_out must be given together");
+  if (!cu_in && (total_in != (long long)nseq * T || total_out != (long long)nseq * Tc || T < block + (Tc - 1) * stride))
+    return fail(-10, "nsa_compress_bwd_kv: %d sequences of %d tokens do not hold %d positions each", nseq, T, Tc);
+  if ((dw_k || dw_v || dbias_k || dbias_v) &&
+      (!ws || ws_bytes < nsa_compress_bwd_kv_workspace_bytes(nseq, Tc, total_out, cu_in != nullptr, H, D, block, stride)))
+    return fail(-6, "nsa_compress_bwd_kv: workspace too small");
+  CompressBwdArgs a = {};
+  a.x[0] = (const bf16*)k; a.w[0] = (const bf16*)w_k; a.dy[0] = (const bf16*)dck; a.dx[0] = (bf16*)dk; a.dw[0] = dw_k; a.dbias[0] = dbias_k;
+  a.x[1] = (const bf16*)v; a.w[1] = (const bf16*)w_v; a.dy[1] = (const bf16*)dcv; a.dx[1] = (bf16*)dv; a.dw[1] = dw_v; a.dbias[1] = dbias_v;
+  a.accumulate = accumulate; a.mode = dw_mode; a.ws = (float*)ws; a.cu_in = cu_in; a.cu_out = cu_out;
+  a.nseq = nseq; a.T = T; a.Tc = Tc; a.total_in = total_in; a.total_out = total_out; a.H = H; a.D = D; a.l = block; a.d = stride;
+  return launch_compress_bwd_tc(a, (cudaStream_t)stream);
 }
 
 int nsa_compress_bwd_noalloc(const void* x, const void* w, const void* dy, void* dx, float* dw, float* dbias,

@@ -176,10 +176,52 @@ int compress_status(int* out);
 int launch_compress_bwd_static(const CompressArgs& a, cudaStream_t s);
 long long compress_static_scratch_floats();
 
-// tcgen05 GEMM for equal-length sequences (x [B,T,H,D], T % d == 0)
-int launch_compress_fwd_uniform(const bf16* x, const bf16* w, const bf16* bias, bf16* y, int B, int T, int H, int D, int l,
-                                int d, cudaStream_t s);
+// tcgen05 GEMM of the forward, one or two tensors per launch
+struct CompressFwdArgs {
+  const bf16* x[2];     // [total_in,H,D]
+  const bf16* w[2];     // [l*D, D]
+  const bf16* bias[2];  // [D] or null
+  bf16* y[2];           // [total_out,H,D]
+  int ntensor;
+  // ragged (device tables [nseq+1]): sequence s starts at token cu_in[s]; its positions first[s] (null: 0) .. are computed,
+  // cu_row[s+1] - cu_row[s] of them, and stored from row cu_out[s] + first[s] on.  cu_in null: nseq sequences of T tokens.
+  const int *cu_in, *cu_out, *cu_row, *first;
+  int nseq, T, Tc;
+  long long total_in, rows;   // tokens in all; positions to compute in all (ragged)
+  int H, D, l, d;
+  int split;                  // the contraction may be split (its sum is then added in a different order)
+};
+int compress_tile_positions(int H);
+int launch_compress_fwd_tc(const CompressFwdArgs& a, cudaStream_t s);
 int compress_tc_status(int* out);
+
+// tcgen05 GEMMs of the backward, both tensors per launch (compress_bwd_tc.cu; l <= 2 d)
+struct CompressBwdArgs {
+  const bf16* x[2];     // [total_in,H,D]
+  const bf16* w[2];     // [l*D, D]
+  const bf16* dy[2];    // [total_out,H,D]
+  bf16* dx[2];          // [total_in,H,D], or null
+  int accumulate;       // dx += instead of =
+  void* dw[2];          // gradient of the weights in the layout of `mode`, or null
+  void* dbias[2];       // [D], fp32 (mode 0) or bf16, or null
+  int mode;             // 0: [l*D, D] fp32; 1: [l*D, D] bf16; 2: Conv1d [D,D,l] bf16
+  float* ws;            // compress_bwd_tc_workspace_bytes()
+  const int *cu_in, *cu_out;   // ragged (device), or null: nseq sequences of T tokens and Tc positions
+  int nseq, T, Tc;
+  long long total_in, total_out;
+  int H, D, l, d;
+};
+bool compress_bwd_tc_supported(int D, int l, int d);
+size_t compress_bwd_tc_workspace_bytes(int nseq, int Tc, long long total_out, bool ragged, int H, int D, int l);
+int launch_compress_bwd_tc(const CompressBwdArgs& a, cudaStream_t s);
+int compress_bwd_tc_status(int* out);
+
+// ---- compressed cache of a generation loop, weight layout (cache.cu) ----------------------------------------
+int cache_plan(const int* cu_new, const int* cu_old, const int* cuc_old, int nseq, int block, int stride, int* table, int* info);
+int launch_upload_table(const int* host, int n, int* dst, cudaStream_t s);
+int launch_move_rows(const bf16* ck0, const bf16* cv0, bf16* ck1, bf16* cv1, const int* cu_old, const int* cu_new, int nseq,
+                     long long rows, int row_elems, cudaStream_t s);
+int launch_conv_weight(const bf16* w0, const bf16* w1, bf16* o0, bf16* o1, int D, int l, cudaStream_t s);
 
 // ---- small helpers ----------------------------------------------------------------------------
 // delta[r] = (gate ? gate[r] : 1) * sum_d o[r,d]*dout[r,d];  dgate[r] = sum_d o[r,d]*dout[r,d]

@@ -5,27 +5,44 @@ the same forward (nsa/nsa.py:94-135) for the single row t = L-1 of every sequenc
 in one kernel launch (nsa_decode_fwd).  The compressed K/V are a cache: ``compress_cache`` builds it once,
 ``extend_compress_cache`` appends only the compressed positions that new tokens complete.
 """
+import ctypes
+
 import torch
 
 from . import _lib
-from .compression_kv import _CompressOne
+from .compression_kv import _CompressPair, _ConvLayout
 
 
 class CompressedCache:
     """Compressed K/V of a packed cache plus the (host and device) length tables the decode kernel needs.
 
     ck, cv [sum Tc,Hkv,D]; cu, cu_c: host lists [nseq+1] (cumulative lengths of k/v and of ck/cv); the device copies and
-    the longest-first launch order are built once here so that a decode step issues no host-to-device copy."""
+    the longest-first launch order are one table that is built with the cache, so that a decode step issues no
+    host-to-device copy."""
 
-    def __init__(self, ck, cv, cu, cu_c):
-        self.ck, self.cv, self.cu, self.cu_c = ck, cv, list(cu), list(cu_c)
-        dev = ck.device
-        n = len(self.cu) - 1
-        self.cu_dev = torch.tensor(self.cu, dtype=torch.int32, device=dev)
-        self.cu_c_dev = torch.tensor(self.cu_c, dtype=torch.int32, device=dev)
-        lens = [self.cu[i + 1] - self.cu[i] for i in range(n)]
-        self.order_dev = torch.tensor(sorted(range(n), key=lambda i: -lens[i]), dtype=torch.int32, device=dev)
-        self.max_tc = max([self.cu_c[i + 1] - self.cu_c[i] for i in range(n)] + [0])
+    def __init__(self, ck, cv, table, table_dev, nseq, max_tc):
+        self.ck, self.cv, self.nseq, self.max_tc = ck, cv, nseq, max_tc
+        self._table, self.table_dev = table, table_dev   # layout: nsa_cache_plan in include/nsa_b200.h
+
+    @property
+    def cu(self):
+        return list(self._table[:self.nseq + 1])
+
+    @property
+    def cu_c(self):
+        return list(self._table[self.nseq + 1:2 * self.nseq + 2])
+
+    @property
+    def cu_dev(self):
+        return self.table_dev[:self.nseq + 1]
+
+    @property
+    def cu_c_dev(self):
+        return self.table_dev[self.nseq + 1:2 * self.nseq + 2]
+
+    @property
+    def order_dev(self):
+        return self.table_dev[5 * self.nseq + 4:]
 
     def workspace(self, nbytes):
         """Scratch of the decode kernels (per-warp partial results), kept with the cache so a step allocates nothing."""
@@ -39,73 +56,59 @@ class CompressedCache:
 
 
 def _lengths(cu_seqlens_k):
-    return [int(c) for c in (cu_seqlens_k.tolist() if torch.is_tensor(cu_seqlens_k) else cu_seqlens_k)]
+    cu = cu_seqlens_k.tolist() if torch.is_tensor(cu_seqlens_k) else cu_seqlens_k
+    return (ctypes.c_int32 * len(cu))(*cu)
 
 
-def _weights(module, D):
-    block = module.compression_block
-    return [(conv.weight.permute(2, 1, 0).reshape(block * D, D), conv.bias)
-            for conv in (module.compressor.compressor_k, module.compressor.compressor_v)]
+@torch.no_grad()
+def _build(module, k, v, cu_seqlens_k, old):
+    """The compressed cache of packed k, v; the positions that ``old`` (a CompressedCache or None) holds are copied."""
+    k, v = _lib.require(k, "k"), _lib.require(v, "v")
+    cu = _lengths(cu_seqlens_k)
+    n, (total, H, D), L = len(cu) - 1, k.shape, _lib.lib()
+    if old is not None and n != old.nseq:
+        raise ValueError("the number of sequences changed")
+    conv_k, conv_v = module.compressor.compressor_k, module.compressor.compressor_v
+    block, stride = module.compression_block, module.compression_stride
+    table, info = (ctypes.c_int32 * (6 * n + 4))(), (ctypes.c_int32 * 3)()
+    rc = L.nsa_cache_plan(cu, old._table if old is not None else None,
+                          ctypes.byref(old._table, 4 * (n + 1)) if old is not None else None, n, block, stride, table, info)
+    if rc == -17:
+        raise ValueError(L.nsa_last_error().decode())
+    _lib.check(rc, "nsa_cache_plan")
+    dev = k.device
+    ck = torch.empty(info[0], H, D, dtype=torch.bfloat16, device=dev)
+    cv = torch.empty(info[0], H, D, dtype=torch.bfloat16, device=dev)
+    # one allocation: the kernel's weight layout (scratch) and the device tables
+    wbytes = 4 * block * D * D
+    buf = torch.empty(wbytes + 4 * (6 * n + 4), dtype=torch.uint8, device=dev)
+    table_dev = buf[wbytes:].view(torch.int32)
+    P = _lib.ptr
+    wk, wv = _lib.require(conv_k.weight, "compressor_k.weight"), _lib.require(conv_v.weight, "compressor_v.weight")
+    bk, bv = _lib.require(conv_k.bias, "compressor_k.bias"), _lib.require(conv_v.bias, "compressor_v.bias")
+    _lib.check(L.nsa_cache_build(P(k), P(v), P(wk), P(wv), P(bk), P(bv), P(buf), P(old.ck) if old is not None else None,
+                                 P(old.cv) if old is not None else None, P(ck), P(cv), table, P(table_dev), n, total, H, D,
+                                 block, stride, _lib.stream()), "nsa_cache_build")
+    return CompressedCache(ck, cv, table, table_dev, n, info[1])
 
 
 def compress_cache(module, k, v, cu_seqlens_k):
     """Compressed K/V of a packed cache: k, v [sum L,Hkv,D] -> CompressedCache (ck, cv [sum Tc,Hkv,D]).
     Tc = (L-block)//stride + 1 per sequence, the module's Conv1d rule (nsa/compression_kv.py:298-307)."""
-    cu = _lengths(cu_seqlens_k)
-    block, stride = module.compression_block, module.compression_stride
-    cu_c = [0]
-    for i in range(len(cu) - 1):
-        L = cu[i + 1] - cu[i]
-        cu_c.append(cu_c[-1] + ((L - block) // stride + 1 if L >= block else 0))
-    (wk, bk), (wv, bv) = _weights(module, k.shape[-1])
-    ck = _CompressOne.apply(k, wk, bk, cu, cu_c, block, stride)
-    cv = _CompressOne.apply(v, wv, bv, cu, cu_c, block, stride)
-    return CompressedCache(ck, cv, cu, cu_c)
+    cache = _build(module, k, v, cu_seqlens_k, None)
+    if torch.is_grad_enabled() and any(t.requires_grad for t in (k, v, *module.compressor.parameters())):
+        comp = module.compressor   # differentiable on request: the same values through the autograd functions
+        w_k, w_v = _ConvLayout.apply(comp.compressor_k.weight, comp.compressor_v.weight)
+        cache.ck, cache.cv = _CompressPair.apply(k, v, w_k, w_v, comp.compressor_k.bias, comp.compressor_v.bias, cache.cu,
+                                                 cache.cu_c, module.compression_block, module.compression_stride, True)
+    return cache
 
 
-@torch.no_grad()
 def extend_compress_cache(module, cache, k, v, cu_seqlens_k):
     """The cache after tokens were appended to the sequences: k, v [sum L',Hkv,D] are the grown packed K/V with lengths
     L' >= L.  Only the compressed positions that the new tokens complete are computed (each is one [block x D] window
     times the Conv1d weight, the same contraction as nsa/compression_kv.py:298-307); the existing entries are copied."""
-    cu_new = _lengths(cu_seqlens_k)
-    block, stride = module.compression_block, module.compression_stride
-    n = len(cu_new) - 1
-    if n != len(cache.cu) - 1:
-        raise ValueError("the number of sequences changed")
-    D, H = k.shape[-1], k.shape[1]
-    old_tc = [cache.cu_c[i + 1] - cache.cu_c[i] for i in range(n)]
-    cu_c = [0]
-    rows = []               # start rows (in the packed k/v) of the windows of the new compressed positions
-    for i in range(n):
-        L = cu_new[i + 1] - cu_new[i]
-        if L < cache.cu[i + 1] - cache.cu[i]:
-            raise ValueError("sequence %d became shorter" % i)
-        tc = (L - block) // stride + 1 if L >= block else 0
-        cu_c.append(cu_c[-1] + tc)
-        rows += [cu_new[i] + j * stride for j in range(old_tc[i], tc)]
-    ck = torch.empty(cu_c[-1], H, D, dtype=cache.ck.dtype, device=k.device)
-    cv = torch.empty_like(ck)
-    for i in range(n):      # old entries keep their values
-        ck[cu_c[i]:cu_c[i] + old_tc[i]] = cache.ck[cache.cu_c[i]:cache.cu_c[i + 1]]
-        cv[cu_c[i]:cu_c[i] + old_tc[i]] = cache.cv[cache.cu_c[i]:cache.cu_c[i + 1]]
-    if rows:
-        nw = len(rows)
-        gather = (torch.tensor(rows, device=k.device).unsqueeze(1) + torch.arange(block, device=k.device)).reshape(-1)
-        win_cu = [block * j for j in range(nw + 1)]          # nw windows of exactly one block: one output each
-        out_cu = list(range(nw + 1))
-        (wk, bk), (wv, bv) = _weights(module, D)
-        new_k = _CompressOne.apply(k[gather].contiguous(), wk, bk, win_cu, out_cu, block, stride)
-        new_v = _CompressOne.apply(v[gather].contiguous(), wv, bv, win_cu, out_cu, block, stride)
-        dst, pos = [], 0
-        for i in range(n):
-            cnt = (cu_c[i + 1] - cu_c[i]) - old_tc[i]
-            dst += list(range(cu_c[i] + old_tc[i], cu_c[i + 1]))
-            pos += cnt
-        dst = torch.tensor(dst, device=k.device)
-        ck[dst] = new_k
-        cv[dst] = new_v
-    return CompressedCache(ck, cv, cu_new, cu_c)
+    return _build(module, k, v, cu_seqlens_k, cache)
 
 
 @torch.no_grad()
@@ -135,12 +138,13 @@ def nsa_decode(module, q, k, v, cu_seqlens_k, cache=None, return_parts=False):
     P, L = _lib.ptr, _lib.lib()
     ws_bytes = L.nsa_decode_workspace_bytes(nseq, Hkv)
     ws = cache.workspace(ws_bytes)
-    _lib.check(L.nsa_decode_fwd(P(q), P(k), P(v), P(cache.ck), P(cache.cv), P(cache.cu_dev), P(cache.cu_c_dev),
-                                         P(cache.order_dev), P(w_gate), P(b_gate), None, None, None, P(o), P(o_cmp), P(o_slc),
-                                         P(o_swa), P(lse), P(idx), P(ws), ws_bytes, nseq, k.shape[0], cache.ck.shape[0],
-                                         cache.max_tc, Hq, Hkv, D, module.compression_block, module.compression_stride,
-                                         module.selection_block_size, n_sel, module.sliding_window, float(scale),
-                                         _lib.stream()), "nsa_decode_fwd")
+    tab = P(cache.table_dev)
+    _lib.check(L.nsa_decode_fwd(P(q), P(k), P(v), P(cache.ck), P(cache.cv), tab, tab + 4 * (nseq + 1),
+                                tab + 4 * (5 * nseq + 4), P(w_gate), P(b_gate), None, None, None, P(o), P(o_cmp), P(o_slc),
+                                P(o_swa), P(lse), P(idx), P(ws), ws_bytes, nseq, k.shape[0], cache.ck.shape[0],
+                                cache.max_tc, Hq, Hkv, D, module.compression_block, module.compression_stride,
+                                module.selection_block_size, n_sel, module.sliding_window, float(scale),
+                                _lib.stream()), "nsa_decode_fwd")
     if return_parts:
         return o, (o_cmp, o_slc, o_swa, lse, idx)
     return o

@@ -1,0 +1,81 @@
+"""The tcgen05 compression GEMMs (forward and backward, both tensors per launch) against fp32 torch on the same bf16
+inputs, at the edges of their tiles: 128-row tiles of (positions x heads), sequences that start off the stride grid, tails,
+sequences without a position, head counts that do not divide the tile, one to many splits."""
+import pytest
+import torch
+
+from parity_util import DEV, close as _close
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def nsa():
+    import nsa_b200
+    yield nsa_b200
+    nsa_b200._lib.device_status()
+
+
+def _ref(x, w, b, cu, block, stride, n_out):
+    """fp32, one sequence after the other: windows unfolded, one matmul."""
+    outs = []
+    for i, n in enumerate(n_out):
+        s = x[cu[i]:cu[i + 1]]
+        if n:
+            win = torch.stack([s[j * stride:j * stride + block] for j in range(n)])          # [n, l, H, D]
+            outs.append(torch.einsum("nlhd,lde->nhe", win, w.view(block, x.shape[-1], -1)) + (0 if b is None else b))
+    return torch.cat(outs)
+
+
+@pytest.mark.parametrize("D,H,block,stride,lens", [
+    (128, 4, 32, 16, [5003]), (128, 4, 32, 16, [33, 1000, 31, 48, 2001, 700]), (128, 1, 32, 16, [2111, 2049]),
+    (128, 3, 32, 16, [700, 45]), (64, 4, 32, 16, [1024, 1037]), (64, 2, 64, 32, [3000, 65, 64]), (128, 4, 16, 16, [640, 17]),
+    (128, 4, 64, 16, [900, 77])])
+@pytest.mark.parametrize("split", [True, False])
+def test_compress_pair_fwd_bwd(nsa, D, H, block, stride, lens, split):
+    gen = torch.Generator(device=DEV).manual_seed(D + H + len(lens))
+    rnd = lambda *s, m=1.0: (torch.randn(*s, generator=gen, device=DEV) * m).bfloat16()
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    n_out = [(n - block) // stride + 1 if n >= block else 0 for n in lens]
+    cu_out = [sum(n_out[:i]) for i in range(len(n_out) + 1)]
+    args = [rnd(cu[-1], H, D), rnd(cu[-1], H, D), rnd(block * D, D, m=0.03), rnd(block * D, D, m=0.03), rnd(D), rnd(D)]
+    dck, dcv = rnd(cu_out[-1], H, D), rnd(cu_out[-1], H, D)
+    ours = [a.clone().requires_grad_(True) for a in args]
+    ck, cv = nsa.compression_kv._CompressPair.apply(*ours, cu, cu_out, block, stride, split)
+    got = torch.autograd.grad([ck, cv], ours, [dck, dcv])
+    ref = [a.float().requires_grad_(True) for a in args]
+    rk, rv = _ref(ref[0], ref[2], ref[4], cu, block, stride, n_out), _ref(ref[1], ref[3], ref[5], cu, block, stride, n_out)
+    want = torch.autograd.grad([rk, rv], ref, [dck.float(), dcv.float()])
+    _close("ck", ck, rk)
+    _close("cv", cv, rv)
+    for name, g, w in zip(("dk", "dv", "dw_k", "dw_v", "db_k", "db_v"), got, want):
+        _close(name, g, w, scaled=name[:2] != "dk" and name[:2] != "dv")
+    nsa._lib.device_status()
+
+
+@pytest.mark.parametrize("D,block,stride", [(128, 32, 16), (64, 64, 32)])
+def test_conv_weight_layout(nsa, D, block, stride):
+    w = torch.randn(D, D, block, device=DEV).bfloat16().requires_grad_(True)
+    a, b = nsa.compression_kv._ConvLayout.apply(w, w)
+    assert torch.equal(a, w.permute(2, 1, 0).reshape(block * D, D)) and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("grow", [[1] * 5, [0, 16, 3, 700, 40]])
+def test_extended_cache_equals_a_new_one(nsa, grow):
+    from nsa_b200.decode import compress_cache, extend_compress_cache
+    old = [2048, 1000, 20, 47, 31]
+    new = [a + b for a, b in zip(old, grow)]
+    mod = nsa.NSAAttention(128, True, device=DEV, dtype=torch.bfloat16).requires_grad_(False)
+    k, v = (torch.randn(sum(new), 4, 128, device=DEV).bfloat16() for _ in range(2))
+    keep = torch.cat([torch.arange(n, device=DEV) < o for n, o in zip(new, old)])
+    cum = lambda ls: [sum(ls[:i]) for i in range(len(ls) + 1)]
+    before = compress_cache(mod, k[keep], v[keep], cum(old))
+    got, want = extend_compress_cache(mod, before, k, v, cum(new)), compress_cache(mod, k, v, cum(new))
+    assert got.cu == want.cu and got.cu_c == want.cu_c and torch.equal(got.table_dev[:12], want.table_dev[:12])
+    _close("extended ck", got.ck, want.ck)
+    _close("extended cv", got.cv, want.cv)
+    with pytest.raises(ValueError):
+        extend_compress_cache(mod, want, k, v, cum([n - 1 for n in new]))
+    nsa._lib.device_status()
