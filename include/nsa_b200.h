@@ -57,6 +57,9 @@ int nsa_compress_fwd_kv(const void* k, const void* v, const void* w_k, const voi
                         const void* bias_v, void* ck, void* cv, const int32_t* cu_in, const int32_t* cu_out, int nseq, int T,
                         int Tc, long long total_in, long long total_out, int H, int D, int block, int stride, int split,
                         void* stream);
+/* Copies n int32 of host memory to the device as kernel parameters: asynchronous, no pinned memory, `host` may be reused at
+ * once (length tables). */
+int nsa_upload_table(const int32_t* host, int n, int32_t* dev, void* stream);
 /* Conv1d weights [D,D,block] (out channel, in channel, offset) -> the [block*D, D] layout above; w_v / out_v may be NULL. */
 int nsa_conv_weight_layout(const void* w_k, const void* w_v, void* out_k, void* out_v, int D, int block, void* stream);
 /* Replaces _compress_kv.backward (nsa/compression_kv.py:219-266, kernels :62-171) and the Conv1d backward.
@@ -151,6 +154,26 @@ size_t nsa_sel_swa_bwd_workspace_bytes(int B, int T, int Hkv, int S, int BS);
  * the two passes that recompute the selected branch's scores.  Extra bytes: B*Tq*Hkv*S*(4 + Hq/Hkv*D*2).  Used when
  * D = 128, BS = 64 and dq, dk, dv are all requested; with the smaller workspace the query-major kernel runs. */
 size_t nsa_sel_swa_bwd_workspace_bytes_dq(int B, int T, int Tq, int Hq, int Hkv, int D, int S, int BS);
+
+/* The reverse index of a selection (per KV head and block the ascending list of the tokens that selected it, and its inverse)
+ * built once for a forward and its backward: nsa_sel_index fills `index` (nsa_sel_index_bytes), which the _ix entry points
+ * take instead of building it in their workspace; they are otherwise nsa_sel_swa_fwd_ws and nsa_sel_swa_bwd_sharded, with
+ * workspaces of their own (without the index; the backward's holds partial sums that let the tokens of a key block be
+ * spread over several CTAs when there are fewer blocks than SMs).  Tq = T, q0 = 0 when not sharded. */
+size_t nsa_sel_swa_fwd_ix_workspace_bytes(int B, int T, int Tq, int Hq, int Hkv, int D, int S, int BS);
+size_t nsa_sel_swa_bwd_ix_workspace_bytes(int B, int T, int Tq, int Hq, int Hkv, int D, int S, int BS);
+size_t nsa_sel_index_bytes(int B, int T, int Tq, int Hkv, int S, int BS);
+int nsa_sel_index(const void* idx, int idx64, const int32_t* counts, void* index, size_t index_bytes, int B, int T, int Tq,
+                  int q0, int Hkv, int S, int BS, void* stream);
+int nsa_sel_swa_fwd_ix(const void* q, const void* k, const void* v, const void* idx, int idx64, const int32_t* counts,
+                       const void* index, void* o_slc, float* lse_slc, void* o_swa, float* lse_swa, const void* g_slc,
+                       const void* g_swa, const void* o_cmp, const void* g_cmp, void* o, void* ws, size_t ws_bytes, int B, int T,
+                       int Hq, int Hkv, int D, int S, int BS, int window, float scale, int Tq, int q0, void* stream);
+int nsa_sel_swa_bwd_ix(const void* q, const void* k, const void* v, const void* idx, int idx64, const int32_t* counts,
+                       const void* index, const void* dout_slc, const float* lse_slc, const float* delta_slc,
+                       const void* gate_slc, const void* dout_swa, const float* lse_swa, const float* delta_swa,
+                       const void* gate_swa, void* dq, int accumulate_dq, void* dk, void* dv, void* ws, size_t ws_bytes, int B,
+                       int T, int Hq, int Hkv, int D, int S, int BS, int window, float scale, int Tq, int q0, void* stream);
 
 /* Measurement aid, no counterpart in the reference: the K/V block gather of nsa_sel_swa_fwd's selected branch (same
  * items, same order, same TMA boxes of [BS keys x D]) with no arithmetic behind it, every SM keeping all of its shared

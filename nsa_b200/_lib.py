@@ -23,6 +23,7 @@ SIGNATURES = {
     "nsa_compress_fwd": (I, [P, P, P, P, P, P, I, I, I, I, I, I, P]),
     "nsa_compress_fwd_uniform": (I, [P, P, P, P, I, I, I, I, I, I, P]),
     "nsa_compress_fwd_kv": (I, [P] * 10 + [I, I, I, L, L, I, I, I, I, I, P]),
+    "nsa_upload_table": (I, [P, I, P, P]),
     "nsa_conv_weight_layout": (I, [P, P, P, P, I, I, P]),
     "nsa_cache_plan": (I, [P, P, P, I, I, I, P, P]),
     "nsa_cache_build": (I, [P] * 13 + [I, L, I, I, I, I, P]),
@@ -44,6 +45,12 @@ SIGNATURES = {
     "nsa_cmp_attn_bwd_sharded": (I, [P, P, P, P, P, P, P, P, I, P, P, P, Z, I, I, I, I, I, I, I, I, I, F, I, I, P]),
     "nsa_sel_swa_fwd_sharded": (I, [P, P, P, P, I, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, I, I, P]),
     "nsa_sel_swa_fwd_ws": (I, [P, P, P, P, I, P, P, P, P, P, P, P, P, P, P, P, Z, I, I, I, I, I, I, I, I, F, I, I, P]),
+    "nsa_sel_index_bytes": (Z, [I, I, I, I, I, I]),
+    "nsa_sel_index": (I, [P, I, P, P, Z, I, I, I, I, I, I, I, P]),
+    "nsa_sel_swa_fwd_ix_workspace_bytes": (Z, [I, I, I, I, I, I, I, I]),
+    "nsa_sel_swa_bwd_ix_workspace_bytes": (Z, [I, I, I, I, I, I, I, I]),
+    "nsa_sel_swa_fwd_ix": (I, [P, P, P, P, I, P, P, P, P, P, P, P, P, P, P, P, P, Z, I, I, I, I, I, I, I, I, F, I, I, P]),
+    "nsa_sel_swa_bwd_ix": (I, [P, P, P, P, I, P, P, P, P, P, P, P, P, P, P, P, I, P, P, P, Z, I, I, I, I, I, I, I, I, F, I, I, P]),
     "nsa_sel_swa_fwd_workspace_bytes": (Z, [I, I, I, I, I, I, I, I]),
     "nsa_sel_swa_bwd_sharded": (I, [P, P, P, P, I, P, P, P, P, P, P, P, P, P, P, I, P, P, P, Z, I, I, I, I, I, I, I, I,
                                     F, I, I, P]),
@@ -108,10 +115,22 @@ def sel_swa_bwd_workspace_bytes(B, T, Tq, Hq, Hkv, D, S, BS):
 SEL_FWD_KV = True
 
 
+def sel_fwd_kv_covers(Hq, Hkv, D, S, BS):
+    return SEL_FWD_KV and D == 128 and BS == 64 and S <= 32 and Hq % (16 * Hkv) == 0
+
+
 def sel_swa_fwd_workspace_bytes(B, T, Tq, Hq, Hkv, D, S, BS):
-    if SEL_FWD_KV and D == 128 and BS == 64 and S <= 32 and Hq % (16 * Hkv) == 0:
+    if sel_fwd_kv_covers(Hq, Hkv, D, S, BS):
         return lib().nsa_sel_swa_fwd_workspace_bytes(B, T, Tq, Hq, Hkv, D, S, BS)
     return 0
+
+
+def device_table(values, device):
+    """A host list of int32 as a device tensor, without a stream synchronisation."""
+    n = len(values)
+    t = torch.empty(n, dtype=torch.int32, device=device)
+    check(lib().nsa_upload_table((ctypes.c_int32 * n)(*values), n, t.data_ptr(), stream()), "nsa_upload_table")
+    return t
 
 
 def ptr(t):

@@ -18,26 +18,12 @@ def calc_compressed_len(x, stride, size):
     return (x - size) // stride
 
 
-_cu_cache = {}
-
-
-def _cu_tensor(values, device):
-    key = (tuple(values), str(device))
-    t = _cu_cache.get(key)
-    if t is None:
-        if len(_cu_cache) > 64:
-            _cu_cache.clear()
-        t = torch.tensor(list(values), dtype=torch.int32, device=device)
-        _cu_cache[key] = t
-    return t
-
-
 class _CompressPair(torch.autograd.Function):
     """(ck, cv) = compress(k; w_k, b_k), compress(v; w_v, b_v).  k, v [tok,H,D]; weights [l*D, D]; biases [D] or None.
     ``split``: see nsa_compress_fwd_kv; False where a block selection follows."""
 
     @staticmethod
-    def forward(ctx, k, v, w_k, w_v, b_k, b_v, cu_in, cu_out, block, stride, split):
+    def forward(ctx, k, v, w_k, w_v, b_k, b_v, cu_in, cu_out, block, stride, split, table=None):
         k, v, w_k, w_v = (_lib.require(t, n) for t, n in ((k, "k"), (v, "v"), (w_k, "w_k"), (w_v, "w_v")))
         b_k, b_v = _lib.require(b_k, "bias"), _lib.require(b_v, "bias")
         tok, H, D = k.shape
@@ -47,21 +33,23 @@ class _CompressPair(torch.autograd.Function):
         nseq, total_out = len(cu_in) - 1, cu_out[-1]
         ck = torch.empty(total_out, H, D, dtype=torch.bfloat16, device=k.device)
         cv = torch.empty(total_out, H, D, dtype=torch.bfloat16, device=k.device)
-        cin, cout = _cu_tensor(cu_in, k.device), _cu_tensor(cu_out, k.device)
-        P = _lib.ptr
+        if table is None:
+            table = _lib.device_table([*cu_in, *cu_out], k.device)   # cu_in, then cu_out
+        P, cin = _lib.ptr, table.data_ptr()
         if total_out > 0:
-            _lib.check(_lib.lib().nsa_compress_fwd_kv(P(k), P(v), P(w_k), P(w_v), P(b_k), P(b_v), P(ck), P(cv), P(cin), P(cout),
-                                                      nseq, 0, 0, tok, total_out, H, D, block, stride, split,
+            _lib.check(_lib.lib().nsa_compress_fwd_kv(P(k), P(v), P(w_k), P(w_v), P(b_k), P(b_v), P(ck), P(cv), cin,
+                                                      cin + 4 * (nseq + 1), nseq, 0, 0, tok, total_out, H, D, block, stride, split,
                                                       _lib.stream()),
                        "nsa_compress_fwd_kv")
-        ctx.save_for_backward(k, v, w_k, w_v, cin, cout)
+        ctx.save_for_backward(k, v, w_k, w_v, table)
         ctx.meta = (nseq, H, D, block, stride, max([b - a for a, b in zip(cu_in[:-1], cu_in[1:])] + [0]), total_out)
         return ck, cv
 
     @staticmethod
     def backward(ctx, dck, dcv):
-        k, v, w_k, w_v, cin, cout = ctx.saved_tensors
+        k, v, w_k, w_v, table = ctx.saved_tensors
         nseq, H, D, block, stride, max_in, total_out = ctx.meta
+        cin, cout = table.data_ptr(), table.data_ptr() + 4 * (nseq + 1)
         L, P, need = _lib.lib(), _lib.ptr, ctx.needs_input_grad
         ws_bytes = L.nsa_compress_bwd_kv_workspace_bytes(nseq, 0, total_out, 1, H, D, block, stride)
         if ws_bytes and total_out > 0:   # both tensors on the tensor cores (block = stride or 2 * stride)
@@ -71,9 +59,9 @@ class _CompressPair(torch.autograd.Function):
             dbk, dbv = (torch.empty(D, dtype=torch.bfloat16, device=k.device) if n else None for n in need[4:6])
             ws = torch.empty(ws_bytes, dtype=torch.uint8, device=k.device) if any(need[2:6]) else None
             _lib.check(L.nsa_compress_bwd_kv(P(k), P(v), P(w_k), P(w_v), P(dck), P(dcv), P(dk), P(dv), 0, P(dwk), P(dwv), P(dbk),
-                                             P(dbv), 1, P(ws), ws_bytes, P(cin), P(cout), nseq, 0, 0, k.shape[0], total_out, H, D,
+                                             P(dbv), 1, P(ws), ws_bytes, cin, cout, nseq, 0, 0, k.shape[0], total_out, H, D,
                                              block, stride, _lib.stream()), "nsa_compress_bwd_kv")
-            return dk, dv, dwk, dwv, dbk, dbv, None, None, None, None, None
+            return dk, dv, dwk, dwv, dbk, dbv, None, None, None, None, None, None
         ws_bytes = L.nsa_compress_bwd_workspace_bytes(nseq, H, D, block) if need[2] or need[3] else 0
         ws = torch.empty(ws_bytes, dtype=torch.uint8, device=k.device) if ws_bytes else None
         grads = []
@@ -83,7 +71,7 @@ class _CompressPair(torch.autograd.Function):
             dw = torch.empty(block * D, D, dtype=torch.float32, device=x.device) if need[2 + i] else None
             db = torch.empty(D, dtype=torch.float32, device=x.device) if need[4 + i] else None
             if total_out > 0:
-                _lib.check(L.nsa_compress_bwd(P(x), P(w), P(dy), P(dx), P(dw), P(db), P(ws), ws_bytes, P(cin), P(cout), nseq, H,
+                _lib.check(L.nsa_compress_bwd(P(x), P(w), P(dy), P(dx), P(dw), P(db), P(ws), ws_bytes, cin, cout, nseq, H,
                                               D, block, stride, max_in, total_out, _lib.stream()), "nsa_compress_bwd")
             else:
                 for t in (dx, dw, db):
@@ -91,7 +79,7 @@ class _CompressPair(torch.autograd.Function):
                         t.zero_()
             grads.append((dx, dw, db))
         (dk, dwk, dbk), (dv, dwv, dbv) = grads
-        return dk, dv, dwk, dwv, dbk, dbv, None, None, None, None, None
+        return dk, dv, dwk, dwv, dbk, dbv, None, None, None, None, None, None
 
 
 def _host_cu(cu_seq_len):
@@ -106,8 +94,9 @@ def compress_kv(k, v, w_k, w_v, cu_seq_len, block_stride, block_size):
     cu_out = [0]
     for i in range(len(cu_in) - 1):
         cu_out.append(cu_out[-1] + max(calc_compressed_len(cu_in[i + 1] - cu_in[i], block_stride, block_size), 0))
-    ck, cv = _CompressPair.apply(k, v, w_k, w_v, None, None, cu_in, cu_out, block_size, block_stride, True)
-    return ck, cv, _cu_tensor(cu_out, k.device)
+    table = _lib.device_table(cu_in + cu_out, k.device)
+    ck, cv = _CompressPair.apply(k, v, w_k, w_v, None, None, cu_in, cu_out, block_size, block_stride, True, table)
+    return ck, cv, table[len(cu_in):]
 
 
 class _ConvLayout(torch.autograd.Function):

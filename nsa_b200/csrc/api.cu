@@ -36,14 +36,34 @@ static int check_attn_shape(const char* who, int B, int T, int Hq, int Hk, int D
   return 0;
 }
 
-static int cmp_segments(int T, int* seg_len) {
-  int nseg = (T + 1023) / 1024;
+static int check_bs(const char* who, int BS) {
+  if (BS != 16 && BS != 32 && BS != 64) return fail(-9, "%s: selection block size %d not supported (16, 32, 64)", who, BS);
+  return 0;
+}
+
+// Token segments of the compressed branch's key-major backward: at least one per 1024 tokens (16 at most), more while the
+// (batch, head, key tile) CTAs alone do not give every SM about four pieces of work, at least 64 tokens each.  `tiles` =
+// B * Hk * ceil(Tc / 64).
+static int cmp_segments(int T, long long tiles, int* seg_len) {
+  long long nseg = (T + 1023) / 1024;
   if (nseg > 16) nseg = 16;
+  const long long want = (4LL * num_sms() + tiles - 1) / (tiles > 0 ? tiles : 1);
+  if (nseg < want) nseg = want;
+  if (nseg > (T + 63) / 64) nseg = (T + 63) / 64;
   if (nseg < 1) nseg = 1;
-  int sl = (T + nseg - 1) / nseg;
+  int sl = (int)((T + nseg - 1) / nseg);
   sl = (sl + 63) / 64 * 64;
   *seg_len = sl;
   return (T + sl - 1) / sl;
+}
+
+// Shares of a key block's token stream in the key-major backward of the selected and window branches: one CTA per block
+// when the blocks fill the GPU four times over (the first blocks are visited most, so one wave is not enough), else enough
+// shares for about that many CTAs (at most 16; a share then still has some dozens of tokens).  With more than one share the
+// CTAs leave fp32 partials that a second kernel adds in order.
+static int kv_shares(long long blocks) {
+  const long long ns = 4LL * num_sms() / (blocks > 0 ? blocks : 1);
+  return (int)(ns < 1 ? 1 : ns > 16 ? 16 : ns);
 }
 
 static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
@@ -130,6 +150,11 @@ int nsa_compress_fwd_kv(const void* k, const void* v, const void* w_k, const voi
   a.ntensor = 2; a.cu_in = cu_in; a.cu_out = cu_out; a.cu_row = cu_out; a.rows = total_out; a.split = split;
   a.nseq = nseq; a.T = T; a.Tc = Tc; a.total_in = total_in; a.H = H; a.D = D; a.l = block; a.d = stride;
   return launch_compress_fwd_tc(a, (cudaStream_t)stream);
+}
+
+int nsa_upload_table(const int32_t* host, int n, int32_t* dev, void* stream) {
+  if (n > 0 && (!host || !dev)) return fail(-1, "nsa_upload_table: null pointer");
+  return launch_upload_table(host, n, dev, (cudaStream_t)stream);
 }
 
 int nsa_conv_weight_layout(const void* w_k, const void* w_v, void* out_k, void* out_v, int D, int block, void* stream) {
@@ -323,7 +348,7 @@ int nsa_cmp_attn_fwd_gated(const void* q, const void* ck, const void* cv, void* 
 
 size_t nsa_cmp_attn_bwd_workspace_bytes(int B, int T, int Tc, int Hk, int D) {
   int sl;
-  const int nseg = cmp_segments(T, &sl);
+  const int nseg = cmp_segments(T, (long long)B * Hk * ((Tc + 63) / 64), &sl);
   return (size_t)2 * nseg * B * Tc * Hk * D * sizeof(float);
 }
 
@@ -374,7 +399,7 @@ static int cmp_attn_bwd_impl(const void* q, const void* ck, const void* cv, cons
     KvArgs a = {};
     a.mode = 1; a.q = (const bf16*)q; a.k = (const bf16*)ck; a.v = (const bf16*)cv;
     a.dout_a = (const bf16*)dout; a.lse_a = lse; a.delta_a = delta; a.gate_a = (const bf16*)gate;
-    a.part = (float*)ws; a.nseg = cmp_segments(Tq, &a.seg_len);
+    a.part = (float*)ws; a.nseg = cmp_segments(Tq, (long long)B * Hk * ((Tc + 63) / 64), &a.seg_len);
     a.B = B; a.T = T; a.Tq = Tq; a.q0 = q0; a.Lk = Tc; a.Hq = Hq; a.Hk = Hk; a.BS = 64; a.cblock = block; a.cstride = stride;
     a.causal = causal; a.scale = scale;
     if (D != 128 && sharded) return fail(-11, "query shards need head_dim 128");
@@ -405,25 +430,61 @@ int nsa_cmp_attn_bwd_sharded(const void* q, const void* ck, const void* cv, cons
 }
 
 // ---- selected + sliding window ----------------------------------------------------------------------
-static int check_bs(const char* who, int BS) {
-  if (BS != 16 && BS != 32 && BS != 64) return fail(-9, "%s: selection block size %d not supported (16, 32, 64)", who, BS);
-  return 0;
+
+// The reverse index of a selection in one buffer: histogram, CSR offsets, token lists, and its inverse.  Returns the bytes.
+static size_t rev_layout(void* base, const void* idx, int idx64, const int32_t* counts, int B, int T, int Tq, int q0, int Hkv,
+                         int S, int BS, RevArgs* r) {
+  const size_t NB = (size_t)(T + BS - 1) / BS, bh = (size_t)B * Hkv;
+  size_t n[4] = {align_up(bh * NB * NB * 4, 256), align_up(bh * (NB + 1) * 4, 256), align_up(bh * (size_t)T * S * 4, 256),
+                 align_up((size_t)B * Tq * Hkv * S * 4, 256)};
+  if (r) {
+    *r = {};
+    r->idx = idx; r->idx64 = idx64; r->counts = counts; r->B = B; r->T = T; r->Tq = Tq; r->q0 = q0; r->H = Hkv; r->S = S;
+    r->BS = BS; r->NB = (int)NB; r->cap = (long long)Tq * S;
+    char* p = (char*)base;
+    r->hist = (int*)p;
+    r->rev_ptr = (int*)(p + n[0]);
+    r->rev_tok = (int*)(p + n[0] + n[1]);
+    r->inv = (int*)(p + n[0] + n[1] + n[2]);
+  }
+  return n[0] + n[1] + n[2] + n[3];
 }
 
-// Workspace of the key-major selected forward: the reverse index (as in the backward), its inverse [B,Tq,Hkv,S] int32,
-// one [16 x D] bf16 tile and 16 (max, sum) pairs per (list position, 16-head sub-group).
+size_t nsa_sel_index_bytes(int B, int T, int Tq, int Hkv, int S, int BS) {
+  return BS <= 0 ? 0 : rev_layout(nullptr, nullptr, 0, nullptr, B, T, Tq, 0, Hkv, S, BS, nullptr);
+}
+
+int nsa_sel_index(const void* idx, int idx64, const int32_t* counts, void* index, size_t index_bytes, int B, int T, int Tq,
+                  int q0, int Hkv, int S, int BS, void* stream) {
+  if (!idx || !index) return fail(-1, "nsa_sel_index: null pointer");
+  if (B <= 0 || T <= 0 || Hkv <= 0 || S <= 0) return fail(-1, "nsa_sel_index: empty or negative shape");
+  if (Tq <= 0 || q0 < 0 || q0 + Tq > T) return fail(-12, "nsa_sel_index: query shard [%d, %d) is outside the sequence of %d tokens", q0, q0 + Tq, T);
+  const int rc = check_bs("nsa_sel_index", BS);
+  if (rc) return rc;
+  if (index_bytes < nsa_sel_index_bytes(B, T, Tq, Hkv, S, BS)) return fail(-6, "nsa_sel_index: buffer too small");
+  RevArgs r;
+  rev_layout(index, idx, idx64, counts, B, T, Tq, q0, Hkv, S, BS, &r);
+  return launch_build_rev(r, (cudaStream_t)stream);
+}
+
+// Workspace of the key-major selected forward: the reverse index, one [16 x D] bf16 tile and 16 (max, sum) pairs per
+// (list position, 16-head sub-group).
+size_t nsa_sel_swa_fwd_ix_workspace_bytes(int B, int T, int Tq, int Hq, int Hkv, int D, int S, int BS) {
+  if (BS <= 0 || Hkv <= 0) return 0;
+  const size_t ent = (size_t)B * Tq * S * Hq;   // (list position, head) pairs
+  return align_up(ent * D * 2, 256) + align_up(ent * 8, 256);
+}
+
 size_t nsa_sel_swa_fwd_workspace_bytes(int B, int T, int Tq, int Hq, int Hkv, int D, int S, int BS) {
   if (BS <= 0 || Hkv <= 0) return 0;
-  const size_t ent = (size_t)B * Tq * Hkv * S;
-  const size_t g = (size_t)(Hq / Hkv);
-  return nsa_sel_swa_bwd_workspace_bytes(B, T, Hkv, S, BS) + align_up(ent * 4, 256) + align_up(ent * g * D * 2, 256) +
-         align_up(ent * g * 8, 256);
+  return nsa_sel_index_bytes(B, T, Tq, Hkv, S, BS) + nsa_sel_swa_fwd_ix_workspace_bytes(B, T, Tq, Hq, Hkv, D, S, BS);
 }
 
 static int sel_swa_fwd_impl(const void* q, const void* k, const void* v, const void* idx, int idx64, const int32_t* counts,
                     void* o_slc, float* lse_slc, void* o_swa, float* lse_swa, const void* g_slc, const void* g_swa,
                     const void* o_cmp, const void* g_cmp, void* o, int B, int T, int Hq, int Hkv, int D, int S, int BS,
-                    int window, float scale, int Tq, int q0, void* stream, void* ws = nullptr, size_t ws_bytes = 0) {
+                    int window, float scale, int Tq, int q0, void* stream, void* ws = nullptr, size_t ws_bytes = 0,
+                    const void* index = nullptr) {
   const bool sharded = (Tq != T) || (q0 != 0);
   if (Tq <= 0 || q0 < 0 || q0 + Tq > T) return fail(-12, "%s: query shard [%d, %d) is outside the sequence of %d tokens", "nsa_sel_swa_fwd", q0, q0 + Tq, T);
   (void)sharded;
@@ -439,27 +500,19 @@ static int sel_swa_fwd_impl(const void* q, const void* k, const void* v, const v
     SelKvArgs ka = {};
     ka.q = (const bf16*)q; ka.k = (const bf16*)k; ka.v = (const bf16*)v; ka.o = (bf16*)o_slc; ka.lse = lse_slc;
     ka.B = B; ka.T = T; ka.Tq = Tq; ka.q0 = q0; ka.Hq = Hq; ka.Hk = Hkv; ka.S = S; ka.BS = BS; ka.scale = scale;
-    if (ws && sel_fwd_kv_supported(ka, D) && ws_bytes >= nsa_sel_swa_fwd_workspace_bytes(B, T, Tq, Hq, Hkv, D, S, BS)) {
+    if (ws && sel_fwd_kv_supported(ka, D) &&
+        ws_bytes >= (index ? nsa_sel_swa_fwd_ix_workspace_bytes(B, T, Tq, Hq, Hkv, D, S, BS)
+                           : nsa_sel_swa_fwd_workspace_bytes(B, T, Tq, Hq, Hkv, D, S, BS))) {
       // key-major: reverse index, then one CTA per key block over the queries that selected it, then the per-token merge
-      const int NB = (T + BS - 1) / BS;
-      const size_t bh = (size_t)B * Hkv, ent = (size_t)B * Tq * Hkv * S, g = (size_t)(Hq / Hkv);
-      char* p = (char*)ws;
-      RevArgs r = {};
-      r.idx = idx; r.idx64 = idx64; r.counts = counts; r.B = B; r.T = T; r.Tq = Tq; r.q0 = q0; r.H = Hkv; r.S = S; r.BS = BS; r.NB = NB;
-      r.hist = (int*)p;
-      p += align_up(bh * NB * NB * 4, 256);
-      r.rev_ptr = (int*)p;
-      p += align_up(bh * (NB + 1) * 4, 256);
-      r.rev_tok = (int*)p;
-      p += align_up(bh * (size_t)T * S * 4, 256);
-      r.cap = (long long)Tq * S;
-      r.inv = (int*)p;
-      p += align_up(ent * 4, 256);
+      RevArgs r;
+      const size_t nrev = rev_layout(index ? const_cast<void*>(index) : ws, idx, idx64, counts, B, T, Tq, q0, Hkv, S, BS, &r);
+      char* p = (char*)ws + (index ? 0 : nrev);
       ka.part = (bf16*)p;
-      p += align_up(ent * g * D * 2, 256);
-      ka.stats = (float*)p;
-      rc = launch_build_rev(r, s);
-      if (rc) return rc;
+      ka.stats = (float*)(p + align_up((size_t)B * Tq * S * Hq * D * 2, 256));
+      if (!index) {
+        rc = launch_build_rev(r, s);
+        if (rc) return rc;
+      }
       ka.rev_ptr = r.rev_ptr; ka.rev_tok = r.rev_tok; ka.rev_cap = r.cap;
       rc = launch_sel_fwd_kv(ka, r, s);
       if (rc) return rc;
@@ -509,6 +562,13 @@ int nsa_sel_swa_fwd_ws(const void* q, const void* k, const void* v, const void* 
   return sel_swa_fwd_impl(q, k, v, idx, idx64, counts, o_slc, lse_slc, o_swa, lse_swa, g_slc, g_swa, o_cmp, g_cmp, o, B, T, Hq, Hkv, D, S, BS, window, scale, Tq, q0, stream, ws, ws_bytes);
 }
 
+int nsa_sel_swa_fwd_ix(const void* q, const void* k, const void* v, const void* idx, int idx64, const int32_t* counts,
+                       const void* index, void* o_slc, float* lse_slc, void* o_swa, float* lse_swa, const void* g_slc,
+                       const void* g_swa, const void* o_cmp, const void* g_cmp, void* o, void* ws, size_t ws_bytes, int B, int T,
+                       int Hq, int Hkv, int D, int S, int BS, int window, float scale, int Tq, int q0, void* stream) {
+  return sel_swa_fwd_impl(q, k, v, idx, idx64, counts, o_slc, lse_slc, o_swa, lse_swa, g_slc, g_swa, o_cmp, g_cmp, o, B, T, Hq, Hkv, D, S, BS, window, scale, Tq, q0, stream, ws, ws_bytes, index);
+}
+
 int nsa_cmp_attn_bwd_fused(const void* q, const void* ck, const void* cv, const void* o_cmp, const float* lse, const void* dout,
                            float* delta, const void* gate, void* dgate, void* dq, int accumulate_dq, void* dck, void* dcv,
                            void* ws, size_t ws_bytes, int B, int T, int Tc, int Hq, int Hk, int D, int block, int stride,
@@ -524,11 +584,25 @@ size_t nsa_sel_swa_bwd_workspace_bytes(int B, int T, int Hkv, int S, int BS) {
   return align_up(bh * NB * NB * 4, 256) + align_up(bh * (NB + 1) * 4, 256) + align_up(bh * (size_t)T * S * 4, 256);
 }
 
-// Extra workspace behind the reverse index for the selected branch's dQ as per-visit partials of the kv-major backward:
-// the inverse index [B,Tq,Hkv,S] int32 and one [16 x D] bf16 tile per (list position, 16-head sub-group).
-static size_t sel_dq_extra_bytes(int B, int Tq, int Hq, int Hkv, int D, int S) {
-  const size_t ent = (size_t)B * Tq * Hkv * S;
-  return align_up(ent * 4, 256) + align_up(ent * (size_t)(Hq / Hkv) * D * 2, 256);
+// Behind the reverse index: one [16 x D] bf16 tile per (list position, 16-head sub-group) for the selected branch's dQ as
+// per-visit partials (tcgen05 kernel only), then the fp32 dK, dV partials of the shares.
+static bool dq_from_kv_covers(int D, int S, int BS) { return D == 128 && BS == 64 && S <= 32; }
+static size_t sel_dq_tile_bytes(int B, int Tq, int Hq, int D, int S, int BS) {
+  return dq_from_kv_covers(D, S, BS) ? align_up((size_t)B * Tq * Hq * S * D * 2, 256) : 0;
+}
+static size_t kv_share_bytes(int B, int T, int Hkv, int D, int BS) {
+  const int ns = kv_shares((long long)B * Hkv * ((T + BS - 1) / BS));
+  return ns > 1 ? (size_t)2 * ns * B * T * Hkv * D * sizeof(float) : 0;
+}
+
+size_t nsa_sel_swa_bwd_workspace_bytes_dq(int B, int T, int Tq, int Hq, int Hkv, int D, int S, int BS) {
+  if (BS <= 0 || Hkv <= 0) return 0;
+  return nsa_sel_index_bytes(B, T, Tq, Hkv, S, BS) + align_up((size_t)B * Tq * Hq * S * D * 2, 256);
+}
+
+size_t nsa_sel_swa_bwd_ix_workspace_bytes(int B, int T, int Tq, int Hq, int Hkv, int D, int S, int BS) {
+  if (BS <= 0 || Hkv <= 0) return 0;
+  return sel_dq_tile_bytes(B, Tq, Hq, D, S, BS) + kv_share_bytes(B, T, Hkv, D, BS);
 }
 
 struct PreSel {   // row pre-pass of the selected and window branches folded into the window's dQ kernel
@@ -541,7 +615,7 @@ static int sel_swa_bwd_impl(const void* q, const void* k, const void* v, const v
                     const void* dout_swa, const float* lse_swa, const float* delta_swa, const void* gate_swa, void* dq,
                     int accumulate_dq, void* dk, void* dv, void* ws, size_t ws_bytes, int B, int T, int Hq, int Hkv,
                     int D, int S, int BS, int window, float scale, int Tq, int q0, void* stream,
-                    const PreSel* pre = nullptr) {
+                    const PreSel* pre = nullptr, const void* index = nullptr) {
   const bool sharded = (Tq != T) || (q0 != 0);
   if (Tq <= 0 || q0 < 0 || q0 + Tq > T) return fail(-12, "%s: query shard [%d, %d) is outside the sequence of %d tokens", "nsa_sel_swa_bwd", q0, q0 + Tq, T);
   (void)sharded;
@@ -558,8 +632,11 @@ static int sel_swa_bwd_impl(const void* q, const void* k, const void* v, const v
   const long long rows = (long long)B * Tq * Hq;
   // With the larger workspace of nsa_sel_swa_bwd_workspace_bytes_dq the selected branch's dQ is produced by the
   // kv-major backward (per-visit partial tiles + a slot-order reduction) instead of the query-major dQ kernel.
-  const bool dq_from_kv = dq && dk && has_slc && D == 128 && BS == 64 && S <= 32 && ws &&
-                          ws_bytes >= nsa_sel_swa_bwd_workspace_bytes(B, T, Hkv, S, BS) + sel_dq_extra_bytes(B, Tq, Hq, Hkv, D, S);
+  // (A caller that hands over a reverse index gives the workspace behind it alone, with room for the shares.)
+  if (index && ws_bytes < nsa_sel_swa_bwd_ix_workspace_bytes(B, T, Tq, Hq, Hkv, D, S, BS))
+    return fail(-6, "nsa_sel_swa_bwd_ix: workspace too small");
+  const bool large_ws = index || (ws && ws_bytes >= nsa_sel_swa_bwd_workspace_bytes_dq(B, T, Tq, Hq, Hkv, D, S, BS));
+  const bool dq_from_kv = dq && dk && has_slc && dq_from_kv_covers(D, S, BS) && large_ws;
   int dq_acc_for_reduce = accumulate_dq;
   bool fold = false;
   if (pre) {
@@ -631,26 +708,15 @@ static int sel_swa_bwd_impl(const void* q, const void* k, const void* v, const v
     a.dk = (bf16*)dk; a.dv = (bf16*)dv;
     RevArgs r = {};
     if (has_slc) {
-      if (!ws || ws_bytes < nsa_sel_swa_bwd_workspace_bytes(B, T, Hkv, S, BS))
+      if (!index && (!ws || ws_bytes < nsa_sel_swa_bwd_workspace_bytes(B, T, Hkv, S, BS)))
         return fail(-6, "nsa_sel_swa_bwd: workspace too small");
-      const int NB = (T + BS - 1) / BS;
-      const size_t bh = (size_t)B * Hkv;
-      char* p = (char*)ws;
-      r.idx = idx; r.idx64 = idx64; r.counts = counts; r.B = B; r.T = T; r.Tq = Tq; r.q0 = q0; r.H = Hkv; r.S = S; r.BS = BS; r.NB = NB;
-      r.hist = (int*)p;
-      p += align_up(bh * NB * NB * 4, 256);
-      r.rev_ptr = (int*)p;
-      p += align_up(bh * (NB + 1) * 4, 256);
-      r.rev_tok = (int*)p;
-      r.cap = (long long)Tq * S;
-      if (dq_from_kv) {
-        p += align_up(bh * (size_t)T * S * 4, 256);
-        r.inv = (int*)p;
-        p += align_up((size_t)B * Tq * Hkv * S * 4, 256);
-        a.dq_part = (bf16*)p;
+      const size_t nrev = rev_layout(index ? const_cast<void*>(index) : ws, idx, idx64, counts, B, T, Tq, q0, Hkv, S, BS, &r);
+      if (!index && !large_ws) r.inv = nullptr;   // the small workspace ends behind the token lists
+      if (dq_from_kv) a.dq_part = (bf16*)((char*)ws + (index ? 0 : nrev));
+      if (!index) {
+        rc = launch_build_rev(r, s);
+        if (rc) return rc;
       }
-      rc = launch_build_rev(r, s);
-      if (rc) return rc;
       a.rev_ptr = r.rev_ptr; a.rev_tok = r.rev_tok; a.rev_cap = r.cap;
       a.dout_a = (const bf16*)dout_slc; a.lse_a = lse_slc; a.delta_a = delta_slc; a.gate_a = (const bf16*)gate_slc;
     }
@@ -658,18 +724,23 @@ static int sel_swa_bwd_impl(const void* q, const void* k, const void* v, const v
       a.dout_b = (const bf16*)dout_swa; a.lse_b = lse_swa; a.delta_b = delta_swa; a.gate_b = (const bf16*)gate_swa;
     }
     if (!(D == 128 && BS == 64) && sharded) return fail(-11, "query shards need head_dim 128 and 64-key selection blocks");
+    a.nshare = 1;
+    if (index) {
+      a.nshare = kv_shares((long long)B * Hkv * ((T + BS - 1) / BS));
+      a.part = (float*)((char*)ws + sel_dq_tile_bytes(B, Tq, Hq, D, S, BS));
+    }
     rc = (D == 128 && BS == 64) ? launch_kv_bwd_tc(a, s) : launch_kv_bwd(a, D, s);
     if (rc) return rc;
+    if (a.nshare > 1) {
+      rc = launch_reduce_shares(a.part, a.dk, a.dv, a.nshare, (long long)B * T * Hkv * D, s);
+      if (rc) return rc;
+    }
     if (dq_from_kv) {   // every token's partial tiles, in slot order, onto dq (after the window's dQ if that ran first)
       rc = launch_sel_dq_reduce(r, a.dq_part, (bf16*)dq, Hq, D, scale, dq_acc_for_reduce, s);
       if (rc) return rc;
     }
   }
   return 0;
-}
-
-size_t nsa_sel_swa_bwd_workspace_bytes_dq(int B, int T, int Tq, int Hq, int Hkv, int D, int S, int BS) {
-  return nsa_sel_swa_bwd_workspace_bytes(B, T, Hkv, S, BS) + sel_dq_extra_bytes(B, Tq, Hq, Hkv, D, S);
 }
 
 int nsa_sel_swa_bwd(const void* q, const void* k, const void* v, const void* idx, int idx64, const int32_t* counts,
@@ -686,6 +757,14 @@ int nsa_sel_swa_bwd_sharded(const void* q, const void* k, const void* v, const v
                     int accumulate_dq, void* dk, void* dv, void* ws, size_t ws_bytes, int B, int T, int Hq, int Hkv,
                     int D, int S, int BS, int window, float scale, int Tq, int q0, void* stream) {
   return sel_swa_bwd_impl(q, k, v, idx, idx64, counts, dout_slc, lse_slc, delta_slc, gate_slc, dout_swa, lse_swa, delta_swa, gate_swa, dq, accumulate_dq, dk, dv, ws, ws_bytes, B, T, Hq, Hkv, D, S, BS, window, scale, Tq, q0, stream);
+}
+
+int nsa_sel_swa_bwd_ix(const void* q, const void* k, const void* v, const void* idx, int idx64, const int32_t* counts,
+                       const void* index, const void* dout_slc, const float* lse_slc, const float* delta_slc,
+                       const void* gate_slc, const void* dout_swa, const float* lse_swa, const float* delta_swa,
+                       const void* gate_swa, void* dq, int accumulate_dq, void* dk, void* dv, void* ws, size_t ws_bytes, int B,
+                       int T, int Hq, int Hkv, int D, int S, int BS, int window, float scale, int Tq, int q0, void* stream) {
+  return sel_swa_bwd_impl(q, k, v, idx, idx64, counts, dout_slc, lse_slc, delta_slc, gate_slc, dout_swa, lse_swa, delta_swa, gate_swa, dq, accumulate_dq, dk, dv, ws, ws_bytes, B, T, Hq, Hkv, D, S, BS, window, scale, Tq, q0, stream, nullptr, index);
 }
 
 int nsa_gather_probe(const void* k, const void* v, const void* idx, int idx64, int B, int T, int Hq, int Hkv, int D, int S,

@@ -271,13 +271,24 @@ __global__ void __launch_bounds__(kGateThreads, 2) gate_bwd_kernel(const bf16* _
   }
 }
 
-// dW[g][c] and db[g] = sum over the block partials, in block order (one thread per output)
-__global__ void gate_reduce_kernel(const float* __restrict__ part, int nblk, int D, bf16* __restrict__ dw,
-                                   bf16* __restrict__ db) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 3 * D + 3) return;
+// dW[g][c] and db[g] = sum over the block partials.  A block owns 32 outputs (one per lane, so loads are coalesced); its
+// eight warps take every eighth partial and meet in shared memory in warp order.
+__global__ void __launch_bounds__(256) gate_reduce_kernel(const float* __restrict__ part, int nblk, int D, bf16* __restrict__ dw,
+                                                         bf16* __restrict__ db) {
+  __shared__ float red[8][33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + lane;
   float s = 0.f;
-  for (int b = 0; b < nblk; ++b) s += part[(long long)b * (3 * D + 4) + i];
+  if (i < 3 * D + 3) {
+#pragma unroll 8
+    for (int b = warp; b < nblk; b += 8) s += part[(long long)b * (3 * D + 4) + i];
+  }
+  red[warp][lane] = s;
+  __syncthreads();
+  if (warp || i >= 3 * D + 3) return;
+  s = red[0][lane];
+#pragma unroll
+  for (int w = 1; w < 8; ++w) s += red[w][lane];
   if (i < 3 * D)
     dw[i] = __float2bfloat16(s);
   else if (db)
@@ -358,7 +369,7 @@ int launch_gate_bwd(const bf16* q, const bf16* dg0, const bf16* dg1, const bf16*
     set_error("head_dim %d not supported (64 or 128)", D);
     return -2;
   }
-  gate_reduce_kernel<<<(3 * D + 3 + 127) / 128, 128, 0, s>>>(workspace, grid, D, dw, db);
+  gate_reduce_kernel<<<(3 * D + 3 + 31) / 32, 256, 0, s>>>(workspace, grid, D, dw, db);
   note_launches(2);
   return (int)cudaGetLastError();
 }

@@ -106,8 +106,9 @@ struct KvArgs {
   bf16* dv;
   bf16* dq_part;          // mode 0, optional: the selected branch's dQ as per-visit partial tiles [B,Hk,rev_cap,G16][16][D]
                           // (position = place in the reverse-index list), summed later by launch_sel_dq_reduce
-  float* part;            // mode 1 workspace: [2][nseg][B,Lk,Hk,D] fp32
-  int nseg, seg_len;
+  float* part;            // fp32 partials [2][nseg or nshare][B,Lk,Hk,D]: dK then dV (mode 0: only with nshare > 1)
+  int nseg, seg_len;      // mode 1: token segments
+  int nshare;             // mode 0: shares of a block's token stream
   int B, T, Lk, Hq, Hk, BS, window;
   int cblock, cstride, causal;
   float scale;
@@ -292,6 +293,8 @@ int launch_sel_dq_reduce(const RevArgs& a, const bf16* part, bf16* dq, int Hq, i
 // out(bf16)[i] = sum over valid segments of part[seg][i]
 int launch_reduce_segments(const float* part, bf16* out, int nseg, long long n_per_seg, int q0, int Tq, int Lk, int Hk,
                            int D, int seg_len, int cblock, int cstride, int causal, cudaStream_t s);
+// dk, dv (bf16) = sum over the shares of part [2][nshare][n]
+int launch_reduce_shares(const float* part, bf16* dk, bf16* dv, int nshare, long long n, cudaStream_t s);
 int misc_status(int* out);
 
 int num_sms();

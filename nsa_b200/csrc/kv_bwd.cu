@@ -17,7 +17,9 @@
 //     S^T = K.Q^T      P^T = exp(S^T*scale - lse)      dV += (g.P^T).dO
 //     dP^T = V.dO^T    dS^T = P^T.(g.dP^T - delta)     dK += dS^T.Q   (times scale at the end)
 // The compressed branch splits its long token range into segments that write fp32 partials, reduced by a
-// second kernel in a fixed order (deterministic).
+// second kernel in a fixed order (deterministic); so does a block of the selected + window branches when there are
+// fewer blocks than SMs (a share walks its tokens one after the other at ~0.9 us each: 1.0 ms for the first block of a
+// 1024-token sequence with one KV head in one piece, 0.07 ms in 16).
 #include "kernels.h"
 #include "tmap.h"
 
@@ -72,6 +74,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     long long item = blockIdx.x;
     const int BH = a.B * a.Hk;
     if (MODE == 0) {
+      seg = (int)(item % a.nshare);
+      item /= a.nshare;
       blk = (int)(item / BH);
       const int bh = (int)(item % BH);
       b = bh / a.Hk;
@@ -86,6 +90,13 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (a.window > 0) {
         tb_lo = blk * a.BS;
         tb_hi = min(a.T, blk * a.BS + a.BS - 1 + a.window);
+      }
+      if (a.nshare > 1) {   // this CTA's share of both streams
+        const int n0 = ta_hi - ta_lo, n1 = tb_hi - tb_lo, a0 = ta_lo, b0 = tb_lo;
+        ta_lo = a0 + (int)((long long)n0 * seg / a.nshare);
+        ta_hi = a0 + (int)((long long)n0 * (seg + 1) / a.nshare);
+        tb_lo = b0 + (int)((long long)n1 * seg / a.nshare);
+        tb_hi = b0 + (int)((long long)n1 * (seg + 1) / a.nshare);
       }
     } else {
       seg = (int)(item % a.nseg);
@@ -253,7 +264,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int kp = kp0 + hrow * 8;
     if (kp >= a.Lk) continue;
     const long long off = (((long long)b * a.Lk + kp) * a.Hk + hk) * D + 2 * tq;
-    if (MODE == 0) {
+    if (MODE == 0 && a.nshare == 1) {
 #pragma unroll
       for (int i = 0; i < D / 8; ++i) {
         *reinterpret_cast<__nv_bfloat162*>(a.dk + off + i * 8) =
@@ -264,7 +275,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     } else {
       const long long N = (long long)a.B * a.Lk * a.Hk * D;
       float* pk = a.part + (long long)seg * N + off;
-      float* pv = a.part + ((long long)a.nseg + seg) * N + off;
+      float* pv = a.part + ((long long)(MODE == 0 ? a.nshare : a.nseg) + seg) * N + off;
 #pragma unroll
       for (int i = 0; i < D / 8; ++i) {
         *reinterpret_cast<float2*>(pk + i * 8) = make_float2(dk[i][2 * hrow] * a.scale, dk[i][2 * hrow + 1] * a.scale);
@@ -303,7 +314,7 @@ int launch(const KvArgs& a, cudaStream_t s) {
   if (e != cudaSuccess) return (int)e;
   long long grid;
   if (MODE == 0)
-    grid = (long long)a.B * a.Hk * ((a.T + a.BS - 1) / a.BS);
+    grid = (long long)a.B * a.Hk * ((a.T + a.BS - 1) / a.BS) * a.nshare;
   else
     grid = (long long)a.B * a.Hk * ((a.Lk + 63) / 64) * a.nseg;
   if (grid <= 0) return 0;

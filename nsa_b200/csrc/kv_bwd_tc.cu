@@ -124,6 +124,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     long long item = blockIdx.x;
     const int BH = a.B * a.Hk;
     if (MODE == 0) {
+      seg = (int)(item % a.nshare);
+      item /= a.nshare;
       // (batch, kv head)-major: the CTAs resident at one time share one 16-head group's Q and dO rows (67 MB at
       // T = 8192), which then stay in L2; block-major order made every gather a DRAM access
       const int NB = (a.T + 63) / 64;
@@ -140,6 +142,15 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (a.window > 0) {
         st.tb_lo = max(blk * 64, a.q0);
         st.nB = max(0, min(a.q0 + a.Tq, blk * 64 + 63 + a.window) - st.tb_lo);
+      }
+      if (a.nshare > 1) {   // this CTA's share of both streams, in whole batches
+        const int ba = (st.nA + kTokB - 1) / kTokB, bb = (st.nB + kTokB - 1) / kTokB;
+        const int a0 = ba * seg / a.nshare * kTokB, a1 = min(st.nA, ba * (seg + 1) / a.nshare * kTokB);
+        const int b0 = bb * seg / a.nshare * kTokB, b1 = min(st.nB, bb * (seg + 1) / a.nshare * kTokB);
+        st.ta_lo += a0;
+        st.nA = a1 - a0;
+        st.tb_lo += b0;
+        st.nB = b1 - b0;
       }
     } else {
       seg = (int)(item % a.nseg);
@@ -538,11 +549,11 @@ __global__ void __launch_bounds__(kThreads, 1)
           const int kp = key0 + c * 16 + e;
           if (!ok || kp >= a.Lk) continue;
           const long long off = (((long long)b * a.Lk + kp) * a.Hk + hk) * D + dch;
-          if (MODE == 0) {
+          if (MODE == 0 && a.nshare == 1) {
             (which ? a.dk : a.dv)[off] = __float2bfloat16(vals[e] * mul);
           } else {
             const long long N = (long long)a.B * a.Lk * a.Hk * D;
-            a.part[((long long)(which ? 0 : a.nseg) + seg) * N + off] = vals[e] * mul;
+            a.part[((long long)(which ? 0 : MODE == 0 ? a.nshare : a.nseg) + seg) * N + off] = vals[e] * mul;
           }
         }
       }
@@ -583,7 +594,7 @@ int launch(const KvArgs& a, cudaStream_t s) {
   if (e != cudaSuccess) return (int)e;
   long long grid;
   if (MODE == 0)
-    grid = (long long)a.B * a.Hk * ((a.T + 63) / 64);
+    grid = (long long)a.B * a.Hk * ((a.T + 63) / 64) * a.nshare;
   else
     grid = (long long)a.B * a.Hk * ((a.Lk + 63) / 64) * a.nseg;
   if (grid <= 0) return 0;

@@ -46,22 +46,34 @@ class ParallelNSAFunction(torch.autograd.Function):
         o_swa = torch.empty_like(q) if window_size > 0 else None
         lse_swa = torch.empty_like(lse_slc) if window_size > 0 else None
         P, i64 = _lib.ptr, 1 if idx.dtype == torch.int64 else 0
+        L, S_, need = _lib.lib(), _lib.stream(), any(ctx.needs_input_grad)
+        covers, indices = _lib.sel_fwd_kv_covers(Hq, Hkv, D, S, block_size), []
         for a, b in (seqs or [(0, T)]):
-            sl = slice(a, b)
-            fws_bytes = _lib.sel_swa_fwd_workspace_bytes(B, b - a, b - a, Hq, Hkv, D, S, block_size)
-            fws = torch.empty(fws_bytes, dtype=torch.uint8, device=q.device) if fws_bytes else None
-            _lib.check(_lib.lib().nsa_sel_swa_fwd_ws(
-                P(q[:, sl]), P(k[:, sl]), P(v[:, sl]), P(idx[:, sl]), i64, P(counts[:, sl]) if counts is not None else None,
+            sl, n = slice(a, b), b - a
+            counts_p = P(counts[:, sl]) if counts is not None else None
+            ix = fws = None
+            fws_bytes = 0
+            if covers or (need and _lib.SEL_DQ_FROM_KV):
+                # one reverse index for the forward and the backward
+                ix = torch.empty(L.nsa_sel_index_bytes(B, n, n, Hkv, S, block_size), dtype=torch.uint8, device=q.device)
+                _lib.check(L.nsa_sel_index(P(idx[:, sl]), i64, counts_p, P(ix), ix.numel(), B, n, n, 0, Hkv, S, block_size, S_),
+                           "nsa_sel_index")
+            if covers:
+                fws_bytes = L.nsa_sel_swa_fwd_ix_workspace_bytes(B, n, n, Hq, Hkv, D, S, block_size)
+                fws = torch.empty(fws_bytes, dtype=torch.uint8, device=q.device)
+            indices.append(ix if need and _lib.SEL_DQ_FROM_KV else None)
+            _lib.check(L.nsa_sel_swa_fwd_ix(
+                P(q[:, sl]), P(k[:, sl]), P(v[:, sl]), P(idx[:, sl]), i64, counts_p, P(ix),
                 P(o_slc[:, sl]), P(lse_slc[:, sl]), P(o_swa[:, sl]) if o_swa is not None else None,
                 P(lse_swa[:, sl]) if lse_swa is not None else None, None, None, None, None, None, P(fws), fws_bytes,
                 B, b - a, Hq, Hkv, D, S, block_size, window_size, float(scale), b - a, 0, _lib.stream()), "nsa_sel_swa_fwd")
-        ctx.save_for_backward(q, k, v, o_slc, lse_slc, o_swa, lse_swa, idx, counts)
+        ctx.save_for_backward(q, k, v, o_slc, lse_slc, o_swa, lse_swa, idx, counts, *indices)
         ctx.meta = (block_size, window_size, float(scale), seqs)
         return o_slc, o_swa
 
     @staticmethod
     def backward(ctx, do_slc, do_swa):
-        q, k, v, o_slc, lse_slc, o_swa, lse_swa, idx, counts = ctx.saved_tensors
+        q, k, v, o_slc, lse_slc, o_swa, lse_swa, idx, counts, *indices = ctx.saved_tensors
         block_size, window_size, scale, seqs = ctx.meta
         B, T, Hq, D = q.shape
         Hkv, S = k.shape[2], idx.shape[-1]
@@ -85,16 +97,17 @@ class ParallelNSAFunction(torch.autograd.Function):
         dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
         P, i64 = _lib.ptr, 1 if idx.dtype == torch.int64 else 0
         opt = lambda t, sl: P(t[:, sl]) if t is not None else None
-        for a, b in (seqs or [(0, T)]):
+        for (a, b), ix in zip(seqs or [(0, T)], indices):
             sl = slice(a, b)
-            ws_bytes = _lib.sel_swa_bwd_workspace_bytes(B, b - a, b - a, Hq, Hkv, D, S, block_size)
+            size = L.nsa_sel_swa_bwd_ix_workspace_bytes if ix is not None else _lib.sel_swa_bwd_workspace_bytes
+            ws_bytes = size(B, b - a, b - a, Hq, Hkv, D, S, block_size)
             ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
-            _lib.check(L.nsa_sel_swa_bwd(
-                P(q[:, sl]), P(k[:, sl]), P(v[:, sl]), P(idx[:, sl]), i64, opt(counts, sl),
+            _lib.check(L.nsa_sel_swa_bwd_ix(
+                P(q[:, sl]), P(k[:, sl]), P(v[:, sl]), P(idx[:, sl]), i64, opt(counts, sl), P(ix),
                 P(do_slc[:, sl]), P(lse_slc[:, sl]), P(delta_slc[:, sl]), None,
                 opt(do_swa, sl), opt(lse_swa, sl), opt(delta_swa, sl), None,
                 P(dq[:, sl]), 0, P(dk[:, sl]), P(dv[:, sl]), P(ws), ws_bytes,
-                B, b - a, Hq, Hkv, D, S, block_size, window_size, scale, _lib.stream()), "nsa_sel_swa_bwd")
+                B, b - a, Hq, Hkv, D, S, block_size, window_size, scale, b - a, 0, _lib.stream()), "nsa_sel_swa_bwd")
         return dq, dk, dv, None, None, None, None, None, None
 
 
