@@ -84,7 +84,7 @@ int nsa_device_status(void) {
   cudaError_t e = cudaDeviceSynchronize();
   if (e != cudaSuccess) return fail(1000 + (int)e, "cudaDeviceSynchronize: %s", cudaGetErrorString(e));
   int worst = 0, v = 0;
-  int (*fns[])(int*) = {sel_status, sel_block_status, dense_status, kv_status, compress_status, misc_status, compress_tc_status, compress_bwd_tc_status, kv_tc_status, dense_dq_tc_status, gather_probe_status, dense_tc2_status, decode_status, sel_fwd_kv_status};
+  int (*fns[])(int*) = {sel_status, sel_block_status, dense_status, kv_status, compress_status, misc_status, compress_tc_status, compress_bwd_tc_status, kv_tc_status, dense_dq_tc_status, gather_probe_status, dense_tc2_status, score_tc_status, decode_status, sel_fwd_kv_status};
   for (auto f : fns) {
     v = 0;
     const int rc = f(&v);
@@ -311,11 +311,21 @@ static int cmp_attn_fwd_impl(const void* q, const void* ck, const void* cv, void
     a.sel_idx = sel_idx; a.sel_scores = sel_scores;
   }
   if (dense_fwd_tc_supported(a, D)) {
+    if (n_sel > 0) {   // the selection has its own kernel
+      ScoreArgs c = {};
+      c.q = a.q; c.ck = a.k; c.sel_idx = sel_idx; c.sel_scores = sel_scores;
+      c.seq.B = B; c.seq.Tq = Tq; c.seq.q0 = q0; c.seq.Tc = Tc;
+      c.Hq = Hq; c.Hk = Hk; c.n_sel = n_sel; c.Tc_max = Tc; c.score_mode = score_mode; c.cblock = block;
+      c.cstride = stride; c.scale = scale;
+      rc = launch_score_tc(c, (cudaStream_t)stream);
+      if (rc) return rc;
+      a.n_sel = 0;
+    }
     if (gate) {
       a.gate_w = (const bf16*)gate->w; a.gate_b = (const bf16*)gate->b;
       for (int i = 0; i < 3; ++i) a.g_out[i] = (bf16*)gate->g[i];
     }
-    return launch_dense_fwd2_tc(a, (cudaStream_t)stream);
+    return launch_dense_fwd2_tc(a, D, (cudaStream_t)stream);
   }
   if (sharded) return fail(-11, "query shards need head_dim 128 and the default pooling geometry");
   if (score_mode == 1 && n_sel > 0) return fail(-16, "causal selection scores need head_dim 128 and the default pooling geometry");
@@ -530,7 +540,7 @@ static int sel_swa_fwd_impl(const void* q, const void* k, const void* v, const v
     a.mode = 0; a.q = (const bf16*)q; a.k = (const bf16*)k; a.v = (const bf16*)v; a.o = (bf16*)o_swa; a.lse = lse_swa;
     a.B = B; a.T = T; a.Tq = Tq; a.q0 = q0; a.Lk = T; a.Hq = Hq; a.Hk = Hkv; a.window = window; a.scale = scale;
     if (!dense_fwd_tc_supported(a, D) && sharded) return fail(-11, "query shards need head_dim 128");
-    rc = dense_fwd_tc_supported(a, D) ? launch_dense_fwd2_tc(a, s) : launch_dense_fwd(a, D, s);
+    rc = dense_fwd_tc_supported(a, D) ? launch_dense_fwd2_tc(a, D, s) : launch_dense_fwd(a, D, s);
     if (rc) return rc;
   }
   if (o) {

@@ -243,12 +243,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int cod
     }
   }
 }
-// The same with a CTA-wide abort flag in shared memory: once any wait of the CTA has given up, every later wait
-// returns false at once, so roles that must keep meeting at named barriers can run their loops to the end without
+// The same with a CTA-wide abort flag in shared memory: once any wait of the CTA has given up, every later wait whose phase
+// is not complete returns false at once, so roles that must keep meeting at named barriers can run their loops to the end without
 // waiting (their results are discarded) instead of leaving a partner stuck at a barrier.
 __device__ __forceinline__ bool mbar_wait_abortable(uint32_t bar, uint32_t parity, int code, volatile int* abort_flag) {
-  if (*abort_flag) return false;
   if (mbar_try(bar, parity)) return true;
+  if (*abort_flag) return false;
   const uint64_t t0 = global_timer_ns();
   for (;;) {
 #pragma unroll 1

@@ -8,6 +8,79 @@
 
 namespace nsa {
 
+// ---- the sequences of a call ------------------------------------------------------------------
+// Equal lengths (cu null): B sequences, Tq query rows each (the tokens q0 .. q0+Tq-1 of a sequence; tensors hold Tq rows per
+// batch) and Tc compressed positions.  Packed (cu, cu_c device [B+1]): sequence s is the tokens cu[s] .. cu[s+1]-1 and the
+// compressed rows cu_c[s] .. cu_c[s+1]-1 of one packed tensor.
+struct Seqs {
+  const int *cu, *cu_c;
+  int B, Tq, q0, Tc;
+  long long total, total_c;   // packed: tokens and compressed rows in all
+};
+// Tiles of G tokens never cross a sequence's end.  Packed: sequence s owns the tile indices from cu[s] / G + s on, never
+// fewer than it has tiles, so no table is needed (an index past its last tile has t0 >= Tq).
+inline int seq_tiles(const Seqs& q, int G) { return q.cu ? (int)(q.total / G) + q.B : q.B * ((q.Tq + G - 1) / G); }
+inline long long seq_rows(const Seqs& q) { return q.cu ? q.total : (long long)q.B * q.Tq; }
+#ifdef __CUDACC__
+struct SeqTile {
+  long long row0;   // first query row (token) of the sequence
+  long long c0;     // row coordinate of its first compressed position (with batch coordinate b)
+  int b, t0, Tq, Tc;
+};
+__device__ __forceinline__ int seq_tiles_dev(const Seqs& q, int G) { return q.cu ? (int)(q.total / G) + q.B : q.B * ((q.Tq + G - 1) / G); }
+__device__ __forceinline__ SeqTile seq_tile(const Seqs& q, int G, int t) {
+  SeqTile r;
+  if (!q.cu) {
+    const int per = (q.Tq + G - 1) / G;
+    r.b = t / per;
+    r.t0 = (t - r.b * per) * G;
+    r.row0 = (long long)r.b * q.Tq;
+    r.c0 = 0;
+    r.Tq = q.Tq;
+    r.Tc = q.Tc;
+    return r;
+  }
+  int lo = 0, hi = q.B - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (q.cu[mid] / G + mid <= t) lo = mid; else hi = mid - 1;
+  }
+  const int c = q.cu[lo];
+  r.b = 0;
+  r.t0 = (t - (c / G + lo)) * G;
+  r.row0 = c;
+  r.c0 = q.cu_c ? q.cu_c[lo] : 0;
+  r.Tq = q.cu[lo + 1] - c;
+  r.Tc = q.cu_c ? q.cu_c[lo + 1] - (int)r.c0 : 0;
+  return r;
+}
+// avg_pool1d(kernel 5, stride 4, no padding, ceil_mode) output length, as nsa_pool_out_len computes it
+__device__ __forceinline__ int pool_len_54(int n) {
+  if (n <= 0) return 0;
+  const int num = n - 5;
+  int out = (num >= 0 ? (num + 3) / 4 : -((-num) / 4)) + 1;
+  if ((out - 1) * 4 >= n) --out;
+  return out < 0 ? 0 : out;
+}
+#endif
+
+// ---- block selection (score_tc.cu; head_dim 128, 5/4/0 pooling) --------------------------------
+struct ScoreArgs {
+  const bf16* q;       // [tok,Hq,D]
+  const bf16* ck;      // compressed keys
+  int* sel_idx;        // [tok,Hq/16,n_sel]
+  float* sel_scores;   // optional dump of the pooled scores [B,Hq/16,Tq,n_pool] (equal lengths), or null
+  Seqs seq;
+  int Hq, Hk, n_sel;
+  int Tc_max;          // compressed positions of the longest sequence
+  int score_mode;      // 0: soft-max of the unscaled, unmasked q.ck over all compressed keys; 1: scaled, over the visible ones
+  int cblock, cstride;
+  float scale;         // score_mode 1
+};
+bool score_tc_supported(int head_dim, int pool_k, int pool_s, int pool_p, int n_pool);
+int launch_score_tc(const ScoreArgs& a, cudaStream_t s);
+int score_tc_status(int* out);
+
 // ---- selected-block attention, query-major (forward and dQ) --------------------------------
 struct SelArgs {
   const bf16* q;       // [B,T,Hq,D]
@@ -74,6 +147,7 @@ struct DenseArgs {
   // optional, dQ kernels (tcgen05): the row pre-pass of the backward folded in.  With pre_o[0] set the kernel computes
   // rowsum(o * dO) itself for its own branch ([0]) and, if given, a second branch ([1]) whose dQ kernel runs later:
   // pre_delta[x] = gate_x * rowsum (fp32, also what this kernel uses as delta), pre_dgate[x] = rowsum (bf16, gate gradient)
+  Seqs seq;            // tcgen05 forward: packed sequences (seq.cu null: B, Tq, q0, Lk above)
   const bf16* pre_o[2];
   const bf16* pre_gate[2];
   float* pre_delta[2];
@@ -82,10 +156,10 @@ struct DenseArgs {
 int launch_dense_fwd(const DenseArgs& a, int D, cudaStream_t s);
 int launch_dense_dq(const DenseArgs& a, int D, cudaStream_t s);
 int dense_status(int* out);
-// tcgen05 forward for head_dim 128 (and, for selection, the 5/4/0 pooling of the default block sizes)
+// tcgen05 forward (with a selection only where score_tc.cu covers it)
 bool dense_fwd_tc_supported(const DenseArgs& a, int head_dim);
-// two query tiles per CTA, P kept in tensor memory (dense_fwd2_tc.cu)
-int launch_dense_fwd2_tc(const DenseArgs& a, cudaStream_t s);
+// two query tiles per CTA (dense_fwd2_tc.cu)
+int launch_dense_fwd2_tc(const DenseArgs& a, int head_dim, cudaStream_t s);
 int dense_tc2_status(int* out);
 int launch_dense_dq_tc(const DenseArgs& a, cudaStream_t s);
 int dense_dq_tc_status(int* out);
