@@ -399,7 +399,7 @@ static int cmp_attn_bwd_impl(const void* q, const void* ck, const void* cv, cons
     a.accumulate = accumulate_dq; a.B = B; a.T = T; a.Tq = Tq; a.q0 = q0; a.Lk = Tc; a.Hq = Hq; a.Hk = Hk; a.cblock = block;
     a.cstride = stride; a.causal = causal; a.scale = scale;
     if (D != 128 && sharded) return fail(-11, "query shards need head_dim 128");
-      rc = (D == 128) ? launch_dense_dq_tc(a, s) : launch_dense_dq(a, D, s);
+    rc = launch_dense_dq_tc(a, D, s);
     if (rc) return rc;
   }
   if (dck || dcv) {
@@ -539,8 +539,7 @@ static int sel_swa_fwd_impl(const void* q, const void* k, const void* v, const v
     DenseArgs a = {};
     a.mode = 0; a.q = (const bf16*)q; a.k = (const bf16*)k; a.v = (const bf16*)v; a.o = (bf16*)o_swa; a.lse = lse_swa;
     a.B = B; a.T = T; a.Tq = Tq; a.q0 = q0; a.Lk = T; a.Hq = Hq; a.Hk = Hkv; a.window = window; a.scale = scale;
-    if (!dense_fwd_tc_supported(a, D) && sharded) return fail(-11, "query shards need head_dim 128");
-    rc = dense_fwd_tc_supported(a, D) ? launch_dense_fwd2_tc(a, D, s) : launch_dense_fwd(a, D, s);
+    rc = launch_dense_fwd2_tc(a, D, s);
     if (rc) return rc;
   }
   if (o) {
@@ -680,7 +679,7 @@ static int sel_swa_bwd_impl(const void* q, const void* k, const void* v, const v
         }
       }
       if (D != 128 && sharded) return fail(-11, "query shards need head_dim 128");
-      return (D == 128) ? launch_dense_dq_tc(a, s) : launch_dense_dq(a, D, s);
+      return launch_dense_dq_tc(a, D, s);
     };
     if (fold) {
       rc = run_swa();

@@ -144,24 +144,27 @@ struct DenseArgs {
   const bf16* gate_w;  // mode 1: [3,D] gate projection weight (rows: selected, window, compressed); writes g_out
   const bf16* gate_b;  // [3] or null
   bf16* g_out[3];      // [B,Tq,Hq] each
-  // optional, dQ kernels (tcgen05): the row pre-pass of the backward folded in.  With pre_o[0] set the kernel computes
+  // tcgen05 dQ, mode 0 with ck given: the compressed branch's dQ in the same pass (its own lse, delta, gate; the same dout)
+  const bf16 *ck, *cv;
+  const float *lse_c, *delta_c;
+  const bf16* gate_c;
+  Seqs seq;            // tcgen05 kernels: packed sequences (seq.cu null: B, Tq, q0, Lk above)
+  // optional, tcgen05 dQ: the row pre-pass of the backward folded in.  With pre_o[0] set the kernel computes
   // rowsum(o * dO) itself for its own branch ([0]) and, if given, a second branch ([1]) whose dQ kernel runs later:
   // pre_delta[x] = gate_x * rowsum (fp32, also what this kernel uses as delta), pre_dgate[x] = rowsum (bf16, gate gradient)
-  Seqs seq;            // tcgen05 forward: packed sequences (seq.cu null: B, Tq, q0, Lk above)
   const bf16* pre_o[2];
   const bf16* pre_gate[2];
   float* pre_delta[2];
   bf16* pre_dgate[2];
 };
 int launch_dense_fwd(const DenseArgs& a, int D, cudaStream_t s);
-int launch_dense_dq(const DenseArgs& a, int D, cudaStream_t s);
 int dense_status(int* out);
 // tcgen05 forward (with a selection only where score_tc.cu covers it)
 bool dense_fwd_tc_supported(const DenseArgs& a, int head_dim);
 // two query tiles per CTA (dense_fwd2_tc.cu)
 int launch_dense_fwd2_tc(const DenseArgs& a, int head_dim, cudaStream_t s);
 int dense_tc2_status(int* out);
-int launch_dense_dq_tc(const DenseArgs& a, cudaStream_t s);
+int launch_dense_dq_tc(const DenseArgs& a, int head_dim, cudaStream_t s);
 int dense_dq_tc_status(int* out);
 
 // ---- key/value-major backward (dK,dV of selected + sliding window; dCK,dCV of compressed) ---
