@@ -161,7 +161,7 @@ size_t nsa_sel_swa_bwd_workspace_bytes_dq(int B, int T, int Tq, int Hq, int Hkv,
  * workspaces of their own (without the index; the backward's holds partial sums that let the tokens of a key block be
  * spread over several CTAs when there are fewer blocks than SMs).  Tq = T, q0 = 0 when not sharded. */
 size_t nsa_sel_swa_fwd_ix_workspace_bytes(int B, int T, int Tq, int Hq, int Hkv, int D, int S, int BS);
-size_t nsa_sel_swa_bwd_ix_workspace_bytes(int B, int T, int Tq, int Hq, int Hkv, int D, int S, int BS);
+size_t nsa_sel_swa_bwd_ix_workspace_bytes(int B, int T, int Tq, int Hq, int Hkv, int D, int S, int BS, int window);
 size_t nsa_sel_index_bytes(int B, int T, int Tq, int Hkv, int S, int BS);
 int nsa_sel_index(const void* idx, int idx64, const int32_t* counts, void* index, size_t index_bytes, int B, int T, int Tq,
                   int q0, int Hkv, int S, int BS, void* stream);
@@ -174,6 +174,15 @@ int nsa_sel_swa_bwd_ix(const void* q, const void* k, const void* v, const void* 
                        const void* gate_slc, const void* dout_swa, const float* lse_swa, const float* delta_swa,
                        const void* gate_swa, void* dq, int accumulate_dq, void* dk, void* dv, void* ws, size_t ws_bytes, int B,
                        int T, int Hq, int Hkv, int D, int S, int BS, int window, float scale, int Tq, int q0, void* stream);
+/* The backward of all three branches for one upstream gradient (nsa_sel_swa_bwd_ix and nsa_cmp_attn_bwd with the gates of the
+ * module's sum; delta_x = g_x * rowsum(o_x * dout)): the window's and the compressed branch's dQ are formed in one pass. */
+size_t nsa_attn_bwd_ix_workspace_bytes(int B, int T, int Tc, int Hq, int Hkv, int D, int S, int BS, int window);
+int nsa_attn_bwd_ix(const void* q, const void* k, const void* v, const void* ck, const void* cv, const void* idx, int idx64,
+                    const int32_t* counts, const void* index, const void* dout, const float* lse_slc, const float* lse_swa,
+                    const float* lse_cmp, const float* delta_slc, const float* delta_swa, const float* delta_cmp,
+                    const void* g_slc, const void* g_swa, const void* g_cmp, void* dq, void* dk, void* dv, void* dck, void* dcv,
+                    void* ws, size_t ws_bytes, int B, int T, int Tc, int Hq, int Hkv, int D, int S, int BS, int window, int block,
+                    int stride, int causal, float scale, void* stream);
 
 /* Measurement aid, no counterpart in the reference: the K/V block gather of nsa_sel_swa_fwd's selected branch (same
  * items, same order, same TMA boxes of [BS keys x D]) with no arithmetic behind it, every SM keeping all of its shared

@@ -3,6 +3,8 @@
 #include <stdarg.h>
 #include <stdio.h>
 
+#include <algorithm>
+
 #include "../../include/nsa_b200.h"
 #include "kernels.h"
 #include "tmap.h"
@@ -41,23 +43,7 @@ static int check_bs(const char* who, int BS) {
   return 0;
 }
 
-// Token segments of the compressed branch's key-major backward: at least one per 1024 tokens (16 at most), more while the
-// (batch, head, key tile) CTAs alone do not give every SM about four pieces of work, at least 64 tokens each.  `tiles` =
-// B * Hk * ceil(Tc / 64).
-static int cmp_segments(int T, long long tiles, int* seg_len) {
-  long long nseg = (T + 1023) / 1024;
-  if (nseg > 16) nseg = 16;
-  const long long want = (4LL * num_sms() + tiles - 1) / (tiles > 0 ? tiles : 1);
-  if (nseg < want) nseg = want;
-  if (nseg > (T + 63) / 64) nseg = (T + 63) / 64;
-  if (nseg < 1) nseg = 1;
-  int sl = (int)((T + nseg - 1) / nseg);
-  sl = (sl + 63) / 64 * 64;
-  *seg_len = sl;
-  return (T + sl - 1) / sl;
-}
-
-// Shares of a key block's token stream in the key-major backward of the selected and window branches: one CTA per block
+// Shares of a key block's token stream in the key-major backward of the selected branch: one CTA per block
 // when the blocks fill the GPU four times over (the first blocks are visited most, so one wave is not enough), else enough
 // shares for about that many CTAs (at most 16; a share then still has some dozens of tokens).  With more than one share the
 // CTAs leave fp32 partials that a second kernel adds in order.
@@ -84,7 +70,7 @@ int nsa_device_status(void) {
   cudaError_t e = cudaDeviceSynchronize();
   if (e != cudaSuccess) return fail(1000 + (int)e, "cudaDeviceSynchronize: %s", cudaGetErrorString(e));
   int worst = 0, v = 0;
-  int (*fns[])(int*) = {sel_status, sel_block_status, dense_status, kv_status, compress_status, misc_status, compress_tc_status, compress_bwd_tc_status, kv_tc_status, dense_dq_tc_status, gather_probe_status, dense_tc2_status, score_tc_status, decode_status, sel_fwd_kv_status};
+  int (*fns[])(int*) = {sel_status, sel_block_status, dense_status, kv_status, compress_status, misc_status, compress_tc_status, compress_bwd_tc_status, kv_tc_status, dense_kv_tc_status, dense_dq_tc_status, gather_probe_status, dense_tc2_status, score_tc_status, decode_status, sel_fwd_kv_status};
   for (auto f : fns) {
     v = 0;
     const int rc = f(&v);
@@ -357,9 +343,25 @@ int nsa_cmp_attn_fwd_gated(const void* q, const void* ck, const void* cv, void* 
 }
 
 size_t nsa_cmp_attn_bwd_workspace_bytes(int B, int T, int Tc, int Hk, int D) {
-  int sl;
-  const int nseg = cmp_segments(T, (long long)B * Hk * ((Tc + 63) / 64), &sl);
-  return (size_t)2 * nseg * B * Tc * Hk * D * sizeof(float);
+  if (T <= 0) return 0;
+  const int rows = dense_kv_segment_rows(B, T, Tc, Hk);
+  return (size_t)2 * ((T + rows - 1) / rows) * B * Tc * Hk * D * sizeof(float);
+}
+
+// dCK, dCV: one launch over segments of the queries and the sum of their fp32 slabs (the workspace), or straight to bf16 when
+// one segment does.
+static int cmp_dkv(const void* q, const void* ck, const void* cv, const float* lse, const void* dout, const float* delta,
+                   const void* gate, void* dck, void* dcv, void* ws, int B, int T, int Tc, int Hq, int Hk, int D, int block,
+                   int stride, int causal, float scale, int Tq, int q0, cudaStream_t s) {
+  DenseKvArgs a = {};
+  a.mode = 1; a.q = (const bf16*)q; a.k = (const bf16*)ck; a.v = (const bf16*)cv; a.dout = (const bf16*)dout;
+  a.lse = lse; a.delta = delta; a.gate = (const bf16*)gate; a.dk = (bf16*)dck; a.dv = (bf16*)dcv;
+  a.seg_len = dense_kv_segment_rows(B, T, Tc, Hk);
+  a.nslab = a.slabs = (Tq + a.seg_len - 1) / a.seg_len;
+  a.part = a.nslab > 1 ? (float*)ws : nullptr;
+  a.Hq = Hq; a.Hk = Hk; a.Lk = Tc; a.cblock = block; a.cstride = stride; a.causal = causal; a.scale = scale;
+  a.seq.B = B; a.seq.Tq = Tq; a.seq.q0 = q0; a.seq.Tc = Tc;
+  return launch_dense_kv_tc(a, D, s);
 }
 
 struct PreCmp {   // row pre-pass folded into the compressed branch's dQ kernel
@@ -406,20 +408,8 @@ static int cmp_attn_bwd_impl(const void* q, const void* ck, const void* cv, cons
     if (!dck || !dcv) return fail(-1, "nsa_cmp_attn_bwd: dck and dcv must be given together");
     if (!ws || ws_bytes < nsa_cmp_attn_bwd_workspace_bytes(B, T, Tc, Hk, D))
       return fail(-6, "nsa_cmp_attn_bwd: workspace too small");
-    KvArgs a = {};
-    a.mode = 1; a.q = (const bf16*)q; a.k = (const bf16*)ck; a.v = (const bf16*)cv;
-    a.dout_a = (const bf16*)dout; a.lse_a = lse; a.delta_a = delta; a.gate_a = (const bf16*)gate;
-    a.part = (float*)ws; a.nseg = cmp_segments(Tq, (long long)B * Hk * ((Tc + 63) / 64), &a.seg_len);
-    a.B = B; a.T = T; a.Tq = Tq; a.q0 = q0; a.Lk = Tc; a.Hq = Hq; a.Hk = Hk; a.BS = 64; a.cblock = block; a.cstride = stride;
-    a.causal = causal; a.scale = scale;
     if (D != 128 && sharded) return fail(-11, "query shards need head_dim 128");
-    rc = (D == 128) ? launch_kv_bwd_tc(a, s) : launch_kv_bwd(a, D, s);
-    if (rc) return rc;
-    const long long N = (long long)B * Tc * Hk * D;
-    rc = launch_reduce_segments(a.part, (bf16*)dck, a.nseg, N, q0, Tq, Tc, Hk, D, a.seg_len, block, stride, causal, s);
-    if (rc) return rc;
-    rc = launch_reduce_segments(a.part + (long long)a.nseg * N, (bf16*)dcv, a.nseg, N, q0, Tq, Tc, Hk, D, a.seg_len, block,
-                                stride, causal, s);
+    rc = cmp_dkv(q, ck, cv, lse, dout, delta, gate, dck, dcv, ws, B, T, Tc, Hq, Hk, D, block, stride, causal, scale, Tq, q0, s);
     if (rc) return rc;
   }
   return 0;
@@ -586,32 +576,45 @@ int nsa_cmp_attn_bwd_fused(const void* q, const void* ck, const void* cv, const 
   return cmp_attn_bwd_impl(q, ck, cv, lse, dout, delta, gate, dq, accumulate_dq, dck, dcv, ws, ws_bytes, B, T, Tc, Hq, Hk, D, block, stride, causal, scale, Tq, q0, stream, &pre);
 }
 
-size_t nsa_sel_swa_bwd_workspace_bytes(int B, int T, int Hkv, int S, int BS) {
-  if (BS <= 0) return 0;
-  const size_t NB = (size_t)(T + BS - 1) / BS;
-  const size_t bh = (size_t)B * Hkv;
+// fp32 dK, dV of `slabs` slabs
+static size_t kv_slab_bytes(int slabs, int B, int T, int Hkv, int D) { return (size_t)2 * slabs * B * T * Hkv * D * sizeof(float); }
+static size_t rev_base_bytes(int B, int T, int Hkv, int S, int BS) {
+  const size_t NB = (size_t)(T + BS - 1) / BS, bh = (size_t)B * Hkv;
   return align_up(bh * NB * NB * 4, 256) + align_up(bh * (NB + 1) * 4, 256) + align_up(bh * (size_t)T * S * 4, 256);
 }
 
+// The reverse index, then the window's dK, dV (fp32, sized for the larger head_dim).
+size_t nsa_sel_swa_bwd_workspace_bytes(int B, int T, int Hkv, int S, int BS) {
+  return BS <= 0 ? 0 : rev_base_bytes(B, T, Hkv, S, BS) + kv_slab_bytes(1, B, T, Hkv, 128);
+}
+
 // Behind the reverse index: one [16 x D] bf16 tile per (list position, 16-head sub-group) for the selected branch's dQ as
-// per-visit partials (tcgen05 kernel only), then the fp32 dK, dV partials of the shares.
+// per-visit partials (tcgen05 kernel only), then the fp32 dK, dV slabs of the shares and of the window.
 static bool dq_from_kv_covers(int D, int S, int BS) { return D == 128 && BS == 64 && S <= 32; }
 static size_t sel_dq_tile_bytes(int B, int Tq, int Hq, int D, int S, int BS) {
   return dq_from_kv_covers(D, S, BS) ? align_up((size_t)B * Tq * Hq * S * D * 2, 256) : 0;
 }
-static size_t kv_share_bytes(int B, int T, int Hkv, int D, int BS) {
-  const int ns = kv_shares((long long)B * Hkv * ((T + BS - 1) / BS));
-  return ns > 1 ? (size_t)2 * ns * B * T * Hkv * D * sizeof(float) : 0;
+struct KvSlabs {
+  int nshare, nwin;                                             // shares of the selected lists, parts of the window
+  int slabs() const { return (nshare > 1 ? nshare : 0) + nwin; }
+};
+static KvSlabs kv_slabs(int B, int T, int Hkv, int BS, int window) {
+  return {kv_shares((long long)B * Hkv * ((T + BS - 1) / BS)), window > 0 ? dense_kv_window_slabs(B, T, Hkv, window) : 0};
 }
 
 size_t nsa_sel_swa_bwd_workspace_bytes_dq(int B, int T, int Tq, int Hq, int Hkv, int D, int S, int BS) {
   if (BS <= 0 || Hkv <= 0) return 0;
-  return nsa_sel_index_bytes(B, T, Tq, Hkv, S, BS) + align_up((size_t)B * Tq * Hq * S * D * 2, 256);
+  return nsa_sel_index_bytes(B, T, Tq, Hkv, S, BS) + align_up((size_t)B * Tq * Hq * S * D * 2, 256) + kv_slab_bytes(1, B, T, Hkv, 128);
 }
 
-size_t nsa_sel_swa_bwd_ix_workspace_bytes(int B, int T, int Tq, int Hq, int Hkv, int D, int S, int BS) {
+size_t nsa_sel_swa_bwd_ix_workspace_bytes(int B, int T, int Tq, int Hq, int Hkv, int D, int S, int BS, int window) {
   if (BS <= 0 || Hkv <= 0) return 0;
-  return sel_dq_tile_bytes(B, Tq, Hq, D, S, BS) + kv_share_bytes(B, T, Hkv, D, BS);
+  return sel_dq_tile_bytes(B, Tq, Hq, D, S, BS) + kv_slab_bytes(kv_slabs(B, T, Hkv, BS, window).slabs(), B, T, Hkv, D);
+}
+
+size_t nsa_attn_bwd_ix_workspace_bytes(int B, int T, int Tc, int Hq, int Hkv, int D, int S, int BS, int window) {
+  return std::max(nsa_sel_swa_bwd_ix_workspace_bytes(B, T, T, Hq, Hkv, D, S, BS, window),
+                  nsa_cmp_attn_bwd_workspace_bytes(B, T, Tc, Hkv, D));
 }
 
 struct PreSel {   // row pre-pass of the selected and window branches folded into the window's dQ kernel
@@ -619,12 +622,19 @@ struct PreSel {   // row pre-pass of the selected and window branches folded int
   void *dg_slc, *dg_swa;
 };
 
+struct CmpBwd {   // the compressed branch in the same call: its dQ shares the window's pass
+  const void *ck, *cv;
+  const float *lse, *delta;
+  const void* gate;
+  int Tc, block, stride, causal;
+};
+
 static int sel_swa_bwd_impl(const void* q, const void* k, const void* v, const void* idx, int idx64, const int32_t* counts,
                     const void* dout_slc, const float* lse_slc, const float* delta_slc, const void* gate_slc,
                     const void* dout_swa, const float* lse_swa, const float* delta_swa, const void* gate_swa, void* dq,
                     int accumulate_dq, void* dk, void* dv, void* ws, size_t ws_bytes, int B, int T, int Hq, int Hkv,
                     int D, int S, int BS, int window, float scale, int Tq, int q0, void* stream,
-                    const PreSel* pre = nullptr, const void* index = nullptr) {
+                    const PreSel* pre = nullptr, const void* index = nullptr, const CmpBwd* cmp = nullptr) {
   const bool sharded = (Tq != T) || (q0 != 0);
   if (Tq <= 0 || q0 < 0 || q0 + Tq > T) return fail(-12, "%s: query shard [%d, %d) is outside the sequence of %d tokens", "nsa_sel_swa_bwd", q0, q0 + Tq, T);
   (void)sharded;
@@ -642,7 +652,7 @@ static int sel_swa_bwd_impl(const void* q, const void* k, const void* v, const v
   // With the larger workspace of nsa_sel_swa_bwd_workspace_bytes_dq the selected branch's dQ is produced by the
   // kv-major backward (per-visit partial tiles + a slot-order reduction) instead of the query-major dQ kernel.
   // (A caller that hands over a reverse index gives the workspace behind it alone, with room for the shares.)
-  if (index && ws_bytes < nsa_sel_swa_bwd_ix_workspace_bytes(B, T, Tq, Hq, Hkv, D, S, BS))
+  if (index && ws_bytes < nsa_sel_swa_bwd_ix_workspace_bytes(B, T, Tq, Hq, Hkv, D, S, BS, has_swa ? window : 0))
     return fail(-6, "nsa_sel_swa_bwd_ix: workspace too small");
   const bool large_ws = index || (ws && ws_bytes >= nsa_sel_swa_bwd_workspace_bytes_dq(B, T, Tq, Hq, Hkv, D, S, BS));
   const bool dq_from_kv = dq && dk && has_slc && dq_from_kv_covers(D, S, BS) && large_ws;
@@ -665,11 +675,25 @@ static int sel_swa_bwd_impl(const void* q, const void* k, const void* v, const v
   }
   if (dq) {
     int acc = accumulate_dq;
-    auto run_swa = [&]() -> int {
+    if (has_swa || cmp) {   // first: with `fold` it also forms the deltas of both branches
+      if (D != 128 && sharded) return fail(-11, "query shards need head_dim 128");
       DenseArgs a = {};
-      a.mode = 0; a.q = (const bf16*)q; a.k = (const bf16*)k; a.v = (const bf16*)v; a.lse = const_cast<float*>(lse_swa);
-      a.dout = (const bf16*)dout_swa; a.delta = delta_swa; a.gate = (const bf16*)gate_swa; a.dq = (bf16*)dq;
-      a.accumulate = acc; a.B = B; a.T = T; a.Tq = Tq; a.q0 = q0; a.Lk = T; a.Hq = Hq; a.Hk = Hkv; a.window = window; a.scale = scale;
+      a.q = (const bf16*)q; a.dout = (const bf16*)(has_swa ? dout_swa : dout_slc); a.dq = (bf16*)dq; a.accumulate = acc;
+      a.B = B; a.T = T; a.Tq = Tq; a.q0 = q0; a.Lk = T; a.Hq = Hq; a.Hk = Hkv; a.scale = scale;
+      if (has_swa) {
+        a.mode = 0; a.k = (const bf16*)k; a.v = (const bf16*)v; a.lse = const_cast<float*>(lse_swa); a.delta = delta_swa;
+        a.gate = (const bf16*)gate_swa; a.window = window;
+      }
+      if (cmp) {
+        a.cblock = cmp->block; a.cstride = cmp->stride; a.causal = cmp->causal; a.seq.Tc = cmp->Tc;
+        if (has_swa) {
+          a.ck = (const bf16*)cmp->ck; a.cv = (const bf16*)cmp->cv; a.lse_c = cmp->lse; a.delta_c = cmp->delta;
+          a.gate_c = (const bf16*)cmp->gate;
+        } else {
+          a.mode = 1; a.k = (const bf16*)cmp->ck; a.v = (const bf16*)cmp->cv; a.lse = const_cast<float*>(cmp->lse);
+          a.delta = cmp->delta; a.gate = (const bf16*)cmp->gate; a.Lk = cmp->Tc;
+        }
+      }
       if (fold) {
         a.pre_o[0] = (const bf16*)pre->o_swa; a.pre_gate[0] = (const bf16*)gate_swa;
         a.pre_delta[0] = const_cast<float*>(delta_swa); a.pre_dgate[0] = (bf16*)pre->dg_swa;
@@ -678,23 +702,12 @@ static int sel_swa_bwd_impl(const void* q, const void* k, const void* v, const v
           a.pre_delta[1] = const_cast<float*>(delta_slc); a.pre_dgate[1] = (bf16*)pre->dg_slc;
         }
       }
-      if (D != 128 && sharded) return fail(-11, "query shards need head_dim 128");
-      return launch_dense_dq_tc(a, D, s);
-    };
-    if (fold) {
-      rc = run_swa();
+      rc = launch_dense_dq_tc(a, D, s);
       if (rc) return rc;
       acc = 1;
     }
-    if (has_slc && dq_from_kv) {
-      // nothing here: the reduction behind the kv-major kernel writes (or adds) the selected branch's dQ.  If the window
-      // kernel has not run yet it must not overwrite that: it runs now and the reduction accumulates.
-      if (has_swa && !fold) {
-        rc = run_swa();
-        if (rc) return rc;
-      }
-      dq_acc_for_reduce = (acc || has_swa) ? 1 : 0;
-    } else if (has_slc) {
+    dq_acc_for_reduce = acc;
+    if (has_slc && !dq_from_kv) {   // (else the reduction behind the key-major kernel adds the selected branch's dQ)
       SelArgs a = {};
       a.q = (const bf16*)q; a.k = (const bf16*)k; a.v = (const bf16*)v; a.idx = idx; a.idx64 = idx64; a.counts = counts;
       a.lse = const_cast<float*>(lse_slc); a.dout = (const bf16*)dout_slc; a.delta = delta_slc;
@@ -702,50 +715,62 @@ static int sel_swa_bwd_impl(const void* q, const void* k, const void* v, const v
       a.B = B; a.T = T; a.Tq = Tq; a.q0 = q0; a.Hq = Hq; a.Hkv = Hkv; a.S = S; a.BS = BS; a.scale = scale;
       rc = launch_sel_dq(a, D, s);
       if (rc) return rc;
-      acc = 1;
-    }
-    if (has_swa && !fold && !(has_slc && dq_from_kv)) {
-      rc = run_swa();
-      if (rc) return rc;
     }
   }
   if (dk || dv) {
     if (!dk || !dv) return fail(-1, "nsa_sel_swa_bwd: dk and dv must be given together");
-    KvArgs a = {};
-    a.mode = 0; a.q = (const bf16*)q; a.k = (const bf16*)k; a.v = (const bf16*)v;
-    a.B = B; a.T = T; a.Tq = Tq; a.q0 = q0; a.Lk = T; a.Hq = Hq; a.Hk = Hkv; a.BS = BS; a.window = has_swa ? window : 0; a.scale = scale;
-    a.dk = (bf16*)dk; a.dv = (bf16*)dv;
+    if (sharded && (D != 128 || (has_slc && BS != 64))) return fail(-11, "query shards need head_dim 128 and 64-key selection blocks");
+    // fp32 slabs behind everything else in the workspace (none for the window alone: it is rounded straight away).  Only a
+    // caller with a reverse index of its own has room for shares and for parts of the window.
+    KvSlabs n = {1, has_swa ? 1 : 0};
+    bf16* tiles = nullptr;
+    if (index) n = kv_slabs(B, T, Hkv, BS, has_swa ? window : 0);
     RevArgs r = {};
+    float* part = nullptr;
     if (has_slc) {
       if (!index && (!ws || ws_bytes < nsa_sel_swa_bwd_workspace_bytes(B, T, Hkv, S, BS)))
         return fail(-6, "nsa_sel_swa_bwd: workspace too small");
       const size_t nrev = rev_layout(index ? const_cast<void*>(index) : ws, idx, idx64, counts, B, T, Tq, q0, Hkv, S, BS, &r);
-      if (!index && !large_ws) r.inv = nullptr;   // the small workspace ends behind the token lists
-      if (dq_from_kv) a.dq_part = (bf16*)((char*)ws + (index ? 0 : nrev));
+      if (!index && !large_ws) r.inv = nullptr;   // the small workspace has the token lists only
+      char* p = (char*)ws + (index ? 0 : nrev);
+      if (dq_from_kv) tiles = (bf16*)p;
+      if (index)
+        part = (float*)(p + sel_dq_tile_bytes(B, Tq, Hq, D, S, BS));
+      else if (large_ws)
+        part = (float*)(p + align_up((size_t)B * Tq * Hq * S * D * 2, 256));
+      else
+        part = (float*)((char*)ws + rev_base_bytes(B, T, Hkv, S, BS));
       if (!index) {
         rc = launch_build_rev(r, s);
         if (rc) return rc;
       }
-      a.rev_ptr = r.rev_ptr; a.rev_tok = r.rev_tok; a.rev_cap = r.cap;
-      a.dout_a = (const bf16*)dout_slc; a.lse_a = lse_slc; a.delta_a = delta_slc; a.gate_a = (const bf16*)gate_slc;
     }
     if (has_swa) {
-      a.dout_b = (const bf16*)dout_swa; a.lse_b = lse_swa; a.delta_b = delta_swa; a.gate_b = (const bf16*)gate_swa;
-    }
-    if (!(D == 128 && BS == 64) && sharded) return fail(-11, "query shards need head_dim 128 and 64-key selection blocks");
-    a.nshare = 1;
-    if (index) {
-      a.nshare = kv_shares((long long)B * Hkv * ((T + BS - 1) / BS));
-      a.part = (float*)((char*)ws + sel_dq_tile_bytes(B, Tq, Hq, D, S, BS));
-    }
-    rc = (D == 128 && BS == 64) ? launch_kv_bwd_tc(a, s) : launch_kv_bwd(a, D, s);
-    if (rc) return rc;
-    if (a.nshare > 1) {
-      rc = launch_reduce_shares(a.part, a.dk, a.dv, a.nshare, (long long)B * T * Hkv * D, s);
+      DenseKvArgs a = {};
+      a.mode = 0; a.q = (const bf16*)q; a.k = (const bf16*)k; a.v = (const bf16*)v; a.dout = (const bf16*)dout_swa;
+      a.lse = lse_swa; a.delta = delta_swa; a.gate = (const bf16*)gate_swa; a.dk = (bf16*)dk; a.dv = (bf16*)dv;
+      a.part = part; a.nslab = part ? n.nwin : 1; a.slab0 = n.nshare > 1 ? n.nshare : 0; a.slabs = n.slabs();
+      a.Hq = Hq; a.Hk = Hkv; a.Lk = T; a.window = window; a.scale = scale;
+      a.seq.B = B; a.seq.Tq = Tq; a.seq.q0 = q0;
+      rc = launch_dense_kv_tc(a, D, s);
       if (rc) return rc;
     }
+    if (has_slc) {
+      KvArgs a = {};
+      a.q = (const bf16*)q; a.k = (const bf16*)k; a.v = (const bf16*)v; a.dout = (const bf16*)dout_slc; a.lse = lse_slc;
+      a.delta = delta_slc; a.gate = (const bf16*)gate_slc;
+      a.B = B; a.T = T; a.Tq = Tq; a.q0 = q0; a.Hq = Hq; a.Hk = Hkv; a.BS = BS; a.scale = scale; a.dk = (bf16*)dk; a.dv = (bf16*)dv;
+      a.rev_ptr = r.rev_ptr; a.rev_tok = r.rev_tok; a.rev_cap = r.cap; a.dq_part = tiles;
+      a.nshare = n.nshare; a.part = part; a.slabs = n.slabs(); a.nadd = n.nwin;
+      rc = (D == 128 && BS == 64) ? launch_kv_bwd_tc(a, s) : launch_kv_bwd(a, D, s);
+      if (rc) return rc;
+      if (n.nshare > 1) {
+        rc = launch_reduce_shares(part, a.dk, a.dv, n.slabs(), (long long)B * T * Hkv * D, s);
+        if (rc) return rc;
+      }
+    }
     if (dq_from_kv) {   // every token's partial tiles, in slot order, onto dq (after the window's dQ if that ran first)
-      rc = launch_sel_dq_reduce(r, a.dq_part, (bf16*)dq, Hq, D, scale, dq_acc_for_reduce, s);
+      rc = launch_sel_dq_reduce(r, tiles, (bf16*)dq, Hq, D, scale, dq_acc_for_reduce, s);
       if (rc) return rc;
     }
   }
@@ -774,6 +799,23 @@ int nsa_sel_swa_bwd_ix(const void* q, const void* k, const void* v, const void* 
                        const void* gate_swa, void* dq, int accumulate_dq, void* dk, void* dv, void* ws, size_t ws_bytes, int B,
                        int T, int Hq, int Hkv, int D, int S, int BS, int window, float scale, int Tq, int q0, void* stream) {
   return sel_swa_bwd_impl(q, k, v, idx, idx64, counts, dout_slc, lse_slc, delta_slc, gate_slc, dout_swa, lse_swa, delta_swa, gate_swa, dq, accumulate_dq, dk, dv, ws, ws_bytes, B, T, Hq, Hkv, D, S, BS, window, scale, Tq, q0, stream, nullptr, index);
+}
+
+int nsa_attn_bwd_ix(const void* q, const void* k, const void* v, const void* ck, const void* cv, const void* idx, int idx64,
+                    const int32_t* counts, const void* index, const void* dout, const float* lse_slc, const float* lse_swa,
+                    const float* lse_cmp, const float* delta_slc, const float* delta_swa, const float* delta_cmp,
+                    const void* g_slc, const void* g_swa, const void* g_cmp, void* dq, void* dk, void* dv, void* dck, void* dcv,
+                    void* ws, size_t ws_bytes, int B, int T, int Tc, int Hq, int Hkv, int D, int S, int BS, int window, int block,
+                    int stride, int causal, float scale, void* stream) {
+  if (!ck || !cv || !lse_cmp || !dout || !delta_cmp || !dq || !dk || !dv || !dck || !dcv || !idx || !index || !ws)
+    return fail(-1, "nsa_attn_bwd_ix: null pointer");
+  if (Tc <= 0) return fail(-1, "nsa_attn_bwd_ix: no compressed position");
+  if (ws_bytes < nsa_attn_bwd_ix_workspace_bytes(B, T, Tc, Hq, Hkv, D, S, BS, window))
+    return fail(-6, "nsa_attn_bwd_ix: workspace too small");
+  const CmpBwd c = {ck, cv, lse_cmp, delta_cmp, g_cmp, Tc, block, stride, causal};
+  int rc = sel_swa_bwd_impl(q, k, v, idx, idx64, counts, dout, lse_slc, delta_slc, g_slc, window > 0 ? dout : nullptr, lse_swa, delta_swa, g_swa, dq, 0, dk, dv, ws, ws_bytes, B, T, Hq, Hkv, D, S, BS, window, scale, T, 0, stream, nullptr, index, &c);
+  if (rc) return rc;
+  return cmp_dkv(q, ck, cv, lse_cmp, dout, delta_cmp, g_cmp, dck, dcv, ws, B, T, Tc, Hq, Hkv, D, block, stride, causal, scale, T, 0, (cudaStream_t)stream);
 }
 
 int nsa_gather_probe(const void* k, const void* v, const void* idx, int idx64, int B, int T, int Hq, int Hkv, int D, int S,

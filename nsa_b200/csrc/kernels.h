@@ -167,27 +167,45 @@ int dense_tc2_status(int* out);
 int launch_dense_dq_tc(const DenseArgs& a, int head_dim, cudaStream_t s);
 int dense_dq_tc_status(int* out);
 
-// ---- key/value-major backward (dK,dV of selected + sliding window; dCK,dCV of compressed) ---
+// ---- dK, dV of the dense branches (dense_kv_tc.cu; head_dim 64 or 128) --------------------
+struct DenseKvArgs {
+  int mode;               // 0 sliding window over k,v; 1 compressed
+  const bf16 *q, *k, *v;  // [B,Tq,Hq,D], [B,Lk,Hk,D]
+  const bf16* dout;
+  const float *lse, *delta;
+  const bf16* gate;       // or null
+  bf16 *dk, *dv;          // part null: the result.  Mode 1 with part: the sum of the segments
+  float* part;            // fp32 slabs [2][slabs][n_out] (dK, then dV), the kernel's own from slab0 on, or null (nslab 1)
+  int nslab, slab0, slabs;   // mode 0: parts of a key tile's query range, each slab complete; mode 1: segments of seg_len query
+  int seg_len;               // rows (a multiple of 8), written where they see something of the key tile; slab0 0, slabs nslab
+  int Hq, Hk, Lk;         // Lk: keys per sequence (equal lengths)
+  int window, cblock, cstride, causal;
+  float scale;
+  long long n_out;        // set by the launcher
+  Seqs seq;
+};
+int launch_dense_kv_tc(const DenseKvArgs& a, int head_dim, cudaStream_t s);
+int dense_kv_window_slabs(int B, int T, int Hk, int window);
+int dense_kv_segment_rows(int B, int T, int Tc, int Hk);
+int dense_kv_tc_status(int* out);
+
+// ---- key/value-major backward of the selected branch (dK, dV, dQ partials) ---
 struct KvArgs {
-  int mode;               // 0 selected (+ window) over k,v; 1 compressed
-  const bf16* q;          // [B,T,Hq,D]
-  const bf16* k;          // [B,Lk,Hk,D]
+  const bf16* q;          // [B,Tq,Hq,D]
+  const bf16* k;          // [B,T,Hk,D]
   const bf16* v;
-  // branch A: selected (mode 0) or compressed (mode 1); branch B: sliding window (mode 0 only)
-  const bf16* dout_a;  const float* lse_a;  const float* delta_a;  const bf16* gate_a;
-  const bf16* dout_b;  const float* lse_b;  const float* delta_b;  const bf16* gate_b;
-  const int* rev_ptr;     // [B,Hk,NB+1]   mode 0: CSR over selection blocks
+  const bf16* dout;  const float* lse;  const float* delta;  const bf16* gate;
+  const int* rev_ptr;     // [B,Hk,NB+1]   CSR over selection blocks
   const int* rev_tok;     // [B,Hk,cap]    tokens ascending inside each block's list
   long long rev_cap;
-  bf16* dk;               // [B,Lk,Hk,D]
+  bf16* dk;               // [B,T,Hk,D]
   bf16* dv;
-  bf16* dq_part;          // mode 0, optional: the selected branch's dQ as per-visit partial tiles [B,Hk,rev_cap,G16][16][D]
-                          // (position = place in the reverse-index list), summed later by launch_sel_dq_reduce
-  float* part;            // fp32 partials [2][nseg or nshare][B,Lk,Hk,D]: dK then dV (mode 0: only with nshare > 1)
-  int nseg, seg_len;      // mode 1: token segments
-  int nshare;             // mode 0: shares of a block's token stream
-  int B, T, Lk, Hq, Hk, BS, window;
-  int cblock, cstride, causal;
+  bf16* dq_part;          // optional: dQ as per-visit partial tiles [B,Hk,rev_cap,G16][16][D] (position = place in the
+                          // reverse-index list), summed later by launch_sel_dq_reduce
+  int nshare;             // shares of a block's token stream; above 1 they are slabs 0 .. of part
+  float* part;            // fp32 [2][slabs][B,T,Hk,D]: dK then dV
+  int slabs, nadd;        // nshare 1: slabs 0 .. nadd-1 (the window's) are added before dk, dv are rounded
+  int B, T, Hq, Hk, BS;
   float scale;
   int Tq, q0;             // query shard (rev_tok holds sequence positions)
 };
@@ -367,11 +385,8 @@ int sel_fwd_kv_status(int* out);
 // backward; dq rows of a (token, group) are the same contiguous tile.
 int launch_sel_dq_reduce(const RevArgs& a, const bf16* part, bf16* dq, int Hq, int D, float scale, int accumulate,
                          cudaStream_t s);
-// out(bf16)[i] = sum over valid segments of part[seg][i]
-int launch_reduce_segments(const float* part, bf16* out, int nseg, long long n_per_seg, int q0, int Tq, int Lk, int Hk,
-                           int D, int seg_len, int cblock, int cstride, int causal, cudaStream_t s);
-// dk, dv (bf16) = sum over the shares of part [2][nshare][n]
-int launch_reduce_shares(const float* part, bf16* dk, bf16* dv, int nshare, long long n, cudaStream_t s);
+// dk, dv (bf16) = sum over the slabs of part [2][nslab][n]
+int launch_reduce_shares(const float* part, bf16* dk, bf16* dv, int nslab, long long n, cudaStream_t s);
 int misc_status(int* out);
 
 int num_sms();

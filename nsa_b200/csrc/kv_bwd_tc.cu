@@ -1,6 +1,5 @@
-// Key/value-major backward on tcgen05 (head_dim 128, 64-key blocks): dK,dV of the selected + sliding-window
-// branches and dCK,dCV of the compressed branch.  Same work decomposition and reference semantics as kv_bwd.cu
-// (nsa/selection_attn.py:151-253 through a reverse index; nsa/triton_attention.py:219-318), different engine.
+// Key/value-major backward of the selected branch on tcgen05 (head_dim 128, 64-key blocks): dK, dV and dQ partials.  Same work
+// decomposition and reference semantics as kv_bwd.cu (nsa/selection_attn.py:151-253 through a reverse index), different engine.
 //
 // One CTA owns 64 keys.  Query tokens that see them arrive in batches of 8: the 8 x 16 (token, head) rows form a
 // [128 x D] tile of Q and of dO in shared memory (8 TMA boxes of 16 rows each, 128-byte swizzle).  Per batch, one
@@ -9,12 +8,12 @@
 //     dP  [128 rows x 64 keys] = dOg . V^T         A = dOg (K-major), B = V  (K-major)
 //     dV^T[128 d    x 64 keys] += dOg^T . (g P)    A = dOg (MN-major), B = P  (MN-major, written by the soft-max warps)
 //     dK^T[128 d    x 64 keys] += Qg^T . dS        A = Qg (MN-major),  B = dS (MN-major)
-// Eight soft-max warps own half a row per thread (lse, delta, gate and the causal/window mask are thread-local, no
+// Eight soft-max warps own half a row per thread (lse, delta, gate and the causal mask are thread-local, no
 // shuffles; warps 2-5 take key columns 0-31, warps 6-9 columns 32-63 of the same TMEM lanes): they read S and dP
 // from TMEM, form P and dS = P (g dP - delta), and store both as bf16 tiles.
 // The MMA thread issues S/dP of batch n+1 before dV/dK of batch n, so the tensor core works while the soft-max
 // warps compute.  dV^T and dK^T stay in TMEM for the CTA's whole token stream and are stored once.
-// Optionally (mode 0) the selected branch's dQ comes out of this kernel too: dS of a batch is already in shared memory,
+// Optionally dQ comes out of this kernel too: dS of a batch is already in shared memory,
 // so one more product  dQ_part[128 rows x 128 d] = dS . K  (A = dS K-major, B = K MN-major, a third accumulator in TMEM)
 // gives the batch's contribution to dQ, which the soft-max warps store as bf16 tiles indexed by the batch's positions
 // in the reverse-index list; a small kernel later sums every token's tiles in slot order.  That replaces the
@@ -53,26 +52,9 @@ constexpr uint32_t kSmem = 2 * KV_TILE + kStages * STAGE + 4 * P_TILE + 256 + 10
 constexpr uint32_t kTmemCols = 512;        // two S/dP buffers: S 0..63, dP 64..127 | 128..255; dV^T 256..319, dK^T 320..383
 constexpr uint32_t kColDV = 256, kColDK = 320, kColDQ = 384;   // dQ_part: 384..511
 
-struct Stream {  // the token stream of one CTA: branch A (list or range) then branch B (window range)
-  int nA, nB, ta_lo, tb_lo;
-  const int* list;
-};
-
-__device__ __forceinline__ int stream_token(const Stream& st, int br, int i) {
-  if (br == 0) {
-    if (i >= st.nA) i = st.nA - 1;
-    return st.list ? st.list[st.ta_lo + i] : st.ta_lo + i;
-  }
-  if (i >= st.nB) i = st.nB - 1;
-  return st.tb_lo + i;
-}
-
-template <int MODE>
 __global__ void __launch_bounds__(kThreads, 1)
-    kv_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDOa,
-                     const __grid_constant__ CUtensorMap tmDOb, const __grid_constant__ CUtensorMap tmK,
-                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmQw,
-                     const __grid_constant__ CUtensorMap tmDOw, const KvArgs a) {
+    kv_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
+                     const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const KvArgs a) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t sbase = (raw + 1023u) & ~1023u;
@@ -115,62 +97,27 @@ __global__ void __launch_bounds__(kThreads, 1)
   tc_fence_after();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(sgen + (tmem_slot - sbase));
 
-  // ---- decode the work item (same mapping as kv_bwd.cu) -----------------------------------------------
+  // ---- decode the work item ------------------------------------------------------------------------------
+  // (batch, kv head)-major: the CTAs resident at one time share one 16-head group's Q and dO rows (67 MB at T = 8192), which
+  // then stay in L2; block-major order made every gather a DRAM access
   const int G16 = (a.Hq / a.Hk) / 16;
-  int b, hk, blk, seg = 0;
-  Stream st = {0, 0, 0, 0, nullptr};
-  bool skip = false;
-  {
-    long long item = blockIdx.x;
-    const int BH = a.B * a.Hk;
-    if (MODE == 0) {
-      seg = (int)(item % a.nshare);
-      item /= a.nshare;
-      // (batch, kv head)-major: the CTAs resident at one time share one 16-head group's Q and dO rows (67 MB at
-      // T = 8192), which then stay in L2; block-major order made every gather a DRAM access
-      const int NB = (a.T + 63) / 64;
-      blk = (int)(item % NB);
-      const int bh = (int)(item / NB);
-      b = bh / a.Hk;
-      hk = bh % a.Hk;
-      if (a.rev_ptr) {
-        const int* rp = a.rev_ptr + (long long)bh * (NB + 1);
-        st.ta_lo = rp[blk];
-        st.nA = rp[blk + 1] - rp[blk];
-        st.list = a.rev_tok + (long long)bh * a.rev_cap;
-      }
-      if (a.window > 0) {
-        st.tb_lo = max(blk * 64, a.q0);
-        st.nB = max(0, min(a.q0 + a.Tq, blk * 64 + 63 + a.window) - st.tb_lo);
-      }
-      if (a.nshare > 1) {   // this CTA's share of both streams, in whole batches
-        const int ba = (st.nA + kTokB - 1) / kTokB, bb = (st.nB + kTokB - 1) / kTokB;
-        const int a0 = ba * seg / a.nshare * kTokB, a1 = min(st.nA, ba * (seg + 1) / a.nshare * kTokB);
-        const int b0 = bb * seg / a.nshare * kTokB, b1 = min(st.nB, bb * (seg + 1) / a.nshare * kTokB);
-        st.ta_lo += a0;
-        st.nA = a1 - a0;
-        st.tb_lo += b0;
-        st.nB = b1 - b0;
-      }
-    } else {
-      seg = (int)(item % a.nseg);
-      item /= a.nseg;
-      const int NT = (a.Lk + 63) / 64;
-      blk = (int)(item % NT);
-      const int bh = (int)(item / NT);
-      b = bh / a.Hk;
-      hk = bh % a.Hk;
-      const int first = a.causal ? blk * 64 * a.cstride + a.cblock : 0;
-      st.ta_lo = max(first, a.q0 + seg * a.seg_len);
-      st.nA = min(a.q0 + a.Tq, a.q0 + (seg + 1) * a.seg_len) - st.ta_lo;
-      if (st.nA <= 0) skip = true;  // the reducer skips this segment too
-    }
+  const int NB = (a.T + 63) / 64;
+  const int seg = blockIdx.x % a.nshare, item = blockIdx.x / a.nshare;
+  const int blk = item % NB, bh = item / NB, b = bh / a.Hk, hk = bh % a.Hk;
+  const int* rp = a.rev_ptr + (long long)bh * (NB + 1);
+  const int* list = a.rev_tok + (long long)bh * a.rev_cap;
+  int lo = rp[blk], nA = rp[blk + 1] - lo;
+  if (a.nshare > 1) {   // this CTA's share of the list, in whole batches
+    const int ba = (nA + kTokB - 1) / kTokB;
+    const int a0 = ba * seg / a.nshare * kTokB, a1 = min(nA, ba * (seg + 1) / a.nshare * kTokB);
+    lo += a0;
+    nA = a1 - a0;
   }
   const int key0 = blk * 64;
-  const int nbA = (st.nA + kTokB - 1) / kTokB, nbB = (st.nB + kTokB - 1) / kTokB;
-  const int nb_sub = nbA + nbB;             // batches per 16-head sub-group
-  const int nb = skip ? 0 : nb_sub * G16;   // batches of this CTA
-  const bool emit_dq = MODE == 0 && a.dq_part != nullptr;   // selected-branch batches also leave their dQ partial
+  const int nb_sub = (nA + kTokB - 1) / kTokB;   // batches per 16-head sub-group
+  const int nb = nb_sub * G16;                   // batches of this CTA
+  const bool emit_dq = a.dq_part != nullptr;     // every batch also leaves its dQ partial
+  auto list_token = [&](int i) { return list[lo + min(i, nA - 1)]; };
 
   // 512 threads start with 128 registers each; the soft-max warps need 168.  Warps 0-3 (TMA, MMA) and 12-15 (drain)
   // give registers back, warps 4-11 take them (each instruction is executed by a whole warpgroup).
@@ -179,14 +126,12 @@ __global__ void __launch_bounds__(kThreads, 1)
   // pool cannot satisfy blocks for ever): 128 x 80 + 256 x 168 + 128 x 88 = 64512.
   if (warp < 4) {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
-  if (!skip && warp < kProd) {
+  if (warp < kProd) {
     // ------------------------------- TMA producers -----------------------------------------------
     // A batch of gathered tokens (a reverse-index list) is 32 boxes of 2 KB: (token j, Q or dO, column panel).  Box
     // x = 3 * lane + warp belongs to this lane; every producer warp issues its 10 or 11 boxes with a single instruction
     // and arms the stage's barrier with their byte count.  Token ids are fetched one batch ahead.
-    // A batch of consecutive tokens (the window's range, the compressed branch's range) is 4 boxes of 16 KB instead:
-    // [64 columns x 16 heads x 8 tokens] through the 4-D maps, rows past the last token read as zero.
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && lane == 0 && nb > 0) {
       mbar_expect_tx(kv_bar, 2 * KV_TILE);
 #pragma unroll
       for (int p = 0; p < 2; ++p) {
@@ -198,46 +143,28 @@ __global__ void __launch_bounds__(kThreads, 1)
     const bool has = x < 4 * kTokB;
     const int bj = x & 7, bwhich = (x >> 3) & 1, bp = x >> 4;
     const int nmine = (4 * kTokB - warp + kProd - 1) / kProd;   // boxes this warp issues per batch
-    const bool has_w = x < 4;                                   // this lane's 16 KB box of a consecutive-token batch
-    const int nmine_w = (4 - warp + kProd - 1) / kProd;
-    auto batch_token = [&](int n) {
-      if (n >= nb || !has) return 0;
-      const int m = n % nb_sub;
-      const int br = m < nbA ? 0 : 1;
-      return stream_token(st, br, (br == 0 ? m : m - nbA) * kTokB + bj);
-    };
+    auto batch_token = [&](int n) { return n >= nb || !has ? 0 : list_token(n % nb_sub * kTokB + bj); };
     int tk_next = batch_token(0);
     for (int n = 0; n < nb; ++n) {
       const int tk = tk_next;
       tk_next = batch_token(n + 1);
-      const int sub = n / nb_sub, m = n % nb_sub;
-      const int br = m < nbA ? 0 : 1;
-      const int hg = hk * G16 + sub;
-      const CUtensorMap* tmDO = br == 0 ? &tmDOa : &tmDOb;
-      const bool contig = br == 1 || st.list == nullptr;
+      const int hg = hk * G16 + n / nb_sub;
       const int stage = n % kStages;
       const uint32_t ph = (n / kStages) & 1;
       const uint32_t fb = full0 + 8 * stage;
       int good = 1;
       if (lane == 0) {
         good = mbar_wait(empty0 + 8 * stage, ph ^ 1, DEV_ERR_EMPTY_WAIT) ? 1 : 0;
-        if (good) mbar_expect_tx(fb, contig ? nmine_w * 16384 : nmine * 2048);
+        if (good) mbar_expect_tx(fb, nmine * 2048);
       }
       if (!__shfl_sync(0xffffffffu, good, 0)) break;
-      if (contig) {
-        if (has_w) {
-          const uint32_t q_s = ring + stage * STAGE, do_s = q_s + Q_TILE;
-          const int t0 = (br == 0 ? st.ta_lo + m * kTokB : st.tb_lo + (m - nbA) * kTokB) - a.q0;
-          const int wh = x >> 1, pp = x & 1;
-          tma_load_4d((wh ? do_s : q_s) + pp * Q_PANEL, wh ? &tmDOw : &tmQw, fb, pp * 64, hg * 16, t0, b);
-        }
-      } else if (has) {
+      if (has) {
         const uint32_t q_s = ring + stage * STAGE, do_s = q_s + Q_TILE;
         const int qrow = (int)(((long long)b * a.Tq + (tk - a.q0)) * a.Hq + hg * 16);
-        tma_load_2d((bwhich ? do_s : q_s) + bp * Q_PANEL + bj * 2048, bwhich ? tmDO : &tmQ, fb, bp * 64, qrow);
+        tma_load_2d((bwhich ? do_s : q_s) + bp * Q_PANEL + bj * 2048, bwhich ? &tmDO : &tmQ, fb, bp * 64, qrow);
       }
     }
-  } else if (!skip && warp == kMmaWarp) {
+  } else if (warp == kMmaWarp) {
     // ------------------------------- MMA issuer A: S and dP ----------------------------------------
     // S/dP of batch n is issued as soon as its Q/dO stage has landed and its TMEM buffer is free (the soft-max warps
     // hold batch n-2 in registers), i.e. ahead of dV/dK of batch n-1, which the second issuer handles.
@@ -268,7 +195,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         umma_commit(sdp_full + 8 * (n & 1));
       }
     }
-  } else if (!skip && warp == kMma2Warp) {
+  } else if (warp == kMma2Warp) {
     // ------------------------------- MMA issuer B: dV, dK, dQ partials -----------------------------
     if (lane == 0 && nb > 0) {
       constexpr uint32_t idesc_mn = umma_idesc_bf16(128, 64, 1, 1);   // both operands MN-major
@@ -288,7 +215,6 @@ __global__ void __launch_bounds__(kThreads, 1)
         dDSk[i] = dDS[i];   // the same tile read K-major for the dQ partial
       }
       const uint64_t dKmn = umma_smem_desc(k_s, KV_PANEL, 1024);
-      int ndq = 0;          // dQ partials issued so far
       for (int n = 0; ok && n < nb; ++n) {
         ok = mbar_wait(pds_full + 8 * (n & 1), (n >> 1) & 1, DEV_ERR_FULL_WAIT);
         if (!ok) break;
@@ -301,9 +227,9 @@ __global__ void __launch_bounds__(kThreads, 1)
           umma_ss(tmem + kColDK, umma_desc_advance(aq, ks * 2048), umma_desc_advance(bds, ks * 2048), idesc_mn, (n | ks) ? 1u : 0u);
         }
         umma_commit(empty0 + 8 * (n % kStages));
-        if (emit_dq && (n % nb_sub) < nbA) {
+        if (emit_dq) {
           // the previous partial must have been read out of its accumulator by the drain warps
-          if (ndq > 0) ok = mbar_wait(dq_free, (ndq - 1) & 1, DEV_ERR_EMPTY_WAIT);
+          if (n > 0) ok = mbar_wait(dq_free, (n - 1) & 1, DEV_ERR_EMPTY_WAIT);
           if (!ok) break;
           tc_fence_after();
           const uint64_t ads = (n & 1) ? dDSk[1] : dDSk[0];
@@ -311,7 +237,6 @@ __global__ void __launch_bounds__(kThreads, 1)
           for (int ks = 0; ks < 4; ++ks)   // contraction over the 64 keys, 16 per step
             umma_ss(tmem + kColDQ, umma_desc_advance(ads, ks * 32), umma_desc_advance(dKmn, ks * 2048), idesc_dq, ks ? 1u : 0u);
           umma_commit(dq_full);
-          ++ndq;
         }
         umma_commit(pds_free + 8 * (n & 1));
       }
@@ -320,9 +245,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
   } else if (warp >= kDrainWarp) {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
-  if (!skip) {
+  {
     // ------------------------------- drain warps: dQ partials, one row per thread ------------------
-    // dQ partial of a selected batch: accumulator -> bf16 -> shared memory -> one bulk store.  The staging area is that
+    // dQ partial of a batch: accumulator -> bf16 -> shared memory -> one bulk store.  The staging area is that
     // batch's own P/dS tile pair (32 KB = 128 rows x 256 bytes): dq_full also says that every MMA that read the pair
     // has completed, and the soft-max warps write it again (batch n+2) only after stg_free.  The 8 tokens' [16 x D]
     // tiles sit at consecutive list positions, i.e. contiguous in dq_part when the KV head has one 16-head group.
@@ -336,11 +261,9 @@ __global__ void __launch_bounds__(kThreads, 1)
       const uint32_t lane_addr = (uint32_t)(32 * quad) << 16;
       const bool elected = warp == kDrainWarp && lane == 0;
       bool ok = true;
-      int k = 0;   // partials drained so far
       for (int n = 0; ok && n < nb; ++n) {
         const int sub = n / nb_sub, mloc = n % nb_sub;
-        if (mloc >= nbA) continue;
-        ok = mbar_wait(dq_full, k & 1, DEV_ERR_FULL_WAIT);
+        ok = mbar_wait(dq_full, n & 1, DEV_ERR_FULL_WAIT);
         if (!ok) break;
         tc_fence_after();
         const uint32_t stg = p_s0 + (uint32_t)(n & 1) * 2 * P_TILE;
@@ -369,11 +292,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         fence_proxy_async();
         mbar_arrive(stg_full);
         if (elected) {
-          ok = mbar_wait(stg_full, k & 1, DEV_ERR_FULL_WAIT);
-          const int nvalid = min(kTokB, st.nA - mloc * kTokB);
+          ok = mbar_wait(stg_full, n & 1, DEV_ERR_FULL_WAIT);
+          const int nvalid = min(kTokB, nA - mloc * kTokB);
           if (ok && nvalid > 0) {
-            const long long bh = (long long)b * a.Hk + hk;
-            bf16* dst = a.dq_part + ((bh * a.rev_cap + st.ta_lo + mloc * kTokB) * G16 + sub) * (16 * D);
+            bf16* dst = a.dq_part + (((long long)bh * a.rev_cap + lo + mloc * kTokB) * G16 + sub) * (16 * D);
             if (G16 == 1) {
               bulk_store_evict_first(dst, stg, (uint32_t)nvalid * 16 * D * 2);
             } else {
@@ -385,14 +307,13 @@ __global__ void __launch_bounds__(kThreads, 1)
           bulk_wait_read();                       // the pair may be written again
           mbar_arrive(stg_free + 8 * (n & 1));
         }
-        ++k;
       }
       if (elected) bulk_wait_all();
     }
   }
   } else {
   asm volatile("setmaxnreg.inc.sync.aligned.u32 168;");
-  if (!skip) {
+  {
     // ------------------------------- soft-max warps: one (token, head) row per thread --------------
     const int quad = warp & 3;
     const int half = (warp - kSoftWarp) >> 2;    // which 32 key columns this thread owns
@@ -401,59 +322,43 @@ __global__ void __launch_bounds__(kThreads, 1)
     const uint32_t lane_addr = (uint32_t)(32 * quad) << 16;
     const float sl2 = a.scale * kLog2e;
     bool ok = true;
-    // per-row operands are fetched one batch ahead (token ids two ahead) so their latency hides behind the MMAs
+    // per-row operands are fetched one batch ahead (token ids two ahead) so their latency hides behind the MMAs; they are kept
+    // as loaded, since converting them would wait for the loads
     struct RowInfo {
       int t;
       bool live;
-      int br;
-      float lse2, del, gv;
+      float lse, del;
+      bf16 g;
     };
-    auto row_token = [&](int n, int& br, bool& live) {
-      br = 0;
+    auto row_token = [&](int n, bool& live) {
       live = false;
       if (n >= nb) return 0;
-      const int m = n % nb_sub;
-      br = m < nbA ? 0 : 1;
-      const int i = (br == 0 ? m : m - nbA) * kTokB + j;
-      live = i < (br == 0 ? st.nA : st.nB);
-      return stream_token(st, br, i);
+      const int i = n % nb_sub * kTokB + j;
+      live = i < nA;
+      return list_token(i);
     };
-    auto row_load = [&](int n, int t, int br, bool live) {
-      RowInfo r;
-      r.t = t;
-      r.live = live;
-      r.br = br;
-      r.lse2 = 0.f;
-      r.del = 0.f;
-      r.gv = 1.f;
+    auto row_load = [&](int n, int t, bool live) {
+      RowInfo r = {t, live, 0.f, 0.f, __float2bfloat16(1.f)};
       if (n < nb) {
-        const int sub = n / nb_sub;
-        const long long qrow = ((long long)b * a.Tq + (t - a.q0)) * a.Hq + (hk * G16 + sub) * 16 + head;
-        r.lse2 = (br == 0 ? a.lse_a : a.lse_b)[qrow] * kLog2e;
-        r.del = (br == 0 ? a.delta_a : a.delta_b)[qrow];
-        const bf16* gp = br == 0 ? a.gate_a : a.gate_b;
-        if (gp) r.gv = __bfloat162float(gp[qrow]);
+        const long long qrow = ((long long)b * a.Tq + (t - a.q0)) * a.Hq + (hk * G16 + n / nb_sub) * 16 + head;
+        r.lse = a.lse[qrow];
+        r.del = a.delta[qrow];
+        if (a.gate) r.g = a.gate[qrow];
       }
       return r;
     };
-    // With dQ partials: the drain warps stage the partial of a selected batch n in that batch's own P/dS pair; the pair
-    // is written again for batch n+2 only after their bulk store has read it (stg_free of that pair).
-    int nstg[2] = {0, 0};   // waits done on each pair's stg_free
-    int br1, br2;
-    bool live1, live2;
-    int t1 = row_token(0, br1, live1);
-    RowInfo cur = row_load(0, t1, br1, live1);
-    t1 = row_token(1, br1, live1);
+    // With dQ partials: the drain warps stage the partial of batch n in that batch's own P/dS pair; the pair is written again
+    // for batch n+2 only after their bulk store has read it (stg_free of that pair).
+    bool live1;
+    int t1 = row_token(0, live1);
+    RowInfo cur = row_load(0, t1, live1);
+    t1 = row_token(1, live1);
     for (int n = 0; ok && n < nb; ++n) {
       const RowInfo ri = cur;
-      cur = row_load(n + 1, t1, br1, live1);          // operands of batch n+1
-      const int t2 = row_token(n + 2, br2, live2);    // token id of batch n+2
-      t1 = t2;
-      br1 = br2;
-      live1 = live2;
-      const int t = ri.t, br = ri.br;
+      cur = row_load(n + 1, t1, live1);     // operands of batch n+1
+      t1 = row_token(n + 2, live1);         // token id of batch n+2
+      const int t = ri.t;
       const bool live = ri.live;
-      const float lse2 = ri.lse2, del = ri.del, gv = ri.gv;
 
       const uint32_t buf = n & 1, use = n >> 1;
       const uint32_t tcol = buf * 128;
@@ -471,11 +376,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         tc_fence_before();
         mbar_arrive(sdp_free + 8 * buf);   // S and dP are in registers: batch n+2 may overwrite this TMEM buffer
         const int kfirst = key0 + half * 32, klast = kfirst + 31;
-        bool all_valid;
-        if (MODE == 0)
-          all_valid = (klast <= t) && (br == 0 || kfirst > t - a.window);
-        else
-          all_valid = klast < a.Lk && (!a.causal || klast * a.cstride + a.cblock <= t);
+        const bool all_valid = klast <= t;
+        const float lse2 = ri.lse * kLog2e, del = ri.del, gv = __bfloat162float(ri.g);
         if (!live || !(lse2 > -INFINITY)) {
 #pragma unroll
           for (int e = 0; e < 16; ++e) pw[e] = dw[e] = 0u;
@@ -494,11 +396,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
               const int kp = kfirst + e + u;
-              bool valid;
-              if (MODE == 0)
-                valid = (kp <= t) && (br == 0 || kp > t - a.window);
-              else
-                valid = kp < a.Lk && (!a.causal || kp * a.cstride + a.cblock <= t);
+              const bool valid = kp <= t;
               pv[u] = valid ? ex2(sv[e + u] * sl2 - lse2) : 0.f;
             }
             pw[e / 2] = pack_bf16(pv[0] * gv, pv[1] * gv);
@@ -510,9 +408,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         ok = mbar_wait(pds_free + 8 * buf, (use - 1) & 1, DEV_ERR_EMPTY_WAIT);   // dV/dK of batch n-2 have read this pair
         if (!ok) break;
       }
-      if (emit_dq && n >= 2 && ((n - 2) % nb_sub) < nbA) {
-        ok = mbar_wait(stg_free + 8 * buf, nstg[buf] & 1, DEV_ERR_EMPTY_WAIT);
-        ++nstg[buf];
+      if (emit_dq && n >= 2) {
+        ok = mbar_wait(stg_free + 8 * buf, (use - 1) & 1, DEV_ERR_EMPTY_WAIT);
         if (!ok) break;
       }
       // this thread's half of row `row` of the [128 x 64] bf16 tiles: 4 chunks of 16 bytes at swizzled positions
@@ -532,7 +429,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     tc_fence_after();
     const int dch = row;  // channel owned by this thread
     {
-      const int which = half;   // warps 2-5 store dV, warps 6-9 store dK
+      const int which = half;   // half 0 stores dV, half 1 dK
+      const float mul = which ? a.scale : 1.f;
+      const long long Nout = (long long)a.B * a.T * a.Hk * D;
+      float* part = a.part + (which ? 0 : a.slabs * Nout);
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         float vals[16];
@@ -543,18 +443,25 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
           for (int e = 0; e < 16; ++e) vals[e] = 0.f;
         }
-        const float mul = which ? a.scale : 1.f;
+        float add[16];   // the window's part
+#pragma unroll
+        for (int e = 0; e < 16; ++e) add[e] = 0.f;
+        for (int w = 0; a.nshare == 1 && w < a.nadd; ++w) {
+#pragma unroll
+          for (int e = 0; e < 16; ++e) {
+            const int kp = key0 + c * 16 + e;
+            if (kp < a.T) add[e] += part[w * Nout + (((long long)b * a.T + kp) * a.Hk + hk) * D + dch];
+          }
+        }
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
           const int kp = key0 + c * 16 + e;
-          if (!ok || kp >= a.Lk) continue;
-          const long long off = (((long long)b * a.Lk + kp) * a.Hk + hk) * D + dch;
-          if (MODE == 0 && a.nshare == 1) {
-            (which ? a.dk : a.dv)[off] = __float2bfloat16(vals[e] * mul);
-          } else {
-            const long long N = (long long)a.B * a.Lk * a.Hk * D;
-            a.part[((long long)(which ? 0 : MODE == 0 ? a.nshare : a.nseg) + seg) * N + off] = vals[e] * mul;
-          }
+          if (!ok || kp >= a.T) continue;
+          const long long off = (((long long)b * a.T + kp) * a.Hk + hk) * D + dch;
+          if (a.nshare > 1)
+            part[seg * Nout + off] = vals[e] * mul;
+          else
+            (which ? a.dk : a.dv)[off] = __float2bfloat16(fmaf(vals[e], mul, add[e]));
         }
       }
     }
@@ -565,44 +472,27 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (warp == kMmaWarp) tmem_dealloc(tmem, kTmemCols);
 }
 
-template <int MODE>
 int launch(const KvArgs& a, cudaStream_t s) {
-  CUtensorMap tmQ, tmA, tmB, tmK, tmV, tmQw, tmDOw;
+  CUtensorMap tmQ, tmDO, tmK, tmV;
   const long long qrows = (long long)a.B * a.Tq * a.Hq;
   if (qrows > 0x7fffffffLL) {
     set_error("B*T*Hq exceeds the 2^31 rows a TMA coordinate can address");
     return -32;
   }
   int rc = make_tmap_rows2d(&tmQ, a.q, D, qrows, 16);
-  if (!rc) rc = make_tmap_rows2d(&tmA, a.dout_a ? a.dout_a : a.dout_b, D, qrows, 16);
-  if (!rc) rc = make_tmap_rows2d(&tmB, a.dout_b ? a.dout_b : a.dout_a, D, qrows, 16);
-  if (!rc) rc = make_tmap_rows4d(&tmK, a.k, D, a.Hk, a.Lk, a.B, 64);
-  if (!rc) rc = make_tmap_rows4d(&tmV, a.v, D, a.Hk, a.Lk, a.B, 64);
-  {   // consecutive-token batches: [64 columns x 16 heads x 8 tokens] boxes of q and of that stream's dO
-    const unsigned long long dims[4] = {(unsigned long long)D, (unsigned long long)a.Hq, (unsigned long long)a.Tq,
-                                        (unsigned long long)a.B};
-    const unsigned long long strides[3] = {(unsigned long long)D * 2, (unsigned long long)a.Hq * D * 2,
-                                           (unsigned long long)a.Tq * a.Hq * D * 2};
-    const unsigned box[4] = {64, 16, (unsigned)kTokB, 1};
-    const void* dow = MODE == 0 ? (a.dout_b ? a.dout_b : a.dout_a) : a.dout_a;
-    if (!rc) rc = make_tmap_generic(&tmQw, a.q, 4, dims, strides, box);
-    if (!rc) rc = make_tmap_generic(&tmDOw, dow, 4, dims, strides, box);
-  }
+  if (!rc) rc = make_tmap_rows2d(&tmDO, a.dout, D, qrows, 16);
+  if (!rc) rc = make_tmap_rows4d(&tmK, a.k, D, a.Hk, a.T, a.B, 64);
+  if (!rc) rc = make_tmap_rows4d(&tmV, a.v, D, a.Hk, a.T, a.B, 64);
   if (rc) return rc;
-  auto kern = kv_bwd_tc_kernel<MODE>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+  cudaError_t e = cudaFuncSetAttribute(kv_bwd_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
   if (e != cudaSuccess) return (int)e;
-  long long grid;
-  if (MODE == 0)
-    grid = (long long)a.B * a.Hk * ((a.T + 63) / 64) * a.nshare;
-  else
-    grid = (long long)a.B * a.Hk * ((a.Lk + 63) / 64) * a.nseg;
+  const long long grid = (long long)a.B * a.Hk * ((a.T + 63) / 64) * a.nshare;
   if (grid <= 0) return 0;
   if (grid > 0x7fffffffLL) {
     set_error("kv backward: grid too large");
     return -33;
   }
-  kern<<<(unsigned)grid, kThreads, kSmem, s>>>(tmQ, tmA, tmB, tmK, tmV, tmQw, tmDOw, a);
+  kv_bwd_tc_kernel<<<(unsigned)grid, kThreads, kSmem, s>>>(tmQ, tmDO, tmK, tmV, a);
   note_launches(1);
   return (int)cudaGetLastError();
 }
@@ -610,7 +500,7 @@ int launch(const KvArgs& a, cudaStream_t s) {
 }  // namespace
 
 // head_dim 128 and 64-key blocks only; the caller falls back to launch_kv_bwd otherwise.
-int launch_kv_bwd_tc(const KvArgs& a, cudaStream_t s) { return a.mode == 0 ? launch<0>(a, s) : launch<1>(a, s); }
+int launch_kv_bwd_tc(const KvArgs& a, cudaStream_t s) { return launch(a, s); }
 int kv_tc_status(int* out) {
   int zero = 0;
   cudaError_t e = cudaMemcpyFromSymbol(out, g_dev_error, sizeof(int));

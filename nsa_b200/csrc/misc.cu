@@ -217,25 +217,6 @@ __global__ void __launch_bounds__(kRevWarps * 32) rev_fill_kernel(const RevArgs 
   }
 }
 
-// ---- fixed-order reduction of segment partials ----------------------------------------------------------
-__global__ void reduce_segments_kernel(const float* __restrict__ part, bf16* __restrict__ out, int nseg,
-                                       long long n_per_seg, int q0, int Tq, int Lk, int HkD, int seg_len, int cblock,
-                                       int cstride, int causal) {
-  const long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 2;
-  if (i >= n_per_seg) return;
-  const int j = (int)((i / HkD) % Lk);
-  const int first = causal ? (j / 64) * 64 * cstride + cblock : 0;
-  float x = 0.f, y = 0.f;
-  for (int seg = 0; seg < nseg; ++seg) {
-    const int lo = max(first, q0 + seg * seg_len), hi = min(q0 + Tq, q0 + (seg + 1) * seg_len);
-    if (hi <= lo) continue;
-    const float2 v = *reinterpret_cast<const float2*>(part + (long long)seg * n_per_seg + i);
-    x += v.x;
-    y += v.y;
-  }
-  *reinterpret_cast<__nv_bfloat162*>(out + i) = __floats2bfloat162_rn(x, y);
-}
-
 // dk, dv = the sum of a key block's shares, in order
 __global__ void __launch_bounds__(256) reduce_shares_kernel(const float* __restrict__ part, bf16* __restrict__ dk, bf16* __restrict__ dv,
                                                             int nshare, long long n) {
@@ -419,16 +400,6 @@ int launch_build_rev(const RevArgs& a, cudaStream_t s) {
   rev_offset_kernel<<<a.B * a.H, 1024, 0, s>>>(a);
   rev_fill_kernel<<<grid, nw * 32, nw * sm, s>>>(a);
   note_launches(4);
-  return (int)cudaGetLastError();
-}
-
-int launch_reduce_segments(const float* part, bf16* out, int nseg, long long n_per_seg, int q0, int Tq, int Lk, int Hk,
-                           int D, int seg_len, int cblock, int cstride, int causal, cudaStream_t s) {
-  if (n_per_seg <= 0) return 0;
-  const long long pairs = n_per_seg / 2;
-  reduce_segments_kernel<<<(unsigned)((pairs + 255) / 256), 256, 0, s>>>(part, out, nseg, n_per_seg, q0, Tq, Lk, Hk * D,
-                                                                          seg_len, cblock, cstride, causal);
-  note_launches(1);
   return (int)cudaGetLastError();
 }
 

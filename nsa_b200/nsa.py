@@ -230,9 +230,11 @@ class _NSAModule(torch.autograd.Function):
         for i, (t0, B, T, c0, Tc) in enumerate(runs):
             r, kv, cb = t0 * Hq, t0 * Hkv * D * 2, c0 * Hkv * D * 2
             rb, ib, r4, r2 = r * D * 2, idx + t0 * Hkv * n_sel * 4, 4 * r, 2 * r
-            size = L.nsa_sel_swa_bwd_ix_workspace_bytes if ix_bytes else _lib.sel_swa_bwd_workspace_bytes
-            n1 = size(B, T, T, Hq, Hkv, D, n_sel, sel_block)
-            n2 = L.nsa_cmp_attn_bwd_workspace_bytes(B, T, Tc, Hkv, D)
+            if ix_bytes:
+                n1, n2 = L.nsa_attn_bwd_ix_workspace_bytes(B, T, Tc, Hq, Hkv, D, n_sel, sel_block, window), 0
+            else:
+                n1 = _lib.sel_swa_bwd_workspace_bytes(B, T, T, Hq, Hkv, D, n_sel, sel_block)
+                n2 = L.nsa_cmp_attn_bwd_workspace_bytes(B, T, Tc, Hkv, D)
             ws = torch.empty(max(n1, n2), dtype=torch.uint8, device=dev)
             qp, kp, vp, dop = P(q) + rb, P(k) + kv, P(v) + kv, P(do) + rb
             if fused:
@@ -245,6 +247,11 @@ class _NSAModule(torch.autograd.Function):
                 chk(L.nsa_cmp_attn_bwd_fused(qp, ck + cb, cv + cb, o_cmp + rb, l_cmp + r4, dop, d_cmp + r4, g_cmp + r2,
                                              dg_cmp + r2, P(dq) + rb, 1, dck + cb, dcv + cb, P(ws), n2, B, T, Tc, Hq, Hkv, D,
                                              block, stride, 1 if causal else 0, scale, T, 0, S), "nsa_cmp_attn_bwd_fused")
+            elif ix_bytes:
+                chk(L.nsa_attn_bwd_ix(qp, kp, vp, ck + cb, cv + cb, ib, 0, None, ix[i], dop, l_slc + r4, at(l_swa, r4), l_cmp + r4,
+                                      d_slc + r4, d_swa + r4, d_cmp + r4, g_slc + r2, g_swa + r2, g_cmp + r2, P(dq) + rb,
+                                      P(dk) + kv, P(dv) + kv, dck + cb, dcv + cb, P(ws), n1, B, T, Tc, Hq, Hkv, D, n_sel,
+                                      sel_block, window, block, stride, 1 if causal else 0, scale, S), "nsa_attn_bwd")
             else:
                 chk(L.nsa_sel_swa_bwd_ix(qp, kp, vp, ib, 0, None, ix[i], dop, l_slc + r4, d_slc + r4, g_slc + r2,
                                          dop if win else None, at(l_swa, r4), d_swa + r4 if win else None, g_swa + r2,

@@ -99,8 +99,9 @@ class ParallelNSAFunction(torch.autograd.Function):
         opt = lambda t, sl: P(t[:, sl]) if t is not None else None
         for (a, b), ix in zip(seqs or [(0, T)], indices):
             sl = slice(a, b)
-            size = L.nsa_sel_swa_bwd_ix_workspace_bytes if ix is not None else _lib.sel_swa_bwd_workspace_bytes
-            ws_bytes = size(B, b - a, b - a, Hq, Hkv, D, S, block_size)
+            shape = (B, b - a, b - a, Hq, Hkv, D, S, block_size)
+            ws_bytes = (L.nsa_sel_swa_bwd_ix_workspace_bytes(*shape, window_size) if ix is not None
+                        else _lib.sel_swa_bwd_workspace_bytes(*shape))
             ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
             _lib.check(L.nsa_sel_swa_bwd_ix(
                 P(q[:, sl]), P(k[:, sl]), P(v[:, sl]), P(idx[:, sl]), i64, opt(counts, sl), P(ix),

@@ -27,8 +27,9 @@ def _attend(q, k, v, mask, scale):
 
 
 @pytest.mark.parametrize("B,T,Hq,Hk,D,window", [(1, 1, 16, 1, 128, 512), (2, 7, 32, 1, 64, 3), (1, 129, 64, 4, 128, 128),
-                                                 (2, 333, 16, 1, 64, 100), (1, 1100, 32, 2, 128, 512), (3, 257, 16, 1, 128, 1000)])
-def test_dense_dq(nsa, B, T, Hq, Hk, D, window):
+                                                 (2, 333, 16, 1, 64, 100), (1, 1100, 32, 2, 128, 512), (3, 257, 16, 1, 128, 1000),
+                                                 (1, 4100, 32, 1, 128, 200)])
+def test_dense_backward(nsa, B, T, Hq, Hk, D, window):
     L, P = nsa._lib.lib(), lambda t: t.data_ptr()
     gen = torch.Generator(device=DEV).manual_seed(T)
     rnd = lambda *s: torch.randn(*s, generator=gen, device=DEV).bfloat16()
@@ -40,19 +41,26 @@ def test_dense_dq(nsa, B, T, Hq, Hk, D, window):
     masks = ((j <= t) & (j > t - window), t >= torch.arange(Tc, device=DEV)[None] * stride + block)
     want, lse, delta = [], [], []
     for (kk, vv), mask in zip(((k, v), (ck, cv)), masks):
-        qf = q.float().requires_grad_(True)
-        o, l = _attend(qf, kk.float(), vv.float(), mask, scale)
-        want.append(torch.autograd.grad(o, qf, do.float() * g.float()[..., None])[0])
+        leaf = [x.float().requires_grad_(True) for x in (q, kk, vv)]
+        o, l = _attend(*leaf, mask, scale)
+        want.append(torch.autograd.grad(o, leaf, do.float() * g.float()[..., None]))
         lse.append(l.detach().contiguous())
         delta.append((g.float() * (o.detach() * do.float()).sum(-1)).contiguous())
-    dq_w, dq_c, both = torch.empty_like(q), torch.empty_like(q), torch.empty_like(q)
-    win = lambda dq, acc: L.nsa_sel_swa_bwd(P(q), P(k), P(v), None, 0, None, None, None, None, None, P(do), P(lse[0]), P(delta[0]),
-                                            P(g), P(dq), acc, None, None, None, 0, B, T, Hq, Hk, D, 16, 64, window, scale, None)
-    cmp = lambda dq, acc: L.nsa_cmp_attn_bwd(P(q), P(ck), P(cv), P(lse[1]), P(do), P(delta[1]), P(g), P(dq), acc, None, None, None,
-                                             0, B, T, Tc, Hq, Hk, D, block, stride, 1, scale, None)
-    for rc in (win(dq_w, 0), cmp(dq_c, 0), win(both, 0), cmp(both, 1)):
-        nsa._lib.check(rc, "dense dQ")
-    _close("dq window", dq_w, want[0])
-    _close("dq compressed", dq_c, want[1])
-    _close("dq accumulated", both, want[0] + want[1])
+    dq_w, dq_c, both, dk, dv, dck, dcv = (torch.empty_like(x) for x in (q, q, q, k, v, ck, cv))
+    nws = L.nsa_cmp_attn_bwd_workspace_bytes(B, T, Tc, Hk, D)
+    ws = torch.full((nws,), 0x7f, dtype=torch.uint8, device=DEV)
+    opt = lambda *ts: [P(x) if x is not None else None for x in ts]
+    win = lambda dq, acc, dk, dv: L.nsa_sel_swa_bwd(
+        P(q), P(k), P(v), None, 0, None, None, None, None, None, P(do), P(lse[0]), P(delta[0]), P(g), P(dq), acc, *opt(dk, dv),
+        None, 0, B, T, Hq, Hk, D, 16, 64, window, scale, None)
+    cmp = lambda dq, acc, dk, dv: L.nsa_cmp_attn_bwd(
+        P(q), P(ck), P(cv), P(lse[1]), P(do), P(delta[1]), P(g), P(dq), acc, *opt(dk, dv), P(ws), nws, B, T, Tc, Hq, Hk, D, block,
+        stride, 1, scale, None)
+    for rc in (win(dq_w, 0, dk, dv), cmp(dq_c, 0, dck, dcv), win(both, 0, None, None), cmp(both, 1, None, None)):
+        nsa._lib.check(rc, "dense backward")
+    _close("dq window", dq_w, want[0][0])
+    _close("dq compressed", dq_c, want[1][0])
+    _close("dq accumulated", both, want[0][0] + want[1][0])
+    for name, x, ref in (("dk", dk, want[0][1]), ("dv", dv, want[0][2]), ("dck", dck, want[1][1]), ("dcv", dcv, want[1][2])):
+        _close(name, x, ref, scaled=True)
     nsa._lib.device_status()
