@@ -175,12 +175,15 @@ int nsa_sel_swa_bwd_ix(const void* q, const void* k, const void* v, const void* 
                        const void* gate_swa, void* dq, int accumulate_dq, void* dk, void* dv, void* ws, size_t ws_bytes, int B,
                        int T, int Hq, int Hkv, int D, int S, int BS, int window, float scale, int Tq, int q0, void* stream);
 /* The backward of all three branches for one upstream gradient (nsa_sel_swa_bwd_ix and nsa_cmp_attn_bwd with the gates of the
- * module's sum; delta_x = g_x * rowsum(o_x * dout)): the window's and the compressed branch's dQ are formed in one pass. */
+ * module's sum; delta_x = g_x * rowsum(o_x * dout)): the window's and the compressed branch's dQ are formed in one pass.
+ * With w_gate [3,D] (head_dim 128, 64-key blocks, S <= 32) dq also gets the gate projection's share sum_x dg_x W_x; nsa_gate_bwd
+ * with dq NULL then gives the rest of its backward. */
 size_t nsa_attn_bwd_ix_workspace_bytes(int B, int T, int Tc, int Hq, int Hkv, int D, int S, int BS, int window);
 int nsa_attn_bwd_ix(const void* q, const void* k, const void* v, const void* ck, const void* cv, const void* idx, int idx64,
                     const int32_t* counts, const void* index, const void* dout, const float* lse_slc, const float* lse_swa,
                     const float* lse_cmp, const float* delta_slc, const float* delta_swa, const float* delta_cmp,
-                    const void* g_slc, const void* g_swa, const void* g_cmp, void* dq, void* dk, void* dv, void* dck, void* dcv,
+                    const void* g_slc, const void* g_swa, const void* g_cmp, const void* dg_slc, const void* dg_swa,
+                    const void* dg_cmp, const void* w_gate, void* dq, void* dk, void* dv, void* dck, void* dcv,
                     void* ws, size_t ws_bytes, int B, int T, int Tc, int Hq, int Hkv, int D, int S, int BS, int window, int block,
                     int stride, int causal, float scale, void* stream);
 

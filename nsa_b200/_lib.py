@@ -50,7 +50,7 @@ SIGNATURES = {
     "nsa_sel_swa_fwd_ix_workspace_bytes": (Z, [I, I, I, I, I, I, I, I]),
     "nsa_sel_swa_bwd_ix_workspace_bytes": (Z, [I, I, I, I, I, I, I, I, I]),
     "nsa_attn_bwd_ix_workspace_bytes": (Z, [I, I, I, I, I, I, I, I, I]),
-    "nsa_attn_bwd_ix": (I, [P] * 6 + [I] + [P] * 18 + [Z] + [I] * 12 + [F, P]),
+    "nsa_attn_bwd_ix": (I, [P] * 6 + [I] + [P] * 22 + [Z] + [I] * 12 + [F, P]),
     "nsa_sel_swa_fwd_ix": (I, [P, P, P, P, I, P, P, P, P, P, P, P, P, P, P, P, P, Z, I, I, I, I, I, I, I, I, F, I, I, P]),
     "nsa_sel_swa_bwd_ix": (I, [P, P, P, P, I, P, P, P, P, P, P, P, P, P, P, P, I, P, P, P, Z, I, I, I, I, I, I, I, I, F, I, I, P]),
     "nsa_sel_swa_fwd_workspace_bytes": (Z, [I, I, I, I, I, I, I, I]),

@@ -492,13 +492,22 @@ static int sel_swa_fwd_impl(const void* q, const void* k, const void* v, const v
   int rc = check_attn_shape("nsa_sel_swa_fwd", B, T, Hq, Hkv, D);
   if (rc) return rc;
   cudaStream_t s = (cudaStream_t)stream;
-  if (o_slc) {
-    if (!idx || !lse_slc) return fail(-1, "nsa_sel_swa_fwd: idx / lse_slc is null");
+  if (window > 0) {   // first: the selected branch's merge adds it
+    if (!o_swa || !lse_swa) return fail(-1, "nsa_sel_swa_fwd: o_swa / lse_swa is null");
+    DenseArgs a = {};
+    a.mode = 0; a.q = (const bf16*)q; a.k = (const bf16*)k; a.v = (const bf16*)v; a.o = (bf16*)o_swa; a.lse = lse_swa;
+    a.B = B; a.T = T; a.Tq = Tq; a.q0 = q0; a.Lk = T; a.Hq = Hq; a.Hk = Hkv; a.window = window; a.scale = scale;
+    rc = launch_dense_fwd2_tc(a, D, s);
+    if (rc) return rc;
+  }
+  const bf16* swa = window > 0 ? (const bf16*)o_swa : nullptr;
+  if (o_slc || (o && index)) {   // (with an index of its own and a workspace a caller may leave out o_slc)
+    if (!idx) return fail(-1, "nsa_sel_swa_fwd: idx is null");
     rc = check_bs("nsa_sel_swa_fwd", BS);
     if (rc) return rc;
     if (S <= 0) return fail(-1, "nsa_sel_swa_fwd: no selected blocks");
     SelKvArgs ka = {};
-    ka.q = (const bf16*)q; ka.k = (const bf16*)k; ka.v = (const bf16*)v; ka.o = (bf16*)o_slc; ka.lse = lse_slc;
+    ka.q = (const bf16*)q; ka.k = (const bf16*)k; ka.v = (const bf16*)v; ka.merge.o = (bf16*)o_slc; ka.merge.lse = lse_slc;
     ka.B = B; ka.T = T; ka.Tq = Tq; ka.q0 = q0; ka.Hq = Hq; ka.Hk = Hkv; ka.S = S; ka.BS = BS; ka.scale = scale;
     if (ws && sel_fwd_kv_supported(ka, D) &&
         ws_bytes >= (index ? nsa_sel_swa_fwd_ix_workspace_bytes(B, T, Tq, Hq, Hkv, D, S, BS)
@@ -514,27 +523,20 @@ static int sel_swa_fwd_impl(const void* q, const void* k, const void* v, const v
         if (rc) return rc;
       }
       ka.rev_ptr = r.rev_ptr; ka.rev_tok = r.rev_tok; ka.rev_cap = r.cap;
-      rc = launch_sel_fwd_kv(ka, r, s);
-      if (rc) return rc;
-    } else {
-      SelArgs a = {};
-      a.q = (const bf16*)q; a.k = (const bf16*)k; a.v = (const bf16*)v; a.idx = idx; a.idx64 = idx64; a.counts = counts;
-      a.o = (bf16*)o_slc; a.lse = lse_slc; a.B = B; a.T = T; a.Tq = Tq; a.q0 = q0; a.Hq = Hq; a.Hkv = Hkv; a.S = S; a.BS = BS; a.scale = scale;
-      rc = launch_sel_fwd(a, D, s);
-      if (rc) return rc;
+      ka.merge.g0 = (const bf16*)g_slc; ka.merge.a1 = swa; ka.merge.g1 = (const bf16*)g_swa; ka.merge.a2 = (const bf16*)o_cmp;
+      ka.merge.g2 = (const bf16*)g_cmp; ka.merge.out = (bf16*)o;
+      return launch_sel_fwd_kv(ka, r, s);
     }
-  }
-  if (window > 0) {
-    if (!o_swa || !lse_swa) return fail(-1, "nsa_sel_swa_fwd: o_swa / lse_swa is null");
-    DenseArgs a = {};
-    a.mode = 0; a.q = (const bf16*)q; a.k = (const bf16*)k; a.v = (const bf16*)v; a.o = (bf16*)o_swa; a.lse = lse_swa;
-    a.B = B; a.T = T; a.Tq = Tq; a.q0 = q0; a.Lk = T; a.Hq = Hq; a.Hk = Hkv; a.window = window; a.scale = scale;
-    rc = launch_dense_fwd2_tc(a, D, s);
+    if (!o_slc || !lse_slc) return fail(-1, "nsa_sel_swa_fwd: o_slc / lse_slc is null");
+    SelArgs a = {};
+    a.q = (const bf16*)q; a.k = (const bf16*)k; a.v = (const bf16*)v; a.idx = idx; a.idx64 = idx64; a.counts = counts;
+    a.o = (bf16*)o_slc; a.lse = lse_slc; a.B = B; a.T = T; a.Tq = Tq; a.q0 = q0; a.Hq = Hq; a.Hkv = Hkv; a.S = S; a.BS = BS; a.scale = scale;
+    rc = launch_sel_fwd(a, D, s);
     if (rc) return rc;
   }
   if (o) {
-    rc = launch_combine((const bf16*)o_slc, (const bf16*)g_slc, window > 0 ? (const bf16*)o_swa : nullptr,
-                        (const bf16*)g_swa, (const bf16*)o_cmp, (const bf16*)g_cmp, (bf16*)o, (long long)B * Tq * Hq, D, s);
+    rc = launch_combine((const bf16*)o_slc, (const bf16*)g_slc, swa, (const bf16*)g_swa, (const bf16*)o_cmp, (const bf16*)g_cmp,
+                        (bf16*)o, (long long)B * Tq * Hq, D, s);
     if (rc) return rc;
   }
   return 0;
@@ -627,6 +629,7 @@ struct CmpBwd {   // the compressed branch in the same call: its dQ shares the w
   const float *lse, *delta;
   const void* gate;
   int Tc, block, stride, causal;
+  GateAdd add;   // the gate projection's share of dq (where dQ comes from the key-major kernel)
 };
 
 static int sel_swa_bwd_impl(const void* q, const void* k, const void* v, const void* idx, int idx64, const int32_t* counts,
@@ -770,7 +773,7 @@ static int sel_swa_bwd_impl(const void* q, const void* k, const void* v, const v
       }
     }
     if (dq_from_kv) {   // every token's partial tiles, in slot order, onto dq (after the window's dQ if that ran first)
-      rc = launch_sel_dq_reduce(r, tiles, (bf16*)dq, Hq, D, scale, dq_acc_for_reduce, s);
+      rc = launch_sel_dq_reduce(r, tiles, (bf16*)dq, Hq, D, cmp ? cmp->add : GateAdd{}, scale, dq_acc_for_reduce, s);
       if (rc) return rc;
     }
   }
@@ -804,7 +807,8 @@ int nsa_sel_swa_bwd_ix(const void* q, const void* k, const void* v, const void* 
 int nsa_attn_bwd_ix(const void* q, const void* k, const void* v, const void* ck, const void* cv, const void* idx, int idx64,
                     const int32_t* counts, const void* index, const void* dout, const float* lse_slc, const float* lse_swa,
                     const float* lse_cmp, const float* delta_slc, const float* delta_swa, const float* delta_cmp,
-                    const void* g_slc, const void* g_swa, const void* g_cmp, void* dq, void* dk, void* dv, void* dck, void* dcv,
+                    const void* g_slc, const void* g_swa, const void* g_cmp, const void* dg_slc, const void* dg_swa,
+                    const void* dg_cmp, const void* w_gate, void* dq, void* dk, void* dv, void* dck, void* dcv,
                     void* ws, size_t ws_bytes, int B, int T, int Tc, int Hq, int Hkv, int D, int S, int BS, int window, int block,
                     int stride, int causal, float scale, void* stream) {
   if (!ck || !cv || !lse_cmp || !dout || !delta_cmp || !dq || !dk || !dv || !dck || !dcv || !idx || !index || !ws)
@@ -812,7 +816,10 @@ int nsa_attn_bwd_ix(const void* q, const void* k, const void* v, const void* ck,
   if (Tc <= 0) return fail(-1, "nsa_attn_bwd_ix: no compressed position");
   if (ws_bytes < nsa_attn_bwd_ix_workspace_bytes(B, T, Tc, Hq, Hkv, D, S, BS, window))
     return fail(-6, "nsa_attn_bwd_ix: workspace too small");
-  const CmpBwd c = {ck, cv, lse_cmp, delta_cmp, g_cmp, Tc, block, stride, causal};
+  if (w_gate && (!dq_from_kv_covers(D, S, BS) || !dg_slc || !dg_swa || !dg_cmp))
+    return fail(-1, "nsa_attn_bwd_ix: the gate projection's share needs its gradients, head_dim 128 and 64-key blocks");
+  const CmpBwd c = {ck, cv, lse_cmp, delta_cmp, g_cmp, Tc, block, stride, causal,
+                    {{(const bf16*)dg_slc, (const bf16*)dg_swa, (const bf16*)dg_cmp}, (const bf16*)w_gate}};
   int rc = sel_swa_bwd_impl(q, k, v, idx, idx64, counts, dout, lse_slc, delta_slc, g_slc, window > 0 ? dout : nullptr, lse_swa, delta_swa, g_swa, dq, 0, dk, dv, ws, ws_bytes, B, T, Hq, Hkv, D, S, BS, window, scale, T, 0, stream, nullptr, index, &c);
   if (rc) return rc;
   return cmp_dkv(q, ck, cv, lse_cmp, dout, delta_cmp, g_cmp, dck, dcv, ws, B, T, Tc, Hq, Hkv, D, block, stride, causal, scale, T, 0, (cudaStream_t)stream);
@@ -895,7 +902,7 @@ long long nsa_gate_bwd_workspace_bytes(long long rows, int D) { return gate_bwd_
 
 int nsa_gate_bwd(const void* q, const void* dg_slc, const void* dg_swa, const void* dg_cmp, const void* w, void* dq,
                  void* dw, void* dbias, void* workspace, long long workspace_bytes, long long rows, int D, void* stream) {
-  if (!q || !dg_slc || !dg_swa || !dg_cmp || !w || !dq || !dw || !workspace) return fail(-1, "nsa_gate_bwd: null pointer");
+  if (!q || !dg_slc || !dg_swa || !dg_cmp || !w || !dw || !workspace) return fail(-1, "nsa_gate_bwd: null pointer");
   if (workspace_bytes < gate_bwd_workspace_bytes(rows, D)) return fail(-3, "nsa_gate_bwd: workspace too small");
   return launch_gate_bwd((const bf16*)q, (const bf16*)dg_slc, (const bf16*)dg_swa, (const bf16*)dg_cmp, (const bf16*)w,
                          (bf16*)dq, (bf16*)dw, (bf16*)dbias, (float*)workspace, rows, D, (cudaStream_t)stream);

@@ -104,59 +104,13 @@ struct Rowdot3Args {
   long long rows;
 };
 
+// (parallel_nsa_bwd_kernel_preprocess, nsa/selection_attn.py:520-530; _attn_bwd_preprocess, nsa/triton_attention.py:184-199; the
+// gate gradients of nsa/nsa.py:133 and nsa/selection_attn.py:808-811.)
+// One row per group of D/8 lanes and one block per 256 / (D/8) rows (no grid-stride loop): few registers, so many small blocks
+// are resident and the memory system sees the access pattern of the combine kernel.  Measured against a persistent form at
+// 4.2 M rows: 0.69 against 1.05 ms (6.25 against 4.1 TB/s); against a warp per row with one branch, 0.5 M rows: 71 -> 53 us.
 template <int D>
-__global__ void __launch_bounds__(kGateThreads) rowdot3_kernel(const Rowdot3Args a) {
-  constexpr int LPR = D / 8, RPW = 32 / LPR;
-  const int lane = threadIdx.x & 31, sub = lane % LPR, rw = lane / LPR;
-  const long long warp0 = (long long)blockIdx.x * (kGateThreads / 32) + (threadIdx.x >> 5);
-  const long long nwarp = (long long)gridDim.x * (kGateThreads / 32);
-  constexpr int U = 4;   // rows in flight per lane (x 4 tensors, raw 16-byte loads)
-  for (long long r0 = warp0 * RPW * U; r0 < a.rows; r0 += nwarp * RPW * U) {
-    uint4 draw[U], vraw[U][3];
-    float gv[U][3];   // the gates are fetched with the rows, not after the reductions that need them
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const long long row = r0 + u * RPW + rw;
-      const bool live = row < a.rows;
-      draw[u] = make_uint4(0u, 0u, 0u, 0u);
-      if (live) draw[u] = ldraw(a.dout + row * D + sub * 8);
-#pragma unroll
-      for (int x = 0; x < 3; ++x) {
-        vraw[u][x] = make_uint4(0u, 0u, 0u, 0u);
-        gv[u][x] = 1.f;
-        if (live && a.o[x]) vraw[u][x] = ldraw(a.o[x] + row * D + sub * 8);
-        if (live && sub == 0 && a.o[x] && a.gate[x]) gv[u][x] = __bfloat162float(a.gate[x][row]);
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const long long row = r0 + u * RPW + rw;
-      const bool live = row < a.rows;
-      float du[8];
-      cvt8(draw[u], du);
-#pragma unroll
-      for (int x = 0; x < 3; ++x) {
-        if (!a.o[x]) continue;   // uniform
-        float vu[8];
-        cvt8(vraw[u][x], vu);
-        float s = 0.f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) s += vu[k] * du[k];
-        s = group_sum<LPR>(s);
-        if (live && sub == 0) {
-          if (a.delta[x]) a.delta[x][row] = s * gv[u][x];
-          if (a.dgate[x]) a.dgate[x][row] = __float2bfloat16(s);
-        }
-      }
-    }
-  }
-}
-
-// The same pre-pass with one row per group of D/8 lanes and one block per 256 / (D/8) rows (no grid-stride loop): few
-// registers, so many small blocks are resident and the memory system sees the access pattern of the combine kernel.
-// Measured against the persistent form above at 4.2 M rows: 0.69 against 1.05 ms (6.25 against 4.1 TB/s).
-template <int D>
-__global__ void __launch_bounds__(256) rowdot3_flat_kernel(const Rowdot3Args a) {
+__global__ void __launch_bounds__(256) rowdot3_kernel(const Rowdot3Args a) {
   constexpr int LPR = D / 8;
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   const long long row = i / LPR;
@@ -189,8 +143,8 @@ __global__ void __launch_bounds__(256) rowdot3_flat_kernel(const Rowdot3Args a) 
   }
 }
 
-// dq[row] += sum_g dg_g[row] * W[g];  per-block partials of dW[g] = sum_rows dg_g[row] * q[row] and db[g] = sum_rows dg_g
-template <int D>
+// (DQ) dq[row] += sum_g dg_g[row] * W[g];  per-block partials of dW[g] = sum_rows dg_g[row] * q[row] and db[g] = sum_rows dg_g
+template <int D, bool DQ>
 __global__ void __launch_bounds__(kGateThreads, 2) gate_bwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ dg0,
                                                                const bf16* __restrict__ dg1, const bf16* __restrict__ dg2,
                                                                const bf16* __restrict__ w, bf16* __restrict__ dq,
@@ -219,7 +173,7 @@ __global__ void __launch_bounds__(kGateThreads, 2) gate_bwd_kernel(const bf16* _
       g[u][0] = g[u][1] = g[u][2] = 0.f;
       if (row < rows) {
         xraw[u] = ldraw(q + row * D + sub * 8);
-        yraw[u] = ldraw(dq + row * D + sub * 8);
+        if (DQ) yraw[u] = ldraw(dq + row * D + sub * 8);
         g[u][0] = __bfloat162float(dg0[row]);
         g[u][1] = __bfloat162float(dg1[row]);
         g[u][2] = __bfloat162float(dg2[row]);
@@ -233,7 +187,7 @@ __global__ void __launch_bounds__(kGateThreads, 2) gate_bwd_kernel(const bf16* _
       cvt8(yraw[u], yu);
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        yu[k] += g[u][0] * wv[0][k] + g[u][1] * wv[1][k] + g[u][2] * wv[2][k];
+        if (DQ) yu[k] += g[u][0] * wv[0][k] + g[u][1] * wv[1][k] + g[u][2] * wv[2][k];
 #pragma unroll
         for (int gg = 0; gg < 3; ++gg) dwacc[gg][k] += g[u][gg] * xu[k];
       }
@@ -241,7 +195,7 @@ __global__ void __launch_bounds__(kGateThreads, 2) gate_bwd_kernel(const bf16* _
 #pragma unroll
         for (int gg = 0; gg < 3; ++gg) dbacc[gg] += g[u][gg];
       }
-      if (row < rows) {
+      if (DQ && row < rows) {
         uint4 out;
         __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&out);
 #pragma unroll
@@ -336,9 +290,9 @@ int launch_rowdot3(const bf16* const o[3], const bf16* dout, const bf16* const g
   a.dout = dout;
   a.rows = rows;
   if (D == 128)
-    rowdot3_flat_kernel<128><<<(unsigned)((rows * 16 + 255) / 256), 256, 0, s>>>(a);
+    rowdot3_kernel<128><<<(unsigned)((rows * 16 + 255) / 256), 256, 0, s>>>(a);
   else if (D == 64)
-    rowdot3_kernel<64><<<stream_grid(rowdot3_kernel<64>, rows, 32), kGateThreads, 0, s>>>(a);
+    rowdot3_kernel<64><<<(unsigned)((rows * 8 + 255) / 256), 256, 0, s>>>(a);
   else {
     set_error("head_dim %d not supported (64 or 128)", D);
     return -2;
@@ -349,7 +303,7 @@ int launch_rowdot3(const bf16* const o[3], const bf16* dout, const bf16* const g
 
 // workspace: one partial of 3*D+4 floats per block
 static int gate_bwd_grid(long long rows, int D) {
-  return D == 128 ? stream_grid(gate_bwd_kernel<128>, rows, 16) : stream_grid(gate_bwd_kernel<64>, rows, 32);
+  return D == 128 ? stream_grid(gate_bwd_kernel<128, true>, rows, 16) : stream_grid(gate_bwd_kernel<64, true>, rows, 32);
 }
 
 long long gate_bwd_workspace_bytes(long long rows, int D) {
@@ -362,9 +316,9 @@ int launch_gate_bwd(const bf16* q, const bf16* dg0, const bf16* dg1, const bf16*
   if (rows <= 0) return 0;
   const int grid = gate_bwd_grid(rows, D);
   if (D == 128)
-    gate_bwd_kernel<128><<<grid, kGateThreads, 0, s>>>(q, dg0, dg1, dg2, w, dq, workspace, rows);
+    (dq ? gate_bwd_kernel<128, true> : gate_bwd_kernel<128, false>)<<<grid, kGateThreads, 0, s>>>(q, dg0, dg1, dg2, w, dq, workspace, rows);
   else if (D == 64)
-    gate_bwd_kernel<64><<<grid, kGateThreads, 0, s>>>(q, dg0, dg1, dg2, w, dq, workspace, rows);
+    (dq ? gate_bwd_kernel<64, true> : gate_bwd_kernel<64, false>)<<<grid, kGateThreads, 0, s>>>(q, dg0, dg1, dg2, w, dq, workspace, rows);
   else {
     set_error("head_dim %d not supported (64 or 128)", D);
     return -2;

@@ -363,12 +363,18 @@ __device__ __forceinline__ int rev_block(const RevArgs& a, long long row, int s,
 // Selected attention forward, key-major (sel_fwd_kv_tc.cu): one CTA per 64-key block, the queries that selected it in
 // batches of 8 tokens x 16 heads from the reverse index; per visit a [16 x D] bf16 tile of unnormalised output and
 // (max, sum) per row, merged per token in slot order by a second kernel.
+// The merge also forms the gated sum of the branches while a row is in registers (each of g0, (a1, g1), (a2, g2) may be null).
+struct SelMerge {
+  bf16* o;              // [B,Tq,Hq,D], or null
+  float* lse;           // [B,Tq,Hq] natural log, or null
+  const bf16 *g0, *a1, *g1, *a2, *g2;
+  bf16* out;            // g0 o + g1 a1 + g2 a2, or null
+};
 struct SelKvArgs {
   const bf16* q;        // [B,Tq,Hq,D]
   const bf16* k;        // [B,T,Hk,D]
   const bf16* v;
-  bf16* o;              // [B,Tq,Hq,D]
-  float* lse;           // [B,Tq,Hq] natural log
+  SelMerge merge;
   const int* rev_ptr;   // reverse index (launch_build_rev, with inv)
   const int* rev_tok;
   long long rev_cap;
@@ -380,10 +386,14 @@ struct SelKvArgs {
 bool sel_fwd_kv_supported(const SelKvArgs& a, int D);
 int launch_sel_fwd_kv(const SelKvArgs& a, const RevArgs& r, cudaStream_t s);
 int sel_fwd_kv_status(int* out);
-// dq[(b,t), 16-head group] (+)= scale * sum over the valid slots s of part[(b,h) list position inv[row,s]] (fixed slot
+struct GateAdd {
+  const bf16* dg[3];    // gradients of the gates [B,Tq,Hq]
+  const bf16* w;        // gate projection [3,D], or null: nothing to add
+};
+// dq[(b,t), 16-head group] (+)= sum_g dg_g W_g + scale * sum over the valid slots s of part[(b,h) list position inv[row,s]] (fixed slot
 // order).  part holds one [16 heads x D] bf16 tile per (list position, 16-head sub-group), written by the kv-major
 // backward; dq rows of a (token, group) are the same contiguous tile.
-int launch_sel_dq_reduce(const RevArgs& a, const bf16* part, bf16* dq, int Hq, int D, float scale, int accumulate,
+int launch_sel_dq_reduce(const RevArgs& a, const bf16* part, bf16* dq, int Hq, int D, const GateAdd& gate, float scale, int accumulate,
                          cudaStream_t s);
 // dk, dv (bf16) = sum over the slabs of part [2][nslab][n]
 int launch_reduce_shares(const float* part, bf16* dk, bf16* dv, int nslab, long long n, cudaStream_t s);

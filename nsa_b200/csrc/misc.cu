@@ -19,34 +19,6 @@ int num_sms() {
 
 namespace {
 
-// ---- delta / gate gradient ------------------------------------------------------------------------
-// Reference: parallel_nsa_bwd_kernel_preprocess (nsa/selection_attn.py:520-530), _attn_bwd_preprocess
-// (nsa/triton_attention.py:184-199) and the autograd of the gate products (nsa/nsa.py:133,
-// nsa/selection_attn.py:808-811).  One warp per (token, head) row.
-template <int D>
-__global__ void rowdot_kernel(const bf16* __restrict__ o, const bf16* __restrict__ dout, const bf16* __restrict__ gate,
-                              float* __restrict__ delta, bf16* __restrict__ dgate, long long rows) {
-  const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (row >= rows) return;
-  const int lane = threadIdx.x & 31;
-  constexpr int PER = D / 32;  // 2 or 4 elements per lane
-  float acc = 0.f;
-  const bf16* po = o + row * D + lane * PER;
-  const bf16* pd = dout + row * D + lane * PER;
-#pragma unroll
-  for (int i = 0; i < PER; i += 2) {
-    const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(po + i));
-    const float2 y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(pd + i));
-    acc += x.x * y.x + x.y * y.y;
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-  if (lane == 0) {
-    if (delta) delta[row] = gate ? acc * __bfloat162float(gate[row]) : acc;
-    if (dgate) dgate[row] = __float2bfloat16(acc);
-  }
-}
-
 // ---- gated combine ------------------------------------------------------------------------------------
 // o = g0*a0 + g1*a1 + g2*a2  (nsa/selection_attn.py:808-811 and nsa/nsa.py:133, as one pass)
 __global__ void combine_kernel(const bf16* __restrict__ a0, const bf16* __restrict__ g0, const bf16* __restrict__ a1,
@@ -243,19 +215,11 @@ int launch_reduce_shares(const float* part, bf16* dk, bf16* dv, int nshare, long
 
 int launch_rowdot(const bf16* o, const bf16* dout, const bf16* gate, float* delta, bf16* dgate, long long rows, int D,
                   cudaStream_t s) {
-  if (rows <= 0) return 0;
-  const int wpb = 8;
-  const unsigned grid = (unsigned)((rows + wpb - 1) / wpb);
-  if (D == 128)
-    rowdot_kernel<128><<<grid, wpb * 32, 0, s>>>(o, dout, gate, delta, dgate, rows);
-  else if (D == 64)
-    rowdot_kernel<64><<<grid, wpb * 32, 0, s>>>(o, dout, gate, delta, dgate, rows);
-  else {
-    set_error("head_dim %d not supported (64 or 128)", D);
-    return -2;
-  }
-  note_launches(1);
-  return (int)cudaGetLastError();
+  const bf16* o3[3] = {o, nullptr, nullptr};
+  const bf16* g3[3] = {gate, nullptr, nullptr};
+  float* d3[3] = {delta, nullptr, nullptr};
+  bf16* dg3[3] = {dgate, nullptr, nullptr};
+  return launch_rowdot3(o3, dout, g3, d3, dg3, rows, D, s);
 }
 
 int launch_combine(const bf16* a0, const bf16* g0, const bf16* a1, const bf16* g1, const bf16* a2, const bf16* g2,
@@ -271,17 +235,20 @@ int launch_combine(const bf16* a0, const bf16* g0, const bf16* a1, const bf16* g
   return (int)cudaGetLastError();
 }
 
-// Two warps per (batch, token, 16-head group), each half of the [16 x D] bf16 tile (heads 0-7 / 8-15): the token's
-// visits are added in slot order.  A load instruction of the warp covers 512 contiguous bytes; the list positions of
-// all slots are fetched first so that the tiles of several slots are in flight at once.
+// Four warps per (batch, token, 16-head group), each four heads of the [16 x D] bf16 tile: the token's visits are added in slot
+// order.  A load instruction of the warp covers 512 contiguous bytes; the list positions of all slots are fetched first so
+// that the tiles of several slots are in flight at once (four heads instead of eight per warp: half the registers, twice the
+// warps).  The gate projection's share of dq (sum_g dg_g W_g) can be added on the way: dq is in registers here, a pass of its
+// own reads and writes it once more.
 template <int D>
 __global__ void __launch_bounds__(256) sel_dq_reduce_kernel(const RevArgs a, const bf16* __restrict__ part, bf16* __restrict__ dq,
-                                                            const int G16, const float scale, const int accumulate) {
-  const long long w2 = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+                                                            const GateAdd gate, const int G16, const float scale, const int accumulate) {
+  constexpr int kHeads = 4, kWarps = 16 / kHeads;
+  const long long w4 = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   const long long total = (long long)a.B * a.Tq * a.H * G16;
-  const long long w = w2 >> 1;
+  const long long w = w4 / kWarps;
   if (w >= total) return;
-  const int hb = (int)(w2 & 1);                        // which half of the tile
+  const int hb = (int)(w4 % kWarps);                   // which heads of the tile
   const int lane = threadIdx.x & 31;
   const int sub = (int)(w % G16);
   const long long row = w / G16;                       // (b, tl, h) row of idx / counts
@@ -289,22 +256,41 @@ __global__ void __launch_bounds__(256) sel_dq_reduce_kernel(const RevArgs a, con
   const long long bt = row / a.H;
   const int tl = (int)(bt % a.Tq), b = (int)(bt / a.Tq);
   const int t = a.q0 + tl;
-  constexpr int NV = 8 * D / 8 / 32;                   // 16-byte vectors per lane: 4 at D = 128
+  constexpr int NV = kHeads * D / 8 / 32;              // 16-byte vectors per lane: 2 at D = 128
+  const long long bh = (long long)b * a.H + h;
+  // lane s holds the list position of slot s (or -1): the same validity rule that built the lists
+  int mypos = -1;
+  if (lane < a.S && rev_block(a, row, lane, t) >= 0) mypos = a.inv[row * a.S + lane];
+  const int Hq = a.H * G16 * 16;
+  const long long row0 = bt * Hq + (long long)(h * G16 + sub) * 16 + hb * kHeads;
+  // the partial tiles keep the staging layout of the kernel that wrote them: within a 128-byte half row the 16-byte
+  // chunk c sits at position c ^ (head & 7).  All tiles share it, so the sum is formed in place and undone at the end:
+  // vector u = 32 i + lane of this part of the tile is its row u / 16, position u % 8.
+  uint4* dst = reinterpret_cast<uint4*>(dq + row0 * D);
+  int ud[NV];
+  uint4 prev[NV];
+  bf16 dg[NV][3];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int u = 32 * i + lane, r = u >> 4;
+    ud[i] = (u & ~7) | ((u & 7) ^ ((hb * kHeads + r) & 7));
+    prev[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (accumulate) prev[i] = __ldcs(dst + ud[i]);
+#pragma unroll
+    for (int g = 0; g < 3; ++g)
+      if (gate.w) dg[i][g] = gate.dg[g][row0 + r];
+  }
+  unsigned live = __ballot_sync(0xffffffffu, mypos >= 0);
+  const uint4* base = reinterpret_cast<const uint4*>(part) + hb * (kHeads * D / 8) + lane;
+  auto tile = [&](int s) {
+    const long long pos = __shfl_sync(0xffffffffu, mypos, s);
+    return base + ((bh * a.cap + pos) * G16 + sub) * (16 * D / 8);
+  };
   float acc[NV][8];
 #pragma unroll
   for (int i = 0; i < NV; ++i)
 #pragma unroll
     for (int k = 0; k < 8; ++k) acc[i][k] = 0.f;
-  const long long bh = (long long)b * a.H + h;
-  // lane s holds the list position of slot s (or -1): the same validity rule that built the lists
-  int mypos = -1;
-  if (lane < a.S && rev_block(a, row, lane, t) >= 0) mypos = a.inv[row * a.S + lane];
-  unsigned live = __ballot_sync(0xffffffffu, mypos >= 0);
-  const uint4* base = reinterpret_cast<const uint4*>(part) + hb * (8 * D / 8) + lane;
-  auto tile = [&](int s) {
-    const long long pos = __shfl_sync(0xffffffffu, mypos, s);
-    return base + ((bh * a.cap + pos) * G16 + sub) * (16 * D / 8);
-  };
   auto add = [&](const uint4 (&v)[NV]) {
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
@@ -334,36 +320,34 @@ __global__ void __launch_bounds__(256) sel_dq_reduce_kernel(const RevArgs a, con
     add(v0);
     if (s1 >= 0) add(v1);
   }
-  const int Hq = a.H * G16 * 16;
-  // the partial tiles keep the staging layout of the kernel that wrote them: within a 128-byte half row the 16-byte
-  // chunk c sits at position c ^ (head & 7).  All tiles share it, so the sum is formed in place and undone here:
-  // vector u = 32 i + lane of this half tile is row u / 16, position u % 8.
-  uint4* dst = reinterpret_cast<uint4*>(dq + ((bt * Hq) + (long long)(h * G16 + sub) * 16) * D) + hb * (8 * D / 8);
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
-    float prev[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    const int u = 32 * i + lane;
-    const int ud = (u & ~7) | ((u & 7) ^ ((u >> 4) & 7));
-    if (accumulate) {
-      const uint4 v = dst[ud];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) acc[i][k] *= scale;
+    auto add8 = [&](const uint4& v, float g) {
       const __nv_bfloat162* hv = reinterpret_cast<const __nv_bfloat162*>(&v);
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const float2 f = __bfloat1622float2(hv[k]);
-        prev[2 * k] = f.x;
-        prev[2 * k + 1] = f.y;
+        acc[i][2 * k] = fmaf(g, f.x, acc[i][2 * k]);
+        acc[i][2 * k + 1] = fmaf(g, f.y, acc[i][2 * k + 1]);
       }
+    };
+    add8(prev[i], 1.f);
+    if (gate.w) {
+#pragma unroll
+      for (int g = 0; g < 3; ++g)
+        add8(__ldg(reinterpret_cast<const uint4*>(gate.w + g * D) + (ud[i] & 15)), __bfloat162float(dg[i][g]));
     }
     uint4 o;
     __nv_bfloat162* ho = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
-      ho[k] = __floats2bfloat162_rn(fmaf(acc[i][2 * k], scale, prev[2 * k]), fmaf(acc[i][2 * k + 1], scale, prev[2 * k + 1]));
-    dst[ud] = o;
+    for (int k = 0; k < 4; ++k) ho[k] = __floats2bfloat162_rn(acc[i][2 * k], acc[i][2 * k + 1]);
+    dst[ud[i]] = o;
   }
 }
 
-int launch_sel_dq_reduce(const RevArgs& a, const bf16* part, bf16* dq, int Hq, int D, float scale, int accumulate,
+int launch_sel_dq_reduce(const RevArgs& a, const bf16* part, bf16* dq, int Hq, int D, const GateAdd& gate, float scale, int accumulate,
                          cudaStream_t s) {
   if (D != 128) {
     set_error("selected dQ reduction: head_dim 128 only");
@@ -376,7 +360,7 @@ int launch_sel_dq_reduce(const RevArgs& a, const bf16* part, bf16* dq, int Hq, i
     set_error("selected dQ reduction: at most 32 selected blocks per token");
     return -2;
   }
-  sel_dq_reduce_kernel<128><<<(unsigned)((2 * total + 7) / 8), 256, 0, s>>>(a, part, dq, G16, scale, accumulate);
+  sel_dq_reduce_kernel<128><<<(unsigned)((4 * total + 7) / 8), 256, 0, s>>>(a, part, dq, gate, G16, scale, accumulate);
   note_launches(1);
   return (int)cudaGetLastError();
 }

@@ -333,18 +333,22 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (warp == kMmaWarp) tmem_dealloc(tmem, kTmemCols);
 }
 
-// Two warps per (batch, token, 16-head group), each half of the 16 heads: the visits' (m, l) and O tiles merged in slot
-// order.  Lanes 0-7 hold the statistics of this half's heads; a load instruction of the warp covers 512 contiguous
-// bytes of a tile.
+// Two warps per (batch, token, 16-head group), each eight of the 16 heads: the visits' (m, l) and O tiles merged in slot order,
+// and the gated sum of the branches.  A load instruction of the warp covers 512 contiguous bytes of a tile.  Bound by reading
+// the tiles, so by what a warp has in flight per register: the first tile and the gates are fetched ahead of the maxima.
+// All slots visible, 4 x 8192 tokens, 64 heads: 1.50 ms with the gate (6.5 TB/s; 1.45 + 0.64 as two passes); half visible,
+// 8 x 8192 tokens, three branches: 2.32 (1.85 + 0.73).  Four heads per warp and two tiles in flight 1.67 and 2.53; two tiles
+// of eight heads 1.62 and 2.73; four of four 1.89 and 3.26 (too few warps).
+constexpr int kMergeHeads = 8, kMergeWarps = 16 / kMergeHeads;
+template <bool SUM>
 __global__ void __launch_bounds__(256) sel_fwd_merge_kernel(const RevArgs a, const bf16* __restrict__ part,
-                                                            const float* __restrict__ stats, bf16* __restrict__ o,
-                                                            float* __restrict__ lse, const int G16) {
-  constexpr int NV = 8 * D / 8 / 32;   // 16-byte vectors per lane: 4
-  const long long w2 = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+                                                            const float* __restrict__ stats, const SelMerge m, const int G16) {
+  constexpr int NV = kMergeHeads * D / 8 / 32;   // 16-byte vectors per lane: 4
+  const long long w4 = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   const long long total = (long long)a.B * a.Tq * a.H * G16;
-  const long long w = w2 >> 1;
+  const long long w = w4 / kMergeWarps;
   if (w >= total) return;
-  const int hb = (int)(w2 & 1);
+  const int hb = (int)(w4 % kMergeWarps);
   const int lane = threadIdx.x & 31;
   const int sub = (int)(w % G16);
   const long long row = w / G16;   // (b, tl, h) row of idx / counts
@@ -355,52 +359,72 @@ __global__ void __launch_bounds__(256) sel_fwd_merge_kernel(const RevArgs a, con
   const long long bh = (long long)b * a.H + h;
   int mypos = -1;
   if (lane < a.S && rev_block(a, row, lane, t) >= 0) mypos = a.inv[row * a.S + lane];
+  const int Hq = a.H * G16 * 16;
+  const long long orow0 = bt * Hq + (long long)(h * G16 + sub) * 16;   // first of the group's 16 (token, head) rows
+  const int myhead = hb * kMergeHeads + lane % kMergeHeads;
+  // vector u = 32 i + lane of this part of the tile belongs to head u / 16 = 2 i + lane / 16 (of this warp's); the staging layout
+  // swizzles a tile's 16-byte chunks by its row
+  int ud[NV];
+  const long long vec0 = orow0 * (D / 8) + hb * (kMergeHeads * D / 8);
+  bf16 graw[3];   // gates of head lane % 8
+#pragma unroll
+  for (int x = 0; x < 3; ++x) graw[x] = __float2bfloat16(1.f);
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int u = 32 * i + lane;
+    ud[i] = ((u & ~7) | ((u & 7) ^ ((hb * kMergeHeads + (u >> 4)) & 7)));
+  }
+  if (SUM && m.g0) graw[0] = m.g0[orow0 + myhead];
+  if (SUM && m.g1) graw[1] = m.g1[orow0 + myhead];
+  if (SUM && m.g2) graw[2] = m.g2[orow0 + myhead];
   const unsigned live = __ballot_sync(0xffffffffu, mypos >= 0);
   auto tile_index = [&](int s) {
     const long long pos = __shfl_sync(0xffffffffu, mypos, s);
     return (bh * a.cap + pos) * G16 + sub;
   };
-  // pass 1: M = max_v m_v per head.  Lane s fetches the maxima of slot s for this half's eight heads (all slots at
-  // once, instead of one dependent load per slot), a butterfly takes the maximum over the slots, and every lane keeps
-  // the value of head lane & 7, the head whose (m, l) it reads in pass 2.
-  const int myhead = hb * 8 + (lane & 7);
-  float mh[8];
+  const uint4* base = reinterpret_cast<const uint4*>(part) + hb * (kMergeHeads * D / 8) + lane;
+  unsigned rem = live;
+  uint4 v[NV];
+  float2 ml;
+  auto fetch = [&]() {   // the next slot's tile and (m, l)
+    const long long ti = tile_index(__ffs(rem) - 1);
+    rem &= rem - 1;
+    ml = reinterpret_cast<const float2*>(stats)[ti * 16 + myhead];
 #pragma unroll
-  for (int e = 0; e < 8; ++e) mh[e] = -INFINITY;
+    for (int i = 0; i < NV; ++i) v[i] = __ldcs(base + ti * (16 * D / 8) + 32 * i);
+  };
+  if (live) fetch();
+  // pass 1: M = max_v m_v per head.  Lane s fetches the maxima of slot s for this warp's heads (all slots at once, instead of
+  // one dependent load per slot), a butterfly takes the maximum over the slots, and every lane keeps the value of head
+  // lane % 8, the head whose (m, l) it reads in pass 2.
+  float mh[kMergeHeads];
+#pragma unroll
+  for (int e = 0; e < kMergeHeads; ++e) mh[e] = -INFINITY;
   if (mypos >= 0) {
-    const float4* sp = reinterpret_cast<const float4*>(stats) + (((bh * a.cap + mypos) * G16 + sub) * 16 + hb * 8) / 2;
+    const float4* sp = reinterpret_cast<const float4*>(stats) + (((bh * a.cap + mypos) * G16 + sub) * 16 + hb * kMergeHeads) / 2;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
+    for (int e = 0; e < kMergeHeads / 2; ++e) {
       const float4 v4 = sp[e];   // (m, l) of two heads
       mh[2 * e] = v4.x;
       mh[2 * e + 1] = v4.z;
     }
   }
 #pragma unroll
-  for (int e = 0; e < 8; ++e)
+  for (int e = 0; e < kMergeHeads; ++e)
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) mh[e] = fmaxf(mh[e], __shfl_xor_sync(0xffffffffu, mh[e], off));
   float M = mh[0];
 #pragma unroll
-  for (int e = 1; e < 8; ++e) M = ((lane & 7) == e) ? mh[e] : M;
+  for (int e = 1; e < kMergeHeads; ++e) M = (lane % kMergeHeads == e) ? mh[e] : M;
   float L = 0.f;
   float acc[NV][8];
 #pragma unroll
   for (int i = 0; i < NV; ++i)
 #pragma unroll
     for (int k = 0; k < 8; ++k) acc[i][k] = 0.f;
-  // vector u = 32 i + lane of this half tile belongs to head u / 16 = 2 i + lane / 16 (of this half)
-  for (unsigned rem = live; rem;) {
-    const int s = __ffs(rem) - 1;
-    rem &= rem - 1;
-    const long long ti = tile_index(s);
-    const float2 ml = reinterpret_cast<const float2*>(stats)[ti * 16 + myhead];
-    const float wgt = ex2(ml.x - M);   // lanes 0-7 (and their copies 8-31) hold head lane & 7
+  for (bool more = live != 0; more;) {
+    const float wgt = ex2(ml.x - M);   // lanes 0-7 (and their copies): own head
     L += wgt * ml.y;
-    const uint4* src = reinterpret_cast<const uint4*>(part) + ti * (16 * D / 8) + hb * (8 * D / 8) + lane;
-    uint4 v[NV];
-#pragma unroll
-    for (int i = 0; i < NV; ++i) v[i] = __ldcs(src + 32 * i);
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const float wi = __shfl_sync(0xffffffffu, wgt, 2 * i + (lane >> 4));
@@ -412,22 +436,36 @@ __global__ void __launch_bounds__(256) sel_fwd_merge_kernel(const RevArgs a, con
         acc[i][2 * k + 1] = fmaf(wi, f.y, acc[i][2 * k + 1]);
       }
     }
+    more = rem != 0;
+    if (more) fetch();
   }
-  const int Hq = a.H * G16 * 16;
-  const long long orow0 = bt * Hq + (long long)(h * G16 + sub) * 16;   // first of the group's 16 (token, head) rows
   const float inv = L > 0.f ? 1.f / L : 0.f;
-  if (lane < 8) lse[orow0 + myhead] = L > 0.f ? (M + log2f(L)) * 0.6931471805599453f : -INFINITY;
-  uint4* dst = reinterpret_cast<uint4*>(o + orow0 * D) + hb * (8 * D / 8);
+  if (m.lse && lane < kMergeHeads) m.lse[orow0 + myhead] = L > 0.f ? (M + log2f(L)) * 0.6931471805599453f : -INFINITY;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
-    const float ii = __shfl_sync(0xffffffffu, inv, 2 * i + (lane >> 4));
-    const int u = 32 * i + lane;
-    const int ud = (u & ~7) | ((u & 7) ^ ((u >> 4) & 7));   // undo the staging layout: position -> chunk
+    const int hl = 2 * i + (lane >> 4);
+    const float ii = __shfl_sync(0xffffffffu, inv, hl);
     uint4 ov;
     __nv_bfloat162* ho = reinterpret_cast<__nv_bfloat162*>(&ov);
 #pragma unroll
     for (int k = 0; k < 4; ++k) ho[k] = __floats2bfloat162_rn(acc[i][2 * k] * ii, acc[i][2 * k + 1] * ii);
-    dst[ud] = ov;
+    if (m.o) reinterpret_cast<uint4*>(m.o)[vec0 + ud[i]] = ov;
+    if (SUM) {   // g0 * (this branch, as rounded) + g1 * a1 + g2 * a2
+      float g[3];
+#pragma unroll
+      for (int x = 0; x < 3; ++x) g[x] = __shfl_sync(0xffffffffu, __bfloat162float(graw[x]), hl);
+      uint4 w1 = make_uint4(0u, 0u, 0u, 0u), w2 = w1;
+      if (m.a1) w1 = __ldcs(reinterpret_cast<const uint4*>(m.a1) + vec0 + ud[i]);
+      if (m.a2) w2 = __ldcs(reinterpret_cast<const uint4*>(m.a2) + vec0 + ud[i]);
+      const __nv_bfloat162* h1 = reinterpret_cast<const __nv_bfloat162*>(&w1);
+      const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&w2);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float2 f0 = __bfloat1622float2(ho[k]), f1 = __bfloat1622float2(h1[k]), f2 = __bfloat1622float2(h2[k]);
+        ho[k] = __floats2bfloat162_rn(fmaf(g[2], f2.x, fmaf(g[1], f1.x, g[0] * f0.x)), fmaf(g[2], f2.y, fmaf(g[1], f1.y, g[0] * f0.y)));
+      }
+      reinterpret_cast<uint4*>(m.out)[vec0 + ud[i]] = ov;
+    }
   }
 }
 
@@ -466,7 +504,11 @@ int launch_sel_fwd_kv(const SelKvArgs& a, const RevArgs& r, cudaStream_t s) {
   if (e != cudaSuccess) return (int)e;
   const int G16 = a.Hq / a.Hk / 16;
   const long long total = (long long)a.B * a.Tq * a.Hk * G16;
-  sel_fwd_merge_kernel<<<(unsigned)((2 * total + 7) / 8), 256, 0, s>>>(r, a.part, a.stats, a.o, a.lse, G16);
+  const unsigned nb = (unsigned)((kMergeWarps * total + 7) / 8);
+  if (a.merge.out)
+    sel_fwd_merge_kernel<true><<<nb, 256, 0, s>>>(r, a.part, a.stats, a.merge, G16);
+  else
+    sel_fwd_merge_kernel<false><<<nb, 256, 0, s>>>(r, a.part, a.stats, a.merge, G16);
   note_launches(1);
   return (int)cudaGetLastError();
 }

@@ -142,7 +142,10 @@ class _NSAModule(torch.autograd.Function):
         covers = _lib.sel_fwd_kv_covers(Hq, Hkv, D, n_sel, sel_block)
         # saved: ck, cv, weights in the kernels' layout (k, v), gates (3), o_slc, o_cmp, o_swa, lse (3), idx, length tables,
         # one reverse index per run
-        off, total = _carve([crow * Hkv * D * 2] * 2 + [w_b] * 2 + [rows * 2] * 3 + [row_b, row_b, row_b if window > 0 else 0] +
+        need = any(ctx.needs_input_grad)
+        keep_slc = need or not (covers and keep_ix)   # the key-major forward can add the gated sum without storing o_slc
+        off, total = _carve([crow * Hkv * D * 2] * 2 + [w_b] * 2 + [rows * 2] * 3 +
+                            [row_b if keep_slc else 0, row_b, row_b if window > 0 else 0] +
                             [rows * 4] * 3 + [tok * Hkv * n_sel * 4, 8 * (len(lens) + 1)] + (ix_bytes if keep_ix else []))
         saved = torch.empty(total, dtype=torch.uint8, device=q.device)
         o = torch.empty_like(q)
@@ -180,14 +183,14 @@ class _NSAModule(torch.autograd.Function):
             if covers:
                 size = L.nsa_sel_swa_fwd_ix_workspace_bytes if keep_ix else L.nsa_sel_swa_fwd_workspace_bytes
                 ws_bytes = size(B, T, T, Hq, Hkv, D, n_sel, sel_block)
-            if keep_ix and (covers or any(ctx.needs_input_grad)):
+            if keep_ix and (covers or need):
                 chk(L.nsa_sel_index(ib, 0, None, ix[i], ix_bytes[i], B, T, T, 0, Hkv, n_sel, sel_block, S), "nsa_sel_index")
             ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device) if ws_bytes else None
-            chk(L.nsa_sel_swa_fwd_ix(P(q) + rb, P(k) + kv, P(v) + kv, ib, 0, None, ix[i], o_slc + rb, l_slc + 4 * r,
+            chk(L.nsa_sel_swa_fwd_ix(P(q) + rb, P(k) + kv, P(v) + kv, ib, 0, None, ix[i], o_slc + rb if keep_slc else None, l_slc + 4 * r,
                                      at(o_swa, rb), at(l_swa, 4 * r), g_slc + 2 * r, g_swa + 2 * r, o_cmp + rb, g_cmp + 2 * r,
                                      P(o) + rb, P(ws), ws_bytes, B, T, Hq, Hkv, D, n_sel, sel_block, window, scale, T, 0, S),
                 "nsa_sel_swa_fwd")
-        if any(ctx.needs_input_grad):
+        if need:
             ctx.save_for_backward(q, k, v, w_gate, saved)
             ctx.meta = (cfg, runs, off, ix_bytes if keep_ix else None, len(lens), b_gate is not None, bias_k is not None)
         return o
@@ -223,6 +226,7 @@ class _NSAModule(torch.autograd.Function):
             scratch[o2[4]:o2[5]].zero_()   # the gate gradient of the branch that is not there
         at = lambda p, x: None if p is None else p + x
         win = window > 0
+        add_gate = bool(ix_bytes) and _lib.sel_fwd_kv_covers(Hq, Hkv, D, n_sel, sel_block)
         if not fused:
             # one streaming pass over dO: delta = g * rowsum(o * dO) and the gate gradients of all three branches
             chk(L.nsa_rowdot3(o_slc, o_swa, o_cmp, P(do), g_slc, g_swa, g_cmp, d_slc, d_swa if win else None, d_cmp, dg_slc, dg_swa,
@@ -249,7 +253,8 @@ class _NSAModule(torch.autograd.Function):
                                              block, stride, 1 if causal else 0, scale, T, 0, S), "nsa_cmp_attn_bwd_fused")
             elif ix_bytes:
                 chk(L.nsa_attn_bwd_ix(qp, kp, vp, ck + cb, cv + cb, ib, 0, None, ix[i], dop, l_slc + r4, at(l_swa, r4), l_cmp + r4,
-                                      d_slc + r4, d_swa + r4, d_cmp + r4, g_slc + r2, g_swa + r2, g_cmp + r2, P(dq) + rb,
+                                      d_slc + r4, d_swa + r4, d_cmp + r4, g_slc + r2, g_swa + r2, g_cmp + r2, dg_slc + r2, dg_swa + r2,
+                                      dg_cmp + r2, P(w_gate) if add_gate else None, P(dq) + rb,
                                       P(dk) + kv, P(dv) + kv, dck + cb, dcv + cb, P(ws), n1, B, T, Tc, Hq, Hkv, D, n_sel,
                                       sel_block, window, block, stride, 1 if causal else 0, scale, S), "nsa_attn_bwd")
             else:
@@ -260,8 +265,9 @@ class _NSAModule(torch.autograd.Function):
                 chk(L.nsa_cmp_attn_bwd_sharded(qp, ck + cb, cv + cb, l_cmp + r4, dop, d_cmp + r4, g_cmp + r2, P(dq) + rb, 1,
                                                dck + cb, dcv + cb, P(ws), n2, B, T, Tc, Hq, Hkv, D, block, stride,
                                                1 if causal else 0, scale, T, 0, S), "nsa_cmp_attn_bwd")
-        # gate projection backward: dq += dg . W in place (dq is complete here), dW and db by fixed-order reduction
-        chk(L.nsa_gate_bwd(P(q), dg_slc, dg_swa, dg_cmp, P(w_gate), P(dq), P(dw), P(db), gws, gw_bytes, rows, D, S), "nsa_gate_bwd")
+        # gate projection backward: dq += dg . W in place (dq is complete here) unless the selected branch's reduction added it,
+        # dW and db by fixed-order reduction
+        chk(L.nsa_gate_bwd(P(q), dg_slc, dg_swa, dg_cmp, P(w_gate), None if add_gate else P(dq), P(dw), P(db), gws, gw_bytes, rows, D, S), "nsa_gate_bwd")
         # compression backward: its dX is added to dk, dv
         if c_bytes:
             cus = (None, None) if len(runs) == 1 else (cu, cu + 4 * (nseq + 1))
