@@ -8,7 +8,10 @@
 //
 // The step is HBM-bound: a sequence contributes its compressed cache (1/16 of its K/V), 16 selected blocks and the
 // window, each read once.  One CTA works on one (sequence, kv head): the 16 query heads of the group are the M = 16
-// rows of mma.sync.m16n8k16.  Two producer warps stream [64 rows x 128] tiles by TMA through a twelve-slot ring (192 KB
+// rows of mma.sync.m16n8k16.  Where there are fewer items than SMs, a cluster of 2, 4 or 8 CTAs shares one: the tile pairs of
+// every phase are dealt out to its CTAs, which exchange the soft-max statistics and the scores through each other's shared
+// memory and then select the blocks each for itself (one CTA alone draws at most 1/148 of the bandwidth: 4 items of 4096 keys
+// took 25 us).  Two producer warps stream [64 rows x 128] tiles by TMA through a twelve-slot ring (192 KB
 // in flight per SM); six consumer warps own two slots each, so every slot is filled and drained by the same pair of
 // warps in order.  The tile stream of an item:
 //   1. ck tiles:           raw scores -> per-row maxima and sums of the unscaled soft-max over ALL compressed keys and
@@ -23,6 +26,8 @@
 // warp, cost seven named barriers and six serialised rounds per branch (0.29 ms per step of the 128-sequence workload
 // against 0.21 ms); merging in the same kernel through an L2-resident scratch idled five of six warps and the TMA ring
 // during the merge (0.30 ms).  No atomics; every wait is bounded.
+#include <algorithm>
+
 #include "kernels.h"
 #include "tmap.h"
 
@@ -41,10 +46,11 @@ constexpr int kMaxTc = 2048;                   // compressed positions of one se
 constexpr int kMaxPoolD = 512;
 constexpr int kMaxSel = 32;
 constexpr int kPartFloats = 16 * D + 32;        // one warp's partial of one branch: O[16][D], m[16], l[16]
+constexpr int kMaxCluster = 8;
 
-struct Plan {   // tile counts of one item; every phase is an even number of tiles
+struct Plan {   // tile pairs of one item's phases; CTA `rank` of a cluster takes the pairs rank, rank + cl, ... of each
   int L, Tc, nvis, row_k, row_c;
-  int n1;      // ck tiles of pass 1 (rounded up to even)
+  int n1p;     // pairs of ck tiles of pass 1
   int n2p;     // (ck, cv) pairs of pass 2: covers all of Tc
   int nw;      // window pairs
   int w0;      // first window key
@@ -60,7 +66,7 @@ __device__ __forceinline__ Plan make_plan(const DecodeArgs& a, int seq) {
   const int t = p.L - 1;
   p.nvis = (t < a.cblock) ? 0 : min(p.Tc, (t - a.cblock) / a.cstride + 1);
   const int nck = (p.Tc + 63) / 64;
-  p.n1 = (nck + 1) & ~1;
+  p.n1p = (nck + 1) / 2;
   p.n2p = nck;
   p.w0 = max(0, p.L - a.window);
   p.nw = a.window > 0 ? (p.L - p.w0 + 63) / 64 : 0;
@@ -72,6 +78,47 @@ __device__ __forceinline__ Plan make_plan(const DecodeArgs& a, int seq) {
 // for lengths uniform in [4096, 32768], against 1.23 for a plain round robin).
 __device__ __forceinline__ int snake_item(int round, int cta, int ncta) {
   return round * ncta + ((round & 1) ? ncta - 1 - cta : cta);
+}
+
+// ---- the CTAs of a cluster -----------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t map_cta(uint32_t saddr, uint32_t cta) {   // the same shared-memory address in another CTA
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(cta));
+  return r;
+}
+__device__ __forceinline__ void st_cluster(uint32_t addr, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+__device__ __forceinline__ void arrive_cluster(uint32_t bar) {   // releases what this thread has seen, to the cluster
+  asm volatile("fence.acq_rel.cluster;" ::: "memory");
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// bounded wait for a barrier that other CTAs arrive at
+__device__ __forceinline__ bool wait_cluster(uint32_t bar, uint32_t parity, int code, volatile int* abort_flag) {
+  const uint64_t t0 = global_timer_ns();
+  for (;;) {
+#pragma unroll 1
+    for (int i = 0; i < 256; ++i) {
+      uint32_t ok;
+      asm volatile("{ .reg .pred p; mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                   : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+      if (ok) return true;
+    }
+    if (*abort_flag) return false;
+    if (global_timer_ns() - t0 > 2000000000ull) {
+      atomicCAS(&g_dev_error, 0, code);
+      *abort_flag = 1;
+      return false;
+    }
+  }
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // avg_pool1d(kernel k, stride s, no padding, ceil_mode) output length, as nsa_pool_out_len computes it
@@ -143,7 +190,7 @@ __device__ __forceinline__ void online_pair(float (&acc)[D / 8][4], float (&m_ru
 
 __global__ void __launch_bounds__(kThreads, 1)
     decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
-                  const __grid_constant__ CUtensorMap tmCK, const __grid_constant__ CUtensorMap tmCV, const DecodeArgs a) {
+                  const __grid_constant__ CUtensorMap tmCK, const __grid_constant__ CUtensorMap tmCV, const DecodeArgs a, const int cl) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t sbase = (raw + 1023u) & ~1023u;
@@ -155,13 +202,16 @@ __global__ void __launch_bounds__(kThreads, 1)
   float* pooled = ps + kMaxTc + 64;                               // [kMaxPoolD]
   float* stat = pooled + kMaxPoolD;                               // [kCons][4][16] per-warp statistics
   float* fin = stat + kCons * 64;                                 // [4][16] merged: M_raw, 1/L_raw, M_att (log2), L_att
-  int* sel = reinterpret_cast<int*>(fin + 64);                    // [kMaxSel] selected blocks of the item, [kMaxSel] = count
+  float* xstat = fin + 64;                                        // [cluster][4][16] the CTAs' statistics
+  int* sel = reinterpret_cast<int*>(xstat + kMaxCluster * 64);    // [kMaxSel] selected blocks of the item, [kMaxSel] = count
   volatile int* abort_flag = sel + kMaxSel + 2;
   const uint32_t bar_base = sbase + kSlots * TILE + (uint32_t)((uint8_t*)(sel + kMaxSel + 4) - after);
   const uint32_t bar0 = (bar_base + 7u) & ~7u;
   auto full_bar = [&](uint32_t s) { return bar0 + 8u * s; };
   auto empty_bar = [&](uint32_t s) { return bar0 + 8u * (kSlots + s); };
   const uint32_t sel_ready = bar0 + 8u * (2 * kSlots);
+  const uint32_t xstat_bar = sel_ready + 8, ps_bar = sel_ready + 16;   // every CTA's statistics / scores have arrived here
+  const int rank = cl > 1 ? (int)cluster_rank() : 0, group = blockIdx.x / cl, ngroup = gridDim.x / cl;
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
@@ -170,9 +220,13 @@ __global__ void __launch_bounds__(kThreads, 1)
       mbar_init(empty_bar(i), 1);
     }
     mbar_init(sel_ready, 1);
+    mbar_init(xstat_bar, cl);
+    mbar_init(ps_bar, cl);
     fence_mbar_init();
   }
   __syncthreads();
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the merge may take its places now: it waits for this grid's end
+  if (cl > 1) cluster_sync_all();   // no CTA writes into another's shared memory before it runs, or after it ended (below)
 
   const int nitem = a.nseq * a.Hkv;
   const int pool_k = a.sel_block / a.cstride + 1, pool_s = a.sel_block / a.cstride;
@@ -208,31 +262,29 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       return good != 0;
     };
-    for (int r = 0; r * (int)gridDim.x < nitem; ++r) {
-      const int item = snake_item(r, blockIdx.x, gridDim.x);
+    for (int r = 0; r * ngroup < nitem; ++r) {
+      const int item = snake_item(r, group, ngroup);
       if (item >= nitem) continue;
       const int sq = item / a.Hkv, h = item % a.Hkv;
       const int seq = a.order ? a.order[sq] : sq;
       const Plan p = make_plan(a, seq);
       bool ok = true;
-      for (int j = 0; ok && j < p.n1; j += 2) ok = issue2(&tmCK, p.row_c + j * 64, &tmCK, p.row_c + (j + 1) * 64, h);
-      for (int j = 0; ok && j < p.n2p; ++j) ok = issue2(&tmCK, p.row_c + j * 64, &tmCV, p.row_c + j * 64, h);
-      for (int j = 0; ok && j < p.nw; ++j) ok = issue2(&tmK, p.row_k + p.w0 + j * 64, &tmV, p.row_k + p.w0 + j * 64, h);
+      for (int j = rank; ok && j < p.n1p; j += cl) ok = issue2(&tmCK, p.row_c + j * 128, &tmCK, p.row_c + j * 128 + 64, h);
+      for (int j = rank; ok && j < p.n2p; j += cl) ok = issue2(&tmCK, p.row_c + j * 64, &tmCV, p.row_c + j * 64, h);
+      for (int j = rank; ok && j < p.nw; j += cl) ok = issue2(&tmK, p.row_k + p.w0 + j * 64, &tmV, p.row_k + p.w0 + j * 64, h);
       // the selected blocks are known once the consumers have pooled the scores
       if (ok && lane == 0) ok = mbar_wait_abortable(sel_ready, it & 1, DEV_ERR_FULL_WAIT, abort_flag);
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
       if (!ok) break;
       const int nsel = *reinterpret_cast<volatile int*>(sel + kMaxSel);
-      for (int j = 0; ok && j < nsel; ++j) {
+      for (int j = rank; ok && j < nsel; j += cl) {
         const int blk = *reinterpret_cast<volatile int*>(sel + j);
         ok = issue2(&tmK, p.row_k + blk * 64, &tmV, p.row_k + blk * 64, h);
       }
       if (!ok) break;
       ++it;
     }
-    return;
-  }
-
+  } else {
   // --------------------------------- consumers ----------------------------------------------------------
   const int g = lane >> 2, tq = lane & 3;
   const float sl2 = a.scale * kLog2e;
@@ -241,8 +293,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint32_t n0 = 0, it = 0;                  // tiles consumed by the CTA before the current phase; items so far
   bool ok = true;
   // tile pair u (two consecutive tiles) of a phase that starts at tile counter base belongs to warp ((base/2 + u) % kCons)
-  for (int r = 0; r * (int)gridDim.x < nitem; ++r) {
-    const int item = snake_item(r, blockIdx.x, gridDim.x);
+  for (int r = 0; r * ngroup < nitem; ++r) {
+    const int item = snake_item(r, group, ngroup);
     if (item >= nitem) continue;
     const int sq = item / a.Hkv, h = item % a.Hkv;
     const int seq = a.order ? a.order[sq] : sq;
@@ -251,18 +303,18 @@ __global__ void __launch_bounds__(kThreads, 1)
     const long long qrow = (long long)seq * a.Hq + h * 16;     // first of the 16 (head) rows of this item
     uint32_t qf[D / 16][4];
     load_a_frags_global<D>(qf, a.q + qrow * D, lane);
-    for (int i = ct; i < kMaxTc + 64; i += cthreads) ps[i] = 0.f;
 
     // ---- pass 1: statistics over all compressed keys ---------------------------------------------------
     float mr[2] = {-INFINITY, -INFINITY}, lr[2] = {0.f, 0.f};   // raw scores, all keys (natural-log domain kept in log2)
     float ma[2] = {-INFINITY, -INFINITY}, la[2] = {0.f, 0.f};   // scaled scores, visible keys
     {
       const uint32_t pair0 = n0 / 2;
-      for (int u = 0; u < p.n1 / 2; ++u) {
-        if ((int)((pair0 + u) % kCons) != warp) continue;
+      int i = 0;   // this CTA's pairs
+      for (int u = rank; u < p.n1p; u += cl, ++i) {
+        if ((int)((pair0 + i) % kCons) != warp) continue;
 #pragma unroll 1
         for (int e = 0; e < 2; ++e) {
-          const uint32_t n = n0 + 2 * u + e, s = n % kSlots;
+          const uint32_t n = n0 + 2 * i + e, s = n % kSlots;
           const int j0 = (2 * u + e) * 64;
           ok = ok && mbar_wait_abortable(full_bar(s), (n / kSlots) & 1, DEV_ERR_FULL_WAIT, abort_flag);
           float sc[8][4];
@@ -301,7 +353,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
         }
       }
-      n0 += p.n1;
+      n0 += 2 * i;
     }
     // merge the per-warp statistics (each value lives in the four lanes of a quad: sum the partial sums)
 #pragma unroll
@@ -328,6 +380,32 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (m1 > -INFINITY) Lr += stat[w * 64 + 16 + ct] * ex2(m1 - Mr);
         if (m2 > -INFINITY) La += stat[w * 64 + 48 + ct] * ex2(m2 - Ma);
       }
+      const float v[4] = {Mr, Lr, Ma, La};
+      for (int c = 0; c < cl; ++c) {
+        const uint32_t dst = smem_u32(xstat + rank * 64 + ct);
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (cl > 1) st_cluster(map_cta(dst, c) + 64 * e, v[e]); else xstat[16 * e + ct] = v[e];
+      }
+    }
+    if (cl > 1) {
+      if (warp == 0) {
+        __syncwarp();
+        if (lane < cl) arrive_cluster(map_cta(xstat_bar, lane));
+        ok = ok && wait_cluster(xstat_bar, it & 1, 320, abort_flag);
+      }
+    }
+    if (ct < 16) {   // (written by this thread, or by the CTAs of the cluster)
+      float Mr = -INFINITY, Ma = -INFINITY, Lr = 0.f, La = 0.f;
+      for (int c = 0; c < cl; ++c) {
+        Mr = fmaxf(Mr, xstat[c * 64 + ct]);
+        Ma = fmaxf(Ma, xstat[c * 64 + 32 + ct]);
+      }
+      for (int c = 0; c < cl; ++c) {
+        const float m1 = xstat[c * 64 + ct], m2 = xstat[c * 64 + 32 + ct];
+        if (m1 > -INFINITY) Lr += xstat[c * 64 + 16 + ct] * ex2(m1 - Mr);
+        if (m2 > -INFINITY) La += xstat[c * 64 + 48 + ct] * ex2(m2 - Ma);
+      }
       fin[ct] = Mr;
       fin[16 + ct] = Lr > 0.f ? 1.f / Lr : 0.f;
       fin[32 + ct] = Ma;
@@ -349,11 +427,14 @@ __global__ void __launch_bounds__(kThreads, 1)
     float acc[D / 8][4];
 #pragma unroll
     for (int i = 0; i < D / 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+    bool full = rank == 0 && warp == 0;   // this warp's partial has an output (the first always: the row sums ride with it)
     {
       const uint32_t pair0 = n0 / 2;
-      for (int u = 0; u < p.n2p; ++u) {
-        if ((int)((pair0 + u) % kCons) != warp) continue;
-        const uint32_t nk = n0 + 2 * u, nv = nk + 1, sk = nk % kSlots, sv = nv % kSlots;
+      int i = 0;
+      for (int u = rank; u < p.n2p; u += cl, ++i) {
+        if ((int)((pair0 + i) % kCons) != warp) continue;
+        full = true;
+        const uint32_t nk = n0 + 2 * i, nv = nk + 1, sk = nk % kSlots, sv = nv % kSlots;
         const int j0 = u * 64;
         ok = ok && mbar_wait_abortable(full_bar(sk), (nk / kSlots) & 1, DEV_ERR_FULL_WAIT, abort_flag);
         float sc[8][4];
@@ -378,8 +459,16 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
           if (g == 0) {
             const int j = j0 + nt * 8 + 2 * tq;
-            if (j < p.Tc) ps[j] = c0;
-            if (j + 1 < p.Tc) ps[j + 1] = c1;
+            if (cl == 1) {
+              if (j < p.Tc) ps[j] = c0;
+              if (j + 1 < p.Tc) ps[j + 1] = c1;
+            } else {
+              for (int c = 0; c < cl; ++c) {
+                const uint32_t dst = map_cta(smem_u32(ps + j), c);
+                if (j < p.Tc) st_cluster(dst, c0);
+                if (j + 1 < p.Tc) st_cluster(dst + 4, c1);
+              }
+            }
           }
         }
         // attention weights with the final maximum (unnormalised; the sum divides at the end)
@@ -395,10 +484,14 @@ __global__ void __launch_bounds__(kThreads, 1)
         __syncwarp();
         if (lane == 0) mbar_arrive(empty_bar(sv));
       }
-      n0 += 2 * p.n2p;
+      n0 += 2 * i;
     }
     // ---- pooled scores and the top-n (warp 0), the compressed-branch output (all warps, fixed order) ------------
     named_bar_sync(1, cthreads);            // ps complete
+    if (cl > 1) {   // in every CTA
+      if (ct < cl) arrive_cluster(map_cta(ps_bar, ct));
+      ok = ok && wait_cluster(ps_bar, it & 1, 321, abort_flag);
+    }
     const int n_pool = min(kMaxPoolD, pool_len(p.Tc, pool_k, pool_s));
     for (int blk = ct; blk < n_pool; blk += cthreads) {
       const int lo = blk * pool_s, hi = min(lo + pool_k, p.Tc);
@@ -406,50 +499,58 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int j = lo; j < hi; ++j) sum += ps[j];
       pooled[blk] = sum / (float)(hi - lo);
     }
+    if (ct < (-n_pool & 3)) pooled[n_pool + ct] = -INFINITY;   // whole groups of four below
+    if (ct < kMaxSel) sel[ct] = -1;
+    named_bar_sync(1, cthreads);
+    // Top-n by counting: a block's rank is the number of blocks with a higher score, or an equal one and a lower index (n
+    // rounds of a warp-wide maximum took 2 us for 64 blocks, 3.4 for 512).
+    {
+      constexpr int kOwn = (kMaxPoolD + kCons * 32 - 1) / (kCons * 32);
+      float v[kOwn];
+      int rk[kOwn];
+#pragma unroll
+      for (int e = 0; e < kOwn; ++e) {
+        const int blk = ct + e * cthreads;
+        v[e] = blk < n_pool ? pooled[blk] : INFINITY;
+        rk[e] = 0;
+      }
+      const int own = (n_pool + cthreads - 1) / cthreads;
+      for (int j = 0; j < n_pool; j += 4) {
+        const float4 x4 = *reinterpret_cast<const float4*>(pooled + j);
+        const float x[4] = {x4.x, x4.y, x4.z, x4.w};
+#pragma unroll
+        for (int e = 0; e < kOwn; ++e) {
+          if (e >= own) continue;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) rk[e] += (x[c] > v[e] || (x[c] == v[e] && j + c < ct + e * cthreads)) ? 1 : 0;
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < kOwn; ++e)
+        if (ct + e * cthreads < n_pool && rk[e] < a.n_sel) sel[rk[e]] = ct + e * cthreads;
+    }
     named_bar_sync(1, cthreads);
     if (warp == 0) {
-      int cnt = 0;
-      int* out = a.idx + ((long long)seq * a.Hkv + h) * a.n_sel;
-      for (int r = 0; r < a.n_sel; ++r) {
-        float bv = -2.f;
-        int bi = 0x7fffffff;
-        for (int blk = lane; blk < n_pool; blk += 32) {
-          const float v = pooled[blk];
-          if (v > bv) {
-            bv = v;
-            bi = blk;
-          }
-        }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-          const float ov = __shfl_xor_sync(0xffffffffu, bv, off);
-          const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
-          if (ov > bv || (ov == bv && oi < bi)) {
-            bv = ov;
-            bi = oi;
-          }
-        }
-        const bool found = bv > -1.5f;
-        if (lane == 0) {
-          out[r] = found ? bi : -1;
-          if (found) {
-            pooled[bi] = -2.f;
-            if ((long long)bi * 64 <= t && cnt < kMaxSel) sel[cnt++] = bi;   // blocks that start after t are skipped
-          }
-        }
-        __syncwarp();
-      }
+      const int blk = lane < a.n_sel ? sel[lane] : -1;   // n_sel <= kMaxSel = 32
+      if (rank == 0 && lane < a.n_sel) a.idx[((long long)seq * a.Hkv + h) * a.n_sel + lane] = blk;
+      const bool use = blk >= 0 && (long long)blk * 64 <= t;   // blocks that start after t are skipped
+      const unsigned m = __ballot_sync(0xffffffffu, use);
+      __syncwarp();
+      if (use) sel[__popc(m & ((1u << lane) - 1))] = blk;
+      __syncwarp();
       if (lane == 0) {
-        sel[kMaxSel] = cnt;
+        sel[kMaxSel] = __popc(m);
         __threadfence_block();
         mbar_arrive(sel_ready);
       }
     }
-    // this warp's partial of a branch -> workspace: [item][branch][warp]{ O[16][D], m[16], l[16] } fp32
-    auto put_partial = [&](int branch, const float (&x)[D / 8][4], const float (&mm)[2], const float (&ll)[2]) {
-      float* dst = a.part + (((long long)item * 3 + branch) * kCons + warp) * kPartFloats;
+    // this warp's partial of a branch -> workspace: [item][branch][warp of the cluster]{ O[16][D], m[16], l[16] } fp32; a warp
+    // that had no tile leaves m = -inf and no O
+    auto put_partial = [&](int branch, const float (&x)[D / 8][4], const float (&mm)[2], const float (&ll)[2], bool has) {
+      float* dst = a.part + (((long long)item * 3 + branch) * (cl * kCons) + rank * kCons + warp) * kPartFloats;
 #pragma unroll
       for (int i = 0; i < D / 8; ++i) {
+        if (!has) break;
         *reinterpret_cast<float2*>(dst + g * D + i * 8 + 2 * tq) = make_float2(x[i][0], x[i][1]);
         *reinterpret_cast<float2*>(dst + (g + 8) * D + i * 8 + 2 * tq) = make_float2(x[i][2], x[i][3]);
       }
@@ -457,7 +558,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int rr = 0; rr < 2; ++rr) {
         const float l = quad_sum(ll[rr]);
         if (tq == 0) {
-          dst[16 * D + g + 8 * rr] = mm[rr];
+          dst[16 * D + g + 8 * rr] = has ? mm[rr] : -INFINITY;
           dst[16 * D + 16 + g + 8 * rr] = l;
         }
       }
@@ -468,29 +569,32 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
       for (int rr = 0; rr < 2; ++rr) {
         mm[rr] = fin[32 + g + 8 * rr];
-        ll[rr] = (warp == 0 && tq == 0) ? La[rr] : 0.f;
+        ll[rr] = (rank == 0 && warp == 0 && tq == 0) ? La[rr] : 0.f;
       }
-      put_partial(0, acc, mm, ll);
+      put_partial(0, acc, mm, ll, full);
     }
 
     // ---- window ---------------------------------------------------------------------------------------
     float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
 #pragma unroll
     for (int i = 0; i < D / 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+    full = false;
     {
       const uint32_t pair0 = n0 / 2;
-      for (int u = 0; u < p.nw; ++u) {
-        if ((int)((pair0 + u) % kCons) != warp) continue;
-        const uint32_t nk = n0 + 2 * u, nv = nk + 1, sk = nk % kSlots, sv = nv % kSlots;
+      int i = 0;
+      for (int u = rank; u < p.nw; u += cl, ++i) {
+        if ((int)((pair0 + i) % kCons) != warp) continue;
+        full = true;
+        const uint32_t nk = n0 + 2 * i, nv = nk + 1, sk = nk % kSlots, sv = nv % kSlots;
         ok = ok && mbar_wait_abortable(full_bar(sk), (nk / kSlots) & 1, DEV_ERR_FULL_WAIT, abort_flag);
         online_pair(acc, m_run, l_run, qf, ring + sk * TILE, ring + sv * TILE, empty_bar(sk), full_bar(sv), (nv / kSlots) & 1,
                     empty_bar(sv), p.w0 + u * 64, p.w0, p.L, sl2, lane, ok, abort_flag);
       }
-      n0 += 2 * p.nw;
+      n0 += 2 * i;
     }
     {
       // l_run holds this lane's share of the row sums (four lanes per row): put_partial adds the quad
-      put_partial(2, acc, m_run, l_run);
+      put_partial(2, acc, m_run, l_run, full);
     }
 
     // ---- selected blocks ---------------------------------------------------------------------------------
@@ -500,135 +604,152 @@ __global__ void __launch_bounds__(kThreads, 1)
     l_run[0] = l_run[1] = 0.f;
 #pragma unroll
     for (int i = 0; i < D / 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+    full = false;
     {
       const uint32_t pair0 = n0 / 2;
-      for (int u = 0; u < nsel; ++u) {
-        if ((int)((pair0 + u) % kCons) != warp) continue;
+      int i = 0;
+      for (int u = rank; u < nsel; u += cl, ++i) {
+        if ((int)((pair0 + i) % kCons) != warp) continue;
+        full = true;
         const int blk = *reinterpret_cast<volatile int*>(sel + u);
-        const uint32_t nk = n0 + 2 * u, nv = nk + 1, sk = nk % kSlots, sv = nv % kSlots;
+        const uint32_t nk = n0 + 2 * i, nv = nk + 1, sk = nk % kSlots, sv = nv % kSlots;
         ok = ok && mbar_wait_abortable(full_bar(sk), (nk / kSlots) & 1, DEV_ERR_FULL_WAIT, abort_flag);
         online_pair(acc, m_run, l_run, qf, ring + sk * TILE, ring + sv * TILE, empty_bar(sk), full_bar(sv), (nv / kSlots) & 1,
                     empty_bar(sv), blk * 64, 0, p.L, sl2, lane, ok, abort_flag);
       }
-      n0 += 2 * nsel;
+      n0 += 2 * i;
     }
-    put_partial(1, acc, m_run, l_run);
+    put_partial(1, acc, m_run, l_run, full);
     named_bar_sync(1, cthreads);   // ps, pooled, fin and sel are reused by the next item
     ++it;
   }
+  }
+  if (cl > 1) {
+    __syncwarp();
+    cluster_sync_all();
+  }
 }
 
-// Merge of the per-warp partials: one CTA of D threads per (sequence, kv head); thread d owns channel d of the 16 rows.
-// Branch order in the workspace: 0 compressed, 1 selected, 2 window.  Fixed summation order (warp 0, 1, ...).  The gates
-// are computed here from q when the gate projection is given.
-// 4 x D threads per item: four groups of four query rows, one thread per output channel; the sums over the six
-// consumer warps are short, so the kernel is pure latency and the rows are spread over as many threads as the GPU holds.
-constexpr int kMergeGroups = 4;
-__global__ void __launch_bounds__(kMergeGroups * D) decode_merge_kernel(const DecodeArgs a) {
-  const int item = blockIdx.x;
+// Merge of the per-warp partials, in a fixed order (CTA by CTA, warp by warp): one block per (item, four query rows), one thread
+// per (branch, channel).  Branch order in the workspace: 0 compressed, 1 selected, 2 window.  Warps that had no tile are left
+// out.  Pure latency: the loads of a branch's partials are independent, and the gates (computed from q when the gate projection
+// is given) do not wait for them.
+constexpr int kMergeRows = 4;
+__global__ void __launch_bounds__(3 * D) decode_merge_kernel(const DecodeArgs a, const int cl) {
+  const int item = blockIdx.x / (16 / kMergeRows), r0 = blockIdx.x % (16 / kMergeRows) * kMergeRows;
+  const int nw = cl * kCons;
   const int sq = item / a.Hkv, h = item % a.Hkv;
   const int seq = a.order ? a.order[sq] : sq;
-  const long long qrow = (long long)seq * a.Hq + h * 16;
-  const int d = threadIdx.x & (D - 1);
-  const int rg = threadIdx.x / D;            // rows 4 rg .. 4 rg + 3
-  const int tid = threadIdx.x;
-  const float* part = a.part + (long long)item * 3 * kCons * kPartFloats;
-  __shared__ float w_s[3][kCons][16];   // per (branch, warp, row): 2^(m_w - M) / L
-  __shared__ float lse_s[3][16];
-  __shared__ float gp_s[D / 32][48];    // gate projection: per-warp partial dot products of (row, gate)
-  __shared__ float gate_s[3][16];       // gates of the item's 16 rows; order: compressed, selected, window
+  const long long qrow = (long long)seq * a.Hq + h * 16 + r0;
+  const int tid = threadIdx.x, lane = tid & 31, br = tid / D, d = tid % D;
+  const float* part = a.part + (long long)item * 3 * nw * kPartFloats;
+  __shared__ int act_s[3][kMaxCluster * kCons], nact_s[3];          // warps with a partial
+  __shared__ __align__(16) float ml_s[3][kMaxCluster * kCons][2][kMergeRows];
+  __shared__ float w_s[3][kMaxCluster * kCons][kMergeRows];         // per (branch, warp, row): 2^(m_w - M) / L
+  __shared__ float gp_s[3][D / 32][kMergeRows];                     // gate projection: per-warp partial dot products
+  __shared__ bf16 out_s[3][kMergeRows][D];
+  __shared__ float gate_s[3][kMergeRows];                           // order: compressed, selected, window
+  const int x = br == 0 ? 2 : br - 1;       // branch (cmp, slc, swa) -> row of the gate weight (slc, swa, cmp)
   if (a.gate_w) {
     // g_x[row] = q[row,:] . W[x,:] + b[x] (nn.Linear(head_dim, 3), rows of W: selected, window, compressed), rounded to
     // bf16 as the module's gate tensors are
-    const float w0 = __bfloat162float(a.gate_w[d]), w1 = __bfloat162float(a.gate_w[D + d]), w2 = __bfloat162float(a.gate_w[2 * D + d]);
-    float qa[4];
+    const float w = __bfloat162float(a.gate_w[x * D + d]);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) qa[i] = __bfloat162float(a.q[(qrow + rg * 4 + i) * D + d]);
+    for (int i = 0; i < kMergeRows; ++i) {
+      float p = __bfloat162float(a.q[(qrow + i) * D + d]) * w;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = rg * 4 + i;
-      float p0 = qa[i] * w0, p1 = qa[i] * w1, p2 = qa[i] * w2;
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
-        p0 += __shfl_xor_sync(0xffffffffu, p0, off);
-        p1 += __shfl_xor_sync(0xffffffffu, p1, off);
-        p2 += __shfl_xor_sync(0xffffffffu, p2, off);
-      }
-      if ((d & 31) == 0) {
-        gp_s[d >> 5][r * 3 + 0] = p0;
-        gp_s[d >> 5][r * 3 + 1] = p1;
-        gp_s[d >> 5][r * 3 + 2] = p2;
-      }
+      for (int off = 16; off > 0; off >>= 1) p += __shfl_xor_sync(0xffffffffu, p, off);
+      if (lane == 0) gp_s[br][d >> 5][i] = p;
     }
   }
   // Launched with programmatic stream serialization: everything above (the gate projection reads only q and the
   // weights) may run while the main kernel is still finishing; its partials are read only behind this wait.
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (tid < 48) {
-    const int br = tid / 16, r = tid % 16;
-    const float* base = part + (long long)br * kCons * kPartFloats;
-    float mw[kCons], lw[kCons];
-#pragma unroll
-    for (int w = 0; w < kCons; ++w) {
-      mw[w] = base[w * kPartFloats + 16 * D + r];
-      lw[w] = base[w * kPartFloats + 16 * D + 16 + r];
+  if (tid % D < 32) {   // the first warp of each branch
+    const float* base = part + (long long)br * nw * kPartFloats + 16 * D + r0;
+    int n = 0;
+    for (int w0 = 0; w0 < nw; w0 += 32) {
+      const int w = w0 + lane;
+      float4 m = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY), l = m;
+      if (w < nw) {
+        m = *reinterpret_cast<const float4*>(base + (long long)w * kPartFloats);
+        l = *reinterpret_cast<const float4*>(base + (long long)w * kPartFloats + 16);
+      }
+      const bool on = fmaxf(fmaxf(m.x, m.y), fmaxf(m.z, m.w)) > -INFINITY;
+      const unsigned mask = __ballot_sync(0xffffffffu, on);
+      if (on) {
+        const int i = n + __popc(mask & ((1u << lane) - 1));
+        act_s[br][i] = w;
+        *reinterpret_cast<float4*>(ml_s[br][i][0]) = m;
+        *reinterpret_cast<float4*>(ml_s[br][i][1]) = l;
+      }
+      n += __popc(mask);
     }
-    float M = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < kCons; ++w) M = fmaxf(M, mw[w]);
-    float Ltot = 0.f;
-#pragma unroll
-    for (int w = 0; w < kCons; ++w)
-      if (mw[w] > -INFINITY) Ltot += lw[w] * ex2(mw[w] - M);
-#pragma unroll
-    for (int w = 0; w < kCons; ++w) w_s[br][w][r] = (mw[w] > -INFINITY && Ltot > 0.f) ? ex2(mw[w] - M) / Ltot : 0.f;
-    lse_s[br][r] = Ltot > 0.f ? (M + log2f(Ltot)) * kLn2 : -INFINITY;
+    __syncwarp();
+    if (lane == 0) nact_s[br] = n;
+    if (lane < kMergeRows) {
+      float M = -INFINITY, L = 0.f;
+      for (int i = 0; i < n; ++i) M = fmaxf(M, ml_s[br][i][0][lane]);
+      for (int i = 0; i < n; ++i)
+        if (ml_s[br][i][0][lane] > -INFINITY) L += ml_s[br][i][1][lane] * ex2(ml_s[br][i][0][lane] - M);
+      for (int i = 0; i < n; ++i) w_s[br][i][lane] = (ml_s[br][i][0][lane] > -INFINITY && L > 0.f) ? ex2(ml_s[br][i][0][lane] - M) / L : 0.f;
+      if (a.lse && !(br == 2 && a.window <= 0))
+        a.lse[(long long)br * a.nseq * a.Hq + qrow + lane] = L > 0.f ? (M + log2f(L)) * kLn2 : -INFINITY;
+    }
   }
   __syncthreads();
-  if (tid < 48) {
-    const int br = tid / 16, r = tid % 16;
-    const bf16* gin[3] = {a.g_cmp, a.g_slc, a.g_swa};
+  if (d < kMergeRows) {
+    const bf16* gin = br == 0 ? a.g_cmp : br == 1 ? a.g_slc : a.g_swa;
     float gv = 1.f;
     if (a.gate_w) {
-      const int x = br == 0 ? 2 : br - 1;     // branch (cmp, slc, swa) -> row of the gate weight (slc, swa, cmp)
       float sum = 0.f;
-      for (int w = 0; w < D / 32; ++w) sum += gp_s[w][r * 3 + x];
+      for (int w = 0; w < D / 32; ++w) sum += gp_s[br][w][d];
       if (a.gate_b) sum += __bfloat162float(a.gate_b[x]);
       gv = __bfloat162float(__float2bfloat16(sum));
-    } else if (gin[br]) {
-      gv = __bfloat162float(gin[br][qrow + r]);
+    } else if (gin) {
+      gv = __bfloat162float(gin[qrow + d]);
     }
-    gate_s[br][r] = gv;
+    gate_s[br][d] = gv;
+  }
+  const float* base = part + (long long)br * nw * kPartFloats + r0 * D + d;
+  float v[kMergeRows];
+#pragma unroll
+  for (int i = 0; i < kMergeRows; ++i) v[i] = 0.f;
+  const int n = nact_s[br];
+#pragma unroll 6
+  for (int k = 0; k < n; ++k) {
+    const float* src = base + (long long)act_s[br][k] * kPartFloats;
+#pragma unroll
+    for (int i = 0; i < kMergeRows; ++i) v[i] += src[i * D] * w_s[br][k][i];
+  }
+  bf16* outs = br == 0 ? a.o_cmp : br == 1 ? a.o_slc : a.window > 0 ? a.o_swa : nullptr;
+#pragma unroll
+  for (int i = 0; i < kMergeRows; ++i) {
+    const bf16 vb = __float2bfloat16(v[i]);
+    out_s[br][i][d] = vb;
+    if (outs) outs[(qrow + i) * D + d] = vb;
   }
   __syncthreads();
-  bf16* outs[3] = {a.o_cmp, a.o_slc, a.o_swa};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {   // this group's four rows: 72 independent loads in flight per thread
-    const int r = rg * 4 + i;
+  for (int i = br; i < kMergeRows; i += 3) {
     float tot = 0.f;
 #pragma unroll
-    for (int br = 0; br < 3; ++br) {
-      if (br == 2 && a.window <= 0) continue;
-      const float* base = part + (long long)br * kCons * kPartFloats + r * D + d;
-      float v = 0.f;
-#pragma unroll
-      for (int w = 0; w < kCons; ++w) v += base[w * kPartFloats] * w_s[br][w][r];
-      const bf16 vb = __float2bfloat16(v);
-      if (outs[br]) outs[br][(qrow + r) * D + d] = vb;
-      tot += gate_s[br][r] * __bfloat162float(vb);
-    }
-    a.o[(qrow + r) * D + d] = __float2bfloat16(tot);
+    for (int b = 0; b < 3; ++b)
+      if (!(b == 2 && a.window <= 0)) tot += gate_s[b][i] * __bfloat162float(out_s[b][i][d]);
+    a.o[(qrow + i) * D + d] = __float2bfloat16(tot);
   }
-  if (a.lse && tid < 48) {
-    const int br = tid / 16, r = tid % 16;
-    if (!(br == 2 && a.window <= 0)) a.lse[(long long)br * a.nseq * a.Hq + qrow + r] = lse_s[br][r];
-  }
+}
+
+// CTAs per item: as many as keep every item in the first wave.
+int decode_cluster(int nitem) {
+  int cl = kMaxCluster;
+  while (cl > 1 && nitem * cl > num_sms()) cl >>= 1;
+  return cl;
 }
 
 }  // namespace
 
 size_t decode_workspace_bytes(int nseq, int Hkv) {
-  return (size_t)nseq * Hkv * 3 * kCons * kPartFloats * sizeof(float);
+  return (size_t)nseq * Hkv * 3 * decode_cluster(nseq * Hkv) * kCons * kPartFloats * sizeof(float);
 }
 
 int launch_decode(const DecodeArgs& a, cudaStream_t s) {
@@ -655,27 +776,37 @@ int launch_decode(const DecodeArgs& a, cudaStream_t s) {
   if (!rc) rc = make_tmap_rows4d(&tmCK, a.ck, D, a.Hkv, a.total_c, 1, 64);
   if (!rc) rc = make_tmap_rows4d(&tmCV, a.cv, D, a.Hkv, a.total_c, 1, 64);
   if (rc) return rc;
-  const int nitem0 = a.nseq * a.Hkv;
   if (!a.part || a.part_bytes < decode_workspace_bytes(a.nseq, a.Hkv)) {
     set_error("decode: workspace too small (%lld bytes needed)", (long long)decode_workspace_bytes(a.nseq, a.Hkv));
     return -6;
   }
-  (void)nitem0;
-  const int smem = kSlots * (int)TILE + (kMaxTc + 64 + kMaxPoolD + kCons * 64 + 64) * 4 + (kMaxSel + 4) * 4 +
-                   (2 * kSlots + 1) * 8 + 16 + 1024;
+  const int smem = kSlots * (int)TILE + (kMaxTc + 64 + kMaxPoolD + kCons * 64 + 64 + kMaxCluster * 64) * 4 + (kMaxSel + 4) * 4 +
+                   (2 * kSlots + 3) * 8 + 16 + 1024;
   cudaError_t e = cudaFuncSetAttribute(decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return (int)e;
   const int nitem = a.nseq * a.Hkv;
-  const int grid = nitem < num_sms() ? nitem : num_sms();
-  if (grid <= 0) return 0;
-  decode_kernel<<<grid, kThreads, smem, s>>>(tmK, tmV, tmCK, tmCV, a);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return (int)e;
+  if (nitem <= 0) return 0;
+  const int cl = decode_cluster(nitem);
+  {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(std::min(nitem, num_sms() / cl) * cl));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cl;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = cl > 1 ? 1 : 0;
+    e = cudaLaunchKernelEx(&cfg, decode_kernel, tmK, tmV, tmCK, tmCV, a, cl);
+    if (e != cudaSuccess) return (int)e;
+  }
   {
     // the merge kernel may be scheduled before the main kernel has drained (it waits with griddepcontrol.wait)
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)nitem);
-    cfg.blockDim = dim3(kMergeGroups * D);
+    cfg.gridDim = dim3((unsigned)nitem * (16 / kMergeRows));
+    cfg.blockDim = dim3(3 * D);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
@@ -683,7 +814,7 @@ int launch_decode(const DecodeArgs& a, cudaStream_t s) {
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, decode_merge_kernel, a);
+    e = cudaLaunchKernelEx(&cfg, decode_merge_kernel, a, cl);
     if (e != cudaSuccess) return (int)e;
   }
   note_launches(2);
