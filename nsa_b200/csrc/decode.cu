@@ -53,10 +53,11 @@ struct Plan {   // tile pairs of one item's phases; CTA `rank` of a cluster take
   int n1p;     // pairs of ck tiles of pass 1
   int n2p;     // (ck, cv) pairs of pass 2: covers all of Tc
   int nw;      // window pairs
+  int cs;      // CTAs that share passes 1 and 2
   int w0;      // first window key
 };
 
-__device__ __forceinline__ Plan make_plan(const DecodeArgs& a, int seq) {
+__device__ __forceinline__ Plan make_plan(const DecodeArgs& a, int seq, int cl) {
   Plan p;
   p.row_k = a.cu_k[seq];
   p.row_c = a.cu_c[seq];
@@ -68,6 +69,10 @@ __device__ __forceinline__ Plan make_plan(const DecodeArgs& a, int seq) {
   const int nck = (p.Tc + 63) / 64;
   p.n1p = (nck + 1) / 2;
   p.n2p = nck;
+  // An exchange costs about as much as one pair (3500 cycles): with no more than a pair for each warp nothing is shared in the
+  // two passes, every CTA makes its own statistics and scores.  (Both passes or neither: that every CTA has sent its statistics
+  // also says that none still reads the scores of the item before.)
+  p.cs = p.n2p > kCons ? cl : 1;
   p.w0 = max(0, p.L - a.window);
   p.nw = a.window > 0 ? (p.L - p.w0 + 63) / 64 : 0;
   return p;
@@ -91,8 +96,8 @@ __device__ __forceinline__ uint32_t map_cta(uint32_t saddr, uint32_t cta) {   //
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(cta));
   return r;
 }
-__device__ __forceinline__ void st_cluster(uint32_t addr, float v) {
-  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+__device__ __forceinline__ void st_cluster(uint32_t addr, float2 v) {
+  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(v.x), "f"(v.y) : "memory");
 }
 __device__ __forceinline__ void arrive_cluster(uint32_t bar) {   // releases what this thread has seen, to the cluster
   asm volatile("fence.acq_rel.cluster;" ::: "memory");
@@ -135,6 +140,39 @@ __device__ __forceinline__ void pv_tile(float (&acc)[D / 8][4], const float (&sc
   uint32_t pf[4][4];
   acc_to_a_frags<8>(pf, sc);
   mma_a_b<D, 64>(acc, pf, vbase, PANEL, 0, lane);
+}
+
+// The n blocks with the highest pooled score (ties to the lower index), in order, by one warp: lane l holds the blocks l + 32 e as
+// integers that order like the scores, a round is two warp reductions and the owner's new maximum.  About 120 cycles per round
+// whatever the length (a shared-memory scan and a butterfly took 6400 cycles for 16 of 512, counting every block's rank 38000).
+template <int E>
+__device__ __forceinline__ int top_blocks(const float* pooled, int n_pool, int n_sel, int lane) {   // lane r: the r-th block, or -1
+  unsigned v[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int blk = lane + 32 * e;
+    const float x = blk < n_pool ? pooled[blk] : -1.f;
+    v[e] = x >= 0.f ? __float_as_uint(x) + 1u : 0u;   // 0: none (or taken)
+  }
+  int mine = -1;
+  for (int r = 0; r < n_sel; ++r) {
+    unsigned best = 0u;
+    int at = 0;
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+      if (v[e] > best) {
+        best = v[e];
+        at = e;
+      }
+    const unsigned top = __reduce_max_sync(0xffffffffu, best);
+    if (top == 0u) break;
+    const unsigned blk = __reduce_min_sync(0xffffffffu, best == top ? (unsigned)(lane + 32 * at) : 0xffffffffu);
+    if (lane == r) mine = (int)blk;
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+      if (blk == (unsigned)(lane + 32 * e)) v[e] = 0u;
+  }
+  return mine;
 }
 
 // One (K, V) pair of an online soft-max: keys key0 .. key0+63 of the tile are valid iff kmin <= key < kmax.
@@ -267,10 +305,10 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (item >= nitem) continue;
       const int sq = item / a.Hkv, h = item % a.Hkv;
       const int seq = a.order ? a.order[sq] : sq;
-      const Plan p = make_plan(a, seq);
+      const Plan p = make_plan(a, seq, cl);
       bool ok = true;
-      for (int j = rank; ok && j < p.n1p; j += cl) ok = issue2(&tmCK, p.row_c + j * 128, &tmCK, p.row_c + j * 128 + 64, h);
-      for (int j = rank; ok && j < p.n2p; j += cl) ok = issue2(&tmCK, p.row_c + j * 64, &tmCV, p.row_c + j * 64, h);
+      for (int j = p.cs > 1 ? rank : 0; ok && j < p.n1p; j += p.cs) ok = issue2(&tmCK, p.row_c + j * 128, &tmCK, p.row_c + j * 128 + 64, h);
+      for (int j = p.cs > 1 ? rank : 0; ok && j < p.n2p; j += p.cs) ok = issue2(&tmCK, p.row_c + j * 64, &tmCV, p.row_c + j * 64, h);
       for (int j = rank; ok && j < p.nw; j += cl) ok = issue2(&tmK, p.row_k + p.w0 + j * 64, &tmV, p.row_k + p.w0 + j * 64, h);
       // the selected blocks are known once the consumers have pooled the scores
       if (ok && lane == 0) ok = mbar_wait_abortable(sel_ready, it & 1, DEV_ERR_FULL_WAIT, abort_flag);
@@ -291,6 +329,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int cthreads = kCons * 32;
   const int ct = threadIdx.x;               // 0 .. cthreads-1
   uint32_t n0 = 0, it = 0;                  // tiles consumed by the CTA before the current phase; items so far
+  uint32_t nx = 0;                          // items with an exchange so far
   bool ok = true;
   // tile pair u (two consecutive tiles) of a phase that starts at tile counter base belongs to warp ((base/2 + u) % kCons)
   for (int r = 0; r * ngroup < nitem; ++r) {
@@ -298,7 +337,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (item >= nitem) continue;
     const int sq = item / a.Hkv, h = item % a.Hkv;
     const int seq = a.order ? a.order[sq] : sq;
-    const Plan p = make_plan(a, seq);
+    const Plan p = make_plan(a, seq, cl);
     const int t = p.L - 1;
     const long long qrow = (long long)seq * a.Hq + h * 16;     // first of the 16 (head) rows of this item
     uint32_t qf[D / 16][4];
@@ -310,7 +349,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     {
       const uint32_t pair0 = n0 / 2;
       int i = 0;   // this CTA's pairs
-      for (int u = rank; u < p.n1p; u += cl, ++i) {
+      for (int u = p.cs > 1 ? rank : 0; u < p.n1p; u += p.cs, ++i) {
         if ((int)((pair0 + i) % kCons) != warp) continue;
 #pragma unroll 1
         for (int e = 0; e < 2; ++e) {
@@ -380,28 +419,30 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (m1 > -INFINITY) Lr += stat[w * 64 + 16 + ct] * ex2(m1 - Mr);
         if (m2 > -INFINITY) La += stat[w * 64 + 48 + ct] * ex2(m2 - Ma);
       }
-      const float v[4] = {Mr, Lr, Ma, La};
-      for (int c = 0; c < cl; ++c) {
-        const uint32_t dst = smem_u32(xstat + rank * 64 + ct);
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (cl > 1) st_cluster(map_cta(dst, c) + 64 * e, v[e]); else xstat[16 * e + ct] = v[e];
-      }
+      float* own = xstat + rank * 64;
+      own[ct] = Mr;
+      own[16 + ct] = Lr;
+      own[32 + ct] = Ma;
+      own[48 + ct] = La;
     }
-    if (cl > 1) {
-      if (warp == 0) {
-        __syncwarp();
-        if (lane < cl) arrive_cluster(map_cta(xstat_bar, lane));
-        ok = ok && wait_cluster(xstat_bar, it & 1, 320, abort_flag);
-      }
+    if (p.cs > 1 && warp == 0) {
+      __syncwarp();
+      float* own = xstat + rank * 64 + 2 * lane;
+      const float2 v = *reinterpret_cast<const float2*>(own);
+      for (int c = 0; c < cl; ++c)
+        if (c != rank) st_cluster(map_cta(smem_u32(own), c), v);
+      __syncwarp();
+      if (lane < cl) arrive_cluster(map_cta(xstat_bar, lane));
+      ok = ok && wait_cluster(xstat_bar, nx & 1, 320, abort_flag);
     }
     if (ct < 16) {   // (written by this thread, or by the CTAs of the cluster)
       float Mr = -INFINITY, Ma = -INFINITY, Lr = 0.f, La = 0.f;
-      for (int c = 0; c < cl; ++c) {
+      const int c0 = p.cs > 1 ? 0 : rank, c1 = p.cs > 1 ? cl : rank + 1;
+      for (int c = c0; c < c1; ++c) {
         Mr = fmaxf(Mr, xstat[c * 64 + ct]);
         Ma = fmaxf(Ma, xstat[c * 64 + 32 + ct]);
       }
-      for (int c = 0; c < cl; ++c) {
+      for (int c = c0; c < c1; ++c) {
         const float m1 = xstat[c * 64 + ct], m2 = xstat[c * 64 + 32 + ct];
         if (m1 > -INFINITY) Lr += xstat[c * 64 + 16 + ct] * ex2(m1 - Mr);
         if (m2 > -INFINITY) La += xstat[c * 64 + 48 + ct] * ex2(m2 - Ma);
@@ -431,9 +472,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     {
       const uint32_t pair0 = n0 / 2;
       int i = 0;
-      for (int u = rank; u < p.n2p; u += cl, ++i) {
+      for (int u = p.cs > 1 ? rank : 0; u < p.n2p; u += p.cs, ++i) {
         if ((int)((pair0 + i) % kCons) != warp) continue;
-        full = true;
+        full = p.cs > 1 || rank == 0;
         const uint32_t nk = n0 + 2 * i, nv = nk + 1, sk = nk % kSlots, sv = nv % kSlots;
         const int j0 = u * 64;
         ok = ok && mbar_wait_abortable(full_bar(sk), (nk / kSlots) & 1, DEV_ERR_FULL_WAIT, abort_flag);
@@ -459,17 +500,16 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
           if (g == 0) {
             const int j = j0 + nt * 8 + 2 * tq;
-            if (cl == 1) {
-              if (j < p.Tc) ps[j] = c0;
-              if (j + 1 < p.Tc) ps[j + 1] = c1;
-            } else {
-              for (int c = 0; c < cl; ++c) {
-                const uint32_t dst = map_cta(smem_u32(ps + j), c);
-                if (j < p.Tc) st_cluster(dst, c0);
-                if (j + 1 < p.Tc) st_cluster(dst + 4, c1);
-              }
-            }
+            if (j < p.Tc) ps[j] = c0;
+            if (j + 1 < p.Tc) ps[j + 1] = c1;
           }
+        }
+        if (p.cs > 1) {   // the tile's 64 scores to the other CTAs (positions past Tc are there, and not read)
+          __syncwarp();
+          const float* src = ps + j0 + 2 * lane;
+          const float2 v = *reinterpret_cast<const float2*>(src);
+          for (int c = 0; c < cl; ++c)
+            if (c != rank) st_cluster(map_cta(smem_u32(src), c), v);
         }
         // attention weights with the final maximum (unnormalised; the sum divides at the end)
 #pragma unroll
@@ -480,7 +520,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             sc[nt][c] = (j < p.nvis) ? ex2(fmaf(sc[nt][c], sl2, -Ma[c >> 1])) : 0.f;
           }
         ok = ok && mbar_wait_abortable(full_bar(sv), (nv / kSlots) & 1, DEV_ERR_FULL_WAIT, abort_flag);
-        if (ok && j0 < p.nvis) pv_tile(acc, sc, ring + sv * TILE, lane);
+        if (ok && j0 < p.nvis && (p.cs > 1 || rank == 0)) pv_tile(acc, sc, ring + sv * TILE, lane);
         __syncwarp();
         if (lane == 0) mbar_arrive(empty_bar(sv));
       }
@@ -488,9 +528,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     // ---- pooled scores and the top-n (warp 0), the compressed-branch output (all warps, fixed order) ------------
     named_bar_sync(1, cthreads);            // ps complete
-    if (cl > 1) {   // in every CTA
+    if (p.cs > 1) {   // in every CTA
       if (ct < cl) arrive_cluster(map_cta(ps_bar, ct));
-      ok = ok && wait_cluster(ps_bar, it & 1, 321, abort_flag);
+      ok = ok && wait_cluster(ps_bar, nx & 1, 321, abort_flag);
+      ++nx;
     }
     const int n_pool = min(kMaxPoolD, pool_len(p.Tc, pool_k, pool_s));
     for (int blk = ct; blk < n_pool; blk += cthreads) {
@@ -499,40 +540,10 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int j = lo; j < hi; ++j) sum += ps[j];
       pooled[blk] = sum / (float)(hi - lo);
     }
-    if (ct < (-n_pool & 3)) pooled[n_pool + ct] = -INFINITY;   // whole groups of four below
-    if (ct < kMaxSel) sel[ct] = -1;
-    named_bar_sync(1, cthreads);
-    // Top-n by counting: a block's rank is the number of blocks with a higher score, or an equal one and a lower index (n
-    // rounds of a warp-wide maximum took 2 us for 64 blocks, 3.4 for 512).
-    {
-      constexpr int kOwn = (kMaxPoolD + kCons * 32 - 1) / (kCons * 32);
-      float v[kOwn];
-      int rk[kOwn];
-#pragma unroll
-      for (int e = 0; e < kOwn; ++e) {
-        const int blk = ct + e * cthreads;
-        v[e] = blk < n_pool ? pooled[blk] : INFINITY;
-        rk[e] = 0;
-      }
-      const int own = (n_pool + cthreads - 1) / cthreads;
-      for (int j = 0; j < n_pool; j += 4) {
-        const float4 x4 = *reinterpret_cast<const float4*>(pooled + j);
-        const float x[4] = {x4.x, x4.y, x4.z, x4.w};
-#pragma unroll
-        for (int e = 0; e < kOwn; ++e) {
-          if (e >= own) continue;
-#pragma unroll
-          for (int c = 0; c < 4; ++c) rk[e] += (x[c] > v[e] || (x[c] == v[e] && j + c < ct + e * cthreads)) ? 1 : 0;
-        }
-      }
-#pragma unroll
-      for (int e = 0; e < kOwn; ++e)
-        if (ct + e * cthreads < n_pool && rk[e] < a.n_sel) sel[rk[e]] = ct + e * cthreads;
-    }
     named_bar_sync(1, cthreads);
     if (warp == 0) {
-      const int blk = lane < a.n_sel ? sel[lane] : -1;   // n_sel <= kMaxSel = 32
-      if (rank == 0 && lane < a.n_sel) a.idx[((long long)seq * a.Hkv + h) * a.n_sel + lane] = blk;
+      const int blk = n_pool <= 128 ? top_blocks<4>(pooled, n_pool, a.n_sel, lane) : top_blocks<kMaxPoolD / 32>(pooled, n_pool, a.n_sel, lane);
+      if (rank == 0 && lane < a.n_sel) a.idx[((long long)seq * a.Hkv + h) * a.n_sel + lane] = blk;   // n_sel <= kMaxSel = 32
       const bool use = blk >= 0 && (long long)blk * 64 <= t;   // blocks that start after t are skipped
       const unsigned m = __ballot_sync(0xffffffffu, use);
       __syncwarp();
