@@ -27,6 +27,7 @@
 // against 0.21 ms); merging in the same kernel through an L2-resident scratch idled five of six warps and the TMA ring
 // during the merge (0.30 ms).  No atomics; every wait is bounded.
 #include <algorithm>
+#include <array>
 
 #include "kernels.h"
 #include "tmap.h"
@@ -750,10 +751,47 @@ __global__ void __launch_bounds__(3 * D) decode_merge_kernel(const DecodeArgs a,
   }
 }
 
+constexpr int decode_smem() {
+  return kSlots * (int)TILE + (kMaxTc + 64 + kMaxPoolD + kCons * 64 + 64 + kMaxCluster * 64) * 4 + (kMaxSel + 4) * 4 +
+         (2 * kSlots + 3) * 8 + 16 + 1024;
+}
+// The launch of `nitem` items with `cl` CTAs each, all resident at once as far as they fit.
+cudaLaunchConfig_t decode_config(int ncta, int cl, cudaLaunchAttribute* at, cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)ncta);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = decode_smem();
+  cfg.stream = s;
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = cl;
+  at->val.clusterDim.y = at->val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = cl > 1 ? 1 : 0;
+  return cfg;
+}
+// Clusters of cl CTAs that the GPU holds at a time (fewer than SMs / cl: a cluster lies within one GPC; 16 of 8 would be 128
+// of 148 SMs, but they do not all fit and the rest would run as a second wave).
+int resident_clusters(int cl) {
+  static const auto held = [] {
+    std::array<int, 4> n = {};
+    for (int i = 0; i < 4; ++i) {
+      n[i] = num_sms() >> i;
+      int c = 0;
+      cudaLaunchAttribute at;
+      const cudaLaunchConfig_t cfg = decode_config(num_sms() >> i << i, 1 << i, &at, nullptr);
+      if (i > 0 && cudaFuncSetAttribute(decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, decode_smem()) == cudaSuccess &&
+          cudaOccupancyMaxActiveClusters(&c, decode_kernel, &cfg) == cudaSuccess)
+        n[i] = c;
+      cudaGetLastError();   // (no device: workspace sizes can be asked for all the same)
+    }
+    return n;
+  }();
+  return held[cl == 8 ? 3 : cl == 4 ? 2 : cl == 2 ? 1 : 0];
+}
 // CTAs per item: as many as keep every item in the first wave.
 int decode_cluster(int nitem) {
   int cl = kMaxCluster;
-  while (cl > 1 && nitem * cl > num_sms()) cl >>= 1;
+  while (cl > 1 && nitem > resident_clusters(cl)) cl >>= 1;
   return cl;
 }
 
@@ -791,25 +829,14 @@ int launch_decode(const DecodeArgs& a, cudaStream_t s) {
     set_error("decode: workspace too small (%lld bytes needed)", (long long)decode_workspace_bytes(a.nseq, a.Hkv));
     return -6;
   }
-  const int smem = kSlots * (int)TILE + (kMaxTc + 64 + kMaxPoolD + kCons * 64 + 64 + kMaxCluster * 64) * 4 + (kMaxSel + 4) * 4 +
-                   (2 * kSlots + 3) * 8 + 16 + 1024;
-  cudaError_t e = cudaFuncSetAttribute(decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaError_t e = cudaFuncSetAttribute(decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, decode_smem());
   if (e != cudaSuccess) return (int)e;
   const int nitem = a.nseq * a.Hkv;
   if (nitem <= 0) return 0;
   const int cl = decode_cluster(nitem);
   {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(std::min(nitem, num_sms() / cl) * cl));
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = cl;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = cl > 1 ? 1 : 0;
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t cfg = decode_config(std::min(nitem, resident_clusters(cl)) * cl, cl, &at, s);
     e = cudaLaunchKernelEx(&cfg, decode_kernel, tmK, tmV, tmCK, tmCV, a, cl);
     if (e != cudaSuccess) return (int)e;
   }
