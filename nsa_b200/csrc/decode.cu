@@ -144,36 +144,59 @@ __device__ __forceinline__ void pv_tile(float (&acc)[D / 8][4], const float (&sc
 }
 
 // The n blocks with the highest pooled score (ties to the lower index), in order, by one warp: lane l holds the blocks l + 32 e as
-// integers that order like the scores, a round is two warp reductions and the owner's new maximum.  About 120 cycles per round
-// whatever the length (a shared-memory scan and a butterfly took 6400 cycles for 16 of 512, counting every block's rank 38000).
+// integers that order like the scores.  The n-th highest is found bit by bit with ballots, the n survivors are ranked among
+// themselves.  (n rounds of a shared-memory scan and a butterfly took 6400 cycles for 16 of 512 blocks, n rounds of two integer
+// warp reductions 18000, counting every block's rank with all warps 38000.)
 template <int E>
-__device__ __forceinline__ int top_blocks(const float* pooled, int n_pool, int n_sel, int lane) {   // lane r: the r-th block, or -1
+__device__ __forceinline__ int top_blocks(const float* pooled, int2* tmp, int n_pool, int n_sel, int lane) {   // lane r: the r-th, or -1
   unsigned v[E];
+  int valid = 0;
 #pragma unroll
   for (int e = 0; e < E; ++e) {
     const int blk = lane + 32 * e;
     const float x = blk < n_pool ? pooled[blk] : -1.f;
-    v[e] = x >= 0.f ? __float_as_uint(x) + 1u : 0u;   // 0: none (or taken)
+    v[e] = x >= 0.f ? __float_as_uint(x) + 1u : 0u;   // 0: none
+    valid += __popc(__ballot_sync(0xffffffffu, v[e] != 0u));
   }
-  int mine = -1;
-  for (int r = 0; r < n_sel; ++r) {
-    unsigned best = 0u;
-    int at = 0;
+  const int n = min(n_sel, valid);
+  if (n == 0) return -1;
+  unsigned thr = 0u;   // the highest value that at least n blocks reach
+  int cnt = 0;         // ... and how many do
+  for (unsigned bit = 1u << 30; bit; bit >>= 1) {
+    int c = 0;
 #pragma unroll
-    for (int e = 0; e < E; ++e)
-      if (v[e] > best) {
-        best = v[e];
-        at = e;
-      }
-    const unsigned top = __reduce_max_sync(0xffffffffu, best);
-    if (top == 0u) break;
-    const unsigned blk = __reduce_min_sync(0xffffffffu, best == top ? (unsigned)(lane + 32 * at) : 0xffffffffu);
-    if (lane == r) mine = (int)blk;
-#pragma unroll
-    for (int e = 0; e < E; ++e)
-      if (blk == (unsigned)(lane + 32 * e)) v[e] = 0u;
+    for (int e = 0; e < E; ++e) c += __popc(__ballot_sync(0xffffffffu, v[e] >= (thr | bit)));
+    if (c >= n) {
+      thr |= bit;
+      cnt = c;
+      if (c == n) break;
+    }
   }
-  return mine;
+  int above = 0;       // all of these, and the first n - above of those at the threshold
+#pragma unroll
+  for (int e = 0; e < E; ++e) above += __popc(__ballot_sync(0xffffffffu, v[e] > thr));
+  const unsigned below = (1u << lane) - 1u;
+  int k = 0, ties = cnt == n ? n : n - above;
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const unsigned eq = __ballot_sync(0xffffffffu, v[e] == thr);
+    const bool take = v[e] > thr || (v[e] == thr && __popc(eq & below) < ties);
+    const unsigned m = __ballot_sync(0xffffffffu, take);
+    if (take) tmp[k + __popc(m & below)] = make_int2((int)v[e], lane + 32 * e);
+    k += __popc(m);
+    ties -= min(ties, __popc(eq));
+  }
+  __syncwarp();
+  const int2 own = lane < n ? tmp[lane] : make_int2(0, 0);
+  int rank = 0;
+  for (int i = 0; i < n; ++i) {
+    const int2 x = tmp[i];
+    rank += (x.x > own.x || (x.x == own.x && x.y < own.y)) ? 1 : 0;
+  }
+  __syncwarp();
+  if (lane < n) tmp[rank].x = own.y;
+  __syncwarp();
+  return lane < n ? tmp[lane].x : -1;
 }
 
 // One (K, V) pair of an online soft-max: keys key0 .. key0+63 of the tile are valid iff kmin <= key < kmax.
@@ -543,7 +566,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     named_bar_sync(1, cthreads);
     if (warp == 0) {
-      const int blk = n_pool <= 128 ? top_blocks<4>(pooled, n_pool, a.n_sel, lane) : top_blocks<kMaxPoolD / 32>(pooled, n_pool, a.n_sel, lane);
+      const int blk = n_pool <= 128 ? top_blocks<4>(pooled, reinterpret_cast<int2*>(stat), n_pool, a.n_sel, lane) : top_blocks<kMaxPoolD / 32>(pooled, reinterpret_cast<int2*>(stat), n_pool, a.n_sel, lane);
       if (rank == 0 && lane < a.n_sel) a.idx[((long long)seq * a.Hkv + h) * a.n_sel + lane] = blk;   // n_sel <= kMaxSel = 32
       const bool use = blk >= 0 && (long long)blk * 64 <= t;   // blocks that start after t are skipped
       const unsigned m = __ballot_sync(0xffffffffu, use);
