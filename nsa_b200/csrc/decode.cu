@@ -669,6 +669,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 // per (branch, channel).  Branch order in the workspace: 0 compressed, 1 selected, 2 window.  Warps that had no tile are left
 // out.  Pure latency: the loads of a branch's partials are independent, and the gates (computed from q when the gate projection
 // is given) do not wait for them.
+static_assert(kMaxCluster * kCons <= 64, "two partials per lane below");
 constexpr int kMergeRows = 4;
 __global__ void __launch_bounds__(3 * D) decode_merge_kernel(const DecodeArgs a, const int cl) {
   const int item = blockIdx.x / (16 / kMergeRows), r0 = blockIdx.x % (16 / kMergeRows) * kMergeRows;
@@ -678,9 +679,9 @@ __global__ void __launch_bounds__(3 * D) decode_merge_kernel(const DecodeArgs a,
   const long long qrow = (long long)seq * a.Hq + h * 16 + r0;
   const int tid = threadIdx.x, lane = tid & 31, br = tid / D, d = tid % D;
   const float* part = a.part + (long long)item * 3 * nw * kPartFloats;
-  __shared__ int act_s[3][kMaxCluster * kCons], nact_s[3];          // warps with a partial
-  __shared__ __align__(16) float ml_s[3][kMaxCluster * kCons][2][kMergeRows];
-  __shared__ float w_s[3][kMaxCluster * kCons][kMergeRows];         // per (branch, warp, row): 2^(m_w - M) / L
+  __shared__ int act_s[3][kMaxCluster * kCons], nact_s[3];                  // warps of the other CTAs with a partial
+  __shared__ __align__(16) float wfirst_s[3][kCons][kMergeRows];            // weights 2^(m_w - M) / L of the first CTA's warps
+  __shared__ __align__(16) float w_s[3][kMaxCluster * kCons][kMergeRows];   // and of those
   __shared__ float gp_s[3][D / 32][kMergeRows];                     // gate projection: per-warp partial dot products
   __shared__ bf16 out_s[3][kMergeRows][D];
   __shared__ float gate_s[3][kMergeRows];                           // order: compressed, selected, window
@@ -700,37 +701,58 @@ __global__ void __launch_bounds__(3 * D) decode_merge_kernel(const DecodeArgs a,
   // Launched with programmatic stream serialization: everything above (the gate projection reads only q and the
   // weights) may run while the main kernel is still finishing; its partials are read only behind this wait.
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (tid % D < 32) {   // the first warp of each branch
-    const float* base = part + (long long)br * nw * kPartFloats + 16 * D + r0;
-    int n = 0;
-    for (int w0 = 0; w0 < nw; w0 += 32) {
-      const int w = w0 + lane;
-      float4 m = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY), l = m;
+  const float* base = part + (long long)br * nw * kPartFloats + r0 * D + d;
+  float first[kCons][kMergeRows];   // the partials of the first CTA, under way while the weights are formed
+#pragma unroll
+  for (int w = 0; w < kCons; ++w)
+#pragma unroll
+    for (int i = 0; i < kMergeRows; ++i) first[w][i] = base[w * kPartFloats + i * D];
+  if (d < 32) {   // the first warp of each branch: weights of up to 64 partials, two per lane
+    const float* hd = part + (long long)br * nw * kPartFloats + 16 * D + r0;
+    float4 m[2], l[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      m[k] = l[k] = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+      const int w = lane + 32 * k;
       if (w < nw) {
-        m = *reinterpret_cast<const float4*>(base + (long long)w * kPartFloats);
-        l = *reinterpret_cast<const float4*>(base + (long long)w * kPartFloats + 16);
+        m[k] = *reinterpret_cast<const float4*>(hd + (long long)w * kPartFloats);
+        l[k] = *reinterpret_cast<const float4*>(hd + (long long)w * kPartFloats + 16);
       }
-      const bool on = fmaxf(fmaxf(m.x, m.y), fmaxf(m.z, m.w)) > -INFINITY;
+    }
+    float wt[2][kMergeRows];
+#pragma unroll
+    for (int i = 0; i < kMergeRows; ++i) {
+      const float m0 = i == 0 ? m[0].x : i == 1 ? m[0].y : i == 2 ? m[0].z : m[0].w;
+      const float m1 = i == 0 ? m[1].x : i == 1 ? m[1].y : i == 2 ? m[1].z : m[1].w;
+      const float l0 = i == 0 ? l[0].x : i == 1 ? l[0].y : i == 2 ? l[0].z : l[0].w;
+      const float l1 = i == 0 ? l[1].x : i == 1 ? l[1].y : i == 2 ? l[1].z : l[1].w;
+      float M = fmaxf(m0, m1);
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
+      const float e0 = m0 > -INFINITY ? ex2(m0 - M) : 0.f, e1 = m1 > -INFINITY ? ex2(m1 - M) : 0.f;
+      float L = (m0 > -INFINITY ? l0 * e0 : 0.f) + (m1 > -INFINITY ? l1 * e1 : 0.f);
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) L += __shfl_xor_sync(0xffffffffu, L, off);
+      wt[0][i] = L > 0.f ? e0 / L : 0.f;
+      wt[1][i] = L > 0.f ? e1 / L : 0.f;
+      if (a.lse && lane == 0 && !(br == 2 && a.window <= 0))
+        a.lse[(long long)br * a.nseq * a.Hq + qrow + i] = L > 0.f ? (M + log2f(L)) * kLn2 : -INFINITY;
+    }
+    int n = 0;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int w = lane + 32 * k;
+      if (w < kCons) *reinterpret_cast<float4*>(wfirst_s[br][w]) = make_float4(wt[k][0], wt[k][1], wt[k][2], wt[k][3]);
+      const bool on = w >= kCons && w < nw && fmaxf(fmaxf(m[k].x, m[k].y), fmaxf(m[k].z, m[k].w)) > -INFINITY;
       const unsigned mask = __ballot_sync(0xffffffffu, on);
       if (on) {
         const int i = n + __popc(mask & ((1u << lane) - 1));
         act_s[br][i] = w;
-        *reinterpret_cast<float4*>(ml_s[br][i][0]) = m;
-        *reinterpret_cast<float4*>(ml_s[br][i][1]) = l;
+        *reinterpret_cast<float4*>(w_s[br][i]) = make_float4(wt[k][0], wt[k][1], wt[k][2], wt[k][3]);
       }
       n += __popc(mask);
     }
-    __syncwarp();
     if (lane == 0) nact_s[br] = n;
-    if (lane < kMergeRows) {
-      float M = -INFINITY, L = 0.f;
-      for (int i = 0; i < n; ++i) M = fmaxf(M, ml_s[br][i][0][lane]);
-      for (int i = 0; i < n; ++i)
-        if (ml_s[br][i][0][lane] > -INFINITY) L += ml_s[br][i][1][lane] * ex2(ml_s[br][i][0][lane] - M);
-      for (int i = 0; i < n; ++i) w_s[br][i][lane] = (ml_s[br][i][0][lane] > -INFINITY && L > 0.f) ? ex2(ml_s[br][i][0][lane] - M) / L : 0.f;
-      if (a.lse && !(br == 2 && a.window <= 0))
-        a.lse[(long long)br * a.nseq * a.Hq + qrow + lane] = L > 0.f ? (M + log2f(L)) * kLn2 : -INFINITY;
-    }
   }
   __syncthreads();
   if (d < kMergeRows) {
@@ -746,10 +768,16 @@ __global__ void __launch_bounds__(3 * D) decode_merge_kernel(const DecodeArgs a,
     }
     gate_s[br][d] = gv;
   }
-  const float* base = part + (long long)br * nw * kPartFloats + r0 * D + d;
   float v[kMergeRows];
 #pragma unroll
   for (int i = 0; i < kMergeRows; ++i) v[i] = 0.f;
+#pragma unroll
+  for (int w = 0; w < kCons; ++w)
+#pragma unroll
+    for (int i = 0; i < kMergeRows; ++i) {
+      const float wt = wfirst_s[br][w][i];
+      if (wt != 0.f) v[i] += first[w][i] * wt;   // (a warp without a tile has left no output)
+    }
   const int n = nact_s[br];
 #pragma unroll 6
   for (int k = 0; k < n; ++k) {
