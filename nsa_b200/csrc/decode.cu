@@ -665,140 +665,125 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
-// Merge of the per-warp partials, in a fixed order (CTA by CTA, warp by warp): one block per (item, four query rows), one thread
-// per (branch, channel).  Branch order in the workspace: 0 compressed, 1 selected, 2 window.  Warps that had no tile are left
-// out.  Pure latency: the loads of a branch's partials are independent, and the gates (computed from q when the gate projection
-// is given) do not wait for them.
+// Merge of the per-warp partials, in a fixed order (CTA by CTA, warp by warp): one warp per (item, query row, branch), a lane holds
+// four channels.  Branch order in the workspace: 0 compressed, 1 selected, 2 window.  Warps that had no tile are left out.  The
+// loads of the first CTA's partials (all of them without clusters) are under way while their weights are formed in the warp;
+// the gates (computed from q when the gate projection is given) do not wait for the main kernel.  Few registers and blocks of
+// two rows: what is in flight is what counts (512 items are 77 MB; four rows and 64 registers took 36 us, one block per item with a
+// thread per channel 19).
+constexpr int kMergeRows = 2;
 static_assert(kMaxCluster * kCons <= 64, "two partials per lane below");
-constexpr int kMergeRows = 4;
-__global__ void __launch_bounds__(3 * D) decode_merge_kernel(const DecodeArgs a, const int cl) {
-  const int item = blockIdx.x / (16 / kMergeRows), r0 = blockIdx.x % (16 / kMergeRows) * kMergeRows;
+__global__ void __launch_bounds__(96 * kMergeRows) decode_merge_kernel(const DecodeArgs a, const int cl) {
+  const int item = blockIdx.x / (16 / kMergeRows);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, br = warp % 3;
+  const int r = blockIdx.x % (16 / kMergeRows) * kMergeRows + warp / 3;
   const int nw = cl * kCons;
   const int sq = item / a.Hkv, h = item % a.Hkv;
   const int seq = a.order ? a.order[sq] : sq;
-  const long long qrow = (long long)seq * a.Hq + h * 16 + r0;
-  const int tid = threadIdx.x, lane = tid & 31, br = tid / D, d = tid % D;
-  const float* part = a.part + (long long)item * 3 * nw * kPartFloats;
-  __shared__ int act_s[3][kMaxCluster * kCons], nact_s[3];                  // warps of the other CTAs with a partial
-  __shared__ __align__(16) float wfirst_s[3][kCons][kMergeRows];            // weights 2^(m_w - M) / L of the first CTA's warps
-  __shared__ __align__(16) float w_s[3][kMaxCluster * kCons][kMergeRows];   // and of those
-  __shared__ float gp_s[3][D / 32][kMergeRows];                     // gate projection: per-warp partial dot products
-  __shared__ bf16 out_s[3][kMergeRows][D];
-  __shared__ float gate_s[3][kMergeRows];                           // order: compressed, selected, window
-  const int x = br == 0 ? 2 : br - 1;       // branch (cmp, slc, swa) -> row of the gate weight (slc, swa, cmp)
-  if (a.gate_w) {
-    // g_x[row] = q[row,:] . W[x,:] + b[x] (nn.Linear(head_dim, 3), rows of W: selected, window, compressed), rounded to
-    // bf16 as the module's gate tensors are
-    const float w = __bfloat162float(a.gate_w[x * D + d]);
-#pragma unroll
-    for (int i = 0; i < kMergeRows; ++i) {
-      float p = __bfloat162float(a.q[(qrow + i) * D + d]) * w;
+  const long long qrow = (long long)seq * a.Hq + h * 16 + r;
+  __shared__ float4 out_s[kMergeRows][3][32];
+  __shared__ float gate_s[kMergeRows][3];
+  const bool has = !(br == 2 && a.window <= 0);
+  {
+    const bf16* gin = br == 0 ? a.g_cmp : br == 1 ? a.g_slc : a.g_swa;
+    float gv = 1.f;
+    if (a.gate_w) {
+      // g_x[row] = q[row,:] . W[x,:] + b[x] (nn.Linear(head_dim, 3), rows of W: selected, window, compressed), rounded to
+      // bf16 as the module's gate tensors are
+      const int x = br == 0 ? 2 : br - 1;
+      const uint2 wv = *reinterpret_cast<const uint2*>(a.gate_w + x * D + lane * 4), qv = *reinterpret_cast<const uint2*>(a.q + qrow * D + lane * 4);
+      const float2 w0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&wv.x)), w1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&wv.y));
+      const float2 q0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&qv.x)), q1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&qv.y));
+      float p = q0.x * w0.x + q0.y * w0.y + q1.x * w1.x + q1.y * w1.y;
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) p += __shfl_xor_sync(0xffffffffu, p, off);
-      if (lane == 0) gp_s[br][d >> 5][i] = p;
+      if (a.gate_b) p += __bfloat162float(a.gate_b[x]);
+      gv = __bfloat162float(__float2bfloat16(p));
+    } else if (gin) {
+      gv = __bfloat162float(gin[qrow]);
     }
+    if (lane == 0) gate_s[warp / 3][br] = gv;
   }
   // Launched with programmatic stream serialization: everything above (the gate projection reads only q and the
   // weights) may run while the main kernel is still finishing; its partials are read only behind this wait.
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  const float* base = part + (long long)br * nw * kPartFloats + r0 * D + d;
-  float first[kCons][kMergeRows];   // the partials of the first CTA, under way while the weights are formed
-#pragma unroll
-  for (int w = 0; w < kCons; ++w)
-#pragma unroll
-    for (int i = 0; i < kMergeRows; ++i) first[w][i] = base[w * kPartFloats + i * D];
-  if (d < 32) {   // the first warp of each branch: weights of up to 64 partials, two per lane
-    const float* hd = part + (long long)br * nw * kPartFloats + 16 * D + r0;
-    float4 m[2], l[2];
+  if (has) {
+    const float* part = a.part + ((long long)item * 3 + br) * nw * kPartFloats;
+    const float* hd = part + 16 * D + r;
+    float m[2], l[2];
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-      m[k] = l[k] = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+      m[k] = -INFINITY;
+      l[k] = 0.f;
       const int w = lane + 32 * k;
       if (w < nw) {
-        m[k] = *reinterpret_cast<const float4*>(hd + (long long)w * kPartFloats);
-        l[k] = *reinterpret_cast<const float4*>(hd + (long long)w * kPartFloats + 16);
+        m[k] = hd[w * kPartFloats];
+        l[k] = hd[w * kPartFloats + 16];
       }
     }
-    float wt[2][kMergeRows];
+    const float4* base = reinterpret_cast<const float4*>(part + r * D) + lane;
+    float4 first[kCons];
 #pragma unroll
-    for (int i = 0; i < kMergeRows; ++i) {
-      const float m0 = i == 0 ? m[0].x : i == 1 ? m[0].y : i == 2 ? m[0].z : m[0].w;
-      const float m1 = i == 0 ? m[1].x : i == 1 ? m[1].y : i == 2 ? m[1].z : m[1].w;
-      const float l0 = i == 0 ? l[0].x : i == 1 ? l[0].y : i == 2 ? l[0].z : l[0].w;
-      const float l1 = i == 0 ? l[1].x : i == 1 ? l[1].y : i == 2 ? l[1].z : l[1].w;
-      float M = fmaxf(m0, m1);
+    for (int w = 0; w < kCons; ++w) first[w] = base[w * (kPartFloats / 4)];
+    float M = fmaxf(m[0], m[1]);
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
-      const float e0 = m0 > -INFINITY ? ex2(m0 - M) : 0.f, e1 = m1 > -INFINITY ? ex2(m1 - M) : 0.f;
-      float L = (m0 > -INFINITY ? l0 * e0 : 0.f) + (m1 > -INFINITY ? l1 * e1 : 0.f);
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) L += __shfl_xor_sync(0xffffffffu, L, off);
-      wt[0][i] = L > 0.f ? e0 / L : 0.f;
-      wt[1][i] = L > 0.f ? e1 / L : 0.f;
-      if (a.lse && lane == 0 && !(br == 2 && a.window <= 0))
-        a.lse[(long long)br * a.nseq * a.Hq + qrow + i] = L > 0.f ? (M + log2f(L)) * kLn2 : -INFINITY;
-    }
-    int n = 0;
+    for (int off = 16; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
+    float e[2], L = 0.f;
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-      const int w = lane + 32 * k;
-      if (w < kCons) *reinterpret_cast<float4*>(wfirst_s[br][w]) = make_float4(wt[k][0], wt[k][1], wt[k][2], wt[k][3]);
-      const bool on = w >= kCons && w < nw && fmaxf(fmaxf(m[k].x, m[k].y), fmaxf(m[k].z, m[k].w)) > -INFINITY;
-      const unsigned mask = __ballot_sync(0xffffffffu, on);
-      if (on) {
-        const int i = n + __popc(mask & ((1u << lane) - 1));
-        act_s[br][i] = w;
-        *reinterpret_cast<float4*>(w_s[br][i]) = make_float4(wt[k][0], wt[k][1], wt[k][2], wt[k][3]);
+      e[k] = m[k] > -INFINITY ? ex2(m[k] - M) : 0.f;
+      if (m[k] > -INFINITY) L += l[k] * e[k];
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) L += __shfl_xor_sync(0xffffffffu, L, off);
+    const float inv = L > 0.f ? 1.f / L : 0.f;
+    e[0] *= inv;
+    e[1] *= inv;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto add = [&](const float4& x, float w) {
+      v.x += x.x * w; v.y += x.y * w; v.z += x.z * w; v.w += x.w * w;
+    };
+#pragma unroll
+    for (int w = 0; w < kCons; ++w) {
+      const float wt = __shfl_sync(0xffffffffu, e[0], w);
+      if (wt != 0.f) add(first[w], wt);   // (a warp without a tile has left no output)
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      unsigned rest = __ballot_sync(0xffffffffu, e[k] != 0.f && (k || lane >= kCons));
+      while (rest) {   // of the other CTAs, four at a time
+        float4 x[4];
+        float wt[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int w = rest ? __ffs(rest) - 1 : 0;
+          wt[u] = rest ? __shfl_sync(0xffffffffu, e[k], w) : 0.f;
+          if (rest) x[u] = base[(w + 32 * k) * (kPartFloats / 4)];
+          rest &= rest - 1;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (wt[u] != 0.f) add(x[u], wt[u]);
       }
-      n += __popc(mask);
     }
-    if (lane == 0) nact_s[br] = n;
+    __nv_bfloat162 b0 = __floats2bfloat162_rn(v.x, v.y), b1 = __floats2bfloat162_rn(v.z, v.w);
+    bf16* out = br == 0 ? a.o_cmp : br == 1 ? a.o_slc : a.o_swa;
+    if (out) *reinterpret_cast<uint2*>(out + qrow * D + lane * 4) = make_uint2(*reinterpret_cast<uint32_t*>(&b0), *reinterpret_cast<uint32_t*>(&b1));
+    if (a.lse && lane == 0) a.lse[(long long)br * a.nseq * a.Hq + qrow] = L > 0.f ? (M + log2f(L)) * kLn2 : -INFINITY;
+    const float2 f0 = __bfloat1622float2(b0), f1 = __bfloat1622float2(b1);
+    out_s[warp / 3][br][lane] = make_float4(f0.x, f0.y, f1.x, f1.y);
   }
   __syncthreads();
-  if (d < kMergeRows) {
-    const bf16* gin = br == 0 ? a.g_cmp : br == 1 ? a.g_slc : a.g_swa;
-    float gv = 1.f;
-    if (a.gate_w) {
-      float sum = 0.f;
-      for (int w = 0; w < D / 32; ++w) sum += gp_s[br][w][d];
-      if (a.gate_b) sum += __bfloat162float(a.gate_b[x]);
-      gv = __bfloat162float(__float2bfloat16(sum));
-    } else if (gin) {
-      gv = __bfloat162float(gin[qrow + d]);
+  if (br == 0) {
+    float4 tot = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+      if (x == 2 && a.window <= 0) continue;
+      const float g = gate_s[warp / 3][x];
+      const float4 f = out_s[warp / 3][x][lane];
+      tot.x += g * f.x; tot.y += g * f.y; tot.z += g * f.z; tot.w += g * f.w;
     }
-    gate_s[br][d] = gv;
-  }
-  float v[kMergeRows];
-#pragma unroll
-  for (int i = 0; i < kMergeRows; ++i) v[i] = 0.f;
-#pragma unroll
-  for (int w = 0; w < kCons; ++w)
-#pragma unroll
-    for (int i = 0; i < kMergeRows; ++i) {
-      const float wt = wfirst_s[br][w][i];
-      if (wt != 0.f) v[i] += first[w][i] * wt;   // (a warp without a tile has left no output)
-    }
-  const int n = nact_s[br];
-#pragma unroll 6
-  for (int k = 0; k < n; ++k) {
-    const float* src = base + (long long)act_s[br][k] * kPartFloats;
-#pragma unroll
-    for (int i = 0; i < kMergeRows; ++i) v[i] += src[i * D] * w_s[br][k][i];
-  }
-  bf16* outs = br == 0 ? a.o_cmp : br == 1 ? a.o_slc : a.window > 0 ? a.o_swa : nullptr;
-#pragma unroll
-  for (int i = 0; i < kMergeRows; ++i) {
-    const bf16 vb = __float2bfloat16(v[i]);
-    out_s[br][i][d] = vb;
-    if (outs) outs[(qrow + i) * D + d] = vb;
-  }
-  __syncthreads();
-  for (int i = br; i < kMergeRows; i += 3) {
-    float tot = 0.f;
-#pragma unroll
-    for (int b = 0; b < 3; ++b)
-      if (!(b == 2 && a.window <= 0)) tot += gate_s[b][i] * __bfloat162float(out_s[b][i][d]);
-    a.o[(qrow + i) * D + d] = __float2bfloat16(tot);
+    *reinterpret_cast<uint2*>(a.o + qrow * D + lane * 4) = make_uint2(pack_bf16(tot.x, tot.y), pack_bf16(tot.z, tot.w));
   }
 }
 
@@ -895,7 +880,7 @@ int launch_decode(const DecodeArgs& a, cudaStream_t s) {
     // the merge kernel may be scheduled before the main kernel has drained (it waits with griddepcontrol.wait)
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)nitem * (16 / kMergeRows));
-    cfg.blockDim = dim3(3 * D);
+    cfg.blockDim = dim3(96 * kMergeRows);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
