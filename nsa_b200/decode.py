@@ -111,37 +111,44 @@ def extend_compress_cache(module, cache, k, v, cu_seqlens_k):
     return _build(module, k, v, cu_seqlens_k, cache)
 
 
-@torch.no_grad()
 def nsa_decode(module, q, k, v, cu_seqlens_k, cache=None, return_parts=False):
     """q [nseq,Hq,D] (the newest token of every sequence), k, v [sum L,Hkv,D] packed with cu_seqlens_k.
     Returns o [nseq,Hq,D].  ``cache`` = a CompressedCache from ``compress_cache`` / ``extend_compress_cache`` skips the
     re-compression.  With ``return_parts`` also returns (o_cmp, o_slc, o_swa, lse [3,nseq,Hq], idx [nseq,Hkv,n])."""
+    # (nothing below is recorded by autograd: the step takes pointers.  For one short sequence the kernels take 17 us, so the
+    # host path counts: no grad-mode switch, no detached views, one allocation)
     q = _lib.require(q, "q")
     k = _lib.require(k, "k")
     v = _lib.require(v, "v")
     nseq, Hq, D = q.shape
     Hkv = k.shape[1]
     if cache is None:
-        cache = compress_cache(module, k, v, cu_seqlens_k)
+        with torch.no_grad():
+            cache = compress_cache(module, k, v, cu_seqlens_k)
     scale = module.softmax_scale
     if scale is None or scale is True:
         scale = 1.0 if scale is True else D ** -0.5
-    w_gate = _lib.require(module.gating.weight.detach(), "gating.weight")
-    b_gate = _lib.require(module.gating.bias.detach(), "gating.bias") if module.gating.bias is not None else None
-    o = torch.empty_like(q)
+    gating = module.gating
+    w_gate, b_gate = _lib.require(gating.weight, "gating.weight"), _lib.require(gating.bias, "gating.bias")
+    P, L = _lib.ptr, _lib.lib()
     n_sel = module.selected_block_count
-    idx = torch.empty(nseq, Hkv, n_sel, dtype=torch.int32, device=q.device)
+    o = torch.empty_like(q)
+    ws_bytes = L.nsa_decode_workspace_bytes(nseq, Hkv)
+    ck, total_k = cache.ck, k.shape[0]
     o_cmp = o_slc = o_swa = lse = None
     if return_parts:
+        idx = torch.empty(nseq, Hkv, n_sel, dtype=torch.int32, device=q.device)
         o_cmp, o_slc, o_swa = (torch.empty_like(q) for _ in range(3))
         lse = torch.empty(3, nseq, Hq, dtype=torch.float32, device=q.device)
-    P, L = _lib.ptr, _lib.lib()
-    ws_bytes = L.nsa_decode_workspace_bytes(nseq, Hkv)
-    ws = cache.workspace(ws_bytes)
+        ws = P(cache.workspace(ws_bytes))
+        idx_p = P(idx)
+    else:   # the selected blocks are scratch too
+        ws = P(cache.workspace(ws_bytes + 4 * nseq * Hkv * n_sel))
+        idx_p = ws + ws_bytes
     tab = P(cache.table_dev)
-    _lib.check(L.nsa_decode_fwd(P(q), P(k), P(v), P(cache.ck), P(cache.cv), tab, tab + 4 * (nseq + 1),
+    _lib.check(L.nsa_decode_fwd(P(q), P(k), P(v), P(ck), P(cache.cv), tab, tab + 4 * (nseq + 1),
                                 tab + 4 * (5 * nseq + 4), P(w_gate), P(b_gate), None, None, None, P(o), P(o_cmp), P(o_slc),
-                                P(o_swa), P(lse), P(idx), P(ws), ws_bytes, nseq, k.shape[0], cache.ck.shape[0],
+                                P(o_swa), P(lse), idx_p, ws, ws_bytes, nseq, total_k, ck.shape[0],
                                 cache.max_tc, Hq, Hkv, D, module.compression_block, module.compression_stride,
                                 module.selection_block_size, n_sel, module.sliding_window, float(scale),
                                 _lib.stream()), "nsa_decode_fwd")
