@@ -2,7 +2,7 @@
 // decomposition and reference semantics as kv_bwd.cu (nsa/selection_attn.py:151-253 through a reverse index), different engine.
 //
 // One CTA owns 64 keys.  Query tokens that see them arrive in batches of 8: the 8 x 16 (token, head) rows form a
-// [128 x D] tile of Q and of dO in shared memory (8 TMA boxes of 16 rows each, 128-byte swizzle).  Per batch, one
+// [128 x D] tile of Q and of dO in shared memory (one 4 KB TMA box per token, 128-byte swizzle).  Per batch, one
 // thread issues four groups of tcgen05.mma (accumulators in TMEM):
 //     S   [128 rows x 64 keys] = Qg . K^T          A = Qg (K-major),  B = K  (K-major)
 //     dP  [128 rows x 64 keys] = dOg . V^T         A = dOg (K-major), B = V  (K-major)
@@ -43,8 +43,7 @@ constexpr int kDrainThreads = 128;         // one thread per row
 constexpr int kTokB = 8;                   // tokens per batch (x16 heads = 128 rows)
 constexpr uint32_t KV_PANEL = 64 * 128;    // [64 keys][64 ch]
 constexpr uint32_t KV_TILE = 2 * KV_PANEL; // 16 KB
-constexpr uint32_t Q_PANEL = 128 * 128;    // [128 rows][64 ch]
-constexpr uint32_t Q_TILE = 2 * Q_PANEL;   // 32 KB
+constexpr uint32_t Q_TILE = 128 * 256;     // 32 KB: [16 row groups][2 column panels][8 rows][128 B]
 constexpr uint32_t STAGE = 2 * Q_TILE;     // Q + dO
 constexpr uint32_t P_TILE = 128 * 128;     // [128 rows][64 keys]
 constexpr int kStages = 2;
@@ -128,8 +127,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
   if (warp < kProd) {
     // ------------------------------- TMA producers -----------------------------------------------
-    // A batch of gathered tokens (a reverse-index list) is 32 boxes of 2 KB: (token j, Q or dO, column panel).  Box
-    // x = 3 * lane + warp belongs to this lane; every producer warp issues its 10 or 11 boxes with a single instruction
+    // A batch of gathered tokens (a reverse-index list) is 16 boxes of 4 KB, one per token of Q and one of dO, through a 4-D
+    // view (64 columns, 8 rows, 2 column panels, row groups) as in the forward: the gather is bound by the number of
+    // boxes.  Box x = 2 * lane + warp belongs to this lane; every producer warp issues its eight with a single instruction
     // and arms the stage's barrier with their byte count.  Token ids are fetched one batch ahead.
     if (warp == 0 && lane == 0 && nb > 0) {
       mbar_expect_tx(kv_bar, 2 * KV_TILE);
@@ -139,10 +139,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         tma_load_4d(v_s + p * KV_PANEL, &tmV, kv_bar, p * 64, hk, key0, b);
       }
     }
-    const int x = kProd * lane + warp;          // this lane's box of every batch (none if >= 32)
-    const bool has = x < 4 * kTokB;
-    const int bj = x & 7, bwhich = (x >> 3) & 1, bp = x >> 4;
-    const int nmine = (4 * kTokB - warp + kProd - 1) / kProd;   // boxes this warp issues per batch
+    const int x = kProd * lane + warp;          // this lane's box of every batch (none if >= 16)
+    const bool has = x < 2 * kTokB;
+    const int bj = x & 7, bwhich = x >> 3;
+    const int nmine = 2 * kTokB / kProd;   // boxes this warp issues per batch
     auto batch_token = [&](int n) { return n >= nb || !has ? 0 : list_token(n % nb_sub * kTokB + bj); };
     int tk_next = batch_token(0);
     for (int n = 0; n < nb; ++n) {
@@ -155,13 +155,13 @@ __global__ void __launch_bounds__(kThreads, 1)
       int good = 1;
       if (lane == 0) {
         good = mbar_wait(empty0 + 8 * stage, ph ^ 1, DEV_ERR_EMPTY_WAIT) ? 1 : 0;
-        if (good) mbar_expect_tx(fb, nmine * 2048);
+        if (good) mbar_expect_tx(fb, nmine * 4096);
       }
       if (!__shfl_sync(0xffffffffu, good, 0)) break;
       if (has) {
         const uint32_t q_s = ring + stage * STAGE, do_s = q_s + Q_TILE;
         const int qrow = (int)(((long long)b * a.Tq + (tk - a.q0)) * a.Hq + hg * 16);
-        tma_load_2d((bwhich ? do_s : q_s) + bp * Q_PANEL + bj * 2048, bwhich ? &tmDO : &tmQ, fb, bp * 64, qrow);
+        tma_load_4d((bwhich ? do_s : q_s) + bj * 4096, bwhich ? &tmDO : &tmQ, fb, 0, 0, 0, qrow >> 3);
       }
     }
   } else if (warp == kMmaWarp) {
@@ -176,8 +176,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
       for (int i = 0; i < kStages; ++i) {
         const uint32_t q_s = ring + i * STAGE, do_s = q_s + Q_TILE;
-        dQk[i] = umma_smem_desc(q_s, 0, 1024);
-        dDOk[i] = umma_smem_desc(do_s, 0, 1024);
+        dQk[i] = umma_smem_desc(q_s, 0, 2048);
+        dDOk[i] = umma_smem_desc(do_s, 0, 2048);
       }
       for (int n = 0; ok && n < nb; ++n) {
         ok = mbar_wait(full0 + 8 * (n % kStages), (n / kStages) & 1, DEV_ERR_FULL_WAIT);
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const uint32_t col = (n & 1) * 128;
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
-          const uint32_t aoff = (ks >> 2) * Q_PANEL + (ks & 3) * 32, boff = (ks >> 2) * KV_PANEL + (ks & 3) * 32;
+          const uint32_t aoff = (ks >> 2) * 1024 + (ks & 3) * 32, boff = (ks >> 2) * KV_PANEL + (ks & 3) * 32;
           umma_ss(tmem + col, umma_desc_advance(aq, aoff), umma_desc_advance(dK, boff), idesc_kk, ks ? 1u : 0u);
           umma_ss(tmem + col + 64, umma_desc_advance(ado, aoff), umma_desc_advance(dV, boff), idesc_kk, ks ? 1u : 0u);
         }
@@ -205,8 +205,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
       for (int i = 0; i < kStages; ++i) {
         const uint32_t q_s = ring + i * STAGE, do_s = q_s + Q_TILE;
-        dQmn[i] = umma_smem_desc(q_s, Q_PANEL, 1024);
-        dDOmn[i] = umma_smem_desc(do_s, Q_PANEL, 1024);
+        dQmn[i] = umma_smem_desc(q_s, 1024, 2048);
+        dDOmn[i] = umma_smem_desc(do_s, 1024, 2048);
       }
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
@@ -223,8 +223,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         const uint64_t bp = (n & 1) ? dP[1] : dP[0], bds = (n & 1) ? dDS[1] : dDS[0];
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {  // contraction over the 128 rows, 16 per step; dV and dK alternate
-          umma_ss(tmem + kColDV, umma_desc_advance(ado, ks * 2048), umma_desc_advance(bp, ks * 2048), idesc_mn, (n | ks) ? 1u : 0u);
-          umma_ss(tmem + kColDK, umma_desc_advance(aq, ks * 2048), umma_desc_advance(bds, ks * 2048), idesc_mn, (n | ks) ? 1u : 0u);
+          umma_ss(tmem + kColDV, umma_desc_advance(ado, ks * 4096), umma_desc_advance(bp, ks * 2048), idesc_mn, (n | ks) ? 1u : 0u);
+          umma_ss(tmem + kColDK, umma_desc_advance(aq, ks * 4096), umma_desc_advance(bds, ks * 2048), idesc_mn, (n | ks) ? 1u : 0u);
         }
         umma_commit(empty0 + 8 * (n % kStages));
         if (emit_dq) {
@@ -479,8 +479,12 @@ int launch(const KvArgs& a, cudaStream_t s) {
     set_error("B*T*Hq exceeds the 2^31 rows a TMA coordinate can address");
     return -32;
   }
-  int rc = make_tmap_rows2d(&tmQ, a.q, D, qrows, 16);
-  if (!rc) rc = make_tmap_rows2d(&tmDO, a.dout, D, qrows, 16);
+  // rows as (64 columns, 8 rows, 2 column panels, groups of 8 rows): one box = 16 rows x 128 columns of one token
+  const unsigned long long qd[4] = {64, 8, 2, (unsigned long long)(qrows / 8)};
+  const unsigned long long qs[3] = {(unsigned long long)D * 2, 128, (unsigned long long)D * 2 * 8};
+  const unsigned qb[4] = {64, 8, 2, 2};
+  int rc = make_tmap_generic(&tmQ, a.q, 4, qd, qs, qb);
+  if (!rc) rc = make_tmap_generic(&tmDO, a.dout, 4, qd, qs, qb);
   if (!rc) rc = make_tmap_rows4d(&tmK, a.k, D, a.Hk, a.T, a.B, 64);
   if (!rc) rc = make_tmap_rows4d(&tmV, a.v, D, a.Hk, a.T, a.B, 64);
   if (rc) return rc;
