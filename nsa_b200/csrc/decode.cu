@@ -144,47 +144,73 @@ __device__ __forceinline__ void pv_tile(float (&acc)[D / 8][4], const float (&sc
 }
 
 // The n blocks with the highest pooled score (ties to the lower index), in order, by one warp: lane l holds the blocks l + 32 e as
-// integers that order like the scores.  The n-th highest is found bit by bit with ballots, the n survivors are ranked among
-// themselves.  (n rounds of a shared-memory scan and a butterfly took 6400 cycles for 16 of 512 blocks, n rounds of two integer
-// warp reductions 18000, counting every block's rank with all warps 38000.)
+// integers that order like the scores.  The n-th highest is found bit by bit, from the first bit in which the scores differ: a
+// lane counts its own and one warp reduction adds.  The n survivors are ranked among themselves.  (A chain, on which the loads of
+// the selected blocks wait; 16 of 512 blocks.  Counting by ballots from the highest bit 8800 cycles, n rounds of a shared-memory
+// scan and a butterfly 6400 with the other warps' help, n rounds of two integer warp reductions 18000, every block's rank by all
+// warps 38000.)
 template <int E>
 __device__ __forceinline__ int top_blocks(const float* pooled, int2* tmp, int n_pool, int n_sel, int lane) {   // lane r: the r-th, or -1
-  unsigned v[E];
+  unsigned v[E], hi = 0u, lo = 0xffffffffu;
   int valid = 0;
 #pragma unroll
   for (int e = 0; e < E; ++e) {
     const int blk = lane + 32 * e;
     const float x = blk < n_pool ? pooled[blk] : -1.f;
     v[e] = x >= 0.f ? __float_as_uint(x) + 1u : 0u;   // 0: none
-    valid += __popc(__ballot_sync(0xffffffffu, v[e] != 0u));
+    valid += v[e] != 0u ? 1 : 0;
+    hi = max(hi, v[e]);
+    lo = min(lo, v[e] - 1u);   // (none: the highest)
   }
+  valid = __reduce_add_sync(0xffffffffu, valid);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  lo = __reduce_min_sync(0xffffffffu, lo) + 1u;
   const int n = min(n_sel, valid);
   if (n == 0) return -1;
-  unsigned thr = 0u;   // the highest value that at least n blocks reach
-  int cnt = 0;         // ... and how many do
-  for (unsigned bit = 1u << 30; bit; bit >>= 1) {
+  // the highest value that at least n blocks reach, and how many do: all of them reach the bits that all have in common
+  const unsigned differ = hi ^ lo;
+  unsigned bit = differ ? 0x80000000u >> __clz(differ) : 0u;
+  unsigned thr = bit ? hi & ~(2u * bit - 1u) : hi;
+  int cnt = valid;
+  for (; bit && cnt != n; bit >>= 1) {
     int c = 0;
 #pragma unroll
-    for (int e = 0; e < E; ++e) c += __popc(__ballot_sync(0xffffffffu, v[e] >= (thr | bit)));
+    for (int e = 0; e < E; ++e) c += v[e] >= (thr | bit) ? 1 : 0;
+    c = __reduce_add_sync(0xffffffffu, c);
     if (c >= n) {
       thr |= bit;
       cnt = c;
-      if (c == n) break;
     }
   }
-  int above = 0;       // all of these, and the first n - above of those at the threshold
-#pragma unroll
-  for (int e = 0; e < E; ++e) above += __popc(__ballot_sync(0xffffffffu, v[e] > thr));
   const unsigned below = (1u << lane) - 1u;
-  int k = 0, ties = cnt == n ? n : n - above;
+  if (cnt == n) {   // exactly these
+    int own = 0;
 #pragma unroll
-  for (int e = 0; e < E; ++e) {
-    const unsigned eq = __ballot_sync(0xffffffffu, v[e] == thr);
-    const bool take = v[e] > thr || (v[e] == thr && __popc(eq & below) < ties);
-    const unsigned m = __ballot_sync(0xffffffffu, take);
-    if (take) tmp[k + __popc(m & below)] = make_int2((int)v[e], lane + 32 * e);
-    k += __popc(m);
-    ties -= min(ties, __popc(eq));
+    for (int e = 0; e < E; ++e) own += v[e] >= thr && v[e] != 0u ? 1 : 0;
+    int k = own;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, k, off);
+      if (lane >= off) k += y;
+    }
+    k -= own;
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+      if (v[e] >= thr && v[e] != 0u) tmp[k++] = make_int2((int)v[e], lane + 32 * e);
+  } else {          // those above the threshold, and the first of those at it
+    int above = 0, k = 0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) above += v[e] > thr ? 1 : 0;
+    int ties = n - __reduce_add_sync(0xffffffffu, above);
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const unsigned eq = __ballot_sync(0xffffffffu, v[e] == thr);
+      const bool take = v[e] > thr || (v[e] == thr && __popc(eq & below) < ties);
+      const unsigned m = __ballot_sync(0xffffffffu, take);
+      if (take) tmp[k + __popc(m & below)] = make_int2((int)v[e], lane + 32 * e);
+      k += __popc(m);
+      ties -= min(ties, __popc(eq));
+    }
   }
   __syncwarp();
   const int2 own = lane < n ? tmp[lane] : make_int2(0, 0);
