@@ -20,12 +20,12 @@
 //                          p_sel summed over the heads into a per-position vector in shared memory;
 //                          then pooling and a warp top-n while the other warps go on;
 //   3. window (k, v) pairs and 4. selected (k, v) pairs: online soft-max per warp.
-// Every warp leaves its partial (maximum, sum, unnormalised output) of each branch in a caller-provided workspace; a
-// second, small kernel merges the six partials of a branch in a fixed order, computes the gates from q and writes the
-// outputs (the split-KV scheme of decode attention).  Measured alternatives: merging through shared memory, warp after
-// warp, cost seven named barriers and six serialised rounds per branch (0.29 ms per step of the 128-sequence workload
-// against 0.21 ms); merging in the same kernel through an L2-resident scratch idled five of six warps and the TMA ring
-// during the merge (0.30 ms).  No atomics; every wait is bounded.
+// Every warp leaves its partial (maximum, sum, unnormalised output) of each branch in a caller-provided workspace (the split-KV
+// scheme of decode attention).  Where one CTA does a whole item, its six warps then merge the item's partials, a row at a
+// time each and in a fixed order, from a scratch that the CTA's next item uses again (22 MB for the grid, it stays in L2), while the
+// ring fills with the next item's tiles.  With clusters a second, small kernel does that.  Measured: the second kernel for
+// all (scratch for every item, 77 MB written and read for 512 of them) @MEAS@; merging through shared memory, warp after warp, cost
+// seven named barriers and six serialised rounds per branch.  No atomics; every wait is bounded.
 #include <algorithm>
 #include <array>
 
@@ -37,10 +37,8 @@ namespace nsa {
 namespace {
 
 constexpr int D = 128;
-constexpr int kCons = 6;                       // consumer warps
-constexpr int kProdW = 2;                      // producer warps
-constexpr int kThreads = (kCons + kProdW) * 32;
-constexpr int kSlots = 2 * kCons;
+constexpr int kCons = 6;                       // consumer warps of a CTA that has an SM to itself
+constexpr int kHalfCons = 3;                   // ... of one that shares it with another
 constexpr uint32_t PANEL = 64 * 128;           // [64 rows][64 columns] bf16
 constexpr uint32_t TILE = 2 * PANEL;           // 16 KB
 constexpr int kMaxTc = 2048;                   // compressed positions of one sequence held in shared memory
@@ -58,6 +56,7 @@ struct Plan {   // tile pairs of one item's phases; CTA `rank` of a cluster take
   int w0;      // first window key
 };
 
+template <int CONS>
 __device__ __forceinline__ Plan make_plan(const DecodeArgs& a, int seq, int cl) {
   Plan p;
   p.row_k = a.cu_k[seq];
@@ -73,7 +72,7 @@ __device__ __forceinline__ Plan make_plan(const DecodeArgs& a, int seq, int cl) 
   // An exchange costs about as much as one pair (3500 cycles): with no more than a pair for each warp nothing is shared in the
   // two passes, every CTA makes its own statistics and scores.  (Both passes or neither: that every CTA has sent its statistics
   // also says that none still reads the scores of the item before.)
-  p.cs = p.n2p > kCons ? cl : 1;
+  p.cs = p.n2p > CONS ? cl : 1;
   p.w0 = max(0, p.L - a.window);
   p.nw = a.window > 0 ? (p.L - p.w0 + 63) / 64 : 0;
   return p;
@@ -225,6 +224,10 @@ __device__ __forceinline__ int top_blocks(const float* pooled, int2* tmp, int n_
   return lane < n ? tmp[lane].x : -1;
 }
 
+// Producer warps: one issues 30 bytes per cycle (see below), what one of two CTAs of an SM can draw at most.
+__host__ __device__ constexpr int decode_producers(int cons) { return cons == kCons ? 2 : 1; }
+__host__ __device__ constexpr int decode_threads(int cons) { return (cons + decode_producers(cons)) * 32; }
+
 // One (K, V) pair of an online soft-max: keys key0 .. key0+63 of the tile are valid iff kmin <= key < kmax.
 __device__ __forceinline__ void online_pair(float (&acc)[D / 8][4], float (&m_run)[2], float (&l_run)[2],
                                             const uint32_t (&qf)[D / 16][4], uint32_t kbase, uint32_t vbase, uint32_t k_empty,
@@ -276,9 +279,13 @@ __device__ __forceinline__ void online_pair(float (&acc)[D / 8][4], float (&m_ru
   if (lane == 0) mbar_arrive(v_empty);
 }
 
-__global__ void __launch_bounds__(kThreads, 1)
+// CONS consumer warps with a pair of slots each; CL: the CTAs of a cluster share an item.
+template <int CONS, bool CL>
+__global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
     decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
-                  const __grid_constant__ CUtensorMap tmCK, const __grid_constant__ CUtensorMap tmCV, const DecodeArgs a, const int cl) {
+                  const __grid_constant__ CUtensorMap tmCK, const __grid_constant__ CUtensorMap tmCV, const DecodeArgs a, const int ncl) {
+  constexpr int kSlots = 2 * CONS, kProdW = decode_producers(CONS);
+  const int cl = CL ? ncl : 1;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t sbase = (raw + 1023u) & ~1023u;
@@ -288,10 +295,12 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint8_t* after = sgen + kSlots * TILE;
   float* ps = reinterpret_cast<float*>(after);                    // [kMaxTc + 64] head-summed p_sel per compressed position
   float* pooled = ps + kMaxTc + 64;                               // [kMaxPoolD]
-  float* stat = pooled + kMaxPoolD;                               // [kCons][4][16] per-warp statistics
-  float* fin = stat + kCons * 64;                                 // [4][16] merged: M_raw, 1/L_raw, M_att (log2), L_att
+  float* stat = pooled + kMaxPoolD;                               // [CONS][4][16] per-warp statistics
+  float* fin = stat + CONS * 64;                                 // [4][16] merged: M_raw, 1/L_raw, M_att (log2), L_att
   float* xstat = fin + 64;                                        // [cluster][4][16] the CTAs' statistics
-  int* sel = reinterpret_cast<int*>(xstat + kMaxCluster * 64);    // [kMaxSel] selected blocks of the item, [kMaxSel] = count
+  float2* ml = reinterpret_cast<float2*>(xstat + kMaxCluster * 64);   // [3][CONS][16] (m, l) of the warps' partials, without clusters
+  float* gates = reinterpret_cast<float*>(ml + 3 * CONS * 16);       // [3][16], branch order as ml's
+  int* sel = reinterpret_cast<int*>(gates + 48);                  // [kMaxSel] selected blocks of the item, [kMaxSel] = count
   volatile int* abort_flag = sel + kMaxSel + 2;
   const uint32_t bar_base = sbase + kSlots * TILE + (uint32_t)((uint8_t*)(sel + kMaxSel + 4) - after);
   const uint32_t bar0 = (bar_base + 7u) & ~7u;
@@ -313,22 +322,25 @@ __global__ void __launch_bounds__(kThreads, 1)
     fence_mbar_init();
   }
   __syncthreads();
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the merge may take its places now: it waits for this grid's end
+  if (cl > 1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the merge may take its places now: it waits for this grid's end
   if (cl > 1) cluster_sync_all();   // no CTA writes into another's shared memory before it runs, or after it ended (below)
 
   const int nitem = a.nseq * a.Hkv;
+  // of the pairs of a phase that cs CTAs share: how many are this CTA's, and which is its i-th
+  auto share = [&](int n, int cs) { return !CL || cs == 1 ? n : (n - rank + cs - 1) / cs; };
+  auto deal = [&](int i, int cs) { return !CL || cs == 1 ? i : rank + i * cs; };
   const int pool_k = a.sel_block / a.cstride + 1, pool_s = a.sel_block / a.cstride;
 
-  if (warp >= kCons) {
+  if (warp >= CONS) {
     // ------------------------------- producers --------------------------------------------------------
     // A warp's TMA instructions run one after another (about 850 + 52 x boxes cycles each, whatever the box size), so
     // a single warp issuing one 16 KB tile per instruction caps the SM at ~16 bytes per clock.  Tiles therefore go out
     // in PAIRS (four boxes per instruction: both tiles of a (K, V) pair, or two consecutive ck tiles of pass 1), and
     // the two producer warps take alternate pairs.
-    const int pw = warp - kCons;
+    const int pw = warp - CONS;
     uint32_t np = 0, it = 0;     // tile pairs issued so far by both producers together; items so far
     auto issue2 = [&](const CUtensorMap* tmA, int rowA, const CUtensorMap* tmB, int rowB, int h) -> bool {
-      const uint32_t mine = (np & 1) == (uint32_t)pw;
+      const uint32_t mine = np % kProdW == (uint32_t)pw;
       const uint32_t n = 2 * np;
       ++np;
       if (!mine) return true;
@@ -355,7 +367,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (item >= nitem) continue;
       const int sq = item / a.Hkv, h = item % a.Hkv;
       const int seq = a.order ? a.order[sq] : sq;
-      const Plan p = make_plan(a, seq, cl);
+      const Plan p = make_plan<CONS>(a, seq, cl);
       bool ok = true;
       for (int j = p.cs > 1 ? rank : 0; ok && j < p.n1p; j += p.cs) ok = issue2(&tmCK, p.row_c + j * 128, &tmCK, p.row_c + j * 128 + 64, h);
       for (int j = p.cs > 1 ? rank : 0; ok && j < p.n2p; j += p.cs) ok = issue2(&tmCK, p.row_c + j * 64, &tmCV, p.row_c + j * 64, h);
@@ -376,18 +388,21 @@ __global__ void __launch_bounds__(kThreads, 1)
   // --------------------------------- consumers ----------------------------------------------------------
   const int g = lane >> 2, tq = lane & 3;
   const float sl2 = a.scale * kLog2e;
-  const int cthreads = kCons * 32;
+  const int cthreads = CONS * 32;
   const int ct = threadIdx.x;               // 0 .. cthreads-1
-  uint32_t n0 = 0, it = 0;                  // tiles consumed by the CTA before the current phase; items so far
+  // tile pair i of the CTA, over all phases and items, is warp i % CONS's, in that warp's own two slots
+  uint32_t np0 = 0, it = 0;                 // pairs of the CTA before the current phase; items so far
+  uint32_t use = 0;                         // pairs of this warp so far
+  const uint32_t sk = 2 * warp, sv = sk + 1;
+  auto first_pair = [&]() { return (int)((warp + CONS - np0 % CONS) % CONS); };
   uint32_t nx = 0;                          // items with an exchange so far
   bool ok = true;
-  // tile pair u (two consecutive tiles) of a phase that starts at tile counter base belongs to warp ((base/2 + u) % kCons)
   for (int r = 0; r * ngroup < nitem; ++r) {
     const int item = snake_item(r, group, ngroup);
     if (item >= nitem) continue;
     const int sq = item / a.Hkv, h = item % a.Hkv;
     const int seq = a.order ? a.order[sq] : sq;
-    const Plan p = make_plan(a, seq, cl);
+    const Plan p = make_plan<CONS>(a, seq, cl);
     const int t = p.L - 1;
     const long long qrow = (long long)seq * a.Hq + h * 16;     // first of the 16 (head) rows of this item
     uint32_t qf[D / 16][4];
@@ -397,15 +412,14 @@ __global__ void __launch_bounds__(kThreads, 1)
     float mr[2] = {-INFINITY, -INFINITY}, lr[2] = {0.f, 0.f};   // raw scores, all keys (natural-log domain kept in log2)
     float ma[2] = {-INFINITY, -INFINITY}, la[2] = {0.f, 0.f};   // scaled scores, visible keys
     {
-      const uint32_t pair0 = n0 / 2;
-      int i = 0;   // this CTA's pairs
-      for (int u = p.cs > 1 ? rank : 0; u < p.n1p; u += p.cs, ++i) {
-        if ((int)((pair0 + i) % kCons) != warp) continue;
+      const int n = share(p.n1p, p.cs);
+      for (int i = first_pair(); i < n; i += CONS, ++use) {
+        const int u = deal(i, p.cs);
 #pragma unroll 1
         for (int e = 0; e < 2; ++e) {
-          const uint32_t n = n0 + 2 * i + e, s = n % kSlots;
+          const uint32_t s = sk + e;
           const int j0 = (2 * u + e) * 64;
-          ok = ok && mbar_wait_abortable(full_bar(s), (n / kSlots) & 1, DEV_ERR_FULL_WAIT, abort_flag);
+          ok = ok && mbar_wait_abortable(full_bar(s), use & 1, DEV_ERR_FULL_WAIT, abort_flag);
           float sc[8][4];
 #pragma unroll
           for (int i = 0; i < 8; ++i) sc[i][0] = sc[i][1] = sc[i][2] = sc[i][3] = 0.f;
@@ -442,7 +456,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
         }
       }
-      n0 += 2 * i;
+      np0 += n;
     }
     // merge the per-warp statistics (each value lives in the four lanes of a quad: sum the partial sums)
 #pragma unroll
@@ -459,12 +473,12 @@ __global__ void __launch_bounds__(kThreads, 1)
     named_bar_sync(1, cthreads);
     if (ct < 16) {
       float Mr = -INFINITY, Ma = -INFINITY;
-      for (int w = 0; w < kCons; ++w) {
+      for (int w = 0; w < CONS; ++w) {
         Mr = fmaxf(Mr, stat[w * 64 + ct]);
         Ma = fmaxf(Ma, stat[w * 64 + 32 + ct]);
       }
       float Lr = 0.f, La = 0.f;
-      for (int w = 0; w < kCons; ++w) {
+      for (int w = 0; w < CONS; ++w) {
         const float m1 = stat[w * 64 + ct], m2 = stat[w * 64 + 32 + ct];
         if (m1 > -INFINITY) Lr += stat[w * 64 + 16 + ct] * ex2(m1 - Mr);
         if (m2 > -INFINITY) La += stat[w * 64 + 48 + ct] * ex2(m2 - Ma);
@@ -520,14 +534,12 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (int i = 0; i < D / 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
     bool full = rank == 0 && warp == 0;   // this warp's partial has an output (the first always: the row sums ride with it)
     {
-      const uint32_t pair0 = n0 / 2;
-      int i = 0;
-      for (int u = p.cs > 1 ? rank : 0; u < p.n2p; u += p.cs, ++i) {
-        if ((int)((pair0 + i) % kCons) != warp) continue;
+      const int n = share(p.n2p, p.cs);
+      for (int i = first_pair(); i < n; i += CONS, ++use) {
+        const int u = deal(i, p.cs);
         full = p.cs > 1 || rank == 0;
-        const uint32_t nk = n0 + 2 * i, nv = nk + 1, sk = nk % kSlots, sv = nv % kSlots;
         const int j0 = u * 64;
-        ok = ok && mbar_wait_abortable(full_bar(sk), (nk / kSlots) & 1, DEV_ERR_FULL_WAIT, abort_flag);
+        ok = ok && mbar_wait_abortable(full_bar(sk), use & 1, DEV_ERR_FULL_WAIT, abort_flag);
         float sc[8][4];
 #pragma unroll
         for (int i = 0; i < 8; ++i) sc[i][0] = sc[i][1] = sc[i][2] = sc[i][3] = 0.f;
@@ -569,12 +581,12 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int j = j0 + nt * 8 + 2 * tq + (c & 1);
             sc[nt][c] = (j < p.nvis) ? ex2(fmaf(sc[nt][c], sl2, -Ma[c >> 1])) : 0.f;
           }
-        ok = ok && mbar_wait_abortable(full_bar(sv), (nv / kSlots) & 1, DEV_ERR_FULL_WAIT, abort_flag);
+        ok = ok && mbar_wait_abortable(full_bar(sv), use & 1, DEV_ERR_FULL_WAIT, abort_flag);
         if (ok && j0 < p.nvis && (p.cs > 1 || rank == 0)) pv_tile(acc, sc, ring + sv * TILE, lane);
         __syncwarp();
         if (lane == 0) mbar_arrive(empty_bar(sv));
       }
-      n0 += 2 * i;
+      np0 += n;
     }
     // ---- pooled scores and the top-n (warp 0), the compressed-branch output (all warps, fixed order) ------------
     named_bar_sync(1, cthreads);            // ps complete
@@ -608,7 +620,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     // this warp's partial of a branch -> workspace: [item][branch][warp of the cluster]{ O[16][D], m[16], l[16] } fp32; a warp
     // that had no tile leaves m = -inf and no O
     auto put_partial = [&](int branch, const float (&x)[D / 8][4], const float (&mm)[2], const float (&ll)[2], bool has) {
-      float* dst = a.part + (((long long)item * 3 + branch) * (cl * kCons) + rank * kCons + warp) * kPartFloats;
+      float* dst = a.part + (((long long)(cl > 1 ? item : (int)blockIdx.x) * 3 + branch) * (cl * CONS) + rank * CONS + warp) * kPartFloats;
 #pragma unroll
       for (int i = 0; i < D / 8; ++i) {
         if (!has) break;
@@ -619,8 +631,13 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int rr = 0; rr < 2; ++rr) {
         const float l = quad_sum(ll[rr]);
         if (tq == 0) {
-          dst[16 * D + g + 8 * rr] = has ? mm[rr] : -INFINITY;
-          dst[16 * D + 16 + g + 8 * rr] = l;
+          const float m = has ? mm[rr] : -INFINITY;
+          if (cl > 1) {
+            dst[16 * D + g + 8 * rr] = m;
+            dst[16 * D + 16 + g + 8 * rr] = l;
+          } else {
+            ml[(branch * CONS + warp) * 16 + g + 8 * rr] = make_float2(m, l);
+          }
         }
       }
     };
@@ -635,23 +652,51 @@ __global__ void __launch_bounds__(kThreads, 1)
       put_partial(0, acc, mm, ll, full);
     }
 
+    // ---- gates, by the last warp (the first one is still choosing blocks) --------------------------------
+    // (what the item before left in gates, ml and the scratch has been read: its rows are merged before anything of this one)
+    if (cl == 1 && warp == CONS - 1) {
+      if (a.gate_w) {
+        // g_x[row] = q[row,:] . W[x,:] + b[x] (nn.Linear(head_dim, 3), rows of W: selected, window, compressed) as one 16 x 8
+        // tile of mma.sync, rounded to bf16 as the module's gate tensors are
+        float c[4] = {0.f, 0.f, 0.f, 0.f};
+        uint32_t wf[D / 16][2];
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks) {
+          const bf16* w = a.gate_w + g * D + ks * 16 + 2 * tq;
+          wf[ks][0] = g < 3 ? *reinterpret_cast<const uint32_t*>(w) : 0u;
+          wf[ks][1] = g < 3 ? *reinterpret_cast<const uint32_t*>(w + 8) : 0u;
+        }
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks) mma_bf16(c, qf[ks], wf[ks][0], wf[ks][1]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int x = 2 * tq + (i & 1);
+          if (x < 3) gates[(x == 2 ? 0 : x + 1) * 16 + g + 8 * (i >> 1)] = __bfloat162float(__float2bfloat16(c[i] + (a.gate_b ? __bfloat162float(a.gate_b[x]) : 0.f)));
+        }
+      } else if (lane < 16) {
+#pragma unroll
+        for (int br = 0; br < 3; ++br) {
+          const bf16* gin = br == 0 ? a.g_cmp : br == 1 ? a.g_slc : a.g_swa;
+          gates[br * 16 + lane] = gin ? __bfloat162float(gin[qrow + lane]) : 1.f;
+        }
+      }
+    }
+
     // ---- window ---------------------------------------------------------------------------------------
     float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
 #pragma unroll
     for (int i = 0; i < D / 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
     full = false;
     {
-      const uint32_t pair0 = n0 / 2;
-      int i = 0;
-      for (int u = rank; u < p.nw; u += cl, ++i) {
-        if ((int)((pair0 + i) % kCons) != warp) continue;
+      const int n = share(p.nw, cl);
+      for (int i = first_pair(); i < n; i += CONS, ++use) {
+        const int u = deal(i, cl);
         full = true;
-        const uint32_t nk = n0 + 2 * i, nv = nk + 1, sk = nk % kSlots, sv = nv % kSlots;
-        ok = ok && mbar_wait_abortable(full_bar(sk), (nk / kSlots) & 1, DEV_ERR_FULL_WAIT, abort_flag);
-        online_pair(acc, m_run, l_run, qf, ring + sk * TILE, ring + sv * TILE, empty_bar(sk), full_bar(sv), (nv / kSlots) & 1,
+        ok = ok && mbar_wait_abortable(full_bar(sk), use & 1, DEV_ERR_FULL_WAIT, abort_flag);
+        online_pair(acc, m_run, l_run, qf, ring + sk * TILE, ring + sv * TILE, empty_bar(sk), full_bar(sv), use & 1,
                     empty_bar(sv), p.w0 + u * 64, p.w0, p.L, sl2, lane, ok, abort_flag);
       }
-      n0 += 2 * i;
+      np0 += n;
     }
     {
       // l_run holds this lane's share of the row sums (four lanes per row): put_partial adds the quad
@@ -667,22 +712,69 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (int i = 0; i < D / 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
     full = false;
     {
-      const uint32_t pair0 = n0 / 2;
-      int i = 0;
-      for (int u = rank; u < nsel; u += cl, ++i) {
-        if ((int)((pair0 + i) % kCons) != warp) continue;
+      const int n = share(nsel, cl);
+      for (int i = first_pair(); i < n; i += CONS, ++use) {
+        const int u = deal(i, cl);
         full = true;
         const int blk = *reinterpret_cast<volatile int*>(sel + u);
-        const uint32_t nk = n0 + 2 * i, nv = nk + 1, sk = nk % kSlots, sv = nv % kSlots;
-        ok = ok && mbar_wait_abortable(full_bar(sk), (nk / kSlots) & 1, DEV_ERR_FULL_WAIT, abort_flag);
-        online_pair(acc, m_run, l_run, qf, ring + sk * TILE, ring + sv * TILE, empty_bar(sk), full_bar(sv), (nv / kSlots) & 1,
+        ok = ok && mbar_wait_abortable(full_bar(sk), use & 1, DEV_ERR_FULL_WAIT, abort_flag);
+        online_pair(acc, m_run, l_run, qf, ring + sk * TILE, ring + sv * TILE, empty_bar(sk), full_bar(sv), use & 1,
                     empty_bar(sv), blk * 64, 0, p.L, sl2, lane, ok, abort_flag);
       }
-      n0 += 2 * i;
+      np0 += n;
     }
     put_partial(1, acc, m_run, l_run, full);
     named_bar_sync(1, cthreads);   // ps, pooled, fin and sel are reused by the next item
     ++it;
+    // ---- this item's rows: partials merged warp by warp, gated sum of the branches (a lane holds four channels) --------
+    for (int row = warp; cl == 1 && row < 16; row += CONS) {
+      const float4* base = reinterpret_cast<const float4*>(a.part + (long long)blockIdx.x * 3 * CONS * kPartFloats + row * D) + lane;
+      float4 x[3][CONS];
+      float e[3][CONS], inv[3], lse[3];
+#pragma unroll
+      for (int br = 0; br < 3; ++br)
+#pragma unroll
+        for (int w = 0; w < CONS; ++w) {
+          e[br][w] = ml[(br * CONS + w) * 16 + row].x;
+          x[br][w] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (e[br][w] > -INFINITY) x[br][w] = __ldcg(base + (br * CONS + w) * (kPartFloats / 4));
+        }
+#pragma unroll
+      for (int br = 0; br < 3; ++br) {
+        float M = e[br][0], L = 0.f;
+#pragma unroll
+        for (int w = 1; w < CONS; ++w) M = fmaxf(M, e[br][w]);
+#pragma unroll
+        for (int w = 0; w < CONS; ++w) {
+          e[br][w] = e[br][w] > -INFINITY ? ex2(e[br][w] - M) : 0.f;
+          L += ml[(br * CONS + w) * 16 + row].y * e[br][w];
+        }
+        inv[br] = L > 0.f ? 1.f / L : 0.f;
+        lse[br] = L > 0.f ? (M + log2f(L)) * kLn2 : -INFINITY;
+      }
+      float4 tot = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int br = 0; br < 3; ++br) {
+        if (br == 2 && a.window <= 0) continue;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int w = 0; w < CONS; ++w) {
+          const float wt = e[br][w] * inv[br];
+          v.x = fmaf(x[br][w].x, wt, v.x);
+          v.y = fmaf(x[br][w].y, wt, v.y);
+          v.z = fmaf(x[br][w].z, wt, v.z);
+          v.w = fmaf(x[br][w].w, wt, v.w);
+        }
+        const __nv_bfloat162 b0 = __floats2bfloat162_rn(v.x, v.y), b1 = __floats2bfloat162_rn(v.z, v.w);
+        bf16* out = br == 0 ? a.o_cmp : br == 1 ? a.o_slc : a.o_swa;
+        if (out) *reinterpret_cast<uint2*>(out + (qrow + row) * D + lane * 4) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+        if (a.lse && lane == 0) a.lse[(long long)br * a.nseq * a.Hq + qrow + row] = lse[br];
+        const float gt = gates[br * 16 + row];
+        const float2 f0 = __bfloat1622float2(b0), f1 = __bfloat1622float2(b1);
+        tot.x += gt * f0.x; tot.y += gt * f0.y; tot.z += gt * f1.x; tot.w += gt * f1.y;
+      }
+      *reinterpret_cast<uint2*>(a.o + (qrow + row) * D + lane * 4) = make_uint2(pack_bf16(tot.x, tot.y), pack_bf16(tot.z, tot.w));
+    }
   }
   }
   if (cl > 1) {
@@ -691,7 +783,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
-// Merge of the per-warp partials, in a fixed order (CTA by CTA, warp by warp): one warp per (item, query row, branch), a lane holds
+// Clusters: merge of the per-warp partials, in a fixed order (CTA by CTA, warp by warp): one warp per (item, query row, branch), a lane holds
 // four channels.  Branch order in the workspace: 0 compressed, 1 selected, 2 window.  Warps that had no tile are left out.  The
 // loads of the first CTA's partials (all of them without clusters) are under way while their weights are formed in the warp;
 // the gates (computed from q when the gate projection is given) do not wait for the main kernel.  Few registers and blocks of
@@ -813,16 +905,18 @@ __global__ void __launch_bounds__(96 * kMergeRows) decode_merge_kernel(const Dec
   }
 }
 
-constexpr int decode_smem() {
-  return kSlots * (int)TILE + (kMaxTc + 64 + kMaxPoolD + kCons * 64 + 64 + kMaxCluster * 64) * 4 + (kMaxSel + 4) * 4 +
-         (2 * kSlots + 3) * 8 + 16 + 1024;
+constexpr int decode_smem(int cons) {
+  return 2 * cons * (int)TILE + (kMaxTc + 64 + kMaxPoolD + cons * 64 + 64 + kMaxCluster * 64 + 3 * cons * 32 + 48) * 4 + (kMaxSel + 4) * 4 +
+         (4 * cons + 3) * 8 + 16 + 1024;
 }
-// The launch of `nitem` items with `cl` CTAs each, all resident at once as far as they fit.
-cudaLaunchConfig_t decode_config(int ncta, int cl, cudaLaunchAttribute* at, cudaStream_t s) {
+static_assert(2 * (decode_smem(kHalfCons) + 1024) <= 228 * 1024, "two CTAs per SM");
+
+// A launch of `ncta` CTAs in clusters of `cl`.
+cudaLaunchConfig_t decode_config(int ncta, int cons, int cl, cudaLaunchAttribute* at, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)ncta);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = decode_smem();
+  cfg.blockDim = dim3(decode_threads(cons));
+  cfg.dynamicSmemBytes = decode_smem(cons);
   cfg.stream = s;
   at->id = cudaLaunchAttributeClusterDimension;
   at->val.clusterDim.x = cl;
@@ -840,9 +934,9 @@ int resident_clusters(int cl) {
       n[i] = num_sms() >> i;
       int c = 0;
       cudaLaunchAttribute at;
-      const cudaLaunchConfig_t cfg = decode_config(num_sms() >> i << i, 1 << i, &at, nullptr);
-      if (i > 0 && cudaFuncSetAttribute(decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, decode_smem()) == cudaSuccess &&
-          cudaOccupancyMaxActiveClusters(&c, decode_kernel, &cfg) == cudaSuccess)
+      const cudaLaunchConfig_t cfg = decode_config(num_sms() >> i << i, kCons, 1 << i, &at, nullptr);
+      if (i > 0 && cudaFuncSetAttribute(decode_kernel<kCons, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, decode_smem(kCons)) == cudaSuccess &&
+          cudaOccupancyMaxActiveClusters(&c, decode_kernel<kCons, true>, &cfg) == cudaSuccess)
         n[i] = c;
       cudaGetLastError();   // (no device: workspace sizes can be asked for all the same)
     }
@@ -850,17 +944,23 @@ int resident_clusters(int cl) {
   }();
   return held[cl == 8 ? 3 : cl == 4 ? 2 : cl == 2 ? 1 : 0];
 }
-// CTAs per item: as many as keep every item in the first wave.
-int decode_cluster(int nitem) {
+// How `nitem` items are spread: CTAs per item, as many as keep every item in the first wave; with more items than SMs two CTAs
+// of half the warps and slots share an SM, so that one streams tiles while the other chooses its blocks or merges its rows.
+struct Spread {
+  int cons, cl, ncta;
+};
+Spread decode_spread(int nitem) {
+  if (nitem > num_sms()) return {kHalfCons, 1, std::min(nitem, 2 * num_sms())};
   int cl = kMaxCluster;
   while (cl > 1 && nitem > resident_clusters(cl)) cl >>= 1;
-  return cl;
+  return {kCons, cl, nitem * cl};
 }
 
 }  // namespace
 
 size_t decode_workspace_bytes(int nseq, int Hkv) {
-  return (size_t)nseq * Hkv * 3 * decode_cluster(nseq * Hkv) * kCons * kPartFloats * sizeof(float);
+  const Spread p = decode_spread(nseq * Hkv);   // a set of partials for every CTA (of a cluster: one item each)
+  return (size_t)p.ncta * 3 * p.cons * kPartFloats * sizeof(float);
 }
 
 int launch_decode(const DecodeArgs& a, cudaStream_t s) {
@@ -891,18 +991,21 @@ int launch_decode(const DecodeArgs& a, cudaStream_t s) {
     set_error("decode: workspace too small (%lld bytes needed)", (long long)decode_workspace_bytes(a.nseq, a.Hkv));
     return -6;
   }
-  cudaError_t e = cudaFuncSetAttribute(decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, decode_smem());
-  if (e != cudaSuccess) return (int)e;
   const int nitem = a.nseq * a.Hkv;
   if (nitem <= 0) return 0;
-  const int cl = decode_cluster(nitem);
+  const Spread p = decode_spread(nitem);
+  const int cl = p.cl;
+  const auto kernel = p.cons == kHalfCons ? decode_kernel<kHalfCons, false> : cl > 1 ? decode_kernel<kCons, true> : decode_kernel<kCons, false>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, decode_smem(p.cons));
+  if (e != cudaSuccess) return (int)e;
   {
     cudaLaunchAttribute at;
-    const cudaLaunchConfig_t cfg = decode_config(std::min(nitem, resident_clusters(cl)) * cl, cl, &at, s);
-    e = cudaLaunchKernelEx(&cfg, decode_kernel, tmK, tmV, tmCK, tmCV, a, cl);
+    const cudaLaunchConfig_t cfg = decode_config(p.ncta, p.cons, cl, &at, s);
+    e = cudaLaunchKernelEx(&cfg, kernel, tmK, tmV, tmCK, tmCV, a, cl);
     if (e != cudaSuccess) return (int)e;
   }
-  {
+  note_launches(1);
+  if (cl > 1) {
     // the merge kernel may be scheduled before the main kernel has drained (it waits with griddepcontrol.wait)
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)nitem * (16 / kMergeRows));
@@ -916,8 +1019,8 @@ int launch_decode(const DecodeArgs& a, cudaStream_t s) {
     cfg.numAttrs = 1;
     e = cudaLaunchKernelEx(&cfg, decode_merge_kernel, a, cl);
     if (e != cudaSuccess) return (int)e;
+    note_launches(1);
   }
-  note_launches(2);
   return (int)cudaGetLastError();
 }
 int decode_status(int* out) {
