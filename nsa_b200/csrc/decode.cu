@@ -11,9 +11,9 @@
 // rows of mma.sync.m16n8k16.  Where there are fewer items than SMs, a cluster of 2, 4 or 8 CTAs shares one: the tile pairs of
 // every phase are dealt out to its CTAs, which exchange the soft-max statistics and the scores through each other's shared
 // memory and then select the blocks each for itself (one CTA alone draws at most 1/148 of the bandwidth: 4 items of 4096 keys
-// took 25 us).  Two producer warps stream [64 rows x 128] tiles by TMA through a twelve-slot ring (192 KB
-// in flight per SM); six consumer warps own two slots each, so every slot is filled and drained by the same pair of
-// warps in order.  The tile stream of an item:
+// took 25 us).  Where there are more, two CTAs of half the size share an SM.  Producer warps stream [64 rows x 128] tiles by TMA
+// through a ring (192 KB in flight per SM); each consumer warp owns two slots, so every slot is filled and drained by the same
+// pair of warps in order.  The tile stream of an item:
 //   1. ck tiles:           raw scores -> per-row maxima and sums of the unscaled soft-max over ALL compressed keys and
 //                          of the scaled, masked attention soft-max (merged over the warps in shared memory);
 //   2. (ck, cv) pairs:     scores again (ck comes from L2 this time) -> attention P.cv with the final statistics, and
@@ -21,11 +21,12 @@
 //                          then pooling and a warp top-n while the other warps go on;
 //   3. window (k, v) pairs and 4. selected (k, v) pairs: online soft-max per warp.
 // Every warp leaves its partial (maximum, sum, unnormalised output) of each branch in a caller-provided workspace (the split-KV
-// scheme of decode attention).  Where one CTA does a whole item, its six warps then merge the item's partials, a row at a
-// time each and in a fixed order, from a scratch that the CTA's next item uses again (22 MB for the grid, it stays in L2), while the
-// ring fills with the next item's tiles.  With clusters a second, small kernel does that.  Measured: the second kernel for
-// all (scratch for every item, 77 MB written and read for 512 of them) @MEAS@; merging through shared memory, warp after warp, cost
-// seven named barriers and six serialised rounds per branch.  No atomics; every wait is bounded.
+// scheme of decode attention).  The CTAs of an item then merge its rows, in a fixed order: without clusters each warp a row at a
+// time, from a scratch that the CTA's next item uses again (it stays in L2) while the ring fills with that item's tiles; with
+// clusters each CTA its share of the rows, a row and branch per warp.  Measured, 128 sequences of 4096 to 32768 keys: a second
+// kernel that merges (77 MB of partials written and read) 179 us, merged here 176, and with two CTAs per SM 149 (4.7 TB/s); one
+// sequence of 4096 keys 18.9 us with the second kernel and 18.4 without.  Merging through shared memory, warp after warp, cost seven
+// named barriers and six serialised rounds per branch.  No atomics; every wait is bounded.
 #include <algorithm>
 #include <array>
 
@@ -279,6 +280,78 @@ __device__ __forceinline__ void online_pair(float (&acc)[D / 8][4], float (&m_ru
   if (lane == 0) mbar_arrive(v_empty);
 }
 
+// One row and branch of an item that a cluster shared: the partials of all its warps merged in a fixed order (CTA by CTA, warp by
+// warp), by one warp, a lane holding four channels.  Branch order in the workspace: 0 compressed, 1 selected, 2 window.  Warps that
+// had no tile are left out.  The first loads are under way while the weights are formed.  Returns the output as rounded.
+static_assert(kMaxCluster * kCons <= 64, "two partials per lane below");
+__device__ __forceinline__ float4 merge_row(const DecodeArgs& a, int item, long long qrow, int r, int br, int nw, int lane) {
+  constexpr int kFirst = 6;   // (no cluster has fewer warps)
+  const float* part = a.part + ((long long)item * 3 + br) * nw * kPartFloats;
+  const float* hd = part + 16 * D + r;
+  float m[2], l[2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    m[k] = -INFINITY;
+    l[k] = 0.f;
+    const int w = lane + 32 * k;
+    if (w < nw) {
+      m[k] = __ldcg(hd + w * kPartFloats);
+      l[k] = __ldcg(hd + w * kPartFloats + 16);
+    }
+  }
+  const float4* base = reinterpret_cast<const float4*>(part + r * D) + lane;
+  float4 first[kFirst];
+#pragma unroll
+  for (int w = 0; w < kFirst; ++w) first[w] = __ldcg(base + w * (kPartFloats / 4));
+  float M = fmaxf(m[0], m[1]);
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
+  float e[2], L = 0.f;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    e[k] = m[k] > -INFINITY ? ex2(m[k] - M) : 0.f;
+    if (m[k] > -INFINITY) L += l[k] * e[k];
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) L += __shfl_xor_sync(0xffffffffu, L, off);
+  const float inv = L > 0.f ? 1.f / L : 0.f;
+  e[0] *= inv;
+  e[1] *= inv;
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto add = [&](const float4& x, float w) {
+    v.x += x.x * w; v.y += x.y * w; v.z += x.z * w; v.w += x.w * w;
+  };
+#pragma unroll
+  for (int w = 0; w < kFirst; ++w) {
+    const float wt = __shfl_sync(0xffffffffu, e[0], w);
+    if (wt != 0.f) add(first[w], wt);   // (a warp without a tile has left no output)
+  }
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    unsigned rest = __ballot_sync(0xffffffffu, e[k] != 0.f && (k || lane >= kFirst));
+    while (rest) {   // eight at a time
+      float4 x[8];
+      float wt[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int w = rest ? __ffs(rest) - 1 : 0;
+        wt[u] = rest ? __shfl_sync(0xffffffffu, e[k], w) : 0.f;
+        if (rest) x[u] = __ldcg(base + (w + 32 * k) * (kPartFloats / 4));
+        rest &= rest - 1;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (wt[u] != 0.f) add(x[u], wt[u]);
+    }
+  }
+  const __nv_bfloat162 b0 = __floats2bfloat162_rn(v.x, v.y), b1 = __floats2bfloat162_rn(v.z, v.w);
+  bf16* out = br == 0 ? a.o_cmp : br == 1 ? a.o_slc : a.o_swa;
+  if (out) *reinterpret_cast<uint2*>(out + qrow * D + lane * 4) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+  if (a.lse && lane == 0) a.lse[(long long)br * a.nseq * a.Hq + qrow] = L > 0.f ? (M + log2f(L)) * kLn2 : -INFINITY;
+  const float2 f0 = __bfloat1622float2(b0), f1 = __bfloat1622float2(b1);
+  return make_float4(f0.x, f0.y, f1.x, f1.y);
+}
+
 // CONS consumer warps with a pair of slots each; CL: the CTAs of a cluster share an item.
 template <int CONS, bool CL>
 __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
@@ -322,7 +395,6 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
     fence_mbar_init();
   }
   __syncthreads();
-  if (cl > 1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the merge may take its places now: it waits for this grid's end
   if (cl > 1) cluster_sync_all();   // no CTA writes into another's shared memory before it runs, or after it ended (below)
 
   const int nitem = a.nseq * a.Hkv;
@@ -336,7 +408,7 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
     // A warp's TMA instructions run one after another (about 850 + 52 x boxes cycles each, whatever the box size), so
     // a single warp issuing one 16 KB tile per instruction caps the SM at ~16 bytes per clock.  Tiles therefore go out
     // in PAIRS (four boxes per instruction: both tiles of a (K, V) pair, or two consecutive ck tiles of pass 1), and
-    // the two producer warps take alternate pairs.
+    // the producer warps (one in a CTA that shares its SM) take alternate pairs.
     const int pw = warp - CONS;
     uint32_t np = 0, it = 0;     // tile pairs issued so far by both producers together; items so far
     auto issue2 = [&](const CUtensorMap* tmA, int rowA, const CUtensorMap* tmB, int rowB, int h) -> bool {
@@ -654,7 +726,7 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
 
     // ---- gates, by the last warp (the first one is still choosing blocks) --------------------------------
     // (what the item before left in gates, ml and the scratch has been read: its rows are merged before anything of this one)
-    if (cl == 1 && warp == CONS - 1) {
+    if (warp == CONS - 1) {
       if (a.gate_w) {
         // g_x[row] = q[row,:] . W[x,:] + b[x] (nn.Linear(head_dim, 3), rows of W: selected, window, compressed) as one 16 x 8
         // tile of mma.sync, rounded to bf16 as the module's gate tensors are
@@ -777,131 +849,24 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
     }
   }
   }
-  if (cl > 1) {
+  if (CL) {
     __syncwarp();
-    cluster_sync_all();
-  }
-}
-
-// Clusters: merge of the per-warp partials, in a fixed order (CTA by CTA, warp by warp): one warp per (item, query row, branch), a lane holds
-// four channels.  Branch order in the workspace: 0 compressed, 1 selected, 2 window.  Warps that had no tile are left out.  The
-// loads of the first CTA's partials (all of them without clusters) are under way while their weights are formed in the warp;
-// the gates (computed from q when the gate projection is given) do not wait for the main kernel.  Few registers and blocks of
-// two rows: what is in flight is what counts (512 items are 77 MB; four rows and 64 registers took 36 us, one block per item with a
-// thread per channel 19).
-constexpr int kMergeRows = 2;
-static_assert(kMaxCluster * kCons <= 64, "two partials per lane below");
-__global__ void __launch_bounds__(96 * kMergeRows) decode_merge_kernel(const DecodeArgs a, const int cl) {
-  const int item = blockIdx.x / (16 / kMergeRows);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, br = warp % 3;
-  const int r = blockIdx.x % (16 / kMergeRows) * kMergeRows + warp / 3;
-  const int nw = cl * kCons;
-  const int sq = item / a.Hkv, h = item % a.Hkv;
-  const int seq = a.order ? a.order[sq] : sq;
-  const long long qrow = (long long)seq * a.Hq + h * 16 + r;
-  __shared__ float4 out_s[kMergeRows][3][32];
-  __shared__ float gate_s[kMergeRows][3];
-  const bool has = !(br == 2 && a.window <= 0);
-  {
-    const bf16* gin = br == 0 ? a.g_cmp : br == 1 ? a.g_slc : a.g_swa;
-    float gv = 1.f;
-    if (a.gate_w) {
-      // g_x[row] = q[row,:] . W[x,:] + b[x] (nn.Linear(head_dim, 3), rows of W: selected, window, compressed), rounded to
-      // bf16 as the module's gate tensors are
-      const int x = br == 0 ? 2 : br - 1;
-      const uint2 wv = *reinterpret_cast<const uint2*>(a.gate_w + x * D + lane * 4), qv = *reinterpret_cast<const uint2*>(a.q + qrow * D + lane * 4);
-      const float2 w0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&wv.x)), w1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&wv.y));
-      const float2 q0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&qv.x)), q1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&qv.y));
-      float p = q0.x * w0.x + q0.y * w0.y + q1.x * w1.x + q1.y * w1.y;
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) p += __shfl_xor_sync(0xffffffffu, p, off);
-      if (a.gate_b) p += __bfloat162float(a.gate_b[x]);
-      gv = __bfloat162float(__float2bfloat16(p));
-    } else if (gin) {
-      gv = __bfloat162float(gin[qrow]);
-    }
-    if (lane == 0) gate_s[warp / 3][br] = gv;
-  }
-  // Launched with programmatic stream serialization: everything above (the gate projection reads only q and the
-  // weights) may run while the main kernel is still finishing; its partials are read only behind this wait.
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (has) {
-    const float* part = a.part + ((long long)item * 3 + br) * nw * kPartFloats;
-    const float* hd = part + 16 * D + r;
-    float m[2], l[2];
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      m[k] = -INFINITY;
-      l[k] = 0.f;
-      const int w = lane + 32 * k;
-      if (w < nw) {
-        m[k] = hd[w * kPartFloats];
-        l[k] = hd[w * kPartFloats + 16];
+    cluster_sync_all();   // every CTA's partials are written (a cluster has one item), and no CTA writes into another's memory any more
+    if (warp >= CONS) return;
+    const int item = group, sq = item / a.Hkv, h = item % a.Hkv, rows = 16 / cl, nb = a.window > 0 ? 3 : 2;
+    const long long qrow = (long long)(a.order ? a.order[sq] : sq) * a.Hq + h * 16 + rank * rows;   // first of this CTA's rows
+    float4* out = reinterpret_cast<float4*>(ps);   // [row][branch][lane], over what the item no longer needs
+    for (int u = warp; u < rows * nb; u += CONS) out[u * 32 + lane] = merge_row(a, item, qrow + u / nb, rank * rows + u / nb, u % nb, cl * CONS, lane);
+    named_bar_sync(1, CONS * 32);
+    for (int row = warp; row < rows; row += CONS) {
+      float4 tot = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int br = 0; br < nb; ++br) {
+        const float gt = gates[br * 16 + rank * rows + row];
+        const float4 f = out[(row * nb + br) * 32 + lane];
+        tot.x += gt * f.x; tot.y += gt * f.y; tot.z += gt * f.z; tot.w += gt * f.w;
       }
+      *reinterpret_cast<uint2*>(a.o + (qrow + row) * D + lane * 4) = make_uint2(pack_bf16(tot.x, tot.y), pack_bf16(tot.z, tot.w));
     }
-    const float4* base = reinterpret_cast<const float4*>(part + r * D) + lane;
-    float4 first[kCons];
-#pragma unroll
-    for (int w = 0; w < kCons; ++w) first[w] = base[w * (kPartFloats / 4)];
-    float M = fmaxf(m[0], m[1]);
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
-    float e[2], L = 0.f;
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      e[k] = m[k] > -INFINITY ? ex2(m[k] - M) : 0.f;
-      if (m[k] > -INFINITY) L += l[k] * e[k];
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) L += __shfl_xor_sync(0xffffffffu, L, off);
-    const float inv = L > 0.f ? 1.f / L : 0.f;
-    e[0] *= inv;
-    e[1] *= inv;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    auto add = [&](const float4& x, float w) {
-      v.x += x.x * w; v.y += x.y * w; v.z += x.z * w; v.w += x.w * w;
-    };
-#pragma unroll
-    for (int w = 0; w < kCons; ++w) {
-      const float wt = __shfl_sync(0xffffffffu, e[0], w);
-      if (wt != 0.f) add(first[w], wt);   // (a warp without a tile has left no output)
-    }
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      unsigned rest = __ballot_sync(0xffffffffu, e[k] != 0.f && (k || lane >= kCons));
-      while (rest) {   // of the other CTAs, four at a time
-        float4 x[4];
-        float wt[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int w = rest ? __ffs(rest) - 1 : 0;
-          wt[u] = rest ? __shfl_sync(0xffffffffu, e[k], w) : 0.f;
-          if (rest) x[u] = base[(w + 32 * k) * (kPartFloats / 4)];
-          rest &= rest - 1;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (wt[u] != 0.f) add(x[u], wt[u]);
-      }
-    }
-    __nv_bfloat162 b0 = __floats2bfloat162_rn(v.x, v.y), b1 = __floats2bfloat162_rn(v.z, v.w);
-    bf16* out = br == 0 ? a.o_cmp : br == 1 ? a.o_slc : a.o_swa;
-    if (out) *reinterpret_cast<uint2*>(out + qrow * D + lane * 4) = make_uint2(*reinterpret_cast<uint32_t*>(&b0), *reinterpret_cast<uint32_t*>(&b1));
-    if (a.lse && lane == 0) a.lse[(long long)br * a.nseq * a.Hq + qrow] = L > 0.f ? (M + log2f(L)) * kLn2 : -INFINITY;
-    const float2 f0 = __bfloat1622float2(b0), f1 = __bfloat1622float2(b1);
-    out_s[warp / 3][br][lane] = make_float4(f0.x, f0.y, f1.x, f1.y);
-  }
-  __syncthreads();
-  if (br == 0) {
-    float4 tot = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int x = 0; x < 3; ++x) {
-      if (x == 2 && a.window <= 0) continue;
-      const float g = gate_s[warp / 3][x];
-      const float4 f = out_s[warp / 3][x][lane];
-      tot.x += g * f.x; tot.y += g * f.y; tot.z += g * f.z; tot.w += g * f.w;
-    }
-    *reinterpret_cast<uint2*>(a.o + qrow * D + lane * 4) = make_uint2(pack_bf16(tot.x, tot.y), pack_bf16(tot.z, tot.w));
   }
 }
 
@@ -927,33 +892,28 @@ cudaLaunchConfig_t decode_config(int ncta, int cons, int cl, cudaLaunchAttribute
 }
 // Clusters of cl CTAs that the GPU holds at a time (fewer than SMs / cl: a cluster lies within one GPC; 16 of 8 would be 128
 // of 148 SMs, but they do not all fit and the rest would run as a second wave).
-int resident_clusters(int cl) {
-  static const auto held = [] {
-    std::array<int, 4> n = {};
-    for (int i = 0; i < 4; ++i) {
-      n[i] = num_sms() >> i;
-      int c = 0;
-      cudaLaunchAttribute at;
-      const cudaLaunchConfig_t cfg = decode_config(num_sms() >> i << i, kCons, 1 << i, &at, nullptr);
-      if (i > 0 && cudaFuncSetAttribute(decode_kernel<kCons, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, decode_smem(kCons)) == cudaSuccess &&
-          cudaOccupancyMaxActiveClusters(&c, decode_kernel<kCons, true>, &cfg) == cudaSuccess)
-        n[i] = c;
-      cudaGetLastError();   // (no device: workspace sizes can be asked for all the same)
-    }
-    return n;
-  }();
-  return held[cl == 8 ? 3 : cl == 4 ? 2 : cl == 2 ? 1 : 0];
+int ask_resident(int cl) {
+  int c = 0;
+  cudaLaunchAttribute at;
+  const cudaLaunchConfig_t cfg = decode_config(num_sms() / cl * cl, kCons, cl, &at, nullptr);
+  if (cudaFuncSetAttribute(decode_kernel<kCons, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, decode_smem(kCons)) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&c, decode_kernel<kCons, true>, &cfg) != cudaSuccess)
+    c = num_sms() / cl;
+  cudaGetLastError();   // (no device: workspace sizes can be asked for all the same)
+  return c;
 }
-// How `nitem` items are spread: CTAs per item, as many as keep every item in the first wave; with more items than SMs two CTAs
-// of half the warps and slots share an SM, so that one streams tiles while the other chooses its blocks or merges its rows.
+// How `nitem` items are spread: up to the number of SMs as many CTAs per item as keep every item in the first wave, with an SM
+// to itself each; with more items two CTAs of half the warps and slots share an SM, so that one streams tiles while the other
+// chooses its blocks or merges its rows.  (128 items of up to 16384 keys: one CTA of six warps each 42 us, a cluster of two of three
+// warps 51.)
 struct Spread {
   int cons, cl, ncta;
 };
 Spread decode_spread(int nitem) {
-  if (nitem > num_sms()) return {kHalfCons, 1, std::min(nitem, 2 * num_sms())};
-  int cl = kMaxCluster;
-  while (cl > 1 && nitem > resident_clusters(cl)) cl >>= 1;
-  return {kCons, cl, nitem * cl};
+  static const std::array<int, 4> held = {num_sms(), ask_resident(2), ask_resident(4), ask_resident(8)};
+  for (int i = 3; i >= 0; --i)
+    if (nitem <= held[i]) return {kCons, 1 << i, nitem << i};
+  return {kHalfCons, 1, std::min(nitem, 2 * num_sms())};
 }
 
 }  // namespace
@@ -1005,22 +965,6 @@ int launch_decode(const DecodeArgs& a, cudaStream_t s) {
     if (e != cudaSuccess) return (int)e;
   }
   note_launches(1);
-  if (cl > 1) {
-    // the merge kernel may be scheduled before the main kernel has drained (it waits with griddepcontrol.wait)
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)nitem * (16 / kMergeRows));
-    cfg.blockDim = dim3(96 * kMergeRows);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, decode_merge_kernel, a, cl);
-    if (e != cudaSuccess) return (int)e;
-    note_launches(1);
-  }
   return (int)cudaGetLastError();
 }
 int decode_status(int* out) {
