@@ -4,14 +4,14 @@
 // block, too few for a tensor-core tile, so here a CTA owns one 64-key block and the QUERIES that selected it arrive in
 // batches of 8 tokens x 16 heads = 128 rows (the block's ascending token list from the reverse index).  Per batch:
 //     S     [128 rows x 64 keys] = Qg . K^T     A = Qg (K-major, gathered by TMA), B = K (K-major)
-//     O_part[128 rows x 128 d  ] = P . V        A = P (K-major, written by the soft-max warps), B = V (MN-major)
+//     O_part[128 rows x 128 d  ] = P . V        A = P (tensor memory, written by the soft-max warps), B = V (MN-major)
 // with P = exp(scale S - m), m the row's maximum over the block's visible keys.  The visit leaves (m, l = sum P) per
 // row and O_part as a [16 heads x D] bf16 tile at the visit's position in the reverse-index list; a second kernel
 // merges a token's visits in slot order (fixed order, no atomics):  o = sum_v 2^(m_v - M) O_v / sum_v 2^(m_v - M) l_v.
 // K and V of a block are read once per CTA instead of once per visiting query (32 KB per visit in the query-major
 // kernel, which is bound by that gather).
-// Roles (512 threads): warps 0-2 TMA producers (4-stage ring of 32 KB Q tiles; a stage is free as soon as its score MMAs
-// have completed), warp 3 the MMA issuer (event loop), warps 4-7 / 8-11 two soft-max groups (even / odd batches, one
+// Roles (512 threads): warps 0-1 TMA producers (4-stage ring of 32 KB Q tiles; a stage is free as soon as its score MMAs
+// have completed), warps 2 and 3 issue S and P.V, warps 4-7 / 8-11 two soft-max groups (even / odd batches, one
 // row per thread), warps 12-15 read O_part out of tensor memory into a staging tile that one bulk store writes.
 // Every wait is bounded; on a time-out the role records an error and leaves its loop.
 #include "kernels.h"
@@ -23,21 +23,21 @@ namespace nsa {
 namespace {
 
 constexpr int D = 128;
-constexpr int kProd = 3;
-constexpr int kMmaWarp = kProd;
-constexpr int kSoftWarp = kProd + 1;        // 8 soft-max warps: two groups of four
+constexpr int kProd = 2;
+constexpr int kMmaWarp = kProd;             // issues S
+constexpr int kMma2Warp = kProd + 1;        // issues P.V: one thread for both took 900 cycles for either
+constexpr int kSoftWarp = kProd + 2;        // 8 soft-max warps: two groups of four
 constexpr int kDrainWarp = kSoftWarp + 8;   // 4 drain warps
 constexpr int kThreads = (kDrainWarp + 4) * 32;
 constexpr int kTokB = 8;
 constexpr uint32_t KV_PANEL = 64 * 128;     // [64 keys][64 ch]
 constexpr uint32_t KV_TILE = 2 * KV_PANEL;  // 16 KB
 constexpr uint32_t Q_TILE = 128 * 256;       // 32 KB: [16 row groups][2 column panels][8 rows][128 B]
-constexpr uint32_t P_TILE = 128 * 128;      // [128 rows][64 keys]
 constexpr uint32_t STG_TILE = 128 * 256;    // [128 rows][128 d] bf16
-constexpr int kStages = 3;
-constexpr uint32_t kSmem = 2 * KV_TILE + kStages * Q_TILE + 2 * P_TILE + 2 * STG_TILE + 256 + 1024;
-constexpr uint32_t kTmemCols = 512;         // S: 0..63 | 64..127; O_part: 128..255 | 256..383
-constexpr uint32_t kColO = 128;
+constexpr int kStages = 4;
+constexpr uint32_t kSmem = 2 * KV_TILE + kStages * Q_TILE + 2 * STG_TILE + 256 + 1024;
+constexpr uint32_t kTmemCols = 512;         // S: 0..63 | 64..127; O_part: 128..255 | 256..383; P: 384..415 | 416..447
+constexpr uint32_t kColO = 128, kColP = 384;
 
 __global__ void __launch_bounds__(kThreads, 1)
     sel_fwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -49,8 +49,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t k_s = sbase, v_s = sbase + KV_TILE;
   const uint32_t ring = sbase + 2 * KV_TILE;
-  const uint32_t p_s0 = ring + kStages * Q_TILE;
-  const uint32_t stg = p_s0 + 2 * P_TILE;
+  const uint32_t stg = ring + kStages * Q_TILE;
   const uint32_t bar_base = stg + 2 * STG_TILE;
   // barriers (8 bytes each); the double ones are indexed by batch & 1
   const uint32_t full0 = bar_base, empty0 = bar_base + 32, kv_bar = bar_base + 64, s_full = bar_base + 72,
@@ -102,7 +101,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     // a batch is 8 boxes of 4 KB, one per token: the token's [16 heads x 128 d] rows through a 4-D view of q
     // (64 columns, 8 rows, 2 column panels, row groups) land as [row group][panel][8 rows][128 B], so the 8-row swizzle
     // atoms of one panel sit 2 KB apart over the whole tile (SBO = 2048, second panel at +1 KB).  One box per token
-    // instead of one per (token, panel): the gather is bound by the number of boxes.  Box x = 3 * lane + warp belongs
+    // instead of one per (token, panel): the gather is bound by the number of boxes.  Box x = 2 * lane + warp belongs
     // to this lane
     if (warp == 0 && lane == 0) {
       mbar_expect_tx(kv_bar, 2 * KV_TILE);
@@ -138,68 +137,46 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     }
   } else if (nb > 0 && warp == kMmaWarp) {
-    // ------------------------------- MMA issuer ---------------------------------------------------------------
+    // ------------------------------- MMA issuer A: S ------------------------------------------------------------
     if (lane == 0) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, 64, 0, 0);    // both operands K-major
-      constexpr uint32_t idesc_o = umma_idesc_bf16(128, 128, 0, 1);   // A = P K-major, B = V MN-major
       bool ok = mbar_wait(kv_bar, 0, DEV_ERR_FULL_WAIT);
-      const uint64_t dK = umma_smem_desc(k_s, 0, 1024);
-      const uint64_t dVmn = umma_smem_desc(v_s, KV_PANEL, 1024);
-      uint64_t dQ[kStages], dP[2];
-#pragma unroll
-      for (int i = 0; i < kStages; ++i) dQ[i] = umma_smem_desc(ring + i * Q_TILE, 0, 2048);
-#pragma unroll
-      for (int i = 0; i < 2; ++i) dP[i] = umma_smem_desc(p_s0 + i * P_TILE, 0, 1024);
-      auto issue_s = [&](int n) {
+      const uint64_t dK = umma_smem_desc(k_s, 0, 1024), dQ0 = umma_smem_desc(ring, 0, 2048);
+      for (int n = 0; ok && n < nb; ++n) {
         const int st = n % kStages;
-        const uint64_t aq = st == 0 ? dQ[0] : st == 1 ? dQ[1] : dQ[2];
+        ok = mbar_wait(full0 + 8 * st, (n / kStages) & 1, DEV_ERR_FULL_WAIT) &&
+             (n < 2 || mbar_wait(s_free + 8 * (n & 1), ((n >> 1) - 1) & 1, DEV_ERR_EMPTY_WAIT));
+        if (!ok) break;
+        tc_fence_after();
+        const uint64_t aq = umma_desc_advance(dQ0, st * Q_TILE);
         const uint32_t col = (n & 1) * 64;
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
           const uint32_t aoff = (ks >> 2) * 1024 + (ks & 3) * 32, boff = (ks >> 2) * KV_PANEL + (ks & 3) * 32;
           umma_ss(tmem + col, umma_desc_advance(aq, aoff), umma_desc_advance(dK, boff), idesc_s, ks ? 1u : 0u);
         }
-        umma_commit(empty0 + 8 * st);          // the Q tile is only needed for the scores
         umma_commit(s_full + 8 * (n & 1));
-      };
-      auto issue_o = [&](int n) {
-        const uint64_t ap = (n & 1) ? dP[1] : dP[0];
+        umma_commit(empty0 + 8 * st);          // the Q tile is only needed for the scores
+      }
+    }
+  } else if (nb > 0 && warp == kMma2Warp) {
+    // ------------------------------- MMA issuer B: P.V ----------------------------------------------------------
+    if (lane == 0) {
+      constexpr uint32_t idesc_o = umma_idesc_bf16(128, 128, 0, 1);   // A = P in tensor memory, B = V MN-major
+      bool ok = mbar_wait(kv_bar, 0, DEV_ERR_FULL_WAIT);
+      const uint64_t dVmn = umma_smem_desc(v_s, KV_PANEL, 1024);
+      for (int n = 0; ok && n < nb; ++n) {
+        ok = mbar_wait(p_full + 8 * (n & 1), (n >> 1) & 1, DEV_ERR_FULL_WAIT) &&
+             (n < 2 || mbar_wait(o_free + 8 * (n & 1), ((n >> 1) - 1) & 1, DEV_ERR_EMPTY_WAIT));
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t ap = tmem + kColP + (n & 1) * 32;   // 16 keys = 8 packed columns per step
         const uint32_t col = kColO + (n & 1) * 128;
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks)   // contraction over the 64 keys, 16 per step
-          umma_ss(tmem + col, umma_desc_advance(ap, ks * 32), umma_desc_advance(dVmn, ks * 2048), idesc_o, ks ? 1u : 0u);
-        umma_commit(p_free + 8 * (n & 1));
+          umma_ts(tmem + col, ap + ks * 8, umma_desc_advance(dVmn, ks * 2048), idesc_o, ks ? 1u : 0u);
         umma_commit(o_full + 8 * (n & 1));
-      };
-      // event loop: whichever of the next score product and the next P.V is ready
-      int ns = 0, no = 0;
-      uint64_t t_idle = 0;
-      while (ok && no < nb) {
-        bool progressed = false;
-        if (ns < nb && mbar_test(full0 + 8 * (ns % kStages), (ns / kStages) & 1) &&
-            (ns < 2 || mbar_test(s_free + 8 * (ns & 1), ((ns >> 1) - 1) & 1))) {
-          tc_fence_after();
-          issue_s(ns);
-          ++ns;
-          progressed = true;
-        }
-        if (no < ns && mbar_test(p_full + 8 * (no & 1), (no >> 1) & 1) &&
-            (no < 2 || mbar_test(o_free + 8 * (no & 1), ((no >> 1) - 1) & 1))) {
-          tc_fence_after();
-          issue_o(no);
-          ++no;
-          progressed = true;
-        }
-        if (progressed) {
-          t_idle = 0;
-        } else {   // bounded: ~2 s without any progress is reported as a pipeline failure
-          const uint64_t now = global_timer_ns();
-          if (t_idle == 0) t_idle = now;
-          else if (now - t_idle > 2000000000ull) {
-            atomicCAS(&g_dev_error, 0, (int)DEV_ERR_FULL_WAIT);
-            ok = false;
-          }
-        }
+        umma_commit(p_free + 8 * (n & 1));
       }
     }
   } else if (nb > 0 && warp >= kDrainWarp) {
@@ -298,29 +275,31 @@ __global__ void __launch_bounds__(kThreads, 1)
         m2 = fmaxf(m2, sv[c]);
       }
       float l = 0.f;
-      uint32_t pw[32];
+      float pw[32];   // packed pairs
       if (nvis > 0) {
 #pragma unroll
         for (int c = 0; c < 64; c += 2) {
           const float p0 = ex2(sv[c] - m2), p1 = ex2(sv[c + 1] - m2);
-          pw[c / 2] = pack_bf16(p0, p1);
+          const uint32_t pk = pack_bf16(p0, p1);
+          pw[c / 2] = __uint_as_float(pk);
           // l is the sum of the rounded probabilities the tensor core multiplies, as in the query-major kernel
-          const __nv_bfloat162 pr = *reinterpret_cast<const __nv_bfloat162*>(&pw[c / 2]);
+          const __nv_bfloat162 pr = *reinterpret_cast<const __nv_bfloat162*>(&pk);
           l += __low2float(pr) + __high2float(pr);
         }
       } else {
 #pragma unroll
-        for (int c = 0; c < 32; ++c) pw[c] = 0u;
+        for (int c = 0; c < 32; ++c) pw[c] = 0.f;
       }
       if (use >= 1) {
-        ok = mbar_wait(p_free + 8 * g, (use - 1) & 1, DEV_ERR_EMPTY_WAIT);   // P.V of batch n-2 has read this tile
+        ok = mbar_wait(p_free + 8 * g, (use - 1) & 1, DEV_ERR_EMPTY_WAIT);   // P.V of batch n-2 has read these columns
         if (!ok) break;
       }
-      uint8_t* prow = sgen + (p_s0 - sbase) + g * P_TILE + row * 128;
-#pragma unroll
-      for (int c = 0; c < 8; ++c)
-        *reinterpret_cast<uint4*>(prow + ((c ^ (row & 7)) * 16)) = make_uint4(pw[4 * c], pw[4 * c + 1], pw[4 * c + 2], pw[4 * c + 3]);
-      fence_proxy_async();
+      tc_fence_after();
+      const uint32_t p_col = tmem + lane_addr + kColP + g * 32;
+      tmem_st16(p_col, *reinterpret_cast<float(*)[16]>(&pw[0]));
+      tmem_st16(p_col + 16, *reinterpret_cast<float(*)[16]>(&pw[16]));
+      tmem_st_wait();
+      tc_fence_before();
       mbar_arrive(p_full + 8 * g);
       if (live) {
         float2* st = reinterpret_cast<float2*>(a.stats) + (((long long)bh * a.rev_cap + ta_lo + i) * G16 + sub) * 16 + head;
