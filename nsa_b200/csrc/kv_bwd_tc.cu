@@ -102,7 +102,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int G16 = (a.Hq / a.Hk) / 16;
   const int NB = (a.T + 63) / 64;
   const int seg = blockIdx.x % a.nshare, item = blockIdx.x / a.nshare;
-  const int blk = item % NB, bh = item / NB, b = bh / a.Hk, hk = bh % a.Hk;
+  const int nbh = a.B * a.Hk;   // shares of a list: longest lists first (few enough items for all of Q and dO to stay in L2)
+  const int blk = a.nshare > 1 ? item / nbh : item % NB, bh = a.nshare > 1 ? item % nbh : item / NB, b = bh / a.Hk, hk = bh % a.Hk;
   const int* rp = a.rev_ptr + (long long)bh * (NB + 1);
   const int* list = a.rev_tok + (long long)bh * a.rev_cap;
   int lo = rp[blk], nA = rp[blk + 1] - lo;

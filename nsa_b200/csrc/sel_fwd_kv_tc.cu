@@ -14,6 +14,7 @@
 // have completed), warps 2 and 3 issue S and P.V, warps 4-7 / 8-11 two soft-max groups (even / odd batches, one
 // row per thread), warps 12-15 read O_part out of tensor memory into a staging tile that one bulk store writes.
 // Every wait is bounded; on a time-out the role records an error and leaves its loop.
+#include <algorithm>
 #include "kernels.h"
 #include "tc.cuh"
 #include "tmap.h"
@@ -41,7 +42,7 @@ constexpr uint32_t kColO = 128, kColP = 384;
 
 __global__ void __launch_bounds__(kThreads, 1)
     sel_fwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                      const __grid_constant__ CUtensorMap tmV, const SelKvArgs a) {
+                      const __grid_constant__ CUtensorMap tmV, const SelKvArgs a, const int nshare) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t sbase = (raw + 1023u) & ~1023u;
@@ -81,15 +82,22 @@ __global__ void __launch_bounds__(kThreads, 1)
   tc_fence_after();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(sgen + (tmem_slot - sbase));
 
-  // ---- work item: (batch, kv head)-major so the resident CTAs share one head group's Q rows in L2 -------------
+  // ---- work item: (batch, kv head)-major so the resident CTAs share one head group's Q rows in L2; shares of a block's
+  // list block-major, longest lists first (there are few enough of them for all of Q to stay in L2) ----------------------
   const int G16 = (a.Hq / a.Hk) / 16;
   const int NB = (a.T + 63) / 64;
-  const int blk = (int)(blockIdx.x % NB);
-  const int bh = (int)(blockIdx.x / NB);
+  const int seg = (int)(blockIdx.x % nshare), item = (int)(blockIdx.x / nshare);
+  const int blk = nshare > 1 ? item / (a.B * a.Hk) : item % NB;
+  const int bh = nshare > 1 ? item % (a.B * a.Hk) : item / NB;
   const int b = bh / a.Hk, hk = bh % a.Hk;
   const int* rp = a.rev_ptr + (long long)bh * (NB + 1);
-  const int ta_lo = rp[blk];
-  const int nA = rp[blk + 1] - ta_lo;
+  int ta_lo = rp[blk], nA = rp[blk + 1] - ta_lo;
+  if (nshare > 1) {   // this CTA's share of the list, in whole batches
+    const int ba = (nA + kTokB - 1) / kTokB;
+    const int a0 = ba * seg / nshare * kTokB, a1 = min(nA, ba * (seg + 1) / nshare * kTokB);
+    ta_lo += a0;
+    nA = a1 - a0;
+  }
   const int* list = a.rev_tok + (long long)bh * a.rev_cap + ta_lo;
   const int key0 = blk * 64;
   const int nb_sub = (nA + kTokB - 1) / kTokB;
@@ -471,13 +479,19 @@ int launch_sel_fwd_kv(const SelKvArgs& a, const RevArgs& r, cudaStream_t s) {
   if (rc) return rc;
   cudaError_t e = cudaFuncSetAttribute(sel_fwd_kv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
   if (e != cudaSuccess) return (int)e;
-  const long long grid = (long long)a.B * a.Hk * ((a.T + 63) / 64);
-  if (grid <= 0) return 0;
+  // The first block is visible to every token, the last to few: with few blocks per SM the first one's CTA would be the last to
+  // end.  Up to eight CTAs then share a block's list, so that there are three or more per SM (a visit's results have a place of
+  // their own, nothing is added up; a CTA's start and end cost about two batches).  One sequence of 5003 tokens, 4 KV heads: 245 us
+  // with one CTA a block, 160 / 159 / 169 / 177 with 3 / 4 / 6 / 8 per SM; 2 x 2080 tokens, 2 KV heads: 140, then 76 / 80 / 88 / 89.
+  const long long blocks = (long long)a.B * a.Hk * ((a.T + 63) / 64), want = 3LL * num_sms();
+  if (blocks <= 0) return 0;
+  const int nshare = (int)std::max(1LL, std::min(8LL, (want + blocks - 1) / blocks));
+  const long long grid = blocks * nshare;
   if (grid > 0x7fffffffLL) {
     set_error("selected forward: grid too large");
     return -33;
   }
-  sel_fwd_kv_kernel<<<(unsigned)grid, kThreads, kSmem, s>>>(tmQ, tmK, tmV, a);
+  sel_fwd_kv_kernel<<<(unsigned)grid, kThreads, kSmem, s>>>(tmQ, tmK, tmV, a, nshare);
   note_launches(1);
   e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
