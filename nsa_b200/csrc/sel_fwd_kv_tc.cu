@@ -480,12 +480,13 @@ int launch_sel_fwd_kv(const SelKvArgs& a, const RevArgs& r, cudaStream_t s) {
   cudaError_t e = cudaFuncSetAttribute(sel_fwd_kv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
   if (e != cudaSuccess) return (int)e;
   // The first block is visible to every token, the last to few: with few blocks per SM the first one's CTA would be the last to
-  // end.  Up to eight CTAs then share a block's list, so that there are three or more per SM (a visit's results have a place of
+  // end.  Up to eight CTAs then share a block's list, so that there are three or more per SM, or at least two CTAs up to six blocks per SM (a visit's results have a place of
   // their own, nothing is added up; a CTA's start and end cost about two batches).  One sequence of 5003 tokens, 4 KV heads: 245 us
   // with one CTA a block, 160 / 159 / 169 / 177 with 3 / 4 / 6 / 8 per SM; 2 x 2080 tokens, 2 KV heads: 140, then 76 / 80 / 88 / 89.
+  // Two CTAs a block, 4 KV heads: 9000 tokens (564 blocks) 374 -> 308, 14000 tokens (876) 557 -> 494, 17000 tokens (1064) 559 -> 616.
   const long long blocks = (long long)a.B * a.Hk * ((a.T + 63) / 64), want = 3LL * num_sms();
   if (blocks <= 0) return 0;
-  const int nshare = (int)std::max(1LL, std::min(8LL, (want + blocks - 1) / blocks));
+  const int nshare = blocks >= 2 * want ? 1 : (int)std::max(2LL, std::min(8LL, (want + blocks - 1) / blocks));
   const long long grid = blocks * nshare;
   if (grid > 0x7fffffffLL) {
     set_error("selected forward: grid too large");
