@@ -11,8 +11,8 @@
 // Eight soft-max warps own half a row per thread (lse, delta, gate and the causal mask are thread-local, no
 // shuffles; warps 2-5 take key columns 0-31, warps 6-9 columns 32-63 of the same TMEM lanes): they read S and dP
 // from TMEM, form P and dS = P (g dP - delta), and store both as bf16 tiles.
-// The MMA thread issues S/dP of batch n+1 before dV/dK of batch n, so the tensor core works while the soft-max
-// warps compute.  dV^T and dK^T stay in TMEM for the CTA's whole token stream and are stored once.
+// The MMA threads issue S/dP of batch n+1 before dV/dK of batch n, so the tensor core works while the soft-max
+// warps compute; the exponentials start when S alone is there, dV when P alone is written.  dV^T and dK^T stay in TMEM for the CTA's whole token stream and are stored once.
 // Optionally dQ comes out of this kernel too: dS of a batch is already in shared memory,
 // so one more product  dQ_part[128 rows x 128 d] = dS . K  (A = dS K-major, B = K MN-major, a third accumulator in TMEM)
 // gives the batch's contribution to dQ, which the soft-max warps store as bf16 tiles indexed by the batch's positions
@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t full0 = bar_base, empty0 = bar_base + 16, kv_bar = bar_base + 32, sdp_full = bar_base + 40,
                  sdp_free = bar_base + 56, pds_full = bar_base + 72, pds_free = bar_base + 88, acc_full = bar_base + 104,
                  tmem_slot = bar_base + 112, dq_full = bar_base + 120, dq_free = bar_base + 128, stg_full = bar_base + 136,
-                 stg_free = bar_base + 144;   // stg_free: two barriers, one per P/dS pair
+                 stg_free = bar_base + 144, s_full = bar_base + 160, p_full = bar_base + 176;   // stg_free: two barriers, one per P/dS pair
   if (threadIdx.x == 0) {
     for (int i = 0; i < kStages; ++i) {
       mbar_init(full0 + 8 * i, kProd);
@@ -77,7 +77,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     mbar_init(kv_bar, 1);
     for (int i = 0; i < 2; ++i) {
+      mbar_init(s_full + 8 * i, 1);
       mbar_init(sdp_full + 8 * i, 1);
+      mbar_init(p_full + 8 * i, kSoftThreads);
       mbar_init(sdp_free + 8 * i, kSoftThreads);
       mbar_init(pds_full + 8 * i, kSoftThreads);
       mbar_init(pds_free + 8 * i, 1);
@@ -191,6 +193,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int ks = 0; ks < 8; ++ks) {
           const uint32_t aoff = (ks >> 2) * 1024 + (ks & 3) * 32, boff = (ks >> 2) * KV_PANEL + (ks & 3) * 32;
           umma_ss(tmem + col, umma_desc_advance(aq, aoff), umma_desc_advance(dK, boff), idesc_kk, ks ? 1u : 0u);
+        }
+        umma_commit(s_full + 8 * (n & 1));   // the exponentials need S alone
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks) {
+          const uint32_t aoff = (ks >> 2) * 1024 + (ks & 3) * 32, boff = (ks >> 2) * KV_PANEL + (ks & 3) * 32;
           umma_ss(tmem + col + 64, umma_desc_advance(ado, aoff), umma_desc_advance(dV, boff), idesc_kk, ks ? 1u : 0u);
         }
         umma_commit(sdp_full + 8 * (n & 1));
@@ -217,16 +224,20 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       const uint64_t dKmn = umma_smem_desc(k_s, KV_PANEL, 1024);
       for (int n = 0; ok && n < nb; ++n) {
-        ok = mbar_wait(pds_full + 8 * (n & 1), (n >> 1) & 1, DEV_ERR_FULL_WAIT);
+        ok = mbar_wait(p_full + 8 * (n & 1), (n >> 1) & 1, DEV_ERR_FULL_WAIT);
         if (!ok) break;
         tc_fence_after();
         const uint64_t aq = (n % kStages) ? dQmn[1] : dQmn[0], ado = (n % kStages) ? dDOmn[1] : dDOmn[0];
         const uint64_t bp = (n & 1) ? dP[1] : dP[0], bds = (n & 1) ? dDS[1] : dDS[0];
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {  // contraction over the 128 rows, 16 per step; dV and dK alternate
+        for (int ks = 0; ks < 8; ++ks)   // contraction over the 128 rows, 16 per step; dV while the soft-max warps form dS
           umma_ss(tmem + kColDV, umma_desc_advance(ado, ks * 4096), umma_desc_advance(bp, ks * 2048), idesc_mn, (n | ks) ? 1u : 0u);
+        ok = mbar_wait(pds_full + 8 * (n & 1), (n >> 1) & 1, DEV_ERR_FULL_WAIT);
+        if (!ok) break;
+        tc_fence_after();
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks)
           umma_ss(tmem + kColDK, umma_desc_advance(aq, ks * 4096), umma_desc_advance(bds, ks * 2048), idesc_mn, (n | ks) ? 1u : 0u);
-        }
         umma_commit(empty0 + 8 * (n % kStages));
         if (emit_dq) {
           // the previous partial must have been read out of its accumulator by the drain warps
@@ -363,48 +374,30 @@ __global__ void __launch_bounds__(kThreads, 1)
 
       const uint32_t buf = n & 1, use = n >> 1;
       const uint32_t tcol = buf * 128;
-      ok = mbar_wait(sdp_full + 8 * buf, use & 1, DEV_ERR_FULL_WAIT);
+      ok = mbar_wait(s_full + 8 * buf, use & 1, DEV_ERR_FULL_WAIT);
       if (!ok) break;
       tc_fence_after();
-      uint32_t pw[16], dw[16];   // 32 bf16 each
-      {
-        float sv[32], dpv[32];
-        tmem_ld16(tmem + lane_addr + tcol + half * 32, *reinterpret_cast<float(*)[16]>(&sv[0]));
-        tmem_ld16(tmem + lane_addr + tcol + half * 32 + 16, *reinterpret_cast<float(*)[16]>(&sv[16]));
-        tmem_ld16(tmem + lane_addr + tcol + 64 + half * 32, *reinterpret_cast<float(*)[16]>(&dpv[0]));
-        tmem_ld16(tmem + lane_addr + tcol + 64 + half * 32 + 16, *reinterpret_cast<float(*)[16]>(&dpv[16]));
-        tmem_ld_wait();
-        tc_fence_before();
-        mbar_arrive(sdp_free + 8 * buf);   // S and dP are in registers: batch n+2 may overwrite this TMEM buffer
-        const int kfirst = key0 + half * 32, klast = kfirst + 31;
-        const bool all_valid = klast <= t;
-        const float lse2 = ri.lse * kLog2e, del = ri.del, gv = __bfloat162float(ri.g);
-        if (!live || !(lse2 > -INFINITY)) {
+      float p[32];
+      uint32_t pw[16];   // 32 bf16
+      tmem_ld16(tmem + lane_addr + tcol + half * 32, *reinterpret_cast<float(*)[16]>(&p[0]));
+      tmem_ld16(tmem + lane_addr + tcol + half * 32 + 16, *reinterpret_cast<float(*)[16]>(&p[16]));
+      tmem_ld_wait();
+      const int kfirst = key0 + half * 32, klast = kfirst + 31;
+      const float lse2 = ri.lse * kLog2e, del = ri.del, gv = __bfloat162float(ri.g);
+      const bool dead = !live || !(lse2 > -INFINITY);
+      if (dead) {
 #pragma unroll
-          for (int e = 0; e < 16; ++e) pw[e] = dw[e] = 0u;
-        } else if (all_valid) {
-          const float nl = -lse2;
+        for (int e = 0; e < 32; ++e) p[e] = 0.f;
+      } else if (klast <= t) {
+        const float nl = -lse2;
 #pragma unroll
-          for (int e = 0; e < 32; e += 2) {
-            const float p0 = ex2(fmaf(sv[e], sl2, nl)), p1 = ex2(fmaf(sv[e + 1], sl2, nl));
-            pw[e / 2] = pack_bf16(p0 * gv, p1 * gv);
-            dw[e / 2] = pack_bf16(p0 * fmaf(gv, dpv[e], -del), p1 * fmaf(gv, dpv[e + 1], -del));
-          }
-        } else {
+        for (int e = 0; e < 32; ++e) p[e] = ex2(fmaf(p[e], sl2, nl));
+      } else {
 #pragma unroll
-          for (int e = 0; e < 32; e += 2) {
-            float pv[2];
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-              const int kp = kfirst + e + u;
-              const bool valid = kp <= t;
-              pv[u] = valid ? ex2(sv[e + u] * sl2 - lse2) : 0.f;
-            }
-            pw[e / 2] = pack_bf16(pv[0] * gv, pv[1] * gv);
-            dw[e / 2] = pack_bf16(pv[0] * fmaf(gv, dpv[e], -del), pv[1] * fmaf(gv, dpv[e + 1], -del));
-          }
-        }
+        for (int e = 0; e < 32; ++e) p[e] = kfirst + e <= t ? ex2(p[e] * sl2 - lse2) : 0.f;
       }
+#pragma unroll
+      for (int e = 0; e < 32; e += 2) pw[e / 2] = pack_bf16(p[e] * gv, p[e + 1] * gv);
       if (n >= 2) {
         ok = mbar_wait(pds_free + 8 * buf, (use - 1) & 1, DEV_ERR_EMPTY_WAIT);   // dV/dK of batch n-2 have read this pair
         if (!ok) break;
@@ -417,11 +410,27 @@ __global__ void __launch_bounds__(kThreads, 1)
       uint8_t* prow = sgen + (p_s0 - sbase) + buf * 2 * P_TILE + row * 128;
       uint8_t* drow = prow + P_TILE;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const int pos = ((4 * half + c) ^ (row & 7)) * 16;
-        *reinterpret_cast<uint4*>(prow + pos) = make_uint4(pw[4 * c], pw[4 * c + 1], pw[4 * c + 2], pw[4 * c + 3]);
-        *reinterpret_cast<uint4*>(drow + pos) = make_uint4(dw[4 * c], dw[4 * c + 1], dw[4 * c + 2], dw[4 * c + 3]);
+      for (int c = 0; c < 4; ++c)
+        *reinterpret_cast<uint4*>(prow + ((4 * half + c) ^ (row & 7)) * 16) = make_uint4(pw[4 * c], pw[4 * c + 1], pw[4 * c + 2], pw[4 * c + 3]);
+      fence_proxy_async();
+      mbar_arrive(p_full + 8 * buf);
+      ok = mbar_wait(sdp_full + 8 * buf, use & 1, DEV_ERR_FULL_WAIT);
+      if (!ok) break;
+      tc_fence_after();
+      float dpv[32];
+      tmem_ld16(tmem + lane_addr + tcol + 64 + half * 32, *reinterpret_cast<float(*)[16]>(&dpv[0]));
+      tmem_ld16(tmem + lane_addr + tcol + 64 + half * 32 + 16, *reinterpret_cast<float(*)[16]>(&dpv[16]));
+      tmem_ld_wait();
+      tc_fence_before();
+      mbar_arrive(sdp_free + 8 * buf);   // S and dP are in registers: batch n+2 may overwrite this TMEM buffer
+#pragma unroll
+      for (int e = 0; e < 32; e += 2) {
+        const uint32_t d2 = pack_bf16(p[e] * fmaf(gv, dpv[e], -del), p[e + 1] * fmaf(gv, dpv[e + 1], -del));
+        pw[e / 2] = dead ? 0u : d2;
       }
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        *reinterpret_cast<uint4*>(drow + ((4 * half + c) ^ (row & 7)) * 16) = make_uint4(pw[4 * c], pw[4 * c + 1], pw[4 * c + 2], pw[4 * c + 3]);
       fence_proxy_async();
       mbar_arrive(pds_full + 8 * buf);
     }
