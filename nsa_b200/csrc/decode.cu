@@ -11,7 +11,7 @@
 // rows of mma.sync.m16n8k16.  Where there are fewer items than SMs, a cluster of 2, 4 or 8 CTAs shares one: the tile pairs of
 // every phase are dealt out to its CTAs, which exchange the soft-max statistics and the scores through each other's shared
 // memory and then select the blocks each for itself (one CTA alone draws at most 1/148 of the bandwidth: 4 items of 4096 keys
-// took 25 us).  Where there are more, two CTAs of half the size share an SM.  Producer warps stream [64 rows x 128] tiles by TMA
+// took 25 us).  Producer warps stream [64 rows x 128] tiles by TMA
 // through a ring (192 KB in flight per SM); each consumer warp owns two slots, so every slot is filled and drained by the same
 // pair of warps in order.  The tile stream of an item:
 //   1. ck tiles:           raw scores -> per-row maxima and sums of the unscaled soft-max over ALL compressed keys and
@@ -24,7 +24,7 @@
 // scheme of decode attention).  The CTAs of an item then merge its rows, in a fixed order: without clusters each warp a row at a
 // time, from a scratch that the CTA's next item uses again (it stays in L2) while the ring fills with that item's tiles; with
 // clusters each CTA its share of the rows, a row and branch per warp.  Measured, 128 sequences of 4096 to 32768 keys: a second
-// kernel that merges (77 MB of partials written and read) 179 us, merged here 176, and with two CTAs per SM 149 (4.7 TB/s); one
+// kernel that merges (77 MB of partials written and read) 179 us, merged here 170; one
 // sequence of 4096 keys 18.9 us with the second kernel and 18.4 without.  Merging through shared memory, warp after warp, cost seven
 // named barriers and six serialised rounds per branch.  No atomics; every wait is bounded.
 #include <algorithm>
@@ -38,8 +38,10 @@ namespace nsa {
 namespace {
 
 constexpr int D = 128;
-constexpr int kCons = 6;                       // consumer warps of a CTA that has an SM to itself
-constexpr int kHalfCons = 3;                   // ... of one that shares it with another
+constexpr int kCons = 6;                       // consumer warps
+constexpr int kProdW = 2;                      // producer warps
+constexpr int kThreads = (kCons + kProdW) * 32;
+constexpr int kSlots = 2 * kCons;
 constexpr uint32_t PANEL = 64 * 128;           // [64 rows][64 columns] bf16
 constexpr uint32_t TILE = 2 * PANEL;           // 16 KB
 constexpr int kMaxTc = 2048;                   // compressed positions of one sequence held in shared memory
@@ -57,7 +59,6 @@ struct Plan {   // tile pairs of one item's phases; CTA `rank` of a cluster take
   int w0;      // first window key
 };
 
-template <int CONS>
 __device__ __forceinline__ Plan make_plan(const DecodeArgs& a, int seq, int cl) {
   Plan p;
   p.row_k = a.cu_k[seq];
@@ -73,7 +74,7 @@ __device__ __forceinline__ Plan make_plan(const DecodeArgs& a, int seq, int cl) 
   // An exchange costs about as much as one pair (3500 cycles): with no more than a pair for each warp nothing is shared in the
   // two passes, every CTA makes its own statistics and scores.  (Both passes or neither: that every CTA has sent its statistics
   // also says that none still reads the scores of the item before.)
-  p.cs = p.n2p > CONS ? cl : 1;
+  p.cs = p.n2p > kCons ? cl : 1;
   p.w0 = max(0, p.L - a.window);
   p.nw = a.window > 0 ? (p.L - p.w0 + 63) / 64 : 0;
   return p;
@@ -225,10 +226,6 @@ __device__ __forceinline__ int top_blocks(const float* pooled, int2* tmp, int n_
   return lane < n ? tmp[lane].x : -1;
 }
 
-// Producer warps: one issues 30 bytes per cycle (see below), what one of two CTAs of an SM can draw at most.
-__host__ __device__ constexpr int decode_producers(int cons) { return cons == kCons ? 2 : 1; }
-__host__ __device__ constexpr int decode_threads(int cons) { return (cons + decode_producers(cons)) * 32; }
-
 // One (K, V) pair of an online soft-max: keys key0 .. key0+63 of the tile are valid iff kmin <= key < kmax.
 __device__ __forceinline__ void online_pair(float (&acc)[D / 8][4], float (&m_run)[2], float (&l_run)[2],
                                             const uint32_t (&qf)[D / 16][4], uint32_t kbase, uint32_t vbase, uint32_t k_empty,
@@ -352,12 +349,11 @@ __device__ __forceinline__ float4 merge_row(const DecodeArgs& a, int item, long 
   return make_float4(f0.x, f0.y, f1.x, f1.y);
 }
 
-// CONS consumer warps with a pair of slots each; CL: the CTAs of a cluster share an item.
-template <int CONS, bool CL>
-__global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
+// CL: the CTAs of a cluster share an item.
+template <bool CL>
+__global__ void __launch_bounds__(kThreads, 1)
     decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                   const __grid_constant__ CUtensorMap tmCK, const __grid_constant__ CUtensorMap tmCV, const DecodeArgs a, const int ncl) {
-  constexpr int kSlots = 2 * CONS, kProdW = decode_producers(CONS);
   const int cl = CL ? ncl : 1;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -368,11 +364,11 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
   uint8_t* after = sgen + kSlots * TILE;
   float* ps = reinterpret_cast<float*>(after);                    // [kMaxTc + 64] head-summed p_sel per compressed position
   float* pooled = ps + kMaxTc + 64;                               // [kMaxPoolD]
-  float* stat = pooled + kMaxPoolD;                               // [CONS][4][16] per-warp statistics
-  float* fin = stat + CONS * 64;                                 // [4][16] merged: M_raw, 1/L_raw, M_att (log2), L_att
+  float* stat = pooled + kMaxPoolD;                               // [kCons][4][16] per-warp statistics
+  float* fin = stat + kCons * 64;                                 // [4][16] merged: M_raw, 1/L_raw, M_att (log2), L_att
   float* xstat = fin + 64;                                        // [cluster][4][16] the CTAs' statistics
-  float2* ml = reinterpret_cast<float2*>(xstat + kMaxCluster * 64);   // [3][CONS][16] (m, l) of the warps' partials, without clusters
-  float* gates = reinterpret_cast<float*>(ml + 3 * CONS * 16);       // [3][16], branch order as ml's
+  float2* ml = reinterpret_cast<float2*>(xstat + kMaxCluster * 64);   // [3][kCons][16] (m, l) of the warps' partials, without clusters
+  float* gates = reinterpret_cast<float*>(ml + 3 * kCons * 16);       // [3][16], branch order as ml's
   int* sel = reinterpret_cast<int*>(gates + 48);                  // [kMaxSel] selected blocks of the item, [kMaxSel] = count
   volatile int* abort_flag = sel + kMaxSel + 2;
   const uint32_t bar_base = sbase + kSlots * TILE + (uint32_t)((uint8_t*)(sel + kMaxSel + 4) - after);
@@ -403,13 +399,13 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
   auto deal = [&](int i, int cs) { return !CL || cs == 1 ? i : rank + i * cs; };
   const int pool_k = a.sel_block / a.cstride + 1, pool_s = a.sel_block / a.cstride;
 
-  if (warp >= CONS) {
+  if (warp >= kCons) {
     // ------------------------------- producers --------------------------------------------------------
     // A warp's TMA instructions run one after another (about 850 + 52 x boxes cycles each, whatever the box size), so
     // a single warp issuing one 16 KB tile per instruction caps the SM at ~16 bytes per clock.  Tiles therefore go out
     // in PAIRS (four boxes per instruction: both tiles of a (K, V) pair, or two consecutive ck tiles of pass 1), and
-    // the producer warps (one in a CTA that shares its SM) take alternate pairs.
-    const int pw = warp - CONS;
+    // the two producer warps take alternate pairs.
+    const int pw = warp - kCons;
     uint32_t np = 0, it = 0;     // tile pairs issued so far by both producers together; items so far
     auto issue2 = [&](const CUtensorMap* tmA, int rowA, const CUtensorMap* tmB, int rowB, int h) -> bool {
       const uint32_t mine = np % kProdW == (uint32_t)pw;
@@ -439,7 +435,7 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
       if (item >= nitem) continue;
       const int sq = item / a.Hkv, h = item % a.Hkv;
       const int seq = a.order ? a.order[sq] : sq;
-      const Plan p = make_plan<CONS>(a, seq, cl);
+      const Plan p = make_plan(a, seq, cl);
       bool ok = true;
       for (int j = p.cs > 1 ? rank : 0; ok && j < p.n1p; j += p.cs) ok = issue2(&tmCK, p.row_c + j * 128, &tmCK, p.row_c + j * 128 + 64, h);
       for (int j = p.cs > 1 ? rank : 0; ok && j < p.n2p; j += p.cs) ok = issue2(&tmCK, p.row_c + j * 64, &tmCV, p.row_c + j * 64, h);
@@ -460,13 +456,13 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
   // --------------------------------- consumers ----------------------------------------------------------
   const int g = lane >> 2, tq = lane & 3;
   const float sl2 = a.scale * kLog2e;
-  const int cthreads = CONS * 32;
+  const int cthreads = kCons * 32;
   const int ct = threadIdx.x;               // 0 .. cthreads-1
-  // tile pair i of the CTA, over all phases and items, is warp i % CONS's, in that warp's own two slots
+  // tile pair i of the CTA, over all phases and items, is warp i % kCons's, in that warp's own two slots
   uint32_t np0 = 0, it = 0;                 // pairs of the CTA before the current phase; items so far
   uint32_t use = 0;                         // pairs of this warp so far
   const uint32_t sk = 2 * warp, sv = sk + 1;
-  auto first_pair = [&]() { return (int)((warp + CONS - np0 % CONS) % CONS); };
+  auto first_pair = [&]() { return (int)((warp + kCons - np0 % kCons) % kCons); };
   uint32_t nx = 0;                          // items with an exchange so far
   bool ok = true;
   for (int r = 0; r * ngroup < nitem; ++r) {
@@ -474,7 +470,7 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
     if (item >= nitem) continue;
     const int sq = item / a.Hkv, h = item % a.Hkv;
     const int seq = a.order ? a.order[sq] : sq;
-    const Plan p = make_plan<CONS>(a, seq, cl);
+    const Plan p = make_plan(a, seq, cl);
     const int t = p.L - 1;
     const long long qrow = (long long)seq * a.Hq + h * 16;     // first of the 16 (head) rows of this item
     uint32_t qf[D / 16][4];
@@ -485,7 +481,7 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
     float ma[2] = {-INFINITY, -INFINITY}, la[2] = {0.f, 0.f};   // scaled scores, visible keys
     {
       const int n = share(p.n1p, p.cs);
-      for (int i = first_pair(); i < n; i += CONS, ++use) {
+      for (int i = first_pair(); i < n; i += kCons, ++use) {
         const int u = deal(i, p.cs);
 #pragma unroll 1
         for (int e = 0; e < 2; ++e) {
@@ -545,12 +541,12 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
     named_bar_sync(1, cthreads);
     if (ct < 16) {
       float Mr = -INFINITY, Ma = -INFINITY;
-      for (int w = 0; w < CONS; ++w) {
+      for (int w = 0; w < kCons; ++w) {
         Mr = fmaxf(Mr, stat[w * 64 + ct]);
         Ma = fmaxf(Ma, stat[w * 64 + 32 + ct]);
       }
       float Lr = 0.f, La = 0.f;
-      for (int w = 0; w < CONS; ++w) {
+      for (int w = 0; w < kCons; ++w) {
         const float m1 = stat[w * 64 + ct], m2 = stat[w * 64 + 32 + ct];
         if (m1 > -INFINITY) Lr += stat[w * 64 + 16 + ct] * ex2(m1 - Mr);
         if (m2 > -INFINITY) La += stat[w * 64 + 48 + ct] * ex2(m2 - Ma);
@@ -607,7 +603,7 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
     bool full = rank == 0 && warp == 0;   // this warp's partial has an output (the first always: the row sums ride with it)
     {
       const int n = share(p.n2p, p.cs);
-      for (int i = first_pair(); i < n; i += CONS, ++use) {
+      for (int i = first_pair(); i < n; i += kCons, ++use) {
         const int u = deal(i, p.cs);
         full = p.cs > 1 || rank == 0;
         const int j0 = u * 64;
@@ -692,7 +688,7 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
     // this warp's partial of a branch -> workspace: [item][branch][warp of the cluster]{ O[16][D], m[16], l[16] } fp32; a warp
     // that had no tile leaves m = -inf and no O
     auto put_partial = [&](int branch, const float (&x)[D / 8][4], const float (&mm)[2], const float (&ll)[2], bool has) {
-      float* dst = a.part + (((long long)(cl > 1 ? item : (int)blockIdx.x) * 3 + branch) * (cl * CONS) + rank * CONS + warp) * kPartFloats;
+      float* dst = a.part + (((long long)(cl > 1 ? item : (int)blockIdx.x) * 3 + branch) * (cl * kCons) + rank * kCons + warp) * kPartFloats;
 #pragma unroll
       for (int i = 0; i < D / 8; ++i) {
         if (!has) break;
@@ -708,7 +704,7 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
             dst[16 * D + g + 8 * rr] = m;
             dst[16 * D + 16 + g + 8 * rr] = l;
           } else {
-            ml[(branch * CONS + warp) * 16 + g + 8 * rr] = make_float2(m, l);
+            ml[(branch * kCons + warp) * 16 + g + 8 * rr] = make_float2(m, l);
           }
         }
       }
@@ -726,7 +722,7 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
 
     // ---- gates, by the last warp (the first one is still choosing blocks) --------------------------------
     // (what the item before left in gates, ml and the scratch has been read: its rows are merged before anything of this one)
-    if (warp == CONS - 1) {
+    if (warp == kCons - 1) {
       if (a.gate_w) {
         // g_x[row] = q[row,:] . W[x,:] + b[x] (nn.Linear(head_dim, 3), rows of W: selected, window, compressed) as one 16 x 8
         // tile of mma.sync, rounded to bf16 as the module's gate tensors are
@@ -761,7 +757,7 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
     full = false;
     {
       const int n = share(p.nw, cl);
-      for (int i = first_pair(); i < n; i += CONS, ++use) {
+      for (int i = first_pair(); i < n; i += kCons, ++use) {
         const int u = deal(i, cl);
         full = true;
         ok = ok && mbar_wait_abortable(full_bar(sk), use & 1, DEV_ERR_FULL_WAIT, abort_flag);
@@ -785,7 +781,7 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
     full = false;
     {
       const int n = share(nsel, cl);
-      for (int i = first_pair(); i < n; i += CONS, ++use) {
+      for (int i = first_pair(); i < n; i += kCons, ++use) {
         const int u = deal(i, cl);
         full = true;
         const int blk = *reinterpret_cast<volatile int*>(sel + u);
@@ -799,27 +795,27 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
     named_bar_sync(1, cthreads);   // ps, pooled, fin and sel are reused by the next item
     ++it;
     // ---- this item's rows: partials merged warp by warp, gated sum of the branches (a lane holds four channels) --------
-    for (int row = warp; cl == 1 && row < 16; row += CONS) {
-      const float4* base = reinterpret_cast<const float4*>(a.part + (long long)blockIdx.x * 3 * CONS * kPartFloats + row * D) + lane;
-      float4 x[3][CONS];
-      float e[3][CONS], inv[3], lse[3];
+    for (int row = warp; cl == 1 && row < 16; row += kCons) {
+      const float4* base = reinterpret_cast<const float4*>(a.part + (long long)blockIdx.x * 3 * kCons * kPartFloats + row * D) + lane;
+      float4 x[3][kCons];
+      float e[3][kCons], inv[3], lse[3];
 #pragma unroll
       for (int br = 0; br < 3; ++br)
 #pragma unroll
-        for (int w = 0; w < CONS; ++w) {
-          e[br][w] = ml[(br * CONS + w) * 16 + row].x;
+        for (int w = 0; w < kCons; ++w) {
+          e[br][w] = ml[(br * kCons + w) * 16 + row].x;
           x[br][w] = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (e[br][w] > -INFINITY) x[br][w] = __ldcg(base + (br * CONS + w) * (kPartFloats / 4));
+          if (e[br][w] > -INFINITY) x[br][w] = __ldcg(base + (br * kCons + w) * (kPartFloats / 4));
         }
 #pragma unroll
       for (int br = 0; br < 3; ++br) {
         float M = e[br][0], L = 0.f;
 #pragma unroll
-        for (int w = 1; w < CONS; ++w) M = fmaxf(M, e[br][w]);
+        for (int w = 1; w < kCons; ++w) M = fmaxf(M, e[br][w]);
 #pragma unroll
-        for (int w = 0; w < CONS; ++w) {
+        for (int w = 0; w < kCons; ++w) {
           e[br][w] = e[br][w] > -INFINITY ? ex2(e[br][w] - M) : 0.f;
-          L += ml[(br * CONS + w) * 16 + row].y * e[br][w];
+          L += ml[(br * kCons + w) * 16 + row].y * e[br][w];
         }
         inv[br] = L > 0.f ? 1.f / L : 0.f;
         lse[br] = L > 0.f ? (M + log2f(L)) * kLn2 : -INFINITY;
@@ -830,7 +826,7 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
         if (br == 2 && a.window <= 0) continue;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int w = 0; w < CONS; ++w) {
+        for (int w = 0; w < kCons; ++w) {
           const float wt = e[br][w] * inv[br];
           v.x = fmaf(x[br][w].x, wt, v.x);
           v.y = fmaf(x[br][w].y, wt, v.y);
@@ -852,13 +848,13 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
   if (CL) {
     __syncwarp();
     cluster_sync_all();   // every CTA's partials are written (a cluster has one item), and no CTA writes into another's memory any more
-    if (warp >= CONS) return;
+    if (warp >= kCons) return;
     const int item = group, sq = item / a.Hkv, h = item % a.Hkv, rows = 16 / cl, nb = a.window > 0 ? 3 : 2;
     const long long qrow = (long long)(a.order ? a.order[sq] : sq) * a.Hq + h * 16 + rank * rows;   // first of this CTA's rows
     float4* out = reinterpret_cast<float4*>(ps);   // [row][branch][lane], over what the item no longer needs
-    for (int u = warp; u < rows * nb; u += CONS) out[u * 32 + lane] = merge_row(a, item, qrow + u / nb, rank * rows + u / nb, u % nb, cl * CONS, lane);
-    named_bar_sync(1, CONS * 32);
-    for (int row = warp; row < rows; row += CONS) {
+    for (int u = warp; u < rows * nb; u += kCons) out[u * 32 + lane] = merge_row(a, item, qrow + u / nb, rank * rows + u / nb, u % nb, cl * kCons, lane);
+    named_bar_sync(1, kCons * 32);
+    for (int row = warp; row < rows; row += kCons) {
       float4 tot = make_float4(0.f, 0.f, 0.f, 0.f);
       for (int br = 0; br < nb; ++br) {
         const float gt = gates[br * 16 + rank * rows + row];
@@ -870,18 +866,17 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
   }
 }
 
-constexpr int decode_smem(int cons) {
-  return 2 * cons * (int)TILE + (kMaxTc + 64 + kMaxPoolD + cons * 64 + 64 + kMaxCluster * 64 + 3 * cons * 32 + 48) * 4 + (kMaxSel + 4) * 4 +
-         (4 * cons + 3) * 8 + 16 + 1024;
+constexpr int decode_smem() {
+  return kSlots * (int)TILE + (kMaxTc + 64 + kMaxPoolD + kCons * 64 + 64 + kMaxCluster * 64 + 3 * kCons * 32 + 48) * 4 + (kMaxSel + 4) * 4 +
+         (2 * kSlots + 3) * 8 + 16 + 1024;
 }
-static_assert(2 * (decode_smem(kHalfCons) + 1024) <= 228 * 1024, "two CTAs per SM");
 
 // A launch of `ncta` CTAs in clusters of `cl`.
-cudaLaunchConfig_t decode_config(int ncta, int cons, int cl, cudaLaunchAttribute* at, cudaStream_t s) {
+cudaLaunchConfig_t decode_config(int ncta, int cl, cudaLaunchAttribute* at, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)ncta);
-  cfg.blockDim = dim3(decode_threads(cons));
-  cfg.dynamicSmemBytes = decode_smem(cons);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = decode_smem();
   cfg.stream = s;
   at->id = cudaLaunchAttributeClusterDimension;
   at->val.clusterDim.x = cl;
@@ -895,32 +890,32 @@ cudaLaunchConfig_t decode_config(int ncta, int cons, int cl, cudaLaunchAttribute
 int ask_resident(int cl) {
   int c = 0;
   cudaLaunchAttribute at;
-  const cudaLaunchConfig_t cfg = decode_config(num_sms() / cl * cl, kCons, cl, &at, nullptr);
-  if (cudaFuncSetAttribute(decode_kernel<kCons, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, decode_smem(kCons)) != cudaSuccess ||
-      cudaOccupancyMaxActiveClusters(&c, decode_kernel<kCons, true>, &cfg) != cudaSuccess)
+  const cudaLaunchConfig_t cfg = decode_config(num_sms() / cl * cl, cl, &at, nullptr);
+  if (cudaFuncSetAttribute(decode_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, decode_smem()) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&c, decode_kernel<true>, &cfg) != cudaSuccess)
     c = num_sms() / cl;
   cudaGetLastError();   // (no device: workspace sizes can be asked for all the same)
   return c;
 }
-// How `nitem` items are spread: up to the number of SMs as many CTAs per item as keep every item in the first wave, with an SM
-// to itself each; with more items two CTAs of half the warps and slots share an SM, so that one streams tiles while the other
-// chooses its blocks or merges its rows.  (128 items of up to 16384 keys: one CTA of six warps each 42 us, a cluster of two of three
-// warps 51.)
+// How `nitem` items are spread: up to the number of SMs as many CTAs per item as keep every item in the first wave, with more a
+// CTA per SM that takes one after another.  (Two CTAs of three warps per SM, so that one streams tiles while the other chooses
+// its blocks, took 155 us for 128 sequences of 4096 to 32768 keys; but they add up the soft-max of the scores in another
+// order, and blocks whose scores tie to within a rounding, which one in 700 items has, were then chosen differently.)
 struct Spread {
-  int cons, cl, ncta;
+  int cl, ncta;
 };
 Spread decode_spread(int nitem) {
   static const std::array<int, 4> held = {num_sms(), ask_resident(2), ask_resident(4), ask_resident(8)};
   for (int i = 3; i >= 0; --i)
-    if (nitem <= held[i]) return {kCons, 1 << i, nitem << i};
-  return {kHalfCons, 1, std::min(nitem, 2 * num_sms())};
+    if (nitem <= held[i]) return {1 << i, nitem << i};
+  return {1, num_sms()};
 }
 
 }  // namespace
 
 size_t decode_workspace_bytes(int nseq, int Hkv) {
   const Spread p = decode_spread(nseq * Hkv);   // a set of partials for every CTA (of a cluster: one item each)
-  return (size_t)p.ncta * 3 * p.cons * kPartFloats * sizeof(float);
+  return (size_t)p.ncta * 3 * kCons * kPartFloats * sizeof(float);
 }
 
 int launch_decode(const DecodeArgs& a, cudaStream_t s) {
@@ -955,12 +950,12 @@ int launch_decode(const DecodeArgs& a, cudaStream_t s) {
   if (nitem <= 0) return 0;
   const Spread p = decode_spread(nitem);
   const int cl = p.cl;
-  const auto kernel = p.cons == kHalfCons ? decode_kernel<kHalfCons, false> : cl > 1 ? decode_kernel<kCons, true> : decode_kernel<kCons, false>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, decode_smem(p.cons));
+  const auto kernel = cl > 1 ? decode_kernel<true> : decode_kernel<false>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, decode_smem());
   if (e != cudaSuccess) return (int)e;
   {
     cudaLaunchAttribute at;
-    const cudaLaunchConfig_t cfg = decode_config(p.ncta, p.cons, cl, &at, s);
+    const cudaLaunchConfig_t cfg = decode_config(p.ncta, cl, &at, s);
     e = cudaLaunchKernelEx(&cfg, kernel, tmK, tmV, tmCK, tmCV, a, cl);
     if (e != cudaSuccess) return (int)e;
   }
