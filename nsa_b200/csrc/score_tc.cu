@@ -254,7 +254,14 @@ __global__ void __launch_bounds__(kThreads, 1)
       const bool ok = mbar_wait_abortable(pool_full0 + 8 * slot, (ic / (uint32_t)nslot) & 1, 306, abort_flag);
       const int t_w = st.t0 + w * 4, nlive = min(4, st.Tq - t_w);   // this warp's four tokens
       if (ok && nlive > 0) {
-        const float* src = pl + w * 4 * pool_floats;
+        float* src = pl + w * 4 * pool_floats;
+        // Causal scores: the soft-max groups have written the tiles up to the item's last visible key; behind them lies what the
+        // slot held before, where every score is zero.
+        if (causal) {
+          for (int u = 0; u < nlive; ++u)
+            for (int blk = 32 * nt + lane; blk < n_pool; blk += 32) src[u * pool_floats + blk] = 0.f;
+          __syncwarp();
+        }
         int* out = a.sel_idx + ((st.row0 + t_w) * HG + hg) * a.n_sel;
         float* dump = a.sel_scores ? a.sel_scores + ((long long)(st.b * HG + hg) * st.Tq + t_w) * n_pool : nullptr;
         const long long os = (long long)HG * a.n_sel;
