@@ -680,7 +680,24 @@ static int sel_swa_bwd_impl(const void* q, const void* k, const void* v, const v
   }
   if (dq) {
     int acc = accumulate_dq;
-    if (has_swa || cmp) {   // first: with `fold` it also forms the deltas of both branches
+    // The selected branch's dQ from its own query-major kernel (else the reduction behind the key-major kernel adds it).  dq is
+    // rounded to bf16 behind every kernel, so with the compressed branch in the dense pass the selected one, the smaller, goes
+    // first (head_dim 64, 1024 tokens, error of dq against fp64: 3.12 to 3.16e-3 with the dense pass first, 3.04e-3 so).
+    auto selected = [&]() {
+      SelArgs a = {};
+      a.q = (const bf16*)q; a.k = (const bf16*)k; a.v = (const bf16*)v; a.idx = idx; a.idx64 = idx64; a.counts = counts;
+      a.lse = const_cast<float*>(lse_slc); a.dout = (const bf16*)dout_slc; a.delta = delta_slc;
+      a.gate = (const bf16*)gate_slc; a.dq = (bf16*)dq; a.accumulate = acc;
+      a.B = B; a.T = T; a.Tq = Tq; a.q0 = q0; a.Hq = Hq; a.Hkv = Hkv; a.S = S; a.BS = BS; a.scale = scale;
+      acc = 1;
+      return launch_sel_dq(a, D, s);
+    };
+    const bool own_dq = has_slc && !dq_from_kv, sel_first = own_dq && cmp && !fold;
+    if (sel_first) {
+      rc = selected();
+      if (rc) return rc;
+    }
+    if (has_swa || cmp) {   // with `fold` it also forms the deltas of both branches
       if (D != 128 && sharded) return fail(-11, "query shards need head_dim 128");
       DenseArgs a = {};
       a.q = (const bf16*)q; a.dout = (const bf16*)(has_swa ? dout_swa : dout_slc); a.dq = (bf16*)dq; a.accumulate = acc;
@@ -712,13 +729,8 @@ static int sel_swa_bwd_impl(const void* q, const void* k, const void* v, const v
       acc = 1;
     }
     dq_acc_for_reduce = acc;
-    if (has_slc && !dq_from_kv) {   // (else the reduction behind the key-major kernel adds the selected branch's dQ)
-      SelArgs a = {};
-      a.q = (const bf16*)q; a.k = (const bf16*)k; a.v = (const bf16*)v; a.idx = idx; a.idx64 = idx64; a.counts = counts;
-      a.lse = const_cast<float*>(lse_slc); a.dout = (const bf16*)dout_slc; a.delta = delta_slc;
-      a.gate = (const bf16*)gate_slc; a.dq = (bf16*)dq; a.accumulate = acc;
-      a.B = B; a.T = T; a.Tq = Tq; a.q0 = q0; a.Hq = Hq; a.Hkv = Hkv; a.S = S; a.BS = BS; a.scale = scale;
-      rc = launch_sel_dq(a, D, s);
+    if (own_dq && !sel_first) {
+      rc = selected();
       if (rc) return rc;
     }
   }

@@ -1,0 +1,46 @@
+"""NSAAttention as a whole: precision of its gradients against fp64."""
+import pytest
+import torch
+
+from parity_util import DEV
+
+pytestmark = pytest.mark.gpu
+
+
+def _attend64(q, k, v, mask):
+    """fp64 attention of one sequence, q [T,H,D], k, v [S,Hk,D], mask [T,S]; rows that see nothing give 0."""
+    g = q.shape[1] // k.shape[1]
+    s = torch.einsum("thd,shd->hts", q, k.repeat_interleave(g, 1)) * q.shape[2] ** -0.5
+    live = mask.any(-1, keepdim=True)
+    p = torch.softmax(torch.where(live, s.masked_fill(~mask, float("-inf")), torch.zeros_like(s)), -1) * live
+    return torch.einsum("hts,shd->thd", p, v.repeat_interleave(g, 1))
+
+
+def test_dq_is_rounded_once_where_the_selected_branch_is_small():
+    """Constant gates 1/16 (selected), 1, 1: dq is the window's and the compressed branch's but for a sixteenth, so its error is that of
+    one rounding to bf16 (1.66e-3 of its norm: 2^-8 / sqrt(12) averaged over a binade) and of dS in bf16, 1.85e-3 alone (the window by
+    itself, 2.48e-3 with the rounding).  Another rounding at full size makes it 3.0e-3.  (head_dim 64, where the selected branch's dQ is a
+    kernel of its own.)"""
+    import nsa_b200
+    T, H, D = 1024, 16, 64
+    gen = torch.Generator(device=DEV).manual_seed(D)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device=DEV).bfloat16()
+    mod = nsa_b200.NSAAttention(D, True, device=DEV, dtype=torch.bfloat16)
+    with torch.no_grad():
+        for p in mod.compressor.parameters():
+            p.normal_(0.0, 0.02, generator=gen)
+        mod.gating.weight.zero_()
+        mod.gating.bias.copy_(torch.tensor([1 / 16, 1.0, 1.0]))
+    q, k, v, do = rnd(T, H, D).requires_grad_(True), rnd(T, 1, D), rnd(T, 1, D), rnd(T, H, D)
+    cu = torch.tensor([0, T], dtype=torch.int32, device=DEV)
+    dq, = torch.autograd.grad(mod(q, k, v, cu, T), q, do)
+    ck, cv, _ = mod.compressor(k, v, cu, None)
+    x = [a.detach().double() for a in (q, k, v, ck[0], cv[0])]
+    x[0].requires_grad_(True)
+    t, j = torch.arange(T, device=DEV)[:, None], torch.arange(T, device=DEV)[None]
+    seen = t >= 16 * torch.arange(ck.shape[1], device=DEV)[None] + 32
+    # 16 of 16 blocks are selected: that branch is causal attention over everything
+    o = _attend64(x[0], x[1], x[2], j <= t) / 16 + _attend64(x[0], x[1], x[2], (j <= t) & (j > t - 512)) + _attend64(x[0], x[3], x[4], seen)
+    want, = torch.autograd.grad(o, x[0], do.double())
+    err = float((dq.double() - want).norm() / want.norm())
+    assert err < 2.7e-3, "relative error %.2e" % err
