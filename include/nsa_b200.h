@@ -261,7 +261,8 @@ int nsa_cmp_attn_bwd_fused(const void* q, const void* ck, const void* cv, const 
  *   info [3]         = compressed rows in all, longest compressed sequence, positions to compute.
  * -17 if a sequence became shorter.  nsa_cache_build copies the table to table_dev, moves the rows of ck_old, cv_old
  * (NULL if there are none) to their new offsets in ck, cv [info[0],H,D] and computes the remaining positions from
- * k, v [total_in,H,D] with the Conv1d weights conv_k, conv_v [D,D,block].  w_ws: 2*block*D*D bf16 of scratch. */
+ * k, v [total_in,H,D] with the Conv1d weights conv_k, conv_v [D,D,block], each summed in the order of nsa_compress_fwd_kv
+ * without split: the values do not depend on how the cache came to be.  w_ws: 2*block*D*D bf16 of scratch. */
 int nsa_cache_plan(const int32_t* cu_new, const int32_t* cu_old, const int32_t* cuc_old, int nseq, int block, int stride,
                    int32_t* table, int32_t* info);
 int nsa_cache_build(const void* k, const void* v, const void* conv_k, const void* conv_v, const void* bias_k,

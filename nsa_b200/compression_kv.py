@@ -20,7 +20,7 @@ def calc_compressed_len(x, stride, size):
 
 class _CompressPair(torch.autograd.Function):
     """(ck, cv) = compress(k; w_k, b_k), compress(v; w_v, b_v).  k, v [tok,H,D]; weights [l*D, D]; biases [D] or None.
-    ``split``: see nsa_compress_fwd_kv; False where a block selection follows."""
+    ``split``: see nsa_compress_fwd_kv; the package leaves it off, a block selection may follow."""
 
     @staticmethod
     def forward(ctx, k, v, w_k, w_v, b_k, b_v, cu_in, cu_out, block, stride, split, table=None):
@@ -95,7 +95,7 @@ def compress_kv(k, v, w_k, w_v, cu_seq_len, block_stride, block_size):
     for i in range(len(cu_in) - 1):
         cu_out.append(cu_out[-1] + max(calc_compressed_len(cu_in[i + 1] - cu_in[i], block_stride, block_size), 0))
     table = _lib.device_table(cu_in + cu_out, k.device)
-    ck, cv = _CompressPair.apply(k, v, w_k, w_v, None, None, cu_in, cu_out, block_size, block_stride, True, table)
+    ck, cv = _CompressPair.apply(k, v, w_k, w_v, None, None, cu_in, cu_out, block_size, block_stride, False, table)
     return ck, cv, table[len(cu_in):]
 
 

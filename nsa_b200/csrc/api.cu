@@ -190,7 +190,7 @@ int nsa_cache_build(const void* k, const void* v, const void* conv_k, const void
   CompressFwdArgs a = {};
   a.x[0] = (const bf16*)k; a.w[0] = wk; a.bias[0] = (const bf16*)bias_k; a.y[0] = (bf16*)ck;
   a.x[1] = (const bf16*)v; a.w[1] = wv; a.bias[1] = (const bf16*)bias_v; a.y[1] = (bf16*)cv;
-  a.ntensor = 2; a.cu_in = cu; a.cu_out = cc; a.cu_row = row; a.first = first; a.rows = nnew; a.split = 1;
+  a.ntensor = 2; a.cu_in = cu; a.cu_out = cc; a.cu_row = row; a.first = first; a.rows = nnew; a.split = 0;
   a.nseq = n; a.total_in = total_in; a.H = H; a.D = D; a.l = block; a.d = stride;
   return launch_compress_fwd_tc(a, s);
 }

@@ -100,7 +100,7 @@ def compress_cache(module, k, v, cu_seqlens_k):
         comp = module.compressor   # differentiable on request: the same values through the autograd functions
         w_k, w_v = _ConvLayout.apply(comp.compressor_k.weight, comp.compressor_v.weight)
         cache.ck, cache.cv = _CompressPair.apply(k, v, w_k, w_v, comp.compressor_k.bias, comp.compressor_v.bias, cache.cu,
-                                                 cache.cu_c, module.compression_block, module.compression_stride, True)
+                                                 cache.cu_c, module.compression_block, module.compression_stride, False)
     return cache
 
 

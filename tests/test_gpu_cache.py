@@ -1,0 +1,58 @@
+"""The compressed cache of a generation loop (compress_cache, extend_compress_cache): its values depend on the sequence alone."""
+import pytest
+import torch
+
+from parity_util import DEV
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def nsa():
+    import nsa_b200
+    yield nsa_b200
+    nsa_b200._lib.device_status()
+
+
+def _cum(lens):
+    return [sum(lens[:i]) for i in range(len(lens) + 1)]
+
+
+def _module(nsa, gen, D=128):
+    mod = nsa.NSAAttention(D, True, device=DEV, dtype=torch.bfloat16).requires_grad_(False)
+    for p in mod.parameters():
+        p.normal_(0.0, 0.02, generator=gen)
+    return mod
+
+
+@pytest.mark.parametrize("H", [1, 4])
+@pytest.mark.parametrize("seed", [1, 2, 3])
+def test_cache_bits_depend_on_the_sequence_alone(nsa, seed, H):
+    """Built whole, extended step by step, each sequence by itself, with gradients and by the module's own compression: the same bits (the
+    block selection depends on them)."""
+    from nsa_b200.decode import compress_cache, extend_compress_cache
+    gen = torch.Generator(device=DEV).manual_seed(seed)
+    mod = _module(nsa, gen)
+    lens = [2100, 4096, 33, 700, 31, 9000]
+    k, v = (torch.randn(sum(lens), H, 128, generator=gen, device=DEV).bfloat16() for _ in range(2))
+    cu = _cum(lens)
+    whole = compress_cache(mod, k, v, cu)
+    grown = None
+    for cut in (1500, 40, 17, 16, 1, 0):
+        part = [max(n - cut, 20) if n > 40 else n for n in lens]
+        keep = torch.cat([torch.arange(n, device=DEV) < p for n, p in zip(lens, part)])
+        args = (k[keep], v[keep], _cum(part))
+        grown = compress_cache(mod, *args) if grown is None else extend_compress_cache(mod, grown, *args)
+    assert torch.equal(grown.ck, whole.ck) and torch.equal(grown.cv, whole.cv) and grown.cu_c == whole.cu_c
+    mod.requires_grad_(True)
+    with_grad = compress_cache(mod, k, v, cu)
+    mod.requires_grad_(False)
+    assert with_grad.ck.requires_grad and torch.equal(with_grad.ck, whole.ck) and torch.equal(with_grad.cv, whole.cv)
+    for i, n in enumerate(lens):
+        if n < 32:
+            continue
+        ks, vs, rows = k[cu[i]:cu[i + 1]], v[cu[i]:cu[i + 1]], slice(whole.cu_c[i], whole.cu_c[i + 1])
+        alone = compress_cache(mod, ks, vs, [0, n])
+        ck, cv, _ = mod.compressor(ks, vs, torch.tensor([0, n], dtype=torch.int32), None)
+        for got_k, got_v in ((alone.ck, alone.cv), (ck[0], cv[0])):
+            assert torch.equal(got_k, whole.ck[rows]) and torch.equal(got_v, whole.cv[rows])
