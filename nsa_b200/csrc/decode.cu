@@ -9,9 +9,13 @@
 // The step is HBM-bound: a sequence contributes its compressed cache (1/16 of its K/V), 16 selected blocks and the
 // window, each read once.  One CTA works on one (sequence, kv head): the 16 query heads of the group are the M = 16
 // rows of mma.sync.m16n8k16.  Where there are fewer items than SMs, a cluster of 2, 4 or 8 CTAs shares one: the tile pairs of
-// every phase are dealt out to its CTAs, which exchange the soft-max statistics and the scores through each other's shared
+// every phase behind the statistics are dealt out to its CTAs, which exchange the scores through each other's shared
 // memory and then select the blocks each for itself (one CTA alone draws at most 1/148 of the bandwidth: 4 items of 4096 keys
-// took 25 us).  Producer warps stream [64 rows x 128] tiles by TMA
+// took 25 us).  The statistics (pass 1) are the same six chains everywhere, added in the same order: every CTA of a cluster
+// makes them for itself, and a chain's place in the sum does not follow from the warp that had it.  In another order near
+// ties of two blocks' scores come out otherwise, and a sequence's blocks would depend on how many others it is decoded with:
+// with pass 1 dealt out like the rest up to one in 16 items chose others (1 x 32768 keys 28.7 us so, 34.8 now; 4 x 16384
+// 30.7 and 32.8; 1 x 9000, where an exchange is saved, 26.6 and 25.5).  Producer warps stream [64 rows x 128] tiles by TMA
 // through a ring (192 KB in flight per SM); each consumer warp owns two slots, so every slot is filled and drained by the same
 // pair of warps in order.  The tile stream of an item:
 //   1. ck tiles:           raw scores -> per-row maxima and sums of the unscaled soft-max over ALL compressed keys and
@@ -25,7 +29,7 @@
 // time, from a scratch that the CTA's next item uses again (it stays in L2) while the ring fills with that item's tiles; with
 // clusters each CTA its share of the rows, a row and branch per warp.  Measured, 128 sequences of 4096 to 32768 keys: a second
 // kernel that merges (77 MB of partials written and read) 179 us, merged here 170; one
-// sequence of 4096 keys 18.9 us with the second kernel and 18.4 without.  Merging through shared memory, warp after warp, cost seven
+// sequence of 4096 keys 18.9 us with the second kernel and 17.5 without.  Merging through shared memory, warp after warp, cost seven
 // named barriers and six serialised rounds per branch.  No atomics; every wait is bounded.
 #include <algorithm>
 #include <array>
@@ -50,12 +54,12 @@ constexpr int kMaxSel = 32;
 constexpr int kPartFloats = 16 * D + 32;        // one warp's partial of one branch: O[16][D], m[16], l[16]
 constexpr int kMaxCluster = 8;
 
-struct Plan {   // tile pairs of one item's phases; CTA `rank` of a cluster takes the pairs rank, rank + cl, ... of each
+struct Plan {   // tile pairs of one item's phases; CTA `rank` of a cluster takes all of pass 1, of the others rank, rank + cl, ...
   int L, Tc, nvis, row_k, row_c;
   int n1p;     // pairs of ck tiles of pass 1
   int n2p;     // (ck, cv) pairs of pass 2: covers all of Tc
   int nw;      // window pairs
-  int cs;      // CTAs that share passes 1 and 2
+  int cs;      // CTAs that share pass 2
   int w0;      // first window key
 };
 
@@ -71,9 +75,8 @@ __device__ __forceinline__ Plan make_plan(const DecodeArgs& a, int seq, int cl) 
   const int nck = (p.Tc + 63) / 64;
   p.n1p = (nck + 1) / 2;
   p.n2p = nck;
-  // An exchange costs about as much as one pair (3500 cycles): with no more than a pair for each warp nothing is shared in the
-  // two passes, every CTA makes its own statistics and scores.  (Both passes or neither: that every CTA has sent its statistics
-  // also says that none still reads the scores of the item before.)
+  // An exchange costs about as much as one pair (3500 cycles): with no more than a pair for each warp the scores are not shared,
+  // every CTA makes its own.
   p.cs = p.n2p > kCons ? cl : 1;
   p.w0 = max(0, p.L - a.window);
   p.nw = a.window > 0 ? (p.L - p.w0 + 63) / 64 : 0;
@@ -366,8 +369,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   float* pooled = ps + kMaxTc + 64;                               // [kMaxPoolD]
   float* stat = pooled + kMaxPoolD;                               // [kCons][4][16] per-warp statistics
   float* fin = stat + kCons * 64;                                 // [4][16] merged: M_raw, 1/L_raw, M_att (log2), L_att
-  float* xstat = fin + 64;                                        // [cluster][4][16] the CTAs' statistics
-  float2* ml = reinterpret_cast<float2*>(xstat + kMaxCluster * 64);   // [3][kCons][16] (m, l) of the warps' partials, without clusters
+  float2* ml = reinterpret_cast<float2*>(fin + 64);               // [3][kCons][16] (m, l) of the warps' partials, without clusters
   float* gates = reinterpret_cast<float*>(ml + 3 * kCons * 16);       // [3][16], branch order as ml's
   int* sel = reinterpret_cast<int*>(gates + 48);                  // [kMaxSel] selected blocks of the item, [kMaxSel] = count
   volatile int* abort_flag = sel + kMaxSel + 2;
@@ -376,7 +378,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   auto full_bar = [&](uint32_t s) { return bar0 + 8u * s; };
   auto empty_bar = [&](uint32_t s) { return bar0 + 8u * (kSlots + s); };
   const uint32_t sel_ready = bar0 + 8u * (2 * kSlots);
-  const uint32_t xstat_bar = sel_ready + 8, ps_bar = sel_ready + 16;   // every CTA's statistics / scores have arrived here
+  const uint32_t ps_bar = sel_ready + 8;   // every CTA's scores have arrived here
   const int rank = cl > 1 ? (int)cluster_rank() : 0, group = blockIdx.x / cl, ngroup = gridDim.x / cl;
 
   if (threadIdx.x == 0) {
@@ -386,7 +388,6 @@ __global__ void __launch_bounds__(kThreads, 1)
       mbar_init(empty_bar(i), 1);
     }
     mbar_init(sel_ready, 1);
-    mbar_init(xstat_bar, cl);
     mbar_init(ps_bar, cl);
     fence_mbar_init();
   }
@@ -437,7 +438,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int seq = a.order ? a.order[sq] : sq;
       const Plan p = make_plan(a, seq, cl);
       bool ok = true;
-      for (int j = p.cs > 1 ? rank : 0; ok && j < p.n1p; j += p.cs) ok = issue2(&tmCK, p.row_c + j * 128, &tmCK, p.row_c + j * 128 + 64, h);
+      for (int j = 0; ok && j < p.n1p; ++j) ok = issue2(&tmCK, p.row_c + j * 128, &tmCK, p.row_c + j * 128 + 64, h);
       for (int j = p.cs > 1 ? rank : 0; ok && j < p.n2p; j += p.cs) ok = issue2(&tmCK, p.row_c + j * 64, &tmCV, p.row_c + j * 64, h);
       for (int j = rank; ok && j < p.nw; j += cl) ok = issue2(&tmK, p.row_k + p.w0 + j * 64, &tmV, p.row_k + p.w0 + j * 64, h);
       // the selected blocks are known once the consumers have pooled the scores
@@ -463,7 +464,6 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint32_t use = 0;                         // pairs of this warp so far
   const uint32_t sk = 2 * warp, sv = sk + 1;
   auto first_pair = [&]() { return (int)((warp + kCons - np0 % kCons) % kCons); };
-  uint32_t nx = 0;                          // items with an exchange so far
   bool ok = true;
   for (int r = 0; r * ngroup < nitem; ++r) {
     const int item = snake_item(r, group, ngroup);
@@ -479,10 +479,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     // ---- pass 1: statistics over all compressed keys ---------------------------------------------------
     float mr[2] = {-INFINITY, -INFINITY}, lr[2] = {0.f, 0.f};   // raw scores, all keys (natural-log domain kept in log2)
     float ma[2] = {-INFINITY, -INFINITY}, la[2] = {0.f, 0.f};   // scaled scores, visible keys
+    const int chain = first_pair();   // this warp's chain: the pairs chain, chain + 6, ...
     {
-      const int n = share(p.n1p, p.cs);
-      for (int i = first_pair(); i < n; i += kCons, ++use) {
-        const int u = deal(i, p.cs);
+      for (int u = chain; u < p.n1p; u += kCons, ++use) {
 #pragma unroll 1
         for (int e = 0; e < 2; ++e) {
           const uint32_t s = sk + e;
@@ -524,14 +523,15 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
         }
       }
-      np0 += n;
+      np0 += p.n1p;
     }
-    // merge the per-warp statistics (each value lives in the four lanes of a quad: sum the partial sums)
+    // merge the statistics of the chains, in their order whichever warps had them, so that an item's scores do not depend on
+    // the items before it (each value lives in the four lanes of a quad: sum the partial sums)
 #pragma unroll
     for (int rr = 0; rr < 2; ++rr) {
       const float l_r = quad_sum(lr[rr]), l_a = quad_sum(la[rr]);
       if (tq == 0) {
-        float* st = stat + warp * 64;
+        float* st = stat + chain * 64;
         st[0 * 16 + g + 8 * rr] = mr[rr];
         st[1 * 16 + g + 8 * rr] = l_r;
         st[2 * 16 + g + 8 * rr] = ma[rr];
@@ -550,34 +550,6 @@ __global__ void __launch_bounds__(kThreads, 1)
         const float m1 = stat[w * 64 + ct], m2 = stat[w * 64 + 32 + ct];
         if (m1 > -INFINITY) Lr += stat[w * 64 + 16 + ct] * ex2(m1 - Mr);
         if (m2 > -INFINITY) La += stat[w * 64 + 48 + ct] * ex2(m2 - Ma);
-      }
-      float* own = xstat + rank * 64;
-      own[ct] = Mr;
-      own[16 + ct] = Lr;
-      own[32 + ct] = Ma;
-      own[48 + ct] = La;
-    }
-    if (p.cs > 1 && warp == 0) {
-      __syncwarp();
-      float* own = xstat + rank * 64 + 2 * lane;
-      const float2 v = *reinterpret_cast<const float2*>(own);
-      for (int c = 0; c < cl; ++c)
-        if (c != rank) st_cluster(map_cta(smem_u32(own), c), v);
-      __syncwarp();
-      if (lane < cl) arrive_cluster(map_cta(xstat_bar, lane));
-      ok = ok && wait_cluster(xstat_bar, nx & 1, 320, abort_flag);
-    }
-    if (ct < 16) {   // (written by this thread, or by the CTAs of the cluster)
-      float Mr = -INFINITY, Ma = -INFINITY, Lr = 0.f, La = 0.f;
-      const int c0 = p.cs > 1 ? 0 : rank, c1 = p.cs > 1 ? cl : rank + 1;
-      for (int c = c0; c < c1; ++c) {
-        Mr = fmaxf(Mr, xstat[c * 64 + ct]);
-        Ma = fmaxf(Ma, xstat[c * 64 + 32 + ct]);
-      }
-      for (int c = c0; c < c1; ++c) {
-        const float m1 = xstat[c * 64 + ct], m2 = xstat[c * 64 + 32 + ct];
-        if (m1 > -INFINITY) Lr += xstat[c * 64 + 16 + ct] * ex2(m1 - Mr);
-        if (m2 > -INFINITY) La += xstat[c * 64 + 48 + ct] * ex2(m2 - Ma);
       }
       fin[ct] = Mr;
       fin[16 + ct] = Lr > 0.f ? 1.f / Lr : 0.f;
@@ -660,8 +632,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     named_bar_sync(1, cthreads);            // ps complete
     if (p.cs > 1) {   // in every CTA
       if (ct < cl) arrive_cluster(map_cta(ps_bar, ct));
-      ok = ok && wait_cluster(ps_bar, nx & 1, 321, abort_flag);
-      ++nx;
+      ok = ok && wait_cluster(ps_bar, 0, 321, abort_flag);   // (a cluster has one item)
     }
     const int n_pool = min(kMaxPoolD, pool_len(p.Tc, pool_k, pool_s));
     for (int blk = ct; blk < n_pool; blk += cthreads) {
@@ -867,8 +838,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 }
 
 constexpr int decode_smem() {
-  return kSlots * (int)TILE + (kMaxTc + 64 + kMaxPoolD + kCons * 64 + 64 + kMaxCluster * 64 + 3 * kCons * 32 + 48) * 4 + (kMaxSel + 4) * 4 +
-         (2 * kSlots + 3) * 8 + 16 + 1024;
+  return kSlots * (int)TILE + (kMaxTc + 64 + kMaxPoolD + kCons * 64 + 64 + 3 * kCons * 32 + 48) * 4 + (kMaxSel + 4) * 4 +
+         (2 * kSlots + 2) * 8 + 16 + 1024;
 }
 
 // A launch of `ncta` CTAs in clusters of `cl`.
@@ -899,8 +870,8 @@ int ask_resident(int cl) {
 }
 // How `nitem` items are spread: up to the number of SMs as many CTAs per item as keep every item in the first wave, with more a
 // CTA per SM that takes one after another.  (Two CTAs of three warps per SM, so that one streams tiles while the other chooses
-// its blocks, took 155 us for 128 sequences of 4096 to 32768 keys; but they add up the soft-max of the scores in another
-// order, and blocks whose scores tie to within a rounding, which one in 700 items has, were then chosen differently.)
+// its blocks, took 155 us for 128 sequences of 4096 to 32768 keys; but three chains add up the soft-max of the scores in another
+// order than six, and blocks whose scores tie to within a rounding, which one in 700 items has, were then chosen differently.)
 struct Spread {
   int cl, ncta;
 };

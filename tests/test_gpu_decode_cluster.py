@@ -8,12 +8,15 @@ from parity_util import DEV, close as _close
 pytestmark = pytest.mark.gpu
 
 
+@pytest.mark.parametrize("seed", range(6))
 @pytest.mark.parametrize("Hkv,parts", [(4, (1, 2, 5, 10)), (1, (3, 20, 40))])
-def test_decode_batches_agree(Hkv, parts):
+def test_decode_batches_agree(Hkv, parts, seed):
+    """The blocks are the same ones whatever the batch: the caches and the scores do not depend on it.  What a branch adds up in another
+    order differs by roundings."""
     import nsa_b200 as nsa
     from nsa_b200.decode import nsa_decode
-    torch.manual_seed(0)   # the module's weights (of other ones two nearly equal scores may change places: see the caches below)
-    gen = torch.Generator(device=DEV).manual_seed(Hkv)
+    torch.manual_seed(seed)   # the module's weights
+    gen = torch.Generator(device=DEV).manual_seed(100 * seed + Hkv)
     rnd = lambda *s: torch.randn(*s, generator=gen, device=DEV).bfloat16()
     lens = [40, 5000, 1, 33, 700, 64, 2047, 9000, 513, 1100] + [100 + 37 * i for i in range(150 // Hkv)]
     cu = [sum(lens[:i]) for i in range(len(lens) + 1)]
@@ -32,6 +35,6 @@ def test_decode_batches_agree(Hkv, parts):
         assert torch.equal(got_parts[4], idx[sl])
         for name, x, ref in (("o", got, o), ("cmp", got_parts[0], o_cmp), ("slc", got_parts[1], o_slc), ("swa", got_parts[2], o_swa)):
             _close("decode %s, %d at %d" % (name, n, at), x, ref[sl])
-        assert torch.allclose(got_parts[3].nan_to_num(neginf=-1e4), lse[:, sl].nan_to_num(neginf=-1e4), atol=5e-3)   # (the caches of the parts are rounded on their own)
+        assert torch.allclose(got_parts[3].nan_to_num(neginf=-1e4), lse[:, sl].nan_to_num(neginf=-1e4), atol=1e-4)
         at = min(at + n, len(lens) - 40)
     nsa._lib.device_status()
