@@ -164,8 +164,8 @@ int nsa_cache_build(const void* k, const void* v, const void* conv_k, const void
                     const void* bias_v, void* w_ws, const void* ck_old, const void* cv_old, void* ck, void* cv,
                     const int32_t* table, int32_t* table_dev, int nseq, long long total_in, int H, int D, int block, int stride,
                     void* stream) {
-  if (!k || !v || !conv_k || !conv_v || !w_ws || !ck || !cv || !table || !table_dev) return fail(-1, "nsa_cache_build: null pointer");
-  if (nseq <= 0 || H <= 0) return fail(-1, "nsa_cache_build: empty shape");
+  if (!table || !table_dev) return fail(-1, "nsa_cache_build: null pointer");
+  if (nseq < 0 || H <= 0) return fail(-1, "nsa_cache_build: empty shape");
   if (D != 64 && D != 128) return fail(-2, "nsa_cache_build: head_dim %d not supported (64 or 128)", D);
   if (block % stride) return fail(-4, "nsa_cache_build: block must be a multiple of stride");
   if (!aligned16(k) || !aligned16(v) || !aligned16(w_ws) || !aligned16(ck) || !aligned16(cv) || !aligned16(ck_old) || !aligned16(cv_old))
@@ -179,7 +179,10 @@ int nsa_cache_build(const void* k, const void* v, const void* conv_k, const void
   const int32_t* first = row + n + 1;
   const long long nold = table[2 * (n + 1) + n], nnew = table[3 * (n + 1) + n];
   if (table[n] > total_in) return fail(-10, "nsa_cache_build: the sequences end at token %d of %lld", table[n], total_in);
-  if (nold > 0 && (!ck_old || !cv_old)) return fail(-1, "nsa_cache_build: null pointer");
+  // (an empty tensor has no address: the caches before a sequence has reached its first block, and what no position is made from)
+  if ((nold > 0 && (!ck_old || !cv_old)) || (nold + nnew > 0 && (!ck || !cv)) ||
+      (nnew > 0 && (!k || !v || !conv_k || !conv_v || !w_ws)))
+    return fail(-1, "nsa_cache_build: null pointer");
   int rc = launch_upload_table(table, 6 * n + 4, table_dev, s);
   if (!rc) rc = launch_move_rows((const bf16*)ck_old, (const bf16*)cv_old, (bf16*)ck, (bf16*)cv, old, cc, n, nold, H * D, s);
   if (rc || nnew <= 0) return rc;

@@ -56,3 +56,26 @@ def test_cache_bits_depend_on_the_sequence_alone(nsa, seed, H):
         ck, cv, _ = mod.compressor(ks, vs, torch.tensor([0, n], dtype=torch.int32), None)
         for got_k, got_v in ((alone.ck, alone.cv), (ck[0], cv[0])):
             assert torch.equal(got_k, whole.ck[rows]) and torch.equal(got_v, whole.cv[rows])
+
+
+def test_cache_before_the_first_block(nsa):
+    """No sequence has reached 32 tokens yet: an empty cache, that grows like any other."""
+    from nsa_b200.decode import compress_cache, extend_compress_cache
+    gen = torch.Generator(device=DEV).manual_seed(1)
+    mod = _module(nsa, gen)
+    k, v = (torch.randn(200, 2, 128, generator=gen, device=DEV).bfloat16() for _ in range(2))
+    cache = compress_cache(mod, k[:0], v[:0], [0, 0, 0, 0])
+    assert cache.ck.shape == (0, 2, 128) and cache.cu_c == [0, 0, 0, 0]
+    for lens in ((20, 5, 31), (20, 20, 31), (20, 20, 32), (33, 48, 100)):
+        n = sum(lens)
+        ks, vs = torch.zeros(2, n, 2, 128, device=DEV, dtype=torch.bfloat16)
+        for i in range(3):   # sequence i is the first tokens of k, v from 10 i on
+            ks[_cum(lens)[i]:_cum(lens)[i + 1]], vs[_cum(lens)[i]:_cum(lens)[i + 1]] = (x[10 * i:10 * i + lens[i]] for x in (k, v))
+        cache = extend_compress_cache(mod, cache, ks, vs, _cum(lens))
+        want = compress_cache(mod, ks, vs, _cum(lens))
+        assert cache.cu == want.cu == _cum(lens) and cache.cu_c == want.cu_c
+        assert torch.equal(cache.ck, want.ck) and torch.equal(cache.cv, want.cv)
+        assert torch.equal(cache.order_dev, want.order_dev)
+    assert cache.cu_c == [0, 1, 3, 8]
+    none = compress_cache(mod, k, v, [0])
+    assert none.ck.shape == (0, 2, 128) and none.cu_c == [0]
