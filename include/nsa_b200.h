@@ -259,7 +259,7 @@ int nsa_cmp_attn_bwd_fused(const void* q, const void* ck, const void* cv, const 
  *                      offsets of the positions to compute (nseq+1), first of them per sequence (nseq), the sequences
  *                      longest first (nseq);
  *   info [3]         = compressed rows in all, longest compressed sequence, positions to compute.
- * -17 if a sequence became shorter.  nsa_cache_build copies the table to table_dev, moves the rows of ck_old, cv_old
+ * -17 if a sequence became shorter, -18 if the old cache holds more positions of one than it has.  nsa_cache_build copies the table to table_dev, moves the rows of ck_old, cv_old
  * (NULL if there are none) to their new offsets in ck, cv [info[0],H,D] and computes the remaining positions from
  * k, v [total_in,H,D] with the Conv1d weights conv_k, conv_v [D,D,block], each summed in the order of nsa_compress_fwd_kv
  * without split: the values do not depend on how the cache came to be.  w_ws: 2*block*D*D bf16 of scratch. */

@@ -157,6 +157,7 @@ int nsa_cache_plan(const int32_t* cu_new, const int32_t* cu_old, const int32_t* 
   if (!cu_new || !table || !info || (!cu_old != !cuc_old)) return fail(-1, "nsa_cache_plan: null pointer");
   if (nseq < 0 || block <= 0 || stride <= 0) return fail(-1, "nsa_cache_plan: empty or negative shape");
   const int rc = cache_plan(cu_new, cu_old, cuc_old, nseq, block, stride, table, info);
+  if (rc < 0) return fail(-18, "the old cache holds more positions of sequence %d than it has now: another block or stride", -rc - 1);
   return rc ? fail(-17, "sequence %d became shorter", rc - 1) : 0;
 }
 

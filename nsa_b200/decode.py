@@ -65,30 +65,47 @@ def _build(module, k, v, cu_seqlens_k, old):
     """The compressed cache of packed k, v; the positions that ``old`` (a CompressedCache or None) holds are copied."""
     k, v = _lib.require(k, "k"), _lib.require(v, "v")
     cu = _lengths(cu_seqlens_k)
-    n, (total, H, D), L = len(cu) - 1, k.shape, _lib.lib()
-    if old is not None and n != old.nseq:
-        raise ValueError("the number of sequences changed")
+    n, L = len(cu) - 1, _lib.lib()
     conv_k, conv_v = module.compressor.compressor_k, module.compressor.compressor_v
     block, stride = module.compression_block, module.compression_stride
+    wk, wv = _lib.require(conv_k.weight, "compressor_k.weight"), _lib.require(conv_v.weight, "compressor_v.weight")
+    bk, bv = _lib.require(conv_k.bias, "compressor_k.bias"), _lib.require(conv_v.bias, "compressor_v.bias")
+    old_table, ck_old, cv_old = None, None, None
+    if old is not None:
+        if n != old.nseq:
+            raise ValueError("the number of sequences changed")
+        old_table, ck_old, cv_old = old._table, _lib.require(old.ck, "cache.ck"), _lib.require(old.cv, "cache.cv")
+    for x, w, b, c in ((k, wk, bk, ck_old), (v, wv, bv, cv_old)):
+        D = x.shape[2]
+        if w.shape != (D, D, block) or (b is not None and b.shape != (D,)):
+            raise RuntimeError("head_dim %d does not fit compression weights %s" % (D, tuple(w.shape)))
+        if c is not None and (c.shape[1:] != x.shape[1:] or c.shape[0] < old_table[2 * n + 1]):
+            raise RuntimeError("a cache of %s does not fit %d positions of %s" % (tuple(c.shape), old_table[2 * n + 1], tuple(x.shape[1:])))
     table, info = (ctypes.c_int32 * (6 * n + 4))(), (ctypes.c_int32 * 3)()
-    rc = L.nsa_cache_plan(cu, old._table if old is not None else None,
-                          ctypes.byref(old._table, 4 * (n + 1)) if old is not None else None, n, block, stride, table, info)
+    rc = L.nsa_cache_plan(cu, old_table, ctypes.byref(old_table, 4 * (n + 1)) if old is not None else None, n, block, stride,
+                          table, info)
     if rc == -17:
         raise ValueError(L.nsa_last_error().decode())
     _lib.check(rc, "nsa_cache_plan")
     dev = k.device
-    ck = torch.empty(info[0], H, D, dtype=torch.bfloat16, device=dev)
-    cv = torch.empty(info[0], H, D, dtype=torch.bfloat16, device=dev)
+    ck, cv = (torch.empty(info[0], *x.shape[1:], dtype=torch.bfloat16, device=dev) for x in (k, v))
     # one allocation: the kernel's weight layout (scratch) and the device tables
+    D = k.shape[2]
     wbytes = 4 * block * D * D
     buf = torch.empty(wbytes + 4 * (6 * n + 4), dtype=torch.uint8, device=dev)
     table_dev = buf[wbytes:].view(torch.int32)
     P = _lib.ptr
-    wk, wv = _lib.require(conv_k.weight, "compressor_k.weight"), _lib.require(conv_v.weight, "compressor_v.weight")
-    bk, bv = _lib.require(conv_k.bias, "compressor_k.bias"), _lib.require(conv_v.bias, "compressor_v.bias")
-    _lib.check(L.nsa_cache_build(P(k), P(v), P(wk), P(wv), P(bk), P(bv), P(buf), P(old.ck) if old is not None else None,
-                                 P(old.cv) if old is not None else None, P(ck), P(cv), table, P(table_dev), n, total, H, D,
-                                 block, stride, _lib.stream()), "nsa_cache_build")
+
+    def run(x, y, wx, wy, bx, by, x_old, y_old, cx, cy):
+        _lib.check(L.nsa_cache_build(P(x), P(y), P(wx), P(wy), P(bx), P(by), P(buf), P(x_old), P(y_old), P(cx), P(cy), table,
+                                     P(table_dev), n, min(x.shape[0], y.shape[0]), x.shape[1], D, block, stride, _lib.stream()),
+                   "nsa_cache_build")
+
+    if k.shape[1] == v.shape[1]:
+        run(k, v, wk, wv, bk, bv, ck_old, cv_old, ck, cv)
+    else:   # the two have different head counts: each by itself
+        run(k, k, wk, wk, bk, bk, ck_old, ck_old, ck, torch.empty_like(ck))
+        run(v, v, wv, wv, bv, bv, cv_old, cv_old, cv, torch.empty_like(cv))
     return CompressedCache(ck, cv, table, table_dev, n, info[1])
 
 

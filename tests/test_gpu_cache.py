@@ -79,3 +79,38 @@ def test_cache_before_the_first_block(nsa):
     assert cache.cu_c == [0, 1, 3, 8]
     none = compress_cache(mod, k, v, [0])
     assert none.ck.shape == (0, 2, 128) and none.cu_c == [0]
+
+
+def test_a_cache_that_does_not_fit_is_refused(nsa):
+    """Other head counts, head_dims or geometries than the old cache's, weights of another head_dim: an error on the host."""
+    from nsa_b200.decode import compress_cache, extend_compress_cache
+    gen = torch.Generator(device=DEV).manual_seed(1)
+    mod = _module(nsa, gen)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device=DEV).bfloat16()
+    k2, k4, k64 = rnd(100, 2, 128), rnd(101, 4, 128), rnd(101, 2, 64)
+    cache = compress_cache(mod, k2, k2, [0, 100])
+    with pytest.raises(RuntimeError, match="does not fit"):
+        extend_compress_cache(mod, cache, k4, k4, [0, 101])
+    with pytest.raises(RuntimeError, match="does not fit"):
+        extend_compress_cache(mod, cache, k64, k64, [0, 101])
+    with pytest.raises(RuntimeError, match="does not fit"):
+        compress_cache(mod, k64, k64, [0, 101])
+    small = nsa.NSAAttention(128, True, compression_block=16, device=DEV, dtype=torch.bfloat16).requires_grad_(False)
+    cache16 = compress_cache(small, k2, k2, [0, 100])
+    with pytest.raises(RuntimeError, match="another block or stride"):
+        extend_compress_cache(mod, cache16, k2, k2, [0, 100])
+
+
+def test_keys_and_values_of_different_shapes(nsa):
+    """More rows of one than of the other, or other head counts: each is compressed as it would be by itself."""
+    from nsa_b200.decode import compress_cache, extend_compress_cache
+    gen = torch.Generator(device=DEV).manual_seed(2)
+    mod = _module(nsa, gen)
+    k, v = (torch.randn(500, h, 128, generator=gen, device=DEV).bfloat16() for h in (2, 4))
+    cu, cu1 = [0, 300, 450], [0, 299, 380]
+    keep = torch.cat([torch.arange(299), 300 + torch.arange(81)]).to(DEV)
+    cache = compress_cache(mod, k, v, cu)
+    grown = extend_compress_cache(mod, compress_cache(mod, k[keep], v[keep], cu1), k, v, cu)
+    kk, vv = compress_cache(mod, k[:450], k[:460], cu), compress_cache(mod, v, v[:450], cu)
+    for c in (cache, grown):
+        assert torch.equal(c.ck, kk.ck) and torch.equal(c.cv, vv.cv)
