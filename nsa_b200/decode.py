@@ -18,11 +18,27 @@ class CompressedCache:
 
     ck, cv [sum Tc,Hkv,D]; cu, cu_c: host lists [nseq+1] (cumulative lengths of k/v and of ck/cv); the device copies and
     the longest-first launch order are one table that is built with the cache, so that a decode step issues no
-    host-to-device copy."""
+    host-to-device copy.  Saving and loading keeps ck, cv, cu and cu_c and makes the table anew."""
 
-    def __init__(self, ck, cv, table, table_dev, nseq, max_tc):
+    def __init__(self, ck, cv, cu, cu_c):
+        cu, cu_c = [int(c) for c in cu], [int(c) for c in cu_c]
+        n = len(cu) - 1
+        lens = [cu[i + 1] - cu[i] for i in range(n)]
+        order = sorted(range(n), key=lambda i: -lens[i])
+        values = [*cu, *cu_c] + [0] * (3 * n + 2) + order   # (the parts in between are read while a cache is built)
+        self._set(ck, cv, (ctypes.c_int32 * len(values))(*values), torch.tensor(values, dtype=torch.int32, device=ck.device), n,
+                  max([cu_c[i + 1] - cu_c[i] for i in range(n)] + [0]))
+
+    def _set(self, ck, cv, table, table_dev, nseq, max_tc):
         self.ck, self.cv, self.nseq, self.max_tc = ck, cv, nseq, max_tc
         self._table, self.table_dev = table, table_dev   # layout: nsa_cache_plan in include/nsa_b200.h
+        return self
+
+    def __getstate__(self):
+        return dict(ck=self.ck, cv=self.cv, cu=self.cu, cu_c=self.cu_c)
+
+    def __setstate__(self, state):
+        self.__init__(state["ck"], state["cv"], state["cu"], state["cu_c"])
 
     @property
     def cu(self):
@@ -106,7 +122,7 @@ def _build(module, k, v, cu_seqlens_k, old):
     else:   # the two have different head counts: each by itself
         run(k, k, wk, wk, bk, bk, ck_old, ck_old, ck, torch.empty_like(ck))
         run(v, v, wv, wv, bv, bv, cv_old, cv_old, cv, torch.empty_like(cv))
-    return CompressedCache(ck, cv, table, table_dev, n, info[1])
+    return CompressedCache.__new__(CompressedCache)._set(ck, cv, table, table_dev, n, info[1])
 
 
 def compress_cache(module, k, v, cu_seqlens_k):

@@ -114,3 +114,17 @@ def test_keys_and_values_of_different_shapes(nsa):
     kk, vv = compress_cache(mod, k[:450], k[:460], cu), compress_cache(mod, v, v[:450], cu)
     for c in (cache, grown):
         assert torch.equal(c.ck, kk.ck) and torch.equal(c.cv, vv.cv)
+
+
+def test_decode_with_a_cache_made_from_its_parts(nsa):
+    from nsa_b200.decode import CompressedCache, compress_cache, extend_compress_cache, nsa_decode
+    gen = torch.Generator(device=DEV).manual_seed(3)
+    mod = _module(nsa, gen)
+    cu = [0, 40, 2040, 2100]
+    k, v = (torch.randn(cu[-1], 4, 128, generator=gen, device=DEV).bfloat16() for _ in range(2))
+    q = torch.randn(3, 64, 128, generator=gen, device=DEV).bfloat16()
+    cache = compress_cache(mod, k, v, cu)
+    same = CompressedCache(*cache)
+    assert torch.equal(same.order_dev, cache.order_dev) and torch.equal(same.cu_c_dev, cache.cu_c_dev)
+    assert torch.equal(nsa_decode(mod, q, k, v, cu, same), nsa_decode(mod, q, k, v, cu, cache))
+    assert torch.equal(extend_compress_cache(mod, same, k, v, cu).ck, cache.ck)
