@@ -127,11 +127,24 @@ def sel_swa_fwd_workspace_bytes(B, T, Tq, Hq, Hkv, D, S, BS):
     return 0
 
 
+def int32_array(values):
+    """Cumulative lengths (whole numbers of any kind, in ascending order) as a host array of int32."""
+    n = len(values)
+    try:
+        a = (ctypes.c_int32 * n)(*values)
+    except TypeError:   # (ctypes takes Python's own ints only)
+        values = [int(x) for x in values]
+        a = (ctypes.c_int32 * n)(*values)
+    if n and not -0x80000000 <= values[-1] <= 0x7fffffff:
+        raise RuntimeError("length %d does not fit 32 bits" % values[-1])
+    return a
+
+
 def device_table(values, device):
     """A host list of int32 as a device tensor, without a stream synchronisation."""
-    n = len(values)
-    t = torch.empty(n, dtype=torch.int32, device=device)
-    check(lib().nsa_upload_table((ctypes.c_int32 * n)(*values), n, t.data_ptr(), stream()), "nsa_upload_table")
+    a = int32_array(values)
+    t = torch.empty(len(a), dtype=torch.int32, device=device)
+    check(lib().nsa_upload_table(a, len(a), t.data_ptr(), stream()), "nsa_upload_table")
     return t
 
 

@@ -72,8 +72,7 @@ class CompressedCache:
 
 
 def _lengths(cu_seqlens_k):
-    cu = cu_seqlens_k.tolist() if torch.is_tensor(cu_seqlens_k) else cu_seqlens_k
-    return (ctypes.c_int32 * len(cu))(*cu)
+    return _lib.int32_array(cu_seqlens_k.tolist() if torch.is_tensor(cu_seqlens_k) else cu_seqlens_k)
 
 
 @torch.no_grad()

@@ -2,10 +2,11 @@
 import copy
 import io
 
+import numpy as np
 import pytest
 import torch
 
-from nsa_b200.decode import CompressedCache
+from nsa_b200.decode import CompressedCache, _lengths
 
 
 def _saved(c):
@@ -32,3 +33,15 @@ def test_a_cache_saved_with_its_tables_as_lists_loads():
     c.__setstate__(dict(ck=torch.zeros(1, 1, 8), cv=torch.zeros(1, 1, 8), cu=[0, 40], cu_c=[0, 1], cu_dev=None, cu_c_dev=None,
                         order_dev=None, max_tc=1))
     assert c.cu == [0, 40] and c.order_dev.tolist() == [0]
+
+
+@pytest.mark.parametrize("cu", [[0, 40, 100], (0, 40, 100), np.array([0, 40, 100]), [np.int64(0), np.int32(40), 100.0],
+                                torch.tensor([0, 40, 100]), torch.tensor([0.0, 40.0, 100.0]),
+                                [torch.tensor(0), torch.tensor(40), torch.tensor(100)]])
+def test_lengths_of_any_kind(cu):
+    assert list(_lengths(cu)) == [0, 40, 100]
+
+
+def test_lengths_beyond_32_bits_are_refused():
+    with pytest.raises(RuntimeError, match="32 bits"):
+        _lengths([0, 2 ** 32 + 40])
