@@ -104,15 +104,13 @@ def _build(module, k, v, cu_seqlens_k, old):
     _lib.check(rc, "nsa_cache_plan")
     dev = k.device
     ck, cv = (torch.empty(info[0], *x.shape[1:], dtype=torch.bfloat16, device=dev) for x in (k, v))
-    # one allocation: the kernel's weight layout (scratch) and the device tables
     D = k.shape[2]
-    wbytes = 4 * block * D * D
-    buf = torch.empty(wbytes + 4 * (6 * n + 4), dtype=torch.uint8, device=dev)
-    table_dev = buf[wbytes:].view(torch.int32)
+    weights = torch.empty(2 * block * D * D, dtype=torch.bfloat16, device=dev)   # scratch: the kernels' layout
+    table_dev = torch.empty(6 * n + 4, dtype=torch.int32, device=dev)            # kept with the cache
     P = _lib.ptr
 
     def run(x, y, wx, wy, bx, by, x_old, y_old, cx, cy):
-        _lib.check(L.nsa_cache_build(P(x), P(y), P(wx), P(wy), P(bx), P(by), P(buf), P(x_old), P(y_old), P(cx), P(cy), table,
+        _lib.check(L.nsa_cache_build(P(x), P(y), P(wx), P(wy), P(bx), P(by), P(weights), P(x_old), P(y_old), P(cx), P(cy), table,
                                      P(table_dev), n, min(x.shape[0], y.shape[0]), x.shape[1], D, block, stride, _lib.stream()),
                    "nsa_cache_build")
 

@@ -128,3 +128,11 @@ def test_decode_with_a_cache_made_from_its_parts(nsa):
     assert torch.equal(same.order_dev, cache.order_dev) and torch.equal(same.cu_c_dev, cache.cu_c_dev)
     assert torch.equal(nsa_decode(mod, q, k, v, cu, same), nsa_decode(mod, q, k, v, cu, cache))
     assert torch.equal(extend_compress_cache(mod, same, k, v, cu).ck, cache.ck)
+
+
+def test_a_cache_keeps_its_tables_alone(nsa):
+    from nsa_b200.decode import compress_cache, extend_compress_cache
+    mod = _module(nsa, torch.Generator(device=DEV).manual_seed(4))
+    k = torch.zeros(100, 1, 128, device=DEV, dtype=torch.bfloat16)
+    cache = extend_compress_cache(mod, compress_cache(mod, k, k, [0, 64]), k, k, [0, 100])
+    assert cache.table_dev.untyped_storage().nbytes() == 4 * (6 * 1 + 4)   # (not the 2 MB of weights in the kernels' layout)
