@@ -19,14 +19,18 @@ def calc_compressed_len(x, stride, size):
 
 
 class _CompressPair(torch.autograd.Function):
-    """(ck, cv) = compress(k; w_k, b_k), compress(v; w_v, b_v).  k, v [tok,H,D]; weights [l*D, D]; biases [D] or None.
+    """(ck, cv) = compress(k; w_k, b_k), compress(v; w_v, b_v).  k, v [tok,H,D]; weights [l*D, D]; biases [D] or None.  An output
+    that nothing uses gives no gradients (None, not zeros).
     ``split``: see nsa_compress_fwd_kv; the package leaves it off, a block selection may follow."""
 
     @staticmethod
     def forward(ctx, k, v, w_k, w_v, b_k, b_v, cu_in, cu_out, block, stride, split, table=None):
         k, v, w_k, w_v = (_lib.require(t, n) for t, n in ((k, "k"), (v, "v"), (w_k, "w_k"), (w_v, "w_v")))
         b_k, b_v = _lib.require(b_k, "bias"), _lib.require(b_v, "bias")
+        ctx.set_materialize_grads(False)
         tok, H, D = k.shape
+        if v.shape != k.shape:
+            raise ValueError("k %s and v %s differ in shape" % (tuple(k.shape), tuple(v.shape)))
         for w in (w_k, w_v):
             if w.shape != (block * D, D):
                 raise ValueError("weight must have shape [block*D, D] = %s, got %s" % ((block * D, D), tuple(w.shape)))
@@ -50,10 +54,14 @@ class _CompressPair(torch.autograd.Function):
         k, v, w_k, w_v, table = ctx.saved_tensors
         nseq, H, D, block, stride, max_in, total_out = ctx.meta
         cin, cout = table.data_ptr(), table.data_ptr() + 4 * (nseq + 1)
-        L, P, need = _lib.lib(), _lib.ptr, ctx.needs_input_grad
+        L, P = _lib.lib(), _lib.ptr
+        used = (dck is not None, dcv is not None)
+        if not any(used):
+            return (None,) * 12
+        need = [n and used[i % 2] for i, n in enumerate(ctx.needs_input_grad[:6])]
         ws_bytes = L.nsa_compress_bwd_kv_workspace_bytes(nseq, 0, total_out, 1, H, D, block, stride)
         if ws_bytes and total_out > 0:   # both tensors on the tensor cores (block = stride or 2 * stride)
-            dck, dcv = _lib.require(dck, "dck"), _lib.require(dcv, "dcv")
+            dck, dcv = _lib.require(dck if used[0] else dcv, "dck"), _lib.require(dcv if used[1] else dck, "dcv")   # (both are read)
             dk, dv = (torch.empty_like(x) if n else None for x, n in ((k, need[0]), (v, need[1])))
             dwk, dwv = (torch.empty_like(w) if n else None for w, n in ((w_k, need[2]), (w_v, need[3])))
             dbk, dbv = (torch.empty(D, dtype=torch.bfloat16, device=k.device) if n else None for n in need[4:6])
@@ -66,6 +74,9 @@ class _CompressPair(torch.autograd.Function):
         ws = torch.empty(ws_bytes, dtype=torch.uint8, device=k.device) if ws_bytes else None
         grads = []
         for i, (x, w, dy) in enumerate(((k, w_k, dck), (v, w_v, dcv))):
+            if not used[i]:
+                grads.append((None, None, None))
+                continue
             dy = _lib.require(dy, "dy")
             dx = torch.empty_like(x) if need[i] else None
             dw = torch.empty(block * D, D, dtype=torch.float32, device=x.device) if need[2 + i] else None
@@ -82,6 +93,14 @@ class _CompressPair(torch.autograd.Function):
         return dk, dv, dwk, dwv, dbk, dbv, None, None, None, None, None, None
 
 
+def _compress(k, v, w_k, w_v, b_k, b_v, cu_in, cu_out, block, stride, table=None):
+    """_CompressPair, or each tensor by itself where their shapes differ (heads, head_dim, tokens behind the last sequence)."""
+    args = (cu_in, cu_out, block, stride, False, table)
+    if k.shape == v.shape:
+        return _CompressPair.apply(k, v, w_k, w_v, b_k, b_v, *args)
+    return _CompressPair.apply(k, k, w_k, w_k, b_k, b_k, *args)[0], _CompressPair.apply(v, v, w_v, w_v, b_v, b_v, *args)[0]
+
+
 def _host_cu(cu_seq_len):
     if torch.is_tensor(cu_seq_len):
         return [int(c) for c in cu_seq_len.tolist()]   # one host sync, as nsa/compression_kv.py:184
@@ -95,7 +114,7 @@ def compress_kv(k, v, w_k, w_v, cu_seq_len, block_stride, block_size):
     for i in range(len(cu_in) - 1):
         cu_out.append(cu_out[-1] + max(calc_compressed_len(cu_in[i + 1] - cu_in[i], block_stride, block_size), 0))
     table = _lib.device_table(cu_in + cu_out, k.device)
-    ck, cv = _CompressPair.apply(k, v, w_k, w_v, None, None, cu_in, cu_out, block_size, block_stride, False, table)
+    ck, cv = _compress(k, v, w_k, w_v, None, None, cu_in, cu_out, block_size, block_stride, table)
     return ck, cv, table[len(cu_in):]
 
 
@@ -106,6 +125,7 @@ class _ConvLayout(torch.autograd.Function):
     def forward(ctx, w_k, w_v):
         w_k, w_v = _lib.require(w_k, "compressor_k.weight"), _lib.require(w_v, "compressor_v.weight")
         D, _, block = w_k.shape
+        ctx.set_materialize_grads(False)
         ctx.dims = (D, block)
         out_k, out_v = (torch.empty(block * D, D, dtype=torch.bfloat16, device=w_k.device) for _ in range(2))
         P = _lib.ptr
@@ -116,19 +136,25 @@ class _ConvLayout(torch.autograd.Function):
     @staticmethod
     def backward(ctx, *grads):
         D, block = ctx.dims
-        return tuple(g.view(block, D, D).permute(2, 1, 0) for g in grads)
+        return tuple(g.view(block, D, D).permute(2, 1, 0) if g is not None else None for g in grads)
 
 
 def compress_conv(k, v, compressor, B):
     """Module-path compression of k, v [B*T,H,D] with the Conv1d parameters of a KVCompressor: the contraction of
     nsa/compression_kv.py:301-307, outputs [B,Tc,H,D] with Tc = (T-block)//stride + 1."""
-    tok, H, D = k.shape
-    T, block, stride = tok // B, compressor.block_size, compressor.block_stride
-    Tc = (T - block) // stride + 1 if T >= block else 0
-    w_k, w_v = _ConvLayout.apply(compressor.compressor_k.weight, compressor.compressor_v.weight)
-    ck, cv = _CompressPair.apply(k, v, w_k, w_v, compressor.compressor_k.bias, compressor.compressor_v.bias,
-                                 range(0, T * B + 1, T), [Tc * i for i in range(B + 1)], block, stride, False)
-    return ck.view(B, Tc, H, D), cv.view(B, Tc, H, D)
+    block, stride = compressor.block_size, compressor.block_stride
+    w = _ConvLayout.apply(compressor.compressor_k.weight, compressor.compressor_v.weight)
+    b = compressor.compressor_k.bias, compressor.compressor_v.bias
+
+    def run(i, j):   # tensors i and j of (k, v)
+        x, y = (k, v)[i], (k, v)[j]
+        T = x.shape[0] // B
+        Tc = (T - block) // stride + 1 if T >= block else 0
+        out = _CompressPair.apply(x, y, w[i], w[j], b[i], b[j], [T * n for n in range(B + 1)], [Tc * n for n in range(B + 1)],
+                                  block, stride, False)
+        return [c.view(B, Tc, *c.shape[1:]) for c in out]
+
+    return tuple(run(0, 1)) if k.shape == v.shape else (run(0, 0)[0], run(1, 1)[0])
 
 
 class KVCompressorVarlen(nn.Module):

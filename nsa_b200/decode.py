@@ -10,7 +10,7 @@ import ctypes
 import torch
 
 from . import _lib
-from .compression_kv import _CompressPair, _ConvLayout
+from .compression_kv import _compress, _ConvLayout
 
 
 class CompressedCache:
@@ -129,8 +129,8 @@ def compress_cache(module, k, v, cu_seqlens_k):
     if torch.is_grad_enabled() and any(t.requires_grad for t in (k, v, *module.compressor.parameters())):
         comp = module.compressor   # differentiable on request: the same values through the autograd functions
         w_k, w_v = _ConvLayout.apply(comp.compressor_k.weight, comp.compressor_v.weight)
-        cache.ck, cache.cv = _CompressPair.apply(k, v, w_k, w_v, comp.compressor_k.bias, comp.compressor_v.bias, cache.cu,
-                                                 cache.cu_c, module.compression_block, module.compression_stride, False)
+        cache.ck, cache.cv = _compress(k, v, w_k, w_v, comp.compressor_k.bias, comp.compressor_v.bias, cache.cu, cache.cu_c,
+                                       module.compression_block, module.compression_stride)
     return cache
 
 

@@ -79,3 +79,42 @@ def test_extended_cache_equals_a_new_one(nsa, grow):
     with pytest.raises(ValueError):
         extend_compress_cache(mod, want, k, v, cum([n - 1 for n in new]))
     nsa._lib.device_status()
+
+
+@pytest.mark.parametrize("block,stride", [(32, 16), (64, 16)])   # the tcgen05 backward and the other one
+def test_an_unused_output_gives_no_gradient(nsa, block, stride):
+    """Gradients of the used output alone are those of both, the other tensor's are None."""
+    gen = torch.Generator(device=DEV).manual_seed(1)
+    comp = nsa.compression_kv.KVCompressorVarlen(stride, block, 128, DEV, torch.bfloat16)
+    k, v = (torch.randn(500, 2, 128, generator=gen, device=DEV).bfloat16().requires_grad_(True) for _ in range(2))
+    leaves = [k, v, comp.k_weight, comp.v_weight]
+    ck, cv, _ = comp(k, v, [0, 300, 500])
+    dck, dcv = (torch.randn(ck.shape, generator=gen, device=DEV).bfloat16() for _ in range(2))
+    both = torch.autograd.grad([ck, cv], leaves, [dck, dcv], retain_graph=True)
+    for out, dy, mine in ((ck, dck, (0, 2)), (cv, dcv, (1, 3))):
+        got = torch.autograd.grad(out, leaves, dy, retain_graph=True, allow_unused=True)
+        for i in range(4):
+            assert (torch.equal(got[i], both[i]) if i in mine else got[i] is None)
+
+
+def test_keys_and_values_of_different_shapes(nsa):
+    """Other head counts, head_dims and lengths of the two: each is compressed as it would be beside a tensor like itself."""
+    gen = torch.Generator(device=DEV).manual_seed(2)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device=DEV).bfloat16().requires_grad_(True)
+    compress_kv, cu = nsa.compression_kv.compress_kv, [0, 300, 480]
+    for v_shape in ((480, 4, 128), (500, 2, 128), (480, 2, 64)):
+        k, v = rnd(480, 2, 128), rnd(*v_shape)
+        w_k, w_v = (rnd(32 * x.shape[2], x.shape[2]) for x in (k, v))
+        ck, cv, cu_out = compress_kv(k, v, w_k, w_v, cu, 16, 32)
+        dck, dcv = rnd(*ck.shape).detach(), rnd(*cv.shape).detach()
+        got = torch.autograd.grad([ck, cv], [k, v, w_k, w_v], [dck, dcv])
+        for x, w, c, dc, i in ((k, w_k, ck, dck, 0), (v, w_v, cv, dcv, 1)):
+            alone, _, cu_alone = compress_kv(x, x.detach(), w, w.detach(), cu, 16, 32)
+            assert torch.equal(alone, c) and torch.equal(cu_alone, cu_out)
+            dx, dw = torch.autograd.grad(alone, [x, w], dc)
+            assert torch.equal(dx[:480], got[i][:480]) and torch.equal(dw, got[2 + i])
+    comp = nsa.compression_kv.KVCompressor(16, 32, 128, DEV, torch.bfloat16)
+    k, v = rnd(600, 2, 128), rnd(600, 4, 128)
+    cu = torch.tensor([0, 300, 600], dtype=torch.int32)
+    ck, cv, _ = comp(k, v, cu)
+    assert torch.equal(ck, comp(k, k, cu)[0]) and torch.equal(cv, comp(v, v, cu)[1])
