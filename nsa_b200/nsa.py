@@ -122,6 +122,11 @@ class _NSAModule(torch.autograd.Function):
             _lib.require(t, n) for t, n in zip((q, k, v, conv_k, conv_v, bias_k, bias_v, w_gate, b_gate), names))
         tok, Hq, D = q.shape
         Hkv = k.shape[1]
+        # (the kernels take the addresses: a module or keys of another head_dim would be read out of range)
+        for t, name, shape in ((k, "k", (tok, Hkv, D)), (conv_k, names[3], (D, D, block)), (conv_v, names[4], (D, D, block)),
+                               (bias_k, names[5], (D,)), (bias_v, names[6], (D,)), (w_gate, names[7], (3, D)), (b_gate, names[8], (3,))):
+            if t is not None and t.shape != shape:
+                raise RuntimeError("%s %s does not fit q %s" % (name, tuple(t.shape), tuple(q.shape)))
         L, P, S, chk = _lib.lib(), _lib.ptr, _lib.stream(), _lib.check
         # runs of equal-length sequences: (first token, sequences, tokens each, first compressed row, positions each)
         runs, t0, c0 = [], 0, 0

@@ -44,3 +44,15 @@ def test_dq_is_rounded_once_where_the_selected_branch_is_small():
     want, = torch.autograd.grad(o, x[0], do.double())
     err = float((dq.double() - want).norm() / want.norm())
     assert err < 2.7e-3, "relative error %.2e" % err
+
+
+def test_shapes_that_do_not_fit_are_refused():
+    """A module of another head_dim, keys of another head_dim: an error on the host."""
+    import nsa_b200
+    cu = torch.tensor([0, 1024], dtype=torch.int32, device=DEV)
+    x = {(h, d): torch.zeros(1024, h, d, device=DEV, dtype=torch.bfloat16) for h in (1, 16) for d in (64, 128)}
+    for D in (64, 128):
+        mod = nsa_b200.NSAAttention(D, True, device=DEV, dtype=torch.bfloat16)
+        for q, k in ((x[16, 192 - D], x[1, 192 - D]), (x[16, D], x[1, 192 - D]), (x[16, 192 - D], x[1, D])):
+            with pytest.raises(RuntimeError, match="does not fit"):
+                mod(q, k, k, cu, 1024)
