@@ -10,8 +10,8 @@ from .compression_kv import KVCompressor
 
 
 class _NSACore(torch.autograd.Function):
-    """Everything of NSAAttention.forward between the compression and the output for a query shard (context parallelism), as
-    one autograd node: compressed attention + block selection, selected + sliding-window attention and the gated three-way
+    """Everything of NSAAttention.forward between the compression and the output, for a query shard (context parallelism) or for a
+    module whose compressor has to be called, as one autograd node: compressed attention + block selection, selected + sliding-window attention and the gated three-way
     sum (nsa/nsa.py:102-133).  Keeping the three branches in one node lets the backward feed dO and the gates straight
     to the kernels (no g*dO tensors are materialised, dQ is accumulated inside the kernels instead of by autograd)."""
 
@@ -19,8 +19,9 @@ class _NSACore(torch.autograd.Function):
     def forward(ctx, q, k, v, ck, cv, w_gate, b_gate, cfg):
         """q: [B,Tq,Hq,D] = the queries at sequence positions q0 .. q0+Tq-1; k, v: [B,T,Hkv,D] and ck, cv:
         [B,Tc,Hkv,D] cover the whole sequence; w_gate [3,D], b_gate [3]: the gate projection (rows: selected,
-        window, compressed; nsa/nsa.py:59,117).  cfg[10] = q0."""
-        (stride, block, causal, scale, pool_k, pool_s, pool_p, n_sel, sel_block, window, q0) = cfg
+        window, compressed; nsa/nsa.py:59,117).  cfg[10] = q0; an optional cfg[11] = 1: causal selection scores."""
+        (stride, block, causal, scale, pool_k, pool_s, pool_p, n_sel, sel_block, window, q0) = cfg[:11]
+        score_mode = cfg[11] if len(cfg) > 11 else 0
         q, k, v, ck, cv = (_lib.require(t, n) for t, n in ((q, "q"), (k, "k"), (v, "v"), (ck, "ck"), (cv, "cv")))
         w_gate = _lib.require(w_gate, "gating.weight")
         b_gate = _lib.require(b_gate, "gating.bias") if b_gate is not None else None
@@ -38,9 +39,9 @@ class _NSACore(torch.autograd.Function):
         lse_swa = torch.empty_like(lse_slc) if window > 0 else None
         idx = torch.empty(B, Tq, Hkv, n_sel, dtype=torch.int32, device=dev)
         _lib.check(L.nsa_gate_fwd(P(q), P(w_gate), P(b_gate), P(g_slc), P(g_swa), P(g_cmp), B * Tq * Hq, D, S()), "nsa_gate_fwd")
-        _lib.check(L.nsa_cmp_attn_fwd_sharded(P(q), P(ck), P(cv), P(o_cmp), P(lse_cmp), P(idx), None, B, T, Tc, Hq, Hkv, D,
-                                              block, stride, 1 if causal else 0, scale, n_sel, pool_k, pool_s, pool_p, Tq, q0,
-                                              S()), "nsa_cmp_attn_fwd")
+        _lib.check(L.nsa_cmp_attn_fwd_gated(P(q), P(ck), P(cv), P(o_cmp), P(lse_cmp), P(idx), None, None, None, None, None, None,
+                                            B, T, Tc, Hq, Hkv, D, block, stride, 1 if causal else 0, scale, n_sel, pool_k,
+                                            pool_s, pool_p, score_mode, Tq, q0, S()), "nsa_cmp_attn_fwd")
         fws_bytes = _lib.sel_swa_fwd_workspace_bytes(B, T, Tq, Hq, Hkv, D, n_sel, sel_block)
         fws = torch.empty(fws_bytes, dtype=torch.uint8, device=dev) if fws_bytes else None
         _lib.check(L.nsa_sel_swa_fwd_ws(P(q), P(k), P(v), P(idx), 0, None, P(o_slc), P(lse_slc), P(o_swa),
@@ -56,7 +57,7 @@ class _NSACore(torch.autograd.Function):
     def backward(ctx, do):
         (q, k, v, ck, cv, g_slc, g_swa, g_cmp, o_slc, o_swa, o_cmp, lse_slc, lse_swa, lse_cmp, idx,
          w_gate) = ctx.saved_tensors
-        (stride, block, causal, scale, pool_k, pool_s, pool_p, n_sel, sel_block, window, q0) = ctx.cfg
+        (stride, block, causal, scale, pool_k, pool_s, pool_p, n_sel, sel_block, window, q0) = ctx.cfg[:11]
         do = _lib.require(do, "do")
         B, Tq, Hq, D = q.shape
         T, Hkv, Tc = k.shape[1], k.shape[2], ck.shape[1]
@@ -303,6 +304,9 @@ class _NSAModule(torch.autograd.Function):
         return dq, dk, dv, dwk, dwv, dbk, dbv, dw, db, None, None
 
 
+_compressor_forward = KVCompressor.forward
+
+
 class NSAAttention(nn.Module):
     """Drop-in for ``nsa.nsa.NSAAttention``.
 
@@ -391,5 +395,30 @@ class NSAAttention(nn.Module):
                self.pool_stride, self.pool_padding, self.selected_block_count, self.selection_block_size,
                self.sliding_window, bool(self.fuse_row_passes), {"reference": 0, "causal": 1}[self.score_mode])
         comp = self.compressor
+        if not self._inlines_compressor():
+            return self._through_compressor(q, k, v, cu_seqlens_k, lens, cfg)
         return _NSAModule.apply(q, k, v, comp.compressor_k.weight, comp.compressor_v.weight, comp.compressor_k.bias,
                                 comp.compressor_v.bias, self.gating.weight, self.gating.bias, lens, cfg)
+
+    def _inlines_compressor(self):
+        """Whether the compression can be part of the module's own node: not where someone would see that ``compressor`` is not
+        called (hooks, a substitute or a wrapper for it) or where its geometry was set apart from the module's."""
+        c = self.compressor
+        return (type(c) is KVCompressor and KVCompressor.forward is _compressor_forward and "forward" not in c.__dict__
+                and not (c._forward_hooks or c._forward_pre_hooks or c._backward_hooks or c._backward_pre_hooks)
+                and not torch.nn.modules.module._has_any_global_hook()
+                and c.block_size == self.compression_block and c.block_stride == self.compression_stride)
+
+    def _through_compressor(self, q, k, v, cu, lens, cfg):
+        """The forward with a call of ``self.compressor``, one sequence length at a time.  (``fuse_row_passes`` does not apply.)"""
+        if any(n != lens[0] for n in lens):
+            outs, t = [], 0
+            for n in lens:
+                one = torch.tensor([0, n], dtype=torch.int32, device=q.device)
+                outs.append(self._through_compressor(q[t:t + n], k[t:t + n], v[t:t + n], one, [n], cfg))
+                t += n
+            return torch.cat(outs, 0)
+        ck, cv, _ = self.compressor(k, v, cu, None)
+        q4, k4, v4 = (x.reshape(len(lens), -1, *x.shape[1:]) for x in (q, k, v))
+        o = _NSACore.apply(q4, k4, v4, ck, cv, self.gating.weight, self.gating.bias, cfg[:10] + (0, cfg[11]))
+        return o.reshape(-1, *o.shape[2:])

@@ -56,3 +56,55 @@ def test_shapes_that_do_not_fit_are_refused():
         for q, k in ((x[16, 192 - D], x[1, 192 - D]), (x[16, D], x[1, 192 - D]), (x[16, 192 - D], x[1, D])):
             with pytest.raises(RuntimeError, match="does not fit"):
                 mod(q, k, k, cu, 1024)
+
+
+class _Scaled(torch.nn.Module):
+    """A stand-in for the compressor that doubles the compressed values."""
+
+    def __init__(self, inner):
+        super().__init__()
+        self.inner = inner
+
+    def forward(self, k, v, cu, group=None):
+        ck, cv, cu = self.inner(k, v, cu, group)
+        return ck, 2 * cv, cu
+
+
+@pytest.mark.parametrize("mode", ["reference", "causal"])
+@pytest.mark.parametrize("lens", [(1100, 1100), (1100, 1037)])
+def test_the_compressor_is_called_where_that_shows(lens, mode):
+    """Forward hooks on it run (and give the same results as without), a substitute is used: twice the compressed values with half their
+    gate is the module itself."""
+    import nsa_b200
+    D, H, n = 128, 32, sum(lens)
+    gen = torch.Generator(device=DEV).manual_seed(n)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device=DEV).bfloat16()
+    mod = nsa_b200.NSAAttention(D, True, device=DEV, dtype=torch.bfloat16)
+    mod.score_mode = mode
+    with torch.no_grad():
+        for p in mod.parameters():
+            p.normal_(0.0, 0.05, generator=gen)
+    q, k, v, do = rnd(n, H, D).requires_grad_(True), rnd(n, 2, D).requires_grad_(True), rnd(n, 2, D).requires_grad_(True), rnd(n, H, D)
+    cu = torch.tensor([0, lens[0], n], dtype=torch.int32, device=DEV)
+
+    def run():
+        o = mod(q, k, v, cu)
+        return [o, *torch.autograd.grad(o, [q, k, v, *mod.parameters()], do)]
+
+    plain = run()
+    seen = []
+    handle = mod.compressor.register_forward_hook(lambda m, args, out: seen.append(tuple(out[0].shape)))
+    hooked = run()
+    handle.remove()
+    assert seen == ([(2, 67, 2, D)] if lens[0] == lens[1] else [(1, 67, 2, D), (1, 63, 2, D)])
+    names = ["o", "dq", "dk", "dv"] + [name for name, _ in mod.named_parameters()]
+    for name, a, b in zip(names, hooked, plain):
+        if name != "compressor.compressor_k.bias":   # zero but for roundings
+            # both round to bf16 on the way, the composed form up to twice as often: 2e-3 apart, the gates' bias (a sum that nearly cancels) 2e-2
+            assert float((a - b).float().norm() / b.float().norm()) < (3e-2 if name == "gating.bias" else 8e-3), name
+    mod.compressor = _Scaled(mod.compressor)
+    with torch.no_grad():
+        mod.gating.weight[2] /= 2
+        mod.gating.bias[2] /= 2
+    doubled = run()
+    assert float((doubled[0] - plain[0]).float().norm() / plain[0].float().norm()) < 8e-3
