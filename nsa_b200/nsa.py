@@ -115,7 +115,8 @@ class _NSAModule(torch.autograd.Function):
     one buffer, every other intermediate in one scratch buffer per piece, so a call makes a handful of allocations."""
 
     @staticmethod
-    def forward(ctx, q, k, v, conv_k, conv_v, bias_k, bias_v, w_gate, b_gate, lens, cfg):
+    def forward(ctx, q, k, v, conv_k, conv_v, bias_k, bias_v, w_gate, b_gate, lens, cfg, need):
+        # need: whether there will be a backward (ctx.needs_input_grad is true under no_grad as well)
         (stride, block, causal, scale, pool_k, pool_s, pool_p, n_sel, sel_block, window, fused, score_mode) = cfg
         names = ("q", "k", "v", "compressor_k.weight", "compressor_v.weight", "compressor_k.bias", "compressor_v.bias",
                  "gating.weight", "gating.bias")
@@ -144,12 +145,12 @@ class _NSAModule(torch.autograd.Function):
         rows, crow = tok * Hq, c0
         row_b, w_b = rows * D * 2, block * D * D * 2
         ix_bytes = [L.nsa_sel_index_bytes(B, T, T, Hkv, n_sel, sel_block) for _, B, T, _, _ in runs]
-        keep_ix = not fused and _lib.SEL_DQ_FROM_KV
+        use_ix = not fused and _lib.SEL_DQ_FROM_KV
         covers = _lib.sel_fwd_kv_covers(Hq, Hkv, D, n_sel, sel_block)
+        keep_ix = use_ix and covers   # (the query-major forward has no use for the reverse index: the backward builds it)
         # saved: ck, cv, weights in the kernels' layout (k, v), gates (3), o_slc, o_cmp, o_swa, lse (3), idx, length tables,
         # one reverse index per run
-        need = any(ctx.needs_input_grad)
-        keep_slc = need or not (covers and keep_ix)   # the key-major forward can add the gated sum without storing o_slc
+        keep_slc = need or not keep_ix   # the key-major forward can add the gated sum without storing o_slc
         off, total = _carve([crow * Hkv * D * 2] * 2 + [w_b] * 2 + [rows * 2] * 3 +
                             [row_b if keep_slc else 0, row_b, row_b if window > 0 else 0] +
                             [rows * 4] * 3 + [tok * Hkv * n_sel * 4, 8 * (len(lens) + 1)] + (ix_bytes if keep_ix else []))
@@ -189,7 +190,7 @@ class _NSAModule(torch.autograd.Function):
             if covers:
                 size = L.nsa_sel_swa_fwd_ix_workspace_bytes if keep_ix else L.nsa_sel_swa_fwd_workspace_bytes
                 ws_bytes = size(B, T, T, Hq, Hkv, D, n_sel, sel_block)
-            if keep_ix and (covers or need):
+            if keep_ix:
                 chk(L.nsa_sel_index(ib, 0, None, ix[i], ix_bytes[i], B, T, T, 0, Hkv, n_sel, sel_block, S), "nsa_sel_index")
             ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device) if ws_bytes else None
             chk(L.nsa_sel_swa_fwd_ix(P(q) + rb, P(k) + kv, P(v) + kv, ib, 0, None, ix[i], o_slc + rb if keep_slc else None, l_slc + 4 * r,
@@ -198,13 +199,13 @@ class _NSAModule(torch.autograd.Function):
                 "nsa_sel_swa_fwd")
         if need:
             ctx.save_for_backward(q, k, v, w_gate, saved)
-            ctx.meta = (cfg, runs, off, ix_bytes if keep_ix else None, len(lens), b_gate is not None, bias_k is not None)
+            ctx.meta = (cfg, runs, off, ix_bytes if use_ix else None, keep_ix, len(lens), b_gate is not None, bias_k is not None)
         return o
 
     @staticmethod
     def backward(ctx, do):
         q, k, v, w_gate, saved = ctx.saved_tensors
-        cfg, runs, off, ix_bytes, nseq, has_bg, has_bc = ctx.meta
+        cfg, runs, off, ix_bytes, keep_ix, nseq, has_bg, has_bc = ctx.meta
         (stride, block, causal, scale, pool_k, pool_s, pool_p, n_sel, sel_block, window, fused, score_mode) = cfg
         do = _lib.require(do, "do")
         tok, Hq, D = q.shape
@@ -212,7 +213,7 @@ class _NSAModule(torch.autograd.Function):
         L, P, S, chk = _lib.lib(), _lib.ptr, _lib.stream(), _lib.check
         base = saved.data_ptr()
         ck, cv, wk, wv, g_slc, g_swa, g_cmp, o_slc, o_cmp, o_swa, l_slc, l_cmp, l_swa, idx, cu = (base + x for x in off[:15])
-        ix = [base + x for x in off[15:]] if ix_bytes else [None] * len(runs)
+        ix = [base + x for x in off[15:]] if keep_ix else [None] * len(runs)
         if window <= 0:
             o_swa = l_swa = None
         crow = sum(B * Tc for _, B, _, _, Tc in runs)
@@ -232,7 +233,7 @@ class _NSAModule(torch.autograd.Function):
             scratch[o2[4]:o2[5]].zero_()   # the gate gradient of the branch that is not there
         at = lambda p, x: None if p is None else p + x
         win = window > 0
-        add_gate = bool(ix_bytes) and _lib.sel_fwd_kv_covers(Hq, Hkv, D, n_sel, sel_block)
+        add_gate = keep_ix
         if not fused:
             # one streaming pass over dO: delta = g * rowsum(o * dO) and the gate gradients of all three branches
             chk(L.nsa_rowdot3(o_slc, o_swa, o_cmp, P(do), g_slc, g_swa, g_cmp, d_slc, d_swa if win else None, d_cmp, dg_slc, dg_swa,
@@ -240,6 +241,10 @@ class _NSAModule(torch.autograd.Function):
         for i, (t0, B, T, c0, Tc) in enumerate(runs):
             r, kv, cb = t0 * Hq, t0 * Hkv * D * 2, c0 * Hkv * D * 2
             rb, ib, r4, r2 = r * D * 2, idx + t0 * Hkv * n_sel * 4, 4 * r, 2 * r
+            if ix_bytes and not keep_ix:
+                index = torch.empty(ix_bytes[i], dtype=torch.uint8, device=dev)
+                ix[i] = index.data_ptr()
+                chk(L.nsa_sel_index(ib, 0, None, ix[i], ix_bytes[i], B, T, T, 0, Hkv, n_sel, sel_block, S), "nsa_sel_index")
             if ix_bytes:
                 n1, n2 = L.nsa_attn_bwd_ix_workspace_bytes(B, T, Tc, Hq, Hkv, D, n_sel, sel_block, window), 0
             else:
@@ -301,7 +306,7 @@ class _NSAModule(torch.autograd.Function):
                     gw.copy_(gw32.view(block, D, D).permute(2, 1, 0))
                 if gb is not None:
                     gb.copy_(gb32)
-        return dq, dk, dv, dwk, dwv, dbk, dbv, dw, db, None, None
+        return dq, dk, dv, dwk, dwv, dbk, dbv, dw, db, None, None, None
 
 
 _compressor_forward = KVCompressor.forward
@@ -397,8 +402,10 @@ class NSAAttention(nn.Module):
         comp = self.compressor
         if not self._inlines_compressor():
             return self._through_compressor(q, k, v, cu_seqlens_k, lens, cfg)
-        return _NSAModule.apply(q, k, v, comp.compressor_k.weight, comp.compressor_v.weight, comp.compressor_k.bias,
-                                comp.compressor_v.bias, self.gating.weight, self.gating.bias, lens, cfg)
+        tensors = (q, k, v, comp.compressor_k.weight, comp.compressor_v.weight, comp.compressor_k.bias, comp.compressor_v.bias,
+                   self.gating.weight, self.gating.bias)
+        need = torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)
+        return _NSAModule.apply(*tensors, lens, cfg, need)
 
     def _inlines_compressor(self):
         """Whether the compression can be part of the module's own node: not where someone would see that ``compressor`` is not

@@ -44,8 +44,8 @@ def _forward(q, k, v, block_indices, block_counts, block_size, window_size, scal
         sl, n = slice(a, b), b - a
         ix = fws = None
         fws_bytes = 0
-        if covers or (need and _lib.SEL_DQ_FROM_KV):
-            # one reverse index for the forward and the backward
+        if covers:
+            # one reverse index for the forward and the backward (a forward that has no use for it leaves it to the backward)
             ix = torch.empty(L.nsa_sel_index_bytes(B, n, n, Hkv, S, block_size), dtype=torch.uint8, device=q.device)
             _lib.check(L.nsa_sel_index(P(idx[:, sl]), i64, opt(counts, sl), P(ix), ix.numel(), B, n, n, 0, Hkv, S, block_size,
                                        S_), "nsa_sel_index")
@@ -69,8 +69,12 @@ def _backward(q, k, v, lse_slc, lse_swa, idx, counts, indices, meta, do_slc, del
     P, i64 = _lib.ptr, 1 if idx.dtype == torch.int64 else 0
     opt = lambda t, sl: P(t[:, sl]) if t is not None else None
     for (a, b), ix in zip(seqs or [(0, T)], indices):
-        sl = slice(a, b)
-        shape = (B, b - a, b - a, Hq, Hkv, D, S, block_size)
+        sl, n = slice(a, b), b - a
+        shape = (B, n, n, Hq, Hkv, D, S, block_size)
+        if ix is None and _lib.SEL_DQ_FROM_KV:
+            ix = torch.empty(L.nsa_sel_index_bytes(B, n, n, Hkv, S, block_size), dtype=torch.uint8, device=q.device)
+            _lib.check(L.nsa_sel_index(P(idx[:, sl]), i64, opt(counts, sl), P(ix), ix.numel(), B, n, n, 0, Hkv, S, block_size,
+                                       _lib.stream()), "nsa_sel_index")
         ws_bytes = (L.nsa_sel_swa_bwd_ix_workspace_bytes(*shape, window_size) if ix is not None
                     else _lib.sel_swa_bwd_workspace_bytes(*shape))
         ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
@@ -124,13 +128,13 @@ class ParallelNSAFunction(torch.autograd.Function):
 
 class _GatedNSA(torch.autograd.Function):
     """parallel_nsa for gates of the queries' type: the gated sum is formed by the selected branch's last kernel, the gates'
-    gradients with the deltas in one pass (as torch operations they cost a further 13 % of the forward)."""
+    gradients with the deltas in one pass (as torch operations they cost a further 13 % of the forward).  ``need``: whether
+    there will be a backward (ctx.needs_input_grad is true under no_grad as well)."""
 
     @staticmethod
-    def forward(ctx, q, k, v, g_slc, g_swa, block_indices, block_counts, block_size, window_size, scale, offsets):
+    def forward(ctx, q, k, v, g_slc, g_swa, block_indices, block_counts, block_size, window_size, scale, offsets, need):
         q, k, v, g_slc, g_swa = (_lib.require(t, n) for t, n in (
             (q, "q"), (k, "k"), (v, "v"), (g_slc, "g_slc"), (g_swa if window_size > 0 else None, "g_swa")))
-        need = any(ctx.needs_input_grad)
         o, o_slc, lse_slc, o_swa, lse_swa, idx, counts, seqs, indices = _forward(
             q, k, v, block_indices, block_counts, block_size, window_size, float(scale), offsets, need, g_slc, g_swa)
         if need:
@@ -149,7 +153,7 @@ class _GatedNSA(torch.autograd.Function):
                                  P(dg_slc), P(dg_swa), None, lse_slc.numel(), q.shape[3], _lib.stream()), "nsa_rowdot3")
         dq, dk, dv = _backward(q, k, v, lse_slc, lse_swa, idx, counts, indices, ctx.meta, do, delta_slc, do if win else None,
                                delta_swa, g_slc, g_swa)
-        return dq, dk, dv, dg_slc, dg_swa, None, None, None, None, None, None
+        return dq, dk, dv, dg_slc, dg_swa, None, None, None, None, None, None, None
 
 
 def parallel_nsa(q: torch.Tensor,
@@ -185,8 +189,9 @@ def parallel_nsa(q: torch.Tensor,
         block_counts = None
     gates = (g_slc, g_swa) if window_size > 0 else (g_slc,)
     if all(torch.is_tensor(g) and g.is_cuda and g.dtype == q.dtype and g.shape == q.shape[:3] for g in gates):
+        need = torch.is_grad_enabled() and any(t.requires_grad for t in (q, k, v, *gates))
         o = _GatedNSA.apply(q, k, v, g_slc, g_swa if window_size > 0 else None, block_indices, block_counts, block_size,
-                            window_size, scale, cu_seqlens)
+                            window_size, scale, cu_seqlens, need)
         return o.transpose(1, 2) if head_first else o
     o_slc, o_swa = ParallelNSAFunction.apply(q, k, v, block_indices, block_counts, block_size, window_size, scale,
                                              cu_seqlens)

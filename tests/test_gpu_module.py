@@ -108,3 +108,39 @@ def test_the_compressor_is_called_where_that_shows(lens, mode):
         mod.gating.bias[2] /= 2
     doubled = run()
     assert float((doubled[0] - plain[0]).float().norm() / plain[0].float().norm()) < 8e-3
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_a_forward_without_gradients_does_no_work_for_a_backward(D):
+    """Under no_grad a module (and gates) with trainable parameters launch the same kernels, take the same memory and give the same bits
+    as frozen ones."""
+    import nsa_b200
+    T, H = 2048, 32
+    gen = torch.Generator(device=DEV).manual_seed(D)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device=DEV).bfloat16()
+    mod = nsa_b200.NSAAttention(D, True, device=DEV, dtype=torch.bfloat16)
+    q, k, v, cu = rnd(T, H, D), rnd(T, 2, D), rnd(T, 2, D), torch.tensor([0, T], dtype=torch.int32, device=DEV)
+    g = rnd(1, T, H).sigmoid()
+    idx = torch.arange(16, device=DEV).expand(1, T, 2, 16).contiguous()
+    calls = (lambda: mod(q, k, v, cu, T),
+             lambda: nsa_b200.selection_attention(q[None], k[None], v[None], g, g, idx, window_size=128))
+
+    def measure(call):
+        launches = nsa_b200._lib.lib().nsa_kernel_launch_count()
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        with torch.no_grad():
+            o = call()
+        return nsa_b200._lib.lib().nsa_kernel_launch_count() - launches, torch.cuda.max_memory_allocated() - before, o
+
+    for call in calls:
+        res = []
+        for train in (True, False):
+            mod.requires_grad_(train)
+            g.requires_grad_(train)
+            res.append(measure(call))
+        assert res[0][:2] == res[1][:2] and torch.equal(res[0][2], res[1][2])
+        mod.requires_grad_(True)
+        g.requires_grad_(True)
+        assert torch.equal(call().detach(), res[0][2])
