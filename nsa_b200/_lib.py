@@ -157,6 +157,11 @@ def stream():
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
+def aligned(t):
+    """The contiguous tensor t, copied where it does not start on a 16-byte boundary (a piece of a larger buffer)."""
+    return t if t is None or t.data_ptr() % 16 == 0 else t.clone()
+
+
 def require(t, name, dtype=torch.bfloat16):
     if t is None:
         return None

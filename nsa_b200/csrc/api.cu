@@ -834,6 +834,7 @@ int nsa_attn_bwd_ix(const void* q, const void* k, const void* v, const void* ck,
   if (Tc <= 0) return fail(-1, "nsa_attn_bwd_ix: no compressed position");
   if (ws_bytes < nsa_attn_bwd_ix_workspace_bytes(B, T, Tc, Hq, Hkv, D, S, BS, window))
     return fail(-6, "nsa_attn_bwd_ix: workspace too small");
+  if (!aligned16(w_gate)) return fail(-5, "nsa_attn_bwd_ix: w_gate must be 16-byte aligned");
   if (w_gate && (!dq_from_kv_covers(D, S, BS) || !dg_slc || !dg_swa || !dg_cmp))
     return fail(-1, "nsa_attn_bwd_ix: the gate projection's share needs its gradients, head_dim 128 and 64-key blocks");
   const CmpBwd c = {ck, cv, lse_cmp, delta_cmp, g_cmp, Tc, block, stride, causal,
@@ -901,6 +902,7 @@ int nsa_rowdot(const void* o, const void* dout, const void* gate, float* delta, 
 int nsa_gate_fwd(const void* q, const void* w, const void* bias, void* g_slc, void* g_swa, void* g_cmp, long long rows,
                  int D, void* stream) {
   if (!q || !w || !g_slc || !g_swa || !g_cmp) return fail(-1, "nsa_gate_fwd: null pointer");
+  if (!aligned16(q) || !aligned16(w)) return fail(-5, "nsa_gate_fwd: pointers must be 16-byte aligned");
   return launch_gate_fwd((const bf16*)q, (const bf16*)w, (const bf16*)bias, (bf16*)g_slc, (bf16*)g_swa, (bf16*)g_cmp, rows,
                          D, (cudaStream_t)stream);
 }
@@ -921,6 +923,7 @@ long long nsa_gate_bwd_workspace_bytes(long long rows, int D) { return gate_bwd_
 int nsa_gate_bwd(const void* q, const void* dg_slc, const void* dg_swa, const void* dg_cmp, const void* w, void* dq,
                  void* dw, void* dbias, void* workspace, long long workspace_bytes, long long rows, int D, void* stream) {
   if (!q || !dg_slc || !dg_swa || !dg_cmp || !w || !dw || !workspace) return fail(-1, "nsa_gate_bwd: null pointer");
+  if (!aligned16(q) || !aligned16(w) || !aligned16(dq)) return fail(-5, "nsa_gate_bwd: pointers must be 16-byte aligned");
   if (workspace_bytes < gate_bwd_workspace_bytes(rows, D)) return fail(-3, "nsa_gate_bwd: workspace too small");
   return launch_gate_bwd((const bf16*)q, (const bf16*)dg_slc, (const bf16*)dg_swa, (const bf16*)dg_cmp, (const bf16*)w,
                          (bf16*)dq, (bf16*)dw, (bf16*)dbias, (float*)workspace, rows, D, (cudaStream_t)stream);

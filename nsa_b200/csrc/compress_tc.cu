@@ -212,9 +212,8 @@ __global__ void __launch_bounds__(kThreads, 1)
           s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
         }
         if (a.bias[z]) {
-          const float2 b0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(a.bias[z] + col));
-          const float2 b1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(a.bias[z] + col + 2));
-          s.x += b0.x; s.y += b0.y; s.z += b1.x; s.w += b1.y;
+          const bf16* b = a.bias[z] + col;   // (of any alignment)
+          s.x += __bfloat162float(b[0]); s.y += __bfloat162float(b[1]); s.z += __bfloat162float(b[2]); s.w += __bfloat162float(b[3]);
         }
         uint2 o = make_uint2(pack_bf16(s.x, s.y), pack_bf16(s.z, s.w));
         *reinterpret_cast<uint2*>(a.y[z] + ((out0 + i0 + p2) * a.H + h2) * D + col) = o;

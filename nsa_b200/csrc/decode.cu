@@ -699,11 +699,15 @@ __global__ void __launch_bounds__(kThreads, 1)
         // tile of mma.sync, rounded to bf16 as the module's gate tensors are
         float c[4] = {0.f, 0.f, 0.f, 0.f};
         uint32_t wf[D / 16][2];
+        auto two = [](const bf16* x) {   // (a parameter may lie at any address)
+          const unsigned short* p = reinterpret_cast<const unsigned short*>(x);
+          return (uint32_t)p[0] | (uint32_t)p[1] << 16;
+        };
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks) {
           const bf16* w = a.gate_w + g * D + ks * 16 + 2 * tq;
-          wf[ks][0] = g < 3 ? *reinterpret_cast<const uint32_t*>(w) : 0u;
-          wf[ks][1] = g < 3 ? *reinterpret_cast<const uint32_t*>(w + 8) : 0u;
+          wf[ks][0] = g < 3 ? two(w) : 0u;
+          wf[ks][1] = g < 3 ? two(w + 8) : 0u;
         }
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks) mma_bf16(c, qf[ks], wf[ks][0], wf[ks][1]);

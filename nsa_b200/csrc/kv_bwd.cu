@@ -233,6 +233,11 @@ int launch(const KvArgs& a, cudaStream_t s) {
     set_error("B*T*Hq exceeds the 2^31 rows a TMA coordinate can address");
     return -32;
   }
+  // the bulk copies of 16 rows' lse, delta and gates
+  if ((((uintptr_t)a.lse | (uintptr_t)a.delta | (uintptr_t)a.gate) & 15) != 0) {
+    set_error("kv backward: lse, delta and gates must be 16-byte aligned");
+    return -5;
+  }
   int rc = make_tmap_rows2d(&tmQ, a.q, D, qrows, 16);
   if (!rc) rc = make_tmap_rows2d(&tmDO, a.dout, D, qrows, 16);
   if (!rc) rc = make_tmap_rows4d(&tmK, a.k, D, a.Hk, a.T, a.B, a.BS);

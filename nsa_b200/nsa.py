@@ -23,7 +23,7 @@ class _NSACore(torch.autograd.Function):
         (stride, block, causal, scale, pool_k, pool_s, pool_p, n_sel, sel_block, window, q0) = cfg[:11]
         score_mode = cfg[11] if len(cfg) > 11 else 0
         q, k, v, ck, cv = (_lib.require(t, n) for t, n in ((q, "q"), (k, "k"), (v, "v"), (ck, "ck"), (cv, "cv")))
-        w_gate = _lib.require(w_gate, "gating.weight")
+        w_gate = _lib.aligned(_lib.require(w_gate, "gating.weight"))
         b_gate = _lib.require(b_gate, "gating.bias") if b_gate is not None else None
         B, Tq, Hq, D = q.shape
         T, Hkv, Tc = k.shape[1], k.shape[2], ck.shape[1]
@@ -129,6 +129,7 @@ class _NSAModule(torch.autograd.Function):
                                (bias_k, names[5], (D,)), (bias_v, names[6], (D,)), (w_gate, names[7], (3, D)), (b_gate, names[8], (3,))):
             if t is not None and t.shape != shape:
                 raise RuntimeError("%s %s does not fit q %s" % (name, tuple(t.shape), tuple(q.shape)))
+        w_gate = _lib.aligned(w_gate)   # (read 16 bytes at a time)
         L, P, S, chk = _lib.lib(), _lib.ptr, _lib.stream(), _lib.check
         # runs of equal-length sequences: (first token, sequences, tokens each, first compressed row, positions each)
         runs, t0, c0 = [], 0, 0

@@ -135,6 +135,7 @@ class _GatedNSA(torch.autograd.Function):
     def forward(ctx, q, k, v, g_slc, g_swa, block_indices, block_counts, block_size, window_size, scale, offsets, need):
         q, k, v, g_slc, g_swa = (_lib.require(t, n) for t, n in (
             (q, "q"), (k, "k"), (v, "v"), (g_slc, "g_slc"), (g_swa if window_size > 0 else None, "g_swa")))
+        g_slc, g_swa = _lib.aligned(g_slc), _lib.aligned(g_swa)   # (the backward at head_dim 64 copies them 32 bytes at a time)
         o, o_slc, lse_slc, o_swa, lse_swa, idx, counts, seqs, indices = _forward(
             q, k, v, block_indices, block_counts, block_size, window_size, float(scale), offsets, need, g_slc, g_swa)
         if need:

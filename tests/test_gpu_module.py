@@ -144,3 +144,49 @@ def test_a_forward_without_gradients_does_no_work_for_a_backward(D):
         mod.requires_grad_(True)
         g.requires_grad_(True)
         assert torch.equal(call().detach(), res[0][2])
+
+
+def _odd(x):
+    """x at an address two bytes behind a 16-byte boundary, as a piece of a flat buffer of parameters may be."""
+    y = torch.empty(x.numel() + 8, dtype=x.dtype, device=x.device)[1:x.numel() + 1].view(x.shape)
+    return y.copy_(x)
+
+
+def test_gates_and_their_weights_at_any_address():
+    import nsa_b200
+    from nsa_b200.decode import compress_cache, nsa_decode
+    gen = torch.Generator(device=DEV).manual_seed(1)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device=DEV).bfloat16()
+    # the gates of selection_attention, at the head_dim whose backward copies them in pieces of 32 bytes
+    q, k, v, do = rnd(1, 300, 16, 64).requires_grad_(True), rnd(1, 300, 1, 64), rnd(1, 300, 1, 64), rnd(1, 300, 16, 64)
+    idx = torch.tensor([0, 2, 4], device=DEV).expand(1, 300, 1, 3).contiguous()
+    g = rnd(1, 300, 16)
+    res = []
+    for gates in (g, _odd(g)):
+        gates = gates.detach().requires_grad_(True)
+        o = nsa_b200.selection_attention(q, k, v, gates, gates, idx, window_size=100)
+        res.append([o.detach(), *torch.autograd.grad(o, [q, gates], do)])
+    assert all(torch.equal(a, b) for a, b in zip(*res))
+    # the module's weights: gates, and the compression's (element by element)
+    mod = nsa_b200.NSAAttention(128, True, device=DEV, dtype=torch.bfloat16).requires_grad_(False)
+    q, k, v = rnd(1100, 16, 128), rnd(1100, 1, 128), rnd(1100, 1, 128)
+    cu = torch.tensor([0, 1100], dtype=torch.int32, device=DEV)
+    res = []
+    for move in (lambda x: x, _odd):
+        for p in mod.parameters():
+            p.data = move(p.data)
+        cache = compress_cache(mod, k, v, [0, 1100])
+        res.append([mod(q, k, v, cu, 1100), cache.ck, cache.cv, nsa_decode(mod, q[-1:], k, v, [0, 1100], cache)])
+    assert mod.gating.weight.data_ptr() % 16 == 2 and all(torch.equal(a, b) for a, b in zip(*res))
+
+
+def test_compression_biases_at_any_address():
+    """Also where the contraction is split, which reads four of them at a time."""
+    from nsa_b200.compression_kv import _CompressPair
+    gen = torch.Generator(device=DEV).manual_seed(1)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device=DEV).bfloat16()
+    k, v, w, b = rnd(64, 1, 128), rnd(64, 1, 128), rnd(4096, 128), rnd(128)
+    with torch.no_grad():
+        for split in (True, False):
+            want, got = (_CompressPair.apply(k, v, w, w, bias, bias, [0, 64], [0, 3], 32, 16, split) for bias in (b, _odd(b)))
+            assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1])
