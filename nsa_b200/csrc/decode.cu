@@ -229,6 +229,10 @@ __device__ __forceinline__ int top_blocks(const float* pooled, int2* tmp, int n_
   return lane < n ? tmp[lane].x : -1;
 }
 
+// A maximum passes over NaN scores, the sum of their exponentials is NaN.  Partials are merged by their maxima, and those of -inf
+// left out: where the sum is NaN the maximum is made so too, and the NaN reaches the output.
+__device__ __forceinline__ float nan_or(float sum, float m) { return sum == sum ? m : sum; }
+
 // One (K, V) pair of an online soft-max: keys key0 .. key0+63 of the tile are valid iff kmin <= key < kmax.
 __device__ __forceinline__ void online_pair(float (&acc)[D / 8][4], float (&m_run)[2], float (&l_run)[2],
                                             const uint32_t (&qf)[D / 16][4], uint32_t kbase, uint32_t vbase, uint32_t k_empty,
@@ -309,8 +313,8 @@ __device__ __forceinline__ float4 merge_row(const DecodeArgs& a, int item, long 
   float e[2], L = 0.f;
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
-    e[k] = m[k] > -INFINITY ? ex2(m[k] - M) : 0.f;
-    if (m[k] > -INFINITY) L += l[k] * e[k];
+    e[k] = m[k] != -INFINITY ? ex2(m[k] - M) : 0.f;
+    if (m[k] != -INFINITY) L += l[k] * e[k];
   }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) L += __shfl_xor_sync(0xffffffffu, L, off);
@@ -534,7 +538,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         float* st = stat + chain * 64;
         st[0 * 16 + g + 8 * rr] = mr[rr];
         st[1 * 16 + g + 8 * rr] = l_r;
-        st[2 * 16 + g + 8 * rr] = ma[rr];
+        st[2 * 16 + g + 8 * rr] = nan_or(l_a, ma[rr]);
         st[3 * 16 + g + 8 * rr] = l_a;
       }
     }
@@ -549,7 +553,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int w = 0; w < kCons; ++w) {
         const float m1 = stat[w * 64 + ct], m2 = stat[w * 64 + 32 + ct];
         if (m1 > -INFINITY) Lr += stat[w * 64 + 16 + ct] * ex2(m1 - Mr);
-        if (m2 > -INFINITY) La += stat[w * 64 + 48 + ct] * ex2(m2 - Ma);
+        if (m2 != -INFINITY) La += stat[w * 64 + 48 + ct] * ex2(m2 - Ma);
       }
       fin[ct] = Mr;
       fin[16 + ct] = Lr > 0.f ? 1.f / Lr : 0.f;
@@ -670,7 +674,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int rr = 0; rr < 2; ++rr) {
         const float l = quad_sum(ll[rr]);
         if (tq == 0) {
-          const float m = has ? mm[rr] : -INFINITY;
+          const float m = has ? nan_or(l, mm[rr]) : -INFINITY;
           if (cl > 1) {
             dst[16 * D + g + 8 * rr] = m;
             dst[16 * D + 16 + g + 8 * rr] = l;
@@ -780,7 +784,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int w = 0; w < kCons; ++w) {
           e[br][w] = ml[(br * kCons + w) * 16 + row].x;
           x[br][w] = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (e[br][w] > -INFINITY) x[br][w] = __ldcg(base + (br * kCons + w) * (kPartFloats / 4));
+          if (e[br][w] != -INFINITY) x[br][w] = __ldcg(base + (br * kCons + w) * (kPartFloats / 4));
         }
 #pragma unroll
       for (int br = 0; br < 3; ++br) {
@@ -789,7 +793,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int w = 1; w < kCons; ++w) M = fmaxf(M, e[br][w]);
 #pragma unroll
         for (int w = 0; w < kCons; ++w) {
-          e[br][w] = e[br][w] > -INFINITY ? ex2(e[br][w] - M) : 0.f;
+          e[br][w] = e[br][w] != -INFINITY ? ex2(e[br][w] - M) : 0.f;
           L += ml[(br * kCons + w) * 16 + row].y * e[br][w];
         }
         inv[br] = L > 0.f ? 1.f / L : 0.f;
