@@ -133,7 +133,7 @@ __device__ __forceinline__ void transpose8(float4 (&x)[8], int lane) {
   }
 }
 
-template <int D>
+template <int D, bool BYSEQ>   // BYSEQ: the query rows come by sequence (see launch)
 __global__ void __launch_bounds__(kThreads, 1)
     dense_kv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
                        const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const DenseKvArgs a) {
@@ -220,8 +220,12 @@ __global__ void __launch_bounds__(kThreads, 1)
           if (good) mbar_expect_tx(full0 + 8 * sl, TILE);
         }
         good = __shfl_sync(0xffffffffu, good, 0);
-        if (good && lane < NP)
-          tma_load_3d(ring + sl * TILE + lane * PANEL, tmX, full0 + 8 * sl, lane * 64, hg * 16, (int)it.row0 + t0);
+        if (good && lane < NP) {
+          if (BYSEQ)
+            tma_load_4d(ring + sl * TILE + lane * PANEL, tmX, full0 + 8 * sl, lane * 64, hg * 16, t0, it.b);
+          else
+            tma_load_3d(ring + sl * TILE + lane * PANEL, tmX, full0 + 8 * sl, lane * 64, hg * 16, (int)it.row0 + t0);
+        }
       }
     } else if (warp == 1) {
       // ------------------------------- MMA issuer: dV(n), S^T(n+1) -----------------------------------------
@@ -506,17 +510,23 @@ __global__ void __launch_bounds__(256) dense_kv_reduce_kernel(const DenseKvArgs 
 template <int D>
 int launch(const DenseKvArgs& a, cudaStream_t s) {
   CUtensorMap tmQ, tmDO, tmK, tmV;
-  const unsigned long long qd[3] = {(unsigned long long)D, (unsigned long long)a.Hq, (unsigned long long)seq_rows(a.seq)};
-  const unsigned long long qs[2] = {(unsigned long long)D * 2, (unsigned long long)a.Hq * D * 2};
-  const unsigned qb[3] = {64, 16, (unsigned)kTok};
   const long long rows = a.seq.cu ? (a.mode ? a.seq.total_c : a.seq.total) : a.Lk;
   const int kb = a.seq.cu ? 1 : a.seq.B;
-  int rc = make_tmap_generic(&tmQ, a.q, 3, qd, qs, qb);
-  if (!rc) rc = make_tmap_generic(&tmDO, a.dout, 3, qd, qs, qb);
+  // Where a sequence's last tile of query rows reaches into the next sequence, rows come by sequence and those past the end are zeros:
+  // they enter the products over the rows with P = 0, and the next sequence's dO or Q there could be NaN or infinite.  (Not
+  // everywhere: the fourth coordinate costs 4 % of the kernel, 65536 tokens 9.9 -> 10.3 ms; a branch in the loop 1 %.)
+  const bool by_seq = !a.seq.cu && a.seq.B > 1 && a.seq.Tq % kTok != 0;
+  const int nq = by_seq ? a.seq.B : 1;
+  const unsigned long long qrows = (unsigned long long)(seq_rows(a.seq) / nq), HD2 = (unsigned long long)a.Hq * D * 2;
+  const unsigned long long qd[4] = {(unsigned long long)D, (unsigned long long)a.Hq, qrows, (unsigned long long)nq};
+  const unsigned long long qs[3] = {(unsigned long long)D * 2, HD2, qrows * HD2};
+  const unsigned qb[4] = {64, 16, (unsigned)kTok, 1};
+  int rc = make_tmap_generic(&tmQ, a.q, by_seq ? 4 : 3, qd, qs, qb);
+  if (!rc) rc = make_tmap_generic(&tmDO, a.dout, by_seq ? 4 : 3, qd, qs, qb);
   if (!rc) rc = make_tmap_rows4d(&tmK, a.k, D, a.Hk, rows, kb, 128);
   if (!rc) rc = make_tmap_rows4d(&tmV, a.v, D, a.Hk, rows, kb, 128);
   if (rc) return rc;
-  auto kern = dense_kv_tc_kernel<D>;
+  const auto kern = by_seq ? dense_kv_tc_kernel<D, true> : dense_kv_tc_kernel<D, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem<D>);
   if (e != cudaSuccess) return (int)e;
   const long long tiles = a.seq.cu ? seq_tiles(a.seq, a.mode ? 128 * a.cstride : 128) : (long long)a.seq.B * ((a.Lk + 127) / 128);

@@ -64,3 +64,26 @@ def test_dense_backward(nsa, B, T, Hq, Hk, D, window):
     for name, x, ref in (("dk", dk, want[0][1]), ("dv", dv, want[0][2]), ("dck", dck, want[1][1]), ("dcv", dcv, want[1][2])):
         _close(name, x, ref, scaled=True)
     nsa._lib.device_status()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_a_sequence_keeps_its_nan_to_itself(nsa, D, bad):
+    """NaN or infinity in dO or q of the second sequence: the first one's gradients are the same bits as without (its last tile of 8 tokens
+    reaches into the second)."""
+    gen = torch.Generator(device=DEV).manual_seed(D)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device=DEV).bfloat16()
+    T, H = 1037, 16
+    mod = nsa.NSAAttention(D, True, device=DEV, dtype=torch.bfloat16).requires_grad_(False)
+    q, k, v, do = rnd(2 * T, H, D), rnd(2 * T, 1, D), rnd(2 * T, 1, D), rnd(2 * T, H, D)
+    cu = torch.tensor([0, T, 2 * T], dtype=torch.int32, device=DEV)
+
+    def grads(q, do):
+        leaf = [x.clone().requires_grad_(True) for x in (q, k, v)]
+        return [g[:T] for g in torch.autograd.grad(mod(*leaf, cu, T), leaf, do)]
+
+    want = grads(q, do)
+    for i in range(2):
+        x = [q.clone(), do.clone()]
+        x[i][T + 2, 0, 3] = bad
+        assert all(torch.equal(a, b) for a, b in zip(grads(*x), want)), ("q", "do")[i]
