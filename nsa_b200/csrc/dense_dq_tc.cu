@@ -263,7 +263,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int tl = row >> 4, head = row & 15;
     const uint32_t lane_addr = (uint32_t)(32 * quad) << 16;
     const uint32_t ds_col = tmem + lane_addr + 384 + half * 32;
-    const float sl2 = a.scale * kLog2e;
+    const float sl2 = (D == 64 && a.scale == 0.f ? 1e-30f : a.scale) * kLog2e;   // (head_dim 64: scales of any sign, see the forward)
+    const float hidden = D == 64 && a.scale < 0.f ? INFINITY : -INFINITY;        // a masked column: scaled it is -inf
     uint32_t c = 0;
     bool ok = true;
     struct Row {   // operands of this thread's row for the (first) branch and, with both, for the compressed one, as loaded:
@@ -379,7 +380,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             const unsigned valid = h0 > l0 ? (0xffffffffu >> (32 - (h0 - l0))) << l0 : 0u;
 #pragma unroll
             for (int e = 0; e < 32; ++e)
-              if (!(valid & (1u << e))) s[32 * q + e] = -INFINITY;
+              if (!(valid & (1u << e))) s[32 * q + e] = hidden;
           }
         }
         const float nl = lse2 > -INFINITY ? -lse2 : 0.f;

@@ -255,7 +255,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int tl = row >> 4, head = row & 15;
     const uint32_t lane_addr = (uint32_t)(32 * quad) << 16;
     const uint32_t s_col = tmem + lane_addr + g * 128, o_col = tmem + lane_addr + 256 + g * 128;
-    const float sl2 = a.scale * kLog2e;
+    // (head_dim 64 takes scales of any sign, as it did on mma.sync: negative ones by negating the scores, zero as nearly so, since
+    // masked scores are -inf)
+    const bool neg = D == 64 && a.scale < 0.f;
+    const float sl2 = (D == 128 ? a.scale : a.scale == 0.f ? 1e-30f : fabsf(a.scale)) * kLog2e;
     const uint64_t sl22 = pack_f32x2(sl2, sl2);
     const uint32_t s_full = s_full0 + 8 * g, s_free = s_free0 + 8 * g, p_full = p_full0 + 8 * g, p_free = p_free0 + 8 * g,
                    o_free = o_free0 + 8 * g;
@@ -320,6 +323,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         tmem_ld_wait();
         tc_fence_before();
         mbar_arrive(s_free);   // S is in registers: the next tile's S may overwrite it
+        if (D == 64 && neg) {
+#pragma unroll
+          for (int e = 0; e < 128; ++e) s[e] = -s[e];
+        }
         // One straight block of code for whole and masked tiles: every branch inside it would drain the exponentials in
         // flight (per-chunk branches that skipped empty chunks cost 800 of 2600 cycles per tile).
         if (!__all_sync(0xffffffffu, lo <= 0 && hi >= 128)) {
