@@ -1,8 +1,8 @@
 """K/V block compression with the reference's API (nsa/compression_kv.py).
 
 ``compress_kv``, ``calc_compressed_len``, ``KVCompressorVarlen`` and ``KVCompressor`` keep the reference's
-names, arguments, parameter names/shapes and return values; the work is done by ``nsa_compress_fwd`` /
-``nsa_compress_bwd`` of libnsa_b200.so.
+names, arguments, parameter names/shapes and return values; the work is done by ``nsa_compress_fwd_kv`` and
+``nsa_compress_bwd_kv`` of libnsa_b200.so (``nsa_compress_bwd`` where a block is not one or two strides).
 """
 import math
 

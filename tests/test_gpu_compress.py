@@ -118,3 +118,24 @@ def test_keys_and_values_of_different_shapes(nsa):
     cu = torch.tensor([0, 300, 600], dtype=torch.int32)
     ck, cv, _ = comp(k, v, cu)
     assert torch.equal(ck, comp(k, k, cu)[0]) and torch.equal(cv, comp(v, v, cu)[1])
+
+
+@pytest.mark.parametrize("D,H,block,stride,lens", [(128, 4, 32, 16, [33, 1000, 31, 700]), (64, 3, 64, 16, [200, 64, 1037]), (128, 1, 16, 16, [640, 17])])
+def test_single_tensor_entry_point(nsa, D, H, block, stride, lens):
+    """nsa_compress_fwd (mma.sync, one tensor) against nsa_compress_fwd_kv without split: one chain of the same products each, so the same
+    bits."""
+    gen = torch.Generator(device=DEV).manual_seed(D)
+    rnd = lambda *s, m=1.0: (torch.randn(*s, generator=gen, device=DEV) * m).bfloat16()
+    cum = lambda ls: [sum(ls[:i]) for i in range(len(ls) + 1)]
+    n_out = [(n - block) // stride + 1 if n >= block else 0 for n in lens]
+    cu, cu_out = cum(lens), cum(n_out)
+    x, w, b = rnd(cu[-1], H, D), rnd(block * D, D, m=0.03), rnd(D)
+    L, P = nsa._lib.lib(), nsa._lib.ptr
+    cin, cout = (torch.tensor(c, dtype=torch.int32, device=DEV) for c in (cu, cu_out))
+    one, pair = (torch.empty(cu_out[-1], H, D, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    nsa._lib.check(L.nsa_compress_fwd(P(x), P(w), P(b), P(one), P(cin), P(cout), len(lens), H, D, block, stride, max(n_out),
+                                      nsa._lib.stream()), "nsa_compress_fwd")
+    nsa._lib.check(L.nsa_compress_fwd_kv(P(x), P(x), P(w), P(w), P(b), P(b), P(pair), P(pair), P(cin), P(cout), len(lens), 0, 0, cu[-1],
+                                         cu_out[-1], H, D, block, stride, 0, nsa._lib.stream()), "nsa_compress_fwd_kv")
+    _close("nsa_compress_fwd", one, _ref(x.float(), w.float(), b.float(), cu, block, stride, n_out))
+    assert torch.equal(one, pair)
