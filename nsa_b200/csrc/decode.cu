@@ -883,8 +883,12 @@ int ask_resident(int cl) {
 struct Spread {
   int cl, ncta;
 };
-Spread decode_spread(int nitem) {
+const std::array<int, 4>& clusters_held() {
   static const std::array<int, 4> held = {num_sms(), ask_resident(2), ask_resident(4), ask_resident(8)};
+  return held;
+}
+Spread decode_spread(int nitem) {
+  const std::array<int, 4>& held = clusters_held();
   for (int i = 3; i >= 0; --i)
     if (nitem <= held[i]) return {1 << i, nitem << i};
   return {1, num_sms()};
@@ -892,9 +896,13 @@ Spread decode_spread(int nitem) {
 
 }  // namespace
 
+// A set of partials for every CTA (of a cluster: one item each): as many as any number of items up to this one needs, so that a
+// workspace made for a batch serves the smaller ones too.
 size_t decode_workspace_bytes(int nseq, int Hkv) {
-  const Spread p = decode_spread(nseq * Hkv);   // a set of partials for every CTA (of a cluster: one item each)
-  return (size_t)p.ncta * 3 * kCons * kPartFloats * sizeof(float);
+  const std::array<int, 4>& held = clusters_held();
+  int ncta = nseq * Hkv > held[0] ? num_sms() : 0;
+  for (int i = 0; i < 4; ++i) ncta = std::max(ncta, std::min(nseq * Hkv, held[i]) << i);
+  return (size_t)ncta * 3 * kCons * kPartFloats * sizeof(float);
 }
 
 int launch_decode(const DecodeArgs& a, cudaStream_t s) {

@@ -85,3 +85,11 @@ def test_no_cpu_fallback():
     with pytest.raises(RuntimeError, match="no CPU path"):
         nsa.selection_attention(q, q[:, :, :1], q[:, :, :1], q[..., 0], q[..., 0],
                                 torch.zeros(1, 64, 1, 2, dtype=torch.long))
+
+
+def test_decode_workspace_of_a_batch_serves_smaller_ones():
+    """A caller allocates once, for its largest batch: the size never falls with the number of sequences."""
+    from nsa_b200 import _lib
+    for hkv in (1, 4):
+        sizes = [_lib.lib().nsa_decode_workspace_bytes(n, hkv) for n in range(1, 400)]
+        assert sizes == sorted(sizes) and sizes[0] > 0
