@@ -389,7 +389,9 @@ class NSAAttention(nn.Module):
             cu = [int(c) for c in cu_seqlens_k.tolist()]
             if any(b - a != cu[1] - cu[0] for a, b in zip(cu[:-1], cu[1:])):
                 lens = [b - a for a, b in zip(cu[:-1], cu[1:])]
-        if sum(lens) != num_token or q.shape[0] != num_token or v.shape != k.shape:
+        # (equal lengths: q may be the first tokens of every sequence alone)
+        prefix = q.shape[0] != num_token and q.shape[0] % bs == 0 and lens == [num_token // bs] * bs
+        if sum(lens) != num_token or (q.shape[0] != num_token and not prefix) or v.shape != k.shape:
             raise ValueError("%d sequences over %d tokens do not fit q %s, k %s, v %s"
                              % (bs, sum(lens), tuple(q.shape), tuple(k.shape), tuple(v.shape)))
         scale = self.softmax_scale
@@ -401,7 +403,7 @@ class NSAAttention(nn.Module):
                self.pool_stride, self.pool_padding, self.selected_block_count, self.selection_block_size,
                self.sliding_window, bool(self.fuse_row_passes), {"reference": 0, "causal": 1}[self.score_mode])
         comp = self.compressor
-        if not self._inlines_compressor():
+        if prefix or not self._inlines_compressor():
             return self._through_compressor(q, k, v, cu_seqlens_k, lens, cfg)
         tensors = (q, k, v, comp.compressor_k.weight, comp.compressor_v.weight, comp.compressor_k.bias, comp.compressor_v.bias,
                    self.gating.weight, self.gating.bias)

@@ -190,3 +190,20 @@ def test_compression_biases_at_any_address():
         for split in (True, False):
             want, got = (_CompressPair.apply(k, v, w, w, bias, bias, [0, 64], [0, 3], 32, 16, split) for bias in (b, _odd(b)))
             assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1])
+
+
+def test_queries_of_the_first_tokens_alone():
+    """q may hold the first tokens of every (equally long) sequence: their rows of the whole result."""
+    import nsa_b200
+    T, Tq, H, D = 1100, 700, 32, 128
+    gen = torch.Generator(device=DEV).manual_seed(5)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device=DEV).bfloat16()
+    mod = nsa_b200.NSAAttention(D, True, device=DEV, dtype=torch.bfloat16).requires_grad_(False)
+    q, k, v = rnd(2, T, H, D), rnd(2 * T, 2, D), rnd(2 * T, 2, D)
+    cu = torch.tensor([0, T, 2 * T], dtype=torch.int32, device=DEV)
+    whole = mod(q.reshape(2 * T, H, D), k, v, cu, T).view(2, T, H, D)
+    part = mod(q[:, :Tq].reshape(2 * Tq, H, D), k, v, cu, T).view(2, Tq, H, D)
+    assert torch.equal(part, whole[:, :Tq])
+    for bad in (q.reshape(2 * T, H, D)[:-1], torch.cat([q, q[:, :2]], 1).reshape(-1, H, D)):
+        with pytest.raises((ValueError, RuntimeError)):
+            mod(bad, k, v, cu, T)
