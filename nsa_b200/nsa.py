@@ -200,7 +200,8 @@ class _NSAModule(torch.autograd.Function):
                 "nsa_sel_swa_fwd")
         if need:
             ctx.save_for_backward(q, k, v, w_gate, saved)
-            ctx.meta = (cfg, runs, off, ix_bytes if use_ix else None, keep_ix, len(lens), b_gate is not None, bias_k is not None)
+            ctx.meta = (cfg, runs, off, ix_bytes if use_ix else None, keep_ix, len(lens), b_gate is not None,
+                        (bias_k is not None, bias_v is not None))
         return o
 
     @staticmethod
@@ -222,7 +223,7 @@ class _NSAModule(torch.autograd.Function):
         empty = lambda *shape: torch.empty(*shape, dtype=torch.bfloat16, device=dev)
         dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
         dwk, dwv = (empty(D, D, block) if n else None for n in need_w[:2])
-        dbk, dbv = (empty(D) if n and has_bc else None for n in need_w[2:])
+        dbk, dbv = (empty(D) if n and has else None for n, has in zip(need_w[2:], has_bc))
         dw, db = torch.empty_like(w_gate), empty(3) if has_bg else None
         c_bytes = L.nsa_compress_bwd_kv_workspace_bytes(nseq, runs[0][4], crow, len(runs) > 1, Hkv, D, block, stride)
         gw_bytes = L.nsa_gate_bwd_workspace_bytes(rows, D)

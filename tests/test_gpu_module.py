@@ -207,3 +207,26 @@ def test_queries_of_the_first_tokens_alone():
     for bad in (q.reshape(2 * T, H, D)[:-1], torch.cat([q, q[:, :2]], 1).reshape(-1, H, D)):
         with pytest.raises((ValueError, RuntimeError)):
             mod(bad, k, v, cu, T)
+
+
+@pytest.mark.parametrize("block", [32, 48])   # the tcgen05 backward of the compression and the other one
+@pytest.mark.parametrize("without", [("k",), ("v",), ("k", "v")])
+def test_biases_of_the_compression_are_independent(without, block):
+    """A compressor with one bias only: the other's gradient is that of a module whose missing bias is zero."""
+    import nsa_b200
+    T, H, D = 1100, 16, 64
+    gen = torch.Generator(device=DEV).manual_seed(block)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device=DEV).bfloat16()
+    mod = nsa_b200.NSAAttention(D, True, compression_block=block, selected_block_count=8, device=DEV, dtype=torch.bfloat16)
+    conv = dict(k=mod.compressor.compressor_k, v=mod.compressor.compressor_v)
+    with torch.no_grad():
+        for name in without:
+            conv[name].bias.zero_()
+    q, k, v, do = rnd(T, H, D), rnd(T, 1, D), rnd(T, 1, D), rnd(T, H, D)
+    cu = torch.tensor([0, T], dtype=torch.int32, device=DEV)
+    grads = lambda: dict(zip([n for n, _ in mod.named_parameters()], torch.autograd.grad(mod(q, k, v, cu, T), list(mod.parameters()), do)))
+    want = grads()
+    for name in without:
+        conv[name].bias = None
+    got = grads()
+    assert len(got) == 6 - len(without) and all(torch.equal(g, want[n]) for n, g in got.items())
