@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           good = __shfl_sync(0xffffffffu, good, 0);
           const bool win = WIN && (!CMP || i < sc.nw);
           const CUtensorMap* tm = is_k ? (win ? &maps.k : &maps.ck) : (win ? &maps.v : &maps.cv);
-          const int row = win ? (a.seq.cu ? (int)st.row0 : 0) + (sc.first + i) * 128 : (int)st.c0 + (i - sc.nw) * 128;
+          const int row = win ? (sc.first + i) * 128 : (i - sc.nw) * 128;
           if (good && lane < NP) tma_load_4d(ring + sl * TILE + lane * PANEL, tm, full0 + 8 * sl, lane * 64, hk, row, st.b);
           ++c;
         }
@@ -496,18 +496,15 @@ int launch(const DenseArgs& a, cudaStream_t s) {
   const unsigned long long qd[3] = {(unsigned long long)D, (unsigned long long)a.Hq, (unsigned long long)seq_rows(a.seq)};
   const unsigned long long qs[2] = {(unsigned long long)D * 2, (unsigned long long)a.Hq * D * 2};
   const unsigned qb[3] = {64, 16, (unsigned)kTok};
-  const int kb = a.seq.cu ? 1 : a.B;
   int rc = make_tmap_generic(&m.q, a.q, 3, qd, qs, qb);
   if (!rc) rc = make_tmap_generic(&m.dout, a.dout, 3, qd, qs, qb);
   if (WIN && !rc) {
-    const long long rows = a.seq.cu ? a.seq.total : a.T;
-    rc = make_tmap_rows4d(&m.k, a.k, D, a.Hk, rows, kb, 128);
-    if (!rc) rc = make_tmap_rows4d(&m.v, a.v, D, a.Hk, rows, kb, 128);
+    rc = make_tmap_rows4d(&m.k, a.k, D, a.Hk, a.T, a.B, 128);
+    if (!rc) rc = make_tmap_rows4d(&m.v, a.v, D, a.Hk, a.T, a.B, 128);
   }
   if (CMP && !rc) {
-    const long long rows = a.seq.cu ? a.seq.total_c : a.seq.Tc;
-    rc = make_tmap_rows4d(&m.ck, WIN ? a.ck : a.k, D, a.Hk, rows, kb, 128);
-    if (!rc) rc = make_tmap_rows4d(&m.cv, WIN ? a.cv : a.v, D, a.Hk, rows, kb, 128);
+    rc = make_tmap_rows4d(&m.ck, WIN ? a.ck : a.k, D, a.Hk, a.seq.Tc, a.B, 128);
+    if (!rc) rc = make_tmap_rows4d(&m.cv, WIN ? a.cv : a.v, D, a.Hk, a.seq.Tc, a.B, 128);
   }
   if (rc) return rc;
   if (!WIN) m.k = m.v = m.ck;
@@ -537,11 +534,7 @@ int dispatch(const DenseArgs& a, cudaStream_t s) {
 
 int launch_dense_dq_tc(const DenseArgs& args, int head_dim, cudaStream_t s) {
   DenseArgs a = args;
-  if (!a.seq.cu) {
-    const int Tc = a.mode == 1 ? a.Lk : a.seq.Tc;
-    a.seq = {};
-    a.seq.B = a.B; a.seq.Tq = a.Tq; a.seq.q0 = a.q0; a.seq.Tc = Tc;
-  }
+  a.seq = {a.B, a.Tq, a.q0, a.mode == 1 ? a.Lk : a.seq.Tc};
   return head_dim == 64 ? dispatch<64>(a, s) : dispatch<128>(a, s);
 }
 int dense_dq_tc_status(int* out) {

@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const SeqTile st = seq_tile(a.seq, kTok, ntile - 1 - item / HG);
       if (st.t0 >= st.Tq) continue;
       const Sched sc = make_sched<MODE>(a, st);
-      const int hk = hg / G16, krow = (int)(MODE == 0 ? (a.seq.cu ? st.row0 : 0) : st.c0);
+      const int hk = hg / G16;
       if (is_k) {
         if (lane == 0) {
           good = mbar_wait_abortable(q_free, (ic & 1) ^ 1, 101, abort_flag) ? 1 : 0;
@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         good = __shfl_sync(0xffffffffu, good, 0);
         if (good && lane < NP)
-          tma_load_4d(ring + sl * TILE + lane * PANEL, tm, full0 + 8 * sl, lane * 64, hk, krow + (sc.first + i) * 128, st.b);
+          tma_load_4d(ring + sl * TILE + lane * PANEL, tm, full0 + 8 * sl, lane * 64, hk, (sc.first + i) * 128, st.b);
       }
       ++ic;
     }
@@ -451,11 +451,9 @@ int launch(const DenseArgs& a, cudaStream_t s) {
   const unsigned long long qd[3] = {(unsigned long long)D, (unsigned long long)a.Hq, (unsigned long long)seq_rows(a.seq)};
   const unsigned long long qs[2] = {(unsigned long long)D * 2, (unsigned long long)a.Hq * D * 2};
   const unsigned qb[3] = {64, 16, (unsigned)kTokT};
-  const long long krows = a.seq.cu ? (MODE == 0 ? a.seq.total : a.seq.total_c) : a.Lk;
-  const int kb = a.seq.cu ? 1 : a.B;
   int rc = make_tmap_generic(&tmQ, a.q, 3, qd, qs, qb);
-  if (!rc) rc = make_tmap_rows4d(&tmK, a.k, D, a.Hk, krows, kb, 128);
-  if (!rc) rc = make_tmap_rows4d(&tmV, a.v, D, a.Hk, krows, kb, 128);
+  if (!rc) rc = make_tmap_rows4d(&tmK, a.k, D, a.Hk, a.Lk, a.B, 128);
+  if (!rc) rc = make_tmap_rows4d(&tmV, a.v, D, a.Hk, a.Lk, a.B, 128);
   if (rc) return rc;
   auto kern = dense_fwd2_tc_kernel<D, MODE>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem<D>);
@@ -481,10 +479,7 @@ bool dense_fwd_tc_supported(const DenseArgs& a, int head_dim) {
 }
 int launch_dense_fwd2_tc(const DenseArgs& args, int head_dim, cudaStream_t s) {
   DenseArgs a = args;
-  if (!a.seq.cu) {
-    a.seq = {};
-    a.seq.B = a.B; a.seq.Tq = a.Tq; a.seq.q0 = a.q0; a.seq.Tc = a.Lk;
-  }
+  a.seq = {a.B, a.Tq, a.q0, a.Lk};
   if (head_dim == 64) return a.mode == 0 ? launch<64, 0>(a, s) : launch<64, 1>(a, s);
   return a.mode == 0 ? launch<128, 0>(a, s) : launch<128, 1>(a, s);
 }

@@ -50,8 +50,7 @@ constexpr uint32_t kTmemCols = 512;           // S^T / P^T 0.., dP^T / dS^T 128.
 
 struct Item {
   long long row0, out_row;   // first query row of the sequence; output row of the tile's first key
-  int hk, b, krow;           // TMA coordinates of the key tile
-  int key0, keys;            // first key (position in its sequence), keys of the tile
+  int hk, b, key0, keys;     // KV head, sequence, first key (position in its sequence) and keys of the tile
   int Tq, qlo, n, shift;     // query rows of the sequence; query tiles qlo .. qlo+n-1, walked from `shift` on
   int slab;
 };
@@ -62,33 +61,18 @@ __device__ __forceinline__ bool decode_item(const DenseKvArgs& a, Item& it) {
     sp = i % a.nslab;
     i /= a.nslab;
   }
-  const int G = a.mode == 0 ? 128 : 128 * a.cstride;   // tokens per key tile
-  const int per = a.seq.cu ? seq_tiles_dev(a.seq, G) : (a.Lk + 127) / 128;
+  const int per = (a.Lk + 127) / 128;
   const int tile = i % per;
   i /= per;
-  int Lk = a.Lk;
   it.hk = i % a.Hk;
   i /= a.Hk;
-  if (a.seq.cu) {
-    const SeqTile st = seq_tile(a.seq, G, tile);
-    if (a.mode == 1) sp = a.nslab - 1 - i;
-    it.b = 0;
-    it.row0 = st.row0;
-    it.Tq = st.Tq;
-    Lk = a.mode == 0 ? st.Tq : st.Tc;
-    it.key0 = a.mode == 0 ? st.t0 : st.t0 / a.cstride;
-    it.krow = (int)(a.mode == 0 ? st.row0 : st.c0) + it.key0;
-    it.out_row = it.krow;
-  } else {
-    it.b = i % a.seq.B;
-    if (a.mode == 1) sp = a.nslab - 1 - i / a.seq.B;
-    it.row0 = (long long)it.b * a.seq.Tq;
-    it.Tq = a.seq.Tq;
-    it.key0 = it.krow = tile * 128;
-    it.out_row = (long long)it.b * Lk + it.key0;
-  }
-  it.keys = min(128, Lk - it.key0);
-  if (it.keys <= 0) return false;
+  it.b = i % a.seq.B;
+  if (a.mode == 1) sp = a.nslab - 1 - i / a.seq.B;
+  it.row0 = (long long)it.b * a.seq.Tq;
+  it.Tq = a.seq.Tq;
+  it.key0 = tile * 128;
+  it.out_row = (long long)it.b * a.Lk + it.key0;
+  it.keys = min(128, a.Lk - it.key0);
   it.slab = sp;
   long long lo, hi;   // query rows that see one of the keys
   if (a.mode == 0) {
@@ -208,7 +192,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (lane == 0) mbar_expect_tx(is_k ? k_full : v_full, TILE);
         __syncwarp();
         if (lane < NP)
-          tma_load_4d((is_k ? k_s : v_s) + lane * PANEL, is_k ? &tmK : &tmV, is_k ? k_full : v_full, lane * 64, it.hk, it.krow, it.b);
+          tma_load_4d((is_k ? k_s : v_s) + lane * PANEL, is_k ? &tmK : &tmV, is_k ? k_full : v_full, lane * 64, it.hk, it.key0, it.b);
       }
       int good = 1;
       for (int c = 0; good && c < N; ++c) {
@@ -483,18 +467,7 @@ __global__ void __launch_bounds__(256) dense_kv_reduce_kernel(const DenseKvArgs 
   const long long i = ((long long)blockIdx.x * 256 + threadIdx.x) * 4;
   if (i >= a.n_out) return;
   const long long row = i / (a.Hk * D);
-  int key, Tq = a.seq.Tq;
-  if (a.seq.cu) {
-    int lo = 0, hi = a.seq.B - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (a.seq.cu_c[mid] <= row) lo = mid; else hi = mid - 1;
-    }
-    key = (int)row - a.seq.cu_c[lo];
-    Tq = a.seq.cu[lo + 1] - a.seq.cu[lo];
-  } else {
-    key = (int)(row % a.Lk);
-  }
+  const int key = (int)(row % a.Lk), Tq = a.seq.Tq;
   const long long first = a.causal ? (long long)(key / 128 * 128) * a.cstride + a.cblock - a.seq.q0 : 0;
   const float* p = a.part + (blockIdx.y ? (long long)a.nslab * a.n_out : 0) + i;
   float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -510,12 +483,10 @@ __global__ void __launch_bounds__(256) dense_kv_reduce_kernel(const DenseKvArgs 
 template <int D>
 int launch(const DenseKvArgs& a, cudaStream_t s) {
   CUtensorMap tmQ, tmDO, tmK, tmV;
-  const long long rows = a.seq.cu ? (a.mode ? a.seq.total_c : a.seq.total) : a.Lk;
-  const int kb = a.seq.cu ? 1 : a.seq.B;
   // Where a sequence's last tile of query rows reaches into the next sequence, rows come by sequence and those past the end are zeros:
   // they enter the products over the rows with P = 0, and the next sequence's dO or Q there could be NaN or infinite.  (Not
   // everywhere: the fourth coordinate costs 4 % of the kernel, 65536 tokens 9.9 -> 10.3 ms; a branch in the loop 1 %.)
-  const bool by_seq = !a.seq.cu && a.seq.B > 1 && a.seq.Tq % kTok != 0;
+  const bool by_seq = a.seq.B > 1 && a.seq.Tq % kTok != 0;
   const int nq = by_seq ? a.seq.B : 1;
   const unsigned long long qrows = (unsigned long long)(seq_rows(a.seq) / nq), HD2 = (unsigned long long)a.Hq * D * 2;
   const unsigned long long qd[4] = {(unsigned long long)D, (unsigned long long)a.Hq, qrows, (unsigned long long)nq};
@@ -523,13 +494,13 @@ int launch(const DenseKvArgs& a, cudaStream_t s) {
   const unsigned qb[4] = {64, 16, (unsigned)kTok, 1};
   int rc = make_tmap_generic(&tmQ, a.q, by_seq ? 4 : 3, qd, qs, qb);
   if (!rc) rc = make_tmap_generic(&tmDO, a.dout, by_seq ? 4 : 3, qd, qs, qb);
-  if (!rc) rc = make_tmap_rows4d(&tmK, a.k, D, a.Hk, rows, kb, 128);
-  if (!rc) rc = make_tmap_rows4d(&tmV, a.v, D, a.Hk, rows, kb, 128);
+  if (!rc) rc = make_tmap_rows4d(&tmK, a.k, D, a.Hk, a.Lk, a.seq.B, 128);
+  if (!rc) rc = make_tmap_rows4d(&tmV, a.v, D, a.Hk, a.Lk, a.seq.B, 128);
   if (rc) return rc;
   const auto kern = by_seq ? dense_kv_tc_kernel<D, true> : dense_kv_tc_kernel<D, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem<D>);
   if (e != cudaSuccess) return (int)e;
-  const long long tiles = a.seq.cu ? seq_tiles(a.seq, a.mode ? 128 * a.cstride : 128) : (long long)a.seq.B * ((a.Lk + 127) / 128);
+  const long long tiles = (long long)a.seq.B * ((a.Lk + 127) / 128);
   const long long grid = tiles * a.Hk * a.nslab;
   if (grid <= 0) return 0;
   if (grid > 0x7fffffffLL) {
@@ -549,7 +520,7 @@ int launch(const DenseKvArgs& a, cudaStream_t s) {
 
 int launch_dense_kv_tc(const DenseKvArgs& args, int head_dim, cudaStream_t s) {
   DenseKvArgs a = args;
-  a.n_out = (a.seq.cu ? (a.mode ? a.seq.total_c : a.seq.total) : (long long)a.seq.B * a.Lk) * a.Hk * head_dim;
+  a.n_out = (long long)a.seq.B * a.Lk * a.Hk * head_dim;
   return head_dim == 64 ? launch<64>(a, s) : launch<128>(a, s);
 }
 

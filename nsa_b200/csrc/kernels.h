@@ -9,49 +9,28 @@
 namespace nsa {
 
 // ---- the sequences of a call ------------------------------------------------------------------
-// Equal lengths (cu null): B sequences, Tq query rows each (the tokens q0 .. q0+Tq-1 of a sequence; tensors hold Tq rows per
-// batch) and Tc compressed positions.  Packed (cu, cu_c device [B+1]): sequence s is the tokens cu[s] .. cu[s+1]-1 and the
-// compressed rows cu_c[s] .. cu_c[s+1]-1 of one packed tensor.
+// B sequences of equal length, Tq query rows each (the tokens q0 .. q0+Tq-1 of a sequence; tensors hold Tq rows per batch) and
+// Tc compressed positions.
 struct Seqs {
-  const int *cu, *cu_c;
   int B, Tq, q0, Tc;
-  long long total, total_c;   // packed: tokens and compressed rows in all
 };
-// Tiles of G tokens never cross a sequence's end.  Packed: sequence s owns the tile indices from cu[s] / G + s on, never
-// fewer than it has tiles, so no table is needed (an index past its last tile has t0 >= Tq).
-inline int seq_tiles(const Seqs& q, int G) { return q.cu ? (int)(q.total / G) + q.B : q.B * ((q.Tq + G - 1) / G); }
-inline long long seq_rows(const Seqs& q) { return q.cu ? q.total : (long long)q.B * q.Tq; }
+// Tiles of G tokens never cross a sequence's end.
+inline int seq_tiles(const Seqs& q, int G) { return q.B * ((q.Tq + G - 1) / G); }
+inline long long seq_rows(const Seqs& q) { return (long long)q.B * q.Tq; }
 #ifdef __CUDACC__
 struct SeqTile {
   long long row0;   // first query row (token) of the sequence
-  long long c0;     // row coordinate of its first compressed position (with batch coordinate b)
   int b, t0, Tq, Tc;
 };
-__device__ __forceinline__ int seq_tiles_dev(const Seqs& q, int G) { return q.cu ? (int)(q.total / G) + q.B : q.B * ((q.Tq + G - 1) / G); }
+__device__ __forceinline__ int seq_tiles_dev(const Seqs& q, int G) { return q.B * ((q.Tq + G - 1) / G); }
 __device__ __forceinline__ SeqTile seq_tile(const Seqs& q, int G, int t) {
   SeqTile r;
-  if (!q.cu) {
-    const int per = (q.Tq + G - 1) / G;
-    r.b = t / per;
-    r.t0 = (t - r.b * per) * G;
-    r.row0 = (long long)r.b * q.Tq;
-    r.c0 = 0;
-    r.Tq = q.Tq;
-    r.Tc = q.Tc;
-    return r;
-  }
-  int lo = 0, hi = q.B - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (q.cu[mid] / G + mid <= t) lo = mid; else hi = mid - 1;
-  }
-  const int c = q.cu[lo];
-  r.b = 0;
-  r.t0 = (t - (c / G + lo)) * G;
-  r.row0 = c;
-  r.c0 = q.cu_c ? q.cu_c[lo] : 0;
-  r.Tq = q.cu[lo + 1] - c;
-  r.Tc = q.cu_c ? q.cu_c[lo + 1] - (int)r.c0 : 0;
+  const int per = (q.Tq + G - 1) / G;
+  r.b = t / per;
+  r.t0 = (t - r.b * per) * G;
+  r.row0 = (long long)r.b * q.Tq;
+  r.Tq = q.Tq;
+  r.Tc = q.Tc;
   return r;
 }
 // avg_pool1d(kernel 5, stride 4, no padding, ceil_mode) output length, as nsa_pool_out_len computes it
@@ -69,7 +48,7 @@ struct ScoreArgs {
   const bf16* q;       // [tok,Hq,D]
   const bf16* ck;      // compressed keys
   int* sel_idx;        // [tok,Hq/16,n_sel]
-  float* sel_scores;   // optional dump of the pooled scores [B,Hq/16,Tq,n_pool] (equal lengths), or null
+  float* sel_scores;   // optional dump of the pooled scores [B,Hq/16,Tq,n_pool], or null
   Seqs seq;
   int Hq, Hk, n_sel;
   int Tc_max;          // compressed positions of the longest sequence
@@ -148,7 +127,7 @@ struct DenseArgs {
   const bf16 *ck, *cv;
   const float *lse_c, *delta_c;
   const bf16* gate_c;
-  Seqs seq;            // tcgen05 kernels: packed sequences (seq.cu null: B, Tq, q0, Lk above)
+  Seqs seq;            // tcgen05 kernels: set by the launchers from B, Tq, q0 and the compressed length
   // optional, tcgen05 dQ: the row pre-pass of the backward folded in.  With pre_o[0] set the kernel computes
   // rowsum(o * dO) itself for its own branch ([0]) and, if given, a second branch ([1]) whose dQ kernel runs later:
   // pre_delta[x] = gate_x * rowsum (fp32, also what this kernel uses as delta), pre_dgate[x] = rowsum (bf16, gate gradient)
@@ -178,7 +157,7 @@ struct DenseKvArgs {
   float* part;            // fp32 slabs [2][slabs][n_out] (dK, then dV), the kernel's own from slab0 on, or null (nslab 1)
   int nslab, slab0, slabs;   // mode 0: parts of a key tile's query range, each slab complete; mode 1: segments of seg_len query
   int seg_len;               // rows (a multiple of 8), written where they see something of the key tile; slab0 0, slabs nslab
-  int Hq, Hk, Lk;         // Lk: keys per sequence (equal lengths)
+  int Hq, Hk, Lk;         // Lk: keys per sequence
   int window, cblock, cstride, causal;
   float scale;
   long long n_out;        // set by the launcher

@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             break;
           }
           const int jt = i < nt ? i : i - nt;
-          if (lane < 2) tma_load_4d(k_ring + ks * TILE + lane * PANEL, &tmK, k_full0 + 8 * ks, lane * 64, hg / G16, (int)st.c0 + jt * 128, st.b);
+          if (lane < 2) tma_load_4d(k_ring + ks * TILE + lane * PANEL, &tmK, k_full0 + 8 * ks, lane * 64, hg / G16, jt * 128, st.b);
         }
         ++ic;
       }
@@ -409,7 +409,7 @@ int launch_score_tc(const ScoreArgs& a, cudaStream_t s) {
   const unsigned long long qs[2] = {(unsigned long long)D * 2, (unsigned long long)a.Hq * D * 2};
   const unsigned qb[3] = {64, 16, (unsigned)kTokT};
   int rc = make_tmap_generic(&tmQ, a.q, 3, qd, qs, qb);
-  if (!rc) rc = make_tmap_rows4d(&tmK, a.ck, D, a.Hk, a.seq.cu ? a.seq.total_c : a.seq.Tc, a.seq.cu ? 1 : a.seq.B, 128);
+  if (!rc) rc = make_tmap_rows4d(&tmK, a.ck, D, a.Hk, a.seq.Tc, a.seq.B, 128);
   if (rc) return rc;
   int dev = 0, max_smem = 0;
   cudaGetDevice(&dev);
