@@ -254,14 +254,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const bool ok = mbar_wait_abortable(pool_full0 + 8 * slot, (ic / (uint32_t)nslot) & 1, 306, abort_flag);
       const int t_w = st.t0 + w * 4, nlive = min(4, st.Tq - t_w);   // this warp's four tokens
       if (ok && nlive > 0) {
-        float* src = pl + w * 4 * pool_floats;
-        // Causal scores: the soft-max groups have written the tiles up to the item's last visible key; behind them lies what the
-        // slot held before, where every score is zero.
-        if (causal) {
-          for (int u = 0; u < nlive; ++u)
-            for (int blk = 32 * nt + lane; blk < n_pool; blk += 32) src[u * pool_floats + blk] = 0.f;
-          __syncwarp();
-        }
+        const float* src = pl + w * 4 * pool_floats;
         int* out = a.sel_idx + ((st.row0 + t_w) * HG + hg) * a.n_sel;
         float* dump = a.sel_scores ? a.sel_scores + ((long long)(st.b * HG + hg) * st.Tq + t_w) * n_pool : nullptr;
         const long long os = (long long)HG * a.n_sel;
@@ -386,6 +379,12 @@ __global__ void __launch_bounds__(kThreads, 1)
           __syncwarp();
           if ((lane & 15) == 8 && i + hh > 0) p0[-1] += v[0];
         }
+      }
+      // Causal scores: behind the item's last visible key lies what the slot held before, and every score is zero.  (Cleared here and
+      // not by the warp that reads them: that took 3 % of the kernel in the other mode too.)
+      if (causal) {
+        const int n_pool = pool_len_54(st.Tc);
+        for (int blk = 32 * nt + (lane & 15); blk < n_pool; blk += 16) pt[blk] = 0.f;
       }
       mbar_arrive(pool_full0 + 8 * slot);
       ++ic;
