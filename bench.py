@@ -12,8 +12,8 @@ gradients are all-reduced over NCCL inside the timed region.
 One JSON line is printed by rank 0: whole-job tokens/s with inputs resident in HBM (`value`), the same through
 the public API from pinned host buffers with the copies timed (`e2e`), the dominant kernel's roofline
 (`roofline`, timed with CUDA events inside this run), a per-kernel breakdown with one roofline entry per kernel
-(`kernel_rooflines`: tensor-pipe fraction on the keys actually visited; for the selected-attention kernels also the
-L2 -> SM gather rate against a measured gather ceiling), the clocks sampled under load, the CPU baseline (the oracle
+(`kernels_ms`: the calls of a module step and their parts; `kernel_rooflines`: tensor-pipe fraction on the keys actually
+visited; for the query-major selected-attention kernels also the L2 -> SM gather rate against a measured gather ceiling), the clocks sampled under load, the CPU baseline (the oracle
 restatement of the reference's naive torch path on the host cores) and, under `secondary`, the other BASELINE.json
 configurations measured in the same process: `selection_microbench` (configs[1], N=1 only), `context` (configs[3] at
 the run's N) and `decode` (configs[4] at the run's N).
@@ -36,14 +36,14 @@ if ROOT not in sys.path:
 CFG = dict(B=8, T=8192, Hq=64, Hkv=4, D=128, block=32, stride=16, sel_block=64, n_sel=16, window=512, seed=2)
 WORKLOAD = "configs[2]: NSAAttention module fwd+bwd bf16, B=8 T=8192 Hq=64 Hkv=4 D=128, cmp 32/16, sel 64 top-16, window 512"
 METRIC = "NSA fwd+bwd tokens/s"
-# ncu DRAM traffic per launch, MB per 8192-token sequence (see run_gpu), and the build it was captured from
-NCU_TRAFFIC_COMMIT = "2bd6f3b"
-NCU_MB_PER_SEQ = {"sel_fwd": 238, "sel_dq": 376, "sel+swa_dkv(+reverse index)": 867, "cmp_attn_fwd+select": 227,
-                  "swa_fwd": 243, "swa_dq": 394, "cmp_dq": 375, "cmp_dkv(+reduce)": 277,
-                  # key-major forward 203 read + 1046 written, its merge 1109 + 88
-                  "sel_fwd_keymajor(+reverse index,+merge)": 2446,
-                  # key-major kernel with dQ partials 1278 read + 1077 written, their reduction 1210 + 81
-                  "sel+swa_dkv+sel_dq(+reverse index,+reduce)": 3646}
+# ncu DRAM traffic, MB per 8192-token sequence (see run_gpu), and the build it was captured from
+NCU_TRAFFIC_COMMIT = "6d75620"
+NCU_MB_PER_SEQ = {"select": 139, "cmp_fwd": 222, "swa_fwd": 242, "swa+cmp_dq": 403, "swa_dkv": 318, "cmp_dkv+reduce": 347,
+                  "compress_fwd": 19, "compress_bwd": 55,
+                  # key-major forward 453 read + 1045 written, its merge with the gated sum 1381 + 217
+                  "sel_fwd+gated_sum": 3096,
+                  # key-major backward 1150 read + 1083 written, the reduction of the dQ partials 1213 + 83
+                  "sel_bwd+reduce": 3529}
 
 
 # ---------------------------------------------------------------------------------------------------------
@@ -182,93 +182,83 @@ def run_reference(args):
 # GPU arm
 # ---------------------------------------------------------------------------------------------------------
 def per_kernel_breakdown(torch, nsa_b200, mod, q4, k4, v4, do4, reps=3):
-    """Times every kernel family of the step separately with CUDA events on the current stream (each call is a
-    C-ABI entry point restricted to one kernel).  Returns {name: ms} and the selection pair count."""
+    """Times the calls of a module step one by one with CUDA events on the current stream: the C entry points that
+    NSAAttention's forward and backward make, with the same arguments, and those of their parts that can be called alone
+    (the names in PARTS; what cannot is the difference).  Returns {name: ms} and the number of selected keys."""
     from nsa_b200 import _lib
     L = _lib.lib()
     B, T, Hq, D = q4.shape
     Hkv = k4.shape[2]
     c = CFG
-    scale = D ** -0.5
-    cu = torch.arange(0, (B + 1) * T, T, dtype=torch.int32, device=q4.device)
-    k3, v3 = k4.view(B * T, Hkv, D), v4.view(B * T, Hkv, D)
-    with torch.no_grad():
-        ck, cv, _ = mod.compressor(k3, v3, cu, None)
-    Tc = ck.shape[1]
-    o_cmp, o_slc, o_swa = (torch.empty_like(q4) for _ in range(3))
-    lse_cmp, lse_slc, lse_swa, delta = (torch.empty(B, T, Hq, dtype=torch.float32, device=q4.device) for _ in range(4))
-    idx = torch.empty(B, T, Hkv, c["n_sel"], dtype=torch.int32, device=q4.device)
-    dq, dk, dv = torch.empty_like(q4), torch.empty_like(k4), torch.empty_like(v4)
-    dck, dcv = torch.empty_like(ck), torch.empty_like(cv)
-    ws1 = torch.empty(max(_lib.sel_swa_bwd_workspace_bytes(B, T, T, Hq, Hkv, D, c["n_sel"], c["sel_block"]),
-                          L.nsa_sel_swa_fwd_workspace_bytes(B, T, T, Hq, Hkv, D, c["n_sel"], c["sel_block"])),
-                      dtype=torch.uint8, device=q4.device)
-    ws2 = torch.empty(L.nsa_cmp_attn_bwd_workspace_bytes(B, T, Tc, Hkv, D), dtype=torch.uint8, device=q4.device)
+    n, BS, W, block, stride = c["n_sel"], c["sel_block"], c["window"], c["block"], c["stride"]
+    scale, dev, rows = D ** -0.5, q4.device, B * T * Hq
+    Tc = (T - block) // stride + 1
     P, S = _lib.ptr, _lib.stream
-    wk = mod.compressor.compressor_k.weight.detach().permute(2, 1, 0).reshape(c["block"] * D, D).contiguous()
-    bk = mod.compressor.compressor_k.bias.detach()
-    cin = torch.arange(0, (B + 1) * T, T, dtype=torch.int32, device=q4.device)
-    cout = torch.arange(0, (B + 1) * Tc, Tc, dtype=torch.int32, device=q4.device)
-    dwk = torch.empty(c["block"] * D, D, dtype=torch.float32, device=q4.device)
-    dbk = torch.empty(D, dtype=torch.float32, device=q4.device)
-    ws3 = torch.empty(L.nsa_compress_bwd_workspace_bytes(B, Hkv, D, c["block"]), dtype=torch.uint8, device=q4.device)
-    g1, g2, g3, dg1, dg2, dg3 = (torch.full((B, T, Hq), 0.5, dtype=torch.bfloat16, device=q4.device) for _ in range(6))
-    delta2, delta3 = torch.empty_like(delta), torch.empty_like(delta)
-    wg, bg = mod.gating.weight.detach(), mod.gating.bias.detach()
-    dwg, dbg = torch.empty_like(wg), torch.empty_like(bg)
-    ws4 = torch.empty(L.nsa_gate_bwd_workspace_bytes(B * T * Hq, D), dtype=torch.uint8, device=q4.device)
+    bf = lambda *shape: torch.empty(*shape, dtype=torch.bfloat16, device=dev)
+    f32 = lambda *shape: torch.empty(*shape, dtype=torch.float32, device=dev)
+    u8 = lambda nbytes: torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    comp, gating = mod.compressor, mod.gating
+    convs = [getattr(comp, "compressor_" + x) for x in "kv"]
+    (cwk, cwv), (bk, bv) = [x.weight.detach() for x in convs], [x.bias.detach() for x in convs]
+    wg, bg = gating.weight.detach(), gating.bias.detach()
+    wk, wv, ck, cv = bf(block * D, D), bf(block * D, D), bf(B, Tc, Hkv, D), bf(B, Tc, Hkv, D)
+    o, o_cmp, o_slc, o_swa, dq = (torch.empty_like(q4) for _ in range(5))
+    lse_cmp, lse_slc, lse_swa, d_slc, d_swa, d_cmp = (f32(B, T, Hq) for _ in range(6))
+    g = [bf(B, T, Hq) for _ in range(3)]      # selected, window, compressed
+    dg = [bf(B, T, Hq) for _ in range(3)]
+    idx = torch.empty(B, T, Hkv, n, dtype=torch.int32, device=dev)
+    index = u8(L.nsa_sel_index_bytes(B, T, T, Hkv, n, BS))
+    dk, dv, dck, dcv = torch.empty_like(k4), torch.empty_like(v4), torch.empty_like(ck), torch.empty_like(cv)
+    dwk, dwv, dbk, dbv, dwg, dbg = bf(D, D, block), bf(D, D, block), bf(D), bf(D), torch.empty_like(wg), bf(3)
+    n_fwd = L.nsa_sel_swa_fwd_ix_workspace_bytes(B, T, T, Hq, Hkv, D, n, BS)
+    n_bwd = L.nsa_attn_bwd_ix_workspace_bytes(B, T, Tc, Hq, Hkv, D, n, BS, W)
+    n_sel = L.nsa_sel_swa_bwd_ix_workspace_bytes(B, T, T, Hq, Hkv, D, n, BS, 0)
+    n_cmp = L.nsa_cmp_attn_bwd_workspace_bytes(B, T, Tc, Hkv, D)
+    ws = u8(max(n_fwd, n_bwd, n_sel, n_cmp))
+    n_gate, n_conv = L.nsa_gate_bwd_workspace_bytes(rows, D), L.nsa_compress_bwd_kv_workspace_bytes(B, Tc, B * Tc, 0, Hkv, D, block, stride)
+    ws_gate, ws_conv = u8(n_gate), u8(n_conv)
+    none = lambda k: (None,) * k
+
+    def cmp_fwd(n_sel_):
+        return lambda: L.nsa_cmp_attn_fwd_gated(P(q4), P(ck), P(cv), P(o_cmp), P(lse_cmp), P(idx), *none(6), B, T, Tc, Hq, Hkv, D, block,
+                                                stride, 1, scale, n_sel_, 5, 4, 0, 0, T, 0, S())
 
     calls = {
-        "compress_fwd(one of k,v)": lambda: L.nsa_compress_fwd_uniform(P(k3), P(wk), P(bk), P(ck), B, T, Hkv, D, c["block"],
-                                                                        c["stride"], S()),
-        "cmp_attn_fwd+select": lambda: L.nsa_cmp_attn_fwd(P(q4), P(ck), P(cv), P(o_cmp), P(lse_cmp), P(idx), None, B, T,
-                                                          Tc, Hq, Hkv, D, c["block"], c["stride"], 1, scale, c["n_sel"],
-                                                          5, 4, 0, S()),
-        "sel_fwd": lambda: L.nsa_sel_swa_fwd(P(q4), P(k4), P(v4), P(idx), 0, None, P(o_slc), P(lse_slc), None, None, None,
-                                             None, None, None, None, B, T, Hq, Hkv, D, c["n_sel"], c["sel_block"], 0,
-                                             scale, S()),
-        # what a module step runs: the same forward key-major on the tensor cores (reverse index, one CTA per key block
-        # over the queries that selected it, per-visit partial tiles, slot-order merge); "sel_fwd" above is the
-        # query-major kernel that runs without a workspace
-        "sel_fwd_keymajor(+reverse index,+merge)": lambda: L.nsa_sel_swa_fwd_ws(
-            P(q4), P(k4), P(v4), P(idx), 0, None, P(o_slc), P(lse_slc), None, None, None, None, None, None, None, P(ws1),
-            ws1.numel(), B, T, Hq, Hkv, D, c["n_sel"], c["sel_block"], 0, scale, T, 0, S()),
-        "gather_probe": lambda: L.nsa_gather_probe(P(k4), P(v4), P(idx), 0, B, T, Hq, Hkv, D, c["n_sel"], c["sel_block"],
-                                                   S()),
-        "swa_fwd": lambda: L.nsa_sel_swa_fwd(P(q4), P(k4), P(v4), None, 0, None, None, None, P(o_swa), P(lse_swa), None,
-                                             None, None, None, None, B, T, Hq, Hkv, D, c["n_sel"], c["sel_block"],
-                                             c["window"], scale, S()),
-        "combine": lambda: L.nsa_combine(P(o_slc), P(g1), P(o_swa), P(g1), P(o_cmp), P(g1), P(dq), B * T * Hq, D, S()),
-        "gate_fwd": lambda: L.nsa_gate_fwd(P(q4), P(wg), P(bg), P(g1), P(g2), P(g3), B * T * Hq, D, S()),
-        "rowdot3(delta,dgate)": lambda: L.nsa_rowdot3(P(o_slc), P(o_swa), P(o_cmp), P(do4), P(g1), P(g2), P(g3), P(delta),
-                                                      P(delta2), P(delta3), P(dg1), P(dg2), P(dg3), B * T * Hq, D, S()),
-        "sel_dq": lambda: L.nsa_sel_swa_bwd(P(q4), P(k4), P(v4), P(idx), 0, None, P(do4), P(lse_slc), P(delta), None, None,
-                                            None, None, None, P(dq), 0, None, None, None, 0, B, T, Hq, Hkv, D, c["n_sel"],
-                                            c["sel_block"], 0, scale, S()),
-        "swa_dq": lambda: L.nsa_sel_swa_bwd(P(q4), P(k4), P(v4), None, 0, None, None, None, None, None, P(do4), P(lse_swa),
-                                            P(delta), None, P(dq), 0, None, None, None, 0, B, T, Hq, Hkv, D, c["n_sel"],
-                                            c["sel_block"], c["window"], scale, S()),
-        "sel+swa_dkv(+reverse index)": lambda: L.nsa_sel_swa_bwd(
-            P(q4), P(k4), P(v4), P(idx), 0, None, P(do4), P(lse_slc), P(delta), None, P(do4), P(lse_swa), P(delta), None,
-            None, 0, P(dk), P(dv), P(ws1), ws1.numel(), B, T, Hq, Hkv, D, c["n_sel"], c["sel_block"], c["window"], scale,
-            S()),
-        # the call the module makes: window dQ, then the key-major kernel (dK, dV and the selected branch's dQ partials)
-        # and the reduction of the partials (large workspace); the query-major "sel_dq" above is what runs instead when
-        # a caller hands over only the small workspace
-        "sel+swa_bwd(all)": lambda: L.nsa_sel_swa_bwd(
-            P(q4), P(k4), P(v4), P(idx), 0, None, P(do4), P(lse_slc), P(delta), None, P(do4), P(lse_swa), P(delta), None,
-            P(dq), 0, P(dk), P(dv), P(ws1), ws1.numel(), B, T, Hq, Hkv, D, c["n_sel"], c["sel_block"], c["window"], scale,
-            S()),
-        "cmp_dq": lambda: L.nsa_cmp_attn_bwd(P(q4), P(ck), P(cv), P(lse_cmp), P(do4), P(delta), None, P(dq), 0, None, None,
-                                             None, 0, B, T, Tc, Hq, Hkv, D, c["block"], c["stride"], 1, scale, S()),
-        "cmp_dkv(+reduce)": lambda: L.nsa_cmp_attn_bwd(P(q4), P(ck), P(cv), P(lse_cmp), P(do4), P(delta), None, None, 0,
-                                                       P(dck), P(dcv), P(ws2), ws2.numel(), B, T, Tc, Hq, Hkv, D,
-                                                       c["block"], c["stride"], 1, scale, S()),
-        "gate_bwd": lambda: L.nsa_gate_bwd(P(q4), P(dg1), P(dg2), P(dg3), P(wg), P(dq), P(dwg), P(dbg), P(ws4), ws4.numel(),
-                                           B * T * Hq, D, S()),
-        "compress_bwd(one of k,v)": lambda: L.nsa_compress_bwd(P(k3), P(wk), P(dck), P(dk), P(dwk), P(dbk), P(ws3),
-                                                                ws3.numel(), P(cin), P(cout), B, Hkv, D, c["block"],
-                                                                c["stride"], T, B * Tc, S()),
+        "conv_weight_layout": lambda: L.nsa_conv_weight_layout(P(cwk), P(cwv), P(wk), P(wv), D, block, S()),
+        "compress_fwd": lambda: L.nsa_compress_fwd_kv(P(k4), P(v4), P(wk), P(wv), P(bk), P(bv), P(ck), P(cv), None, None, B, T, Tc,
+                                                      B * T, B * Tc, Hkv, D, block, stride, 0, S()),
+        "gate_fwd": lambda: L.nsa_gate_fwd(P(q4), P(wg), P(bg), *map(P, g), rows, D, S()),
+        "select+cmp_fwd": cmp_fwd(n),
+        "cmp_fwd": cmp_fwd(0),
+        "sel_index": lambda: L.nsa_sel_index(P(idx), 0, None, P(index), index.numel(), B, T, T, 0, Hkv, n, BS, S()),
+        "swa_fwd": lambda: L.nsa_sel_swa_fwd(P(q4), P(k4), P(v4), None, 0, None, None, None, P(o_swa), P(lse_swa), *none(5), B, T,
+                                             Hq, Hkv, D, n, BS, W, scale, S()),
+        "swa+sel_fwd+gated_sum": lambda: L.nsa_sel_swa_fwd_ix(
+            P(q4), P(k4), P(v4), P(idx), 0, None, P(index), P(o_slc), P(lse_slc), P(o_swa), P(lse_swa), P(g[0]), P(g[1]), P(o_cmp),
+            P(g[2]), P(o), P(ws), n_fwd, B, T, Hq, Hkv, D, n, BS, W, scale, T, 0, S()),
+        "rowdot3": lambda: L.nsa_rowdot3(P(o_slc), P(o_swa), P(o_cmp), P(do4), *map(P, g), P(d_slc), P(d_swa), P(d_cmp),
+                                         *map(P, dg), rows, D, S()),
+        "attn_bwd": lambda: L.nsa_attn_bwd_ix(
+            P(q4), P(k4), P(v4), P(ck), P(cv), P(idx), 0, None, P(index), P(do4), P(lse_slc), P(lse_swa), P(lse_cmp), P(d_slc),
+            P(d_swa), P(d_cmp), *map(P, g), *map(P, dg), P(wg), P(dq), P(dk), P(dv), P(dck), P(dcv), P(ws), n_bwd, B, T, Tc, Hq, Hkv,
+            D, n, BS, W, block, stride, 1, scale, S()),
+        "sel_bwd+reduce": lambda: L.nsa_sel_swa_bwd_ix(
+            P(q4), P(k4), P(v4), P(idx), 0, None, P(index), P(do4), P(lse_slc), P(d_slc), P(g[0]), *none(4), P(dq), 1, P(dk), P(dv),
+            P(ws), n_sel, B, T, Hq, Hkv, D, n, BS, 0, scale, T, 0, S()),
+        "swa_dkv": lambda: L.nsa_sel_swa_bwd(P(q4), P(k4), P(v4), None, 0, *none(5), P(do4), P(lse_swa), P(d_swa), P(g[1]), None, 0,
+                                             P(dk), P(dv), None, 0, B, T, Hq, Hkv, D, n, BS, W, scale, S()),
+        "cmp_dkv+reduce": lambda: L.nsa_cmp_attn_bwd(P(q4), P(ck), P(cv), P(lse_cmp), P(do4), P(d_cmp), P(g[2]), None, 0, P(dck),
+                                                     P(dcv), P(ws), n_cmp, B, T, Tc, Hq, Hkv, D, block, stride, 1, scale, S()),
+        "gate_bwd": lambda: L.nsa_gate_bwd(P(q4), *map(P, dg), P(wg), None, P(dwg), P(dbg), P(ws_gate), n_gate, rows, D, S()),
+        "compress_bwd": lambda: L.nsa_compress_bwd_kv(P(k4), P(v4), P(wk), P(wv), P(dck), P(dcv), P(dk), P(dv), 1, P(dwk), P(dwv),
+                                                      P(dbk), P(dbv), 2, P(ws_conv), n_conv, None, None, B, T, Tc, B * T, B * Tc,
+                                                      Hkv, D, block, stride, S()),
+        # not in a step: the query-major kernels that run without a workspace, and their gather with nothing behind it
+        "sel_fwd_query_major": lambda: L.nsa_sel_swa_fwd(P(q4), P(k4), P(v4), P(idx), 0, None, P(o_slc), P(lse_slc), *none(7), B, T, Hq,
+                                                         Hkv, D, n, BS, 0, scale, S()),
+        "sel_dq_query_major": lambda: L.nsa_sel_swa_bwd(P(q4), P(k4), P(v4), P(idx), 0, None, P(do4), P(lse_slc), P(d_slc), *none(5),
+                                                        P(dq), 0, None, None, None, 0, B, T, Hq, Hkv, D, n, BS, 0, scale, S()),
+        "gather_probe": lambda: L.nsa_gather_probe(P(k4), P(v4), P(idx), 0, B, T, Hq, Hkv, D, n, BS, S()),
     }
     out = {}
     for name, fn in calls.items():
@@ -281,14 +271,22 @@ def per_kernel_breakdown(torch, nsa_b200, mod, q4, k4, v4, do4, reps=3):
         e1.record()
         torch.cuda.synchronize()
         out[name] = e0.elapsed_time(e1) / reps
-    # derived: the composite call minus the window dQ kernel timed alone
-    out["sel+swa_dkv+sel_dq(+reverse index,+reduce)"] = out["sel+swa_bwd(all)"] - out["swa_dq"]
-    t = torch.arange(T, device=q4.device).view(1, T, 1, 1)
-    valid = (idx >= 0) & (idx.long() * c["sel_block"] <= t)
+    # parts that are not calls of their own
+    out["select"] = out["select+cmp_fwd"] - out["cmp_fwd"]
+    out["sel_fwd+gated_sum"] = out["swa+sel_fwd+gated_sum"] - out["swa_fwd"]
+    out["swa+cmp_dq"] = out["attn_bwd"] - out["sel_bwd+reduce"] - out["swa_dkv"] - out["cmp_dkv+reduce"]
+    t = torch.arange(T, device=dev).view(1, T, 1, 1)
+    valid = (idx >= 0) & (idx.long() * BS <= t)
     pairs = int(valid.sum().item())               # (token, kv head, block) visits
-    keys_per_seq_head = pairs * c["sel_block"] / (B * Hkv)
+    keys_per_seq_head = pairs * BS / (B * Hkv)
     _lib.device_status()
     return out, keys_per_seq_head
+
+
+# What a module step consists of, and the parts of its calls that are timed alone
+STEP = ("conv_weight_layout", "compress_fwd", "gate_fwd", "select+cmp_fwd", "sel_index", "swa+sel_fwd+gated_sum", "rowdot3",
+        "attn_bwd", "gate_bwd", "compress_bwd")
+PARTS = ("select", "cmp_fwd", "swa_fwd", "sel_fwd+gated_sum", "sel_bwd+reduce", "swa_dkv", "cmp_dkv+reduce", "swa+cmp_dq")
 
 
 def bind_to_gpu_numa_node(local):
@@ -468,24 +466,21 @@ def run_gpu(args):
                             nsel_pairs=keys_per)
         fm_loc = flop_model(Bl, T, Hq, Hkv, D, c["block"], c["stride"], c["sel_block"], c["n_sel"], c["window"],
                             nsel_pairs=keys_per)
-        # algorithmic flops per kernel launch (per rank): forward 4D per (row,key); the backward's 10D per (row,key)
-        # is split 4D to the dQ kernel (dQ + half of the S/dP recompute) and 6D to the dK/dV kernel
+        # algorithmic flops per part (per rank): forward 4D per (row,key); the backward's 10D per (row,key) is split 4D to the
+        # dQ kernel (dQ + half of the S/dP recompute) and 6D to the dK/dV kernel, all 10D to the selected branch's one kernel;
+        # the selection one product over all compressed keys
+        Tc = (T - c["block"]) // c["stride"] + 1
         kflops = {
-            "sel_fwd": fm_loc["slc"], "sel_fwd_keymajor(+reverse index,+merge)": fm_loc["slc"], "swa_fwd": fm_loc["swa"],
-            "cmp_attn_fwd+select": fm_loc["cmp"],
-            "sel_dq": fm_loc["slc"], "swa_dq": fm_loc["swa"], "cmp_dq": fm_loc["cmp"],
-            "sel+swa_dkv(+reverse index)": 1.5 * (fm_loc["slc"] + fm_loc["swa"]), "cmp_dkv(+reduce)": 1.5 * fm_loc["cmp"],
-            # the whole 10D of the selected branch (S, dP, dV, dK, dQ) and the window's 6D in one pass over the keys
-            "sel+swa_dkv+sel_dq(+reverse index,+reduce)": 2.5 * fm_loc["slc"] + 1.5 * fm_loc["swa"],
-            "compress_fwd(one of k,v)": fm_loc["comp"] / 2, "compress_bwd(one of k,v)": fm_loc["comp"],
+            "compress_fwd": fm_loc["comp"], "compress_bwd": 2 * fm_loc["comp"], "cmp_fwd": fm_loc["cmp"], "swa_fwd": fm_loc["swa"],
+            "select": 2.0 * D * Bl * Hq * T * Tc, "sel_fwd+gated_sum": fm_loc["slc"], "sel_fwd_query_major": fm_loc["slc"],
+            "sel_bwd+reduce": 2.5 * fm_loc["slc"], "swa_dkv": 1.5 * fm_loc["swa"], "cmp_dkv+reduce": 1.5 * fm_loc["cmp"],
+            "swa+cmp_dq": fm_loc["swa"] + fm_loc["cmp"], "sel_dq_query_major": fm_loc["slc"],
         }
-        # DRAM traffic per launch (dram__bytes_read.sum + dram__bytes_write.sum) of the kernels that can dominate, from
-        # one ncu capture of the B=1 slice of this workload (`--profile-case`), in MB per sequence; traffic grows in
-        # proportion to the number of sequences (every sequence's K/V stays in L2, q/dO/o/dq are streamed once).
-        # NCU_TRAFFIC_COMMIT names the build the capture was taken from: a kernel changed since then has a stale entry.
-        # not part of the module's step with the workspaces: the query-major selected forward and dQ, the dK/dV-only call
-        not_in_step = ("sel_fwd", "sel_dq", "sel+swa_dkv(+reverse index)")
-        dom = max((n for n in kern if n in kflops and n not in not_in_step), key=lambda n: kern[n])
+        # DRAM traffic per launch (dram__bytes_read.sum + dram__bytes_write.sum), from one ncu capture of the B=1 slice of this
+        # workload (`--profile-case`), in MB per sequence; traffic grows in proportion to the number of sequences (every
+        # sequence's K/V stays in L2, q/dO/o/dq are streamed once).  NCU_TRAFFIC_COMMIT names the build the capture was taken
+        # from: a kernel changed since then has a stale entry.
+        dom = max((n for n in PARTS if n in kflops), key=lambda n: kern[n])
         # kernels timed alone (three launches back to back): the burst bf16 peak is their denominator
         peak = peaks["tf_burst"]
         kroof = {}
@@ -496,7 +491,7 @@ def run_gpu(args):
         # 16 query rows only, against the rate of the same gather with no arithmetic behind it (nsa_gather_probe)
         visits = keys_per * Bl * Hkv / c["sel_block"]
         gbytes = visits * 2 * c["sel_block"] * D * 2
-        for n in ("sel_fwd", "sel_dq"):
+        for n in ("sel_fwd_query_major", "sel_dq_query_major"):
             kroof[n].update({"pipe": "mma.sync (peak 574 TFLOP/s measured for m16n8k16 bf16)",
                              "frac_of_mma_sync_peak": round(kroof[n]["tflops"] / 574.0, 4),
                              "gather_bytes": gbytes, "gather_tbs": round(gbytes / (kern[n] * 1e-3) / 1e12, 2),
@@ -509,8 +504,6 @@ def run_gpu(args):
                 "traffic": (NCU_MB_PER_SEQ[dom] * 1e6 * Bl) if dom in NCU_MB_PER_SEQ else None,
                 "traffic_source": "ncu capture at B=1 (build %s) x sequences per rank" % NCU_TRAFFIC_COMMIT,
                 "ms_per_launch": round(kern[dom], 3), "algorithmic_flops_per_launch": kflops[dom]}
-        if dom in ("sel_fwd", "sel_dq"):
-            roof.update({k_: v_ for k_, v_ in kroof[dom].items() if k_.startswith(("pipe", "frac_of_", "gather"))})
         cb = None
         if world == 1 and not args.no_cpu:
             cb, _ = cpu_step(1024, 1, 0)
@@ -534,7 +527,8 @@ def run_gpu(args):
                     "d2h_bytes_per_step": d2h_bytes * world, "ms_per_step": ms_e2e,
                     "host_gbs_aggregate": round((h2d_bytes + d2h_bytes) * world / (ms_e2e * 1e-3) / 1e9, 1)},
             "gpu_launches": int(launches[1] - launches[0]),
-            "roofline": roof, "kernels_ms": {n: round(v_, 3) for n, v_ in kern.items()}, "kernel_rooflines": kroof,
+            "roofline": roof, "kernels_ms": {n: round(v_, 3) for n, v_ in kern.items()},
+            "step_calls_ms": round(sum(kern[n] for n in STEP), 3), "kernel_rooflines": kroof,
             "selected_keys_per_seq_kvhead": keys_per, "clocks": clocks, "cpu_baseline": cb, "secondary": secondary,
         }
         print(json.dumps(line))
