@@ -1,8 +1,7 @@
 """Context (sequence) parallelism for NSAAttention: every rank owns a slice of the query tokens of one long
 sequence, K/V are all-gathered over NCCL, and each rank runs the NSA kernels for its queries only.
 
-The reference has no distributed code; this follows the sharding of BASELINE config 4 (B=1, T=65536 split over
-2/4/8 GPUs).  What moves over NVLink per layer:
+The reference has no distributed code.  The case it is made for: one sequence of 65536 tokens over 2, 4 or 8 GPUs.  What moves over NVLink per layer:
   * one all-gather of the rank's K and V tokens (K and V travel as one tensor; Hkv is small: 134 MB in total at T=64K)
     and, in the backward, one reduce-scatter of dK/dV;
   * one all-gather of the compressed K/V (8.4 MB at T=64K): every rank compresses only its own 1/P of the compressed

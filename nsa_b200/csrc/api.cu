@@ -44,10 +44,14 @@ static int check_bs(const char* who, int BS) {
 }
 
 // Shares of a key block's token stream in the key-major backward of the selected branch.  The first blocks are visited
-// most: one CTA per block is enough only when there are six blocks per SM; with fewer a list is shared by two CTAs, or by as many as
-// give every SM two (at most 16; a share then still has some dozens of tokens).  The CTAs of a shared list leave fp32 partials that a
-// second kernel adds in order.  kv_bwd_tc_kernel with 4 KV heads, one CTA a block -> two: 5000 tokens (316 blocks) 647 -> 330 us + 24
-// for the sums, 9000 tokens (564) 854 -> 636 + 24, 14000 tokens (876) 1300 -> 999 + 35, 17000 tokens (1064) 1297 -> 1260 + 43, so not
+// most: one CTA per block is enough only when there are six blocks per SM; with fewer a list is shared by two CTAs, or by as
+// many as
+// give every SM two (at most 16; a share then still has some dozens of tokens).  The CTAs of a shared list leave fp32
+// partials that a
+// second kernel adds in order.  kv_bwd_tc_kernel with 4 KV heads, one CTA a block -> two: 5000 tokens (316 blocks) 647 -> 330
+// us + 24
+// for the sums, 9000 tokens (564) 854 -> 636 + 24, 14000 tokens (876) 1300 -> 999 + 35, 17000 tokens (1064) 1297 -> 1260 +
+// 43, so not
 // there; 2 x 2080 tokens, 2 KV heads (132) three shares 154 us, four 162, five 172, seven 189.
 static int kv_shares(long long blocks) {
   if (blocks <= 0 || blocks >= 6LL * num_sms()) return 1;

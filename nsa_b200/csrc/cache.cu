@@ -105,7 +105,8 @@ int launch_conv_weight(const bf16* w0, const bf16* w1, bf16* o0, bf16* o1, int D
 //   table = [ cu_new (n+1) | new compressed offsets (n+1) | old compressed offsets (n+1) | offsets of the rows to compute
 //             (n+1) | first position to compute (n) | sequences, longest first (n) ]
 //   info  = { compressed rows in all, longest compressed sequence, rows to compute }
-// With cu_old = null everything is new.  Returns 0, s + 1 if sequence s became shorter, or -(s + 1) if more of its positions are in
+// With cu_old = null everything is new.  Returns 0, s + 1 if sequence s became shorter, or -(s + 1) if more of its positions
+// are in
 // the old cache than it has (that cache was built with another block or stride).
 int cache_plan(const int* cu_new, const int* cu_old, const int* cuc_old, int nseq, int block, int stride, int* table, int* info) {
   const int n = nseq;

@@ -243,6 +243,15 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int cod
     }
   }
 }
+// ---- the CTAs of a cluster -----------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t map_cta(uint32_t saddr, uint32_t cta) {   // the same shared-memory address in another CTA
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(cta));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 // The same with a CTA-wide abort flag in shared memory: once any wait of the CTA has given up, every later wait whose phase
 // is not complete returns false at once, so roles that must keep meeting at named barriers can run their loops to the end without
 // waiting (their results are discarded) instead of leaving a partner stuck at a barrier.

@@ -38,15 +38,6 @@ struct Maps {
   CUtensorMap w[2];
 };
 
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t cluster_addr(uint32_t saddr, uint32_t rank) {
-  uint32_t r;
-  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
-  return r;
-}
 __device__ __forceinline__ float4 cluster_ld4(uint32_t addr) {
   float4 v;
   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
@@ -208,7 +199,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const uint32_t addr = sbase + (uint32_t)(r * RS + col) * 4;
         float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
         for (int k = 0; k < ks; ++k) {
-          const float4 v = cluster_ld4(cluster_addr(addr, (uint32_t)k));
+          const float4 v = cluster_ld4(map_cta(addr, (uint32_t)k));
           s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
         }
         if (a.bias[z]) {

@@ -29,7 +29,8 @@
 // time, from a scratch that the CTA's next item uses again (it stays in L2) while the ring fills with that item's tiles; with
 // clusters each CTA its share of the rows, a row and branch per warp.  Measured, 128 sequences of 4096 to 32768 keys: a second
 // kernel that merges (77 MB of partials written and read) 179 us, merged here 170; one
-// sequence of 4096 keys 18.9 us with the second kernel and 17.5 without.  Merging through shared memory, warp after warp, cost seven
+// sequence of 4096 keys 18.9 us with the second kernel and 17.5 without.  Merging through shared memory, warp after warp,
+// cost seven
 // named barriers and six serialised rounds per branch.  No atomics; every wait is bounded.
 #include <algorithm>
 #include <array>
@@ -96,11 +97,6 @@ __device__ __forceinline__ uint32_t cluster_rank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-__device__ __forceinline__ uint32_t map_cta(uint32_t saddr, uint32_t cta) {   // the same shared-memory address in another CTA
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(cta));
-  return r;
-}
 __device__ __forceinline__ void st_cluster(uint32_t addr, float2 v) {
   asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(v.x), "f"(v.y) : "memory");
 }
@@ -127,9 +123,6 @@ __device__ __forceinline__ bool wait_cluster(uint32_t bar, uint32_t parity, int 
     }
   }
 }
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 
 // avg_pool1d(kernel k, stride s, no padding, ceil_mode) output length, as nsa_pool_out_len computes it
 __device__ __forceinline__ int pool_len(int n, int k, int s) {
@@ -147,7 +140,8 @@ __device__ __forceinline__ void pv_tile(float (&acc)[D / 8][4], const float (&sc
   mma_a_b<D, 64>(acc, pf, vbase, PANEL, 0, lane);
 }
 
-// The n blocks with the highest pooled score (ties to the lower index), in order, by one warp: lane l holds the blocks l + 32 e as
+// The n blocks with the highest pooled score (ties to the lower index), in order, by one warp: lane l holds the blocks l + 32
+// e as
 // integers that order like the scores.  The n-th highest is found bit by bit, from the first bit in which the scores differ: a
 // lane counts its own and one warp reduction adds.  The n survivors are ranked among themselves.  (A chain, on which the loads of
 // the selected blocks wait; 16 of 512 blocks.  Counting by ballots from the highest bit 8800 cycles, n rounds of a shared-memory
@@ -285,7 +279,8 @@ __device__ __forceinline__ void online_pair(float (&acc)[D / 8][4], float (&m_ru
 }
 
 // One row and branch of an item that a cluster shared: the partials of all its warps merged in a fixed order (CTA by CTA, warp by
-// warp), by one warp, a lane holding four channels.  Branch order in the workspace: 0 compressed, 1 selected, 2 window.  Warps that
+// warp), by one warp, a lane holding four channels.  Branch order in the workspace: 0 compressed, 1 selected, 2 window.
+// Warps that
 // had no tile are left out.  The first loads are under way while the weights are formed.  Returns the output as rounded.
 static_assert(kMaxCluster * kCons <= 64, "two partials per lane below");
 __device__ __forceinline__ float4 merge_row(const DecodeArgs& a, int item, long long qrow, int r, int br, int nw, int lane) {

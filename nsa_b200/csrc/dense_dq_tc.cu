@@ -12,7 +12,8 @@
 //
 // Bound: the MMAs, 24 per tile at about 90 cycles (an SS product of this shape reads 8 KB of shared memory, 64 cycles' worth),
 // 2050 cycles per tile; the soft-max takes about 1500.  So nothing may make the tensor core wait: the next tile's S and dP are
-// issued each as soon as this tile's is in registers (P is formed while dP is still being computed); dS in tensor memory leaves room for a third K slot (with two stages of
+// issued each as soon as this tile's is in registers (P is formed while dP is still being computed); dS in tensor memory
+// leaves room for a third K slot (with two stages of
 // K and V together a stage came back 2500 cycles after its dQ, 3700 per tile); Q and dO of the next item load as soon as the
 // last S and dP have read them; the epilogue has its own four warps.
 #include "kernels.h"
@@ -60,24 +61,6 @@ __device__ __forceinline__ Sched make_sched(const DenseArgs& a, const SeqTile& s
 struct Maps {
   CUtensorMap q, dout, k, v, ck, cv;
 };
-
-// The 16-byte pieces x[0..7] of the eight lanes of a group are a matrix, lane = row: transposed in place (its own inverse).
-__device__ __forceinline__ void transpose8(uint4 (&x)[8], int lane) {
-#pragma unroll
-  for (int b = 1; b < 8; b <<= 1) {
-    const bool up = (lane & b) != 0;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      if (i & b) continue;
-      uint4 send = up ? x[i] : x[i | b];
-      send.x = __shfl_xor_sync(0xffffffffu, send.x, b);
-      send.y = __shfl_xor_sync(0xffffffffu, send.y, b);
-      send.z = __shfl_xor_sync(0xffffffffu, send.z, b);
-      send.w = __shfl_xor_sync(0xffffffffu, send.w, b);
-      if (up) x[i] = send; else x[i | b] = send;
-    }
-  }
-}
 
 template <int D, bool WIN, bool CMP>
 __global__ void __launch_bounds__(kThreads, 1)

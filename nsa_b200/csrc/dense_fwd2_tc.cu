@@ -255,7 +255,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int tl = row >> 4, head = row & 15;
     const uint32_t lane_addr = (uint32_t)(32 * quad) << 16;
     const uint32_t s_col = tmem + lane_addr + g * 128, o_col = tmem + lane_addr + 256 + g * 128;
-    // (head_dim 64 takes scales of any sign, as it did on mma.sync: negative ones by negating the scores, zero as nearly so, since
+    // (head_dim 64 takes scales of any sign, as it did on mma.sync: negative ones by negating the scores, zero as nearly so,
+    // since
     // masked scores are -inf)
     const bool neg = D == 64 && a.scale < 0.f;
     const float sl2 = (D == 128 ? a.scale : a.scale == 0.f ? 1e-30f : fabsf(a.scale)) * kLog2e;

@@ -99,24 +99,6 @@ __device__ __forceinline__ bool decode_item(const DenseKvArgs& a, Item& it) {
   return true;
 }
 
-// The 16-byte pieces x[0..7] of the eight lanes of a group are a matrix, lane = row: transposed in place.
-__device__ __forceinline__ void transpose8(float4 (&x)[8], int lane) {
-#pragma unroll
-  for (int b = 1; b < 8; b <<= 1) {
-    const bool up = (lane & b) != 0;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      if (i & b) continue;
-      float4 send = up ? x[i] : x[i | b];
-      send.x = __shfl_xor_sync(0xffffffffu, send.x, b);
-      send.y = __shfl_xor_sync(0xffffffffu, send.y, b);
-      send.z = __shfl_xor_sync(0xffffffffu, send.z, b);
-      send.w = __shfl_xor_sync(0xffffffffu, send.w, b);
-      if (up) x[i] = send; else x[i | b] = send;
-    }
-  }
-}
-
 template <int D, bool BYSEQ>   // BYSEQ: the query rows come by sequence (see launch)
 __global__ void __launch_bounds__(kThreads, 1)
     dense_kv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
@@ -483,7 +465,8 @@ __global__ void __launch_bounds__(256) dense_kv_reduce_kernel(const DenseKvArgs 
 template <int D>
 int launch(const DenseKvArgs& a, cudaStream_t s) {
   CUtensorMap tmQ, tmDO, tmK, tmV;
-  // Where a sequence's last tile of query rows reaches into the next sequence, rows come by sequence and those past the end are zeros:
+  // Where a sequence's last tile of query rows reaches into the next sequence, rows come by sequence and those past the end
+  // are zeros:
   // they enter the products over the rows with P = 0, and the next sequence's dO or Q there could be NaN or infinite.  (Not
   // everywhere: the fourth coordinate costs 4 % of the kernel, 65536 tokens 9.9 -> 10.3 ms; a branch in the loop 1 %.)
   const bool by_seq = a.seq.B > 1 && a.seq.Tq % kTok != 0;

@@ -369,7 +369,8 @@ struct GateAdd {
   const bf16* dg[3];    // gradients of the gates [B,Tq,Hq]
   const bf16* w;        // gate projection [3,D], or null: nothing to add
 };
-// dq[(b,t), 16-head group] (+)= sum_g dg_g W_g + scale * sum over the valid slots s of part[(b,h) list position inv[row,s]] (fixed slot
+// dq[(b,t), 16-head group] (+)= sum_g dg_g W_g + scale * sum over the valid slots s of part[(b,h) list position inv[row,s]]
+// (fixed slot
 // order).  part holds one [16 heads x D] bf16 tile per (list position, 16-head sub-group), written by the kv-major
 // backward; dq rows of a (token, group) are the same contiguous tile.
 int launch_sel_dq_reduce(const RevArgs& a, const bf16* part, bf16* dq, int Hq, int D, const GateAdd& gate, float scale, int accumulate,

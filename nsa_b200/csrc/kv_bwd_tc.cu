@@ -12,10 +12,11 @@
 // shuffles; warps 2-5 take key columns 0-31, warps 6-9 columns 32-63 of the same TMEM lanes): they read S and dP
 // from TMEM, form P and dS = P (g dP - delta), and store both as bf16 tiles.
 // The MMA threads issue S/dP of batch n+1 before dV/dK of batch n, so the tensor core works while the soft-max
-// warps compute; the exponentials start when S alone is there, dV when P alone is written.  dV^T and dK^T stay in TMEM for the CTA's whole token stream and are stored once.
+// warps compute; the exponentials start when S alone is there, dV when P alone is written.  dV^T and dK^T stay in TMEM for
+// the CTA's whole token stream and are stored once.
 // Optionally dQ comes out of this kernel too: dS of a batch is already in shared memory,
 // so one more product  dQ_part[128 rows x 128 d] = dS . K  (A = dS K-major, B = K MN-major, a third accumulator in TMEM)
-// gives the batch's contribution to dQ, which the soft-max warps store as bf16 tiles indexed by the batch's positions
+// gives the batch's contribution to dQ, which the drain warps store as bf16 tiles indexed by the batch's positions
 // in the reverse-index list; a small kernel later sums every token's tiles in slot order.  That replaces the
 // query-major dQ kernel, which gathers every selected block again (32 KB per visit for 16 rows) and recomputes S and dP.
 // Every wait is bounded; on a time-out the role records an error and leaves its loop.

@@ -380,7 +380,8 @@ __global__ void __launch_bounds__(kThreads, 1)
           if ((lane & 15) == 8 && i + hh > 0) p0[-1] += v[0];
         }
       }
-      // Causal scores: behind the item's last visible key lies what the slot held before, and every score is zero.  (Cleared here and
+      // Causal scores: behind the item's last visible key lies what the slot held before, and every score is zero.  (Cleared
+      // here and
       // not by the warp that reads them: that took 3 % of the kernel in the other mode too.)
       if (causal) {
         const int n_pool = pool_len_54(st.Tc);

@@ -229,8 +229,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       fence_proxy_async();
       mbar_arrive(stg_full);
       if (warp == kDrainWarp) {
-        // one 4 KB bulk store per token, issued by eight lanes at once: a single 32 KB store is read out of shared
-        // memory at about 20 bytes per cycle, which made this read-out the kernel's bottleneck
+        // one 32 KB bulk store (the tokens' tiles are contiguous), or one of 4 KB per token where the KV head has several
+        // 16-head groups.  Eight 4 KB stores by eight lanes were no faster than the one (4.31 against 4.20 ms)
         bool good = mbar_wait(stg_full, n & 1, DEV_ERR_FULL_WAIT);
         const int nvalid = min(kTokB, nA - mloc * kTokB);
         if (good && G16 == 1 && lane == 0 && nvalid > 0) {
@@ -480,10 +480,14 @@ int launch_sel_fwd_kv(const SelKvArgs& a, const RevArgs& r, cudaStream_t s) {
   cudaError_t e = cudaFuncSetAttribute(sel_fwd_kv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
   if (e != cudaSuccess) return (int)e;
   // The first block is visible to every token, the last to few: with few blocks per SM the first one's CTA would be the last to
-  // end.  Up to eight CTAs then share a block's list, so that there are three or more per SM, or at least two CTAs up to six blocks per SM (a visit's results have a place of
-  // their own, nothing is added up; a CTA's start and end cost about two batches).  One sequence of 5003 tokens, 4 KV heads: 245 us
-  // with one CTA a block, 160 / 159 / 169 / 177 with 3 / 4 / 6 / 8 per SM; 2 x 2080 tokens, 2 KV heads: 140, then 76 / 80 / 88 / 89.
-  // Two CTAs a block, 4 KV heads: 9000 tokens (564 blocks) 374 -> 308, 14000 tokens (876) 557 -> 494, 17000 tokens (1064) 559 -> 616.
+  // end.  Up to eight CTAs then share a block's list, so that there are three or more per SM, or at least two CTAs up to six
+  // blocks per SM (a visit's results have a place of
+  // their own, nothing is added up; a CTA's start and end cost about two batches).  One sequence of 5003 tokens, 4 KV heads:
+  // 245 us
+  // with one CTA a block, 160 / 159 / 169 / 177 with 3 / 4 / 6 / 8 per SM; 2 x 2080 tokens, 2 KV heads: 140, then 76 / 80 /
+  // 88 / 89.
+  // Two CTAs a block, 4 KV heads: 9000 tokens (564 blocks) 374 -> 308, 14000 tokens (876) 557 -> 494, 17000 tokens (1064) 559
+  // -> 616.
   const long long blocks = (long long)a.B * a.Hk * ((a.T + 63) / 64), want = 3LL * num_sms();
   if (blocks <= 0) return 0;
   const int nshare = blocks >= 2 * want ? 1 : (int)std::max(2LL, std::min(8LL, (want + blocks - 1) / blocks));

@@ -139,6 +139,26 @@ __device__ __forceinline__ float max3f(float a, float b, float c) {
   return r;
 }
 
+// The 16-byte pieces x[0..7] (uint4, float4) of the eight lanes of a group are a matrix, lane = row: transposed in place (its own
+// inverse).
+template <typename V>
+__device__ __forceinline__ void transpose8(V (&x)[8], int lane) {
+#pragma unroll
+  for (int b = 1; b < 8; b <<= 1) {
+    const bool up = (lane & b) != 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if (i & b) continue;
+      V send = up ? x[i] : x[i | b];
+      send.x = __shfl_xor_sync(0xffffffffu, send.x, b);
+      send.y = __shfl_xor_sync(0xffffffffu, send.y, b);
+      send.z = __shfl_xor_sync(0xffffffffu, send.z, b);
+      send.w = __shfl_xor_sync(0xffffffffu, send.w, b);
+      if (up) x[i] = send; else x[i | b] = send;
+    }
+  }
+}
+
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* tm, uint32_t bar, int c0, int c1, int c2) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst),

@@ -101,13 +101,13 @@ def test_the_compressor_is_called_where_that_shows(lens, mode):
     for name, a, b in zip(names, hooked, plain):
         if name != "compressor.compressor_k.bias":   # zero but for roundings
             # both round to bf16 on the way, the composed form up to twice as often: 2e-3 apart, the gates' bias (a sum that nearly cancels) 2e-2
-            assert float((a - b).float().norm() / b.float().norm()) < (3e-2 if name == "gating.bias" else 8e-3), name
+            assert float((a - b).detach().float().norm() / b.detach().float().norm()) < (3e-2 if name == "gating.bias" else 8e-3), name
     mod.compressor = _Scaled(mod.compressor)
     with torch.no_grad():
         mod.gating.weight[2] /= 2
         mod.gating.bias[2] /= 2
     doubled = run()
-    assert float((doubled[0] - plain[0]).float().norm() / plain[0].float().norm()) < 8e-3
+    assert float((doubled[0] - plain[0]).detach().float().norm() / plain[0].detach().float().norm()) < 8e-3
 
 
 @pytest.mark.parametrize("D", [64, 128])
