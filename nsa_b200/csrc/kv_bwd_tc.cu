@@ -8,8 +8,8 @@
 //     dP  [128 rows x 64 keys] = dOg . V^T         A = dOg (K-major), B = V  (K-major)
 //     dV^T[128 d    x 64 keys] += dOg^T . (g P)    A = dOg (MN-major), B = P  (MN-major, written by the soft-max warps)
 //     dK^T[128 d    x 64 keys] += Qg^T . dS        A = Qg (MN-major),  B = dS (MN-major)
-// Eight soft-max warps own half a row per thread (lse, delta, gate and the causal mask are thread-local, no
-// shuffles; warps 2-5 take key columns 0-31, warps 6-9 columns 32-63 of the same TMEM lanes): they read S and dP
+// Eight soft-max warps own half a row per thread (warps 4-7 take key columns 0-31, warps 8-11 columns 32-63 of the same TMEM
+// lanes; a row's lse, delta, gate and number of visible keys lie in shared memory): they read S and dP
 // from TMEM, form P and dS = P (g dP - delta), and store both as bf16 tiles.
 // The MMA threads issue S/dP of batch n+1 before dV/dK of batch n, so the tensor core works while the soft-max
 // warps compute; the exponentials start when S alone is there, dV when P alone is written.  dV^T and dK^T stay in TMEM for
@@ -19,6 +19,12 @@
 // gives the batch's contribution to dQ, which the drain warps store as bf16 tiles indexed by the batch's positions
 // in the reverse-index list; a small kernel later sums every token's tiles in slot order.  That replaces the
 // query-major dQ kernel, which gathers every selected block again (32 KB per visit for 16 rows) and recomputes S and dP.
+//
+// Bound: the round trip of the two Q/dO stages (gather 1800 cycles, S, soft-max, dV and dK: 3650 cycles per batch) and shared
+// memory (3100 cycles of operands, arriving rows and stores).  Before, the soft-max warps were busy 3500 of 4070 cycles: each fetched
+// and addressed its row's lse, delta and gate (now the drain warps, once per row), divided by the batch count, did its arithmetic in
+// three unrolled variants (now one, two columns at a time), and the unrolled epilogue cost another 55 000 cycles a CTA.
+// 8 x 8192 tokens, 64 heads: 4.90 -> 4.08 ms; 65536 tokens: 5.0 -> 4.1; 2 x 2080 tokens, 32 heads: 153 -> 129 us.
 // Every wait is bounded; on a time-out the role records an error and leaves its loop.
 #include "kernels.h"
 #include "tc.cuh"
@@ -48,33 +54,41 @@ constexpr uint32_t Q_TILE = 128 * 256;     // 32 KB: [16 row groups][2 column pa
 constexpr uint32_t STAGE = 2 * Q_TILE;     // Q + dO
 constexpr uint32_t P_TILE = 128 * 128;     // [128 rows][64 keys]
 constexpr int kStages = 2;
-constexpr uint32_t kSmem = 2 * KV_TILE + kStages * STAGE + 4 * P_TILE + 256 + 1024;
+// K, V | Q and dO stages | two P/dS pairs | barriers | a batch's row data
+constexpr uint32_t kOffBar = 2 * KV_TILE + kStages * STAGE + 4 * P_TILE, kOffRow = kOffBar + 256, kSmem = kOffRow + 128 * 16;   // no room to align
 constexpr uint32_t kTmemCols = 512;        // two S/dP buffers: S 0..63, dP 64..127 | 128..255; dV^T 256..319, dK^T 320..383
 constexpr uint32_t kColDV = 256, kColDK = 320, kColDQ = 384;   // dQ_part: 384..511
 
 __global__ void __launch_bounds__(kThreads, 1)
     kv_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
                      const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const KvArgs a) {
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t raw = smem_u32(smem_raw);
-  const uint32_t sbase = (raw + 1023u) & ~1023u;
-  uint8_t* sgen = smem_raw + (sbase - raw);
+  extern __shared__ __align__(1024) uint8_t kv_bwd_smem[];
+  uint8_t* const sgen = kv_bwd_smem;
+  const uint32_t sbase = smem_u32(kv_bwd_smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (sbase & 1023u) {   // the 128-byte swizzle repeats every 1024 bytes
+    if (threadIdx.x == 0) atomicCAS(&g_dev_error, 0, 330);
+    return;
+  }
   const uint32_t k_s = sbase, v_s = sbase + KV_TILE;
   const uint32_t ring = sbase + 2 * KV_TILE;
   const uint32_t p_s0 = ring + kStages * STAGE;   // two [P | dS] tile pairs
-  const uint32_t bar_base = p_s0 + 4 * P_TILE;
+  const uint32_t bar_base = sbase + kOffBar;
   // barriers
   // sdp_* and pds_* exist twice (index = batch & 1): S/dP of batch n+1 are computed while the soft-max warps still
   // hold batch n, and P/dS of batch n+1 are written while dV/dK of batch n still read theirs
-  const uint32_t full0 = bar_base, empty0 = bar_base + 16, kv_bar = bar_base + 32, sdp_full = bar_base + 40,
+  // q* and do* by stage: Q is held until dK, dO until dP and dV
+  const uint32_t qfull0 = bar_base, qempty0 = bar_base + 16, dofull0 = bar_base + 192, doempty0 = bar_base + 208, kv_bar = bar_base + 32, sdp_full = bar_base + 40,
                  sdp_free = bar_base + 56, pds_full = bar_base + 72, pds_free = bar_base + 88, acc_full = bar_base + 104,
-                 tmem_slot = bar_base + 112, dq_full = bar_base + 120, dq_free = bar_base + 128, stg_full = bar_base + 136,
-                 stg_free = bar_base + 144, s_full = bar_base + 160, p_full = bar_base + 176;   // stg_free: two barriers, one per P/dS pair
+                 tmem_slot = bar_base + 112, dq_full = bar_base + 120, dq_free = bar_base + 128, stg_full = bar_base + 240,
+                 stg_free = bar_base + 144, s_full = bar_base + 160, p_full = bar_base + 176,
+                 row_full = bar_base + 224, row_empty = bar_base + 232;   // stg_full, stg_free: one per P/dS pair
   if (threadIdx.x == 0) {
     for (int i = 0; i < kStages; ++i) {
-      mbar_init(full0 + 8 * i, kProd);
-      mbar_init(empty0 + 8 * i, 1);
+      mbar_init(qfull0 + 8 * i, 1);
+      mbar_init(qempty0 + 8 * i, 1);
+      mbar_init(dofull0 + 8 * i, 1);
+      mbar_init(doempty0 + 8 * i, 2);
     }
     mbar_init(kv_bar, 1);
     for (int i = 0; i < 2; ++i) {
@@ -86,9 +100,12 @@ __global__ void __launch_bounds__(kThreads, 1)
       mbar_init(pds_free + 8 * i, 1);
     }
     mbar_init(acc_full, 1);
+    mbar_init(row_full, kDrainThreads);
+    mbar_init(row_empty, kSoftThreads);
     mbar_init(dq_full, 1);
     mbar_init(dq_free, kDrainThreads);
     mbar_init(stg_full, kDrainThreads);
+    mbar_init(stg_full + 8, kDrainThreads);
     mbar_init(stg_free, 1);
     mbar_init(stg_free + 8, 1);
     fence_mbar_init();
@@ -143,11 +160,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         tma_load_4d(v_s + p * KV_PANEL, &tmV, kv_bar, p * 64, hk, key0, b);
       }
     }
-    const int x = kProd * lane + warp;          // this lane's box of every batch (none if >= 16)
-    const bool has = x < 2 * kTokB;
-    const int bj = x & 7, bwhich = x >> 3;
-    const int nmine = 2 * kTokB / kProd;   // boxes this warp issues per batch
-    auto batch_token = [&](int n) { return n >= nb || !has ? 0 : list_token(n % nb_sub * kTokB + bj); };
+    const bool has = lane < kTokB;
+    const uint32_t full0 = warp ? dofull0 : qfull0, empty0 = warp ? doempty0 : qempty0, dst0 = ring + (warp ? Q_TILE : 0);
+    const CUtensorMap* const tm = warp ? &tmDO : &tmQ;
+    auto batch_token = [&](int n) { return n >= nb || !has ? 0 : list_token(n % nb_sub * kTokB + lane); };
     int tk_next = batch_token(0);
     for (int n = 0; n < nb; ++n) {
       const int tk = tk_next;
@@ -159,13 +175,12 @@ __global__ void __launch_bounds__(kThreads, 1)
       int good = 1;
       if (lane == 0) {
         good = mbar_wait(empty0 + 8 * stage, ph ^ 1, DEV_ERR_EMPTY_WAIT) ? 1 : 0;
-        if (good) mbar_expect_tx(fb, nmine * 4096);
+        if (good) mbar_expect_tx(fb, Q_TILE);
       }
       if (!__shfl_sync(0xffffffffu, good, 0)) break;
       if (has) {
-        const uint32_t q_s = ring + stage * STAGE, do_s = q_s + Q_TILE;
         const int qrow = (int)(((long long)b * a.Tq + (tk - a.q0)) * a.Hq + hg * 16);
-        tma_load_4d((bwhich ? do_s : q_s) + bj * 4096, bwhich ? &tmDO : &tmQ, fb, 0, 0, 0, qrow >> 3);
+        tma_load_4d(dst0 + stage * STAGE + lane * 4096, tm, fb, 0, 0, 0, qrow >> 3);
       }
     }
   } else if (warp == kMmaWarp) {
@@ -184,7 +199,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         dDOk[i] = umma_smem_desc(do_s, 0, 2048);
       }
       for (int n = 0; ok && n < nb; ++n) {
-        ok = mbar_wait(full0 + 8 * (n % kStages), (n / kStages) & 1, DEV_ERR_FULL_WAIT);
+        ok = mbar_wait(qfull0 + 8 * (n % kStages), (n / kStages) & 1, DEV_ERR_FULL_WAIT);
         if (ok && n >= 2) ok = mbar_wait(sdp_free + 8 * (n & 1), ((n >> 1) - 1) & 1, DEV_ERR_EMPTY_WAIT);
         if (!ok) break;
         tc_fence_after();
@@ -196,12 +211,16 @@ __global__ void __launch_bounds__(kThreads, 1)
           umma_ss(tmem + col, umma_desc_advance(aq, aoff), umma_desc_advance(dK, boff), idesc_kk, ks ? 1u : 0u);
         }
         umma_commit(s_full + 8 * (n & 1));   // the exponentials need S alone
+        ok = mbar_wait(dofull0 + 8 * (n % kStages), (n / kStages) & 1, DEV_ERR_FULL_WAIT);
+        if (!ok) break;
+        tc_fence_after();
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
           const uint32_t aoff = (ks >> 2) * 1024 + (ks & 3) * 32, boff = (ks >> 2) * KV_PANEL + (ks & 3) * 32;
           umma_ss(tmem + col + 64, umma_desc_advance(ado, aoff), umma_desc_advance(dV, boff), idesc_kk, ks ? 1u : 0u);
         }
         umma_commit(sdp_full + 8 * (n & 1));
+        umma_commit(doempty0 + 8 * (n % kStages));
       }
     }
   } else if (warp == kMma2Warp) {
@@ -225,7 +244,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       const uint64_t dKmn = umma_smem_desc(k_s, KV_PANEL, 1024);
       for (int n = 0; ok && n < nb; ++n) {
-        ok = mbar_wait(p_full + 8 * (n & 1), (n >> 1) & 1, DEV_ERR_FULL_WAIT);
+        ok = mbar_wait(dofull0 + 8 * (n % kStages), (n / kStages) & 1, DEV_ERR_FULL_WAIT) &&
+             mbar_wait(p_full + 8 * (n & 1), (n >> 1) & 1, DEV_ERR_FULL_WAIT);
         if (!ok) break;
         tc_fence_after();
         const uint64_t aq = (n % kStages) ? dQmn[1] : dQmn[0], ado = (n % kStages) ? dDOmn[1] : dDOmn[0];
@@ -233,13 +253,14 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)   // contraction over the 128 rows, 16 per step; dV while the soft-max warps form dS
           umma_ss(tmem + kColDV, umma_desc_advance(ado, ks * 4096), umma_desc_advance(bp, ks * 2048), idesc_mn, (n | ks) ? 1u : 0u);
+        umma_commit(doempty0 + 8 * (n % kStages));
         ok = mbar_wait(pds_full + 8 * (n & 1), (n >> 1) & 1, DEV_ERR_FULL_WAIT);
         if (!ok) break;
         tc_fence_after();
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)
           umma_ss(tmem + kColDK, umma_desc_advance(aq, ks * 4096), umma_desc_advance(bds, ks * 2048), idesc_mn, (n | ks) ? 1u : 0u);
-        umma_commit(empty0 + 8 * (n % kStages));
+        umma_commit(qempty0 + 8 * (n % kStages));
         if (emit_dq) {
           // the previous partial must have been read out of its accumulator by the drain warps
           if (n > 0) ok = mbar_wait(dq_free, (n - 1) & 1, DEV_ERR_EMPTY_WAIT);
@@ -268,13 +289,48 @@ __global__ void __launch_bounds__(kThreads, 1)
     // row & 7 == head & 7, and the reduction kernel undoes it).  Plain stores from the accumulator's layout (a thread
     // owns a row: 16 bytes per lane at a 256-byte stride) cost a tenth of the kernel in store wavefronts, and reading
     // the partials out in the soft-max warps delayed the next batch's soft-max.
-    if (emit_dq) {
+    // Before that, the thread's row of the batch after next: what the soft-max warps need to know of it (the two that share a row
+    // would each fetch and address it themselves, a quarter of their time).
+    {
       const int quad = warp & 3;
       const int row = 32 * quad + lane;
+      const int j = row >> 4;
       const uint32_t lane_addr = (uint32_t)(32 * quad) << 16;
       const bool elected = warp == kDrainWarp && lane == 0;
-      bool ok = true;
+      const long long head0 = (long long)b * a.Tq * a.Hq + hk * G16 * 16 + (row & 15);
+      float4* const row_s = reinterpret_cast<float4*>(sgen + kOffRow) + row;
+      // batch to be fetched next: place in its 16-head sub-group, sub-group; its token (two batches ahead of the publication)
+      int fm = 0, fsub = 0, ft = nA > 0 ? list_token(j) : 0;
+      float lse = 0.f, del = 0.f;
+      bf16 g = __float2bfloat16(1.f);
+      int nv = 0;
+      auto fetch = [&](int n) {   // row data of batch n, kept as loaded: converting them would wait for the loads
+        if (n >= nb) return;
+        const long long qrow = head0 + (long long)(ft - a.q0) * a.Hq + fsub * 16;
+        lse = a.lse[qrow];
+        del = a.delta[qrow];
+        if (a.gate) g = a.gate[qrow];
+        nv = fm * kTokB + j < nA ? min(64, ft - key0 + 1) : 0;   // keys that the row sees (the block's first at least)
+        if (++fm == nb_sub) {
+          fm = 0;
+          ++fsub;
+        }
+        ft = list_token(fm * kTokB + j);
+      };
+      auto publish = [&](int n) {
+        if (n >= nb) return true;
+        if (n > 0 && !mbar_wait(row_empty, (n - 1) & 1, DEV_ERR_EMPTY_WAIT)) return false;
+        const uint32_t gn = (uint32_t)__bfloat16_as_ushort(g) << 16 | (lse > -INFINITY ? nv : 0);   // (a row that sees nothing: none)
+        *row_s = make_float4(-lse * kLog2e, -del, __uint_as_float(gn), 0.f);
+        mbar_arrive(row_full);
+        fetch(n + 1);
+        return true;
+      };
+      fetch(0);
+      bool ok = publish(0) && publish(1);
       for (int n = 0; ok && n < nb; ++n) {
+        ok = publish(n + 2);
+        if (!ok || !emit_dq) continue;
         const int sub = n / nb_sub, mloc = n % nb_sub;
         ok = mbar_wait(dq_full, n & 1, DEV_ERR_FULL_WAIT);
         if (!ok) break;
@@ -303,9 +359,9 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
         }
         fence_proxy_async();
-        mbar_arrive(stg_full);
+        mbar_arrive(stg_full + 8 * (n & 1));   // (two: a warp may be a batch ahead of the slowest)
         if (elected) {
-          ok = mbar_wait(stg_full, n & 1, DEV_ERR_FULL_WAIT);
+          ok = mbar_wait(stg_full + 8 * (n & 1), (n >> 1) & 1, DEV_ERR_FULL_WAIT);
           const int nvalid = min(kTokB, nA - mloc * kTokB);
           if (ok && nvalid > 0) {
             bf16* dst = a.dq_part + (((long long)bh * a.rev_cap + lo + mloc * kTokB) * G16 + sub) * (16 * D);
@@ -331,85 +387,57 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int quad = warp & 3;
     const int half = (warp - kSoftWarp) >> 2;    // which 32 key columns this thread owns
     const int row = 32 * quad + lane;           // TMEM lane == tile row
-    const int j = row >> 4, head = row & 15;
     const uint32_t lane_addr = (uint32_t)(32 * quad) << 16;
     const float sl2 = a.scale * kLog2e;
     bool ok = true;
-    // per-row operands are fetched one batch ahead (token ids two ahead) so their latency hides behind the MMAs; they are kept
-    // as loaded, since converting them would wait for the loads
-    struct RowInfo {
-      int t;
-      bool live;
-      float lse, del;
-      bf16 g;
-    };
-    auto row_token = [&](int n, bool& live) {
-      live = false;
-      if (n >= nb) return 0;
-      const int i = n % nb_sub * kTokB + j;
-      live = i < nA;
-      return list_token(i);
-    };
-    auto row_load = [&](int n, int t, bool live) {
-      RowInfo r = {t, live, 0.f, 0.f, __float2bfloat16(1.f)};
-      if (n < nb) {
-        const long long qrow = ((long long)b * a.Tq + (t - a.q0)) * a.Hq + (hk * G16 + n / nb_sub) * 16 + head;
-        r.lse = a.lse[qrow];
-        r.del = a.delta[qrow];
-        if (a.gate) r.g = a.gate[qrow];
-      }
-      return r;
-    };
     // With dQ partials: the drain warps stage the partial of batch n in that batch's own P/dS pair; the pair is written again
     // for batch n+2 only after their bulk store has read it (stg_free of that pair).
-    bool live1;
-    int t1 = row_token(0, live1);
-    RowInfo cur = row_load(0, t1, live1);
-    t1 = row_token(1, live1);
+    const uint64_t sl22 = pack_f32x2(sl2, sl2);
+    uint8_t* const prow0 = sgen + (p_s0 - sbase) + row * 128;
+    const float4* const row_s = reinterpret_cast<const float4*>(sgen + kOffRow) + row;
     for (int n = 0; ok && n < nb; ++n) {
-      const RowInfo ri = cur;
-      cur = row_load(n + 1, t1, live1);     // operands of batch n+1
-      t1 = row_token(n + 2, live1);         // token id of batch n+2
-      const int t = ri.t;
-      const bool live = ri.live;
-
+      ok = mbar_wait(row_full, n & 1, DEV_ERR_FULL_WAIT);
+      if (!ok) break;
+      const float4 ri = *row_s;
+      mbar_arrive(row_empty);
       const uint32_t buf = n & 1, use = n >> 1;
-      const uint32_t tcol = buf * 128;
+      const uint32_t scol = tmem + lane_addr + buf * 128 + half * 32;
       ok = mbar_wait(s_full + 8 * buf, use & 1, DEV_ERR_FULL_WAIT);
       if (!ok) break;
       tc_fence_after();
       float p[32];
-      uint32_t pw[16];   // 32 bf16
-      tmem_ld16(tmem + lane_addr + tcol + half * 32, *reinterpret_cast<float(*)[16]>(&p[0]));
-      tmem_ld16(tmem + lane_addr + tcol + half * 32 + 16, *reinterpret_cast<float(*)[16]>(&p[16]));
+      tmem_ld32(scol, p);
+      const uint32_t gn = __float_as_uint(ri.z);
+      const float gv = __uint_as_float(gn & 0xffff0000u);
+      const int nrow = gn & 0xffff, nvis = nrow - 32 * half;   // visible keys of the block, of this half (0: a row that is not there)
+      const uint64_t nl2 = pack_f32x2(ri.x, ri.x), g2 = pack_f32x2(gv, gv), nd2 = pack_f32x2(ri.y, ri.y);
       tmem_ld_wait();
-      const int kfirst = key0 + half * 32, klast = kfirst + 31;
-      const float lse2 = ri.lse * kLog2e, del = ri.del, gv = __bfloat162float(ri.g);
-      const bool dead = !live || !(lse2 > -INFINITY);
-      if (dead) {
 #pragma unroll
-        for (int e = 0; e < 32; ++e) p[e] = 0.f;
-      } else if (klast <= t) {
-        const float nl = -lse2;
-#pragma unroll
-        for (int e = 0; e < 32; ++e) p[e] = ex2(fmaf(p[e], sl2, nl));
-      } else {
-#pragma unroll
-        for (int e = 0; e < 32; ++e) p[e] = kfirst + e <= t ? ex2(p[e] * sl2 - lse2) : 0.f;
+      for (int e = 0; e < 32; e += 2) {
+        const uint64_t x = fma_f32x2(pack_f32x2(p[e], p[e + 1]), sl22, nl2);
+        p[e] = lo_f32x2(x);
+        p[e + 1] = hi_f32x2(x);
       }
+      if (nvis < 32) {
 #pragma unroll
-      for (int e = 0; e < 32; e += 2) pw[e / 2] = pack_bf16(p[e] * gv, p[e + 1] * gv);
+        for (int e = 0; e < 32; ++e) p[e] = e < nvis ? p[e] : -INFINITY;
+      }
+      uint32_t pw[16];   // 32 bf16
+#pragma unroll
+      for (int e = 0; e < 32; e += 2) {
+        p[e] = ex2(p[e]);
+        p[e + 1] = ex2(p[e + 1]);
+        const uint64_t gp = mul_f32x2(g2, pack_f32x2(p[e], p[e + 1]));
+        pw[e / 2] = pack_bf16(lo_f32x2(gp), hi_f32x2(gp));
+      }
+      // dV/dK of batch n-2 have read this pair, and the bulk stores of its dQ partial
       if (n >= 2) {
-        ok = mbar_wait(pds_free + 8 * buf, (use - 1) & 1, DEV_ERR_EMPTY_WAIT);   // dV/dK of batch n-2 have read this pair
-        if (!ok) break;
-      }
-      if (emit_dq && n >= 2) {
-        ok = mbar_wait(stg_free + 8 * buf, (use - 1) & 1, DEV_ERR_EMPTY_WAIT);
+        ok = mbar_wait(pds_free + 8 * buf, (use - 1) & 1, DEV_ERR_EMPTY_WAIT);
+        if (ok && emit_dq) ok = mbar_wait(stg_free + 8 * buf, (use - 1) & 1, DEV_ERR_EMPTY_WAIT);
         if (!ok) break;
       }
       // this thread's half of row `row` of the [128 x 64] bf16 tiles: 4 chunks of 16 bytes at swizzled positions
-      uint8_t* prow = sgen + (p_s0 - sbase) + buf * 2 * P_TILE + row * 128;
-      uint8_t* drow = prow + P_TILE;
+      uint8_t* const prow = prow0 + buf * 2 * P_TILE;
 #pragma unroll
       for (int c = 0; c < 4; ++c)
         *reinterpret_cast<uint4*>(prow + ((4 * half + c) ^ (row & 7)) * 16) = make_uint4(pw[4 * c], pw[4 * c + 1], pw[4 * c + 2], pw[4 * c + 3]);
@@ -419,61 +447,67 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (!ok) break;
       tc_fence_after();
       float dpv[32];
-      tmem_ld16(tmem + lane_addr + tcol + 64 + half * 32, *reinterpret_cast<float(*)[16]>(&dpv[0]));
-      tmem_ld16(tmem + lane_addr + tcol + 64 + half * 32 + 16, *reinterpret_cast<float(*)[16]>(&dpv[16]));
+      tmem_ld32(scol + 64, dpv);
       tmem_ld_wait();
       tc_fence_before();
       mbar_arrive(sdp_free + 8 * buf);   // S and dP are in registers: batch n+2 may overwrite this TMEM buffer
 #pragma unroll
       for (int e = 0; e < 32; e += 2) {
-        const uint32_t d2 = pack_bf16(p[e] * fmaf(gv, dpv[e], -del), p[e + 1] * fmaf(gv, dpv[e + 1], -del));
-        pw[e / 2] = dead ? 0u : d2;
+        const uint64_t x = fma_f32x2(g2, pack_f32x2(dpv[e], dpv[e + 1]), nd2);
+        const uint64_t d2 = mul_f32x2(pack_f32x2(p[e], p[e + 1]), x);
+        pw[e / 2] = pack_bf16(lo_f32x2(d2), hi_f32x2(d2));
+      }
+      if (nrow == 0) {   // (0 times whatever dP is)
+#pragma unroll
+        for (int e = 0; e < 16; ++e) pw[e] = 0u;
       }
 #pragma unroll
       for (int c = 0; c < 4; ++c)
-        *reinterpret_cast<uint4*>(drow + ((4 * half + c) ^ (row & 7)) * 16) = make_uint4(pw[4 * c], pw[4 * c + 1], pw[4 * c + 2], pw[4 * c + 3]);
+        *reinterpret_cast<uint4*>(prow + P_TILE + ((4 * half + c) ^ (row & 7)) * 16) = make_uint4(pw[4 * c], pw[4 * c + 1], pw[4 * c + 2], pw[4 * c + 3]);
       fence_proxy_async();
       mbar_arrive(pds_full + 8 * buf);
     }
     // ---- epilogue: dV^T / dK^T [d lanes x 64 key columns] -> global ---------------------------------------
     if (ok && nb > 0) ok = mbar_wait(acc_full, 0, DEV_ERR_FULL_WAIT);
     tc_fence_after();
-    const int dch = row;  // channel owned by this thread
-    {
-      const int which = half;   // half 0 stores dV, half 1 dK
-      const float mul = which ? a.scale : 1.f;
-      const long long Nout = (long long)a.B * a.T * a.Hk * D;
-      float* part = a.part + (which ? 0 : a.slabs * Nout);
+    // Half 0 stores dV, half 1 dK; a thread has one channel.  The loop is not unrolled: straight-line code that a CTA runs once comes
+    // from beyond the instruction cache (all 64 keys unrolled, with their variants, took 55 000 cycles beside 384 000 for 94 batches)
+    const float mul = half ? a.scale : 1.f;
+    const long long Nout = (long long)a.B * a.T * a.Hk * D;
+    const int step = a.Hk * D, nk = ok ? min(64, a.T - key0) : 0;
+    const long long off0 = (((long long)b * a.T + key0) * a.Hk + hk) * D + row;
+    const float* const win = a.part + (half ? 0 : a.slabs * Nout) + off0;   // the window's part, or where a share goes
+#pragma unroll 1
+    for (int c = 0; c < 64; c += 16) {
+      float vals[16];
+      if (nb > 0) {
+        tmem_ld16(tmem + lane_addr + kColDV + half * 64 + c, vals);
+      } else {
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        float vals[16];
-        if (nb > 0) {
-          tmem_ld16(tmem + lane_addr + kColDV + which * 64 + c * 16, vals);
-          tmem_ld_wait();
-        } else {
+        for (int e = 0; e < 16; ++e) vals[e] = 0.f;
+      }
+      if (a.nshare > 1) {
+        float* const dst = const_cast<float*>(win) + seg * Nout + (long long)c * step;
+        tmem_ld_wait();
 #pragma unroll
-          for (int e = 0; e < 16; ++e) vals[e] = 0.f;
-        }
-        float add[16];   // the window's part
+        for (int e = 0; e < 16; ++e)
+          if (c + e < nk) dst[e * step] = vals[e] * mul;
+      } else {
+        float add[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) add[e] = 0.f;
-        for (int w = 0; a.nshare == 1 && w < a.nadd; ++w) {
+#pragma unroll 1
+        for (int w = 0; w < a.nadd; ++w) {
+          const float* const src = win + w * Nout + (long long)c * step;
 #pragma unroll
-          for (int e = 0; e < 16; ++e) {
-            const int kp = key0 + c * 16 + e;
-            if (kp < a.T) add[e] += part[w * Nout + (((long long)b * a.T + kp) * a.Hk + hk) * D + dch];
-          }
+          for (int e = 0; e < 16; ++e)
+            if (c + e < nk) add[e] += src[e * step];
         }
+        bf16* const dst = (half ? a.dk : a.dv) + off0 + (long long)c * step;
+        tmem_ld_wait();
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          const int kp = key0 + c * 16 + e;
-          if (!ok || kp >= a.T) continue;
-          const long long off = (((long long)b * a.T + kp) * a.Hk + hk) * D + dch;
-          if (a.nshare > 1)
-            part[seg * Nout + off] = vals[e] * mul;
-          else
-            (which ? a.dk : a.dv)[off] = __float2bfloat16(fmaf(vals[e], mul, add[e]));
-        }
+        for (int e = 0; e < 16; ++e)
+          if (c + e < nk) dst[e * step] = __float2bfloat16(fmaf(vals[e], mul, add[e]));
       }
     }
   }
