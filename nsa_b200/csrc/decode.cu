@@ -11,8 +11,9 @@
 // rows of mma.sync.m16n8k16.  Where there are fewer items than SMs, a cluster of 2, 4 or 8 CTAs shares one: the tile pairs of
 // every phase behind the statistics are dealt out to its CTAs, which exchange the scores through each other's shared
 // memory and then select the blocks each for itself (one CTA alone draws at most 1/148 of the bandwidth: 4 items of 4096 keys
-// took 25 us).  The statistics (pass 1) are the same six chains everywhere, added in the same order: every CTA of a cluster
-// makes them for itself, and a chain's place in the sum does not follow from the warp that had it.  In another order near
+// took 25 us).  Where there are more, two CTAs of half the size share an SM.  The statistics (pass 1) are the same six chains
+// everywhere, added in the same order: every CTA of a cluster makes them for itself, a warp of a CTA of three has two of them in
+// turn, and a chain's place in the sum does not follow from the warp that had it.  In another order near
 // ties of two blocks' scores come out otherwise, and a sequence's blocks would depend on how many others it is decoded with:
 // with pass 1 dealt out like the rest up to one in 16 items chose others (1 x 32768 keys 28.7 us so, 34.8 now; 4 x 16384
 // 30.7 and 32.8; 1 x 9000, where an exchange is saved, 26.6 and 25.5).  Producer warps stream [64 rows x 128] tiles by TMA
@@ -28,7 +29,7 @@
 // scheme of decode attention).  The CTAs of an item then merge its rows, in a fixed order: without clusters each warp a row at a
 // time, from a scratch that the CTA's next item uses again (it stays in L2) while the ring fills with that item's tiles; with
 // clusters each CTA its share of the rows, a row and branch per warp.  Measured, 128 sequences of 4096 to 32768 keys: a second
-// kernel that merges (77 MB of partials written and read) 179 us, merged here 170; one
+// kernel that merges (77 MB of partials written and read) 179 us, merged here 170, and with two CTAs per SM 150 (4.7 TB/s); one
 // sequence of 4096 keys 18.9 us with the second kernel and 17.5 without.  Merging through shared memory, warp after warp,
 // cost seven
 // named barriers and six serialised rounds per branch.  No atomics; every wait is bounded.
@@ -43,10 +44,12 @@ namespace nsa {
 namespace {
 
 constexpr int D = 128;
-constexpr int kCons = 6;                       // consumer warps
-constexpr int kProdW = 2;                      // producer warps
-constexpr int kThreads = (kCons + kProdW) * 32;
-constexpr int kSlots = 2 * kCons;
+constexpr int kCons = 6;                       // consumer warps of a CTA that has an SM to itself, chains of the statistics
+constexpr int kHalfCons = 3;                   // ... of one that shares it with another
+// Producer warps: one issues 30 bytes per cycle (see below), what one of two CTAs of an SM can draw at most.
+__host__ __device__ constexpr int decode_producers(int cons) { return cons == kCons ? 2 : 1; }
+__host__ __device__ constexpr int decode_threads(int cons) { return (cons + decode_producers(cons)) * 32; }
+static_assert(kCons == 2 * kHalfCons, "one chain of the statistics per warp, or two");
 constexpr uint32_t PANEL = 64 * 128;           // [64 rows][64 columns] bf16
 constexpr uint32_t TILE = 2 * PANEL;           // 16 KB
 constexpr int kMaxTc = 2048;                   // compressed positions of one sequence held in shared memory
@@ -351,11 +354,12 @@ __device__ __forceinline__ float4 merge_row(const DecodeArgs& a, int item, long 
   return make_float4(f0.x, f0.y, f1.x, f1.y);
 }
 
-// CL: the CTAs of a cluster share an item.
-template <bool CL>
-__global__ void __launch_bounds__(kThreads, 1)
+// CONS consumer warps with a pair of slots each; CL: the CTAs of a cluster share an item.
+template <int CONS, bool CL>
+__global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
     decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                   const __grid_constant__ CUtensorMap tmCK, const __grid_constant__ CUtensorMap tmCV, const DecodeArgs a, const int ncl) {
+  constexpr int kSlots = 2 * CONS, kProdW = decode_producers(CONS);
   const int cl = CL ? ncl : 1;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -366,10 +370,10 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint8_t* after = sgen + kSlots * TILE;
   float* ps = reinterpret_cast<float*>(after);                    // [kMaxTc + 64] head-summed p_sel per compressed position
   float* pooled = ps + kMaxTc + 64;                               // [kMaxPoolD]
-  float* stat = pooled + kMaxPoolD;                               // [kCons][4][16] per-warp statistics
+  float* stat = pooled + kMaxPoolD;                               // [kCons][4][16] the chains' statistics
   float* fin = stat + kCons * 64;                                 // [4][16] merged: M_raw, 1/L_raw, M_att (log2), L_att
-  float2* ml = reinterpret_cast<float2*>(fin + 64);               // [3][kCons][16] (m, l) of the warps' partials, without clusters
-  float* gates = reinterpret_cast<float*>(ml + 3 * kCons * 16);       // [3][16], branch order as ml's
+  float2* ml = reinterpret_cast<float2*>(fin + 64);               // [3][CONS][16] (m, l) of the warps' partials, without clusters
+  float* gates = reinterpret_cast<float*>(ml + 3 * CONS * 16);       // [3][16], branch order as ml's
   int* sel = reinterpret_cast<int*>(gates + 48);                  // [kMaxSel] selected blocks of the item, [kMaxSel] = count
   volatile int* abort_flag = sel + kMaxSel + 2;
   const uint32_t bar_base = sbase + kSlots * TILE + (uint32_t)((uint8_t*)(sel + kMaxSel + 4) - after);
@@ -399,13 +403,13 @@ __global__ void __launch_bounds__(kThreads, 1)
   auto deal = [&](int i, int cs) { return !CL || cs == 1 ? i : rank + i * cs; };
   const int pool_k = a.sel_block / a.cstride + 1, pool_s = a.sel_block / a.cstride;
 
-  if (warp >= kCons) {
+  if (warp >= CONS) {
     // ------------------------------- producers --------------------------------------------------------
     // A warp's TMA instructions run one after another (about 850 + 52 x boxes cycles each, whatever the box size), so
     // a single warp issuing one 16 KB tile per instruction caps the SM at ~16 bytes per clock.  Tiles therefore go out
     // in PAIRS (four boxes per instruction: both tiles of a (K, V) pair, or two consecutive ck tiles of pass 1), and
-    // the two producer warps take alternate pairs.
-    const int pw = warp - kCons;
+    // the producer warps (one in a CTA that shares its SM) take alternate pairs.
+    const int pw = warp - CONS;
     uint32_t np = 0, it = 0;     // tile pairs issued so far by both producers together; items so far
     auto issue2 = [&](const CUtensorMap* tmA, int rowA, const CUtensorMap* tmB, int rowB, int h) -> bool {
       const uint32_t mine = np % kProdW == (uint32_t)pw;
@@ -456,13 +460,13 @@ __global__ void __launch_bounds__(kThreads, 1)
   // --------------------------------- consumers ----------------------------------------------------------
   const int g = lane >> 2, tq = lane & 3;
   const float sl2 = a.scale * kLog2e;
-  const int cthreads = kCons * 32;
+  const int cthreads = CONS * 32;
   const int ct = threadIdx.x;               // 0 .. cthreads-1
-  // tile pair i of the CTA, over all phases and items, is warp i % kCons's, in that warp's own two slots
+  // tile pair i of the CTA, over all phases and items, is warp i % CONS's, in that warp's own two slots
   uint32_t np0 = 0, it = 0;                 // pairs of the CTA before the current phase; items so far
   uint32_t use = 0;                         // pairs of this warp so far
   const uint32_t sk = 2 * warp, sv = sk + 1;
-  auto first_pair = [&]() { return (int)((warp + kCons - np0 % kCons) % kCons); };
+  auto first_pair = [&]() { return (int)((warp + CONS - np0 % CONS) % CONS); };
   bool ok = true;
   for (int r = 0; r * ngroup < nitem; ++r) {
     const int item = snake_item(r, group, ngroup);
@@ -476,11 +480,19 @@ __global__ void __launch_bounds__(kThreads, 1)
     load_a_frags_global<D>(qf, a.q + qrow * D, lane);
 
     // ---- pass 1: statistics over all compressed keys ---------------------------------------------------
-    float mr[2] = {-INFINITY, -INFINITY}, lr[2] = {0.f, 0.f};   // raw scores, all keys (natural-log domain kept in log2)
-    float ma[2] = {-INFINITY, -INFINITY}, la[2] = {0.f, 0.f};   // scaled scores, visible keys
-    const int chain = first_pair();   // this warp's chain: the pairs chain, chain + 6, ...
+    // Six chains, whatever the number of warps: chain c has the pairs c, c + 6, ...  One of six warps has one, one of three warps two,
+    // whose pairs come in turn.
+    struct Stat {
+      float mr[2] = {-INFINITY, -INFINITY}, lr[2] = {0.f, 0.f};   // raw scores, all keys (natural-log domain kept in log2)
+      float ma[2] = {-INFINITY, -INFINITY}, la[2] = {0.f, 0.f};   // scaled scores, visible keys
+      int chain;
+    };
+    Stat st0, st1;   // of the pair's chain and (three warps) of the one whose turn is next
+    st0.chain = first_pair();
+    st1.chain = st0.chain + CONS;
     {
-      for (int u = chain; u < p.n1p; u += kCons, ++use) {
+      for (int u = st0.chain; u < p.n1p; u += CONS, ++use) {
+        float(&mr)[2] = st0.mr, (&lr)[2] = st0.lr, (&ma)[2] = st0.ma, (&la)[2] = st0.la;
 #pragma unroll 1
         for (int e = 0; e < 2; ++e) {
           const uint32_t s = sk + e;
@@ -521,22 +533,31 @@ __global__ void __launch_bounds__(kThreads, 1)
             ma[rr] = na;
           }
         }
+        if (CONS != kCons) {
+          const Stat x = st0;
+          st0 = st1;
+          st1 = x;
+        }
       }
       np0 += p.n1p;
     }
     // merge the statistics of the chains, in their order whichever warps had them, so that an item's scores do not depend on
     // the items before it (each value lives in the four lanes of a quad: sum the partial sums)
+    auto leave = [&](const Stat& x) {
 #pragma unroll
-    for (int rr = 0; rr < 2; ++rr) {
-      const float l_r = quad_sum(lr[rr]), l_a = quad_sum(la[rr]);
-      if (tq == 0) {
-        float* st = stat + chain * 64;
-        st[0 * 16 + g + 8 * rr] = mr[rr];
-        st[1 * 16 + g + 8 * rr] = l_r;
-        st[2 * 16 + g + 8 * rr] = nan_or(l_a, ma[rr]);
-        st[3 * 16 + g + 8 * rr] = l_a;
+      for (int rr = 0; rr < 2; ++rr) {
+        const float l_r = quad_sum(x.lr[rr]), l_a = quad_sum(x.la[rr]);
+        if (tq == 0) {
+          float* st = stat + x.chain * 64;
+          st[0 * 16 + g + 8 * rr] = x.mr[rr];
+          st[1 * 16 + g + 8 * rr] = l_r;
+          st[2 * 16 + g + 8 * rr] = nan_or(l_a, x.ma[rr]);
+          st[3 * 16 + g + 8 * rr] = l_a;
+        }
       }
-    }
+    };
+    leave(st0);
+    if (CONS != kCons) leave(st1);
     named_bar_sync(1, cthreads);
     if (ct < 16) {
       float Mr = -INFINITY, Ma = -INFINITY;
@@ -574,7 +595,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     bool full = rank == 0 && warp == 0;   // this warp's partial has an output (the first always: the row sums ride with it)
     {
       const int n = share(p.n2p, p.cs);
-      for (int i = first_pair(); i < n; i += kCons, ++use) {
+      for (int i = first_pair(); i < n; i += CONS, ++use) {
         const int u = deal(i, p.cs);
         full = p.cs > 1 || rank == 0;
         const int j0 = u * 64;
@@ -658,7 +679,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     // this warp's partial of a branch -> workspace: [item][branch][warp of the cluster]{ O[16][D], m[16], l[16] } fp32; a warp
     // that had no tile leaves m = -inf and no O
     auto put_partial = [&](int branch, const float (&x)[D / 8][4], const float (&mm)[2], const float (&ll)[2], bool has) {
-      float* dst = a.part + (((long long)(cl > 1 ? item : (int)blockIdx.x) * 3 + branch) * (cl * kCons) + rank * kCons + warp) * kPartFloats;
+      float* dst = a.part + (((long long)(cl > 1 ? item : (int)blockIdx.x) * 3 + branch) * (cl * CONS) + rank * CONS + warp) * kPartFloats;
 #pragma unroll
       for (int i = 0; i < D / 8; ++i) {
         if (!has) break;
@@ -674,7 +695,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             dst[16 * D + g + 8 * rr] = m;
             dst[16 * D + 16 + g + 8 * rr] = l;
           } else {
-            ml[(branch * kCons + warp) * 16 + g + 8 * rr] = make_float2(m, l);
+            ml[(branch * CONS + warp) * 16 + g + 8 * rr] = make_float2(m, l);
           }
         }
       }
@@ -692,7 +713,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
     // ---- gates, by the last warp (the first one is still choosing blocks) --------------------------------
     // (what the item before left in gates, ml and the scratch has been read: its rows are merged before anything of this one)
-    if (warp == kCons - 1) {
+    if (warp == CONS - 1) {
       if (a.gate_w) {
         // g_x[row] = q[row,:] . W[x,:] + b[x] (nn.Linear(head_dim, 3), rows of W: selected, window, compressed) as one 16 x 8
         // tile of mma.sync, rounded to bf16 as the module's gate tensors are
@@ -731,7 +752,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     full = false;
     {
       const int n = share(p.nw, cl);
-      for (int i = first_pair(); i < n; i += kCons, ++use) {
+      for (int i = first_pair(); i < n; i += CONS, ++use) {
         const int u = deal(i, cl);
         full = true;
         ok = ok && mbar_wait_abortable(full_bar(sk), use & 1, DEV_ERR_FULL_WAIT, abort_flag);
@@ -755,7 +776,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     full = false;
     {
       const int n = share(nsel, cl);
-      for (int i = first_pair(); i < n; i += kCons, ++use) {
+      for (int i = first_pair(); i < n; i += CONS, ++use) {
         const int u = deal(i, cl);
         full = true;
         const int blk = *reinterpret_cast<volatile int*>(sel + u);
@@ -769,27 +790,27 @@ __global__ void __launch_bounds__(kThreads, 1)
     named_bar_sync(1, cthreads);   // ps, pooled, fin and sel are reused by the next item
     ++it;
     // ---- this item's rows: partials merged warp by warp, gated sum of the branches (a lane holds four channels) --------
-    for (int row = warp; cl == 1 && row < 16; row += kCons) {
-      const float4* base = reinterpret_cast<const float4*>(a.part + (long long)blockIdx.x * 3 * kCons * kPartFloats + row * D) + lane;
-      float4 x[3][kCons];
-      float e[3][kCons], inv[3], lse[3];
+    for (int row = warp; cl == 1 && row < 16; row += CONS) {
+      const float4* base = reinterpret_cast<const float4*>(a.part + (long long)blockIdx.x * 3 * CONS * kPartFloats + row * D) + lane;
+      float4 x[3][CONS];
+      float e[3][CONS], inv[3], lse[3];
 #pragma unroll
       for (int br = 0; br < 3; ++br)
 #pragma unroll
-        for (int w = 0; w < kCons; ++w) {
-          e[br][w] = ml[(br * kCons + w) * 16 + row].x;
+        for (int w = 0; w < CONS; ++w) {
+          e[br][w] = ml[(br * CONS + w) * 16 + row].x;
           x[br][w] = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (e[br][w] != -INFINITY) x[br][w] = __ldcg(base + (br * kCons + w) * (kPartFloats / 4));
+          if (e[br][w] != -INFINITY) x[br][w] = __ldcg(base + (br * CONS + w) * (kPartFloats / 4));
         }
 #pragma unroll
       for (int br = 0; br < 3; ++br) {
         float M = e[br][0], L = 0.f;
 #pragma unroll
-        for (int w = 1; w < kCons; ++w) M = fmaxf(M, e[br][w]);
+        for (int w = 1; w < CONS; ++w) M = fmaxf(M, e[br][w]);
 #pragma unroll
-        for (int w = 0; w < kCons; ++w) {
+        for (int w = 0; w < CONS; ++w) {
           e[br][w] = e[br][w] != -INFINITY ? ex2(e[br][w] - M) : 0.f;
-          L += ml[(br * kCons + w) * 16 + row].y * e[br][w];
+          L += ml[(br * CONS + w) * 16 + row].y * e[br][w];
         }
         inv[br] = L > 0.f ? 1.f / L : 0.f;
         lse[br] = L > 0.f ? (M + log2f(L)) * kLn2 : -INFINITY;
@@ -800,7 +821,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (br == 2 && a.window <= 0) continue;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int w = 0; w < kCons; ++w) {
+        for (int w = 0; w < CONS; ++w) {
           const float wt = e[br][w] * inv[br];
           v.x = fmaf(x[br][w].x, wt, v.x);
           v.y = fmaf(x[br][w].y, wt, v.y);
@@ -822,13 +843,13 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (CL) {
     __syncwarp();
     cluster_sync_all();   // every CTA's partials are written (a cluster has one item), and no CTA writes into another's memory any more
-    if (warp >= kCons) return;
+    if (warp >= CONS) return;
     const int item = group, sq = item / a.Hkv, h = item % a.Hkv, rows = 16 / cl, nb = a.window > 0 ? 3 : 2;
     const long long qrow = (long long)(a.order ? a.order[sq] : sq) * a.Hq + h * 16 + rank * rows;   // first of this CTA's rows
     float4* out = reinterpret_cast<float4*>(ps);   // [row][branch][lane], over what the item no longer needs
-    for (int u = warp; u < rows * nb; u += kCons) out[u * 32 + lane] = merge_row(a, item, qrow + u / nb, rank * rows + u / nb, u % nb, cl * kCons, lane);
-    named_bar_sync(1, kCons * 32);
-    for (int row = warp; row < rows; row += kCons) {
+    for (int u = warp; u < rows * nb; u += CONS) out[u * 32 + lane] = merge_row(a, item, qrow + u / nb, rank * rows + u / nb, u % nb, cl * CONS, lane);
+    named_bar_sync(1, CONS * 32);
+    for (int row = warp; row < rows; row += CONS) {
       float4 tot = make_float4(0.f, 0.f, 0.f, 0.f);
       for (int br = 0; br < nb; ++br) {
         const float gt = gates[br * 16 + rank * rows + row];
@@ -840,17 +861,18 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
-constexpr int decode_smem() {
-  return kSlots * (int)TILE + (kMaxTc + 64 + kMaxPoolD + kCons * 64 + 64 + 3 * kCons * 32 + 48) * 4 + (kMaxSel + 4) * 4 +
-         (2 * kSlots + 2) * 8 + 16 + 1024;
+constexpr int decode_smem(int cons) {
+  return 2 * cons * (int)TILE + (kMaxTc + 64 + kMaxPoolD + kCons * 64 + 64 + 3 * cons * 32 + 48) * 4 + (kMaxSel + 4) * 4 +
+         (4 * cons + 2) * 8 + 16 + 1024;
 }
+static_assert(2 * (decode_smem(kHalfCons) + 1024) <= 228 * 1024, "two CTAs per SM");
 
 // A launch of `ncta` CTAs in clusters of `cl`.
-cudaLaunchConfig_t decode_config(int ncta, int cl, cudaLaunchAttribute* at, cudaStream_t s) {
+cudaLaunchConfig_t decode_config(int ncta, int cons, int cl, cudaLaunchAttribute* at, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)ncta);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = decode_smem();
+  cfg.blockDim = dim3(decode_threads(cons));
+  cfg.dynamicSmemBytes = decode_smem(cons);
   cfg.stream = s;
   at->id = cudaLaunchAttributeClusterDimension;
   at->val.clusterDim.x = cl;
@@ -864,29 +886,36 @@ cudaLaunchConfig_t decode_config(int ncta, int cl, cudaLaunchAttribute* at, cuda
 int ask_resident(int cl) {
   int c = 0;
   cudaLaunchAttribute at;
-  const cudaLaunchConfig_t cfg = decode_config(num_sms() / cl * cl, cl, &at, nullptr);
-  if (cudaFuncSetAttribute(decode_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, decode_smem()) != cudaSuccess ||
-      cudaOccupancyMaxActiveClusters(&c, decode_kernel<true>, &cfg) != cudaSuccess)
+  const cudaLaunchConfig_t cfg = decode_config(num_sms() / cl * cl, kCons, cl, &at, nullptr);
+  if (cudaFuncSetAttribute(decode_kernel<kCons, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, decode_smem(kCons)) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&c, decode_kernel<kCons, true>, &cfg) != cudaSuccess)
     c = num_sms() / cl;
   cudaGetLastError();   // (no device: workspace sizes can be asked for all the same)
   return c;
 }
-// How `nitem` items are spread: up to the number of SMs as many CTAs per item as keep every item in the first wave, with more a
-// CTA per SM that takes one after another.  (Two CTAs of three warps per SM, so that one streams tiles while the other chooses
-// its blocks, took 155 us for 128 sequences of 4096 to 32768 keys; but three chains add up the soft-max of the scores in another
-// order than six, and blocks whose scores tie to within a rounding, which one in 700 items has, were then chosen differently.)
+// How `nitem` items are spread: up to the number of SMs as many CTAs per item as keep every item in the first wave, with an SM to
+// itself each; with more items two CTAs of half the warps and slots share an SM, so that one streams tiles while the other chooses
+// its blocks or merges its rows.  Below two items per SM such a CTA has one item and takes 38 us + 1.46 us per 1000 keys for the
+// longest, against two items, a long and a short one, behind each other.  One CTA per SM -> two: 160 items of up to 5500 keys 55 ->
+// 45.6 us, 196 of 10000 58.7 -> 55.7, 260 of 18000 72.7 -> 69.6; but 164 of 21500 54 -> 69.5, 192 of 28000 67 -> 81, 236 of 25000 78.4 ->
+// 80.5, so not there.  512 items of 4096 to 32768 keys 165 -> 150, 512 of 1500 103 -> 90, 320 of 4096 to 32768 118 -> 102.  Three
+// rounds of equal items are no more than two of pairs, the second half empty: 300 to 440 items of 16384 keys 120 to 132 us, as pairs 131 to
+// 142 (of 8192 95 to 109, 97 to 107); four are: 448 of 16384 161 -> 144.
 struct Spread {
-  int cl, ncta;
+  int cons, cl, ncta;
 };
 const std::array<int, 4>& clusters_held() {
   static const std::array<int, 4> held = {num_sms(), ask_resident(2), ask_resident(4), ask_resident(8)};
   return held;
 }
-Spread decode_spread(int nitem) {
+Spread decode_spread(int nitem, int max_Tc, bool even) {   // even: the longest sequence is within 1.3 of the mean
   const std::array<int, 4>& held = clusters_held();
   for (int i = 3; i >= 0; --i)
-    if (nitem <= held[i]) return {1 << i, nitem << i};
-  return {1, num_sms()};
+    if (nitem <= held[i]) return {kCons, 1 << i, nitem << i};
+  const int sms = num_sms();
+  if (nitem < 2 * sms && max_Tc > 768 + (int)(640LL * (nitem - sms) / sms)) return {kCons, 1, sms};   // (12 K keys, 22 K with two items per SM)
+  if (even && nitem > 2 * sms && nitem <= 3 * sms) return {kCons, 1, sms};
+  return {kHalfCons, 1, std::min(nitem, 2 * sms)};
 }
 
 }  // namespace
@@ -930,14 +959,14 @@ int launch_decode(const DecodeArgs& a, cudaStream_t s) {
   }
   const int nitem = a.nseq * a.Hkv;
   if (nitem <= 0) return 0;
-  const Spread p = decode_spread(nitem);
+  const Spread p = decode_spread(nitem, a.max_Tc, 10LL * a.max_Tc * a.nseq <= 13 * a.total_c);
   const int cl = p.cl;
-  const auto kernel = cl > 1 ? decode_kernel<true> : decode_kernel<false>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, decode_smem());
+  const auto kernel = p.cons == kHalfCons ? decode_kernel<kHalfCons, false> : cl > 1 ? decode_kernel<kCons, true> : decode_kernel<kCons, false>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, decode_smem(p.cons));
   if (e != cudaSuccess) return (int)e;
   {
     cudaLaunchAttribute at;
-    const cudaLaunchConfig_t cfg = decode_config(p.ncta, cl, &at, s);
+    const cudaLaunchConfig_t cfg = decode_config(p.ncta, p.cons, cl, &at, s);
     e = cudaLaunchKernelEx(&cfg, kernel, tmK, tmV, tmCK, tmCV, a, cl);
     if (e != cudaSuccess) return (int)e;
   }
