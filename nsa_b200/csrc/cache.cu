@@ -21,6 +21,7 @@ struct TabChunk {
 };
 
 __global__ void upload_table_kernel(const __grid_constant__ TabChunk c, int* __restrict__ dst, const int n) {
+  after_previous();
   for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = c.v[i];
 }
 
@@ -30,6 +31,7 @@ __global__ void __launch_bounds__(256) move_rows_kernel(const uint4* __restrict_
                                                         uint4* __restrict__ ck1, uint4* __restrict__ cv1,
                                                         const int* __restrict__ cu_old, const int* __restrict__ cu_new,
                                                         const int nseq, const int vec_per_row, const long long nvec) {
+  after_previous();
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   if (i >= nvec) return;
   const uint4 a = __ldcs(ck0 + i), b = __ldcs(cv0 + i);
@@ -47,6 +49,7 @@ __global__ void __launch_bounds__(256) move_rows_kernel(const uint4* __restrict_
 // Conv1d weight [o][c][j] -> [j*D + c][o], both tensors.  Block = one input channel c: D x 32 tile through shared memory.
 __global__ void __launch_bounds__(256) conv_weight_kernel(const bf16* __restrict__ w0, const bf16* __restrict__ w1,
                                                           bf16* __restrict__ o0, bf16* __restrict__ o1, const int D, const int l) {
+  after_previous();
   __shared__ bf16 t[32][130];
   const bf16* w = blockIdx.y ? w1 : w0;
   bf16* out = blockIdx.y ? o1 : o0;
@@ -74,7 +77,7 @@ int launch_upload_table(const int* host, int n, int* dst, cudaStream_t s) {
     TabChunk c;
     const int m = std::min(kTabInts, n - i);
     std::copy(host + i, host + i + m, c.v);
-    upload_table_kernel<<<1, 256, 0, s>>>(c, dst + i, m);
+    launch_next(upload_table_kernel, 1, 256, 0, s, c, dst + i, m);
     note_launches(1);
   }
   return (int)cudaGetLastError();
@@ -85,7 +88,7 @@ int launch_move_rows(const bf16* ck0, const bf16* cv0, bf16* ck1, bf16* cv1, con
   if (rows <= 0) return 0;
   const int vpr = row_elems / 8;
   const long long nvec = rows * vpr;
-  move_rows_kernel<<<(unsigned)((nvec + 255) / 256), 256, 0, s>>>((const uint4*)ck0, (const uint4*)cv0, (uint4*)ck1, (uint4*)cv1,
+  launch_next(move_rows_kernel, (unsigned)((nvec + 255) / 256), 256, 0, s, (const uint4*)ck0, (const uint4*)cv0, (uint4*)ck1, (uint4*)cv1,
                                                                  cu_old, cu_new, nseq, vpr, nvec);
   note_launches(1);
   return (int)cudaGetLastError();
@@ -96,7 +99,7 @@ int launch_conv_weight(const bf16* w0, const bf16* w1, bf16* o0, bf16* o1, int D
     set_error("head_dim %d not supported (64 or 128)", D);
     return -2;
   }
-  conv_weight_kernel<<<dim3((unsigned)D, w1 ? 2 : 1), 256, 0, s>>>(w0, w1, o0, o1, D, l);
+  launch_next(conv_weight_kernel, dim3((unsigned)D, w1 ? 2 : 1), 256, 0, s, w0, w1, o0, o1, D, l);
   note_launches(1);
   return (int)cudaGetLastError();
 }

@@ -77,6 +77,7 @@ __device__ __forceinline__ void clear_row(uint8_t* tile, uint32_t panel, int row
 template <int D>
 __global__ void __launch_bounds__(kThreads, 1)
     compress_dx_tc_kernel(const __grid_constant__ Maps maps, const CompressBwdArgs a, const int P, const int HB, const int NS) {
+  after_previous();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t sbase = (raw + 1023u) & ~1023u;
@@ -224,6 +225,7 @@ template <int D>
 __global__ void __launch_bounds__(kThreads, 1)
     compress_dw_tc_kernel(const __grid_constant__ Maps maps, const CompressBwdArgs a, const int P, const int HB, const int ntile,
                           const int nsplit) {
+  after_previous();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t sbase = (raw + 1023u) & ~1023u;
@@ -389,6 +391,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 // mode 0: [l*D, D] fp32; 1: [l*D, D] bf16; 2: Conv1d [o][c][j] bf16.  Block = one channel c: rows j*D + c of all j.
 template <int D>
 __global__ void __launch_bounds__(256) compress_dw_finish_kernel(const CompressBwdArgs a, const int nsplit, const int ngrp) {
+  after_previous();
   __shared__ float t[32][D + 1];
   const int z = blockIdx.y, c = blockIdx.x;
   const long long nW = (long long)a.l * D * D;
@@ -494,7 +497,7 @@ int launch(const CompressBwdArgs& a, cudaStream_t s) {
         ns = k;
       }
     }
-    kern<<<dim3((unsigned)gx, (unsigned)ns, 2), kThreads, smem, s>>>(m, a, g.P, g.HB, ns);
+    launch_next(kern, dim3((unsigned)gx, (unsigned)ns, 2), kThreads, smem, s, m, a, g.P, g.HB, ns);
     note_launches(1);
   }
   if (a.dw[0] || a.dw[1] || a.dbias[0] || a.dbias[1]) {
@@ -502,8 +505,8 @@ int launch(const CompressBwdArgs& a, cudaStream_t s) {
     auto kern = compress_dw_tc_kernel<D>;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
-    kern<<<dim3((unsigned)g.ngrp, (unsigned)g.nsplit, 2), kThreads, smem, s>>>(m, a, g.P, g.HB, g.ntile_w, g.nsplit);
-    compress_dw_finish_kernel<D><<<dim3(D + 1, 2), 256, 0, s>>>(a, g.nsplit, g.ngrp);
+    launch_next(kern, dim3((unsigned)g.ngrp, (unsigned)g.nsplit, 2), kThreads, smem, s, m, a, g.P, g.HB, g.ntile_w, g.nsplit);
+    launch_next(compress_dw_finish_kernel<D>, dim3(D + 1, 2), 256, 0, s, a, g.nsplit, g.ngrp);
     note_launches(2);
   }
   return (int)cudaGetLastError();

@@ -47,6 +47,7 @@ __device__ __forceinline__ float4 cluster_ld4(uint32_t addr) {
 template <int D>
 __global__ void __launch_bounds__(kThreads, 1)
     compress_fwd_tc_kernel(const __grid_constant__ Maps maps, const CompressFwdArgs a, const int P, const int HB, const int ks) {
+  after_previous();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t sbase = (raw + 1023u) & ~1023u;
@@ -260,18 +261,13 @@ int launch(const CompressFwdArgs& a, cudaStream_t s) {
   auto kern = compress_fwd_tc_kernel<D>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return (int)e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)gx, (unsigned)ks, (unsigned)a.ntensor);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 1;
-  at[0].val.clusterDim.y = (unsigned)ks;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cudaLaunchAttribute at[2];
+  cudaLaunchConfig_t cfg = next_config(dim3((unsigned)gx, (unsigned)ks, (unsigned)a.ntensor), dim3(kThreads), smem, s, at);
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = 1;
+  at[1].val.clusterDim.y = (unsigned)ks;
+  at[1].val.clusterDim.z = 1;
+  cfg.numAttrs = 2;
   e = cudaLaunchKernelEx(&cfg, kern, m, a, P, HB, ks);
   if (e != cudaSuccess) return (int)e;
   note_launches(1);

@@ -359,6 +359,7 @@ template <int CONS, bool CL>
 __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
     decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                   const __grid_constant__ CUtensorMap tmCK, const __grid_constant__ CUtensorMap tmCV, const DecodeArgs a, const int ncl) {
+  after_previous();
   constexpr int kSlots = 2 * CONS, kProdW = decode_producers(CONS);
   const int cl = CL ? ncl : 1;
   extern __shared__ uint8_t smem_raw[];
@@ -867,26 +868,23 @@ constexpr int decode_smem(int cons) {
 }
 static_assert(2 * (decode_smem(kHalfCons) + 1024) <= 228 * 1024, "two CTAs per SM");
 
-// A launch of `ncta` CTAs in clusters of `cl`.
+// A launch of `ncta` CTAs in clusters of `cl`; at: two attributes.
 cudaLaunchConfig_t decode_config(int ncta, int cons, int cl, cudaLaunchAttribute* at, cudaStream_t s) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)ncta);
-  cfg.blockDim = dim3(decode_threads(cons));
-  cfg.dynamicSmemBytes = decode_smem(cons);
-  cfg.stream = s;
-  at->id = cudaLaunchAttributeClusterDimension;
-  at->val.clusterDim.x = cl;
-  at->val.clusterDim.y = at->val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = cl > 1 ? 1 : 0;
+  cudaLaunchConfig_t cfg = next_config(dim3((unsigned)ncta), dim3(decode_threads(cons)), decode_smem(cons), s, at);
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = cl;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+  if (cl > 1) cfg.numAttrs = 2;
   return cfg;
 }
 // Clusters of cl CTAs that the GPU holds at a time (fewer than SMs / cl: a cluster lies within one GPC; 16 of 8 would be 128
 // of 148 SMs, but they do not all fit and the rest would run as a second wave).
 int ask_resident(int cl) {
   int c = 0;
-  cudaLaunchAttribute at;
-  const cudaLaunchConfig_t cfg = decode_config(num_sms() / cl * cl, kCons, cl, &at, nullptr);
+  cudaLaunchAttribute at[2];
+  cudaLaunchConfig_t cfg = decode_config(num_sms() / cl * cl, kCons, cl, at, nullptr);
+  cfg.attrs = at + 1;
+  cfg.numAttrs = 1;
   if (cudaFuncSetAttribute(decode_kernel<kCons, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, decode_smem(kCons)) != cudaSuccess ||
       cudaOccupancyMaxActiveClusters(&c, decode_kernel<kCons, true>, &cfg) != cudaSuccess)
     c = num_sms() / cl;
@@ -965,8 +963,8 @@ int launch_decode(const DecodeArgs& a, cudaStream_t s) {
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, decode_smem(p.cons));
   if (e != cudaSuccess) return (int)e;
   {
-    cudaLaunchAttribute at;
-    const cudaLaunchConfig_t cfg = decode_config(p.ncta, p.cons, cl, &at, s);
+    cudaLaunchAttribute at[2];
+    const cudaLaunchConfig_t cfg = decode_config(p.ncta, p.cons, cl, at, s);
     e = cudaLaunchKernelEx(&cfg, kernel, tmK, tmV, tmCK, tmCV, a, cl);
     if (e != cudaSuccess) return (int)e;
   }

@@ -42,6 +42,7 @@ template <int D>
 __global__ void __launch_bounds__(kThreads, 1)
     dense_select_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                         const DenseArgs a, const int nst, const int pool_stride_f) {
+  after_previous();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t sbase = (raw + 1023u) & ~1023u;
@@ -334,7 +335,7 @@ int launch(const DenseArgs& a, cudaStream_t s) {
   const long long total = (long long)a.B * (a.Hq / 16) * ((a.T + kTok - 1) / kTok);
   const int grid = (int)(total < num_sms() ? total : num_sms());
   if (grid <= 0) return 0;
-  kern<<<grid, kThreads, smem, s>>>(tmK, tmV, a, nst, pool_stride_f);
+  launch_next(kern, grid, kThreads, smem, s, tmK, tmV, a, nst, pool_stride_f);
   note_launches(1);
   return (int)cudaGetLastError();
 }

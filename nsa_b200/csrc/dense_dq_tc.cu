@@ -65,6 +65,7 @@ struct Maps {
 template <int D, bool WIN, bool CMP>
 __global__ void __launch_bounds__(kThreads, 1)
     dense_dq_tc_kernel(const __grid_constant__ Maps maps, const DenseArgs a) {
+  after_previous();
   constexpr int NP = D / 64;
   constexpr uint32_t TILE = NP * PANEL;
   extern __shared__ uint8_t smem_raw[];
@@ -502,7 +503,7 @@ int launch(const DenseArgs& a, cudaStream_t s) {
   }
   const int grid = (int)(total < num_sms() ? total : num_sms());
   if (grid <= 0) return 0;
-  kern<<<grid, kThreads, kSmem<D>, s>>>(m, a);
+  launch_next(kern, grid, kThreads, kSmem<D>, s, m, a);
   note_launches(1);
   return (int)cudaGetLastError();
 }

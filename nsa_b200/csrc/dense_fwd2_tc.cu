@@ -67,6 +67,7 @@ template <int D, int MODE>
 __global__ void __launch_bounds__(kThreads, 1)
     dense_fwd2_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                          const __grid_constant__ CUtensorMap tmV, const DenseArgs a) {
+  after_previous();
   constexpr int NP = D / 64;                  // 64-channel panels
   constexpr uint32_t TILE = NP * PANEL;
   extern __shared__ uint8_t smem_raw[];
@@ -466,7 +467,7 @@ int launch(const DenseArgs& a, cudaStream_t s) {
   }
   const int grid = (int)(total < num_sms() ? total : num_sms());
   if (grid <= 0) return 0;
-  kern<<<grid, kThreads, kSmem<D>, s>>>(tmQ, tmK, tmV, a);
+  launch_next(kern, grid, kThreads, kSmem<D>, s, tmQ, tmK, tmV, a);
   note_launches(1);
   return (int)cudaGetLastError();
 }

@@ -103,6 +103,7 @@ template <int D, bool BYSEQ>   // BYSEQ: the query rows come by sequence (see la
 __global__ void __launch_bounds__(kThreads, 1)
     dense_kv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
                        const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const DenseKvArgs a) {
+  after_previous();
   constexpr int NP = D / 64;
   constexpr uint32_t TILE = NP * PANEL;
   constexpr uint32_t kColDV = 256, kColDK = 256 + D;
@@ -446,6 +447,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 // dk, dv (bf16) = sum over the segments that see the row's key tile of part [2][nslab][n_out]
 __global__ void __launch_bounds__(256) dense_kv_reduce_kernel(const DenseKvArgs a, int D) {
+  after_previous();
   const long long i = ((long long)blockIdx.x * 256 + threadIdx.x) * 4;
   if (i >= a.n_out) return;
   const long long row = i / (a.Hk * D);
@@ -490,10 +492,10 @@ int launch(const DenseKvArgs& a, cudaStream_t s) {
     set_error("dense dK, dV: grid too large");
     return -33;
   }
-  kern<<<(unsigned)grid, kThreads, kSmem<D>, s>>>(tmQ, tmDO, tmK, tmV, a);
+  launch_next(kern, (unsigned)grid, kThreads, kSmem<D>, s, tmQ, tmDO, tmK, tmV, a);
   note_launches(1);
   if (a.mode == 1 && a.part) {
-    dense_kv_reduce_kernel<<<dim3((unsigned)((a.n_out / 4 + 255) / 256), 2), 256, 0, s>>>(a, D);
+    launch_next(dense_kv_reduce_kernel, dim3((unsigned)((a.n_out / 4 + 255) / 256), 2), 256, 0, s, a, D);
     note_launches(1);
   }
   return (int)cudaGetLastError();

@@ -52,6 +52,7 @@ template <int D>
 __global__ void __launch_bounds__(kGateThreads) gate_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w,
                                                                const bf16* __restrict__ bias, bf16* __restrict__ g0,
                                                                bf16* __restrict__ g1, bf16* __restrict__ g2, long long rows) {
+  after_previous();
   constexpr int LPR = D / 8;                 // lanes per row
   constexpr int RPW = 32 / LPR;              // rows per warp and pass
   const int lane = threadIdx.x & 31, sub = lane % LPR, rw = lane / LPR;
@@ -111,6 +112,7 @@ struct Rowdot3Args {
 // 4.2 M rows: 0.69 against 1.05 ms (6.25 against 4.1 TB/s); against a warp per row with one branch, 0.5 M rows: 71 -> 53 us.
 template <int D>
 __global__ void __launch_bounds__(256) rowdot3_kernel(const Rowdot3Args a) {
+  after_previous();
   constexpr int LPR = D / 8;
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   const long long row = i / LPR;
@@ -149,6 +151,7 @@ __global__ void __launch_bounds__(kGateThreads, 2) gate_bwd_kernel(const bf16* _
                                                                const bf16* __restrict__ dg1, const bf16* __restrict__ dg2,
                                                                const bf16* __restrict__ w, bf16* __restrict__ dq,
                                                                float* __restrict__ part, long long rows) {
+  after_previous();
   constexpr int LPR = D / 8, RPW = 32 / LPR;
   constexpr int NW = kGateThreads / 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane % LPR, rw = lane / LPR;
@@ -229,6 +232,7 @@ __global__ void __launch_bounds__(kGateThreads, 2) gate_bwd_kernel(const bf16* _
 // eight warps take every eighth partial and meet in shared memory in warp order.
 __global__ void __launch_bounds__(256) gate_reduce_kernel(const float* __restrict__ part, int nblk, int D, bf16* __restrict__ dw,
                                                          bf16* __restrict__ db) {
+  after_previous();
   __shared__ float red[8][33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int i = blockIdx.x * 32 + lane;
@@ -266,9 +270,9 @@ int launch_gate_fwd(const bf16* q, const bf16* w, const bf16* bias, bf16* g0, bf
                     cudaStream_t s) {
   if (rows <= 0) return 0;
   if (D == 128)
-    gate_fwd_kernel<128><<<stream_grid(gate_fwd_kernel<128>, rows, 16), kGateThreads, 0, s>>>(q, w, bias, g0, g1, g2, rows);
+    launch_next(gate_fwd_kernel<128>, stream_grid(gate_fwd_kernel<128>, rows, 16), kGateThreads, 0, s, q, w, bias, g0, g1, g2, rows);
   else if (D == 64)
-    gate_fwd_kernel<64><<<stream_grid(gate_fwd_kernel<64>, rows, 32), kGateThreads, 0, s>>>(q, w, bias, g0, g1, g2, rows);
+    launch_next(gate_fwd_kernel<64>, stream_grid(gate_fwd_kernel<64>, rows, 32), kGateThreads, 0, s, q, w, bias, g0, g1, g2, rows);
   else {
     set_error("head_dim %d not supported (64 or 128)", D);
     return -2;
@@ -290,9 +294,9 @@ int launch_rowdot3(const bf16* const o[3], const bf16* dout, const bf16* const g
   a.dout = dout;
   a.rows = rows;
   if (D == 128)
-    rowdot3_kernel<128><<<(unsigned)((rows * 16 + 255) / 256), 256, 0, s>>>(a);
+    launch_next(rowdot3_kernel<128>, (unsigned)((rows * 16 + 255) / 256), 256, 0, s, a);
   else if (D == 64)
-    rowdot3_kernel<64><<<(unsigned)((rows * 8 + 255) / 256), 256, 0, s>>>(a);
+    launch_next(rowdot3_kernel<64>, (unsigned)((rows * 8 + 255) / 256), 256, 0, s, a);
   else {
     set_error("head_dim %d not supported (64 or 128)", D);
     return -2;
@@ -316,14 +320,14 @@ int launch_gate_bwd(const bf16* q, const bf16* dg0, const bf16* dg1, const bf16*
   if (rows <= 0) return 0;
   const int grid = gate_bwd_grid(rows, D);
   if (D == 128)
-    (dq ? gate_bwd_kernel<128, true> : gate_bwd_kernel<128, false>)<<<grid, kGateThreads, 0, s>>>(q, dg0, dg1, dg2, w, dq, workspace, rows);
+    launch_next(dq ? gate_bwd_kernel<128, true> : gate_bwd_kernel<128, false>, grid, kGateThreads, 0, s, q, dg0, dg1, dg2, w, dq, workspace, rows);
   else if (D == 64)
-    (dq ? gate_bwd_kernel<64, true> : gate_bwd_kernel<64, false>)<<<grid, kGateThreads, 0, s>>>(q, dg0, dg1, dg2, w, dq, workspace, rows);
+    launch_next(dq ? gate_bwd_kernel<64, true> : gate_bwd_kernel<64, false>, grid, kGateThreads, 0, s, q, dg0, dg1, dg2, w, dq, workspace, rows);
   else {
     set_error("head_dim %d not supported (64 or 128)", D);
     return -2;
   }
-  gate_reduce_kernel<<<(3 * D + 3 + 31) / 32, 256, 0, s>>>(workspace, grid, D, dw, db);
+  launch_next(gate_reduce_kernel, (3 * D + 3 + 31) / 32, 256, 0, s, workspace, grid, D, dw, db);
   note_launches(2);
   return (int)cudaGetLastError();
 }

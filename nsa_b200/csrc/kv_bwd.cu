@@ -28,6 +28,7 @@ template <int D>
 __global__ void __launch_bounds__(kThreads, 1)
     kv_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
                   const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const KvArgs a, const int nst) {
+  after_previous();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t sbase = (raw + 1023u) & ~1023u;
@@ -261,7 +262,7 @@ int launch(const KvArgs& a, cudaStream_t s) {
     set_error("kv backward: grid too large");
     return -33;
   }
-  kern<<<(unsigned)grid, kThreads, smem, s>>>(tmQ, tmDO, tmK, tmV, a, nst);
+  launch_next(kern, (unsigned)grid, kThreads, smem, s, tmQ, tmDO, tmK, tmV, a, nst);
   note_launches(1);
   return (int)cudaGetLastError();
 }

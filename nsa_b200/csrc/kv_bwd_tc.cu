@@ -62,6 +62,7 @@ constexpr uint32_t kColDV = 256, kColDK = 320, kColDQ = 384;   // dQ_part: 384..
 __global__ void __launch_bounds__(kThreads, 1)
     kv_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
                      const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const KvArgs a) {
+  after_previous();
   extern __shared__ __align__(1024) uint8_t kv_bwd_smem[];
   uint8_t* const sgen = kv_bwd_smem;
   const uint32_t sbase = smem_u32(kv_bwd_smem);
@@ -541,7 +542,7 @@ int launch(const KvArgs& a, cudaStream_t s) {
     set_error("kv backward: grid too large");
     return -33;
   }
-  kv_bwd_tc_kernel<<<(unsigned)grid, kThreads, kSmem, s>>>(tmQ, tmDO, tmK, tmV, a);
+  launch_next(kv_bwd_tc_kernel, (unsigned)grid, kThreads, kSmem, s, tmQ, tmDO, tmK, tmV, a);
   note_launches(1);
   return (int)cudaGetLastError();
 }

@@ -24,6 +24,7 @@ namespace {
 __global__ void combine_kernel(const bf16* __restrict__ a0, const bf16* __restrict__ g0, const bf16* __restrict__ a1,
                                const bf16* __restrict__ g1, const bf16* __restrict__ a2, const bf16* __restrict__ g2,
                                bf16* __restrict__ o, long long n8, int D8) {
+  after_previous();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n8) return;
   const long long row = i / D8;
@@ -62,6 +63,7 @@ constexpr int kRevWarps = 8;
 
 // grid (NB chunks, B*H): histogram of the block ids selected by the BS tokens of one chunk
 __global__ void rev_hist_kernel(const RevArgs a) {
+  after_previous();
   extern __shared__ int sh[];
   const int chunk = blockIdx.x, bh = blockIdx.y;
   const int b = bh / a.H, h = bh % a.H;
@@ -83,6 +85,7 @@ __global__ void rev_hist_kernel(const RevArgs a) {
 // grid (ceil(NB / 32), B*H), 1024 threads: exclusive prefix over the chunks of 32 block ids (in place), one lane per id,
 // one warp per thirty-second of the chunks; the totals go to rev_ptr[blk] (the fill kernel turns them into offsets)
 __global__ void __launch_bounds__(1024) rev_scan_kernel(const RevArgs a, const int nchunk) {
+  after_previous();
   __shared__ int part[32][33];
   const int bh = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int blk = blockIdx.x * 32 + lane;
@@ -109,6 +112,7 @@ __global__ void __launch_bounds__(1024) rev_scan_kernel(const RevArgs a, const i
 
 // grid (B*H), 1024 threads: totals per block id -> exclusive CSR offsets (in place)
 __global__ void __launch_bounds__(1024) rev_offset_kernel(const RevArgs a) {
+  after_previous();
   __shared__ int ws[32];
   int* rp = a.rev_ptr + (long long)blockIdx.x * (a.NB + 1);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -138,6 +142,7 @@ __global__ void __launch_bounds__(1024) rev_offset_kernel(const RevArgs a) {
 // grid (NB chunks, B*H), eight warps: write the tokens of the chunk, in order, behind each block's cursor.  A warp owns
 // an eighth of the chunk's tokens; the cursors of a warp start behind the counts of the warps before it.
 __global__ void __launch_bounds__(kRevWarps * 32) rev_fill_kernel(const RevArgs a) {
+  after_previous();
   extern __shared__ int cur[];   // [warps][NB]
   const int nw = blockDim.x >> 5;
   const int chunk = blockIdx.x, bh = blockIdx.y;
@@ -192,6 +197,7 @@ __global__ void __launch_bounds__(kRevWarps * 32) rev_fill_kernel(const RevArgs 
 // dk, dv = the sum of a key block's shares, in order
 __global__ void __launch_bounds__(256) reduce_shares_kernel(const float* __restrict__ part, bf16* __restrict__ dk, bf16* __restrict__ dv,
                                                             int nshare, long long n) {
+  after_previous();
   const long long i = ((long long)blockIdx.x * 256 + threadIdx.x) * 4;
   if (i >= n) return;
   const float* p = part + (blockIdx.y ? nshare * n : 0) + i;
@@ -208,7 +214,7 @@ __global__ void __launch_bounds__(256) reduce_shares_kernel(const float* __restr
 
 int launch_reduce_shares(const float* part, bf16* dk, bf16* dv, int nshare, long long n, cudaStream_t s) {
   if (n <= 0) return 0;
-  reduce_shares_kernel<<<dim3((unsigned)((n / 4 + 255) / 256), 2), 256, 0, s>>>(part, dk, dv, nshare, n);
+  launch_next(reduce_shares_kernel, dim3((unsigned)((n / 4 + 255) / 256), 2), 256, 0, s, part, dk, dv, nshare, n);
   note_launches(1);
   return (int)cudaGetLastError();
 }
@@ -230,7 +236,7 @@ int launch_combine(const bf16* a0, const bf16* g0, const bf16* a1, const bf16* g
     return -2;
   }
   const long long n8 = rows * (D / 8);
-  combine_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, s>>>(a0, g0, a1, g1, a2, g2, o, n8, D / 8);
+  launch_next(combine_kernel, (unsigned)((n8 + 255) / 256), 256, 0, s, a0, g0, a1, g1, a2, g2, o, n8, D / 8);
   note_launches(1);
   return (int)cudaGetLastError();
 }
@@ -243,6 +249,7 @@ int launch_combine(const bf16* a0, const bf16* g0, const bf16* a1, const bf16* g
 template <int D>
 __global__ void __launch_bounds__(256) sel_dq_reduce_kernel(const RevArgs a, const bf16* __restrict__ part, bf16* __restrict__ dq,
                                                             const GateAdd gate, const int G16, const float scale, const int accumulate) {
+  after_previous();
   constexpr int kHeads = 4, kWarps = 16 / kHeads;
   const long long w4 = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   const long long total = (long long)a.B * a.Tq * a.H * G16;
@@ -360,7 +367,7 @@ int launch_sel_dq_reduce(const RevArgs& a, const bf16* part, bf16* dq, int Hq, i
     set_error("selected dQ reduction: at most 32 selected blocks per token");
     return -2;
   }
-  sel_dq_reduce_kernel<128><<<(unsigned)((4 * total + 7) / 8), 256, 0, s>>>(a, part, dq, gate, G16, scale, accumulate);
+  launch_next(sel_dq_reduce_kernel<128>, (unsigned)((4 * total + 7) / 8), 256, 0, s, a, part, dq, gate, G16, scale, accumulate);
   note_launches(1);
   return (int)cudaGetLastError();
 }
@@ -379,10 +386,10 @@ int launch_build_rev(const RevArgs& a, cudaStream_t s) {
   if (sm > 48 * 1024) cudaFuncSetAttribute(rev_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (nw * sm > 48 * 1024)
     cudaFuncSetAttribute(rev_fill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(nw * sm));
-  rev_hist_kernel<<<grid, 256, sm, s>>>(a);
-  rev_scan_kernel<<<dim3((a.NB + 31) / 32, a.B * a.H), 1024, 0, s>>>(a, nchunk);
-  rev_offset_kernel<<<a.B * a.H, 1024, 0, s>>>(a);
-  rev_fill_kernel<<<grid, nw * 32, nw * sm, s>>>(a);
+  launch_next(rev_hist_kernel, grid, 256, sm, s, a);
+  launch_next(rev_scan_kernel, dim3((a.NB + 31) / 32, a.B * a.H), 1024, 0, s, a, nchunk);
+  launch_next(rev_offset_kernel, a.B * a.H, 1024, 0, s, a);
+  launch_next(rev_fill_kernel, grid, nw * 32, nw * sm, s, a);
   note_launches(4);
   return (int)cudaGetLastError();
 }

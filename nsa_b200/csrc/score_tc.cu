@@ -104,6 +104,7 @@ __device__ __forceinline__ void halve(float (&v)[32], int lane) {
 __global__ void __launch_bounds__(kThreads, 1)
     score_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const ScoreArgs a,
                     const int QST, const int KST, const int nslot, const int pool_floats) {
+  after_previous();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t sbase = (raw + 1023u) & ~1023u;
@@ -439,7 +440,7 @@ int launch_score_tc(const ScoreArgs& a, cudaStream_t s) {
   }
   const int grid = (int)(total < num_sms() ? total : num_sms());
   if (grid <= 0) return 0;
-  score_tc_kernel<<<grid, kThreads, smem, s>>>(tmQ, tmK, a, QST, KST, nslot, pool_floats);
+  launch_next(score_tc_kernel, grid, kThreads, smem, s, tmQ, tmK, a, QST, KST, nslot, pool_floats);
   note_launches(1);
   return (int)cudaGetLastError();
 }

@@ -153,6 +153,7 @@ __global__ void __launch_bounds__(2 * kWarps * 32, 1)
     sel_block_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                      const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO, const SelArgs a,
                      const int spw) {
+  after_previous();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t sbase = (raw + 1023u) & ~1023u;
@@ -488,7 +489,7 @@ int launch_nw(const SelArgs& a, cudaStream_t s) {
   const long long ctas = (total + kWarps - 1) / kWarps;
   const int grid = (int)(ctas < num_sms() ? ctas : num_sms());
   if (grid <= 0) return 0;
-  kern<<<grid, kThreads, smem, s>>>(tmK, tmV, tmQ, tmDO, a, spw);
+  launch_next(kern, grid, kThreads, smem, s, tmK, tmV, tmQ, tmDO, a, spw);
   note_launches(1);
   return (int)cudaGetLastError();
 }

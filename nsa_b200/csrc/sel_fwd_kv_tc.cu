@@ -43,6 +43,7 @@ constexpr uint32_t kColO = 128, kColP = 384;
 __global__ void __launch_bounds__(kThreads, 1)
     sel_fwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, const SelKvArgs a, const int nshare) {
+  after_previous();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t sbase = (raw + 1023u) & ~1023u;
@@ -330,6 +331,7 @@ constexpr int kMergeHeads = 8, kMergeWarps = 16 / kMergeHeads;
 template <bool SUM>
 __global__ void __launch_bounds__(256) sel_fwd_merge_kernel(const RevArgs a, const bf16* __restrict__ part,
                                                             const float* __restrict__ stats, const SelMerge m, const int G16) {
+  after_previous();
   constexpr int NV = kMergeHeads * D / 8 / 32;   // 16-byte vectors per lane: 4
   const long long w4 = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   const long long total = (long long)a.B * a.Tq * a.H * G16;
@@ -496,7 +498,7 @@ int launch_sel_fwd_kv(const SelKvArgs& a, const RevArgs& r, cudaStream_t s) {
     set_error("selected forward: grid too large");
     return -33;
   }
-  sel_fwd_kv_kernel<<<(unsigned)grid, kThreads, kSmem, s>>>(tmQ, tmK, tmV, a, nshare);
+  launch_next(sel_fwd_kv_kernel, (unsigned)grid, kThreads, kSmem, s, tmQ, tmK, tmV, a, nshare);
   note_launches(1);
   e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
@@ -504,9 +506,9 @@ int launch_sel_fwd_kv(const SelKvArgs& a, const RevArgs& r, cudaStream_t s) {
   const long long total = (long long)a.B * a.Tq * a.Hk * G16;
   const unsigned nb = (unsigned)((kMergeWarps * total + 7) / 8);
   if (a.merge.out)
-    sel_fwd_merge_kernel<true><<<nb, 256, 0, s>>>(r, a.part, a.stats, a.merge, G16);
+    launch_next(sel_fwd_merge_kernel<true>, nb, 256, 0, s, r, a.part, a.stats, a.merge, G16);
   else
-    sel_fwd_merge_kernel<false><<<nb, 256, 0, s>>>(r, a.part, a.stats, a.merge, G16);
+    launch_next(sel_fwd_merge_kernel<false>, nb, 256, 0, s, r, a.part, a.stats, a.merge, G16);
   note_launches(1);
   return (int)cudaGetLastError();
 }
