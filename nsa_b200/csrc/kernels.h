@@ -348,7 +348,7 @@ struct RevArgs {
   int* rev_tok;   // [B,H,cap]
   long long cap;  // Tq*S
   int Tq, q0;     // query shard: idx/counts hold Tq rows per batch; T is the key sequence length
-  int* inv;       // optional [B,Tq,H,S]: for every valid (row, slot) its position in the (b,h) list of rev_tok
+  int* inv;       // optional [B,Tq,H,S]: for every (row, slot) its position in the (b,h) list of rev_tok, -1 where the slot does not count
 };
 int launch_build_rev(const RevArgs& a, cudaStream_t s);
 #ifdef __CUDACC__

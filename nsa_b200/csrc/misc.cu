@@ -186,6 +186,8 @@ __global__ void __launch_bounds__(kRevWarps * 32) rev_fill_kernel(const RevArgs 
           out[pos] = t;
           if (a.inv) a.inv[row * a.S + s] = pos;
         }
+      } else if (a.inv && s < a.S) {
+        a.inv[row * a.S + s] = -1;
       }
       __syncwarp();
       if (blk >= 0 && (lane == 31 || (same >> (lane + 1)) == 0)) mine[blk] += __popc(same);  // highest lane of the group
@@ -262,12 +264,10 @@ __global__ void __launch_bounds__(256) sel_dq_reduce_kernel(const RevArgs a, con
   const int h = (int)(row % a.H);
   const long long bt = row / a.H;
   const int tl = (int)(bt % a.Tq), b = (int)(bt / a.Tq);
-  const int t = a.q0 + tl;
   constexpr int NV = kHeads * D / 8 / 32;              // 16-byte vectors per lane: 2 at D = 128
   const long long bh = (long long)b * a.H + h;
-  // lane s holds the list position of slot s (or -1): the same validity rule that built the lists
-  int mypos = -1;
-  if (lane < a.S && rev_block(a, row, lane, t) >= 0) mypos = a.inv[row * a.S + lane];
+  // lane s holds the list position of slot s (-1: the slot does not count)
+  const int mypos = lane < a.S ? a.inv[row * a.S + lane] : -1;
   const int Hq = a.H * G16 * 16;
   const long long row0 = bt * Hq + (long long)(h * G16 + sub) * 16 + hb * kHeads;
   // the partial tiles keep the staging layout of the kernel that wrote them: within a 128-byte half row the 16-byte

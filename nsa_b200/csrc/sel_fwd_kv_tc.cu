@@ -344,10 +344,8 @@ __global__ void __launch_bounds__(256) sel_fwd_merge_kernel(const RevArgs a, con
   const int h = (int)(row % a.H);
   const long long bt = row / a.H;
   const int tl = (int)(bt % a.Tq), b = (int)(bt / a.Tq);
-  const int t = a.q0 + tl;
   const long long bh = (long long)b * a.H + h;
-  int mypos = -1;
-  if (lane < a.S && rev_block(a, row, lane, t) >= 0) mypos = a.inv[row * a.S + lane];
+  const int mypos = lane < a.S ? a.inv[row * a.S + lane] : -1;   // -1: the slot does not count
   const int Hq = a.H * G16 * 16;
   const long long orow0 = bt * Hq + (long long)(h * G16 + sub) * 16;   // first of the group's 16 (token, head) rows
   const int myhead = hb * kMergeHeads + lane % kMergeHeads;
