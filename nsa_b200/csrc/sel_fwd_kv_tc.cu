@@ -324,16 +324,18 @@ __global__ void __launch_bounds__(kThreads, 1)
 // Two warps per (batch, token, 16-head group), each eight of the 16 heads: the visits' (m, l) and O tiles merged in slot order,
 // and the gated sum of the branches.  A load instruction of the warp covers 512 contiguous bytes of a tile.  Bound by reading
 // the tiles, so by what a warp has in flight per register: the first tile and the gates are fetched ahead of the maxima.
-// All slots visible, 4 x 8192 tokens, 64 heads: 1.50 ms with the gate (6.5 TB/s; 1.45 + 0.64 as two passes); half visible,
-// 8 x 8192 tokens, three branches: 2.32 (1.85 + 0.73).  Four heads per warp and two tiles in flight 1.67 and 2.53; two tiles
-// of eight heads 1.62 and 2.73; four of four 1.89 and 3.26 (too few warps).
-constexpr int kMergeHeads = 8, kMergeWarps = 16 / kMergeHeads;
+// All slots visible, 4 x 8192 tokens, 64 heads: 1.41 ms with the gate (6.9 TB/s); half visible, 8 x 8192 tokens, three
+// branches: 2.25; one sequence of 5003 tokens: 162 us; 2 x 2080 tokens: 80.  Small blocks at 64 registers keep 32 warps on an
+// SM: with eight warps a block at the compiler's 76 registers (24 warps) 1.49 ms, 2.50 ms, 182 us and 85 us; seven blocks of
+// four as eight, nine (spilling) 2.32 ms and 167 us.  Four heads per warp, one tile in flight: 2.60 ms and 190 us; more than
+// one tile in flight leaves too few warps.
+constexpr int kMergeHeads = 8, kMergeWarps = 16 / kMergeHeads, kMergeBlock = 4;   // warps per tile, per block
 template <bool SUM>
-__global__ void __launch_bounds__(256) sel_fwd_merge_kernel(const RevArgs a, const bf16* __restrict__ part,
+__global__ void __launch_bounds__(32 * kMergeBlock, 8) sel_fwd_merge_kernel(const RevArgs a, const bf16* __restrict__ part,
                                                             const float* __restrict__ stats, const SelMerge m, const int G16) {
   after_previous();
   constexpr int NV = kMergeHeads * D / 8 / 32;   // 16-byte vectors per lane: 4
-  const long long w4 = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const long long w4 = (long long)blockIdx.x * kMergeBlock + (threadIdx.x >> 5);
   const long long total = (long long)a.B * a.Tq * a.H * G16;
   const long long w = w4 / kMergeWarps;
   if (w >= total) return;
@@ -502,11 +504,11 @@ int launch_sel_fwd_kv(const SelKvArgs& a, const RevArgs& r, cudaStream_t s) {
   if (e != cudaSuccess) return (int)e;
   const int G16 = a.Hq / a.Hk / 16;
   const long long total = (long long)a.B * a.Tq * a.Hk * G16;
-  const unsigned nb = (unsigned)((kMergeWarps * total + 7) / 8);
+  const unsigned nb = (unsigned)((kMergeWarps * total + kMergeBlock - 1) / kMergeBlock);
   if (a.merge.out)
-    launch_next(sel_fwd_merge_kernel<true>, nb, 256, 0, s, r, a.part, a.stats, a.merge, G16);
+    launch_next(sel_fwd_merge_kernel<true>, nb, 32 * kMergeBlock, 0, s, r, a.part, a.stats, a.merge, G16);
   else
-    launch_next(sel_fwd_merge_kernel<false>, nb, 256, 0, s, r, a.part, a.stats, a.merge, G16);
+    launch_next(sel_fwd_merge_kernel<false>, nb, 32 * kMergeBlock, 0, s, r, a.part, a.stats, a.merge, G16);
   note_launches(1);
   return (int)cudaGetLastError();
 }
