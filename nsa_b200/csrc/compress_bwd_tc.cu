@@ -119,25 +119,27 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(sgen + (tmem_slot - sbase));
 
   if (warp == 0) {
-    if (lane == 0) mbar_expect_tx(a_full, (uint32_t)(R * NP * P * HB) * 128);
-    __syncwarp();
-    if (lane < R * NP)
-      tma_load_4d(sbase + (lane / NP) * A_TILE + (lane % NP) * PANEL, &maps.y[z], a_full, 0, h0,
-                  (int)t.out0 + t.i0 - lane / NP, lane % NP);
+    if (elect_one()) {
+      mbar_expect_tx(a_full, (uint32_t)(R * NP * P * HB) * 128);
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int p = 0; p < NP; ++p)
+          tma_load_4d(sbase + r * A_TILE + p * PANEL, &maps.y[z], a_full, 0, h0, (int)t.out0 + t.i0 - r, p);
+    }
   } else if (warp == 1) {
-    for (int n = 0; n < (j_hi - j_lo) * R; ++n) {
-      const int jj = j_lo + n / R, r = n % R;
-      const int stage = n % NR;
-      int good = 1;
-      if (lane == 0) {
-        good = mbar_wait(empty_bar(stage), ((n / NR) & 1) ^ 1, DEV_ERR_EMPTY_WAIT) ? 1 : 0;
-        if (good) mbar_expect_tx(full_bar(stage), W_TILE);
+    if (elect_one()) {
+      for (int n = 0; n < (j_hi - j_lo) * R; ++n) {
+        const int jj = j_lo + n / R, r = n % R;
+        const int stage = n % NR;
+        if (!mbar_wait(empty_bar(stage), ((n / NR) & 1) ^ 1, DEV_ERR_EMPTY_WAIT)) break;
+        mbar_expect_tx(full_bar(stage), W_TILE);
+#pragma unroll
+        for (int p = 0; p < NP; ++p)
+          tma_load_2d(ring + stage * W_TILE + p * W_PANEL, &maps.w[z], full_bar(stage), p * 64, (jj + r * a.d) * D);
       }
-      if (!__shfl_sync(0xffffffffu, good, 0)) break;
-      if (lane < NP) tma_load_2d(ring + stage * W_TILE + lane * W_PANEL, &maps.w[z], full_bar(stage), lane * 64, (jj + r * a.d) * D);
     }
   } else if (warp == 2) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc_bf16(128, D, 0, 0);   // both operands K-major (contraction over the outputs)
       bool ok = mbar_wait(a_ready, 0, DEV_ERR_FULL_WAIT);
       int n = 0;
@@ -268,33 +270,35 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   if (warp < 2) {
     // warp 0: the x panels, warp 1: dY
-    const int rem = (int)(a.total_in % a.d);
-    uint32_t k = 0;
-    for (long long n = n_lo; n < n_hi; ++n) {
-      const Tile t = tile_of(n);
-      if (t.i0 >= t.nout) continue;
-      const int h0 = (int)(n % nhg) * HB;
-      const int stage = k % NR;
-      int good = 1;
-      if (lane == 0) {
-        good = mbar_wait(empty_bar(stage), ((k / NR) & 1) ^ 1, DEV_ERR_EMPTY_WAIT) ? 1 : 0;
-        if (good) mbar_expect_tx(full_bar(stage), (uint32_t)(P * HB) * 128 * (warp == 0 ? XP : NP));
-      }
-      if (!__shfl_sync(0xffffffffu, good, 0)) break;
-      const uint32_t st = sbase + stage * STAGE;
-      if (warp == 0) {
-        if (lane < XP) {
-          const int r = (grp * XP + lane) * 64, j = r / D, c0 = r % D;   // first dW row of the panel
-          const int jj = (int)((t.in0 + j) % a.d), u = (int)((t.in0 + j) / a.d) + t.i0;
-          tma_load_5d(st + lane * PANEL, &maps.x[z][jj < rem ? 1 : 0], full_bar(stage), 0, h0, jj, u, c0 / 64);
+    if (elect_one()) {
+      const int rem = (int)(a.total_in % a.d);
+      uint32_t k = 0;
+      for (long long n = n_lo; n < n_hi; ++n) {
+        const Tile t = tile_of(n);
+        if (t.i0 >= t.nout) continue;
+        const int h0 = (int)(n % nhg) * HB;
+        const int stage = k % NR;
+        if (!mbar_wait(empty_bar(stage), ((k / NR) & 1) ^ 1, DEV_ERR_EMPTY_WAIT)) break;
+        mbar_expect_tx(full_bar(stage), (uint32_t)(P * HB) * 128 * (warp == 0 ? XP : NP));
+        const uint32_t st = sbase + stage * STAGE;
+        if (warp == 0) {
+          const int jj0 = (int)(t.in0 % a.d), u0 = (int)(t.in0 / a.d) + t.i0;
+#pragma unroll
+          for (int p = 0; p < XP; ++p) {
+            const int r = (grp * XP + p) * 64, j = jj0 + r / D, c0 = r % D;   // first dW row of the panel
+            const int jj = j % a.d;
+            tma_load_5d(st + p * PANEL, &maps.x[z][jj < rem ? 1 : 0], full_bar(stage), 0, h0, jj, u0 + j / a.d, c0 / 64);
+          }
+        } else {
+#pragma unroll
+          for (int p = 0; p < NP; ++p)
+            tma_load_4d(st + (XP + p) * PANEL, &maps.y[z], full_bar(stage), 0, h0, (int)t.out0 + t.i0, p);
         }
-      } else if (lane < NP) {
-        tma_load_4d(st + (XP + lane) * PANEL, &maps.y[z], full_bar(stage), 0, h0, (int)t.out0 + t.i0, lane);
+        ++k;
       }
-      ++k;
     }
   } else if (warp == 2) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc_bf16(128, D, 1, 1);   // both operands MN-major (contraction over the rows)
       uint32_t k = 0;
       bool ok = true;

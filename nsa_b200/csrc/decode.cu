@@ -406,10 +406,8 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
 
   if (warp >= CONS) {
     // ------------------------------- producers --------------------------------------------------------
-    // A warp's TMA instructions run one after another (about 850 + 52 x boxes cycles each, whatever the box size), so
-    // a single warp issuing one 16 KB tile per instruction caps the SM at ~16 bytes per clock.  Tiles therefore go out
-    // in PAIRS (four boxes per instruction: both tiles of a (K, V) pair, or two consecutive ck tiles of pass 1), and
-    // the producer warps (one in a CTA that shares its SM) take alternate pairs.
+    // Tiles go out in pairs (both tiles of a (K, V) pair, or two consecutive ck tiles of pass 1: the two slots of a consumer
+    // warp), and the producer warps (one in a CTA that shares its SM) take alternate pairs.
     const int pw = warp - CONS;
     uint32_t np = 0, it = 0;     // tile pairs issued so far by both producers together; items so far
     auto issue2 = [&](const CUtensorMap* tmA, int rowA, const CUtensorMap* tmB, int rowB, int h) -> bool {
@@ -418,22 +416,19 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
       ++np;
       if (!mine) return true;
       const uint32_t s0 = n % kSlots, ph = (n / kSlots) & 1;     // the pair's slots s0, s0+1 belong to one consumer warp
-      int good = 1;
-      if (lane == 0) {
-        good = mbar_wait_abortable(empty_bar(s0), ph ^ 1, DEV_ERR_EMPTY_WAIT, abort_flag) &&
-               mbar_wait_abortable(empty_bar(s0 + 1), ph ^ 1, DEV_ERR_EMPTY_WAIT, abort_flag) ? 1 : 0;
-        if (good) {
-          mbar_expect_tx(full_bar(s0), TILE);
-          mbar_expect_tx(full_bar(s0 + 1), TILE);
+      const bool good = mbar_wait_abortable(empty_bar(s0), ph ^ 1, DEV_ERR_EMPTY_WAIT, abort_flag) &&
+                        mbar_wait_abortable(empty_bar(s0 + 1), ph ^ 1, DEV_ERR_EMPTY_WAIT, abort_flag);
+      if (!__all_sync(0xffffffffu, good)) return false;
+      if (elect_one()) {
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+          mbar_expect_tx(full_bar(s0 + w), TILE);
+#pragma unroll
+          for (int p = 0; p < 2; ++p)
+            tma_load_4d(ring + (s0 + w) * TILE + p * PANEL, w ? tmB : tmA, full_bar(s0 + w), p * 64, h, w ? rowB : rowA, 0);
         }
       }
-      good = __shfl_sync(0xffffffffu, good, 0);
-      if (good && lane < 4) {
-        const int which = lane >> 1, panel = lane & 1;
-        tma_load_4d(ring + (s0 + which) * TILE + panel * PANEL, which ? tmB : tmA, full_bar(s0 + which), panel * 64, h,
-                    which ? rowB : rowA, 0);
-      }
-      return good != 0;
+      return true;
     };
     for (int r = 0; r * ngroup < nitem; ++r) {
       const int item = snake_item(r, group, ngroup);

@@ -82,22 +82,20 @@ __global__ void __launch_bounds__(kThreads, 1)
         const bool withv = i < sc.nAttn;
         const int jt = i < sc.nA ? i : i - sc.nA;
         const int stage = it % nst;
-        int good = 1;
-        if (lane == 0) {
-          const uint32_t ph = (it / nst) & 1;
-          good = mbar_wait(empty_bar(stage), ph ^ 1, DEV_ERR_EMPTY_WAIT) ? 1 : 0;
-          if (good) mbar_expect_tx(full_bar(stage), withv ? stage_bytes : tile_bytes);
-        }
-        if (!__shfl_sync(0xffffffffu, good, 0)) return;
-        if (lane < 2 * (D / 64)) {
-          const uint32_t dst = sbase + stage * stage_bytes;
-          const int p = lane >> 1;
-          if (lane & 1) {
-            if (withv) tma_load_4d(dst + tile_bytes + p * kPanel, &tmV, full_bar(stage), p * 64, hk, jt * 64, b);
-          } else {
-            tma_load_4d(dst + p * kPanel, &tmK, full_bar(stage), p * 64, hk, jt * 64, b);
+        bool good = true;
+        if (elect_one()) {
+          good = mbar_wait(empty_bar(stage), ((it / nst) & 1) ^ 1, DEV_ERR_EMPTY_WAIT);
+          if (good) {
+            mbar_expect_tx(full_bar(stage), withv ? stage_bytes : tile_bytes);
+            const uint32_t dst = sbase + stage * stage_bytes;
+#pragma unroll
+            for (int p = 0; p < D / 64; ++p) {
+              tma_load_4d(dst + p * kPanel, &tmK, full_bar(stage), p * 64, hk, jt * 64, b);
+              if (withv) tma_load_4d(dst + tile_bytes + p * kPanel, &tmV, full_bar(stage), p * 64, hk, jt * 64, b);
+            }
           }
         }
+        if (!__all_sync(0xffffffffu, good)) return;
         ++it;
       }
     }

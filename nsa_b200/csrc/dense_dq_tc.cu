@@ -129,41 +129,41 @@ __global__ void __launch_bounds__(kThreads, 1)
     const CUtensorMap* tmX = is_k ? &maps.q : &maps.dout;
     const uint32_t nst = is_k ? KST : VST;
     uint32_t c = 0, ic = 0;
-    int good = 1;
-    for (int item = blockIdx.x; good && item < total; item += gridDim.x) {
-      const int hg = item % HG;
-      const SeqTile st = seq_tile(a.seq, kTok, ntile - 1 - item / HG);
-      if (st.t0 >= st.Tq) continue;
-      const Sched sc = make_sched<WIN, CMP>(a, st);
-      const int hk = hg / G16;
-      for (int i = 0; good && i < max(sc.n, 1); ++i) {
-        if (i < sc.n) {
-          const uint32_t sl = c % nst;
-          if (lane == 0) {
-            good = mbar_wait_abortable(empty0 + 8 * sl, ((c / nst) & 1) ^ 1, 202, abort_flag) ? 1 : 0;
-            if (good) mbar_expect_tx(full0 + 8 * sl, TILE);
+    if (elect_one()) {
+      bool good = true;
+      for (int item = blockIdx.x; good && item < total; item += gridDim.x) {
+        const int hg = item % HG;
+        const SeqTile st = seq_tile(a.seq, kTok, ntile - 1 - item / HG);
+        if (st.t0 >= st.Tq) continue;
+        const Sched sc = make_sched<WIN, CMP>(a, st);
+        const int hk = hg / G16;
+        for (int i = 0; good && i < max(sc.n, 1); ++i) {
+          if (i < sc.n) {
+            const uint32_t sl = c % nst;
+            good = mbar_wait_abortable(empty0 + 8 * sl, ((c / nst) & 1) ^ 1, 202, abort_flag);
+            if (!good) break;
+            mbar_expect_tx(full0 + 8 * sl, TILE);
+            const bool win = WIN && (!CMP || i < sc.nw);
+            const CUtensorMap* tm = is_k ? (win ? &maps.k : &maps.ck) : (win ? &maps.v : &maps.cv);
+            const int row = win ? (sc.first + i) * 128 : (i - sc.nw) * 128;
+#pragma unroll
+            for (int p = 0; p < NP; ++p) tma_load_4d(ring + sl * TILE + p * PANEL, tm, full0 + 8 * sl, p * 64, hk, row, st.b);
+            ++c;
           }
-          good = __shfl_sync(0xffffffffu, good, 0);
-          const bool win = WIN && (!CMP || i < sc.nw);
-          const CUtensorMap* tm = is_k ? (win ? &maps.k : &maps.ck) : (win ? &maps.v : &maps.cv);
-          const int row = win ? (sc.first + i) * 128 : (i - sc.nw) * 128;
-          if (good && lane < NP) tma_load_4d(ring + sl * TILE + lane * PANEL, tm, full0 + 8 * sl, lane * 64, hk, row, st.b);
-          ++c;
-        }
-        if (i == 0 && good) {
-          if (lane == 0) {
-            good = mbar_wait_abortable(x_free, (ic & 1) ^ 1, 201, abort_flag) ? 1 : 0;
-            if (good) mbar_expect_tx(x_full, TILE);
+          if (i == 0) {
+            good = mbar_wait_abortable(x_free, (ic & 1) ^ 1, 201, abort_flag);
+            if (!good) break;
+            mbar_expect_tx(x_full, TILE);
+#pragma unroll
+            for (int p = 0; p < NP; ++p) tma_load_3d(x_s + p * PANEL, tmX, x_full, p * 64, hg * 16, (int)st.row0 + st.t0);
           }
-          good = __shfl_sync(0xffffffffu, good, 0);
-          if (good && lane < NP) tma_load_3d(x_s + lane * PANEL, tmX, x_full, lane * 64, hg * 16, (int)st.row0 + st.t0);
         }
+        ++ic;
       }
-      ++ic;
     }
   } else if (warp == 1) {
     // ------------------------------- MMA issuer: S and dP ---------------------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128, 0, 0);
       uint32_t c = 0, ic = 0;
       bool ok = true;
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else {
     // ------------------------------- MMA issuer: dQ ---------------------------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_dq = umma_idesc_bf16(128, D, 0, 1);
       uint32_t c = 0, ic = 0;
       bool ok = true;

@@ -129,39 +129,40 @@ __global__ void __launch_bounds__(kThreads, 1)
     const uint32_t full0 = is_k ? k_full0 : v_full0, empty0 = is_k ? k_empty0 : v_empty0, ring = is_k ? k_ring : v_ring;
     const CUtensorMap* tm = is_k ? &tmK : &tmV;
     uint32_t c = 0, ic = 0;
-    int good = 1;
-    for (int item = blockIdx.x; good && item < total; item += gridDim.x) {
-      const int hg = item % HG;
-      const SeqTile st = seq_tile(a.seq, kTok, ntile - 1 - item / HG);
-      if (st.t0 >= st.Tq) continue;
-      const Sched sc = make_sched<MODE>(a, st);
-      const int hk = hg / G16;
-      if (is_k) {
-        if (lane == 0) {
-          good = mbar_wait_abortable(q_free, (ic & 1) ^ 1, 101, abort_flag) ? 1 : 0;
-          if (good) mbar_expect_tx(q_full, 2 * TILE);
+    if (elect_one()) {
+      bool good = true;
+      for (int item = blockIdx.x; good && item < total; item += gridDim.x) {
+        const int hg = item % HG;
+        const SeqTile st = seq_tile(a.seq, kTok, ntile - 1 - item / HG);
+        if (st.t0 >= st.Tq) continue;
+        const Sched sc = make_sched<MODE>(a, st);
+        const int hk = hg / G16;
+        if (is_k) {
+          good = mbar_wait_abortable(q_free, (ic & 1) ^ 1, 101, abort_flag);
+          if (!good) break;
+          mbar_expect_tx(q_full, 2 * TILE);
+#pragma unroll
+          for (int t = 0; t < 2; ++t)
+#pragma unroll
+            for (int p = 0; p < NP; ++p)
+              tma_load_3d(q_s + t * TILE + p * PANEL, &tmQ, q_full, p * 64, hg * 16, (int)st.row0 + st.t0 + t * kTokT);
         }
-        good = __shfl_sync(0xffffffffu, good, 0);
-        if (good && lane < 2 * NP)   // lane = NP * tile + panel
-          tma_load_3d(q_s + (lane / NP) * TILE + (lane % NP) * PANEL, &tmQ, q_full, (lane % NP) * 64, hg * 16,
-                      (int)st.row0 + st.t0 + (lane / NP) * kTokT);
-      }
-      for (int i = 0; good && i < sc.n; ++i, ++c) {
-        const uint32_t sl = c & 1;
-        if (lane == 0) {
-          good = mbar_wait_abortable(empty0 + 8 * sl, ((c >> 1) & 1) ^ 1, 102, abort_flag) ? 1 : 0;
-          if (good) mbar_expect_tx(full0 + 8 * sl, TILE);
+        for (int i = 0; i < sc.n; ++i, ++c) {
+          const uint32_t sl = c & 1;
+          good = mbar_wait_abortable(empty0 + 8 * sl, ((c >> 1) & 1) ^ 1, 102, abort_flag);
+          if (!good) break;
+          mbar_expect_tx(full0 + 8 * sl, TILE);
+#pragma unroll
+          for (int p = 0; p < NP; ++p)
+            tma_load_4d(ring + sl * TILE + p * PANEL, tm, full0 + 8 * sl, p * 64, hk, (sc.first + i) * 128, st.b);
         }
-        good = __shfl_sync(0xffffffffu, good, 0);
-        if (good && lane < NP)
-          tma_load_4d(ring + sl * TILE + lane * PANEL, tm, full0 + 8 * sl, lane * 64, hk, (sc.first + i) * 128, st.b);
+        ++ic;
       }
-      ++ic;
     }
   } else if (warp == 1) {
     // ------------------------------- MMA issuer: S ---------------------------------------------------
     // S of a group's tile c as soon as its K tile has landed and the group holds tile c - 1 in registers
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128, 0, 0);
       uint32_t c = 0, ic = 0;     // tiles so far; items so far
       bool ok = true;
@@ -196,7 +197,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (warp == 2) {
     // ------------------------------- MMA issuer: P.V -------------------------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_pv = umma_idesc_bf16(128, D, 0, 1);
       uint32_t c0 = 0;            // tiles of the items before
       uint32_t npi = 0;           // items with tiles so far (= o_free phases the groups will have arrived on)

@@ -171,32 +171,29 @@ __global__ void __launch_bounds__(kThreads, 1)
       const uint32_t full0 = is_k ? q_full0 : do_full0, empty0 = is_k ? q_empty0 : do_empty0, ring = is_k ? q_ring : do_ring;
       const uint32_t nst = is_k ? QST : DST;
       const CUtensorMap* tmX = is_k ? &tmQ : &tmDO;
-      if (N > 0) {
-        if (lane == 0) mbar_expect_tx(is_k ? k_full : v_full, TILE);
-        __syncwarp();
-        if (lane < NP)
-          tma_load_4d((is_k ? k_s : v_s) + lane * PANEL, is_k ? &tmK : &tmV, is_k ? k_full : v_full, lane * 64, it.hk, it.key0, it.b);
-      }
-      int good = 1;
-      for (int c = 0; good && c < N; ++c) {
-        int hg;
-        const int t0 = tile_of(c, hg);
-        const uint32_t sl = c % nst;
-        if (lane == 0) {
-          good = mbar_wait_abortable(empty0 + 8 * sl, ((c / nst) & 1) ^ 1, 331, abort_flag) ? 1 : 0;
-          if (good) mbar_expect_tx(full0 + 8 * sl, TILE);
-        }
-        good = __shfl_sync(0xffffffffu, good, 0);
-        if (good && lane < NP) {
-          if (BYSEQ)
-            tma_load_4d(ring + sl * TILE + lane * PANEL, tmX, full0 + 8 * sl, lane * 64, hg * 16, t0, it.b);
-          else
-            tma_load_3d(ring + sl * TILE + lane * PANEL, tmX, full0 + 8 * sl, lane * 64, hg * 16, (int)it.row0 + t0);
+      if (N > 0 && elect_one()) {
+        mbar_expect_tx(is_k ? k_full : v_full, TILE);
+#pragma unroll
+        for (int p = 0; p < NP; ++p)
+          tma_load_4d((is_k ? k_s : v_s) + p * PANEL, is_k ? &tmK : &tmV, is_k ? k_full : v_full, p * 64, it.hk, it.key0, it.b);
+        for (int c = 0; c < N; ++c) {
+          int hg;
+          const int t0 = tile_of(c, hg);
+          const uint32_t sl = c % nst;
+          if (!mbar_wait_abortable(empty0 + 8 * sl, ((c / nst) & 1) ^ 1, 331, abort_flag)) break;
+          mbar_expect_tx(full0 + 8 * sl, TILE);
+#pragma unroll
+          for (int p = 0; p < NP; ++p) {
+            if (BYSEQ)
+              tma_load_4d(ring + sl * TILE + p * PANEL, tmX, full0 + 8 * sl, p * 64, hg * 16, t0, it.b);
+            else
+              tma_load_3d(ring + sl * TILE + p * PANEL, tmX, full0 + 8 * sl, p * 64, hg * 16, (int)it.row0 + t0);
+          }
         }
       }
     } else if (warp == 1) {
       // ------------------------------- MMA issuer: dV(n), S^T(n+1) -----------------------------------------
-      if (lane == 0 && N > 0) {
+      if (N > 0 && elect_one()) {
         constexpr uint32_t idesc_s = umma_idesc_bf16(128, 64, 0, 0), idesc_dv = umma_idesc_bf16(128, D, 0, 1);
         const uint64_t dk = umma_smem_desc(k_s, 0, 1024), dq_base = umma_smem_desc(q_ring, 0, 1024);
         const uint64_t ddo_base = umma_smem_desc(do_ring, PANEL, 1024);
@@ -235,7 +232,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     } else {
       // ------------------------------- MMA issuer: dK(n), dP^T(n+1) ----------------------------------------
-      if (lane == 0 && N > 0) {
+      if (N > 0 && elect_one()) {
         constexpr uint32_t idesc_s = umma_idesc_bf16(128, 64, 0, 0), idesc_dk = umma_idesc_bf16(128, D, 0, 1);
         const uint64_t dv = umma_smem_desc(v_s, 0, 1024), ddo_base = umma_smem_desc(do_ring, 0, 1024);
         const uint64_t dq_base = umma_smem_desc(q_ring, PANEL, 1024);

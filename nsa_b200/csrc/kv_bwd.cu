@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   if (warp == kConsumerWarps) {
     // ------------------------------- producer ------------------------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(kv_bar, 2 * kv_tile);
 #pragma unroll
       for (int p = 0; p < D / 64; ++p) {
@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int j = 0; j < nn; ++j) {
           const int t = __shfl_sync(0xffffffffu, tok, j);
           bool okw = true;
-          if (lane == 0) {
+          if (elect_one()) {
             const int stage = it % nst;
             const uint32_t ph = (it / nst) & 1;
             okw = mbar_wait(empty_bar(stage), ph ^ 1, DEV_ERR_EMPTY_WAIT);
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(kThreads, 1)
               if (a.gate) bulk_load(dst + 2 * q_tile + 128, a.gate + qrow, 32, full_bar(stage));
             }
           }
-          if (!__shfl_sync(0xffffffffu, (int)okw, 0)) return;
+          if (!__all_sync(0xffffffffu, okw)) return;
           ++it;
         }
       }

@@ -35,13 +35,9 @@ namespace nsa {
 namespace {
 
 constexpr int D = 128;
-constexpr int kProd = 2;                   // TMA producer warps (a warp's TMA instructions run one after another,
-                                           // ~900 cycles each whatever their size, so the boxes of a batch are
-                                           // spread over two warps and issued by one instruction per warp)
+constexpr int kProd = 2;                   // TMA producer warps: Q, dO
 constexpr int kMmaWarp = 2;                // issues S and dP
-constexpr int kMma2Warp = 3;               // issues dV, dK and the dQ partials: tcgen05.mma costs its issuing thread
-                                           // ~60 cycles per instruction, so two threads issue the kernel's 32-36 MMAs
-                                           // per batch
+constexpr int kMma2Warp = 3;               // issues dV, dK and the dQ partials
 constexpr int kSoftWarp = 4;               // eight soft-max / epilogue warps
 constexpr int kDrainWarp = 12;             // four more warps read the dQ partials out of tensor memory
 constexpr int kThreads = 16 * 32;          // 512: four warpgroups, registers redistributed by setmaxnreg
@@ -151,9 +147,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     // ------------------------------- TMA producers -----------------------------------------------
     // A batch of gathered tokens (a reverse-index list) is 16 boxes of 4 KB, one per token of Q and one of dO, through a 4-D
     // view (64 columns, 8 rows, 2 column panels, row groups) as in the forward: the gather is bound by the number of
-    // boxes.  Box x = 2 * lane + warp belongs to this lane; every producer warp issues its eight with a single instruction
-    // and arms the stage's barrier with their byte count.  Token ids are fetched one batch ahead.
-    if (warp == 0 && lane == 0 && nb > 0) {
+    // boxes.  Warp 0 gathers Q, warp 1 dO; lane j finds where the batch's token j is, one lane issues the eight boxes and
+    // arms the stage's barrier with their byte count.  Token ids are fetched one batch ahead.
+    if (warp == 0 && nb > 0 && elect_one()) {
       mbar_expect_tx(kv_bar, 2 * KV_TILE);
 #pragma unroll
       for (int p = 0; p < 2; ++p) {
@@ -173,22 +169,23 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int stage = n % kStages;
       const uint32_t ph = (n / kStages) & 1;
       const uint32_t fb = full0 + 8 * stage;
-      int good = 1;
-      if (lane == 0) {
-        good = mbar_wait(empty0 + 8 * stage, ph ^ 1, DEV_ERR_EMPTY_WAIT) ? 1 : 0;
-        if (good) mbar_expect_tx(fb, Q_TILE);
-      }
-      if (!__shfl_sync(0xffffffffu, good, 0)) break;
-      if (has) {
-        const int qrow = (int)(((long long)b * a.Tq + (tk - a.q0)) * a.Hq + hg * 16);
-        tma_load_4d(dst0 + stage * STAGE + lane * 4096, tm, fb, 0, 0, 0, qrow >> 3);
+      const int grp = (int)((((long long)b * a.Tq + (tk - a.q0)) * a.Hq + hg * 16) >> 3);
+      int row_group[kTokB];
+#pragma unroll
+      for (int j = 0; j < kTokB; ++j) row_group[j] = __shfl_sync(0xffffffffu, grp, j);
+      const bool good = mbar_wait(empty0 + 8 * stage, ph ^ 1, DEV_ERR_EMPTY_WAIT);
+      if (!__all_sync(0xffffffffu, good)) break;
+      if (elect_one()) {
+        mbar_expect_tx(fb, Q_TILE);
+#pragma unroll
+        for (int j = 0; j < kTokB; ++j) tma_load_4d(dst0 + stage * STAGE + j * 4096, tm, fb, 0, 0, 0, row_group[j]);
       }
     }
   } else if (warp == kMmaWarp) {
     // ------------------------------- MMA issuer A: S and dP ----------------------------------------
     // S/dP of batch n is issued as soon as its Q/dO stage has landed and its TMEM buffer is free (the soft-max warps
     // hold batch n-2 in registers), i.e. ahead of dV/dK of batch n-1, which the second issuer handles.
-    if (lane == 0 && nb > 0) {
+    if (nb > 0 && elect_one()) {
       constexpr uint32_t idesc_kk = umma_idesc_bf16(128, 64, 0, 0);   // both operands K-major
       bool ok = mbar_wait(kv_bar, 0, DEV_ERR_FULL_WAIT);
       const uint64_t dK = umma_smem_desc(k_s, 0, 1024), dV = umma_smem_desc(v_s, 0, 1024);
@@ -226,7 +223,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (warp == kMma2Warp) {
     // ------------------------------- MMA issuer B: dV, dK, dQ partials -----------------------------
-    if (lane == 0 && nb > 0) {
+    if (nb > 0 && elect_one()) {
       constexpr uint32_t idesc_mn = umma_idesc_bf16(128, 64, 1, 1);   // both operands MN-major
       constexpr uint32_t idesc_dq = umma_idesc_bf16(128, 128, 0, 1);  // A = dS K-major, B = K MN-major
       bool ok = mbar_wait(kv_bar, 0, DEV_ERR_FULL_WAIT);

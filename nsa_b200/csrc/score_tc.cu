@@ -159,40 +159,37 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (warp == 0) {
       // ------------------------------- TMA producer ------------------------------------------------
       uint32_t ck = 0, ic = 0;
-      bool alive = true;
-      for (int item = blockIdx.x; alive && item < total; item += gridDim.x) {
-        const int hg = item % HG;
-        const SeqTile st = seq_tile(a.seq, kTok, ntile - 1 - item / HG);
-        const int nt = tiles_of(st);
-        if (st.t0 >= st.Tq || nt == 0) continue;
-        int good = 1;
-        const uint32_t qs = ic % (uint32_t)QST;   // two Q slots: the next item's tiles land while this one is scored
-        if (lane == 0) {
-          good = mbar_wait_abortable(q_free0 + 8 * qs, ((ic / (uint32_t)QST) & 1) ^ 1, 301, abort_flag) ? 1 : 0;
-          if (good) mbar_expect_tx(q_full0 + 8 * qs, 2 * TILE);
-        }
-        if (!__shfl_sync(0xffffffffu, good, 0)) break;
-        if (lane < 4)   // lane = 2 * tile + panel
-          tma_load_3d(q_s + (2 * qs + (lane >> 1)) * TILE + (lane & 1) * PANEL, &tmQ, q_full0 + 8 * qs, (lane & 1) * 64, hg * 16,
-                      (int)(st.row0 + st.t0) + (lane >> 1) * kTokT);
-        for (int i = 0; i < 2 * nt; ++i, ++ck) {
-          const uint32_t ks = ck % (uint32_t)KST;
-          if (lane == 0) {
-            good = mbar_wait_abortable(k_empty0 + 8 * ks, ((ck / (uint32_t)KST) & 1) ^ 1, 302, abort_flag) ? 1 : 0;
-            if (good) mbar_expect_tx(k_full0 + 8 * ks, TILE);
+      if (elect_one()) {
+        bool good = true;
+        for (int item = blockIdx.x; good && item < total; item += gridDim.x) {
+          const int hg = item % HG;
+          const SeqTile st = seq_tile(a.seq, kTok, ntile - 1 - item / HG);
+          const int nt = tiles_of(st);
+          if (st.t0 >= st.Tq || nt == 0) continue;
+          const uint32_t qs = ic % (uint32_t)QST;   // two Q slots: the next item's tiles land while this one is scored
+          good = mbar_wait_abortable(q_free0 + 8 * qs, ((ic / (uint32_t)QST) & 1) ^ 1, 301, abort_flag);
+          if (!good) break;
+          mbar_expect_tx(q_full0 + 8 * qs, 2 * TILE);
+#pragma unroll
+          for (int x = 0; x < 4; ++x)   // x = 2 * tile + panel
+            tma_load_3d(q_s + (2 * qs + (x >> 1)) * TILE + (x & 1) * PANEL, &tmQ, q_full0 + 8 * qs, (x & 1) * 64, hg * 16,
+                        (int)(st.row0 + st.t0) + (x >> 1) * kTokT);
+          for (int i = 0; i < 2 * nt; ++i, ++ck) {
+            const uint32_t ks = ck % (uint32_t)KST;
+            good = mbar_wait_abortable(k_empty0 + 8 * ks, ((ck / (uint32_t)KST) & 1) ^ 1, 302, abort_flag);
+            if (!good) break;
+            mbar_expect_tx(k_full0 + 8 * ks, TILE);
+            const int jt = i < nt ? i : i - nt;
+#pragma unroll
+            for (int p = 0; p < 2; ++p)
+              tma_load_4d(k_ring + ks * TILE + p * PANEL, &tmK, k_full0 + 8 * ks, p * 64, hg / G16, jt * 128, st.b);
           }
-          if (!__shfl_sync(0xffffffffu, good, 0)) {
-            alive = false;
-            break;
-          }
-          const int jt = i < nt ? i : i - nt;
-          if (lane < 2) tma_load_4d(k_ring + ks * TILE + lane * PANEL, &tmK, k_full0 + 8 * ks, lane * 64, hg / G16, jt * 128, st.b);
+          ++ic;
         }
-        ++ic;
       }
     } else if (warp == 1) {
       // ------------------------------- MMA issuer ----------------------------------------------------
-      if (lane == 0) {
+      if (elect_one()) {
         constexpr uint32_t idesc = umma_idesc_bf16(128, 128, 0, 0);
         uint32_t ck = 0, ic = 0;
         bool ok = true;

@@ -210,10 +210,6 @@ __global__ void __launch_bounds__(2 * kWarps * 32, 1)
 
   if (warp >= kWarps) {
     // ------------------------------- producer of consumer warp cw ---------------------------------
-    // lane -> (K or V, panel) for block boxes, (Q or dO, panel) for row tiles; every issuing lane waits for its own
-    // slot, the first lane of a slot also arms the barrier
-    const int bkv = lane / NP, bp = lane % NP;
-    const int qwhich = lane / NP, qp = lane % NP;
     int ent_next = fetch_entry(a, decode_item(a, first, total, HG, G16), lane);
     for (long long idx = first; idx < total; idx += step) {
       const Item item = decode_item(a, idx, total, HG, G16);
@@ -221,13 +217,17 @@ __global__ void __launch_bounds__(2 * kWarps * 32, 1)
       unsigned mask = __ballot_sync(0xffffffffu, ent >= 0);
       ent_next = fetch_entry(a, decode_item(a, idx + step, total, HG, G16), lane);
       if (mask == 0) continue;
-      int good = 1;
-      if (lane < NQ * NP) {
-        good = mbar_wait_abortable(qempty_bar(cw), (qn & 1) ^ 1, DEV_ERR_EMPTY_WAIT, abort_flag) ? 1 : 0;
+      bool good = true;
+      if (elect_one()) {
+        good = mbar_wait_abortable(qempty_bar(cw), (qn & 1) ^ 1, DEV_ERR_EMPTY_WAIT, abort_flag);
         if (good) {
-          if (lane == 0) mbar_expect_tx(qfull_bar(cw), NQ * qtile_bytes);
-          tma_load_2d(sbase + q_off + (cw * NQ + qwhich) * qtile_bytes + qp * qpanel_bytes, qwhich ? &tmDO : &tmQ,
-                      qfull_bar(cw), qp * 64, (int)item.qrow);
+          mbar_expect_tx(qfull_bar(cw), NQ * qtile_bytes);
+#pragma unroll
+          for (int x = 0; x < NQ; ++x)
+#pragma unroll
+            for (int p = 0; p < NP; ++p)
+              tma_load_2d(sbase + q_off + (cw * NQ + x) * qtile_bytes + p * qpanel_bytes, x ? &tmDO : &tmQ, qfull_bar(cw), p * 64,
+                          (int)item.qrow);
         }
       }
       ++qn;
@@ -236,22 +236,28 @@ __global__ void __launch_bounds__(2 * kWarps * 32, 1)
         const int bit = __ffs(mask) - 1;
         mask &= mask - 1;
         const int blk = __shfl_sync(0xffffffffu, ent, bit);
-        if (lane < 2 * NP) {
+        if (elect_one()) {
           // Forward: K takes the ring position `rs`, V the next one.  Backward: V first, then K -- V is released
           // after dP, well before the block ends, and the slot freed early is the one the SECOND tensor of the next
           // block reuses (three slots per ring), so both tensors of the next block land while this one computes.
-          int stage = rs;
+          int slot = rs;
           uint32_t par = rp;
-          if ((BWD ? !bkv : bkv) && ++stage == spw) {
-            stage = 0;
-            par ^= 1;
-          }
-          stage += ring0;
-          good = mbar_wait_abortable(empty_bar(stage), par ^ 1, DEV_ERR_EMPTY_WAIT, abort_flag) ? 1 : 0;
-          if (good) {
-            if (bp == 0) mbar_expect_tx(full_bar(stage), slot_bytes);
-            tma_load_4d(sbase + stage * slot_bytes + bp * panel_bytes, bkv ? &tmV : &tmK, full_bar(stage), bp * 64,
-                        item.hkv, blk * BS, item.b);
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            const bool is_v = BWD ? x == 0 : x == 1;
+            const int stage = ring0 + slot;
+            good = good && mbar_wait_abortable(empty_bar(stage), par ^ 1, DEV_ERR_EMPTY_WAIT, abort_flag);
+            if (good) {
+              mbar_expect_tx(full_bar(stage), slot_bytes);
+#pragma unroll
+              for (int p = 0; p < NP; ++p)
+                tma_load_4d(sbase + stage * slot_bytes + p * panel_bytes, is_v ? &tmV : &tmK, full_bar(stage), p * 64, item.hkv,
+                            blk * BS, item.b);
+            }
+            if (++slot == spw) {
+              slot = 0;
+              par ^= 1;
+            }
           }
         }
         ring_advance2();

@@ -26,7 +26,7 @@ namespace {
 constexpr int D = 128;
 constexpr int kProd = 2;
 constexpr int kMmaWarp = kProd;             // issues S
-constexpr int kMma2Warp = kProd + 1;        // issues P.V: one thread for both took 900 cycles for either
+constexpr int kMma2Warp = kProd + 1;        // issues P.V
 constexpr int kSoftWarp = kProd + 2;        // 8 soft-max warps: two groups of four
 constexpr int kDrainWarp = kSoftWarp + 8;   // 4 drain warps
 constexpr int kThreads = (kDrainWarp + 4) * 32;
@@ -110,9 +110,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     // a batch is 8 boxes of 4 KB, one per token: the token's [16 heads x 128 d] rows through a 4-D view of q
     // (64 columns, 8 rows, 2 column panels, row groups) land as [row group][panel][8 rows][128 B], so the 8-row swizzle
     // atoms of one panel sit 2 KB apart over the whole tile (SBO = 2048, second panel at +1 KB).  One box per token
-    // instead of one per (token, panel): the gather is bound by the number of boxes.  Box x = 2 * lane + warp belongs
-    // to this lane
-    if (warp == 0 && lane == 0) {
+    // instead of one per (token, panel): the gather is bound by the number of boxes.  Lane j finds
+    // where the token of the warp's box j is, one lane issues the warp's four
+    if (warp == 0 && elect_one()) {
       mbar_expect_tx(kv_bar, 2 * KV_TILE);
 #pragma unroll
       for (int p = 0; p < 2; ++p) {
@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int x = kProd * lane + warp;
     const bool has = x < kTokB;
     const int bj = x;
-    const int nmine = (kTokB - warp + kProd - 1) / kProd;
+    constexpr int kMine = kTokB / kProd;   // boxes of this warp
     int tk_next = has ? token(bj) : 0;
     for (int n = 0; n < nb; ++n) {
       const int tk = tk_next;
@@ -134,20 +134,22 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int stage = n % kStages;
       const uint32_t ph = (n / kStages) & 1;
       const uint32_t fb = full0 + 8 * stage;
-      int good = 1;
-      if (lane == 0) {
-        good = mbar_wait(empty0 + 8 * stage, ph ^ 1, DEV_ERR_EMPTY_WAIT) ? 1 : 0;
-        if (good) mbar_expect_tx(fb, nmine * 4096);
-      }
-      if (!__shfl_sync(0xffffffffu, good, 0)) break;
-      if (has) {
-        const int qrow = (int)(((long long)b * a.Tq + (tk - a.q0)) * a.Hq + hg * 16);
-        tma_load_4d(ring + stage * Q_TILE + bj * 4096, &tmQ, fb, 0, 0, 0, qrow >> 3);
+      const int grp = (int)((((long long)b * a.Tq + (tk - a.q0)) * a.Hq + hg * 16) >> 3);
+      int row_group[kMine];
+#pragma unroll
+      for (int j = 0; j < kMine; ++j) row_group[j] = __shfl_sync(0xffffffffu, grp, j);
+      const bool good = mbar_wait(empty0 + 8 * stage, ph ^ 1, DEV_ERR_EMPTY_WAIT);
+      if (!__all_sync(0xffffffffu, good)) break;
+      if (elect_one()) {
+        mbar_expect_tx(fb, kMine * 4096);
+#pragma unroll
+        for (int j = 0; j < kMine; ++j)
+          tma_load_4d(ring + stage * Q_TILE + (kProd * j + warp) * 4096, &tmQ, fb, 0, 0, 0, row_group[j]);
       }
     }
   } else if (nb > 0 && warp == kMmaWarp) {
     // ------------------------------- MMA issuer A: S ------------------------------------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, 64, 0, 0);    // both operands K-major
       bool ok = mbar_wait(kv_bar, 0, DEV_ERR_FULL_WAIT);
       const uint64_t dK = umma_smem_desc(k_s, 0, 1024), dQ0 = umma_smem_desc(ring, 0, 2048);
@@ -170,7 +172,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (nb > 0 && warp == kMma2Warp) {
     // ------------------------------- MMA issuer B: P.V ----------------------------------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_o = umma_idesc_bf16(128, 128, 0, 1);   // A = P in tensor memory, B = V MN-major
       bool ok = mbar_wait(kv_bar, 0, DEV_ERR_FULL_WAIT);
       const uint64_t dVmn = umma_smem_desc(v_s, KV_PANEL, 1024);
