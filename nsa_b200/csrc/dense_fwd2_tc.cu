@@ -123,8 +123,6 @@ __global__ void __launch_bounds__(kThreads, 1)
   asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
   if (warp == 0 || warp == 3) {
     // ------------------------------- TMA producers: Q and K (warp 0), V (warp 3) -------------------------
-    // (A warp's TMA instructions run one after another, about 950 cycles each: one warp for both rings took 2800 cycles per
-    // pair of tiles with nothing else going on.)
     const bool is_k = warp == 0;
     const uint32_t full0 = is_k ? k_full0 : v_full0, empty0 = is_k ? k_empty0 : v_empty0, ring = is_k ? k_ring : v_ring;
     const CUtensorMap* tm = is_k ? &tmK : &tmV;

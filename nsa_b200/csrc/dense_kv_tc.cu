@@ -17,7 +17,9 @@
 // cycles per tile.  Tried: whole tiles (32 products): S^T(n+1) waits for P^T(n) and dV(n), 4150; whole tiles with S^T(n+1) over
 // dP^T(n) as soon as that is in registers, in one or two issuing threads: 3600.
 // Window, 8 x 8192 tokens, 64 heads, 4 KV heads, window 512: 3670 us (64-key CTAs, below) -> 2260; compressed 1900 -> 1270;
-// 32768 tokens, compressed 3700 -> 1970; 1024 tokens, head_dim 64 (mma.sync before), compressed 654 -> 23.
+// 32768 tokens, compressed 3700 -> 1970; 1024 tokens, head_dim 64 (mma.sync before), compressed 654 -> 23.  Products issued
+// under elect_one instead of a lane number, so that issuing is no longer what takes the time: both together 4.11 -> 3.53 ms at
+// 8 x 8192 tokens (below full clocks), 128 -> 107 us at 2 x 2080 tokens, 32 heads.
 // The keys of a 64-row CTA with P and dS in shared memory (this kernel's predecessor, still the selected branch's) took the same
 // number of products for half the keys.
 //

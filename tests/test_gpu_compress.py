@@ -55,6 +55,27 @@ def test_compress_pair_fwd_bwd(nsa, D, H, block, stride, lens, split):
     nsa._lib.device_status()
 
 
+@pytest.mark.parametrize("D,H,lens", [(128, 4, [13007, 12999, 12100]), (128, 4, [15001, 16010]), (64, 4, [13007, 12999, 12100]),
+                                      (128, 130, [640, 523])])
+def test_forward_tile_of_a_call_keeps_the_bits(nsa, D, H, lens):
+    """Few rows: half of the columns per CTA; a little more than one CTA per SM: two row tiles; else one.  A sequence gets the same
+    bits from the tile that it gets alone and from the packed call's."""
+    gen = torch.Generator(device=DEV).manual_seed(D + H)
+    rnd = lambda *s, m=1.0: (torch.randn(*s, generator=gen, device=DEV) * m).bfloat16()
+    cu = [sum(lens[:i]) for i in range(len(lens) + 1)]
+    n_out = [(n - 32) // 16 + 1 for n in lens]
+    cu_out = [sum(n_out[:i]) for i in range(len(n_out) + 1)]
+    k, v, w_k, w_v, b = rnd(cu[-1], H, D), rnd(cu[-1], H, D), rnd(32 * D, D, m=0.03), rnd(32 * D, D, m=0.03), rnd(D)
+    run = lambda i, j: nsa.compression_kv._CompressPair.apply(k[cu[i]:cu[j]], v[cu[i]:cu[j]], w_k, w_v, b, b, [c - cu[i] for c in cu[i:j + 1]],
+                                                              [c - cu_out[i] for c in cu_out[i:j + 1]], 32, 16, False)
+    packed = run(0, len(lens))
+    for i in range(len(lens)):
+        for alone, both in zip(run(i, i + 1), packed):
+            assert torch.equal(alone, both[cu_out[i]:cu_out[i + 1]])
+    _close("ck", packed[0][:n_out[0]], _ref(k[:lens[0]].float(), w_k.float(), b.float(), [0, lens[0]], 32, 16, n_out[:1]))
+    nsa._lib.device_status()
+
+
 @pytest.mark.parametrize("D,block,stride", [(128, 32, 16), (64, 64, 32)])
 def test_conv_weight_layout(nsa, D, block, stride):
     w = torch.randn(D, D, block, device=DEV).bfloat16().requires_grad_(True)
