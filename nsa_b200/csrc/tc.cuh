@@ -61,6 +61,13 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
+// A warp's 32 rows, one per thread as they come out of tensor memory, meet in shared memory and are stored as contiguous lines
+// (16 bytes per lane at a row's stride touch 32 lines with every store).  The 16-byte chunk c of row r sits at c ^ (r & 7): no
+// bank conflicts either way.
+__device__ __forceinline__ uint4* staged(uint8_t* warp_rows, int row_bytes, int r, int c) {
+  return reinterpret_cast<uint4*>(warp_rows + r * row_bytes + (c ^ (r & 7)) * 16);
+}
+
 // 16 consecutive fp32 columns.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   uint32_t r[16];
