@@ -47,9 +47,13 @@ __device__ __forceinline__ float group_sum(float v) {
   return v;
 }
 
-// gates[row][g] = q[row] . W[g] + b[g], written to three contiguous [rows] tensors
+// gates[row][g] = q[row] . W[g] + b[g], written to three contiguous [rows] tensors.  Eight rows per lane group and no loop; the group
+// sums them by halves (every exchange leaves a lane half of the rows: the sums of a butterfly, in a quarter of its shuffles), and
+// ends with a row per lane pair, so a gate of 16 rows is one store.  Bound by reading q and by issue (24 products, 8 conversions per
+// 16 bytes): 8 x 8192 tokens, 64 heads 300 -> 235 us (4.6 TB/s), 5003 tokens 26.5 -> 24.2; left to the compiler 253, four rows per
+// lane 263.
 template <int D>
-__global__ void __launch_bounds__(kGateThreads) gate_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w,
+__global__ void __launch_bounds__(kGateThreads, 4) gate_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w,
                                                                const bf16* __restrict__ bias, bf16* __restrict__ g0,
                                                                bf16* __restrict__ g1, bf16* __restrict__ g2, long long rows) {
   after_previous();
@@ -63,35 +67,47 @@ __global__ void __launch_bounds__(kGateThreads) gate_fwd_kernel(const bf16* __re
     bv[g] = bias ? __bfloat162float(bias[g]) : 0.f;
   }
   const long long warp0 = (long long)blockIdx.x * (kGateThreads / 32) + (threadIdx.x >> 5);
-  const long long nwarp = (long long)gridDim.x * (kGateThreads / 32);
   constexpr int U = 8;   // rows in flight per lane (raw 16-byte loads, converted when used)
-  for (long long r0 = warp0 * RPW * U; r0 < rows; r0 += nwarp * RPW * U) {
-    uint4 raw[U];
+  const long long r0 = warp0 * RPW * U;
+  uint4 raw[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const long long row = r0 + u * RPW + rw;
-      raw[u] = make_uint4(0u, 0u, 0u, 0u);
-      if (row < rows) raw[u] = ldraw(q + row * D + sub * 8);
+  for (int u = 0; u < U; ++u) {
+    const long long row = r0 + u * RPW + rw;
+    raw[u] = make_uint4(0u, 0u, 0u, 0u);
+    if (row < rows) raw[u] = ldraw(q + row * D + sub * 8);
+  }
+  float acc[3][U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    float xu[8];
+    cvt8(raw[u], xu);
+#pragma unroll
+    for (int g = 0; g < 3; ++g) {
+      acc[g][u] = 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) acc[g][u] += xu[k] * wv[g][k];
     }
+  }
+  int u = 0;   // of the rows, the one whose sums this lane ends up with
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const long long row = r0 + u * RPW + rw;
-      float xu[8];
-      cvt8(raw[u], xu);
-      float acc[3];
+  for (int off = LPR / 2, n = U / 2; off > 0; off >>= 1, n >>= 1) {
+    const bool hi = (sub & off) != 0;
+    if (n) u += hi ? n : 0;
 #pragma unroll
-      for (int g = 0; g < 3; ++g) {
-        float s = 0.f;
+    for (int g = 0; g < 3; ++g) {
+      if (n == 0) acc[g][0] += __shfl_xor_sync(0xffffffffu, acc[g][0], off);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) s += xu[k] * wv[g][k];
-        acc[g] = group_sum<LPR>(s) + bv[g];
-      }
-      if (row < rows && sub == 0) {
-        g0[row] = __float2bfloat16(acc[0]);
-        g1[row] = __float2bfloat16(acc[1]);
-        g2[row] = __float2bfloat16(acc[2]);
+      for (int e = 0; e < n; ++e) {
+        const float send = hi ? acc[g][e] : acc[g][e + n], keep = hi ? acc[g][e + n] : acc[g][e];
+        acc[g][e] = keep + __shfl_xor_sync(0xffffffffu, send, off);
       }
     }
+  }
+  const long long row = r0 + u * RPW + rw;
+  if (row < rows && sub % (LPR / U) == 0) {
+    g0[row] = __float2bfloat16(acc[0][0] + bv[0]);
+    g1[row] = __float2bfloat16(acc[1][0] + bv[1]);
+    g2[row] = __float2bfloat16(acc[2][0] + bv[2]);
   }
 }
 
@@ -270,9 +286,9 @@ int launch_gate_fwd(const bf16* q, const bf16* w, const bf16* bias, bf16* g0, bf
                     cudaStream_t s) {
   if (rows <= 0) return 0;
   if (D == 128)
-    launch_next(gate_fwd_kernel<128>, stream_grid(gate_fwd_kernel<128>, rows, 16), kGateThreads, 0, s, q, w, bias, g0, g1, g2, rows);
+    launch_next(gate_fwd_kernel<128>, (unsigned)((rows + 127) / 128), kGateThreads, 0, s, q, w, bias, g0, g1, g2, rows);
   else if (D == 64)
-    launch_next(gate_fwd_kernel<64>, stream_grid(gate_fwd_kernel<64>, rows, 32), kGateThreads, 0, s, q, w, bias, g0, g1, g2, rows);
+    launch_next(gate_fwd_kernel<64>, (unsigned)((rows + 255) / 256), kGateThreads, 0, s, q, w, bias, g0, g1, g2, rows);
   else {
     set_error("head_dim %d not supported (64 or 128)", D);
     return -2;
