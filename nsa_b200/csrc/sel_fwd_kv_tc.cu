@@ -42,7 +42,7 @@ constexpr uint32_t kColO = 128, kColP = 384;
 
 __global__ void __launch_bounds__(kThreads, 1)
     sel_fwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                      const __grid_constant__ CUtensorMap tmV, const SelKvArgs a, const int nshare) {
+                      const __grid_constant__ CUtensorMap tmV, const SelKvArgs a, const int nshare, const int nfirst) {
   after_previous();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -84,18 +84,31 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(sgen + (tmem_slot - sbase));
 
   // ---- work item: (batch, kv head)-major so the resident CTAs share one head group's Q rows in L2; shares of a block's
-  // list block-major, longest lists first (there are few enough of them for all of Q to stay in L2) ----------------------
+  // list block-major, longest lists first (there are few enough of them for all of Q to stay in L2); nfirst > 0: shares of
+  // every head group's first block before the other blocks --------------------------------------------------------------
   const int G16 = (a.Hq / a.Hk) / 16;
   const int NB = (a.T + 63) / 64;
-  const int seg = (int)(blockIdx.x % nshare), item = (int)(blockIdx.x / nshare);
-  const int blk = nshare > 1 ? item / (a.B * a.Hk) : item % NB;
-  const int bh = nshare > 1 ? item % (a.B * a.Hk) : item / NB;
+  const int BH = a.B * a.Hk;
+  int nseg = nshare, seg = (int)(blockIdx.x % nshare), item = (int)(blockIdx.x / nshare);
+  int blk = nshare > 1 ? item / BH : item % NB, bh = nshare > 1 ? item % BH : item / NB;
+  if (nfirst > 0) {   // (nshare = 1)
+    if (item < BH * nfirst) {
+      nseg = nfirst;
+      seg = item % nfirst;
+      blk = 0;
+      bh = item / nfirst;
+    } else {
+      item -= BH * nfirst;
+      blk = 1 + item % (NB - 1);
+      bh = item / (NB - 1);
+    }
+  }
   const int b = bh / a.Hk, hk = bh % a.Hk;
   const int* rp = a.rev_ptr + (long long)bh * (NB + 1);
   int ta_lo = rp[blk], nA = rp[blk + 1] - ta_lo;
-  if (nshare > 1) {   // this CTA's share of the list, in whole batches
+  if (nseg > 1) {   // this CTA's share of the list, in whole batches
     const int ba = (nA + kTokB - 1) / kTokB;
-    const int a0 = ba * seg / nshare * kTokB, a1 = min(nA, ba * (seg + 1) / nshare * kTokB);
+    const int a0 = (int)((long long)ba * seg / nseg) * kTokB, a1 = min(nA, (int)((long long)ba * (seg + 1) / nseg) * kTokB);
     ta_lo += a0;
     nA = a1 - a0;
   }
@@ -495,12 +508,18 @@ int launch_sel_fwd_kv(const SelKvArgs& a, const RevArgs& r, cudaStream_t s) {
   const long long blocks = (long long)a.B * a.Hk * ((a.T + 63) / 64), want = 3LL * num_sms();
   if (blocks <= 0) return 0;
   const int nshare = blocks >= 2 * want ? 1 : (int)std::max(2LL, std::min(8LL, (want + blocks - 1) / blocks));
-  const long long grid = blocks * nshare;
+  // Many blocks: the first one may still be selected by every token (a fixed choice of it is part of the method), a list as long as
+  // many others together, and the last head group's would begin last.  It goes first, in shares, about one per SM over the head
+  // groups (up to twice as many blocks as a token selects every list is long).  The whole branch, block 0 and 15 drawn ones, 4 KV
+  // heads: 4 x 8192 tokens 4.75 -> 3.83 ms, 8 x 8192 8.8 -> 7.9, 65536 14.8 -> 7.5; drawn ones alone 4.07 / 3.98, 7.88 / 7.85.
+  const long long BH = (long long)a.B * a.Hk;
+  const int nfirst = nshare == 1 && (a.T + 63) / 64 > 2 * a.S ? (int)std::max(2LL, std::min(32LL, (num_sms() + BH - 1) / BH)) : 0;
+  const long long grid = nfirst ? blocks + BH * (nfirst - 1) : blocks * nshare;
   if (grid > 0x7fffffffLL) {
     set_error("selected forward: grid too large");
     return -33;
   }
-  launch_next(sel_fwd_kv_kernel, (unsigned)grid, kThreads, kSmem, s, tmQ, tmK, tmV, a, nshare);
+  launch_next(sel_fwd_kv_kernel, (unsigned)grid, kThreads, kSmem, s, tmQ, tmK, tmV, a, nshare, nfirst);
   note_launches(1);
   e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
