@@ -48,11 +48,11 @@ static int check_bs(const char* who, int BS) {
 // many as
 // give every SM two (at most 16; a share then still has some dozens of tokens).  The CTAs of a shared list leave fp32
 // partials that a
-// second kernel adds in order.  kv_bwd_tc_kernel with 4 KV heads, one CTA a block -> two: 5000 tokens (316 blocks) 647 -> 330
+// second kernel adds in order.  kv_bwd_tc_kernel with 4 KV heads, one CTA a block -> two: 5008 tokens (316 blocks) 498 -> 282
 // us + 24
-// for the sums, 9000 tokens (564) 854 -> 636 + 24, 14000 tokens (876) 1300 -> 999 + 35, 17000 tokens (1064) 1297 -> 1260 +
-// 43, so not
-// there; 2 x 2080 tokens, 2 KV heads (132) three shares 154 us, four 162, five 172, seven 189.
+// for the sums, 9008 tokens (564) 711 -> 531 + 23, 14000 tokens (876) 1049 -> 848 + 34, 17008 tokens (1064) 1050 -> 1031 +
+// 41, so not
+// there; 2 x 2080 tokens, 2 KV heads (132) three shares 126 us, two 144, four 130, five 135.
 static int kv_shares(long long blocks) {
   if (blocks <= 0 || blocks >= 6LL * num_sms()) return 1;
   return (int)std::min(16LL, std::max(2LL, (2LL * num_sms() + blocks - 1) / blocks));
