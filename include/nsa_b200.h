@@ -273,7 +273,7 @@ int nsa_cache_build(const void* k, const void* v, const void* conv_k, const void
 /* ---- decode ---------------------------------------------------------------------------------------------
  * No entry point of the reference does this (its module assumes len(q) == len(k), nsa/nsa.py:97); it is the
  * module's forward (nsa/nsa.py:94-135) for ONE new query token per sequence, at position L-1 of a packed, ragged
- * K/V cache, all sequences in ONE kernel launch (one CTA per (sequence, kv head), see csrc/decode.cu).
+ * K/V cache, all sequences in ONE kernel launch (one or several CTAs per (sequence, kv head), see csrc/decode.cu).
  * q, o [nseq,Hq,D]; k, v [total_k,Hkv,D]; ck, cv [total_c,Hkv,D] = the compressed cache (nsa_compress_fwd with the
  * Conv1d length rule Tc = (L-block)/stride + 1); cu_k, cu_c: DEVICE int32 [nseq+1] cumulative lengths of k/v and of
  * ck/cv; order: DEVICE int32 [nseq] = the order in which sequences are dealt to the CTAs (pass them longest first for
@@ -282,9 +282,9 @@ int nsa_cache_build(const void* k, const void* v, const void* conv_k, const void
  * gate_w NULL, precomputed g_slc, g_swa, g_cmp [nseq,Hq] (NULL = 1).  Optional outputs (NULL to skip): the branch outputs o_cmp, o_slc,
  * o_swa [nseq,Hq,D] and lse fp32 [3,nseq,Hq] (compressed, selected, window); idx int32 [nseq,Hkv,n_sel] receives the
  * selected blocks.  max_Tc = the largest per-sequence compressed length (host-known; at most 2048, i.e. caches up to
- * 32 K tokens).  ws: nsa_decode_workspace_bytes(nseq, Hkv) bytes of scratch (the per-warp partial results that a second,
- * small kernel merges in a fixed order).  Needs head_dim 128, 16 query heads per KV head, 64-key blocks, stride 16 /
- * block 32.  Two launches, no host synchronisation, no internal streams: everything is enqueued on `stream`. */
+ * 32 K tokens).  ws: nsa_decode_workspace_bytes(nseq, Hkv) bytes of scratch (the partial results of an item's tiles,
+ * which the kernel merges in a fixed order; it is scratch within the call).  Needs head_dim 128, 16 query heads per KV head, 64-key blocks, stride 16 /
+ * block 32.  One launch, no host synchronisation, no internal streams: everything is enqueued on `stream`. */
 int nsa_decode_fwd(const void* q, const void* k, const void* v, const void* ck, const void* cv, const int32_t* cu_k,
                    const int32_t* cu_c, const int32_t* order, const void* gate_w, const void* gate_b, const void* g_slc,
                    const void* g_swa, const void* g_cmp, void* o, void* o_cmp, void* o_slc, void* o_swa, float* lse,

@@ -11,12 +11,14 @@
 // rows of mma.sync.m16n8k16.  Where there are fewer items than SMs, a cluster of 2, 4 or 8 CTAs shares one: the tile pairs of
 // every phase behind the statistics are dealt out to its CTAs, which exchange the scores through each other's shared
 // memory and then select the blocks each for itself (one CTA alone draws at most 1/148 of the bandwidth: 4 items of 4096 keys
-// took 25 us).  Where there are more, two CTAs of half the size share an SM.  The statistics (pass 1) are the same six chains
-// everywhere, added in the same order: every CTA of a cluster makes them for itself, a warp of a CTA of three has two of them in
-// turn, and a chain's place in the sum does not follow from the warp that had it.  In another order near
-// ties of two blocks' scores come out otherwise, and a sequence's blocks would depend on how many others it is decoded with:
+// took 25 us).  Where there are more, a CTA takes one after another, and two CTAs of half the size share an SM unless lengths or
+// their evenness speak against it (the rule at decode_spread).  The sums of a phase are six chains of tile pairs: a warp of six has
+// one of them, a warp of three two, one after the other, and their partials are merged in one order, so that either form gives
+// the same bits.  The statistics (pass 1) are the same six chains in a cluster too, where every CTA makes them for itself.  In another
+// order near ties of two blocks' scores come out otherwise, and a sequence's blocks would depend on how many others it is decoded with:
 // with pass 1 dealt out like the rest up to one in 16 items chose others (1 x 32768 keys 28.7 us so, 34.8 now; 4 x 16384
-// 30.7 and 32.8; 1 x 9000, where an exchange is saved, 26.6 and 25.5).  Producer warps stream [64 rows x 128] tiles by TMA
+// 30.7 and 32.8; 1 x 9000, where an exchange is saved, 26.6 and 25.5).  Three chains of a CTA of three warps instead of six gave outputs
+// that differed by 0.2 % with the form that a batch took (P is rounded against the maximum of its chain).  Producer warps stream [64 rows x 128] tiles by TMA
 // through a ring (192 KB in flight per SM); each consumer warp owns two slots, so every slot is filled and drained by the same
 // pair of warps in order.  The tile stream of an item:
 //   1. ck tiles:           raw scores -> per-row maxima and sums of the unscaled soft-max over ALL compressed keys and
@@ -25,13 +27,16 @@
 //                          p_sel summed over the heads into a per-position vector in shared memory;
 //                          then pooling and a warp top-n while the other warps go on;
 //   3. window (k, v) pairs and 4. selected (k, v) pairs: online soft-max per warp.
-// Every warp leaves its partial (maximum, sum, unnormalised output) of each branch in a caller-provided workspace (the split-KV
-// scheme of decode attention).  The CTAs of an item then merge its rows, in a fixed order: without clusters each warp a row at a
-// time, from a scratch that the CTA's next item uses again (it stays in L2) while the ring fills with that item's tiles; with
-// clusters each CTA its share of the rows, a row and branch per warp.  Measured, 128 sequences of 4096 to 32768 keys: a second
-// kernel that merges (77 MB of partials written and read) 179 us, merged here 170, and with two CTAs per SM 150 (4.7 TB/s); one
-// sequence of 4096 keys 18.9 us with the second kernel and 17.5 without.  Merging through shared memory, warp after warp,
-// cost seven
+// Every chain leaves its partial (maximum, sum, unnormalised output) of each branch in a caller-provided workspace (the split-KV
+// scheme of decode attention).  The CTAs of an item then merge its rows, in a fixed order: without clusters each warp two rows at a
+// time, from a scratch that the CTA's next item uses again while the ring fills with that item's tiles; with
+// clusters each CTA its share of the rows, a row and branch per warp.  The scratch is to stay in L2 beside the caches that stream
+// through it: CTAs that share an SM fetch what they read for the last time under an evict-first policy.
+// Measured, 128 sequences of 4096 to 32768 keys, 4 KV heads, one CTA per SM / two: 164 / 146 us (4.7 TB/s); two without the policy
+// 163, and with one row per warp at a time 165; a second kernel that merges (77 MB of partials written and read) 179; one
+// sequence of 4096 keys 18.9 us with the second kernel and 17.5 without.  Also tried, with the same bits: two accumulators per warp of
+// three, the chains' pairs in turn (185 us: twice the code); six warps in a CTA that shares its SM, on a ring of three pairs
+// (196: too few tiles under way for a warp to wait as little).  Merging through shared memory, warp after warp, cost seven
 // named barriers and six serialised rounds per branch.  No atomics; every wait is bounded.
 #include <algorithm>
 #include <array>
@@ -44,12 +49,12 @@ namespace nsa {
 namespace {
 
 constexpr int D = 128;
-constexpr int kCons = 6;                       // consumer warps of a CTA that has an SM to itself, chains of the statistics
+constexpr int kCons = 6;                       // consumer warps of a CTA that has an SM to itself; chains of a phase
 constexpr int kHalfCons = 3;                   // ... of one that shares it with another
-// Producer warps: one issues 30 bytes per cycle (see below), what one of two CTAs of an SM can draw at most.
+// Producer warps of a CTA.
 __host__ __device__ constexpr int decode_producers(int cons) { return cons == kCons ? 2 : 1; }
 __host__ __device__ constexpr int decode_threads(int cons) { return (cons + decode_producers(cons)) * 32; }
-static_assert(kCons == 2 * kHalfCons, "one chain of the statistics per warp, or two");
+static_assert(kCons == 2 * kHalfCons, "one chain per warp, or two");
 constexpr uint32_t PANEL = 64 * 128;           // [64 rows][64 columns] bf16
 constexpr uint32_t TILE = 2 * PANEL;           // 16 KB
 constexpr int kMaxTc = 2048;                   // compressed positions of one sequence held in shared memory
@@ -134,6 +139,19 @@ __device__ __forceinline__ int pool_len(int n, int k, int s) {
   int out = (num >= 0 ? (num + s - 1) / s : -((-num) / s)) + 1;
   if ((out - 1) * s >= n) --out;
   return out < 0 ? 0 : out;
+}
+
+// How many tile pairs a CTA that has one of the GPU's `sms` SMs to itself has behind it when it comes to `item` (by one warp).
+// Counts every block that can be selected: NaN among the scores takes some out, which then changes the order of a sum and no more.
+__device__ __forceinline__ uint32_t pairs_before(const DecodeArgs& a, int item, int sms, int lane) {
+  const int rounds = item / sms, x = item % sms, cta = rounds & 1 ? sms - 1 - x : x;
+  uint32_t n = 0;
+  for (int r = lane; r < rounds; r += 32) {
+    const int sq = snake_item(r, cta, sms) / a.Hkv;
+    const Plan p = make_plan(a, a.order ? a.order[sq] : sq, 1);
+    n += p.n1p + p.n2p + p.nw + min(a.n_sel, min(kMaxPoolD, pool_len(p.Tc, a.sel_block / a.cstride + 1, a.sel_block / a.cstride)));
+  }
+  return __reduce_add_sync(0xffffffffu, n);
 }
 
 // acc (16 x 128) += P (16 x 64, in sc as mma C layout) . V tile
@@ -358,9 +376,11 @@ __device__ __forceinline__ float4 merge_row(const DecodeArgs& a, int item, long 
 template <int CONS, bool CL>
 __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
     decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
-                  const __grid_constant__ CUtensorMap tmCK, const __grid_constant__ CUtensorMap tmCV, const DecodeArgs a, const int ncl) {
+                  const __grid_constant__ CUtensorMap tmCK, const __grid_constant__ CUtensorMap tmCV, const DecodeArgs a, const int ncl,
+                  const int sms) {
   after_previous();
   constexpr int kSlots = 2 * CONS, kProdW = decode_producers(CONS);
+  constexpr int kOwn = kCons / CONS;   // chains of a warp
   const int cl = CL ? ncl : 1;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -373,8 +393,8 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
   float* pooled = ps + kMaxTc + 64;                               // [kMaxPoolD]
   float* stat = pooled + kMaxPoolD;                               // [kCons][4][16] the chains' statistics
   float* fin = stat + kCons * 64;                                 // [4][16] merged: M_raw, 1/L_raw, M_att (log2), L_att
-  float2* ml = reinterpret_cast<float2*>(fin + 64);               // [3][CONS][16] (m, l) of the warps' partials, without clusters
-  float* gates = reinterpret_cast<float*>(ml + 3 * CONS * 16);       // [3][16], branch order as ml's
+  float2* ml = reinterpret_cast<float2*>(fin + 64);               // [3][kCons][16] (m, l) of the chains' partials, without clusters
+  float* gates = reinterpret_cast<float*>(ml + 3 * kCons * 16);      // [3][16], branch order as ml's
   int* sel = reinterpret_cast<int*>(gates + 48);                  // [kMaxSel] selected blocks of the item, [kMaxSel] = count
   volatile int* abort_flag = sel + kMaxSel + 2;
   const uint32_t bar_base = sbase + kSlots * TILE + (uint32_t)((uint8_t*)(sel + kMaxSel + 4) - after);
@@ -410,6 +430,9 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
     // warp), and the producer warps (one in a CTA that shares its SM) take alternate pairs.
     const int pw = warp - CONS;
     uint32_t np = 0, it = 0;     // tile pairs issued so far by both producers together; items so far
+    // what an item reads for the last time goes first from L2, before the partials of 2 x 148 CTAs (44 MB)
+    const uint64_t once = l2_evict_first();
+    bool last = false;
     auto issue2 = [&](const CUtensorMap* tmA, int rowA, const CUtensorMap* tmB, int rowB, int h) -> bool {
       const uint32_t mine = np % kProdW == (uint32_t)pw;
       const uint32_t n = 2 * np;
@@ -424,11 +447,22 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
         for (int w = 0; w < 2; ++w) {
           mbar_expect_tx(full_bar(s0 + w), TILE);
 #pragma unroll
-          for (int p = 0; p < 2; ++p)
-            tma_load_4d(ring + (s0 + w) * TILE + p * PANEL, w ? tmB : tmA, full_bar(s0 + w), p * 64, h, w ? rowB : rowA, 0);
+          for (int p = 0; p < 2; ++p) {
+            const uint32_t dst = ring + (s0 + w) * TILE + p * PANEL;
+            if (kOwn > 1 && last)
+              tma_load_4d(dst, w ? tmB : tmA, full_bar(s0 + w), p * 64, h, w ? rowB : rowA, 0, once);
+            else
+              tma_load_4d(dst, w ? tmB : tmA, full_bar(s0 + w), p * 64, h, w ? rowB : rowA, 0);
+          }
         }
       }
       return true;
+    };
+    // the n pairs of a phase as the warps take them: those of the first CONS chains, then (CONS < kCons) of the others
+    auto each_pair = [&](int n, bool& ok, auto&& issue) {
+      for (int e = 0; e < kCons; e += CONS)
+        for (int c = e; c < n; c += kCons)
+          for (int i = c; ok && i < min(c + CONS, n); ++i) ok = issue(i);
     };
     for (int r = 0; r * ngroup < nitem; ++r) {
       const int item = snake_item(r, group, ngroup);
@@ -437,18 +471,26 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
       const int seq = a.order ? a.order[sq] : sq;
       const Plan p = make_plan(a, seq, cl);
       bool ok = true;
-      for (int j = 0; ok && j < p.n1p; ++j) ok = issue2(&tmCK, p.row_c + j * 128, &tmCK, p.row_c + j * 128 + 64, h);
-      for (int j = p.cs > 1 ? rank : 0; ok && j < p.n2p; j += p.cs) ok = issue2(&tmCK, p.row_c + j * 64, &tmCV, p.row_c + j * 64, h);
-      for (int j = rank; ok && j < p.nw; j += cl) ok = issue2(&tmK, p.row_k + p.w0 + j * 64, &tmV, p.row_k + p.w0 + j * 64, h);
+      last = false;
+      each_pair(p.n1p, ok, [&](int j) { return issue2(&tmCK, p.row_c + j * 128, &tmCK, p.row_c + j * 128 + 64, h); });
+      last = true;
+      each_pair(share(p.n2p, p.cs), ok, [&](int i) {
+        const int j = deal(i, p.cs);
+        return issue2(&tmCK, p.row_c + j * 64, &tmCV, p.row_c + j * 64, h);
+      });
+      each_pair(share(p.nw, cl), ok, [&](int i) {
+        const int j = deal(i, cl);
+        return issue2(&tmK, p.row_k + p.w0 + j * 64, &tmV, p.row_k + p.w0 + j * 64, h);
+      });
       // the selected blocks are known once the consumers have pooled the scores
       if (ok && lane == 0) ok = mbar_wait_abortable(sel_ready, it & 1, DEV_ERR_FULL_WAIT, abort_flag);
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
       if (!ok) break;
       const int nsel = *reinterpret_cast<volatile int*>(sel + kMaxSel);
-      for (int j = rank; ok && j < nsel; j += cl) {
-        const int blk = *reinterpret_cast<volatile int*>(sel + j);
-        ok = issue2(&tmK, p.row_k + blk * 64, &tmV, p.row_k + blk * 64, h);
-      }
+      each_pair(share(nsel, cl), ok, [&](int i) {
+        const int blk = *reinterpret_cast<volatile int*>(sel + deal(i, cl));
+        return issue2(&tmK, p.row_k + blk * 64, &tmV, p.row_k + blk * 64, h);
+      });
       if (!ok) break;
       ++it;
     }
@@ -458,11 +500,18 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
   const float sl2 = a.scale * kLog2e;
   const int cthreads = CONS * 32;
   const int ct = threadIdx.x;               // 0 .. cthreads-1
+  // Six chains in every phase: chain c has the pairs c, c + 6, ...  A warp of six has one of them.  A warp of three has two, one after
+  // the other: the same terms in the same order, so that outputs have the same bits, with one accumulator.
   // tile pair i of the CTA, over all phases and items, is warp i % CONS's, in that warp's own two slots
-  uint32_t np0 = 0, it = 0;                 // pairs of the CTA before the current phase; items so far
+  uint32_t np0 = 0, it = 0;                 // pairs of the CTA so far (before the current phase's current chains); items so far
+  uint32_t own0 = 0;                        // pairs before the current phase of the CTA of six warps that would have the item
   uint32_t use = 0;                         // pairs of this warp so far
   const uint32_t sk = 2 * warp, sv = sk + 1;
-  auto first_pair = [&]() { return (int)((warp + CONS - np0 % CONS) % CONS); };
+  // this warp's chain of a phase: of the first CONS ones (e = 0) or of the others
+  auto chain_of = [&](int e) { return (int)((warp + CONS - np0 % CONS) % CONS) + e * CONS; };
+  auto pairs_of = [&](int n, int e) { return kOwn == 1 ? n : n / kCons * CONS + max(0, min(n % kCons - e * CONS, CONS)); };   // of all warps
+  // where its partial goes: to the warp that has the chain in a CTA of six
+  auto part_of = [&](int chain) { return kOwn == 1 ? warp : (int)((own0 + chain) % kCons); };
   bool ok = true;
   for (int r = 0; r * ngroup < nitem; ++r) {
     const int item = snake_item(r, group, ngroup);
@@ -474,25 +523,19 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
     const long long qrow = (long long)seq * a.Hq + h * 16;     // first of the 16 (head) rows of this item
     uint32_t qf[D / 16][4];
     load_a_frags_global<D>(qf, a.q + qrow * D, lane);
+    if (kOwn > 1) own0 = pairs_before(a, item, sms, lane);
 
     // ---- pass 1: statistics over all compressed keys ---------------------------------------------------
-    // Six chains, whatever the number of warps: chain c has the pairs c, c + 6, ...  One of six warps has one, one of three warps two,
-    // whose pairs come in turn.
-    struct Stat {
+#pragma unroll 1
+    for (int e = 0; e < kOwn; ++e) {
       float mr[2] = {-INFINITY, -INFINITY}, lr[2] = {0.f, 0.f};   // raw scores, all keys (natural-log domain kept in log2)
       float ma[2] = {-INFINITY, -INFINITY}, la[2] = {0.f, 0.f};   // scaled scores, visible keys
-      int chain;
-    };
-    Stat st0, st1;   // of the pair's chain and (three warps) of the one whose turn is next
-    st0.chain = first_pair();
-    st1.chain = st0.chain + CONS;
-    {
-      for (int u = st0.chain; u < p.n1p; u += CONS, ++use) {
-        float(&mr)[2] = st0.mr, (&lr)[2] = st0.lr, (&ma)[2] = st0.ma, (&la)[2] = st0.la;
+      const int chain = chain_of(e);
+      for (int u = chain; u < p.n1p; u += kCons, ++use) {
 #pragma unroll 1
-        for (int e = 0; e < 2; ++e) {
-          const uint32_t s = sk + e;
-          const int j0 = (2 * u + e) * 64;
+        for (int t2 = 0; t2 < 2; ++t2) {
+          const uint32_t s = sk + t2;
+          const int j0 = (2 * u + t2) * 64;
           ok = ok && mbar_wait_abortable(full_bar(s), use & 1, DEV_ERR_FULL_WAIT, abort_flag);
           float sc[8][4];
 #pragma unroll
@@ -529,31 +572,23 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
             ma[rr] = na;
           }
         }
-        if (CONS != kCons) {
-          const Stat x = st0;
-          st0 = st1;
-          st1 = x;
-        }
       }
-      np0 += p.n1p;
-    }
-    // merge the statistics of the chains, in their order whichever warps had them, so that an item's scores do not depend on
-    // the items before it (each value lives in the four lanes of a quad: sum the partial sums)
-    auto leave = [&](const Stat& x) {
+      // the statistics of the chains are merged in their order whichever warps had them, so that an item's scores do not depend on
+      // the items before it (each value lives in the four lanes of a quad: sum the partial sums)
 #pragma unroll
       for (int rr = 0; rr < 2; ++rr) {
-        const float l_r = quad_sum(x.lr[rr]), l_a = quad_sum(x.la[rr]);
+        const float l_r = quad_sum(lr[rr]), l_a = quad_sum(la[rr]);
         if (tq == 0) {
-          float* st = stat + x.chain * 64;
-          st[0 * 16 + g + 8 * rr] = x.mr[rr];
+          float* st = stat + chain * 64;
+          st[0 * 16 + g + 8 * rr] = mr[rr];
           st[1 * 16 + g + 8 * rr] = l_r;
-          st[2 * 16 + g + 8 * rr] = nan_or(l_a, x.ma[rr]);
+          st[2 * 16 + g + 8 * rr] = nan_or(l_a, ma[rr]);
           st[3 * 16 + g + 8 * rr] = l_a;
         }
       }
-    };
-    leave(st0);
-    if (CONS != kCons) leave(st1);
+      np0 += pairs_of(p.n1p, e);
+    }
+    own0 += p.n1p;
     named_bar_sync(1, cthreads);
     if (ct < 16) {
       float Mr = -INFINITY, Ma = -INFINITY;
@@ -584,14 +619,51 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
       if (Ma[rr] == -INFINITY) Ma[rr] = 0.f;
     }
 
+    // a chain's partial of a branch -> workspace: [item][branch][chain of the cluster]{ O[16][D], m[16], l[16] } fp32; a chain
+    // that had no tile leaves m = -inf and no O
+    auto put_partial = [&](int branch, int w, const float (&x)[D / 8][4], const float (&mm)[2], const float (&ll)[2], bool has) {
+      float* dst = a.part + (((long long)(cl > 1 ? item : (int)blockIdx.x) * 3 + branch) * (cl * kCons) + rank * kCons + w) * kPartFloats;
+#pragma unroll
+      for (int i = 0; i < D / 8; ++i) {
+        if (!has) break;
+        *reinterpret_cast<float2*>(dst + g * D + i * 8 + 2 * tq) = make_float2(x[i][0], x[i][1]);
+        *reinterpret_cast<float2*>(dst + (g + 8) * D + i * 8 + 2 * tq) = make_float2(x[i][2], x[i][3]);
+      }
+#pragma unroll
+      for (int rr = 0; rr < 2; ++rr) {
+        const float l = quad_sum(ll[rr]);
+        if (tq == 0) {
+          const float m = has ? nan_or(l, mm[rr]) : -INFINITY;
+          if (cl > 1) {
+            dst[16 * D + g + 8 * rr] = m;
+            dst[16 * D + 16 + g + 8 * rr] = l;
+          } else {
+            ml[(branch * kCons + w) * 16 + g + 8 * rr] = make_float2(m, l);
+          }
+        }
+      }
+    };
+    // compressed branch: every chain used the final maximum; the row sum is known to the CTA and rides with the first partial
+    auto put_compressed = [&](int w, const float (&x)[D / 8][4], bool has) {
+      float mm[2], ll[2];
+#pragma unroll
+      for (int rr = 0; rr < 2; ++rr) {
+        mm[rr] = fin[32 + g + 8 * rr];
+        ll[rr] = (rank == 0 && w == 0 && tq == 0) ? La[rr] : 0.f;
+      }
+      put_partial(0, w, x, mm, ll, has);
+    };
+
     // ---- pass 2: attention over the visible compressed keys and the block scores -------------------------
     float acc[D / 8][4];
+    bool full = false;   // the chain's partial has an output
+#pragma unroll 1
+    for (int e = 0; e < kOwn; ++e) {
+      const int n = share(p.n2p, p.cs), chain = chain_of(e), part = part_of(chain);
 #pragma unroll
-    for (int i = 0; i < D / 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
-    bool full = rank == 0 && warp == 0;   // this warp's partial has an output (the first always: the row sums ride with it)
-    {
-      const int n = share(p.n2p, p.cs);
-      for (int i = first_pair(); i < n; i += CONS, ++use) {
+      for (int i = 0; i < D / 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+      full = rank == 0 && part == 0;   // (the first always: the row sums ride with it)
+      for (int i = chain; i < n; i += kCons, ++use) {
         const int u = deal(i, p.cs);
         full = p.cs > 1 || rank == 0;
         const int j0 = u * 64;
@@ -642,8 +714,10 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
         __syncwarp();
         if (lane == 0) mbar_arrive(empty_bar(sv));
       }
-      np0 += n;
+      np0 += pairs_of(n, e);
+      if (kOwn > 1) put_compressed(part, acc, full);
     }
+    own0 += p.n2p;
     // ---- pooled scores and the top-n (warp 0), the compressed-branch output (all warps, fixed order) ------------
     named_bar_sync(1, cthreads);            // ps complete
     if (p.cs > 1) {   // in every CTA
@@ -672,40 +746,7 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
         mbar_arrive(sel_ready);
       }
     }
-    // this warp's partial of a branch -> workspace: [item][branch][warp of the cluster]{ O[16][D], m[16], l[16] } fp32; a warp
-    // that had no tile leaves m = -inf and no O
-    auto put_partial = [&](int branch, const float (&x)[D / 8][4], const float (&mm)[2], const float (&ll)[2], bool has) {
-      float* dst = a.part + (((long long)(cl > 1 ? item : (int)blockIdx.x) * 3 + branch) * (cl * CONS) + rank * CONS + warp) * kPartFloats;
-#pragma unroll
-      for (int i = 0; i < D / 8; ++i) {
-        if (!has) break;
-        *reinterpret_cast<float2*>(dst + g * D + i * 8 + 2 * tq) = make_float2(x[i][0], x[i][1]);
-        *reinterpret_cast<float2*>(dst + (g + 8) * D + i * 8 + 2 * tq) = make_float2(x[i][2], x[i][3]);
-      }
-#pragma unroll
-      for (int rr = 0; rr < 2; ++rr) {
-        const float l = quad_sum(ll[rr]);
-        if (tq == 0) {
-          const float m = has ? nan_or(l, mm[rr]) : -INFINITY;
-          if (cl > 1) {
-            dst[16 * D + g + 8 * rr] = m;
-            dst[16 * D + 16 + g + 8 * rr] = l;
-          } else {
-            ml[(branch * CONS + warp) * 16 + g + 8 * rr] = make_float2(m, l);
-          }
-        }
-      }
-    };
-    {
-      // compressed branch: every warp used the final maximum; the row sum is known to the CTA and rides with warp 0
-      float mm[2], ll[2];
-#pragma unroll
-      for (int rr = 0; rr < 2; ++rr) {
-        mm[rr] = fin[32 + g + 8 * rr];
-        ll[rr] = (rank == 0 && warp == 0 && tq == 0) ? La[rr] : 0.f;
-      }
-      put_partial(0, acc, mm, ll, full);
-    }
+    if (kOwn == 1) put_compressed(warp, acc, full);
 
     // ---- gates, by the last warp (the first one is still choosing blocks) --------------------------------
     // (what the item before left in gates, ml and the scratch has been read: its rows are merged before anything of this one)
@@ -742,37 +783,37 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
     }
 
     // ---- window ---------------------------------------------------------------------------------------
-    float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
+#pragma unroll 1
+    for (int e = 0; e < kOwn; ++e) {
+      const int n = share(p.nw, cl), chain = chain_of(e), part = part_of(chain);
+      float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
 #pragma unroll
-    for (int i = 0; i < D / 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
-    full = false;
-    {
-      const int n = share(p.nw, cl);
-      for (int i = first_pair(); i < n; i += CONS, ++use) {
+      for (int i = 0; i < D / 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+      full = false;
+      for (int i = chain; i < n; i += kCons, ++use) {
         const int u = deal(i, cl);
         full = true;
         ok = ok && mbar_wait_abortable(full_bar(sk), use & 1, DEV_ERR_FULL_WAIT, abort_flag);
         online_pair(acc, m_run, l_run, qf, ring + sk * TILE, ring + sv * TILE, empty_bar(sk), full_bar(sv), use & 1,
                     empty_bar(sv), p.w0 + u * 64, p.w0, p.L, sl2, lane, ok, abort_flag);
       }
-      np0 += n;
-    }
-    {
+      np0 += pairs_of(n, e);
       // l_run holds this lane's share of the row sums (four lanes per row): put_partial adds the quad
-      put_partial(2, acc, m_run, l_run, full);
+      put_partial(2, part, acc, m_run, l_run, full);
     }
+    own0 += p.nw;
 
     // ---- selected blocks ---------------------------------------------------------------------------------
     ok = ok && mbar_wait_abortable(sel_ready, it & 1, DEV_ERR_FULL_WAIT, abort_flag);
     const int nsel = *reinterpret_cast<volatile int*>(sel + kMaxSel);
-    m_run[0] = m_run[1] = -INFINITY;
-    l_run[0] = l_run[1] = 0.f;
+#pragma unroll 1
+    for (int e = 0; e < kOwn; ++e) {
+      const int n = share(nsel, cl), chain = chain_of(e), part = part_of(chain);
+      float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
 #pragma unroll
-    for (int i = 0; i < D / 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
-    full = false;
-    {
-      const int n = share(nsel, cl);
-      for (int i = first_pair(); i < n; i += CONS, ++use) {
+      for (int i = 0; i < D / 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+      full = false;
+      for (int i = chain; i < n; i += kCons, ++use) {
         const int u = deal(i, cl);
         full = true;
         const int blk = *reinterpret_cast<volatile int*>(sel + u);
@@ -780,59 +821,70 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
         online_pair(acc, m_run, l_run, qf, ring + sk * TILE, ring + sv * TILE, empty_bar(sk), full_bar(sv), use & 1,
                     empty_bar(sv), blk * 64, 0, p.L, sl2, lane, ok, abort_flag);
       }
-      np0 += n;
+      np0 += pairs_of(n, e);
+      put_partial(1, part, acc, m_run, l_run, full);
     }
-    put_partial(1, acc, m_run, l_run, full);
     named_bar_sync(1, cthreads);   // ps, pooled, fin and sel are reused by the next item
     ++it;
-    // ---- this item's rows: partials merged warp by warp, gated sum of the branches (a lane holds four channels) --------
-    for (int row = warp; cl == 1 && row < 16; row += CONS) {
-      const float4* base = reinterpret_cast<const float4*>(a.part + (long long)blockIdx.x * 3 * CONS * kPartFloats + row * D) + lane;
-      float4 x[3][CONS];
-      float e[3][CONS], inv[3], lse[3];
+    // ---- this item's rows: partials merged chain by chain, gated sum of the branches; two rows per warp at a time, a lane holds four
+    // channels of either half -------------------------------------------------------------------------------------------
+    for (int r2 = warp; cl == 1 && r2 < 8; r2 += CONS) {
+      const int row = 2 * r2 + (lane >> 4), c0 = 4 * (lane & 15);
+      const float4* base = reinterpret_cast<const float4*>(a.part + (long long)blockIdx.x * 3 * kCons * kPartFloats + row * D + c0);
+      float4 x[3][kCons][2];
+      float e[3][kCons], inv[3], lse[3];
 #pragma unroll
       for (int br = 0; br < 3; ++br)
 #pragma unroll
-        for (int w = 0; w < CONS; ++w) {
-          e[br][w] = ml[(br * CONS + w) * 16 + row].x;
-          x[br][w] = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (e[br][w] != -INFINITY) x[br][w] = __ldcg(base + (br * CONS + w) * (kPartFloats / 4));
+        for (int w = 0; w < kCons; ++w) {
+          e[br][w] = ml[(br * kCons + w) * 16 + row].x;
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            x[br][w][k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (e[br][w] != -INFINITY) x[br][w][k] = __ldcg(base + (br * kCons + w) * (kPartFloats / 4) + 16 * k);
+          }
         }
 #pragma unroll
       for (int br = 0; br < 3; ++br) {
         float M = e[br][0], L = 0.f;
 #pragma unroll
-        for (int w = 1; w < CONS; ++w) M = fmaxf(M, e[br][w]);
+        for (int w = 1; w < kCons; ++w) M = fmaxf(M, e[br][w]);
 #pragma unroll
-        for (int w = 0; w < CONS; ++w) {
+        for (int w = 0; w < kCons; ++w) {
           e[br][w] = e[br][w] != -INFINITY ? ex2(e[br][w] - M) : 0.f;
-          L += ml[(br * CONS + w) * 16 + row].y * e[br][w];
+          L += ml[(br * kCons + w) * 16 + row].y * e[br][w];
         }
         inv[br] = L > 0.f ? 1.f / L : 0.f;
         lse[br] = L > 0.f ? (M + log2f(L)) * kLn2 : -INFINITY;
       }
-      float4 tot = make_float4(0.f, 0.f, 0.f, 0.f);
+      float4 tot[2];
+      tot[0] = tot[1] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int br = 0; br < 3; ++br) {
         if (br == 2 && a.window <= 0) continue;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int w = 0; w < CONS; ++w) {
-          const float wt = e[br][w] * inv[br];
-          v.x = fmaf(x[br][w].x, wt, v.x);
-          v.y = fmaf(x[br][w].y, wt, v.y);
-          v.z = fmaf(x[br][w].z, wt, v.z);
-          v.w = fmaf(x[br][w].w, wt, v.w);
-        }
-        const __nv_bfloat162 b0 = __floats2bfloat162_rn(v.x, v.y), b1 = __floats2bfloat162_rn(v.z, v.w);
         bf16* out = br == 0 ? a.o_cmp : br == 1 ? a.o_slc : a.o_swa;
-        if (out) *reinterpret_cast<uint2*>(out + (qrow + row) * D + lane * 4) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
-        if (a.lse && lane == 0) a.lse[(long long)br * a.nseq * a.Hq + qrow + row] = lse[br];
         const float gt = gates[br * 16 + row];
-        const float2 f0 = __bfloat1622float2(b0), f1 = __bfloat1622float2(b1);
-        tot.x += gt * f0.x; tot.y += gt * f0.y; tot.z += gt * f1.x; tot.w += gt * f1.y;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+          for (int w = 0; w < kCons; ++w) {
+            const float wt = e[br][w] * inv[br];
+            v.x = fmaf(x[br][w][k].x, wt, v.x);
+            v.y = fmaf(x[br][w][k].y, wt, v.y);
+            v.z = fmaf(x[br][w][k].z, wt, v.z);
+            v.w = fmaf(x[br][w][k].w, wt, v.w);
+          }
+          const __nv_bfloat162 b0 = __floats2bfloat162_rn(v.x, v.y), b1 = __floats2bfloat162_rn(v.z, v.w);
+          if (out) *reinterpret_cast<uint2*>(out + (qrow + row) * D + c0 + 64 * k) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+          const float2 f0 = __bfloat1622float2(b0), f1 = __bfloat1622float2(b1);
+          tot[k].x += gt * f0.x; tot[k].y += gt * f0.y; tot[k].z += gt * f1.x; tot[k].w += gt * f1.y;
+        }
+        if (a.lse && (lane & 15) == 0) a.lse[(long long)br * a.nseq * a.Hq + qrow + row] = lse[br];
       }
-      *reinterpret_cast<uint2*>(a.o + (qrow + row) * D + lane * 4) = make_uint2(pack_bf16(tot.x, tot.y), pack_bf16(tot.z, tot.w));
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+        *reinterpret_cast<uint2*>(a.o + (qrow + row) * D + c0 + 64 * k) = make_uint2(pack_bf16(tot[k].x, tot[k].y), pack_bf16(tot[k].z, tot[k].w));
     }
   }
   }
@@ -843,7 +895,7 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
     const int item = group, sq = item / a.Hkv, h = item % a.Hkv, rows = 16 / cl, nb = a.window > 0 ? 3 : 2;
     const long long qrow = (long long)(a.order ? a.order[sq] : sq) * a.Hq + h * 16 + rank * rows;   // first of this CTA's rows
     float4* out = reinterpret_cast<float4*>(ps);   // [row][branch][lane], over what the item no longer needs
-    for (int u = warp; u < rows * nb; u += CONS) out[u * 32 + lane] = merge_row(a, item, qrow + u / nb, rank * rows + u / nb, u % nb, cl * CONS, lane);
+    for (int u = warp; u < rows * nb; u += CONS) out[u * 32 + lane] = merge_row(a, item, qrow + u / nb, rank * rows + u / nb, u % nb, cl * kCons, lane);
     named_bar_sync(1, CONS * 32);
     for (int row = warp; row < rows; row += CONS) {
       float4 tot = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -858,7 +910,7 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
 }
 
 constexpr int decode_smem(int cons) {
-  return 2 * cons * (int)TILE + (kMaxTc + 64 + kMaxPoolD + kCons * 64 + 64 + 3 * cons * 32 + 48) * 4 + (kMaxSel + 4) * 4 +
+  return 2 * cons * (int)TILE + (kMaxTc + 64 + kMaxPoolD + kCons * 64 + 64 + 3 * kCons * 32 + 48) * 4 + (kMaxSel + 4) * 4 +
          (4 * cons + 2) * 8 + 16 + 1024;
 }
 static_assert(2 * (decode_smem(kHalfCons) + 1024) <= 228 * 1024, "two CTAs per SM");
@@ -888,12 +940,12 @@ int ask_resident(int cl) {
 }
 // How `nitem` items are spread: up to the number of SMs as many CTAs per item as keep every item in the first wave, with an SM to
 // itself each; with more items two CTAs of half the warps and slots share an SM, so that one streams tiles while the other chooses
-// its blocks or merges its rows.  Below two items per SM such a CTA has one item and takes 38 us + 1.46 us per 1000 keys for the
-// longest, against two items, a long and a short one, behind each other.  One CTA per SM -> two: 160 items of up to 5500 keys 55 ->
-// 45.6 us, 196 of 10000 58.7 -> 55.7, 260 of 18000 72.7 -> 69.6; but 164 of 21500 54 -> 69.5, 192 of 28000 67 -> 81, 236 of 25000 78.4 ->
-// 80.5, so not there.  512 items of 4096 to 32768 keys 165 -> 150, 512 of 1500 103 -> 90, 320 of 4096 to 32768 118 -> 102.  Three
-// rounds of equal items are no more than two of pairs, the second half empty: 300 to 440 items of 16384 keys 120 to 132 us, as pairs 131 to
-// 142 (of 8192 95 to 109, 97 to 107); four are: 448 of 16384 161 -> 144.
+// its blocks or merges its rows.  Below two items per SM such a CTA has one item and takes 32 us + 1.2 us per 1000 keys for the
+// longest, against two items, a long and a short one, behind each other.  One CTA per SM -> two, 4 KV heads, lengths from 1024 up to the
+// given one: 152 items of 4000 keys 44.2 -> 36.9 us, 192 of 9000 51.2 -> 45.4, 272 of 16000 68.4 -> 58.9; but 152 of 20000 46.6 -> 56.5, 168 of
+// 26000 54.9 -> 63.8, 248 of 32000 75.7 -> 77.6, so not there.  512 items of 4096 to 32768 keys 164 -> 146, 512 of 1500 99 -> 85.
+// Three rounds of equal items are no more than two of pairs, the second half empty: 300 to 444 items of 32000 keys 160 to 179 us, as
+// pairs 169 to 184 (of 12000 100 to 114, 103 to 114); four are: 452 of 32000 218 -> 185.
 struct Spread {
   int cons, cl, ncta;
 };
@@ -917,7 +969,7 @@ Spread decode_spread(int nitem, int max_Tc, bool even) {   // even: the longest 
 // workspace made for a batch serves the smaller ones too.
 size_t decode_workspace_bytes(int nseq, int Hkv) {
   const std::array<int, 4>& held = clusters_held();
-  int ncta = nseq * Hkv > held[0] ? num_sms() : 0;
+  int ncta = nseq * Hkv > held[0] ? std::min(nseq * Hkv, 2 * num_sms()) : 0;
   for (int i = 0; i < 4; ++i) ncta = std::max(ncta, std::min(nseq * Hkv, held[i]) << i);
   return (size_t)ncta * 3 * kCons * kPartFloats * sizeof(float);
 }
@@ -960,7 +1012,7 @@ int launch_decode(const DecodeArgs& a, cudaStream_t s) {
   {
     cudaLaunchAttribute at[2];
     const cudaLaunchConfig_t cfg = decode_config(p.ncta, p.cons, cl, at, s);
-    e = cudaLaunchKernelEx(&cfg, kernel, tmK, tmV, tmCK, tmCV, a, cl);
+    e = cudaLaunchKernelEx(&cfg, kernel, tmK, tmV, tmCK, tmCV, a, cl, num_sms());
     if (e != cudaSuccess) return (int)e;
   }
   note_launches(1);
