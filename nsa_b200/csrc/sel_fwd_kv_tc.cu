@@ -56,8 +56,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   // barriers (8 bytes each); the double ones are indexed by batch & 1
   const uint32_t full0 = bar_base, empty0 = bar_base + 32, kv_bar = bar_base + 64, s_full = bar_base + 72,
                  s_free = bar_base + 88, p_full = bar_base + 104, p_free = bar_base + 120, o_full = bar_base + 136,
-                 o_free = bar_base + 152, stg_full = bar_base + 168, stg_free = bar_base + 176,   // stg_free: two
-                 tmem_slot = bar_base + 192;
+                 o_free = bar_base + 152, stg_full = bar_base + 168, stg_free = bar_base + 184, tmem_slot = bar_base + 200;
   if (threadIdx.x == 0) {
     for (int i = 0; i < kStages; ++i) {
       mbar_init(full0 + 8 * i, kProd);
@@ -72,9 +71,10 @@ __global__ void __launch_bounds__(kThreads, 1)
       mbar_init(o_full + 8 * i, 1);
       mbar_init(o_free + 8 * i, 128);
     }
-    mbar_init(stg_full, 128);
-    mbar_init(stg_free, 1);
-    mbar_init(stg_free + 8, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(stg_full + 8 * i, 128);
+      mbar_init(stg_free + 8 * i, 1);
+    }
     fence_mbar_init();
   }
   if (warp == kMmaWarp) tmem_alloc(tmem_slot, kTmemCols);
@@ -243,11 +243,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       }
       fence_proxy_async();
-      mbar_arrive(stg_full);
+      mbar_arrive(stg_full + 8 * (n & 1));   // (two: of batches 0 and 1 a warp may be at the second before the slowest is through the first)
       if (warp == kDrainWarp) {
         // one 32 KB bulk store (the tokens' tiles are contiguous), or one of 4 KB per token where the KV head has several
         // 16-head groups.  Eight 4 KB stores by eight lanes were no faster than the one (4.31 against 4.20 ms)
-        bool good = mbar_wait(stg_full, n & 1, DEV_ERR_FULL_WAIT);
+        bool good = mbar_wait(stg_full + 8 * (n & 1), (n >> 1) & 1, DEV_ERR_FULL_WAIT);
         const int nvalid = min(kTokB, nA - mloc * kTokB);
         if (good && G16 == 1 && lane == 0 && nvalid > 0) {
           bf16* dst = a.part + (((long long)bh * a.rev_cap + ta_lo + mloc * kTokB) * (16 * D));
