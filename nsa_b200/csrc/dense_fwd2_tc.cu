@@ -123,39 +123,42 @@ __global__ void __launch_bounds__(kThreads, 1)
   asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
   if (warp == 0 || warp == 3) {
     // ------------------------------- TMA producers: Q and K (warp 0), V (warp 3) -------------------------
+    // These and the products P.V at head_dim 128 are issued under a lane number, not elected (elect_one): compressed branch, 64 heads,
+    // 8 x 8192 tokens, both elected 1037 us, neither 975, P.V alone 1069, TMA alone 980; 2 x 4096 tokens 99.3, 95.7, 100.9, 98.8.  P.V issued
+    // in one go gets ahead of the other group's S, which the soft-max waits for.  (S elected or not: 979 / 975, and 23.9 / 24.2 at 2 x 2080
+    // tokens, 32 heads, where all elected take 23.3; head_dim 64, 4 x 2048 tokens, window 87.4 / 88.2.)
     const bool is_k = warp == 0;
     const uint32_t full0 = is_k ? k_full0 : v_full0, empty0 = is_k ? k_empty0 : v_empty0, ring = is_k ? k_ring : v_ring;
     const CUtensorMap* tm = is_k ? &tmK : &tmV;
     uint32_t c = 0, ic = 0;
-    if (elect_one()) {
-      bool good = true;
-      for (int item = blockIdx.x; good && item < total; item += gridDim.x) {
-        const int hg = item % HG;
-        const SeqTile st = seq_tile(a.seq, kTok, ntile - 1 - item / HG);
-        if (st.t0 >= st.Tq) continue;
-        const Sched sc = make_sched<MODE>(a, st);
-        const int hk = hg / G16;
-        if (is_k) {
-          good = mbar_wait_abortable(q_free, (ic & 1) ^ 1, 101, abort_flag);
-          if (!good) break;
-          mbar_expect_tx(q_full, 2 * TILE);
-#pragma unroll
-          for (int t = 0; t < 2; ++t)
-#pragma unroll
-            for (int p = 0; p < NP; ++p)
-              tma_load_3d(q_s + t * TILE + p * PANEL, &tmQ, q_full, p * 64, hg * 16, (int)st.row0 + st.t0 + t * kTokT);
+    int good = 1;
+    for (int item = blockIdx.x; good && item < total; item += gridDim.x) {
+      const int hg = item % HG;
+      const SeqTile st = seq_tile(a.seq, kTok, ntile - 1 - item / HG);
+      if (st.t0 >= st.Tq) continue;
+      const Sched sc = make_sched<MODE>(a, st);
+      const int hk = hg / G16;
+      if (is_k) {
+        if (lane == 0) {
+          good = mbar_wait_abortable(q_free, (ic & 1) ^ 1, 101, abort_flag) ? 1 : 0;
+          if (good) mbar_expect_tx(q_full, 2 * TILE);
         }
-        for (int i = 0; i < sc.n; ++i, ++c) {
-          const uint32_t sl = c & 1;
-          good = mbar_wait_abortable(empty0 + 8 * sl, ((c >> 1) & 1) ^ 1, 102, abort_flag);
-          if (!good) break;
-          mbar_expect_tx(full0 + 8 * sl, TILE);
-#pragma unroll
-          for (int p = 0; p < NP; ++p)
-            tma_load_4d(ring + sl * TILE + p * PANEL, tm, full0 + 8 * sl, p * 64, hk, (sc.first + i) * 128, st.b);
-        }
-        ++ic;
+        good = __shfl_sync(0xffffffffu, good, 0);
+        if (good && lane < 2 * NP)   // lane = NP * tile + panel
+          tma_load_3d(q_s + (lane / NP) * TILE + (lane % NP) * PANEL, &tmQ, q_full, (lane % NP) * 64, hg * 16,
+                      (int)st.row0 + st.t0 + (lane / NP) * kTokT);
       }
+      for (int i = 0; good && i < sc.n; ++i, ++c) {
+        const uint32_t sl = c & 1;
+        if (lane == 0) {
+          good = mbar_wait_abortable(empty0 + 8 * sl, ((c >> 1) & 1) ^ 1, 102, abort_flag) ? 1 : 0;
+          if (good) mbar_expect_tx(full0 + 8 * sl, TILE);
+        }
+        good = __shfl_sync(0xffffffffu, good, 0);
+        if (good && lane < NP)
+          tma_load_4d(ring + sl * TILE + lane * PANEL, tm, full0 + 8 * sl, lane * 64, hk, (sc.first + i) * 128, st.b);
+      }
+      ++ic;
     }
   } else if (warp == 1) {
     // ------------------------------- MMA issuer: S ---------------------------------------------------
@@ -195,7 +198,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (warp == 2) {
     // ------------------------------- MMA issuer: P.V -------------------------------------------------
-    if (elect_one()) {
+    if (D == 64 ? elect_one() : lane == 0) {   // (see the producers)
       constexpr uint32_t idesc_pv = umma_idesc_bf16(128, D, 0, 1);
       uint32_t c0 = 0;            // tiles of the items before
       uint32_t npi = 0;           // items with tiles so far (= o_free phases the groups will have arrived on)
