@@ -20,6 +20,7 @@
 // 32768 tokens, compressed 3700 -> 1970; 1024 tokens, head_dim 64 (mma.sync before), compressed 654 -> 23.  Products issued
 // under elect_one instead of a lane number, so that issuing is no longer what takes the time: both together 4.11 -> 3.53 ms at
 // 8 x 8192 tokens (below full clocks), 128 -> 107 us at 2 x 2080 tokens, 32 heads.
+// At head_dim 64 they stay under the lane number: elected 8 x 4096 tokens, 64 heads, window 925 -> 1046 us, compressed 355 -> 382.
 // The keys of a 64-row CTA with P and dS in shared memory (this kernel's predecessor, still the selected branch's) took the same
 // number of products for half the keys.
 //
@@ -195,7 +196,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     } else if (warp == 1) {
       // ------------------------------- MMA issuer: dV(n), S^T(n+1) -----------------------------------------
-      if (N > 0 && elect_one()) {
+      if (N > 0 && (D == 64 ? lane == 0 : elect_one())) {
         constexpr uint32_t idesc_s = umma_idesc_bf16(128, 64, 0, 0), idesc_dv = umma_idesc_bf16(128, D, 0, 1);
         const uint64_t dk = umma_smem_desc(k_s, 0, 1024), dq_base = umma_smem_desc(q_ring, 0, 1024);
         const uint64_t ddo_base = umma_smem_desc(do_ring, PANEL, 1024);
@@ -234,7 +235,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     } else {
       // ------------------------------- MMA issuer: dK(n), dP^T(n+1) ----------------------------------------
-      if (N > 0 && elect_one()) {
+      if (N > 0 && (D == 64 ? lane == 0 : elect_one())) {
         constexpr uint32_t idesc_s = umma_idesc_bf16(128, 64, 0, 0), idesc_dk = umma_idesc_bf16(128, D, 0, 1);
         const uint64_t dv = umma_smem_desc(v_s, 0, 1024), ddo_base = umma_smem_desc(do_ring, 0, 1024);
         const uint64_t dq_base = umma_smem_desc(q_ring, PANEL, 1024);
