@@ -252,8 +252,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int cod
 // True in one lane, always the same, of a converged warp.  TMA and tcgen05 instructions take warp-uniform operands, and only under it
 // does the compiler know that one lane is active: under a condition on the lane number an instruction with a lane's operands cost a
 // TMA warp 850 + 52 x lanes cycles and a tcgen05.mma its thread ~60.  The dense K/V gradients of 8 x 8192 tokens went from 4.11 to
-// 3.53 ms with it.  The kernels issue under it but for the dense forward at head_dim 128, which is faster with its products P.V and its
-// TMA under a lane number (dense_fwd2_tc.cu), and sel_attn.cu and gather_probe.cu, whose boxes differ by lane.
+// 3.53 ms with it.  Not faster, and so under a lane number, are the TMA and P.V of the dense forward (dense_fwd2_tc.cu), all its products
+// and those of the dense K/V gradients at head_dim 64 (dense_kv_tc.cu); sel_attn.cu and gather_probe.cu were left so.
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));

@@ -123,10 +123,11 @@ __global__ void __launch_bounds__(kThreads, 1)
   asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
   if (warp == 0 || warp == 3) {
     // ------------------------------- TMA producers: Q and K (warp 0), V (warp 3) -------------------------
-    // These and the products P.V at head_dim 128 are issued under a lane number, not elected (elect_one): compressed branch, 64 heads,
-    // 8 x 8192 tokens, both elected 1037 us, neither 975, P.V alone 1069, TMA alone 980; 2 x 4096 tokens 99.3, 95.7, 100.9, 98.8.  P.V issued
-    // in one go gets ahead of the other group's S, which the soft-max waits for.  (S elected or not: 979 / 975, and 23.9 / 24.2 at 2 x 2080
-    // tokens, 32 heads, where all elected take 23.3; head_dim 64, 4 x 2048 tokens, window 87.4 / 88.2.)
+    // These, the products P.V and at head_dim 64 also S are issued under a lane number, not elected (elect_one).  Compressed branch, 64
+    // heads, 8 x 8192 tokens: all elected 1037 us, none 975, P.V alone 1069, TMA alone 980, S alone 979; 2 x 4096 tokens 99.3, 95.7, 100.9,
+    // 98.8, 95.8; 2 x 2080 tokens, 32 heads 23.3, 24.2, 24.5, 24.0, 23.9.  P.V issued in one go gets ahead of the other group's S, which the
+    // soft-max waits for.  head_dim 64, window, 8 x 4096 tokens, 64 heads: all elected 658, none 639, S alone 646; 3 x 1999, 32 heads: 66.5,
+    // 67.8, 67.5.
     const bool is_k = warp == 0;
     const uint32_t full0 = is_k ? k_full0 : v_full0, empty0 = is_k ? k_empty0 : v_empty0, ring = is_k ? k_ring : v_ring;
     const CUtensorMap* tm = is_k ? &tmK : &tmV;
@@ -163,7 +164,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   } else if (warp == 1) {
     // ------------------------------- MMA issuer: S ---------------------------------------------------
     // S of a group's tile c as soon as its K tile has landed and the group holds tile c - 1 in registers
-    if (elect_one()) {
+    if (D == 128 ? elect_one() : lane == 0) {   // (see the producers)
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128, 0, 0);
       uint32_t c = 0, ic = 0;     // tiles so far; items so far
       bool ok = true;
@@ -198,7 +199,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (warp == 2) {
     // ------------------------------- MMA issuer: P.V -------------------------------------------------
-    if (D == 64 ? elect_one() : lane == 0) {   // (see the producers)
+    if (lane == 0) {   // (see the producers)
       constexpr uint32_t idesc_pv = umma_idesc_bf16(128, D, 0, 1);
       uint32_t c0 = 0;            // tiles of the items before
       uint32_t npi = 0;           // items with tiles so far (= o_free phases the groups will have arrived on)
