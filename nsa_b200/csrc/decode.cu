@@ -28,11 +28,11 @@
 //                          then pooling and a warp top-n while the other warps go on;
 //   3. window (k, v) pairs and 4. selected (k, v) pairs: online soft-max per warp.
 // Every chain leaves its partial (maximum, sum, unnormalised output) of each branch in a caller-provided workspace (the split-KV
-// scheme of decode attention).  The CTAs of an item then merge its rows, in a fixed order: without clusters each warp two rows at a
-// time, from a scratch that the CTA's next item uses again while the ring fills with that item's tiles; with
+// scheme of decode attention).  The CTAs of an item then merge its rows, in a fixed order: without clusters each warp a row (of three warps
+// two rows) at a time, from a scratch that the CTA's next item uses again while the ring fills with that item's tiles; with
 // clusters each CTA its share of the rows, a row and branch per warp.  The scratch is to stay in L2 beside the caches that stream
 // through it: CTAs that share an SM fetch what they read for the last time under an evict-first policy.
-// Measured, 128 sequences of 4096 to 32768 keys, 4 KV heads, one CTA per SM / two: 164 / 146 us (4.7 TB/s); two without the policy
+// Measured, 128 sequences of 4096 to 32768 keys, 4 KV heads, one CTA per SM / two: 164 / 145 us (4.7 TB/s); two without the policy
 // 163, and with one row per warp at a time 165; a second kernel that merges (77 MB of partials written and read) 179; one
 // sequence of 4096 keys 18.9 us with the second kernel and 17.5 without.  Also tried, with the same bits: two accumulators per warp of
 // three, the chains' pairs in turn (185 us: twice the code); six warps in a CTA that shares its SM, on a ring of three pairs
@@ -381,6 +381,7 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
   after_previous();
   constexpr int kSlots = 2 * CONS, kProdW = decode_producers(CONS);
   constexpr int kOwn = kCons / CONS;   // chains of a warp
+  constexpr int kRows = kOwn, kLanes = 32 / kRows;   // rows that a warp merges at a time, lanes of one
   const int cl = CL ? ncl : 1;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -826,12 +827,12 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
     }
     named_bar_sync(1, cthreads);   // ps, pooled, fin and sel are reused by the next item
     ++it;
-    // ---- this item's rows: partials merged chain by chain, gated sum of the branches; two rows per warp at a time, a lane holds four
-    // channels of either half -------------------------------------------------------------------------------------------
-    for (int r2 = warp; cl == 1 && r2 < 8; r2 += CONS) {
-      const int row = 2 * r2 + (lane >> 4), c0 = 4 * (lane & 15);
+    // ---- this item's rows: partials merged chain by chain, gated sum of the branches (a lane holds four channels of every kRows-th of a
+    // row; two rows at a time where three warps share them) -----------------------------------------------------------------
+    for (int r0 = warp; cl == 1 && r0 < 16 / kRows; r0 += CONS) {
+      const int row = kRows * r0 + lane / kLanes, c0 = 4 * (lane % kLanes);
       const float4* base = reinterpret_cast<const float4*>(a.part + (long long)blockIdx.x * 3 * kCons * kPartFloats + row * D + c0);
-      float4 x[3][kCons][2];
+      float4 x[3][kCons][kRows];
       float e[3][kCons], inv[3], lse[3];
 #pragma unroll
       for (int br = 0; br < 3; ++br)
@@ -839,9 +840,9 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
         for (int w = 0; w < kCons; ++w) {
           e[br][w] = ml[(br * kCons + w) * 16 + row].x;
 #pragma unroll
-          for (int k = 0; k < 2; ++k) {
+          for (int k = 0; k < kRows; ++k) {
             x[br][w][k] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (e[br][w] != -INFINITY) x[br][w][k] = __ldcg(base + (br * kCons + w) * (kPartFloats / 4) + 16 * k);
+            if (e[br][w] != -INFINITY) x[br][w][k] = __ldcg(base + (br * kCons + w) * (kPartFloats / 4) + kLanes * k);
           }
         }
 #pragma unroll
@@ -857,15 +858,16 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
         inv[br] = L > 0.f ? 1.f / L : 0.f;
         lse[br] = L > 0.f ? (M + log2f(L)) * kLn2 : -INFINITY;
       }
-      float4 tot[2];
-      tot[0] = tot[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+      float4 tot[kRows];
+#pragma unroll
+      for (int k = 0; k < kRows; ++k) tot[k] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int br = 0; br < 3; ++br) {
         if (br == 2 && a.window <= 0) continue;
         bf16* out = br == 0 ? a.o_cmp : br == 1 ? a.o_slc : a.o_swa;
         const float gt = gates[br * 16 + row];
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
+        for (int k = 0; k < kRows; ++k) {
           float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
           for (int w = 0; w < kCons; ++w) {
@@ -876,15 +878,15 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
             v.w = fmaf(x[br][w][k].w, wt, v.w);
           }
           const __nv_bfloat162 b0 = __floats2bfloat162_rn(v.x, v.y), b1 = __floats2bfloat162_rn(v.z, v.w);
-          if (out) *reinterpret_cast<uint2*>(out + (qrow + row) * D + c0 + 64 * k) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+          if (out) *reinterpret_cast<uint2*>(out + (qrow + row) * D + c0 + 4 * kLanes * k) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
           const float2 f0 = __bfloat1622float2(b0), f1 = __bfloat1622float2(b1);
           tot[k].x += gt * f0.x; tot[k].y += gt * f0.y; tot[k].z += gt * f1.x; tot[k].w += gt * f1.y;
         }
-        if (a.lse && (lane & 15) == 0) a.lse[(long long)br * a.nseq * a.Hq + qrow + row] = lse[br];
+        if (a.lse && lane % kLanes == 0) a.lse[(long long)br * a.nseq * a.Hq + qrow + row] = lse[br];
       }
 #pragma unroll
-      for (int k = 0; k < 2; ++k)
-        *reinterpret_cast<uint2*>(a.o + (qrow + row) * D + c0 + 64 * k) = make_uint2(pack_bf16(tot[k].x, tot[k].y), pack_bf16(tot[k].z, tot[k].w));
+      for (int k = 0; k < kRows; ++k)
+        *reinterpret_cast<uint2*>(a.o + (qrow + row) * D + c0 + 4 * kLanes * k) = make_uint2(pack_bf16(tot[k].x, tot[k].y), pack_bf16(tot[k].z, tot[k].w));
     }
   }
   }
