@@ -21,10 +21,10 @@
 // query-major dQ kernel, which gathers every selected block again (32 KB per visit for 16 rows) and recomputes S and dP.
 //
 // Bound: the round trip of the two Q/dO stages (gather 1800 cycles, S, soft-max, dV and dK: 3650 cycles per batch) and shared
-// memory (3100 cycles of operands, arriving rows and stores).  Before, the soft-max warps were busy 3500 of 4070 cycles: each fetched
-// and addressed its row's lse, delta and gate (now the drain warps, once per row), divided by the batch count, did its arithmetic in
-// three unrolled variants (now one, two columns at a time), and the unrolled epilogue cost another 55 000 cycles a CTA.
-// 8 x 8192 tokens, 64 heads: 4.90 -> 4.08 ms; 65536 tokens: 5.0 -> 4.1; 2 x 2080 tokens, 32 heads: 153 -> 129 us.
+// memory (3100 cycles of operands, arriving rows and stores).  A row's lse, delta and gate are fetched once, by the drain warps: both
+// soft-max threads of a row fetching them, with a division by the batch count and three unrolled variants of the arithmetic, kept those
+// warps busy 3500 of 4070 cycles.  The epilogue is a loop: unrolled it cost 55 000 cycles a CTA in instruction fetches.
+// 8 x 8192 tokens, 64 heads: 4.90 -> 4.08 ms with both; 65536 tokens: 5.0 -> 4.1; 2 x 2080 tokens, 32 heads: 153 -> 129 us.
 // Every wait is bounded; on a time-out the role records an error and leaves its loop.
 #include "kernels.h"
 #include "tc.cuh"
@@ -51,7 +51,8 @@ constexpr uint32_t STAGE = 2 * Q_TILE;     // Q + dO
 constexpr uint32_t P_TILE = 128 * 128;     // [128 rows][64 keys]
 constexpr int kStages = 2;
 // K, V | Q and dO stages | two P/dS pairs | barriers | a batch's row data
-constexpr uint32_t kOffBar = 2 * KV_TILE + kStages * STAGE + 4 * P_TILE, kOffRow = kOffBar + 256, kSmem = kOffRow + 128 * 16;   // no room to align
+constexpr uint32_t kOffBar = 2 * KV_TILE + kStages * STAGE + 4 * P_TILE, kOffRow = kOffBar + 256, kSmem = kOffRow + 128 * 12 + 1024;
+static_assert(kSmem <= 227 * 1024, "with the bytes that it takes to align the tiles");
 constexpr uint32_t kTmemCols = 512;        // two S/dP buffers: S 0..63, dP 64..127 | 128..255; dV^T 256..319, dK^T 320..383
 constexpr uint32_t kColDV = 256, kColDK = 320, kColDQ = 384;   // dQ_part: 384..511
 
@@ -59,14 +60,11 @@ __global__ void __launch_bounds__(kThreads, 1)
     kv_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
                      const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const KvArgs a) {
   after_previous();
-  extern __shared__ __align__(1024) uint8_t kv_bwd_smem[];
-  uint8_t* const sgen = kv_bwd_smem;
-  const uint32_t sbase = smem_u32(kv_bwd_smem);
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = smem_u32(smem_raw);
+  const uint32_t sbase = (raw + 1023u) & ~1023u;   // the 128-byte swizzle repeats every 1024 bytes
+  uint8_t* const sgen = smem_raw + (sbase - raw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (sbase & 1023u) {   // the 128-byte swizzle repeats every 1024 bytes
-    if (threadIdx.x == 0) atomicCAS(&g_dev_error, 0, 330);
-    return;
-  }
   const uint32_t k_s = sbase, v_s = sbase + KV_TILE;
   const uint32_t ring = sbase + 2 * KV_TILE;
   const uint32_t p_s0 = ring + kStages * STAGE;   // two [P | dS] tile pairs
@@ -296,7 +294,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       const uint32_t lane_addr = (uint32_t)(32 * quad) << 16;
       const bool elected = warp == kDrainWarp && lane == 0;
       const long long head0 = (long long)b * a.Tq * a.Hq + hk * G16 * 16 + (row & 15);
-      float4* const row_s = reinterpret_cast<float4*>(sgen + kOffRow) + row;
+      float2* const row_ld = reinterpret_cast<float2*>(sgen + kOffRow) + row;
+      uint32_t* const row_gn = reinterpret_cast<uint32_t*>(sgen + kOffRow + 128 * 8) + row;
       // batch to be fetched next: place in its 16-head sub-group, sub-group; its token (two batches ahead of the publication)
       int fm = 0, fsub = 0, ft = nA > 0 ? list_token(j) : 0;
       float lse = 0.f, del = 0.f;
@@ -319,7 +318,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (n >= nb) return true;
         if (n > 0 && !mbar_wait(row_empty, (n - 1) & 1, DEV_ERR_EMPTY_WAIT)) return false;
         const uint32_t gn = (uint32_t)__bfloat16_as_ushort(g) << 16 | (lse > -INFINITY ? nv : 0);   // (a row that sees nothing: none)
-        *row_s = make_float4(-lse * kLog2e, -del, __uint_as_float(gn), 0.f);
+        *row_ld = make_float2(-lse * kLog2e, -del);
+        *row_gn = gn;
         mbar_arrive(row_full);
         fetch(n + 1);
         return true;
@@ -392,11 +392,13 @@ __global__ void __launch_bounds__(kThreads, 1)
     // for batch n+2 only after their bulk store has read it (stg_free of that pair).
     const uint64_t sl22 = pack_f32x2(sl2, sl2);
     uint8_t* const prow0 = sgen + (p_s0 - sbase) + row * 128;
-    const float4* const row_s = reinterpret_cast<const float4*>(sgen + kOffRow) + row;
+    const float2* const row_ld = reinterpret_cast<const float2*>(sgen + kOffRow) + row;
+    const uint32_t* const row_gn = reinterpret_cast<const uint32_t*>(sgen + kOffRow + 128 * 8) + row;
     for (int n = 0; ok && n < nb; ++n) {
       ok = mbar_wait(row_full, n & 1, DEV_ERR_FULL_WAIT);
       if (!ok) break;
-      const float4 ri = *row_s;
+      const float2 ri = *row_ld;
+      const uint32_t gn = *row_gn;
       mbar_arrive(row_empty);
       const uint32_t buf = n & 1, use = n >> 1;
       const uint32_t scol = tmem + lane_addr + buf * 128 + half * 32;
@@ -405,7 +407,6 @@ __global__ void __launch_bounds__(kThreads, 1)
       tc_fence_after();
       float p[32];
       tmem_ld32(scol, p);
-      const uint32_t gn = __float_as_uint(ri.z);
       const float gv = __uint_as_float(gn & 0xffff0000u);
       const int nrow = gn & 0xffff, nvis = nrow - 32 * half;   // visible keys of the block, of this half (0: a row that is not there)
       const uint64_t nl2 = pack_f32x2(ri.x, ri.x), g2 = pack_f32x2(gv, gv), nd2 = pack_f32x2(ri.y, ri.y);
