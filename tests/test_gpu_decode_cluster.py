@@ -40,7 +40,7 @@ def test_decode_batches_agree(Hkv, parts, seed):
     nsa._lib.device_status()
 
 
-@pytest.mark.parametrize("nseq", [2, 40])   # clusters, one CTA an item
+@pytest.mark.parametrize("nseq", [2, 30, 40])   # clusters, an SM an item, a CTA of half of an SM's warps an item
 def test_decode_passes_nan_on(nseq):
     """A NaN in a key, a value or the query makes the outputs that see it NaN, and no others."""
     import nsa_b200 as nsa

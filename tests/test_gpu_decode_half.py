@@ -3,13 +3,14 @@ either, so the blocks and the outputs are the same bit for bit.  Batches on both
 import pytest
 import torch
 
+from oracle import nsa_oracle as O
 from parity_util import DEV, close as _close
 
 pytestmark = pytest.mark.gpu
 
 
 # items (sequences x KV heads): 148 SMs; two CTAs per SM from 149 items on, but below 296 only up to 12 K (22 K with 295) keys, and up
-# to 444 only where lengths differ
+# to 444 only where lengths differ (test_equal_lengths)
 @pytest.mark.parametrize("nseq,Hkv,longest", [(150, 1, 700), (74, 2, 12000), (75, 2, 14000), (150, 2, 3000), (40, 4, 1), (300, 1, 1), (300, 1, 2100)])
 def test_blocks_do_not_depend_on_the_spread(nseq, Hkv, longest):
     import nsa_b200 as nsa
@@ -64,3 +65,48 @@ def test_outputs_do_not_depend_on_the_form(nseq, short, long):
     for name in pair:
         assert torch.equal(pair[name][1:], one[name][1:]), name
     nsa._lib.device_status()
+
+
+@pytest.mark.parametrize("nseq,Hkv,L", [(160, 1, 2100), (75, 4, 2100), (150, 3, 1000)])   # 160 items: pairs; 300: one CTA per SM; 450: pairs
+def test_equal_lengths(nseq, Hkv, L):
+    """Sequences of one length, up to three items per SM of which are not dealt to pairs of CTAs: the blocks of small batches."""
+    import nsa_b200 as nsa
+    from nsa_b200.decode import nsa_decode
+    torch.manual_seed(nseq)
+    gen = torch.Generator(device=DEV).manual_seed(nseq)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device=DEV).bfloat16()
+    k, v, q = rnd(nseq * L, Hkv, 128), rnd(nseq * L, Hkv, 128), rnd(nseq, 16 * Hkv, 128)
+    mod = nsa.NSAAttention(128, True, device=DEV, dtype=torch.bfloat16).requires_grad_(False)
+    run = lambda a, b: nsa_decode(mod, q[a:b], k[a * L:b * L], v[a * L:b * L], [L * i for i in range(b - a + 1)], return_parts=True)
+    o, parts = run(0, nseq)
+    for a in range(0, nseq, 30):
+        b = min(a + 30, nseq)
+        got, got_parts = run(a, b)
+        assert torch.equal(got_parts[4], parts[4][a:b])
+        _close("decode o, %d equal of %d" % (b - a, nseq), got, o[a:b])
+    nsa._lib.device_status()
+
+
+def test_rows_match_the_oracle():
+    """Rows of a batch that is dealt to pairs of CTAs (160 items) against the fp32 oracle on the kernel's compressed cache."""
+    import nsa_b200 as nsa
+    from nsa_b200.decode import compress_cache, nsa_decode
+    gen = torch.Generator().manual_seed(160)
+    r = lambda *s, m=1.0: (torch.randn(*s, generator=gen) * m).bfloat16().float()
+    lens = [(20, 40, 95, 300, 517, 700, 1061, 2048)[i % 8] for i in range(160)]
+    cu = [sum(lens[:i]) for i in range(161)]
+    q, k, v = r(160, 16, 128), r(cu[-1], 1, 128), r(cu[-1], 1, 128)
+    mod = nsa.NSAAttention(128, True, device=DEV, dtype=torch.bfloat16).requires_grad_(False)
+    for p in mod.parameters():
+        p.copy_(r(*p.shape, m=0.02))
+    d = lambda x: x.to(DEV, torch.bfloat16)
+    cache = compress_cache(mod, d(k), d(v), cu)
+    o = nsa_decode(mod, d(q), d(k), d(v), cu, cache)
+    nsa._lib.device_status()
+    ck, cv, _, cu_c = cache
+    weights = [t.detach().float().cpu() for c in (mod.compressor.compressor_k, mod.compressor.compressor_v) for t in (c.weight, c.bias)]
+    gate = [t.detach().float().cpu() for t in (mod.gating.weight, mod.gating.bias)]
+    for i in [*range(8), *range(152, 160)]:
+        s, c = slice(cu[i], cu[i + 1]), slice(cu_c[i], cu_c[i + 1])
+        ref, _ = O.nsa_decode_row(q[i], k[s], v[s], *weights, *gate, n_sel=16, window=512, ck=ck[c].cpu(), cv=cv[c].cpu())
+        _close("decode row %d of 160 (%d keys)" % (i, lens[i]), o[i], ref, atol=3e-2)   # (as for the rows of small batches)
