@@ -253,7 +253,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int cod
 // does the compiler know that one lane is active: under a condition on the lane number an instruction with a lane's operands cost a
 // TMA warp 850 + 52 x lanes cycles and a tcgen05.mma its thread ~60.  The dense K/V gradients of 8 x 8192 tokens went from 4.11 to
 // 3.53 ms with it.  Not faster, and so under a lane number, are the TMA and P.V of the dense forward (dense_fwd2_tc.cu), all its products
-// and those of the dense K/V gradients at head_dim 64 (dense_kv_tc.cu); sel_attn.cu and gather_probe.cu were left so.
+// and those of the dense K/V gradients at head_dim 64 (dense_kv_tc.cu), and the gathers of the query-major dQ (sel_block.cu); sel_attn.cu
+// and gather_probe.cu were left so.
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
