@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(kThreads, BWD ? 1 : 2)
             if (good) mbar_expect_tx(full_bar(stage), stage_bytes);
           }
           good = __shfl_sync(0xffffffffu, good, 0);
-          // one box per lane (K/V x column panel): a single thread issuing them back to back is several times slower
+          // one box per lane (K/V x column panel)
           if (good && lane < 2 * (D / 64)) {
             const uint32_t dst = sbase + stage * stage_bytes;
             const int p = lane >> 1;
