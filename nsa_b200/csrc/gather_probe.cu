@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1)
           ok = false;
           break;
         }
-        if (lane < NP)
+        if (lane < NP)   // (a lane per box: 2.85 ms at 4 x 8192 tokens, all slots visible, against 2.95 by one elected lane)
           tma_load_4d(sbase + s * slot_bytes + lane * panel_bytes, kv ? &tmV : &tmK, bar, lane * 64, hkv, blk * BS, b);
         ++issued;
         if (++slot == spw) slot = 0;
