@@ -318,6 +318,12 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* tm,
       "l"(tm), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "l"(pol)
       : "memory");
 }
+__device__ __forceinline__ float4 ld_l2(const float4* p, uint64_t pol) {   // past L1
+  float4 v;
+  asm volatile("ld.global.L1::no_allocate.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p), "l"(pol) : "memory");
+  return v;
+}
 // Bulk copy shared -> global (asynchronous, tracked by the issuing thread's bulk groups); both addresses 16-byte
 // aligned, bytes a multiple of 16.  The shared-memory writes it reads must be ordered before it by fence_proxy_async.
 __device__ __forceinline__ void bulk_store(void* dst, uint32_t src, uint32_t bytes) {

@@ -31,7 +31,9 @@
 // scheme of decode attention).  The CTAs of an item then merge its rows, in a fixed order: without clusters each warp a row (of three warps
 // two rows) at a time, from a scratch that the CTA's next item uses again while the ring fills with that item's tiles; with
 // clusters each CTA its share of the rows, a row and branch per warp.  The scratch is to stay in L2 beside the caches that stream
-// through it: CTAs that share an SM fetch what they read for the last time under an evict-first policy.
+// through it: CTAs that share an SM fetch what they read for the last time under an evict-first policy, the partials
+// themselves when they merge them (the rows of the compressed cache then stay for the next step: 128 sequences of 1024 to 4000 keys,
+// cache extended and decoded, 138 -> 135 us).
 // Measured, 128 sequences of 4096 to 32768 keys, 4 KV heads, one CTA per SM / two: 164 / 145 us (4.7 TB/s); two without the policy
 // 163, and with one row per warp at a time 165; a second kernel that merges (77 MB of partials written and read) 179; one
 // sequence of 4096 keys 18.9 us with the second kernel and 17.5 without.  Also tried, with the same bits: two accumulators per warp of
@@ -829,6 +831,7 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
     ++it;
     // ---- this item's rows: partials merged chain by chain, gated sum of the branches (a lane holds four channels of every kRows-th of a
     // row; two rows at a time where three warps share them) -----------------------------------------------------------------
+    const uint64_t once = l2_evict_first();
     for (int r0 = warp; cl == 1 && r0 < 16 / kRows; r0 += CONS) {
       const int row = kRows * r0 + lane / kLanes, c0 = 4 * (lane % kLanes);
       const float4* base = reinterpret_cast<const float4*>(a.part + (long long)blockIdx.x * 3 * kCons * kPartFloats + row * D + c0);
@@ -842,7 +845,8 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
 #pragma unroll
           for (int k = 0; k < kRows; ++k) {
             x[br][w][k] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (e[br][w] != -INFINITY) x[br][w][k] = __ldcg(base + (br * kCons + w) * (kPartFloats / 4) + kLanes * k);
+            const float4* src = base + (br * kCons + w) * (kPartFloats / 4) + kLanes * k;
+            if (e[br][w] != -INFINITY) x[br][w][k] = kOwn > 1 ? ld_l2(src, once) : __ldcg(src);
           }
         }
 #pragma unroll
