@@ -37,13 +37,13 @@ CFG = dict(B=8, T=8192, Hq=64, Hkv=4, D=128, block=32, stride=16, sel_block=64, 
 WORKLOAD = "configs[2]: NSAAttention module fwd+bwd bf16, B=8 T=8192 Hq=64 Hkv=4 D=128, cmp 32/16, sel 64 top-16, window 512"
 METRIC = "NSA fwd+bwd tokens/s"
 # ncu DRAM traffic, MB per 8192-token sequence (see run_gpu), and the build it was captured from
-NCU_TRAFFIC_COMMIT = "137dcb5"
-NCU_MB_PER_SEQ = {"select": 140, "cmp_fwd": 221, "swa_fwd": 243, "swa+cmp_dq": 405, "swa_dkv": 317, "cmp_dkv+reduce": 345,
+NCU_TRAFFIC_COMMIT = "536221e"
+NCU_MB_PER_SEQ = {"select": 140, "cmp_fwd": 222, "swa_fwd": 242, "swa+cmp_dq": 404, "swa_dkv": 319, "cmp_dkv+reduce": 346,
                   "compress_fwd": 19, "compress_bwd": 55,
-                  # key-major forward 453 read + 1046 written, its merge with the gated sum 1379 + 229
-                  "sel_fwd+gated_sum": 3107,
-                  # key-major backward 1172 read + 1082 written, the reduction of the dQ partials 1211 + 84
-                  "sel_bwd+reduce": 3549}
+                  # key-major forward 454 read + 1046 written, its merge with the gated sum 1379 + 229
+                  "sel_fwd+gated_sum": 3108,
+                  # key-major backward 1166 read + 1082 written, the reduction of the dQ partials 1211 + 85
+                  "sel_bwd+reduce": 3544}
 
 
 # ---------------------------------------------------------------------------------------------------------

@@ -13,8 +13,9 @@
 // bf16.
 //
 // A CTA is a serial chain of l * D / 64 stages however few rows there are; one stage takes 300 cycles with half of the columns,
-// about what its 24 KB take from L2.  With a 64-bit division per stage and TMA instructions whose operands differed by lane it
-// took 600: 5008 tokens of 4 heads 22.6 -> 15.6 us, eight sequences with 38100 tokens in all 54 -> 43 us.
+// about what its 24 KB take from L2 (600 with a 64-bit division per stage and TMA instructions whose operands differ by lane;
+// without these, and with the tile that fits the rows, below: 5008 tokens of 4 heads 22.6 -> 15.6 us, eight sequences with 38100
+// tokens in all 54 -> 43 us).
 // Where the caller allows it (`split`) the contraction is split over a cluster of up to eight CTAs when
 // that shortens the waves; the partial accumulators meet in distributed shared memory and are added in rank order.  The
 // package does not allow it anywhere: a block selection turns last-bit differences of ck into other blocks, and with one

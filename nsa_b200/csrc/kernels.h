@@ -11,7 +11,7 @@ namespace nsa {
 // ---- launches ---------------------------------------------------------------------------------
 // Programmatic dependent launch: the next grid is set up while the one before it in the stream ends, and its blocks wait for the
 // results at their start (after_previous()).  A step is some 24 kernels, with plain launches about 2 us apart.  Plain -> so: a
-// training step of 2 x 2080 tokens 877 -> 821 us, a prompt of 5003 tokens 767 -> 734, a decode step of one sequence 17.8 -> 15.9 and of 32
+// training step of 2 x 2080 tokens 868 -> 821 us, a prompt of 5003 tokens 767 -> 734, a decode step of one sequence 17.8 -> 15.9 and of 32
 // with its cache extended 89 -> 78; no case slower.
 inline cudaLaunchConfig_t next_config(dim3 grid, dim3 block, size_t smem, cudaStream_t s, cudaLaunchAttribute* at) {
   cudaLaunchConfig_t c = {};
