@@ -463,9 +463,13 @@ __global__ void __launch_bounds__(decode_threads(CONS), CONS == kCons ? 1 : 2)
     };
     // the n pairs of a phase as the warps take them: those of the first CONS chains, then (CONS < kCons) of the others
     auto each_pair = [&](int n, bool& ok, auto&& issue) {
-      for (int e = 0; e < kCons; e += CONS)
-        for (int c = e; c < n; c += kCons)
-          for (int i = c; ok && i < min(c + CONS, n); ++i) ok = issue(i);
+      if constexpr (kOwn == 1) {
+        for (int i = 0; ok && i < n; ++i) ok = issue(i);
+      } else {
+        for (int e = 0; e < kCons; e += CONS)
+          for (int c = e; c < n; c += kCons)
+            for (int i = c; ok && i < min(c + CONS, n); ++i) ok = issue(i);
+      }
     };
     for (int r = 0; r * ngroup < nitem; ++r) {
       const int item = snake_item(r, group, ngroup);
