@@ -34,7 +34,7 @@
 // through it: CTAs that share an SM fetch what they read for the last time under an evict-first policy, the partials
 // themselves when they merge them (the rows of the compressed cache then stay for the next step: 128 sequences of 1024 to 4000 keys,
 // cache extended and decoded, 138 -> 135 us).
-// Measured, 128 sequences of 4096 to 32768 keys, 4 KV heads, one CTA per SM / two: 164 / 145 us (4.7 TB/s); two without the policy
+// Measured, 128 sequences of 4096 to 32768 keys, 4 KV heads, one CTA per SM / two: 164 / 140 us (4.9 TB/s); two without the policies
 // 163, and with one row per warp at a time 165; a second kernel that merges (77 MB of partials written and read) 179; one
 // sequence of 4096 keys 18.9 us with the second kernel and 17.5 without.  Also tried, with the same bits: two accumulators per warp of
 // three, the chains' pairs in turn (185 us: twice the code); six warps in a CTA that shares its SM, on a ring of three pairs
@@ -953,7 +953,7 @@ int ask_resident(int cl) {
 // its blocks or merges its rows.  Below two items per SM such a CTA has one item and takes 32 us + 1.2 us per 1000 keys for the
 // longest, against two items, a long and a short one, behind each other.  One CTA per SM -> two, 4 KV heads, lengths from 1024 up to the
 // given one: 152 items of 4000 keys 44.2 -> 36.9 us, 192 of 9000 51.2 -> 45.4, 272 of 16000 68.4 -> 58.9; but 152 of 20000 46.6 -> 56.5, 168 of
-// 26000 54.9 -> 63.8, 248 of 32000 75.7 -> 77.6, so not there.  512 items of 4096 to 32768 keys 164 -> 146, 512 of 1500 99 -> 85.
+// 26000 54.9 -> 63.8, 248 of 32000 75.7 -> 77.6, so not there.  512 items of 4096 to 32768 keys 164 -> 140, 512 of 1500 99 -> 85.
 // Three rounds of equal items are no more than two of pairs, the second half empty: 300 to 444 items of 32000 keys 160 to 179 us, as
 // pairs 169 to 184 (of 12000 100 to 114, 103 to 114); four are: 452 of 32000 218 -> 185.
 struct Spread {
