@@ -34,7 +34,7 @@
 // through it: CTAs that share an SM fetch what they read for the last time under an evict-first policy, the partials
 // themselves when they merge them (the rows of the compressed cache then stay for the next step: 128 sequences of 1024 to 4000 keys,
 // cache extended and decoded, 138 -> 135 us).
-// Measured, 128 sequences of 4096 to 32768 keys, 4 KV heads, one CTA per SM / two: 164 / 140 us (4.9 TB/s); two without the policies
+// Measured, 128 sequences of 4096 to 32768 keys, 4 KV heads, one CTA per SM / two: 164 / 140 to 144 us (4.7 to 4.9 TB/s); two without the policies
 // 163, and with one row per warp at a time 165; a second kernel that merges (77 MB of partials written and read) 179; one
 // sequence of 4096 keys 18.9 us with the second kernel and 17.5 without.  Also tried, with the same bits: two accumulators per warp of
 // three, the chains' pairs in turn (185 us: twice the code); six warps in a CTA that shares its SM, on a ring of three pairs
